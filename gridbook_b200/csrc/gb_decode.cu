@@ -498,6 +498,241 @@ int launch_expand_fp8_fast(const gb_weight* w, int64_t row0, int64_t nrows, void
   GB_LAUNCH_OK("expand_fp8_fast_kernel");
   return GB_OK;
 }
+
+// ---- product formats of any width, fast -----------------------------------------------------
+// fp4 grid, two sub-indices (K12 .. K24, either scale coding) and fp8 grid, four sub-indices (ragged
+// rungs included) -> the native NVFP4 pair, the E4M3 plane or the bf16 tile.  The generic kernel
+// above gathers eight values one by one from global memory and converts each: 566 us for the NVFP4
+// view of a 34816 x 5120 K20 layer (0.29 TB/s of 233 bytes moved per superblock).  Here a sub-index
+// is ONE shared-memory lookup of its finished output bits (four E2M1 nibbles or two E4M3 bytes: a
+// 16-bit entry; four bf16: an 8-byte entry), the scale byte comes out of a 4096-entry table, and
+// eight lanes share a superblock so that every store instruction writes 128 contiguous bytes: bound
+// by memory from about K20 down, by the lookups (bank conflicts between random entries; copies
+// interleaved per lane where they fit) above.
+// A CTA takes a contiguous run of rows; where the rows change codebook (fused modules with one
+// book per role) it rebuilds its tables.
+constexpr int kProdThreads = 512;
+constexpr int kProdLutCap = 64 * 1024;                     // three CTAs per SM keep the loads in flight
+
+GB_DEVINL uint32_t e2m1_nibble(uint32_t bf16_bits) {
+  const float v = gb_bf16_bits_to_f32(bf16_bits), m = fabsf(v);
+  const uint32_t c = m < 2.0f ? (uint32_t)(m * 2.0f) : (m < 4.0f ? (uint32_t)m + 2u : (m < 6.0f ? 6u : 7u));
+  return c | (v < 0.0f ? 8u : 0u);
+}
+
+struct ProdArgs {
+  ExpandArgs a;
+  int entries;        // sub-table entries of one codebook block
+  int copies;         // interleaved copies of every entry (a power of two)
+  int n_sb;
+  int64_t rows_per_cta;
+};
+
+// Bits [bit, bit + n) of the stream at `p` (any alignment), n <= 64: only words that hold a wanted bit are read.
+GB_DEVINL uint64_t stream_bits(const uint8_t* p, uint32_t bit, int n) {
+  const uintptr_t at = (uintptr_t)p + (bit >> 3);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(at & ~(uintptr_t)3);
+  const uint32_t s = ((uint32_t)(at & 3u) << 3) | (bit & 7u);
+  const uint32_t w0 = __ldg(w), w1 = s + n > 32 ? __ldg(w + 1) : 0u, w2 = s + n > 64 ? __ldg(w + 2) : 0u;
+  const uint64_t lo = __funnelshift_r(w0, w1, s), hi = __funnelshift_r(w1, w2, s);
+  const uint64_t v = lo | (hi << 32);
+  return n >= 64 ? v : v & ((1ull << n) - 1ull);
+}
+
+template <int kOut>
+__global__ void __launch_bounds__(kProdThreads)
+expand_product_kernel(const __grid_constant__ ProdArgs p, void* __restrict__ out0, uint8_t* __restrict__ out_sf,
+                      int fold_sign) {
+  constexpr bool kFp8 = kOut == kOutFp8 || kOut == kOutFp8Bf16;
+  constexpr bool kWide = kOut == kOutBf16;                 // 8-byte entries
+  constexpr int kSubs = kFp8 ? 4 : 2;
+  extern __shared__ uint8_t smem[];
+  __shared__ int run_end_s;
+  const ExpandArgs& a = p.a;
+  uint8_t* comp_s = smem;                                  // two-tier scale bytes (NVFP4 output only)
+  uint8_t* lut_s = smem + (kOut == kOutNvfp4 ? 4096 : 0);
+  const int tid = threadIdx.x, lane = tid & 31, sub = lane & 7, which = lane >> 3;
+  const int k = a.fmt.k_bits;
+  const bool v2 = a.fmt.scale_coding == GB_SCALE_V2;
+  const uint32_t my = (uint32_t)(sub & (p.copies - 1));
+  if (kOut == kOutNvfp4 && v2)
+    for (int i = tid; i < 4096; i += kProdThreads) comp_s[i] = (uint8_t)gb_f32_to_e4m3(fminf(__ldg(a.compose + i), 448.0f));
+
+  const int64_t r_begin = (int64_t)blockIdx.x * p.rows_per_cta;
+  const int64_t r_end = r_begin + p.rows_per_cta < a.nrows ? r_begin + p.rows_per_cta : a.nrows;
+  for (int64_t run = r_begin; run < r_end;) {
+    int64_t cb_base = 0, run_end = r_end;
+    if (a.cb_row_offset) {                                 // rows [run, run_end) use one codebook block
+      cb_base = a.cb_row_offset[a.row0 + run];
+      __syncthreads();
+      if (tid == 0) run_end_s = (int)(r_end - run);
+      __syncthreads();
+      for (int64_t r = run + tid; r < r_end; r += kProdThreads)
+        if (a.cb_row_offset[a.row0 + r] != (int32_t)cb_base) { atomicMin(&run_end_s, (int)(r - run)); break; }
+      __syncthreads();
+      run_end = run + run_end_s;
+    }
+    for (int e = tid; e < p.entries; e += kProdThreads) {
+      if constexpr (kFp8) {
+        const uint8_t* c = reinterpret_cast<const uint8_t*>(a.codebook) + cb_base + (int64_t)e * 2;
+        const uint16_t v = (uint16_t)(c[0] | (c[1] << 8));
+        for (int j = 0; j < p.copies; ++j) reinterpret_cast<uint16_t*>(lut_s)[e * p.copies + j] = v;
+      } else {
+        const uint16_t* c = reinterpret_cast<const uint16_t*>(a.codebook) + cb_base + (int64_t)e * 4;
+        const uint32_t c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
+        if constexpr (kWide) {
+          for (int j = 0; j < p.copies; ++j)
+            reinterpret_cast<uint2*>(lut_s)[e * p.copies + j] = make_uint2(c0 | (c1 << 16), c2 | (c3 << 16));
+        } else {
+          const uint16_t v = (uint16_t)(e2m1_nibble(c0) | (e2m1_nibble(c1) << 4) | (e2m1_nibble(c2) << 8) | (e2m1_nibble(c3) << 12));
+          for (int j = 0; j < p.copies; ++j) reinterpret_cast<uint16_t*>(lut_s)[e * p.copies + j] = v;
+        }
+      }
+    }
+    __syncthreads();
+
+    // entry offset of sub-index i inside the table
+    uint32_t base[kSubs], mask[kSubs];
+    int shift[kSubs];
+#pragma unroll
+    for (int i = 0; i < kSubs; ++i) {
+      base[i] = (uint32_t)(a.split.base[i] / a.split.sub_dim);
+      mask[i] = (1u << a.split.width[i]) - 1u;
+      shift[i] = a.split.shift[i];
+    }
+    auto entry = [&](uint64_t code, int i) { return (base[i] + ((uint32_t)(code >> shift[i]) & mask[i])) * (uint32_t)p.copies + my; };
+    auto lut16 = [&](uint64_t code, int i) { return (uint32_t)reinterpret_cast<const uint16_t*>(lut_s)[entry(code, i)]; };
+
+    const int64_t units = (run_end - run) * p.n_sb;
+    for (int64_t u = (int64_t)(tid >> 5) * 4 + which; u < units; u += kProdThreads / 8) {
+      const uint32_t rr = (uint32_t)u / (uint32_t)p.n_sb;  // rows_per_cta * n_sb fits 32 bits
+      const int s = (int)((uint32_t)u - rr * (uint32_t)p.n_sb);
+      const int64_t r = run + rr;
+      const uint8_t* sb = a.qw + r * a.row_stride + (int64_t)s * a.fmt.type_size;
+      const uint8_t* plane = sb + 4 * k;
+      const int64_t at = r * a.K + (int64_t)s * 256;
+      if constexpr (kOut == kOutNvfp4) {
+        // four neighbouring codewords, one 16-byte store
+        const uint64_t ca = stream_bits(sb, (uint32_t)(sub * 4 * k), 2 * k), cb = stream_bits(sb, (uint32_t)(sub * 4 + 2) * k, 2 * k);
+        const uint64_t m = (1ull << k) - 1ull;
+        const uint64_t code[4] = {ca & m, ca >> k, cb & m, cb >> k};
+        uint32_t w[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) w[c] = lut16(code[c], 0) | (lut16(code[c], 1) << 16);
+        uint32_t sc2, sc4 = 0;                             // the lane's two groups; atom `sub`'s four groups
+        if (v2) {
+          const uint8_t* t = comp_s + (uint32_t)plane[0] * 16u;
+          const uint32_t n2 = plane[1 + sub];
+          sc2 = t[n2 & 15u] | ((uint32_t)t[n2 >> 4] << 8);
+          if (sub < 4) {
+            const uint32_t n0 = plane[1 + 2 * sub], n1 = plane[2 + 2 * sub];
+            sc4 = t[n0 & 15u] | ((uint32_t)t[n0 >> 4] << 8) | ((uint32_t)t[n1 & 15u] << 16) | ((uint32_t)t[n1 >> 4] << 24);
+          }
+        } else {
+          sc2 = plane[2 * sub] | ((uint32_t)plane[2 * sub + 1] << 8);
+          if (sub < 4)
+            sc4 = plane[4 * sub] | ((uint32_t)plane[4 * sub + 1] << 8) | ((uint32_t)plane[4 * sub + 2] << 16) |
+                  ((uint32_t)plane[4 * sub + 3] << 24);
+        }
+        if (fold_sign) {                                   // UE4M3 scale factors carry no sign
+          if (sc2 & 0x80u) { w[0] ^= 0x88888888u; w[1] ^= 0x88888888u; }
+          if (sc2 & 0x8000u) { w[2] ^= 0x88888888u; w[3] ^= 0x88888888u; }
+          sc4 &= 0x7F7F7F7Fu;
+        }
+        reinterpret_cast<uint4*>(out0)[(at >> 5) + sub] = make_uint4(w[0], w[1], w[2], w[3]);
+        if (sub < 4) {
+          const int64_t off = (r / 128) * (512 * (int64_t)p.n_sb * 4) + ((int64_t)s * 4 + sub) * 512 + (r % 32) * 16 + ((r / 32) % 4) * 4;
+          *reinterpret_cast<uint32_t*>(out_sf + off) = sc4;
+        }
+      } else if constexpr (kOut == kOutFp8) {
+        // two codewords of each half of the superblock: two 16-byte stores
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t w[4];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const uint64_t code = stream_bits(sb, (uint32_t)(h * 16 + sub * 2 + c) * k, k);
+            w[2 * c] = lut16(code, 0) | (lut16(code, 1) << 16);
+            w[2 * c + 1] = lut16(code, 2) | (lut16(code, 3) << 16);
+          }
+          reinterpret_cast<uint4*>(out0)[(at >> 4) + h * 8 + sub] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      } else {
+        // bf16(value * scale), the product taken in fp32: one codeword per 16-byte store
+        const float rs = kOut == kOutFp8Bf16 ? __ldg(a.weight_scale + a.row0 + r) : 0.0f;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const int v = h * 8 + sub;
+          const uint64_t code = stream_bits(sb, (uint32_t)(v * k), k);
+          uint32_t w[4];
+          if constexpr (kOut == kOutFp8Bf16) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t e2 = lut16(code, i);
+              w[i] = gb_pack_bf16x2(__fmul_rn(gb_e4m3_to_f32(e2 & 0xFFu), rs), __fmul_rn(gb_e4m3_to_f32(e2 >> 8), rs));
+            }
+          } else {
+            const int g = v >> 1;
+            float sc;
+            if (v2) sc = __ldg(a.compose + (uint32_t)plane[0] * 16u + ((plane[1 + (g >> 1)] >> ((g & 1) * 4)) & 0xFu));
+            else sc = gb_e4m3_to_f32(plane[g]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const uint2 e = reinterpret_cast<const uint2*>(lut_s)[entry(code, i)];
+              w[2 * i] = gb_pack_bf16x2(__fmul_rn(__uint_as_float(e.x << 16), sc), __fmul_rn(__uint_as_float(e.x & 0xFFFF0000u), sc));
+              w[2 * i + 1] = gb_pack_bf16x2(__fmul_rn(__uint_as_float(e.y << 16), sc), __fmul_rn(__uint_as_float(e.y & 0xFFFF0000u), sc));
+            }
+          }
+          reinterpret_cast<uint4*>(out0)[(at >> 3) + v] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+    }
+    run = run_end;
+    if (run < r_end) __syncthreads();                      // the next run rebuilds the tables
+  }
+}
+
+// Whether the product kernel takes the weight: the mode it decodes, sub-tables that fit shared
+// memory, 16-byte stores.
+bool product_serves(const gb_weight* w, const void* out, int kout) {
+  const gb_format& f = w->fmt;
+  if (f.mode != GB_MODE_PRODUCT || f.n_sub != (f.grid == GB_GRID_FP8 ? 4 : 2) || ((uintptr_t)out & 15u) != 0) return false;
+  if (f.grid == GB_GRID_FP4 && f.k_bits > 32) return false;
+  const int64_t entry_bytes = kout == kOutBf16 ? 8 : 2;
+  const int64_t entries = gb_codebook_elems(f) / (8 / f.n_sub);
+  return entries * entry_bytes <= kProdLutCap;
+}
+
+template <int kOut>
+int launch_expand_product(const gb_weight* w, int64_t row0, int64_t nrows, void* out0, void* out_sf, int fold_sign,
+                          void* stream) {
+  ProdArgs p = {};
+  int rc = make_expand_args(w, row0, nrows, &p.a);
+  if (rc != GB_OK) return rc;
+  p.a.qw = w->qw + row0 * w->row_stride;
+  p.n_sb = (int)(w->K / 256);
+  p.entries = (int)(gb_codebook_elems(w->fmt) / (8 / w->fmt.n_sub));
+  const int entry_bytes = kOut == kOutBf16 ? 8 : 2;
+  p.copies = 8;
+  while (p.copies > 1 && p.entries * entry_bytes * p.copies > kProdLutCap) p.copies >>= 1;
+  const int smem = p.entries * entry_bytes * p.copies + (kOut == kOutNvfp4 ? 4096 : 0);
+  const int sms = gb_sm_count();
+  if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
+  const int per_sm = smem * 4 <= 200 * 1024 ? 4 : smem * 3 <= 216 * 1024 ? 3 : 2;
+  // one wave of CTAs over the rows, at least 64 superblocks each so that the tables pay
+  int64_t rows_per = (nrows + (int64_t)sms * per_sm - 1) / ((int64_t)sms * per_sm);
+  const int64_t least = (64 + p.n_sb - 1) / p.n_sb;
+  if (rows_per < least) rows_per = least;
+  GB_REQUIRE(rows_per * p.n_sb < (1ll << 31), "too many superblocks per CTA");
+  p.rows_per_cta = rows_per;
+  const unsigned blocks = (unsigned)((nrows + rows_per - 1) / rows_per);
+  if (smem > 48 * 1024)
+    GB_CUDA_OK(cudaFuncSetAttribute((const void*)expand_product_kernel<kOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  gb_count_launch();
+  expand_product_kernel<kOut><<<blocks, kProdThreads, smem, (cudaStream_t)stream>>>(p, out0, (uint8_t*)out_sf, fold_sign);
+  GB_LAUNCH_OK("expand_product_kernel");
+  return GB_OK;
+}
 }  // namespace
 
 extern "C" {
@@ -517,16 +752,19 @@ int gb_expand_fp8(const gb_weight* w, int64_t row0, int64_t nrows, void* out, vo
     if (nrows == 0) return GB_OK;
     return launch_expand_fp8_fast(w, row0, nrows, out, stream);
   }
+  if (product_serves(w, out, kOutFp8)) return launch_expand_product<kOutFp8>(w, row0, nrows, out, nullptr, 0, stream);
   return launch_expand<kOutFp8>(w, row0, nrows, out, nullptr, 0, stream);
 }
 
 int gb_expand_fp8_bf16(const gb_weight* w, int64_t row0, int64_t nrows, void* out, void* stream) {
   GB_REQUIRE(w && w->fmt.grid == GB_GRID_FP8 && w->weight_scale, "gb_expand_fp8_bf16 wants an fp8-grid weight with its row scales");
+  if (product_serves(w, out, kOutFp8Bf16)) return launch_expand_product<kOutFp8Bf16>(w, row0, nrows, out, nullptr, 0, stream);
   return launch_expand<kOutFp8Bf16>(w, row0, nrows, out, nullptr, 0, stream);
 }
 
 int gb_expand_fp4_bf16(const gb_weight* w, int64_t row0, int64_t nrows, void* out, void* stream) {
   GB_REQUIRE(w && w->fmt.grid == GB_GRID_FP4, "gb_expand_fp4_bf16 wants an fp4-grid weight");
+  if (product_serves(w, out, kOutBf16)) return launch_expand_product<kOutBf16>(w, row0, nrows, out, nullptr, 0, stream);
   return launch_expand<kOutBf16>(w, row0, nrows, out, nullptr, 0, stream);
 }
 
@@ -546,6 +784,8 @@ int gb_expand_fp4_nvfp4(const gb_weight* w, int64_t row0, int64_t nrows, void* o
     if (nrows == 0) return GB_OK;
     return launch_expand_literal(w, row0, nrows, out_packed, out_sf, sf_swizzled == 2, stream);
   }
+  if (sf_swizzled != 0 && ((uintptr_t)out_sf & 3u) == 0 && product_serves(w, out_packed, kOutNvfp4))
+    return launch_expand_product<kOutNvfp4>(w, row0, nrows, out_packed, out_sf, sf_swizzled == 2, stream);
   return launch_expand<kOutNvfp4>(w, row0, nrows, out_packed, out_sf, sf_swizzled, stream);
 }
 

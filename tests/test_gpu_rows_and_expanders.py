@@ -1,0 +1,107 @@
+"""Edges of the row kernels and of the product-format expanders: rows of every register count and the
+longer ones, values on and next to the rounding boundaries, codebooks that change inside and between
+the row runs of a CTA, one row, ragged row counts."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import cb_oracle as O
+from oracle import oracle_kwargs
+from tests.helpers import bits_of, nvfp4_quantize_rows_ref, oracle_weight
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    from gridbook_b200 import _native
+    _native.prepare(0)
+    return torch.device("cuda:0")
+
+
+def _near_boundaries(M, K, seed):
+    """Rows whose values sit on, one bf16 step above and one below grid midpoints of their scale."""
+    rng = np.random.default_rng(seed)
+    x = rng.standard_normal((M, K)).astype(np.float32) * np.exp2(rng.integers(-12, 12, (M, 1))).astype(np.float32)
+    g = x[:, :K // 16 * 16].reshape(M, -1, 16)
+    amax = np.abs(g).max(axis=-1)
+    mids = np.array([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0], np.float32) / 6.0
+    for j in range(1, 8):
+        g[:, ::2, j] = amax[:, ::2] * mids[j - 1] * (1.0 if j % 2 else -1.0)
+    b = O.f32_to_bf16_bits(x).astype(np.int64) + rng.integers(-1, 2, (M, K))
+    return O.bf16_bits_to_f32(np.clip(b, 0, 65535).astype(np.uint16))
+
+
+@pytest.mark.parametrize("K", [16, 1040, 4096, 5120, 8192, 17408, 40960, 65536 + 16])
+def test_row_buckets_are_bit_exact(dev, K):
+    from gridbook_b200 import kernels
+    M = 3 if K > 8192 else 33
+    x = _near_boundaries(M, K, K)
+    x[-1] = 0.0
+    x = np.where(np.isfinite(x), x, np.float32(1.0)).astype(np.float32)
+    xd = torch.from_numpy(x).to(torch.bfloat16).to(dev)
+    for rule in ("recip", "div"):
+        assert np.array_equal(bits_of(kernels.fp4_act_qdq(xd, rule)), O.f32_to_bf16_bits(O.fp4_group16_act_qdq(x, rule)))
+        want = O.f32_to_bf16_bits(O.fp8_dynamic_act_qdq(x, rule))
+        assert np.array_equal(bits_of(kernels.fp8_act_qdq(xd, rule)), want)
+        q, s = kernels.fp8_quantize_rows(xd, rule)
+        back = (q.float() * s[:, None]).to(torch.bfloat16)
+        assert np.array_equal(bits_of(back), want)
+    if K % 64 == 0:
+        packed, sf, a_scale = kernels.nvfp4_quantize_rows(xd)
+        rp, rs, ra = nvfp4_quantize_rows_ref(x)
+        assert np.array_equal(packed.cpu().numpy(), rp)
+        assert np.array_equal(a_scale.cpu().numpy(), ra)
+        assert np.array_equal(sf.cpu().numpy(), O.swizzle_sf_plane(rs))
+
+
+def _formats():
+    from gridbook_b200.formats import CBFormat
+    fp4 = [CBFormat("fp4", k, n_sub=2, scale_coding=c) for k, c in ((12, "v2"), (13, "v1"), (16, "v2"), (20, "v2"), (21, "v1"), (24, "v2"))]
+    return fp4 + [fp4[2].padded(80)] + [CBFormat("fp8", k, n_sub=4) for k in (28, 30, 33, 48)]
+
+
+@pytest.mark.parametrize("rows,K,books", [(1, 256, 1), (129, 512, 3), (1000, 1024, 7)])
+@pytest.mark.parametrize("idx", range(11))
+def test_product_expanders_are_bit_exact(dev, idx, rows, K, books):
+    from gridbook_b200 import kernels, synth
+    fmt = _formats()[idx]
+    if books == 7 and fmt.k > 24 and not fmt.is_fp4 and fmt.k == 48:
+        books = 2
+    base = fmt if fmt.sb_pad == 0 else fmt.padded(fmt.packed_type_size)
+    d = synth.make_linear(base, rows, K, seed=rows + idx, n_books=books, super_span=None)
+    up = d
+    if fmt.sb_pad:
+        from gridbook_b200 import codec
+        up = dict(d, fmt=fmt, qw=codec.pad_superblocks(torch.from_numpy(d["qw"]), base.type_size, fmt.type_size).numpy())
+    w = synth.to_device_weight(up, dev)
+    ref = O.f32_to_bf16_bits(oracle_weight(d))
+    lo, n = rows // 3, max(1, rows // 2)
+    off = d["cb_row_offset"] if d["cb_row_offset"] is not None else np.zeros(rows, np.int32)
+    if fmt.is_fp4:
+        assert np.array_equal(bits_of(kernels.expand_fp4_bf16(w)), ref)
+        assert np.array_equal(bits_of(kernels.expand_fp4_bf16(w, lo, n)), ref[lo:lo + n])
+        rp, rs = O.decode_nvfp4_tile(d["qw"], d["cb"], off, N=rows, K=K, compose=d["compose"],
+                                     **{k: v for k, v in oracle_kwargs(base).items() if k != "grid"})
+        packed, sf = kernels.expand_fp4_nvfp4(w, swizzled=True)
+        assert np.array_equal(packed.cpu().numpy(), rp)
+        assert np.array_equal(sf.cpu().numpy(), O.swizzle_sf_plane(rs))
+    else:
+        vals = O.decode_values(d["qw"], d["cb"], off, N=rows, K=K, k_bits=base.k, n_sub=base.n_sub, type_size=base.type_size)
+        assert np.array_equal(kernels.expand_fp8(w).view(torch.uint8).cpu().numpy(), O.f32_to_e4m3(vals))
+        assert np.array_equal(bits_of(kernels.expand_fp8_bf16(w)), ref)
+        assert np.array_equal(bits_of(kernels.expand_fp8_bf16(w, lo, n)), ref[lo:lo + n])
+
+
+@pytest.mark.parametrize("T,topk,H", [(1, 1, 2), (3, 8, 2048), (700, 5, 2048), (2500, 8, 258)])
+def test_combine_both_widths(dev, T, topk, H):
+    from gridbook_b200 import kernels
+    gen = torch.Generator(device=dev).manual_seed(T)
+    y = torch.randn(T * topk, H, generator=gen, device=dev).to(torch.bfloat16)
+    w = torch.rand(T * topk, generator=gen, device=dev)
+    ids = torch.randint(-1, 9, (T, topk), generator=gen, device=dev, dtype=torch.int32)
+    got = kernels.moe_combine(y, w, T, topk, topk_ids=ids, E=8, round_weights=True).float()
+    live = ((ids >= 0) & (ids < 8)).reshape(-1)
+    yw = torch.where(live[:, None], y.float() * w.to(torch.bfloat16).float()[:, None], torch.zeros((), device=dev))
+    want = yw.reshape(T, topk, H).double().sum(1)
+    assert torch.all((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-6)
