@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <stdint.h>
 #include <stdio.h>
 #include <stdarg.h>
@@ -155,74 +156,147 @@ GB_DEVINL float gb_e2m1_rtn(float v) {
   return fabsf(__fsub_rn(hi, v)) < fabsf(__fsub_rn(v, lo)) ? hi : lo;
 }
 
+// The two roundings above cost a division and some thirty selects per value.  Both only ask which
+// side of a few midpoints the quotient lies on, so they are taken from an approximate quotient (a
+// multiply by the reciprocal, off by less than 2^-21 relative) with the hardware's conversion, and
+// done again the slow way when the two ends of [x (1 - 2^-20), x (1 + 2^-20)] convert differently:
+// about one pair of values in 2^17, ties among them.  Same bits as the slow way, always.
+constexpr float kGbNear = 0x1p-20f;
+
+// Two fp32 -> one byte of two E2M1 codes (a in the low nibble), nearest, |value| clamped to 6.
+GB_DEVINL uint32_t gb_cvt_e2m1x2(float a, float b) {
+  uint32_t r;
+  asm("{ .reg .b8 t;\n  cvt.rn.satfinite.e2m1x2.f32 t, %1, %2;\n  cvt.u32.u8 %0, t; }" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+
+// Two fp32 -> two E4M3 bytes (a in the low byte), nearest, |value| clamped to 448.
+GB_DEVINL uint32_t gb_cvt_e4m3x2(float a, float b) {
+  uint16_t r;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(b), "f"(a));
+  return r;
+}
+
+// The E2M1 code of a value on the grid.
+GB_DEVINL uint32_t gb_e2m1_code(float v) {
+  const float m = fabsf(v);
+  const uint32_t c = m < 2.0f ? (uint32_t)(m * 2.0f) : (m < 4.0f ? (uint32_t)m + 2u : (m < 6.0f ? 6u : 7u));
+  return c | (v < 0.0f ? 8u : 0u);
+}
+
+// E2M1 codes of v0 / scale and v1 / scale under the reference's tie rule; `rinv` is 1 / scale to
+// within a few ulp.  Finite arguments.  A zero may carry either sign.
+GB_DEVINL uint32_t gb_e2m1_div2(float v0, float v1, float scale, float rinv) {
+  const float x0 = v0 * rinv, x1 = v1 * rinv;
+  const uint32_t hi = gb_cvt_e2m1x2(fmaf(x0, kGbNear, x0), fmaf(x1, kGbNear, x1));
+  const uint32_t lo = gb_cvt_e2m1x2(fmaf(x0, -kGbNear, x0), fmaf(x1, -kGbNear, x1));
+  if (hi == lo) return hi;
+  return gb_e2m1_code(gb_e2m1_rtn(__fdiv_rn(v0, scale))) | (gb_e2m1_code(gb_e2m1_rtn(__fdiv_rn(v1, scale))) << 4);
+}
+
+// E4M3 bytes of clamp(v / scale, +-448), one rounding each; NaN clamps to -448 as fmaxf leaves it.
+GB_DEVINL uint32_t gb_e4m3_div2(float v0, float v1, float scale, float rinv) {
+  const float x0 = fminf(fmaxf(v0 * rinv, -448.0f), 448.0f), x1 = fminf(fmaxf(v1 * rinv, -448.0f), 448.0f);
+  const uint32_t hi = gb_cvt_e4m3x2(fmaf(x0, kGbNear, x0), fmaf(x1, kGbNear, x1));
+  const uint32_t lo = gb_cvt_e4m3x2(fmaf(x0, -kGbNear, x0), fmaf(x1, -kGbNear, x1));
+  if (hi == lo) return hi;
+  return gb_f32_to_e4m3(fminf(fmaxf(__fdiv_rn(v0, scale), -448.0f), 448.0f)) |
+         (gb_f32_to_e4m3(fminf(fmaxf(__fdiv_rn(v1, scale), -448.0f), 448.0f)) << 8);
+}
+
+// Two E2M1 codes (one byte) -> fp32.
+GB_DEVINL float2 gb_e2m1x2_to_f32(uint32_t byte) {
+  uint32_t h2;
+  asm("{ .reg .b8 t;\n  cvt.u8.u32 t, %1;\n  cvt.rn.f16x2.e2m1x2 %0, t; }" : "=r"(h2) : "r"(byte));
+  return __half22float2(*reinterpret_cast<const __half2*>(&h2));
+}
+
+// Two E4M3 bytes -> fp32.
+GB_DEVINL float2 gb_e4m3x2_to_f32(uint32_t bytes) {
+  uint32_t h2;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"((uint16_t)bytes));
+  return __half22float2(*reinterpret_cast<const __half2*>(&h2));
+}
+
+// The fp32 scale of a group whose largest magnitude is `amax` (already floored at 1e-8).
+GB_DEVINL float gb_fp4_group_scale(float amax, int scale_rule) {
+  return scale_rule == GB_SCALE_RULE_DIV ? __fdiv_rn(amax, 6.0f) : __fmul_rn(amax, 1.0f / 6.0f);
+}
+
+// bf16 pair of the bucket: E2M1(v / scale) * scale, rounded once each; a zero comes out positive.
+// `odd` (an infinity or a NaN in the group): the plain formulation, which spreads it as the
+// reference's codec does.
+GB_DEVINL uint32_t gb_fp4_bucket2(float v0, float v1, float scale, float rinv, bool odd) {
+  if (odd) {
+    const float q0 = __fmul_rn(gb_e2m1_rtn(__fdiv_rn(v0, scale)), scale);
+    const float q1 = __fmul_rn(gb_e2m1_rtn(__fdiv_rn(v1, scale)), scale);
+    return gb_f32_to_bf16_bits(q0) | (gb_f32_to_bf16_bits(q1) << 16);
+  }
+  const float2 q = gb_e2m1x2_to_f32(gb_e2m1_div2(v0, v1, scale, rinv));
+  return gb_pack_bf16x2(fmaf(q.x, scale, 0.0f), fmaf(q.y, scale, 0.0f));
+}
+
+// Largest magnitude of the words' bf16 values, NaNs ignored, and whether one of them is a NaN.
+template <int kWords>
+GB_DEVINL float gb_amax_bf16(const uint32_t (&w)[kWords], bool* has_nan) {
+  float amax = 0.0f;
+  bool nan = false;
+#pragma unroll
+  for (int i = 0; i < kWords; ++i) {
+    const float a = gb_bf16_bits_to_f32(w[i] & 0xFFFFu), b = gb_bf16_bits_to_f32(w[i] >> 16);
+    amax = fmaxf(amax, fmaxf(fabsf(a), fabsf(b)));
+    nan |= isnan(a) || isnan(b);
+  }
+  *has_nan = nan;
+  return amax;
+}
+
+template <int kWords>
+GB_DEVINL void gb_fp4_bucket_words(uint32_t (&w)[kWords], float amax, bool nan, int scale_rule) {
+  amax = fmaxf(amax, 1e-8f);
+  float scale = gb_fp4_group_scale(amax, scale_rule);
+  if (nan) scale = __int_as_float(0x7FC00000);
+  const bool odd = !(amax < __int_as_float(0x7F800000)) || nan;
+  const float rinv = __frcp_rn(scale);
+#pragma unroll
+  for (int i = 0; i < kWords; ++i)
+    w[i] = gb_fp4_bucket2(gb_bf16_bits_to_f32(w[i] & 0xFFFFu), gb_bf16_bits_to_f32(w[i] >> 16), scale, rinv, odd);
+}
+
 // Group-16 E2M1 bucket of sixteen bf16 values (eight packed words), in place.
 GB_DEVINL void gb_fp4_group16_qdq(uint32_t (&w)[8], int scale_rule) {
-  float v[16];
-  float amax = 0.0f;
-  bool has_nan = false;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    v[2 * i] = gb_bf16_bits_to_f32(w[i] & 0xFFFFu);
-    v[2 * i + 1] = gb_bf16_bits_to_f32(w[i] >> 16);
-    amax = fmaxf(amax, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
-    has_nan |= isnan(v[2 * i]) || isnan(v[2 * i + 1]);
-  }
-  amax = fmaxf(amax, 1e-8f);
-  float scale = scale_rule == GB_SCALE_RULE_DIV ? __fdiv_rn(amax, 6.0f) : __fmul_rn(amax, 1.0f / 6.0f);
-  if (has_nan) scale = __int_as_float(0x7FC00000);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float q0 = __fmul_rn(gb_e2m1_rtn(__fdiv_rn(v[2 * i], scale)), scale);
-    const float q1 = __fmul_rn(gb_e2m1_rtn(__fdiv_rn(v[2 * i + 1], scale)), scale);
-    w[i] = gb_f32_to_bf16_bits(q0) | (gb_f32_to_bf16_bits(q1) << 16);
-  }
+  bool nan;
+  const float amax = gb_amax_bf16(w, &nan);
+  gb_fp4_bucket_words(w, amax, nan, scale_rule);
 }
 
 // The same bucket with the group spread over eight consecutive lanes (lane % 8 = word of the
 // group): every lane of the warp must call it.  Bit-identical to gb_fp4_group16_qdq: the
 // maximum ignores NaNs and does not depend on the order, everything else is per value.
 GB_DEVINL uint32_t gb_fp4_group16_qdq_lanes(uint32_t w, int scale_rule) {
-  const float v0 = gb_bf16_bits_to_f32(w & 0xFFFFu), v1 = gb_bf16_bits_to_f32(w >> 16);
-  float amax = fmaxf(fabsf(v0), fabsf(v1));
-  uint32_t nan = (isnan(v0) || isnan(v1)) ? 1u : 0u;
+  uint32_t one[1] = {w};
+  bool has_nan;
+  float amax = gb_amax_bf16(one, &has_nan);
+  uint32_t nan = has_nan ? 1u : 0u;
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1) {
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     nan |= __shfl_xor_sync(0xffffffffu, nan, o);
   }
-  amax = fmaxf(amax, 1e-8f);
-  float scale = scale_rule == GB_SCALE_RULE_DIV ? __fdiv_rn(amax, 6.0f) : __fmul_rn(amax, 1.0f / 6.0f);
-  if (nan) scale = __int_as_float(0x7FC00000);
-  const float q0 = __fmul_rn(gb_e2m1_rtn(__fdiv_rn(v0, scale)), scale);
-  const float q1 = __fmul_rn(gb_e2m1_rtn(__fdiv_rn(v1, scale)), scale);
-  return gb_f32_to_bf16_bits(q0) | (gb_f32_to_bf16_bits(q1) << 16);
+  gb_fp4_bucket_words(one, amax, nan != 0, scale_rule);
+  return one[0];
 }
 
 // The same bucket with a group split over two adjacent lanes (eight values each, lane ^ 1 holds
 // the other half): both lanes must call it.  Bit-identical to gb_fp4_group16_qdq.
 GB_DEVINL uint4 gb_fp4_group16_qdq_pair(uint4 in, int scale_rule) {
   uint32_t w[4] = {in.x, in.y, in.z, in.w};
-  float v[8];
-  float amax = 0.0f;
-  uint32_t nan = 0u;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[2 * i] = gb_bf16_bits_to_f32(w[i] & 0xFFFFu);
-    v[2 * i + 1] = gb_bf16_bits_to_f32(w[i] >> 16);
-    amax = fmaxf(amax, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
-    nan |= (isnan(v[2 * i]) || isnan(v[2 * i + 1])) ? 1u : 0u;
-  }
+  bool has_nan;
+  float amax = gb_amax_bf16(w, &has_nan);
+  uint32_t nan = has_nan ? 1u : 0u;
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
   nan |= __shfl_xor_sync(0xffffffffu, nan, 1);
-  amax = fmaxf(amax, 1e-8f);
-  float scale = scale_rule == GB_SCALE_RULE_DIV ? __fdiv_rn(amax, 6.0f) : __fmul_rn(amax, 1.0f / 6.0f);
-  if (nan) scale = __int_as_float(0x7FC00000);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float q0 = __fmul_rn(gb_e2m1_rtn(__fdiv_rn(v[2 * i], scale)), scale);
-    const float q1 = __fmul_rn(gb_e2m1_rtn(__fdiv_rn(v[2 * i + 1], scale)), scale);
-    w[i] = gb_f32_to_bf16_bits(q0) | (gb_f32_to_bf16_bits(q1) << 16);
-  }
+  gb_fp4_bucket_words(w, amax, nan != 0, scale_rule);
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 

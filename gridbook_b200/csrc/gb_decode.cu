@@ -28,15 +28,73 @@ fp4_group16_qdq_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ ou
   dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
 }
 
-// One block per token row: block-wide amax, then every element is scaled,
-// rounded once to E4M3 and scaled back.
+// Per-token E4M3 bucket: one CTA per row, the row held in registers (kVec vectors of eight values
+// per thread), so it is read once: block-wide amax, then every element is scaled and rounded once
+// to E4M3.  kQuantize: the E4M3 bytes and the row's scale; otherwise scaled back to bf16.
+// Bound by memory for many rows (8192 x 17408: 257 us when each element was loaded twice on its own
+// and divided), by the two round trips for a few.
+template <int kVec, bool kQuantize>
+__global__ void __launch_bounds__(1024)
+fp8_rows_kernel(const uint4* __restrict__ x, void* __restrict__ out, float* __restrict__ scale_out, int vecs,
+                int scale_rule) {
+  gb_pdl_launch_dependents();
+  gb_pdl_wait();
+  const uint4* row = x + (int64_t)blockIdx.x * vecs;
+  __shared__ float red[32];
+  uint4 v[kVec];
+#pragma unroll
+  for (int j = 0; j < kVec; ++j) {
+    const int i = threadIdx.x + j * blockDim.x;
+    v[j] = i < vecs ? row[i] : make_uint4(0u, 0u, 0u, 0u);
+  }
+  float amax = 0.0f;
+#pragma unroll
+  for (int j = 0; j < kVec; ++j) {
+    const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      amax = fmaxf(amax, fmaxf(fabsf(gb_bf16_bits_to_f32(w[q] & 0xFFFFu)), fabsf(gb_bf16_bits_to_f32(w[q] >> 16))));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = (int)(threadIdx.x & 31) < (int)(blockDim.x + 31) / 32 ? red[threadIdx.x & 31] : 0.0f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float s = scale_rule == GB_SCALE_RULE_DIV ? __fdiv_rn(amax, 448.0f) : __fmul_rn(amax, 1.0f / 448.0f);
+  const float scale = fmaxf(s, 1.0f / (448.0f * 512.0f)), rinv = __frcp_rn(scale);
+  if (kQuantize && threadIdx.x == 0) scale_out[blockIdx.x] = scale;
+#pragma unroll
+  for (int j = 0; j < kVec; ++j) {
+    const int i = threadIdx.x + j * blockDim.x;
+    if (i >= vecs) break;
+    const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+    uint32_t q[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) q[c] = gb_e4m3_div2(gb_bf16_bits_to_f32(w[c] & 0xFFFFu), gb_bf16_bits_to_f32(w[c] >> 16), scale, rinv);
+    if (kQuantize) {
+      reinterpret_cast<uint2*>(out)[(int64_t)blockIdx.x * vecs + i] = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
+    } else {
+      uint32_t r[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float2 f = gb_e4m3x2_to_f32(q[c]);
+        r[c] = gb_pack_bf16x2(__fmul_rn(f.x, scale), __fmul_rn(f.y, scale));
+      }
+      reinterpret_cast<uint4*>(out)[(int64_t)blockIdx.x * vecs + i] = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+  }
+}
+
+// The same for rows that are not whole aligned vectors (or longer than the registers of a CTA hold).
+template <bool kQuantize>
 __global__ void __launch_bounds__(kThreads)
-fp8_token_qdq_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ out, int64_t K,
-                     int scale_rule) {
+fp8_rows_any_kernel(const uint16_t* __restrict__ x, void* __restrict__ out, float* __restrict__ scale_out, int64_t K,
+                    int scale_rule) {
   gb_pdl_launch_dependents();
   gb_pdl_wait();
   const uint16_t* row = x + (int64_t)blockIdx.x * K;
-  uint16_t* orow = out + (int64_t)blockIdx.x * K;
   __shared__ float red[kThreads / 32];
   __shared__ float s_scale;
   float amax = 0.0f;
@@ -52,15 +110,42 @@ fp8_token_qdq_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ out,
     const float s = scale_rule == GB_SCALE_RULE_DIV ? __fdiv_rn(a, 448.0f)
                                                     : __fmul_rn(a, 1.0f / 448.0f);
     s_scale = fmaxf(s, 1.0f / (448.0f * 512.0f));
+    if (kQuantize) scale_out[blockIdx.x] = s_scale;
   }
   __syncthreads();
   const float scale = s_scale;
   for (int64_t i = threadIdx.x; i < K; i += blockDim.x) {
     const float v = gb_bf16_bits_to_f32(row[i]);
-    const float q = fminf(fmaxf(__fdiv_rn(v, scale), -448.0f), 448.0f);
-    const float dq = gb_e4m3_to_f32(gb_f32_to_e4m3(q));
-    orow[i] = (uint16_t)gb_f32_to_bf16_bits(__fmul_rn(dq, scale));
+    const uint32_t q = gb_f32_to_e4m3(fminf(fmaxf(__fdiv_rn(v, scale), -448.0f), 448.0f));
+    if (kQuantize) reinterpret_cast<uint8_t*>(out)[(int64_t)blockIdx.x * K + i] = (uint8_t)q;
+    else reinterpret_cast<uint16_t*>(out)[(int64_t)blockIdx.x * K + i] = (uint16_t)gb_f32_to_bf16_bits(__fmul_rn(gb_e4m3_to_f32(q), scale));
   }
+}
+
+// Rows of up to 8 x 1024 vectors stay in registers; the fewest vectors per thread that 512 threads
+// (or, past that, 1024) can hold, since a few long rows are bound by latency.
+template <bool kQuantize>
+int launch_fp8_rows(const void* x, void* out, float* scale, int64_t M, int64_t K, int scale_rule, void* stream) {
+  const int64_t vecs = K / 8;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (K % 8 != 0 || vecs > 8 * 1024 || ((uintptr_t)x & 15u) != 0 || ((uintptr_t)out & (kQuantize ? 7u : 15u)) != 0) {
+    GB_CUDA_OK(gb_launch(fp8_rows_any_kernel<kQuantize>, dim3((unsigned)M), dim3(kThreads), 0, st, (const uint16_t*)x, out,
+                         scale, K, scale_rule));
+    return GB_OK;
+  }
+  const int per = vecs <= 512 ? 1 : vecs <= 1024 ? 2 : vecs <= 2048 + 512 ? 4 : 8;
+  const unsigned threads = (unsigned)(((vecs + per - 1) / per + 31) / 32 * 32);
+#define GB_FP8_ROWS(V)                                                                                        \
+  GB_CUDA_OK(gb_launch(fp8_rows_kernel<V, kQuantize>, dim3((unsigned)M), dim3(threads), 0, st, (const uint4*)x, out, scale, \
+                       (int)vecs, scale_rule))
+  switch (per) {
+    case 1: GB_FP8_ROWS(1); break;
+    case 2: GB_FP8_ROWS(2); break;
+    case 4: GB_FP8_ROWS(4); break;
+    default: GB_FP8_ROWS(8); break;
+  }
+#undef GB_FP8_ROWS
+  return GB_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -306,9 +391,14 @@ int gb_fp8_act_qdq(const void* x, void* out, int64_t M, int64_t K, int scale_rul
   GB_REQUIRE(x && out, "null activation pointer");
   GB_REQUIRE(M >= 0 && K > 0, "bad shape M=%lld K=%lld", (long long)M, (long long)K);
   if (M == 0) return GB_OK;
-  GB_CUDA_OK(gb_launch(fp8_token_qdq_kernel, dim3((unsigned)M), dim3(kThreads), 0, (cudaStream_t)stream,
-                       (const uint16_t*)x, (uint16_t*)out, K, scale_rule));
-  return GB_OK;
+  return launch_fp8_rows<false>(x, out, nullptr, M, K, scale_rule, stream);
+}
+
+int gb_fp8_quantize_rows(const void* x, void* q, float* scale, int64_t M, int64_t K, int scale_rule, void* stream) {
+  GB_REQUIRE(x && q && scale, "null pointer argument");
+  GB_REQUIRE(M >= 0 && K > 0, "bad shape M=%lld K=%lld", (long long)M, (long long)K);
+  if (M == 0) return GB_OK;
+  return launch_fp8_rows<true>(x, q, scale, M, K, scale_rule, stream);
 }
 
 }  // extern "C"

@@ -307,35 +307,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
-// ---- per-token E4M3 quantisation of the activations (fp8-grid prefill) ----------------
-__global__ void __launch_bounds__(256)
-fp8_quantize_rows_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale_out,
-                         int64_t K, int scale_rule) {
-  const uint16_t* row = x + (int64_t)blockIdx.x * K;
-  uint8_t* qrow = q + (int64_t)blockIdx.x * K;
-  __shared__ float red[8];
-  __shared__ float s_scale;
-  float amax = 0.0f;
-  for (int64_t i = threadIdx.x; i < K; i += blockDim.x) amax = fmaxf(amax, fabsf(gb_bf16_bits_to_f32(row[i])));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float a = red[0];
-    for (int w = 1; w < 8; ++w) a = fmaxf(a, red[w]);
-    const float s = scale_rule == GB_SCALE_RULE_DIV ? __fdiv_rn(a, 448.0f) : __fmul_rn(a, 1.0f / 448.0f);
-    s_scale = fmaxf(s, 1.0f / (448.0f * 512.0f));
-    scale_out[blockIdx.x] = s_scale;
-  }
-  __syncthreads();
-  const float scale = s_scale;
-  for (int64_t i = threadIdx.x; i < K; i += blockDim.x) {
-    const float v = gb_bf16_bits_to_f32(row[i]);
-    qrow[i] = (uint8_t)gb_f32_to_e4m3(fminf(fmaxf(__fdiv_rn(v, scale), -448.0f), 448.0f));
-  }
-}
-
 // ---- routed prefill helpers: rows in expert order ---------------------------------------
 // out[j] = x[x_row[order[j]]] (or x[order[j]] without x_row) for the sorted rows j < *n_rows.
 __global__ void __launch_bounds__(128)
@@ -457,17 +428,6 @@ int gb_prepare_gemm() {
 }
 
 extern "C" {
-
-int gb_fp8_quantize_rows(const void* x, void* q, float* scale, int64_t M, int64_t K, int scale_rule, void* stream) {
-  GB_REQUIRE(x && q && scale, "null pointer argument");
-  GB_REQUIRE(M >= 0 && K > 0, "bad shape M=%lld K=%lld", (long long)M, (long long)K);
-  if (M == 0) return GB_OK;
-  gb_count_launch();
-  fp8_quantize_rows_kernel<<<(unsigned)M, 256, 0, (cudaStream_t)stream>>>((const uint16_t*)x, (uint8_t*)q, scale, K,
-                                                                        scale_rule);
-  GB_LAUNCH_OK("fp8_quantize_rows_kernel");
-  return GB_OK;
-}
 
 int gb_gemm_tn(const void* A, const void* B, void* D, int64_t M, int64_t N, int64_t K, int kind, const float* a_scale,
                const float* b_scale, float global_scale, void* stream) {

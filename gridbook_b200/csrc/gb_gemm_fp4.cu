@@ -313,71 +313,97 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 //   sign bit = sign of xs (kept on zeros); a zero SF zeroes its group.
 // Every operation is a correctly rounded fp32 one (no approximate reciprocal), so the bytes are
 // those of the torch formulation.
-// Two fp32 -> one byte of two E2M1 codes (lo in the low nibble): round to nearest, a tie to the
-// even code, clamped to +-6, the sign kept on a zero.
-GB_DEVINL uint32_t e2m1x2(float lo, float hi) {
-  uint32_t r;
-  asm("{ .reg .b8 t;\n  cvt.rn.satfinite.e2m1x2.f32 t, %1, %2;\n  cvt.u32.u8 %0, t; }" : "=r"(r) : "f"(hi), "f"(lo));
-  return r;
+// The quotient xs / SF is taken as a product with the reciprocal and redone as a division when it
+// lies near a rounding boundary (gb_common.cuh, kGbNear).
+//
+// One CTA per row, one to four groups per thread kept in registers: the row is read once
+// (2048 x 17408: 38.6 us when it was read twice and every value divided twice).
+GB_DEVINL uint32_t e2m1_div2_even(float v0, float v1, float d, float rinv) {
+  const float x0 = v0 * rinv, x1 = v1 * rinv;
+  const uint32_t hi = gb_cvt_e2m1x2(fmaf(x0, kGbNear, x0), fmaf(x1, kGbNear, x1));
+  const uint32_t lo = gb_cvt_e2m1x2(fmaf(x0, -kGbNear, x0), fmaf(x1, -kGbNear, x1));
+  return hi == lo ? hi : gb_cvt_e2m1x2(__fdiv_rn(v0, d), __fdiv_rn(v1, d));
 }
 
-__global__ void __launch_bounds__(256)
-nvfp4_quantize_rows_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ packed, uint8_t* __restrict__ sfa,
-                           float* __restrict__ a_scale, int64_t M, int64_t K, float range) {
+constexpr int kQuantMaxGroups = 4;
+
+template <int kG>
+__global__ void __launch_bounds__(1024)
+nvfp4_quantize_rows_kernel(const uint4* __restrict__ x, uint2* __restrict__ packed, uint8_t* __restrict__ sfa,
+                           float* __restrict__ a_scale, int64_t M, int groups, float range) {
+  gb_pdl_launch_dependents();
+  gb_pdl_wait();
   const int64_t row = blockIdx.x;
-  const int64_t groups = K / 16, k_atoms = (groups + 3) / 4;
-  auto sf_offset = [&](int64_t g) {
-    return (row % 32) * 16 + ((row / 32) % 4) * 4 + (g % 4) + (g / 4) * 512 + (row / 128) * (512 * k_atoms);
+  const int64_t k_atoms = (groups + 3) / 4;
+  auto sf_offset = [&](int g) {
+    return (row % 32) * 16 + ((row / 32) % 4) * 4 + (g % 4) + (int64_t)(g / 4) * 512 + (row / 128) * (512 * k_atoms);
   };
   if (row >= M) {                                        // padding rows of the last 128-row tile: zero scales
-    for (int64_t g = threadIdx.x; g < groups; g += blockDim.x) sfa[sf_offset(g)] = 0;
+    for (int g = threadIdx.x; g < groups; g += blockDim.x) sfa[sf_offset(g)] = 0;
     return;
   }
-  const uint16_t* xr = x + row * K;
-  __shared__ float red[8];
+  const uint4* xr = x + row * 2 * groups;
+  __shared__ float red[32];
+  uint32_t w[kG][8];
   float amax = 0.0f;
-  for (int64_t i = threadIdx.x; i < K / 8; i += blockDim.x) {
-    const uint4 v = reinterpret_cast<const uint4*>(xr)[i];
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  for (int g0 = threadIdx.x; g0 < groups; g0 += kG * blockDim.x) {    // once, unless the row is longer than the registers
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      amax = fmaxf(amax, fmaxf(fabsf(gb_bf16_bits_to_f32(w[j] & 0xffffu)), fabsf(gb_bf16_bits_to_f32(w[j] >> 16))));
+    for (int j = 0; j < kG; ++j) {
+      const int g = g0 + j * blockDim.x;
+      const bool in = g < groups;
+      const uint4 a = in ? xr[2 * g] : make_uint4(0u, 0u, 0u, 0u), b = in ? xr[2 * g + 1] : make_uint4(0u, 0u, 0u, 0u);
+      w[j][0] = a.x; w[j][1] = a.y; w[j][2] = a.z; w[j][3] = a.w;
+      w[j][4] = b.x; w[j][5] = b.y; w[j][6] = b.z; w[j][7] = b.w;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        amax = fmaxf(amax, fmaxf(fabsf(gb_bf16_bits_to_f32(w[j][i] & 0xffffu)), fabsf(gb_bf16_bits_to_f32(w[j][i] >> 16))));
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
   __syncthreads();
-  amax = red[0];
+  amax = (int)(threadIdx.x & 31) < (int)(blockDim.x >> 5) ? red[threadIdx.x & 31] : 0.0f;
 #pragma unroll
-  for (int w = 1; w < 8; ++w) amax = fmaxf(amax, red[w]);
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   const bool live = amax > 0.0f && isfinite(amax);
   const float gs = live ? __fdiv_rn(__fmul_rn(range, 6.0f), amax) : 1.0f;
   if (threadIdx.x == 0) a_scale[row] = live ? __fdiv_rn(1.0f, gs) : 0.0f;
-  for (int64_t g = threadIdx.x; g < groups; g += blockDim.x) {
-    const uint4 v0 = reinterpret_cast<const uint4*>(xr)[2 * g], v1 = reinterpret_cast<const uint4*>(xr)[2 * g + 1];
-    const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-    float xs[16];
-    float gmax = 0.0f;
+  const bool reload = groups > kG * (int)blockDim.x;
+  for (int g0 = threadIdx.x; g0 < groups; g0 += kG * blockDim.x) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      xs[2 * j] = __fmul_rn(gb_bf16_bits_to_f32(w[j] & 0xffffu), gs);
-      xs[2 * j + 1] = __fmul_rn(gb_bf16_bits_to_f32(w[j] >> 16), gs);
-      gmax = fmaxf(gmax, fmaxf(fabsf(xs[2 * j]), fabsf(xs[2 * j + 1])));
-    }
-    const float sf = live ? fminf(__fdiv_rn(gmax, 6.0f), 448.0f) : 0.0f;
-    const uint32_t sf_byte = gb_f32_to_e4m3(sf);
-    const float sf_f = gb_e4m3_to_f32(sf_byte);
-    sfa[sf_offset(g)] = (uint8_t)sf_byte;
-    uint32_t lo = 0, hi = 0;
+    for (int j = 0; j < kG; ++j) {
+      const int g = g0 + j * blockDim.x;
+      if (g >= groups) break;
+      if (reload) {
+        const uint4 a = xr[2 * g], b = xr[2 * g + 1];
+        w[j][0] = a.x; w[j][1] = a.y; w[j][2] = a.z; w[j][3] = a.w;
+        w[j][4] = b.x; w[j][5] = b.y; w[j][6] = b.z; w[j][7] = b.w;
+      }
+      float xs[16];
+      float gmax = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      uint32_t byte;
-      if (sf_f != 0.0f) byte = e2m1x2(__fdiv_rn(xs[2 * j], sf_f), __fdiv_rn(xs[2 * j + 1], sf_f));
-      else byte = ((__float_as_uint(xs[2 * j]) >> 31) << 3) | ((__float_as_uint(xs[2 * j + 1]) >> 31) << 7);
-      if (j < 4) lo |= byte << (8 * j);
-      else hi |= byte << (8 * (j - 4));
+      for (int i = 0; i < 8; ++i) {
+        xs[2 * i] = __fmul_rn(gb_bf16_bits_to_f32(w[j][i] & 0xffffu), gs);
+        xs[2 * i + 1] = __fmul_rn(gb_bf16_bits_to_f32(w[j][i] >> 16), gs);
+        gmax = fmaxf(gmax, fmaxf(fabsf(xs[2 * i]), fabsf(xs[2 * i + 1])));
+      }
+      const float sf = live ? fminf(__fdiv_rn(gmax, 6.0f), 448.0f) : 0.0f;
+      const uint32_t sf_byte = gb_f32_to_e4m3(sf);
+      const float sf_f = gb_e4m3_to_f32(sf_byte);
+      sfa[sf_offset(g)] = (uint8_t)sf_byte;
+      const float rinv = sf_f != 0.0f ? __frcp_rn(sf_f) : 0.0f;
+      uint32_t lo = 0, hi = 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        uint32_t byte;
+        if (sf_f != 0.0f) byte = e2m1_div2_even(xs[2 * i], xs[2 * i + 1], sf_f, rinv);
+        else byte = ((__float_as_uint(xs[2 * i]) >> 31) << 3) | ((__float_as_uint(xs[2 * i + 1]) >> 31) << 7);
+        if (i < 4) lo |= byte << (8 * i);
+        else hi |= byte << (8 * (i - 4));
+      }
+      packed[row * groups + g] = make_uint2(lo, hi);
     }
-    reinterpret_cast<uint2*>(packed + row * (K / 2))[g] = make_uint2(lo, hi);
   }
 }
 
@@ -402,11 +428,20 @@ int gb_nvfp4_quantize_rows(const void* x, int64_t M, int64_t K, float range, voi
   GB_REQUIRE(((uintptr_t)x & 15u) == 0 && ((uintptr_t)packed & 7u) == 0, "rows must be 16-byte aligned");
   GB_REQUIRE(range > 0.0f && range <= 448.0f, "range multiplier %g outside (0, 448]", (double)range);
   if (M == 0) return GB_OK;
-  const int64_t padded = (M + 127) / 128 * 128;
-  gb_count_launch();
-  nvfp4_quantize_rows_kernel<<<(unsigned)padded, 256, 0, (cudaStream_t)stream>>>(
-      (const uint16_t*)x, (uint8_t*)packed, (uint8_t*)sf, a_scale, M, K, range);
-  GB_LAUNCH_OK("nvfp4_quantize_rows_kernel");
+  GB_REQUIRE(K / 16 < (1ll << 31), "dimension too large");
+  const int64_t padded = (M + 127) / 128 * 128, groups = K / 16;
+  const int per = groups <= 512 ? 1 : groups <= 1024 ? 2 : kQuantMaxGroups;
+  int64_t threads = ((groups + per - 1) / per + 31) / 32 * 32;
+  if (threads > 1024) threads = 1024;
+#define GB_NVFP4_ROWS(G)                                                                                          \
+  GB_CUDA_OK(gb_launch(nvfp4_quantize_rows_kernel<G>, dim3((unsigned)padded), dim3((unsigned)threads), 0, (cudaStream_t)stream, \
+                       (const uint4*)x, (uint2*)packed, (uint8_t*)sf, a_scale, M, (int)groups, range))
+  switch (per) {
+    case 1: GB_NVFP4_ROWS(1); break;
+    case 2: GB_NVFP4_ROWS(2); break;
+    default: GB_NVFP4_ROWS(kQuantMaxGroups); break;
+  }
+#undef GB_NVFP4_ROWS
   return GB_OK;
 }
 
