@@ -816,7 +816,7 @@ int launch_expand_product(const gb_weight* w, int64_t row0, int64_t nrows, void*
   GB_REQUIRE(rows_per * p.n_sb < (1ll << 31), "too many superblocks per CTA");
   p.rows_per_cta = rows_per;
   const unsigned blocks = (unsigned)((nrows + rows_per - 1) / rows_per);
-  if (smem > 48 * 1024)
+  if (smem > 47 * 1024)                                   // the default limit counts the static words too
     GB_CUDA_OK(cudaFuncSetAttribute((const void*)expand_product_kernel<kOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   gb_count_launch();
   expand_product_kernel<kOut><<<blocks, kProdThreads, smem, (cudaStream_t)stream>>>(p, out0, (uint8_t*)out_sf, fold_sign);
