@@ -300,6 +300,18 @@ GB_DEVINL uint4 gb_fp4_group16_qdq_pair(uint4 in, int scale_rule) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// gate / (1 + exp(-gate)) with the quotient taken as a product with the reciprocal and one correction
+// step.  The plain division leaves its fast path when the exponential is huge, and gates far below
+// zero are common: the routed SwiGLU launch over 32768 x 768 values spent 186 us, four times what
+// its bytes take.
+GB_DEVINL float gb_silu(float gate) {
+  const float d = 1.0f + __expf(-gate);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = gate * r;
+  return d < 0x1p100f && fabsf(gate) < 0x1p100f ? fmaf(fmaf(-q, d, gate), r, q) : q;
+}
+
 // ---------------------------------------------------------------------------
 // bit-stream extraction (docs/SPEC.md:56-92): codeword c of a superblock
 // occupies stream bits [c*k, c*k+k), least significant bit first.

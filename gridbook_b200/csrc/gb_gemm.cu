@@ -347,7 +347,7 @@ moe_swiglu_rows_kernel(const uint4* __restrict__ h, const int32_t* __restrict__ 
       for (int hlf = 0; hlf < 2; ++hlf) {
         const float gate = gb_bf16_bits_to_f32((gw[q] >> (16 * hlf)) & 0xffffu);
         const float up = gb_bf16_bits_to_f32((uw[q] >> (16 * hlf)) & 0xffffu);
-        const float sl = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gate / (1.0f + __expf(-gate))));
+        const float sl = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_silu(gate)));
         packed |= gb_f32_to_bf16_bits(sl * up) << (16 * hlf);
       }
       r[q] = packed;

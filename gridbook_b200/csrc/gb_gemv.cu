@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(kLit ? 512 : 256, 1) gemv_kernel(const __grid_
           if (m < t.mcount && 4 * warp + n < t.nrows) {
             const float gate = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(c[i]));
             const float upv = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(up[i]));
-            const float sl = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gate / (1.0f + __expf(-gate))));
+            const float sl = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_silu(gate)));
             const int pair = p.order[t.m0 + m];
             p.y[(int64_t)pair * (p.N / 2) + t.row0 + 4 * warp + n] = (uint16_t)gb_f32_to_bf16_bits(sl * upv);
           }

@@ -235,7 +235,7 @@ gemv_dot_kernel(const __grid_constant__ CUtensorMap map_w, const DotParams p) {
       auto act1 = [&](float graw, float uraw) {
         const float gate = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(graw * p.xws_scale));
         const float up = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(uraw * p.xws_scale));
-        const float sl = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gate / (1.0f + __expf(-gate))));
+        const float sl = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_silu(gate)));
         return gb_f32_to_bf16_bits(sl * up);
       };
       w = act1(g0, u0) | (act1(g1, u1) << 16);
@@ -458,7 +458,7 @@ __global__ void dot_pairs_finalize_kernel(const __grid_constant__ DotParams p, i
   if (swiglu) {
     const float gate = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(out));
     const float up = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(b * p.global_scale));
-    const float sl = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gate / (1.0f + __expf(-gate))));
+    const float sl = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_silu(gate)));
     out = sl * up;
   }
   pair_out_row(p, pair, width)[j] = (uint16_t)gb_f32_to_bf16_bits(out);
