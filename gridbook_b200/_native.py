@@ -87,6 +87,7 @@ class GbPeerRows(ctypes.Structure):
 
 _LOCK = threading.Lock()
 _LIB = None
+_HOST = None
 _PREPARED: set[int] = set()
 
 
@@ -197,6 +198,28 @@ def load(what: str = "gridbook_b200 kernels"):
                 f"wants {GB_ABI_VERSION}; rebuild it")
         _LIB = lib
         return lib
+
+
+def host(what: str = "gridbook_b200 host path"):
+    """The compiled host path (csrc/gb_torch.cpp), bound to the same library file as :func:`load`."""
+    global _HOST
+    if _HOST is not None:
+        return _HOST
+    load(what)
+    with _LOCK:
+        if _HOST is None:
+            try:
+                from . import _gb_torch
+            except ImportError as exc:
+                raise NativeKernelUnavailableError(
+                    f"[prismaquant-cb] {what}: the compiled host path is missing or does not match this torch: {exc}. "
+                    "Build it with `python -m gridbook_b200.build`; there is no fallback path.") from exc
+            if _gb_torch.abi_version() != GB_ABI_VERSION:
+                raise StaleExtensionError(f"[prismaquant-cb] {what}: _gb_torch.so was built for ABI version "
+                                          f"{_gb_torch.abi_version()}, this package wants {GB_ABI_VERSION}; rebuild it")
+            _gb_torch.bind(library_path())
+            _HOST = _gb_torch
+        return _HOST
 
 
 def check(rc: int, lib=None) -> None:

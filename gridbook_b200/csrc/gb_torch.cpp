@@ -1,0 +1,514 @@
+// Host path of the layers: one call from Python per forward.
+//
+// A plan (LinearPlan, MoEPlan) is built once after loading and owns everything a forward needs - the
+// C-ABI weight descriptors, references to the tensors behind them, slot buffers, workspaces.  Its
+// call picks the route, allocates the outputs and one workspace with torch's allocator and launches
+// the library's kernels on the current stream.  The same sequence from Python (custom-op dispatch,
+// ctypes structs rebuilt per call, one torch.empty per intermediate) cost 40 us for the one launch of
+// a 4096 x 4096 decode row and 70 to 100 us for the seven of a routed layer, several times what
+// their kernels take.
+//
+// The library is reached through dlsym on the path the ctypes loader uses, so that both bind the
+// same file and a missing symbol fails closed.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <atomic>
+#include <dlfcn.h>
+#include <map>
+#include <memory>
+#include <mutex>
+#include <stdexcept>
+#include <string>
+#include <tuple>
+#include <vector>
+
+#include "../../include/gridbook_b200.h"
+
+namespace py = pybind11;
+
+namespace {
+
+struct Lib {
+#define GB_FN(name) decltype(&::name) name = nullptr
+  GB_FN(gb_last_error);
+  GB_FN(gb_gemv_workspace_bytes);
+  GB_FN(gb_gemv);
+  GB_FN(gb_gemv_row_batch_max);
+  GB_FN(gb_gemv_tab);
+  GB_FN(gb_gemv_tab_slots_bytes);
+  GB_FN(gb_fp4_act_qdq);
+  GB_FN(gb_fp8_act_qdq);
+  GB_FN(gb_fp8_quantize_rows);
+  GB_FN(gb_nvfp4_sf_bytes);
+  GB_FN(gb_nvfp4_quantize_rows);
+  GB_FN(gb_expand_fp4_nvfp4);
+  GB_FN(gb_expand_fp4_bf16);
+  GB_FN(gb_expand_fp8);
+  GB_FN(gb_expand_fp8_bf16);
+  GB_FN(gb_gemm_fp4);
+  GB_FN(gb_gemm_tn);
+  GB_FN(gb_gemm_tn_grouped);
+  GB_FN(gb_moe_route_ws);
+  GB_FN(gb_moe_route_workspace_bytes);
+  GB_FN(gb_moe_gather_rows);
+  GB_FN(gb_moe_swiglu_rows);
+  GB_FN(gb_moe_gemv);
+  GB_FN(gb_moe_gemv_sorted);
+  GB_FN(gb_moe_mlp_pairs);
+  GB_FN(gb_moe_mlp_pairs_workspace_bytes);
+  GB_FN(gb_moe_combine);
+#undef GB_FN
+};
+Lib L;
+
+void bind(const std::string& path) {
+  void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  if (!h) throw std::runtime_error("cannot load " + path + ": " + dlerror());
+#define GB_FN(name)                                                                   \
+  L.name = reinterpret_cast<decltype(L.name)>(dlsym(h, #name));                       \
+  if (!L.name) throw std::runtime_error(path + " lacks the required symbol " #name)
+  GB_FN(gb_last_error);
+  GB_FN(gb_gemv_workspace_bytes);
+  GB_FN(gb_gemv);
+  GB_FN(gb_gemv_row_batch_max);
+  GB_FN(gb_gemv_tab);
+  GB_FN(gb_gemv_tab_slots_bytes);
+  GB_FN(gb_fp4_act_qdq);
+  GB_FN(gb_fp8_act_qdq);
+  GB_FN(gb_fp8_quantize_rows);
+  GB_FN(gb_nvfp4_sf_bytes);
+  GB_FN(gb_nvfp4_quantize_rows);
+  GB_FN(gb_expand_fp4_nvfp4);
+  GB_FN(gb_expand_fp4_bf16);
+  GB_FN(gb_expand_fp8);
+  GB_FN(gb_expand_fp8_bf16);
+  GB_FN(gb_gemm_fp4);
+  GB_FN(gb_gemm_tn);
+  GB_FN(gb_gemm_tn_grouped);
+  GB_FN(gb_moe_route_ws);
+  GB_FN(gb_moe_route_workspace_bytes);
+  GB_FN(gb_moe_gather_rows);
+  GB_FN(gb_moe_swiglu_rows);
+  GB_FN(gb_moe_gemv);
+  GB_FN(gb_moe_gemv_sorted);
+  GB_FN(gb_moe_mlp_pairs);
+  GB_FN(gb_moe_mlp_pairs_workspace_bytes);
+  GB_FN(gb_moe_combine);
+#undef GB_FN
+}
+
+void check(int rc) {
+  if (rc != GB_OK)
+    throw std::runtime_error(std::string("gridbook_b200: ") + L.gb_last_error() + " (status " + std::to_string(rc) + ")");
+}
+
+using Opt = c10::optional<at::Tensor>;
+
+// A weight as the kernels see it, and the tensors that keep its pointers valid.
+struct Weight {
+  gb_weight w{};
+  int64_t expert_stride = 0, experts = 1;
+  std::vector<at::Tensor> keep;
+  bool fp4() const { return w.fmt.grid == GB_GRID_FP4; }
+  int act() const { return fp4() ? GB_ACT_FP4_GROUP16 : GB_ACT_FP8_TOKEN; }
+};
+
+Weight make_weight(const at::Tensor& qw, const at::Tensor& codebook, std::array<int, 6> fmt, int64_t K, int64_t rows,
+                   int64_t row_stride, const Opt& off, const Opt& compose, const Opt& scale, double global_scale,
+                   int64_t expert_stride, int64_t experts) {
+  Weight r;
+  r.w.qw = static_cast<const uint8_t*>(qw.data_ptr());
+  r.w.row_stride = row_stride;
+  r.w.codebook = codebook.data_ptr();
+  r.keep = {qw, codebook};
+  auto hold = [&](const Opt& t) -> void* {
+    if (!t.has_value() || !t->defined()) return nullptr;
+    r.keep.push_back(*t);
+    return t->data_ptr();
+  };
+  r.w.cb_row_offset = static_cast<const int32_t*>(hold(off));
+  r.w.compose = static_cast<const float*>(hold(compose));
+  r.w.weight_scale = static_cast<const float*>(hold(scale));
+  r.w.global_scale = (float)global_scale;
+  r.w.rows = rows;
+  r.w.K = K;
+  r.w.fmt = {fmt[0], fmt[1], fmt[2], fmt[3], fmt[4], fmt[5]};
+  r.expert_stride = expert_stride;
+  r.experts = experts;
+  return r;
+}
+
+// Everything one forward needs between its kernels, cut from a single allocation.
+struct Arena {
+  std::vector<int64_t> at;
+  int64_t total = 0;
+  at::Tensor buf;
+  uint8_t* base = nullptr;
+  int add(int64_t bytes) {
+    at.push_back(total);
+    total += (bytes + 255) & ~int64_t(255);
+    return (int)at.size() - 1;
+  }
+  void alloc(const at::Tensor& like) {
+    buf = at::empty({total > 0 ? total : 1}, like.options().dtype(at::kByte));
+    base = static_cast<uint8_t*>(buf.data_ptr());
+  }
+  template <typename T = void>
+  T* ptr(int i) const { return reinterpret_cast<T*>(base + at[i]); }
+};
+
+void need_cuda(const at::Tensor& t) {
+  if (!t.is_cuda()) throw std::runtime_error("gridbook_b200 kernels take CUDA tensors only (no CPU path exists)");
+}
+
+void need_bf16(const at::Tensor& t, const char* what) {
+  if (t.scalar_type() != at::kBFloat16) throw py::type_error(std::string(what) + " takes bf16 activations");
+}
+
+constexpr int64_t kDecodeMaxRows = 16;
+constexpr float kNvfp4ActRange = 448.0f;      // a row's largest group scale factor: the top of the UE4M3 range
+
+// Routes a plan has taken, reported to the host code by number.
+enum { kRouteNone = 0, kRouteNvfp4 = 1, kRouteBf16 = 2, kRouteFp8 = 3 };
+enum { kMoePrefill = 1, kMoeSorted = 2, kMoePairs = 3, kMoeGrouped = 4 };
+
+struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
+  Weight w;
+  at::Tensor workspace, slots;
+  int64_t row_batch_max = 16;
+  std::atomic<int> prefill_route{kRouteNone};
+  std::mutex mutex;
+  std::map<std::vector<const LinearPlan*>, at::Tensor> shared_slots;
+
+  LinearPlan(Weight weight, at::Tensor ws, const Opt& armed) : w(std::move(weight)), workspace(std::move(ws)) {
+    if (armed.has_value() && armed->defined()) slots = *armed;
+    row_batch_max = L.gb_gemv_row_batch_max(&w.w);
+  }
+
+  at::Tensor forward(const at::Tensor& x, int rule, bool nvfp4, int64_t midm_max) {
+    need_cuda(x);
+    const int64_t N = w.w.rows, K = w.w.K;
+    if (x.dim() < 1 || x.numel() % K != 0) throw std::runtime_error("activations do not divide into rows of " + std::to_string(K));
+    const int64_t M = x.numel() / K;
+    std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = N;
+    if (M == 0) return at::empty(shape, x.options());
+    need_bf16(x, "the codebook linear");
+    const c10::cuda::CUDAGuard guard(x.device());
+    void* stream = c10::cuda::getCurrentCUDAStream().stream();
+    const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+    at::Tensor out = at::empty(shape, x.options());
+    if (M == 1 && slots.defined()) {
+      const gb_weight* ws[1] = {&w.w};
+      void* ys[1] = {out.data_ptr()};
+      const int rc = L.gb_gemv_tab(xc.data_ptr(), ws, ys, 1, w.act(), rule, slots.data_ptr(), slots.numel(), stream);
+      if (rc == GB_OK) return out;
+      if (rc != GB_EUNSUPPORTED) check(rc);
+    }
+    if (M <= kDecodeMaxRows || M <= std::min(midm_max, row_batch_max)) {
+      at::Tensor ws = workspace;
+      const int64_t need = L.gb_gemv_workspace_bytes(M, N, K);
+      if (!ws.defined() || ws.numel() < need) ws = at::empty({need}, x.options().dtype(at::kByte));
+      check(L.gb_gemv(xc.data_ptr(), M, &w.w, w.act(), rule, out.data_ptr(), ws.data_ptr(), ws.numel(), stream));
+      return out;
+    }
+    prefill(xc, M, out, rule, nvfp4, stream);
+    return out;
+  }
+
+  // M > 16: the layer is expanded once into a transient decoded operand and multiplied on the tensor
+  // cores.  fp4 grid: native NVFP4 activations x the native NVFP4 view of the layer, block-scaled MMA
+  // (the reference's fused FP4 prefill lane, gridbook/csrc/cb_fused_fp4_gemm.cu:758-903; its
+  // activation bucket is NOT the decode contract's), or with nvfp4 off the decode contract kept:
+  // bucketed bf16 rows x bf16(value * scale) (gridbook/linear.py:983-1023,1146-1152).  fp8 grid:
+  // per-token E4M3 activations x the E4M3 value plane, both scales on the fp32 accumulator
+  // (gridbook/linear.py:1221-1264; epilogue of gridbook/csrc/cb_fused_gemm.cu:476-486).
+  void prefill(const at::Tensor& x, int64_t M, at::Tensor& out, int rule, bool nvfp4, void* stream) {
+    const int64_t N = w.w.rows, K = w.w.K;
+    Arena a;
+    if (w.fp4() && nvfp4) {
+      const int qa = a.add(M * K / 2), sa = a.add(L.gb_nvfp4_sf_bytes(M, K)), as = a.add(M * 4);
+      const int qb = a.add(N * K / 2), sb = a.add(L.gb_nvfp4_sf_bytes(N, K));
+      a.alloc(x);
+      check(L.gb_nvfp4_quantize_rows(x.data_ptr(), M, K, kNvfp4ActRange, a.ptr(qa), a.ptr(sa), a.ptr<float>(as), stream));
+      // scale factors of the rows past N stay unset: they only reach columns that are not stored
+      check(L.gb_expand_fp4_nvfp4(&w.w, 0, N, a.ptr(qb), a.ptr(sb), 2, stream));
+      check(L.gb_gemm_fp4(a.ptr(qa), a.ptr(sa), a.ptr(qb), a.ptr(sb), out.data_ptr(), M, N, K, a.ptr<float>(as),
+                          w.w.global_scale, stream));
+      prefill_route = kRouteNvfp4;
+    } else if (w.fp4()) {
+      const int xq = a.add(M * K * 2), wt = a.add(N * K * 2);
+      a.alloc(x);
+      check(L.gb_fp4_act_qdq(x.data_ptr(), a.ptr(xq), M, K, rule, stream));
+      check(L.gb_expand_fp4_bf16(&w.w, 0, N, a.ptr(wt), stream));
+      check(L.gb_gemm_tn(a.ptr(xq), a.ptr(wt), out.data_ptr(), M, N, K, GB_GEMM_BF16, nullptr, nullptr, w.w.global_scale, stream));
+      prefill_route = kRouteBf16;
+    } else {
+      const int q = a.add(M * K), as = a.add(M * 4), wt = a.add(N * K);
+      a.alloc(x);
+      check(L.gb_fp8_quantize_rows(x.data_ptr(), a.ptr(q), a.ptr<float>(as), M, K, rule, stream));
+      check(L.gb_expand_fp8(&w.w, 0, N, a.ptr(wt), stream));
+      check(L.gb_gemm_tn(a.ptr(q), a.ptr(wt), out.data_ptr(), M, N, K, GB_GEMM_E4M3, a.ptr<float>(as), w.w.weight_scale,
+                         w.w.global_scale, stream));
+      prefill_route = kRouteFp8;
+    }
+  }
+};
+
+// Several linears that read the same activation row, one launch; None when they have no such kernel.
+py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, const at::Tensor& x, int rule) {
+  const size_t n = plans.size();
+  if (n < 2 || n > 4 || !x.is_cuda() || x.dim() < 1) return py::none();
+  const int64_t K = plans[0]->w.w.K;
+  if (x.numel() != K) return py::none();
+  for (const auto& p : plans)
+    if (!p->slots.defined() || p->w.w.K != K) return py::none();
+  need_bf16(x, "the table GEMV");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const gb_weight* ws[4];
+  void* ys[4];
+  std::vector<const LinearPlan*> key;
+  for (size_t i = 0; i < n; ++i) {
+    ws[i] = &plans[i]->w.w;
+    key.push_back(plans[i].get());
+  }
+  at::Tensor slots;
+  {
+    std::lock_guard<std::mutex> lock(plans[0]->mutex);
+    at::Tensor& s = plans[0]->shared_slots[key];
+    if (!s.defined()) s = at::full({L.gb_gemv_tab_slots_bytes(ws, (int)n)}, 0xFF, x.options().dtype(at::kByte));
+    slots = s;
+  }
+  const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+  std::vector<at::Tensor> outs;
+  for (size_t i = 0; i < n; ++i) {
+    std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = ws[i]->rows;
+    outs.push_back(at::empty(shape, x.options()));
+    ys[i] = outs.back().data_ptr();
+  }
+  const int rc = L.gb_gemv_tab(xc.data_ptr(), ws, ys, (int)n, plans[0]->w.act(), rule, slots.data_ptr(), slots.numel(),
+                               c10::cuda::getCurrentCUDAStream().stream());
+  if (rc == GB_EUNSUPPORTED) return py::none();
+  check(rc);
+  return py::cast(outs);
+}
+
+struct MoEPlan {
+  Weight w13, w2;
+  Weight rows13, rows2;          // the stacks seen as one matrix of E * rows rows (for the expanders)
+  int64_t E, hidden, inter;
+  bool sorted_ok, pair_ok;
+  std::atomic<int> route{kRouteNone};
+  std::mutex mutex;
+  std::map<std::pair<int64_t, int64_t>, at::Tensor> x_rows;
+
+  MoEPlan(Weight a, Weight b, Weight ra, Weight rb, int64_t E_, int64_t hidden_, int64_t inter_, bool sorted_, bool pair_)
+      : w13(std::move(a)), w2(std::move(b)), rows13(std::move(ra)), rows2(std::move(rb)), E(E_), hidden(hidden_),
+        inter(inter_), sorted_ok(sorted_), pair_ok(pair_) {}
+
+  // token of every routed pair, one tensor per batch shape
+  const int32_t* x_row(int64_t T, int64_t topk, const at::Tensor& like) {
+    std::lock_guard<std::mutex> lock(mutex);
+    at::Tensor& t = x_rows[{T, topk}];
+    if (!t.defined())
+      t = at::arange(T * topk, like.options().dtype(at::kInt)).floor_divide(topk).to(at::kInt).contiguous();
+    return t.data_ptr<int32_t>();
+  }
+
+  struct Limits { int64_t pair_max, sorted_per_expert, sorted_other, prefill_per_expert, prefill_other, fused_bucket_max; };
+
+  at::Tensor forward(const at::Tensor& x, const at::Tensor& topk_weights, const at::Tensor& topk_ids, int rule,
+                     std::array<int64_t, 6> limits) {
+    need_cuda(x);
+    need_cuda(topk_ids);
+    need_cuda(topk_weights);
+    const Limits lim{limits[0], limits[1], limits[2], limits[3], limits[4], limits[5]};
+    const int64_t T = topk_ids.size(0), topk = topk_ids.size(1);
+    if (T == 0) return at::empty_like(x);
+    if (x.numel() != T * hidden) throw std::runtime_error("routed layer: " + std::to_string(T) + " tokens of " +
+                                                          std::to_string(hidden) + " values expected");
+    const c10::cuda::CUDAGuard guard(x.device());
+    Call c;
+    c.x = x.to(at::kBFloat16).contiguous();
+    c.ids = topk_ids.to(at::kInt).contiguous();
+    c.tw = topk_weights.to(at::kFloat).contiguous();
+    c.T = T; c.topk = topk; c.P = T * topk; c.rule = rule;
+    c.stream = c10::cuda::getCurrentCUDAStream().stream();
+    c.out = at::empty({T, hidden}, c.x.options());
+    const int64_t prefill_min = sorted_ok ? lim.prefill_per_expert : std::min(lim.prefill_per_expert, lim.prefill_other);
+    if (c.P >= prefill_min * E) prefill(c);
+    else if (sorted_ok && c.P >= (pair_ok ? lim.sorted_per_expert * E : lim.sorted_other)) sorted(c);
+    else if (!(c.P <= lim.pair_max && w13.fp4() && w2.fp4() && pairs(c))) grouped(c, c.P <= lim.fused_bucket_max);
+    at::Tensor out = c.out;
+    if (x.scalar_type() != at::kBFloat16) out = out.to(x.scalar_type());
+    return out.reshape(x.sizes());
+  }
+
+ private:
+  struct Call {
+    at::Tensor x, ids, tw, out;
+    int64_t T, topk, P;
+    int rule;
+    void* stream;
+  };
+
+  struct Routing { int counts, offsets, order, pair_w, ws; int64_t ws_bytes; };
+  Routing plan_routing(Arena& a, const Call& c) const {
+    Routing r;
+    r.counts = a.add(E * 4);
+    r.offsets = a.add((E + 1) * 4);
+    r.order = a.add(c.P * 4);
+    r.pair_w = a.add(c.P * 4);
+    r.ws_bytes = L.gb_moe_route_workspace_bytes(c.T, c.topk, E);
+    r.ws = a.add(r.ws_bytes);
+    return r;
+  }
+  void run_routing(const Arena& a, const Routing& r, const Call& c) const {
+    check(L.gb_moe_route_ws(c.ids.data_ptr<int32_t>(), c.T, c.topk, E, 0, a.ptr<int32_t>(r.counts), a.ptr<int32_t>(r.offsets),
+                            a.ptr<int32_t>(r.order), c.tw.data_ptr<float>(), a.ptr<float>(r.pair_w),
+                            r.ws_bytes ? a.ptr(r.ws) : nullptr, r.ws_bytes, c.stream));
+  }
+  static void bucket(const Weight& w, const void* in, void* out, int64_t rows, const Call& c) {
+    check(w.fp4() ? L.gb_fp4_act_qdq(in, out, rows, w.w.K, c.rule, c.stream)
+                  : L.gb_fp8_act_qdq(in, out, rows, w.w.K, c.rule, c.stream));
+  }
+  void combine(const void* y, const float* pair_w, const Call& c, bool round) const {
+    check(L.gb_moe_combine(y, pair_w, c.ids.data_ptr<int32_t>(), E, c.T, c.topk, hidden, round ? 1 : 0, c.out.data_ptr(),
+                           c.stream));
+  }
+
+  // Small batches of the literal format: every routed pair is its own M = 1 linear through the
+  // inner-product-table kernel (bucket fused; the down projection sums the gate/up K slices and
+  // applies SwiGLU while it stages its rows), then the combine.  False when there is no such kernel.
+  bool pairs(Call& c) {
+    if (!pair_ok) return false;
+    Arena a;
+    const int64_t need = L.gb_moe_mlp_pairs_workspace_bytes(c.P, w13.w.K, w2.w.K);
+    const int y = a.add(c.P * hidden * 2), ws = a.add(need);
+    a.alloc(c.x);
+    const int rc = L.gb_moe_mlp_pairs(c.x.data_ptr(), x_row(c.T, c.topk, c.x), &w13.w, w13.expert_stride, &w2.w,
+                                      w2.expert_stride, E, 0, c.ids.data_ptr<int32_t>(), c.P, 0, GB_ACT_FP4_GROUP16, c.rule,
+                                      a.ptr(y), nullptr, a.ptr(ws), std::max<int64_t>(need, 16), c.stream);
+    if (rc == GB_EUNSUPPORTED) return false;
+    check(rc);
+    combine(a.ptr(y), c.tw.data_ptr<float>(), c, true);
+    route = kMoePairs;
+    return true;
+  }
+
+  // Route -> bucket -> grouped gate/up GEMV with SwiGLU -> bucket -> grouped down GEMV -> combine.  Any
+  // format and token count: an expert's tokens are taken in passes of up to sixteen rows, its weights
+  // stream once per pass.  `fuse`: the fp4 bucket runs inside the grouped kernel while it stages the
+  // rows (two launches fewer for small batches; for large ones every row tile would repeat it).
+  void grouped(Call& c, bool fuse) {
+    Arena a;
+    const Routing r = plan_routing(a, c);
+    const bool fuse13 = fuse && w13.fp4(), fuse2 = fuse && w2.fp4();
+    const int xq = a.add(fuse13 ? 0 : c.T * hidden * 2), h = a.add(c.P * inter * 2);
+    const int hq = a.add(fuse2 ? 0 : c.P * inter * 2), y = a.add(c.P * hidden * 2);
+    a.alloc(c.x);
+    run_routing(a, r, c);
+    const int32_t *off = a.ptr<int32_t>(r.offsets), *ord = a.ptr<int32_t>(r.order);
+    const void* in = c.x.data_ptr();
+    if (!fuse13) {
+      bucket(w13, in, a.ptr(xq), c.T, c);
+      in = a.ptr(xq);
+    }
+    check(L.gb_moe_gemv(in, x_row(c.T, c.topk, c.x), &w13.w, w13.expert_stride, E, off, ord, c.P, 1,
+                        fuse13 ? GB_ACT_FP4_GROUP16 : GB_ACT_NONE, c.rule, a.ptr(h), nullptr, nullptr, 0, c.stream));
+    in = a.ptr(h);
+    if (!fuse2) {
+      bucket(w2, in, a.ptr(hq), c.P, c);
+      in = a.ptr(hq);
+    }
+    check(L.gb_moe_gemv(in, nullptr, &w2.w, w2.expert_stride, E, off, ord, c.P, 0,
+                        fuse2 ? GB_ACT_FP4_GROUP16 : GB_ACT_NONE, c.rule, a.ptr(y), nullptr, nullptr, 0, c.stream));
+    combine(a.ptr(y), a.ptr<float>(r.pair_w), c, false);
+    route = kMoeGrouped;
+  }
+
+  // SwiGLU over the sorted rows and the down projection's bucket on top.
+  void swiglu(const Arena& a, const Call& c, const Routing& r, int h13, int hs, int h) const {
+    const int32_t* off = a.ptr<int32_t>(r.offsets);
+    if (w2.fp4() && inter % 16 == 0) {
+      check(L.gb_moe_swiglu_rows(a.ptr(h13), off, E, c.P, inter, GB_ACT_FP4_GROUP16, c.rule, a.ptr(h), c.stream));
+      return;
+    }
+    check(L.gb_moe_swiglu_rows(a.ptr(h13), off, E, c.P, inter, GB_ACT_NONE, c.rule, a.ptr(hs), c.stream));
+    bucket(w2, a.ptr(hs), a.ptr(h), c.P, c);
+  }
+
+  // Mid-size batches: the rows in expert order, then per projection one launch in which every
+  // (expert, 128-row tile) decodes its packed rows into tensor memory and multiplies them with the
+  // expert's rows on the tensor cores; the down projection stores its rows back in pair order.  The
+  // two stacks may be of different grids: each projection's rows go through its own grid's bucket.
+  void sorted(Call& c) {
+    Arena a;
+    const Routing r = plan_routing(a, c);
+    const int xq = a.add(c.T * hidden * 2), xs = a.add(c.P * hidden * 2), h13 = a.add(c.P * 2 * inter * 2);
+    const int hs = a.add(w2.fp4() ? 0 : c.P * inter * 2), h = a.add(c.P * inter * 2), y = a.add(c.P * hidden * 2);
+    a.alloc(c.x);
+    run_routing(a, r, c);
+    const int32_t *off = a.ptr<int32_t>(r.offsets), *ord = a.ptr<int32_t>(r.order);
+    bucket(w13, c.x.data_ptr(), a.ptr(xq), c.T, c);
+    check(L.gb_moe_gather_rows(a.ptr(xq), x_row(c.T, c.topk, c.x), ord, off, E, c.P, hidden, a.ptr(xs), c.stream));
+    check(L.gb_moe_gemv_sorted(a.ptr(xs), &w13.w, w13.expert_stride, E, off, nullptr, c.P, a.ptr(h13), nullptr, c.stream));
+    swiglu(a, c, r, h13, hs, h);
+    check(L.gb_moe_gemv_sorted(a.ptr(h), &w2.w, w2.expert_stride, E, off, ord, c.P, a.ptr(y), nullptr, c.stream));
+    combine(a.ptr(y), a.ptr<float>(r.pair_w), c, false);
+    route = kMoeSorted;
+  }
+
+  // Many tokens per expert: each stack decoded once into a transient bf16 tile of the exact served
+  // weights, one grouped tensor-core GEMM over the expert segments per projection - the reference's
+  // grouped bf16 route (gridbook/moe.py:2388-2504 with gridbook/ops.py:137-306).  Both grids keep the
+  // decode contract: the buckets between the two projections are coarse enough to turn a last-place
+  // difference of the first projection into whole quantisation steps, so the fp8 grid does not take
+  // the scales-in-the-epilogue E4M3 GEMM of the dense prefill.
+  void prefill(Call& c) {
+    Arena a;
+    const Routing r = plan_routing(a, c);
+    const int64_t tile13 = E * w13.w.rows * w13.w.K * 2, tile2 = E * w2.w.rows * w2.w.K * 2;
+    const int tile = a.add(std::max(tile13, tile2));
+    const int xq = a.add(c.T * hidden * 2), xs = a.add(c.P * hidden * 2), h13 = a.add(c.P * 2 * inter * 2);
+    const int hs = a.add(w2.fp4() && inter % 16 == 0 ? 0 : c.P * inter * 2), h = a.add(c.P * inter * 2);
+    const int y = a.add(c.P * hidden * 2);
+    a.alloc(c.x);
+    run_routing(a, r, c);
+    const int32_t *off = a.ptr<int32_t>(r.offsets), *ord = a.ptr<int32_t>(r.order);
+    auto stage = [&](const Weight& stack, const Weight& one, const void* in, void* out, const int32_t* map) {
+      check(stack.fp4() ? L.gb_expand_fp4_bf16(&stack.w, 0, stack.w.rows, a.ptr(tile), c.stream)
+                        : L.gb_expand_fp8_bf16(&stack.w, 0, stack.w.rows, a.ptr(tile), c.stream));
+      check(L.gb_gemm_tn_grouped(in, a.ptr(tile), out, c.P, one.w.rows, one.w.K, GB_GEMM_BF16, E, off, map, nullptr, nullptr,
+                                 one.w.global_scale, c.stream));
+    };
+    bucket(w13, c.x.data_ptr(), a.ptr(xq), c.T, c);
+    check(L.gb_moe_gather_rows(a.ptr(xq), x_row(c.T, c.topk, c.x), ord, off, E, c.P, hidden, a.ptr(xs), c.stream));
+    stage(rows13, w13, a.ptr(xs), a.ptr(h13), nullptr);
+    swiglu(a, c, r, h13, hs, h);
+    stage(rows2, w2, a.ptr(h), a.ptr(y), ord);             // rows back in pair order
+    combine(a.ptr(y), a.ptr<float>(r.pair_w), c, false);
+    route = kMoePrefill;
+  }
+};
+
+}  // namespace
+
+PYBIND11_MODULE(_gb_torch, m) {
+  m.def("bind", &bind);
+  m.def("abi_version", [] { return GB_ABI_VERSION; });
+  py::class_<Weight>(m, "Weight").def(py::init(&make_weight));
+  py::class_<LinearPlan, std::shared_ptr<LinearPlan>>(m, "LinearPlan")
+      .def(py::init<Weight, at::Tensor, const Opt&>())
+      .def("__call__", &LinearPlan::forward, py::call_guard<py::gil_scoped_release>())
+      .def_property_readonly("prefill_route", [](const LinearPlan& p) { return p.prefill_route.load(); });
+  py::class_<MoEPlan, std::shared_ptr<MoEPlan>>(m, "MoEPlan")
+      .def(py::init<Weight, Weight, Weight, Weight, int64_t, int64_t, int64_t, bool, bool>())
+      .def("__call__", &MoEPlan::forward, py::call_guard<py::gil_scoped_release>())
+      .def_property_readonly("route", [](const MoEPlan& p) { return p.route.load(); });
+  m.def("shared_row", &shared_row);
+}

@@ -80,8 +80,30 @@ def make_weight(qw, codebook, fmt: CBFormat, K: int, *, cb_row_offset=None, comp
                         weight_scale, global_scale)
 
 
-def _rule(scale_rule: str) -> int:
+def host_weight(w: PackedWeight):
+    """The weight for the compiled host path, which keeps its tensors alive."""
+    f = w.fmt.to_native()
+    return nat.host().Weight(
+        w.qw, w.codebook, [f.grid, f.mode, f.k_bits, f.n_sub, f.type_size, f.scale_coding], w.K, w.rows, w.row_stride,
+        w.cb_row_offset, w.compose, w.weight_scale, float(w.global_scale), w.expert_stride, w.experts)
+
+
+_is_compiling = torch.compiler.is_compiling
+_dispatch_modes = torch._C._len_torch_dispatch_stack
+
+
+def takes_plan(x: torch.Tensor) -> bool:
+    """Whether a layer may call its plan without the opaque operator in between: nothing is tracing,
+    no dispatch mode watches the operators and no gradient is asked for.  (The operator costs more
+    than the launches of a decode row.)"""
+    return (not _is_compiling() and type(x) is torch.Tensor and not x.requires_grad and _dispatch_modes() == 0)
+
+
+def rule_code(scale_rule: str) -> int:
     return nat.SCALE_RULE_DIV if scale_rule == "div" else nat.SCALE_RULE_RECIP
+
+
+_rule = rule_code
 
 
 def fp4_act_qdq(x: torch.Tensor, scale_rule: str = "recip") -> torch.Tensor:

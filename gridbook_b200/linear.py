@@ -5,7 +5,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _native, codec, kernels
+from . import _native, codec, kernels, ops
 from ._native import NativeKernelUnavailableError
 from ._vllm_compat import (ChannelQuantScaleParameter, LinearMethodBase, ModelWeightParameter,
                            PerTensorScaleParameter, register_weight_loader_v2_supported_method)
@@ -13,6 +13,31 @@ from .formats import CBFormat
 
 DECODE_MAX_M = 16          # the decode-batch kernels take up to sixteen rows
 MIDM_MAX_M = 128           # ... and the literal format's tensor-core decode kernel up to this many
+
+
+_PREFILL_ROUTES = {
+    1: "nvfp4 activations + expand_fp4_nvfp4 + gemm_fp4(kind::mxf4nvf4)",
+    2: "expand_fp4_bf16 + gemm_tn(kind::f16)",
+    3: "expand_fp8 + gemm_tn(kind::f8f6f4)",
+}
+
+
+class _Route(dict):
+    """What a layer runs on; "prefill" is the route its last prefill took."""
+
+    def __init__(self, plan, **fixed):
+        super().__init__(fixed)
+        self._plan = plan
+
+    def get(self, key, default=None):
+        if key == "prefill":
+            return _PREFILL_ROUTES.get(self._plan.prefill_route, default)
+        return super().get(key, default)
+
+    def __getitem__(self, key):
+        if key == "prefill" and self.get(key) is not None:
+            return self.get(key)
+        return super().__getitem__(key)
 
 
 @register_weight_loader_v2_supported_method
@@ -136,75 +161,33 @@ class PrismaQuantCBLinearMethod(LinearMethodBase):
         layer._cb_N, layer._cb_K = N, K
         layer._cb_workspace = torch.empty(
             _native.load().gb_gemv_workspace_bytes(DECODE_MAX_M, N, K), dtype=torch.uint8, device=dev)
-        from .ops import register_cb_layer, warn_if_capture_sizes_exceed_the_decode_gates
-        layer._cb_layer_id = register_cb_layer(self, layer)
-        warn_if_capture_sizes_exceed_the_decode_gates()
-        layer._cb_route = {"kernel": "gemv_kernel", "format": str(self.fmt), "N": N, "K": K}
+        layer._cb_layer_id = ops.register_cb_layer(self, layer)
+        ops.warn_if_capture_sizes_exceed_the_decode_gates()
         # one activation row of the literal format: the one-launch table kernel and its armed slots
         layer._cb_slots = (kernels.new_tab_slots([layer._cb_weight])
                            if kernels.table_kernel_applies(layer._cb_weight) else None)
+        layer._cb_plan = _native.host(f"{self.prefix}: CB Linear").LinearPlan(
+            kernels.host_weight(layer._cb_weight), layer._cb_workspace, layer._cb_slots)
+        layer._cb_route = _Route(layer._cb_plan, kernel="gemv_kernel", format=str(self.fmt), N=N, K=K)
 
     # ------------------------------------------------------------------ forward
     def apply(self, layer, x, bias=None):
         if bias is not None:
             raise NativeKernelUnavailableError(f"{self.prefix}: biased CB Linear has no native operator")
+        plan = layer.__dict__.get("_cb_plan")
+        if plan is not None and kernels.takes_plan(x):
+            return plan(x, kernels.rule_code(ops.ACT_SCALE_RULE), self.prefill_route == "nvfp4", self.midm_max_rows)
         lid = getattr(layer, "_cb_layer_id", None)
         if lid is None:
             raise NativeKernelUnavailableError(
                 f"{self.prefix}: CB Linear was not registered during process_weights_after_loading")
-        from .ops import cb_linear_forward
-        return cb_linear_forward(x, lid)
+        return ops.cb_linear_forward(x, lid)
 
     def _apply_inline(self, layer, x, bias=None):
-        from . import ops
-        w = layer._cb_weight
-        N, K = layer._cb_N, layer._cb_K
-        x2 = x.reshape(-1, K)
-        M = x2.shape[0]
-        if M == 0:
-            return x.new_empty((*x.shape[:-1], N))
-        if M == 1 and getattr(layer, "_cb_slots", None) is not None:
-            outs = kernels.gemv_tab(x2, [w], layer._cb_slots, act=self.fmt.grid, scale_rule=ops.ACT_SCALE_RULE)
-            if outs is not None:
-                return outs[0].reshape(*x.shape[:-1], N)
-        if M <= DECODE_MAX_M or M <= min(self.midm_max_rows, kernels.row_batch_max_rows(w)):
-            # past sixteen rows: the literal format's tensor-core decode kernel, no decoded transient
-            return kernels.gemv(x2, w, act=self.fmt.grid, scale_rule=ops.ACT_SCALE_RULE,
-                                workspace=layer._cb_workspace).reshape(*x.shape[:-1], N)
-        return self._apply_prefill(layer, x2).reshape(*x.shape[:-1], N)
-
-    def _apply_prefill(self, layer, x2):
-        """M > 16: expand the layer once into a transient decoded tile and run one tensor-core
-        GEMM over it (tcgen05, accumulator in tensor memory).
-
-        fp4 grid, route "nvfp4" (default): the rows are quantised to native NVFP4 (per-row scale,
-        UE4M3 group scale factors, nearest-even E2M1), the layer is expanded to its native NVFP4
-        view (packed E2M1 + E4M3 group scales, 0.56 bytes per weight) and the two meet in a
-        block-scaled kind::mxf4nvf4 MMA — the reference's fused FP4 prefill lane
-        (gridbook/csrc/cb_fused_fp4_gemm.cu:758-903); its activation bucket is NOT the decode
-        contract's (UE4M3 scale factors instead of fp32 amax / 6).  Route "bf16": activations go
-        through the group-16 bucket, the tile is the exact bf16 served weight, kind::f16 MMA —
-        the reference's expand + bf16 GEMM route with the decode numerics
-        (gridbook/linear.py:983-1023,1146-1152).  fp8 grid: activations are quantised per token to
-        E4M3, the tile is the E4M3 value plane, kind::f8f6f4 MMA, and both scales multiply the
-        fp32 accumulator — the reference's fp8 prefill lanes
-        (gridbook/linear.py:1221-1264; epilogue of gridbook/csrc/cb_fused_gemm.cu:476-486)."""
-        from . import ops
-        w = layer._cb_weight
-        if self.is_fp4 and self.prefill_route == "nvfp4":
-            a, sfa, a_scale = kernels.nvfp4_quantize_rows(x2.contiguous())
-            b, sfb = kernels.expand_fp4_nvfp4(w, operand=True)
-            layer._cb_route["prefill"] = "nvfp4 activations + expand_fp4_nvfp4 + gemm_fp4(kind::mxf4nvf4)"
-            return kernels.gemm_fp4(a, sfa, b, sfb, a_scale=a_scale, global_scale=w.global_scale)
-        if self.is_fp4:
-            xq = kernels.fp4_act_qdq(x2.contiguous(), ops.ACT_SCALE_RULE)
-            wt = kernels.expand_fp4_bf16(w)
-            layer._cb_route["prefill"] = "expand_fp4_bf16 + gemm_tn(kind::f16)"
-            return kernels.gemm_tn(xq, wt, global_scale=w.global_scale)
-        q, a_scale = kernels.fp8_quantize_rows(x2.contiguous(), ops.ACT_SCALE_RULE)
-        wt = kernels.expand_fp8(w)
-        layer._cb_route["prefill"] = "expand_fp8 + gemm_tn(kind::f8f6f4)"
-        return kernels.gemm_tn(q, wt, a_scale=a_scale, b_scale=w.weight_scale, global_scale=w.global_scale)
+        """What the opaque operator runs: decode batches (one row of the literal format through its
+        one-launch table kernel, up to sixteen rows - or what the tensor-core decode kernel takes -
+        without a decoded transient), expand + GEMM past them (LinearPlan in csrc/gb_torch.cpp)."""
+        return layer._cb_plan(x, kernels.rule_code(ops.ACT_SCALE_RULE), self.prefill_route == "nvfp4", self.midm_max_rows)
 
 
 def apply_shared_row(layers, x: torch.Tensor):
@@ -212,20 +195,12 @@ def apply_shared_row(layers, x: torch.Tensor):
     and up kept as separate modules): one launch builds the inner-product tables once per CTA and
     streams all of them.  Falls back to one call per layer when the batch is not a single row or a
     layer's format has no table kernel.  -> list of outputs, in the order of ``layers``."""
-    from . import ops
     layers = list(layers)
-    ws = [l._cb_weight for l in layers]
-    x2 = x.reshape(-1, ws[0].K)
-    if (x2.shape[0] == 1 and 1 < len(layers) <= 4 and all(getattr(l, "_cb_slots", None) is not None for l in layers)
-            and all(w.K == ws[0].K for w in ws)):
-        key = tuple(l._cb_layer_id for l in layers)
-        cache = layers[0].__dict__.setdefault("_cb_shared_slots", {})
-        slots = cache.get(key)
-        if slots is None:
-            slots = cache[key] = kernels.new_tab_slots(ws)
-        outs = kernels.gemv_tab(x2, ws, slots, act=ws[0].fmt.grid, scale_rule=ops.ACT_SCALE_RULE)
+    plans = [l.__dict__.get("_cb_plan") for l in layers]
+    if all(p is not None for p in plans) and kernels.takes_plan(x):
+        outs = _native.host().shared_row(plans, x, kernels.rule_code(ops.ACT_SCALE_RULE))
         if outs is not None:
-            return [o.reshape(*x.shape[:-1], w.rows) for o, w in zip(outs, ws)]
+            return outs
     return [l(x) for l in layers]
 
 

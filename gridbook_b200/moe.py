@@ -7,7 +7,7 @@ import sys
 
 import torch
 
-from . import _native, codec, kernels
+from . import _native, codec, kernels, ops
 from ._native import NativeKernelUnavailableError
 from ._vllm_compat import FusedMoEMethodBase
 from .formats import CBFormat
@@ -36,6 +36,10 @@ SORTED_MIN_PAIRS_OTHER = 16
 # the decode kernel's 16-row passes straight to the decoded stack + grouped GEMM, whose crossover
 # with the decode kernel was measured at ~800 tokens of 128 experts top-8.
 PREFILL_MIN_PAIRS_OTHER = 50
+
+
+_ROUTES = {0: "", 1: "grouped prefill: expand + gemm_tn_grouped",
+           2: "sorted rows: decode into tensor memory + tcgen05", 3: "per-pair table kernel", 4: "grouped decode kernel"}
 
 
 def _row_bytes(in_features: int, type_size: int) -> int:
@@ -266,9 +270,14 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
         layer._cb_w2 = self._stack_weight(layer, "w2_cb_qweight", "w2_weight_scale", self.fmt2,
                                           layer._cb_inter, "w2")
         layer._cb_E = layer.w13_cb_qweight.shape[0]
-        layer._cb_xrow_cache = {}
-        from .ops import register_cb_layer
-        layer._cb_layer_id = register_cb_layer(self, layer)
+        w13, w2 = layer._cb_w13, layer._cb_w2
+        sorted_ok = (kernels.moe_gemv_sorted_applies(w13) and kernels.moe_gemv_sorted_applies(w2)
+                     and not (w2.fmt.is_fp4 and layer._cb_inter % 16))
+        pair_ok = kernels.pair_kernel_applies(w13) and kernels.pair_kernel_applies(w2)
+        layer._cb_plan = _native.host(f"{self.prefix}: CB routed experts").MoEPlan(
+            kernels.host_weight(w13), kernels.host_weight(w2), kernels.host_weight(kernels.stack_rows(w13)),
+            kernels.host_weight(kernels.stack_rows(w2)), layer._cb_E, layer._cb_hidden, layer._cb_inter, sorted_ok, pair_ok)
+        layer._cb_layer_id = ops.register_cb_layer(self, layer)
         print(f"[prismaquant-cb] {self.prefix}: decode=grouped-cuda (sm_100a) "
               f"w13={self.fmt13.grid}/k{self.fmt13.k} w2={self.fmt2.grid}/k{self.fmt2.k}",
               file=sys.stderr, flush=True)
@@ -295,152 +304,25 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
             raise NativeKernelUnavailableError(
                 f"{self.prefix}: argument {key}={val!r} changes the routed computation and has no native "
                 "Gridbook operator")
+        if layer.__dict__.get("_cb_plan") is not None and kernels.takes_plan(x):
+            return self._apply_inline(layer, x, topk_weights, topk_ids)
         lid = getattr(layer, "_cb_layer_id", None)
         if lid is None:
             raise NativeKernelUnavailableError(
                 f"{self.prefix}: CB experts were not registered during process_weights_after_loading")
-        from .ops import cb_moe_forward
-        return cb_moe_forward(x, topk_weights, topk_ids, lid)
-
-    def _x_row(self, layer, T: int, topk: int, device):
-        key = (T, topk)
-        cached = layer._cb_xrow_cache.get(key)
-        if cached is None:
-            cached = (torch.arange(T * topk, device=device, dtype=torch.int32) // topk).contiguous()
-            layer._cb_xrow_cache[key] = cached
-        return cached
+        return ops.cb_moe_forward(x, topk_weights, topk_ids, lid)
 
     def _apply_inline(self, layer, x, topk_weights, topk_ids):
-        """route -> bucket -> grouped gate/up GEMV with SwiGLU -> bucket -> grouped down GEMV ->
-        combine.  Four launches for small batches (the buckets fused into the grouped kernels), six
-        otherwise; no host read, any token count (an expert's tokens are taken
-        in passes of up to sixteen rows, its weights stream once per pass)."""
-        from . import ops
-        rule = ops.ACT_SCALE_RULE
-        T, topk = topk_ids.shape
-        if T == 0:
-            return torch.empty_like(x)
-        x2 = x.reshape(T, -1).to(torch.bfloat16).contiguous()
-        ids = topk_ids.to(torch.int32).contiguous()
-        sorted_ok = (kernels.moe_gemv_sorted_applies(layer._cb_w13) and kernels.moe_gemv_sorted_applies(layer._cb_w2)
-                     and not (layer._cb_w2.fmt.is_fp4 and layer._cb_inter % 16))
-        prefill_min = (self.prefill_min_pairs_per_expert if sorted_ok
-                       else min(self.prefill_min_pairs_per_expert, self.prefill_min_pairs_other))
-        if T * topk >= prefill_min * layer._cb_E:
-            return self._apply_prefill(layer, x2, topk_weights, ids, rule).to(x.dtype).reshape(x.shape)
-        pair_kernel = kernels.pair_kernel_applies(layer._cb_w13) and kernels.pair_kernel_applies(layer._cb_w2)
-        if T * topk >= (self.sorted_min_pairs_per_expert * layer._cb_E if pair_kernel else self.sorted_min_pairs_other):
-            out = self._apply_sorted(layer, x2, topk_weights, ids, rule)
-            if out is not None:
-                return out.to(x.dtype).reshape(x.shape)
-        if T * topk <= self.pair_kernel_max_pairs and self.fmt13.is_fp4 and self.fmt2.is_fp4:
-            out = self._apply_pairs(layer, x2, topk_weights, ids, rule)
-            if out is not None:
-                layer._cb_route = "per-pair table kernel"
-                return out.to(x.dtype).reshape(x.shape)
-        # the loop chain multiplies by the bf16-rounded router weight (gridbook/moe.py:2407-2408);
-        # the routing launch writes it, zeroed for padded pairs
-        _, offsets, order, pair_w = kernels.moe_route(ids, layer._cb_E, topk_weights)
-        # Small batches: the fp4 bucket runs inside the grouped kernel while it stages the rows
-        # (two launches fewer); large ones bucket once up front, since every row tile of an expert
-        # would otherwise bucket the same rows again.
-        fuse = T * topk <= FUSED_BUCKET_MAX_PAIRS
-        x_row = self._x_row(layer, T, topk, x.device)
-        if fuse and self.fmt13.is_fp4:
-            a = kernels.moe_gemv(x2, layer._cb_w13, offsets, order, x_row=x_row, swiglu=True, clear=False,
-                                 act="fp4", scale_rule=rule)
-        else:
-            bucket13 = kernels.fp4_act_qdq if self.fmt13.is_fp4 else kernels.fp8_act_qdq
-            a = kernels.moe_gemv(bucket13(x2, rule), layer._cb_w13, offsets, order, x_row=x_row, swiglu=True,
-                                 clear=False)
-        if fuse and self.fmt2.is_fp4:
-            y = kernels.moe_gemv(a, layer._cb_w2, offsets, order, clear=False, act="fp4", scale_rule=rule)
-        else:
-            bucket2 = kernels.fp4_act_qdq if self.fmt2.is_fp4 else kernels.fp8_act_qdq
-            y = kernels.moe_gemv(bucket2(a, rule), layer._cb_w2, offsets, order, clear=False)
-        out = kernels.moe_combine(y, pair_w, T, topk, topk_ids=ids, E=layer._cb_E)
-        layer._cb_route = "grouped decode kernel"
-        return out.to(x.dtype).reshape(x.shape)
-
-
-    def _apply_prefill(self, layer, x2, topk_weights, ids, rule):
-        """Many tokens per expert: decode each stack once into a transient bf16 tile of the exact
-        served weights and run one grouped tensor-core GEMM over the expert segments per
-        projection (tcgen05 kind::f16, accumulators in tensor memory; segment offsets stay on the
-        device) - the reference's grouped bf16 route (gridbook/moe.py:2388-2504 with
-        gridbook/ops.py:137-306).  Both grids keep the decode contract here (bucketed bf16 rows,
-        per-weight bf16(value * scale)): the buckets between the two projections are coarse
-        enough to turn a last-place difference of the first projection into whole quantisation
-        steps, so the fp8 grid does not take the scales-in-the-epilogue E4M3 GEMM of the dense
-        prefill."""
-        T, topk = ids.shape
-        E = layer._cb_E
-        _, offsets, order, pair_w = kernels.moe_route(ids, E, topk_weights)
-        x_row = self._x_row(layer, T, topk, x2.device)
-
-        def bucket(rows, w):
-            return (kernels.fp4_act_qdq if w.fmt.is_fp4 else kernels.fp8_act_qdq)(rows, rule)
-
-        def stage(rows_sorted, w, row_map):
-            wm = kernels.stack_rows(w)
-            tile = kernels.expand_fp4_bf16(wm) if w.fmt.is_fp4 else kernels.expand_fp8_bf16(wm)
-            return kernels.gemm_tn_grouped(rows_sorted, tile, offsets, w.rows, row_map=row_map,
-                                           global_scale=w.global_scale)
-
-        w13, w2 = layer._cb_w13, layer._cb_w2
-        # bucket the T rows once, then bring them into expert order
-        a = kernels.moe_gather_rows(bucket(x2, w13), order, offsets, x_row=x_row)
-        if w2.fmt.is_fp4 and layer._cb_inter % 16 == 0:       # SwiGLU and the fp4 bucket in one launch
-            h = kernels.moe_swiglu_rows(stage(a, w13, None), offsets, act="fp4", scale_rule=rule)
-        else:
-            h = bucket(kernels.moe_swiglu_rows(stage(a, w13, None), offsets), w2)
-        y = stage(h, w2, order)                               # rows back in pair order
-        layer._cb_route = "grouped prefill: expand + gemm_tn_grouped"
-        return kernels.moe_combine(y, pair_w, T, topk, topk_ids=ids, E=E)
-
-    def _apply_sorted(self, layer, x2, topk_weights, ids, rule):
-        """Mid-size batches: route, bucket, bring the rows into expert order, then per projection one
-        launch in which every (expert, 128-row tile) decodes its packed rows into tensor memory and
-        multiplies them with the expert's rows on the tensor cores (tcgen05, 64 rows per pass);
-        SwiGLU and the second bucket between them; the down projection stores its rows back in pair
-        order for the combine.  The two stacks may be of different grids (an fp8-grid gate_up over an
-        fp4-grid down): each projection's rows go through its own grid's bucket.  None when a stack
-        is not of a format that kernel decodes (kernels.moe_gemv_sorted_applies)."""
-        w13, w2 = layer._cb_w13, layer._cb_w2
-        if not (kernels.moe_gemv_sorted_applies(w13) and kernels.moe_gemv_sorted_applies(w2)):
-            return None
-        if w2.fmt.is_fp4 and layer._cb_inter % 16:
-            return None
-        T, topk = ids.shape
-        E = layer._cb_E
-        _, offsets, order, pair_w = kernels.moe_route(ids, E, topk_weights)
-        x_row = self._x_row(layer, T, topk, x2.device)
-        xq = kernels.fp4_act_qdq(x2, rule) if w13.fmt.is_fp4 else kernels.fp8_act_qdq(x2, rule)
-        a = kernels.moe_gather_rows(xq, order, offsets, x_row=x_row)
-        h13 = kernels.moe_gemv_sorted(a, w13, offsets)
-        if h13 is None:
-            return None
-        if w2.fmt.is_fp4:
-            h = kernels.moe_swiglu_rows(h13, offsets, act="fp4", scale_rule=rule)
-        else:
-            h = kernels.fp8_act_qdq(kernels.moe_swiglu_rows(h13, offsets), rule)
-        y = kernels.moe_gemv_sorted(h, w2, offsets, row_map=order)
-        if y is None:
-            return None
-        layer._cb_route = "sorted rows: decode into tensor memory + tcgen05"
-        return kernels.moe_combine(y, pair_w, T, topk, topk_ids=ids, E=E)
-
-    def _apply_pairs(self, layer, x2, topk_weights, ids, rule):
-        """Small batches of the literal format: every routed pair is its own M = 1 linear through
-        the inner-product-table kernel (bucket fused; the down projection sums the gate/up K
-        slices and applies SwiGLU while it stages its rows), then the combine.  Three launches, no
-        routing tables.  None when the format has no such kernel."""
-        T, topk = ids.shape
-        x_row = self._x_row(layer, T, topk, x2.device)
-        y = kernels.moe_mlp_pairs(x2, layer._cb_w13, layer._cb_w2, ids, x_row=x_row, act="fp4", scale_rule=rule)
-        if y is None:
-            return None
-        return kernels.moe_combine(y, topk_weights, T, topk, topk_ids=ids, E=layer._cb_E, round_weights=True)
+        """The routed MLP of a batch of any size: per-pair table kernels, sorted rows on the tensor-core
+        decode kernel, decoded stacks + grouped GEMMs, or the grouped decode kernel, chosen from the
+        number of routed pairs and this method's thresholds (MoEPlan in csrc/gb_torch.cpp).  No host
+        read, so every size can be captured."""
+        plan = layer._cb_plan
+        out = plan(x, topk_weights, topk_ids, kernels.rule_code(ops.ACT_SCALE_RULE),
+                   (self.pair_kernel_max_pairs, self.sorted_min_pairs_per_expert, self.sorted_min_pairs_other,
+                    self.prefill_min_pairs_per_expert, self.prefill_min_pairs_other, FUSED_BUCKET_MAX_PAIRS))
+        layer.__dict__["_cb_route"] = _ROUTES[plan.route]
+        return out
 
 
 class CBMoE(torch.nn.Module):
