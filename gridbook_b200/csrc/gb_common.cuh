@@ -156,12 +156,18 @@ GB_DEVINL float gb_e2m1_rtn(float v) {
   return fabsf(__fsub_rn(hi, v)) < fabsf(__fsub_rn(v, lo)) ? hi : lo;
 }
 
-// The two roundings above cost a division and some thirty selects per value.  Both only ask which
-// side of a few midpoints the quotient lies on, so they are taken from an approximate quotient (a
-// multiply by the reciprocal, off by less than 2^-21 relative) with the hardware's conversion, and
-// done again the slow way when the two ends of [x (1 - 2^-20), x (1 + 2^-20)] convert differently:
-// about one pair of values in 2^17, ties among them.  Same bits as the slow way, always.
-constexpr float kGbNear = 0x1p-20f;
+// v / d, correctly rounded, given rinv = RN(1 / d): a product and one correction step with an exact
+// remainder (Markstein's theorem; it excludes a divisor whose significand is all ones and needs a
+// finite quotient, see gb_plain_division).  Three instructions where __fdiv_rn takes about ten.
+GB_DEVINL float gb_div(float v, float d, float rinv) {
+  const float q = v * rinv;
+  return fmaf(fmaf(-q, d, v), rinv, q);
+}
+
+// Divisors gb_div does not take.
+GB_DEVINL bool gb_plain_division(float d) {
+  return (__float_as_uint(d) & 0x7FFFFFu) == 0x7FFFFFu || !(d < __int_as_float(0x7F800000));
+}
 
 // Two fp32 -> one byte of two E2M1 codes (a in the low nibble), nearest, |value| clamped to 6.
 GB_DEVINL uint32_t gb_cvt_e2m1x2(float a, float b) {
@@ -177,31 +183,26 @@ GB_DEVINL uint32_t gb_cvt_e4m3x2(float a, float b) {
   return r;
 }
 
-// The E2M1 code of a value on the grid.
-GB_DEVINL uint32_t gb_e2m1_code(float v) {
-  const float m = fabsf(v);
-  const uint32_t c = m < 2.0f ? (uint32_t)(m * 2.0f) : (m < 4.0f ? (uint32_t)m + 2u : (m < 6.0f ? 6u : 7u));
-  return c | (v < 0.0f ? 8u : 0u);
-}
-
-// E2M1 codes of v0 / scale and v1 / scale under the reference's tie rule; `rinv` is 1 / scale to
-// within a few ulp.  Finite arguments.  A zero may carry either sign.
+// E2M1 codes of v0 / scale and v1 / scale under the reference's tie rule (finite arguments, a divisor
+// gb_div takes).  The conversion rounds a tie to the even code; the rule wants the lower value.  Every
+// midpoint has its low 21 significand bits clear, so a quotient with those bits clear moves down by
+// an ulp first: grid values among them convert as before.  A zero may carry either sign.
+// (Midpoints are no rare accident: bf16 values reach them in half a percent of cases, so nearly
+// every warp holds one and a slow path for them cost 160 us of the routed SwiGLU launch.)
 GB_DEVINL uint32_t gb_e2m1_div2(float v0, float v1, float scale, float rinv) {
-  const float x0 = v0 * rinv, x1 = v1 * rinv;
-  const uint32_t hi = gb_cvt_e2m1x2(fmaf(x0, kGbNear, x0), fmaf(x1, kGbNear, x1));
-  const uint32_t lo = gb_cvt_e2m1x2(fmaf(x0, -kGbNear, x0), fmaf(x1, -kGbNear, x1));
-  if (hi == lo) return hi;
-  return gb_e2m1_code(gb_e2m1_rtn(__fdiv_rn(v0, scale))) | (gb_e2m1_code(gb_e2m1_rtn(__fdiv_rn(v1, scale))) << 4);
+  float x0 = gb_div(v0, scale, rinv), x1 = gb_div(v1, scale, rinv);
+  if ((__float_as_uint(x0) & 0x1FFFFFu) == 0) x0 = fmaf(fabsf(x0), -0x1p-22f, x0);
+  if ((__float_as_uint(x1) & 0x1FFFFFu) == 0) x1 = fmaf(fabsf(x1), -0x1p-22f, x1);
+  return gb_cvt_e2m1x2(x0, x1);
 }
 
 // E4M3 bytes of clamp(v / scale, +-448), one rounding each; NaN clamps to -448 as fmaxf leaves it.
-GB_DEVINL uint32_t gb_e4m3_div2(float v0, float v1, float scale, float rinv) {
-  const float x0 = fminf(fmaxf(v0 * rinv, -448.0f), 448.0f), x1 = fminf(fmaxf(v1 * rinv, -448.0f), 448.0f);
-  const uint32_t hi = gb_cvt_e4m3x2(fmaf(x0, kGbNear, x0), fmaf(x1, kGbNear, x1));
-  const uint32_t lo = gb_cvt_e4m3x2(fmaf(x0, -kGbNear, x0), fmaf(x1, -kGbNear, x1));
-  if (hi == lo) return hi;
-  return gb_f32_to_e4m3(fminf(fmaxf(__fdiv_rn(v0, scale), -448.0f), 448.0f)) |
-         (gb_f32_to_e4m3(fminf(fmaxf(__fdiv_rn(v1, scale), -448.0f), 448.0f)) << 8);
+// `plain`: a divisor gb_div does not take.
+GB_DEVINL uint32_t gb_e4m3_div2(float v0, float v1, float scale, float rinv, bool plain) {
+  float x0, x1;
+  if (plain) { x0 = __fdiv_rn(v0, scale); x1 = __fdiv_rn(v1, scale); }
+  else { x0 = gb_div(v0, scale, rinv); x1 = gb_div(v1, scale, rinv); }
+  return gb_cvt_e4m3x2(fminf(fmaxf(x0, -448.0f), 448.0f), fminf(fmaxf(x1, -448.0f), 448.0f));
 }
 
 // Two E2M1 codes (one byte) -> fp32.
@@ -224,8 +225,8 @@ GB_DEVINL float gb_fp4_group_scale(float amax, int scale_rule) {
 }
 
 // bf16 pair of the bucket: E2M1(v / scale) * scale, rounded once each; a zero comes out positive.
-// `odd` (an infinity or a NaN in the group): the plain formulation, which spreads it as the
-// reference's codec does.
+// `odd` (an infinity or a NaN in the group, which spreads as in the reference's codec, or a scale
+// gb_div does not take): the plain formulation.
 GB_DEVINL uint32_t gb_fp4_bucket2(float v0, float v1, float scale, float rinv, bool odd) {
   if (odd) {
     const float q0 = __fmul_rn(gb_e2m1_rtn(__fdiv_rn(v0, scale)), scale);
@@ -256,7 +257,7 @@ GB_DEVINL void gb_fp4_bucket_words(uint32_t (&w)[kWords], float amax, bool nan, 
   amax = fmaxf(amax, 1e-8f);
   float scale = gb_fp4_group_scale(amax, scale_rule);
   if (nan) scale = __int_as_float(0x7FC00000);
-  const bool odd = !(amax < __int_as_float(0x7F800000)) || nan;
+  const bool odd = gb_plain_division(scale) || nan;
   const float rinv = __frcp_rn(scale);
 #pragma unroll
   for (int i = 0; i < kWords; ++i)

@@ -64,6 +64,7 @@ fp8_rows_kernel(const uint4* __restrict__ x, void* __restrict__ out, float* __re
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   const float s = scale_rule == GB_SCALE_RULE_DIV ? __fdiv_rn(amax, 448.0f) : __fmul_rn(amax, 1.0f / 448.0f);
   const float scale = fmaxf(s, 1.0f / (448.0f * 512.0f)), rinv = __frcp_rn(scale);
+  const bool plain = gb_plain_division(scale);
   if (kQuantize && threadIdx.x == 0) scale_out[blockIdx.x] = scale;
 #pragma unroll
   for (int j = 0; j < kVec; ++j) {
@@ -72,7 +73,7 @@ fp8_rows_kernel(const uint4* __restrict__ x, void* __restrict__ out, float* __re
     const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
     uint32_t q[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) q[c] = gb_e4m3_div2(gb_bf16_bits_to_f32(w[c] & 0xFFFFu), gb_bf16_bits_to_f32(w[c] >> 16), scale, rinv);
+    for (int c = 0; c < 4; ++c) q[c] = gb_e4m3_div2(gb_bf16_bits_to_f32(w[c] & 0xFFFFu), gb_bf16_bits_to_f32(w[c] >> 16), scale, rinv, plain);
     if (kQuantize) {
       reinterpret_cast<uint2*>(out)[(int64_t)blockIdx.x * vecs + i] = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
     } else {

@@ -313,18 +313,8 @@ gemm_fp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 //   sign bit = sign of xs (kept on zeros); a zero SF zeroes its group.
 // Every operation is a correctly rounded fp32 one (no approximate reciprocal), so the bytes are
 // those of the torch formulation.
-// The quotient xs / SF is taken as a product with the reciprocal and redone as a division when it
-// lies near a rounding boundary (gb_common.cuh, kGbNear).
-//
 // One CTA per row, one to four groups per thread kept in registers: the row is read once
 // (2048 x 17408: 38.6 us when it was read twice and every value divided twice).
-GB_DEVINL uint32_t e2m1_div2_even(float v0, float v1, float d, float rinv) {
-  const float x0 = v0 * rinv, x1 = v1 * rinv;
-  const uint32_t hi = gb_cvt_e2m1x2(fmaf(x0, kGbNear, x0), fmaf(x1, kGbNear, x1));
-  const uint32_t lo = gb_cvt_e2m1x2(fmaf(x0, -kGbNear, x0), fmaf(x1, -kGbNear, x1));
-  return hi == lo ? hi : gb_cvt_e2m1x2(__fdiv_rn(v0, d), __fdiv_rn(v1, d));
-}
-
 constexpr int kQuantMaxGroups = 4;
 
 template <int kG>
@@ -370,11 +360,12 @@ nvfp4_quantize_rows_kernel(const uint4* __restrict__ x, uint2* __restrict__ pack
   const float gs = live ? __fdiv_rn(__fmul_rn(range, 6.0f), amax) : 1.0f;
   if (threadIdx.x == 0) a_scale[row] = live ? __fdiv_rn(1.0f, gs) : 0.0f;
   const bool reload = groups > kG * (int)blockDim.x;
-  for (int g0 = threadIdx.x; g0 < groups; g0 += kG * blockDim.x) {
+  for (int base = 0; base < groups; base += kG * blockDim.x) {        // whole warps stay together: the shuffles below
 #pragma unroll
     for (int j = 0; j < kG; ++j) {
-      const int g = g0 + j * blockDim.x;
-      if (g >= groups) break;
+      const int g = base + threadIdx.x + j * blockDim.x;
+      const unsigned here = __ballot_sync(0xffffffffu, g < groups);
+      if (g >= groups) continue;
       if (reload) {
         const uint4 a = xr[2 * g], b = xr[2 * g + 1];
         w[j][0] = a.x; w[j][1] = a.y; w[j][2] = a.z; w[j][3] = a.w;
@@ -391,13 +382,17 @@ nvfp4_quantize_rows_kernel(const uint4* __restrict__ x, uint2* __restrict__ pack
       const float sf = live ? fminf(__fdiv_rn(gmax, 6.0f), 448.0f) : 0.0f;
       const uint32_t sf_byte = gb_f32_to_e4m3(sf);
       const float sf_f = gb_e4m3_to_f32(sf_byte);
-      sfa[sf_offset(g)] = (uint8_t)sf_byte;
+      // four neighbouring groups share a word of the scale-factor plane
+      const uint32_t b1 = __shfl_down_sync(here, sf_byte, 1), b2 = __shfl_down_sync(here, sf_byte, 2);
+      const uint32_t b3 = __shfl_down_sync(here, sf_byte, 3);
+      if (groups % 4 != 0) sfa[sf_offset(g)] = (uint8_t)sf_byte;
+      else if ((g & 3) == 0) *reinterpret_cast<uint32_t*>(sfa + sf_offset(g)) = sf_byte | (b1 << 8) | (b2 << 16) | (b3 << 24);
       const float rinv = sf_f != 0.0f ? __frcp_rn(sf_f) : 0.0f;
       uint32_t lo = 0, hi = 0;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         uint32_t byte;
-        if (sf_f != 0.0f) byte = e2m1_div2_even(xs[2 * i], xs[2 * i + 1], sf_f, rinv);
+        if (sf_f != 0.0f) byte = gb_cvt_e2m1x2(gb_div(xs[2 * i], sf_f, rinv), gb_div(xs[2 * i + 1], sf_f, rinv));
         else byte = ((__float_as_uint(xs[2 * i]) >> 31) << 3) | ((__float_as_uint(xs[2 * i + 1]) >> 31) << 7);
         if (i < 4) lo |= byte << (8 * i);
         else hi |= byte << (8 * (i - 4));
