@@ -20,13 +20,14 @@ REQUIRED_SYMBOLS = (
     "gb_abi_version", "gb_last_error", "gb_prepare", "gb_device_status", "gb_gemv_row_batch_max",
     "gb_fp8_act_qdq", "gb_fp4_act_qdq",
     "gb_expand_fp8", "gb_expand_fp4_bf16", "gb_expand_fp4_nvfp4",
-    "gb_gemv_workspace_bytes", "gb_gemv", "gb_gemv_static",
+    "gb_gemv_workspace_bytes", "gb_gemv", "gb_gemv_static", "gb_gemv_hinted", "gb_scales_e4m3",
     "gb_gemv_tab_slots_bytes", "gb_gemv_tab_arm", "gb_gemv_tab", "gb_device_status_reset", "gb_set_wait_limit_ms",
     "gb_set_row_routes", "gb_nvfp4_sf_bytes", "gb_nvfp4_quantize_rows", "gb_gemm_fp4",
     "gb_moe_route", "gb_moe_route_ws", "gb_moe_route_workspace_bytes", "gb_moe_gemv_workspace_bytes", "gb_moe_gemv", "gb_moe_combine",
     "gb_moe_gemv_pairs_workspace_bytes", "gb_moe_gemv_pairs",
     "gb_moe_mlp_pairs_workspace_bytes", "gb_moe_mlp_pairs",
     "gb_expand_fp8_bf16", "gb_fp8_quantize_rows", "gb_gemm_tn", "gb_gemm_tn_grouped", "gb_moe_gather_rows", "gb_moe_swiglu_rows", "gb_moe_gemv_sorted",
+    "gb_moe_route_inv", "gb_moe_fp4_pass_rows", "gb_moe_fp4_operand_bytes", "gb_moe_fp4_rows", "gb_moe_fp4_swiglu_rows", "gb_moe_gemv_fp4",
     "gb_peer_alloc", "gb_peer_free", "gb_peer_export", "gb_peer_open", "gb_peer_close",
     "gb_peer_allgather", "gb_peer_allgather_ll", "gb_peer_barrier", "gb_launch_count", "gb_gemv_allgather", "gb_moe_combine_peer",
 )

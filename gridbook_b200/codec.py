@@ -140,6 +140,20 @@ def pad_qweight(qw: torch.Tensor) -> torch.Tensor:
     return torch.nn.functional.pad(qw.contiguous(), (0, PAD_BYTES), value=0).contiguous()
 
 
+# Two-tier product widths the tensor-core decode kernels take, with their superblocks in slots of a
+# multiple of sixteen bytes.
+_SLOTTED_WIDTHS = (12, 16, 20, 24)
+
+
+def resident_slot(fmt) -> int | None:
+    """Bytes of the slot a superblock of this format is kept in while resident, or None to keep the
+    shipped layout."""
+    if not (fmt.is_fp4 and fmt.mode == "product" and fmt.n_sub == 2 and fmt.scale_coding == "v2"
+            and fmt.k in _SLOTTED_WIDTHS and fmt.sb_pad == 0):
+        return None
+    return -(-fmt.type_size // 16) * 16
+
+
 def pad_superblocks(qw: torch.Tensor, type_size: int, stride: int) -> torch.Tensor:
     """Packed rows [..., n_sb * type_size] with every superblock moved to a `stride`-byte slot (zero
     filled): the resident layout the tensor-core decode kernel needs for superblocks whose size is

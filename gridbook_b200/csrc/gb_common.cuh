@@ -68,6 +68,7 @@ int gb_prepare_dot();
 int gb_prepare_umma();
 int gb_prepare_tab();
 int gb_prepare_gemm_fp4();
+int gb_prepare_gemv_fp4();
 // Longest a device-side wait may spin before it gives up and raises the status word
 // (two seconds unless gb_set_wait_limit_ms changed it).
 unsigned long long gb_wait_limit_ns();
@@ -84,6 +85,14 @@ int gb_gemv_umma_max_rows(const gb_weight* w);
 bool gb_gemv_umma_is_literal(const gb_weight* w);
 int gb_tensor_map_bytes_2d(void* map_out, const void* base, uint64_t inner_bytes, uint64_t rows,
                            uint64_t pitch_bytes, uint32_t box_bytes, uint32_t box_rows);
+// Decode batches of the fp4 grid on the block-scaled FP4 tensor cores (gb_gemv_fp4.cu): the literal format
+// and, where the caller knows that every two-tier scale is an exact E4M3 value, the product formats
+// k = 12, 16, 20, 24 in 16-byte aligned superblock slots.  `role_rows`: row counts of the parts of a
+// fused matrix that carry their own codebook (n_roles <= 1: one codebook).
+bool gb_gemv_fp4_applies(const gb_weight* w, bool scales_e4m3);
+int64_t gb_gemv_fp4_workspace_bytes(int64_t M, int64_t K);
+int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, int n_roles, const int64_t* role_rows,
+                int scale_rule, void* y, void* workspace, int64_t workspace_bytes, void* stream);
 // M = 1 literal-format linear by per-column inner-product tables (gb_gemv_dot.cu); GB_EUNSUPPORTED when
 // the shape or layout is not its own, and the caller falls back to the MMA kernel.
 int gb_gemv_dot_rows(const void* x, int64_t M, const gb_weight* w, int act, int scale_rule, void* y, void* workspace,

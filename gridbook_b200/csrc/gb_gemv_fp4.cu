@@ -1,0 +1,1246 @@
+// Decode-batch linear of the fp4 grid on the block-scaled FP4 tensor cores, the decode contract kept:
+// y[M, N] = bucket(x)[M, K] . W^T for 1 <= M <= 64 rows per pass, dense and per expert.
+//
+// A weight of the fp4 grid IS E2M1 x (E4M3 group scale), so the packed rows only have to be turned
+// into the MMA's own operand format: one 32-bit word of nibbles per codeword, one scale byte per group
+// (the kernel of gb_gemv_umma.cu multiplies every weight out to bf16 first: four times the
+// operand bytes, sixteen MMAs per superblock instead of four).  What does not fit the format is the
+// ACTIVATION: the contract's value is bf16(q * s) with q on the E2M1 grid and a full fp32 group scale
+// s.  It is split exactly into three E2M1 x UE4M3 terms, i.e. three columns of the N side per row:
+//   * the eight magnitudes of q share two significands: m1 = bf16(s) (q = 0.5, 1, 2, 4) and
+//     bf16(1.5 s) (q = 1.5, 3, 6), each times a power of two;
+//   * hi  : q x (m1 rounded down to four significant bits),
+//   * lo  : q x (the other four bits of m1), its own power of two on the column,
+//   * dlt : bf16(1.5 s) - 1.5 m1 is n half-ulps of m1 with |n| <= 3, so for q = 1.5, 3, 6 the missing
+//           part is (n q / 3) half-ulps: again an E2M1 value times a power of two.
+// Every term is normalised per row by a power of two that puts the row's largest m1 into [128, 256).
+// UE4M3 reaches down to 2^-9, so the split is exact for groups within 2^13 of the row's largest; a
+// smaller group loses less than 2^-21 of the row's largest scale, below the fp32 sum's own rounding.
+//
+// Up to sixteen rows the three terms are columns of one MMA (N <= 48).  Past them two MMAs share the
+// codes of q: N = 2 R with the scale factors [hi | dlt] over the code rows [q | e], N = R with lo over
+// [q], so a row costs two code rows of shared memory and L2 traffic instead of three.
+//
+// Work split as in gb_gemv_umma.cu: a CTA owns 128 weight rows (the M side) and a K slice; one warp
+// streams the packed rows (tiled TMA), one the operand of the activations (one bulk copy per superblock:
+// the rows kernel below writes it swizzled, scale factors in front), sixteen warps decode.  A UNIT is
+// one superblock of K (256 weights): unit u is decoded by warpgroup u mod 4 into operand buffer u mod 4
+// of TENSOR MEMORY (32 columns of nibbles, 16 of scale factors) and multiplied by four MMAs of K = 64
+// (or eight); the issuing thread copies the activations' scale factors to tensor memory itself.
+// Bound by the decoders' instructions and the latency of the hand-overs between the roles
+// (a tcgen05.mma takes 72 clocks of its issuer whatever its N up to 128, a commit reaches its waiter
+// after about 250), then by shared-memory lookups (4 bytes per codeword from 32 copies: no conflicts).
+//
+// A layer with few 128-row tiles is sliced along K over a thread-block cluster: every CTA of the
+// cluster pushes its fp32 sums into the shared memory of the CTA that owns the activation row, which
+// adds them in slice order - no partial sums in HBM and no second launch.
+#include "gb_common.cuh"
+
+#include <cuda.h>
+#include <mutex>
+
+namespace {
+
+constexpr int kBM = 128;
+constexpr int kDecWarps = 16;
+constexpr int kCtlWarps = 6;                              // packed rows, activations, up to four MMA issuers
+constexpr int kThreads = 32 * (kCtlWarps + kDecWarps);
+constexpr int kMaxRows = 64;                              // activation rows per pass (three columns each)
+constexpr int kMaxRaw = 4, kMaxX = 8;
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kDynBase = 0x400u;                     // dynamic shared memory starts here (checked); in a
+                                                          // cluster the CTA's rank sits in the address's top byte
+constexpr uint32_t kSmemMax = 227 * 1024;
+constexpr uint32_t kSmemEnd = kDynBase + kSmemMax;
+constexpr uint32_t kLut = 0x10000u;                       // shared-window address of the lookup tables
+constexpr int kMaxRoles = GB_MAX_ROLES;
+constexpr int kMaxSlices = 8;
+
+enum { kLit = 8 };                                        // other formats: the product format's k
+
+// Packed superblocks as they sit in memory and the lookup tables of a format.
+template <int F> struct Fmt {                             // two-tier product format, k = F
+  static constexpr int kW0 = (F + 1) / 2, kW1 = F / 2;    // sub-index widths
+  static constexpr int kSb = (4 * F + 9 + 15) / 16 * 16;  // slot of a superblock
+  static constexpr int kSbPerStage = F > 16 ? 1 : 2;       // the tables of the wide formats leave less room
+  static constexpr int kEntries = 1 << kW0;
+  static constexpr int kCopies = kEntries <= 1024 ? 32 : 32 * 1024 / kEntries;
+  static constexpr uint32_t kStride = kCopies * 4;        // bytes between entries: both sub-tables in one word
+  static constexpr uint32_t kLutBytes = kEntries * kStride;
+  static constexpr uint32_t kScaleTab = 4096;             // E4M3 byte of every (super, sub) pair
+};
+template <> struct Fmt<kLit> {
+  static constexpr int kSb = 48, kSbPerStage = 2;
+  static constexpr uint32_t kStride = 256;                // a code dropped into byte 1 is the entry's offset
+  static constexpr uint32_t kLutBytes = 256 * 256, kScaleTab = 0;
+};
+template <int F> struct Geo {
+  static constexpr int kPitch0 = Fmt<F>::kSbPerStage * Fmt<F>::kSb;
+  static constexpr int kPitch = kPitch0 + ((kPitch0 / 16) % 2 ? 32 : 16);   // an odd number of 16-byte units
+  static constexpr int kBoxBytes = kBM * kPitch;
+  static_assert(kPitch <= 256 && (kPitch / 16) % 2 == 1, "row pitch");
+};
+
+struct Role { int row0, rows, tile0; int64_t cb; };        // rows that share a codebook; first tile; element offset
+
+struct Fp4Params {
+  int64_t N, K;
+  int M;                     // dense: activation rows
+  int n_sb, units;           // superblocks per row / per K slice (the last slice may have fewer)
+  int slices;                // = cluster size along y
+  int pass_rows;             // most rows per pass (dense: M)
+  int x_stages, raw_stages;  // ring depths: 4 or 8, 2 to 4
+  uint32_t x_off, raw_off[kMaxRaw], misc_off, red_off;
+  const uint8_t* xop;        // activation operand: [tile][superblock][scale factors | codes]
+  int64_t x_unit;            // bytes of one superblock of it
+  const float* x_scale;      // [tile][pass_rows] power of two of every row
+  const void* codebook;      // bf16 flat
+  const float* compose;
+  float global_scale;
+  uint16_t* y;
+  int* status;
+  int n_roles, n_tiles;
+  Role role[kMaxRoles];
+  const int32_t* seg;        // grouped: [E + 1]
+  const int32_t* row_map;
+  int tiles_n;
+};
+
+// Columns.  Narrow (up to 16 rows per pass): column t * R + m of term t of row m, one MMA of N = 3 R
+// rounded up to 16.  Wide: R code rows of q and R of the correction, scale factors [hi | dlt] and [lo].
+// R = rows rounded up to 8 (narrow) or 16.
+constexpr int kNarrowRows = 16;
+__host__ __device__ constexpr bool is_wide(int pass_rows) { return pass_rows > kNarrowRows; }
+__host__ __device__ constexpr int term_rows(bool wide, int rows) { return wide ? (rows + 15) / 16 * 16 : (rows + 7) / 8 * 8; }
+__host__ __device__ constexpr int mma_cols(bool wide, int rows) {
+  return wide ? 2 * term_rows(true, rows) : (3 * term_rows(false, rows) + 15) / 16 * 16;
+}
+// Bytes in front of the codes of a unit: scale-factor atoms of 128 columns (wide: two sets).
+__host__ __device__ constexpr int sf_bytes(bool wide) { return wide ? 4096 : 2048; }
+__host__ __device__ constexpr int unit_bytes(bool wide, int rows) { return sf_bytes(wide) + mma_cols(wide, rows) * 128; }
+
+// ---- PTX ---------------------------------------------------------------------------------------
+GB_DEVINL void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+GB_DEVINL void mbar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+GB_DEVINL void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+GB_DEVINL bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+// Acquire at cluster scope: the arrivals come from other CTAs of the cluster.
+GB_DEVINL bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+// A bounded wait that remembers a timeout for the rest of the CTA: later waits return at once.  The
+// spin is kept out of line: a dozen inlined copies crowd the instruction cache.
+template <bool kCluster>
+__device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  uint64_t t0 = 0;
+  for (uint32_t spin = 0; !*abort_flag; ++spin) {
+    if (kCluster ? mbar_try_cluster(bar, parity) : mbar_try(bar, parity)) return;
+    if ((spin & 255u) == 255u) {
+      const uint64_t now = gb_globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > 2000000000ull) { *abort_flag = 1; atomicExch(status, code); }
+    }
+  }
+}
+template <bool kCluster = false>
+GB_DEVINL void wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (!(kCluster ? mbar_try_cluster(bar, parity) : mbar_try(bar, parity))) wait_slow<kCluster>(bar, parity, abort_flag, status, code);
+}
+GB_DEVINL void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar) : "memory");
+}
+GB_DEVINL void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+GB_DEVINL uint64_t desc_sw128(uint32_t addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)(1024u >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+// D[tmem] (+)= (A SFA)[tmem] . (B SFB)[smem]: A holds 128 rows (lanes) x 64 E2M1 in 8 columns.
+GB_DEVINL void umma_fp4_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb, bool acc) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%1], %2, %3, [%5], [%6], p;\n}\n"
+      ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)acc), "r"(sfa), "r"(sfb) : "memory");
+}
+// 512 bytes of scale factors (128 columns x 4 groups) from shared to tensor memory, into all four lane
+// quarters; in order with the MMAs the same thread issues.
+GB_DEVINL void copy_sf(uint32_t taddr, uint32_t smem_addr) {
+  uint64_t d = (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)(128u >> 4) << 32;                        // eight-row groups of 16-byte rows, no swizzle
+  d |= (uint64_t)1 << 46;
+  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(d) : "memory");
+}
+GB_DEVINL void umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+GB_DEVINL void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+GB_DEVINL void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
+}
+GB_DEVINL void tmem_ld4(uint32_t taddr, uint32_t (&v)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr));
+}
+GB_DEVINL void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+GB_DEVINL uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+GB_DEVINL void sts128(uint32_t a, uint4 v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+template <uint32_t kImm>
+GB_DEVINL uint32_t lds_imm(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(kImm));
+  return v;
+}
+template <uint32_t kImm>
+GB_DEVINL uint32_t lds_imm16(uint32_t a) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1+%2];" : "=h"(v) : "r"(a), "n"(kImm));
+  return v;
+}
+
+// Four E2M1 nibbles of four bf16 codebook values.
+GB_DEVINL uint32_t nib4(uint2 w) {
+  uint32_t r = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float v = gb_bf16_bits_to_f32(((j < 2 ? w.x : w.y) >> (16 * (j & 1))) & 0xFFFFu), m = fabsf(v);
+    const uint32_t c = m < 2.0f ? (uint32_t)(m * 2.0f) : (m < 4.0f ? (uint32_t)m + 2u : (m < 6.0f ? 6u : 7u));
+    r |= (c | (v < 0.0f ? 8u : 0u)) << (4 * j);
+  }
+  return r;
+}
+
+// Lookup tables of one codebook, built by the 512 decoder threads.
+template <int F>
+GB_DEVINL void build_lut(const uint16_t* cb, int d, uint32_t lut) {
+  if constexpr (F == kLit) {
+    const int e = d & 255, half = d >> 8;
+    const uint4 q = *reinterpret_cast<const uint4*>(cb + e * 8);
+    const uint32_t w = nib4(make_uint2(q.x, q.y)) | (nib4(make_uint2(q.z, q.w)) << 16);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sts128(lut + (uint32_t)e * 256u + (uint32_t)(half * 4 + j) * 16u, make_uint4(w, w, w, w));
+  } else {
+    using T = Fmt<F>;
+    const uint2* t0 = reinterpret_cast<const uint2*>(cb);
+    const uint2* t1 = t0 + T::kEntries;
+    for (int e = d; e < T::kEntries; e += 32 * kDecWarps) {
+      uint32_t w = nib4(t0[e]);
+      if (e < (1 << T::kW1)) w |= nib4(t1[e]) << 16;
+#pragma unroll
+      for (int j = 0; j < T::kCopies / 4; ++j) sts128(lut + (uint32_t)e * T::kStride + (uint32_t)j * 16u, make_uint4(w, w, w, w));
+    }
+  }
+}
+
+// Byte offset of the sub-index at bits [bit, bit + width) of the code words, times the entry stride.
+template <int F, int kWidth>
+GB_DEVINL uint32_t entry_offset(const uint32_t* w, int bit, uint32_t lane4) {
+  constexpr int kShift = F == kLit ? 8 : (Fmt<F>::kStride == 128 ? 7 : Fmt<F>::kStride == 64 ? 6 : 5);
+  constexpr uint32_t kMask = ((1u << kWidth) - 1u) << kShift;
+  const int i = bit >> 5, s = bit & 31;
+  uint32_t x;
+  if (s + kWidth <= 32) x = s >= kShift ? w[i] >> (s - kShift) : w[i] << (kShift - s);
+  else x = s >= kShift ? __funnelshift_r(w[i], w[i + 1], s - kShift) : 0u;
+  return (x & kMask) | lane4;
+}
+
+// Eight weights of codeword c as nibbles.
+template <int F>
+GB_DEVINL uint32_t codeword(const uint32_t* w, int c, uint32_t lane4) {
+  if constexpr (F == kLit) {
+    // [lane4's byte 0, code, lane4's bytes 2 and 3]: lane offset, entry, the window's rank byte
+    const uint32_t a = c % 4 == 0 ? __byte_perm(w[c / 4], lane4, 0x7604) : c % 4 == 1 ? __byte_perm(w[c / 4], lane4, 0x7614)
+                     : c % 4 == 2 ? __byte_perm(w[c / 4], lane4, 0x7624) : __byte_perm(w[c / 4], lane4, 0x7634);
+    return lds_imm<kLut>(a);
+  } else {
+    using T = Fmt<F>;
+    const uint32_t a0 = entry_offset<F, T::kW0>(w, c * F, lane4), a1 = entry_offset<F, T::kW1>(w, c * F + T::kW0, lane4);
+    return lds_imm16<kLut>(a0) | (lds_imm16<kLut + 2>(a1) << 16);
+  }
+}
+
+// Two-tier scales: four E4M3 bytes of four nibble codes (low 16 bits of c) from the sixteen bytes t.
+GB_DEVINL uint32_t four_scales(uint4 t, uint32_t c) {
+  const uint32_t sel = c & 0x7777u;
+  const uint32_t lo = __byte_perm(t.x, t.y, sel), hi = __byte_perm(t.z, t.w, sel);
+  uint32_t m;                                              // 0xFF where the code is 8..15 (sign replication), else 0x80
+  asm("prmt.b32 %0, %1, %1, %2;" : "=r"(m) : "r"(0x80808080u), "r"(c & 0x8888u));
+  return lo ^ ((lo ^ hi) & m & 0x7F7F7F7Fu);
+}
+
+template <bool kGrouped, int F>
+__global__ void __launch_bounds__(kThreads, 1)
+fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Fp4Params p) {
+  using T = Fmt<F>;
+  using G = Geo<F>;
+  extern __shared__ uint8_t smem_raw[];
+  // barriers and small state
+  const uint32_t win = gb_smem_u32(smem_raw) & 0xFF000000u;
+  const uint32_t misc = p.misc_off | win;
+  const uint32_t raw_full = misc, raw_empty = misc + 8 * kMaxRaw;
+  // per unit slot: activations landed / operand complete (decoded, and narrow: landed) / multiplied
+  const uint32_t x_full = misc + 64, full = x_full + 8 * kMaxX, done = full + 8 * kMaxX;
+  const uint32_t acc_full = done + 8 * kMaxX, acc_empty = acc_full + 8, red_full = acc_full + 16;
+  const uint32_t slot_addr = acc_full + 24;
+  uint8_t* misc_ptr = smem_raw + (p.misc_off - kDynBase);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(misc_ptr + (slot_addr - misc));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(misc_ptr + (slot_addr - misc) + 4);
+  const uint32_t sfa_stage = misc + 512;                   // two-tier: scale bytes of a unit, two buffers of 2 KiB per warpgroup
+  const uint32_t scale_tab = sfa_stage + (F == kLit ? 0u : 16384u);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slice = blockIdx.y;
+  const int sb_begin = slice * p.units;
+  const int units = min(p.units, p.n_sb - sb_begin);
+  // Layout of tensor memory.  Narrow: four accumulators of 64 columns, one per warpgroup and issuer; wide:
+  // [hi | dlt] in columns [0, 128), [lo] in [128, 192), one issuer each.  Then the four operand
+  // buffers: nibbles (32), weight scale factors (16), activation scale factors (16 per set).
+  const bool wide = is_wide(p.pass_rows);
+  const int n_iss = wide ? 2 : 4;
+  const uint32_t acc_stride = wide ? 128u : 64u;
+  const uint32_t buf_col0 = wide ? 192u : 256u, buf_stride = wide ? 80u : 64u;
+  const int sfx = sf_bytes(wide);
+  const int x_mask = p.x_stages - 1, x_log = p.x_stages == 8 ? 3 : 2;
+  const uint32_t x_ring = p.x_off | win, x_stage = (uint32_t)p.x_unit;
+
+  gb_pdl_launch_dependents();
+  if ((gb_smem_u32(smem_raw) ^ win) != kDynBase) {                 // the addresses above assume it
+    if (threadIdx.x == 0) atomicExch(p.status, 41);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kMaxRaw; ++s) {
+      mbar_init(raw_full + 8 * s, 1);
+      mbar_init(raw_empty + 8 * s, kDecWarps);
+    }
+    for (int s = 0; s < kMaxX; ++s) {
+      mbar_init(x_full + 8 * s, 1);
+      mbar_init(full + 8 * s, wide ? 4 : 5);
+      mbar_init(done + 8 * s, wide ? 2 : 1);
+    }
+    mbar_init(acc_full, (uint32_t)n_iss);
+    mbar_init(acc_empty, kDecWarps);
+    mbar_init(red_full, (uint32_t)(p.slices * kDecWarps));
+    *abort_flag = 0;
+    gb_fence_barrier_init();
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_addr), "r"(kTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (p.slices > 1) {
+    uint32_t size, rank;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    if (threadIdx.x == 0 && ((int)size != p.slices || (int)rank != slice)) {
+      *abort_flag = 1;
+      atomicExch(p.status, 51);
+    }
+    cluster_sync();                                        // peers write into this CTA's shared memory later: all must have started
+  }
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (kGrouped) gb_pdl_wait();                             // the segment offsets come from an earlier launch
+  struct Tile { int n0, n_end, w_row0, lo, cnt, n_pass, x_tile, role; };
+  auto tile_at = [&](int t) {
+    Tile R;
+    if (kGrouped) {
+      const int e = t / p.tiles_n;
+      R.n0 = (t - e * p.tiles_n) * kBM;
+      R.n_end = (int)p.N;
+      R.w_row0 = e * (int)p.N + R.n0;
+      R.lo = p.seg[e];
+      R.cnt = p.seg[e + 1] - R.lo;
+      R.n_pass = R.cnt > 0 ? (R.cnt + p.pass_rows - 1) / p.pass_rows : 0;
+      R.x_tile = R.lo / p.pass_rows + e;                   // tiles of different (expert, pass) never coincide
+      R.role = 0;
+    } else {
+      int r = 0;
+      while (r + 1 < p.n_roles && t >= p.role[r + 1].tile0) ++r;
+      R.n0 = p.role[r].row0 + (t - p.role[r].tile0) * kBM;
+      R.n_end = p.role[r].row0 + p.role[r].rows;
+      R.w_row0 = R.n0;
+      R.lo = 0; R.cnt = p.M; R.n_pass = 1; R.x_tile = 0; R.role = r;
+    }
+    return R;
+  };
+
+  if (warp == 0) {
+    // ------------------------- packed weight rows -------------------------
+    if (lane == 0) {
+      int rs = 0;
+      uint32_t ph = 1;
+      for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
+        const Tile R = tile_at(t);
+        for (int pass = 0; pass < R.n_pass; ++pass)
+          for (int u = 0; u < units; u += T::kSbPerStage) {
+            wait(raw_empty + 8 * rs, ph, abort_flag, p.status, 42);
+            mbar_expect(raw_full + 8 * rs, G::kBoxBytes);
+            tma_load_2d(p.raw_off[rs] | win, &map_w, (sb_begin + u) * T::kSb, R.w_row0, raw_full + 8 * rs);
+            if (++rs == p.raw_stages) { rs = 0; ph ^= 1; }
+          }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------- activation operand --------------------------
+    if (lane == 0) {
+      gb_pdl_wait();
+      const uint32_t land = wide ? x_full : full;
+      int g = 0;                                           // units since the start, over all tiles and passes
+      for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
+        const Tile R = tile_at(t);
+        for (int pass = 0; pass < R.n_pass; ++pass) {
+          const int rows = min(p.pass_rows, R.cnt - pass * p.pass_rows);
+          const uint32_t bytes = (uint32_t)unit_bytes(wide, rows);
+          const uint8_t* src = p.xop + ((int64_t)(R.x_tile + pass) * p.n_sb + sb_begin) * p.x_unit;
+          for (int u = 0; u < units; ++u, ++g, src += p.x_unit) {
+            const int s = g & x_mask;
+            wait(done + 8 * s, ((uint32_t)(g >> x_log) & 1u) ^ 1u, abort_flag, p.status, 43);
+            mbar_expect(land + 8 * s, bytes);
+            bulk_load(x_ring + (uint32_t)s * x_stage, src, bytes, land + 8 * s);
+          }
+        }
+      }
+    }
+  } else if (warp < kCtlWarps) {
+    // ------------------------- MMA issuers ---------------------------------
+    // Narrow: issuer i takes the units of warpgroup i into accumulator i.  Wide: issuer 0 multiplies every
+    // unit with [hi | dlt], issuer 1 with [lo].
+    const int i = warp - 2;
+    if (lane == 0 && i < n_iss) {
+      const uint32_t acc = tmem_base + (uint32_t)i * acc_stride;
+      const uint32_t sf_col = 48u + (wide ? (uint32_t)i * 16u : 0u);
+      const int u_first = wide ? 0 : i, u_step = wide ? 1 : 4;
+      const uint64_t db0 = desc_sw128(x_ring + (uint32_t)sfx);
+      int g0 = 0, item = 0;                                // units / (tile, pass) items since the start
+      for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
+        const Tile R = tile_at(t);
+        for (int pass = 0; pass < R.n_pass; ++pass, ++item, g0 += units) {
+          const int rows = min(p.pass_rows, R.cnt - pass * p.pass_rows);
+          const int n = wide && i == 1 ? term_rows(true, rows) : mma_cols(wide, rows);
+          // E2M1 x E2M1, UE4M3 scale factors, both K-major, fp32 accumulate; N >> 3, M >> 4
+          const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+          if (item > 0) {
+            wait(acc_empty, (item - 1) & 1, abort_flag, p.status, 44);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
+          for (int u = u_first; u < units; u += u_step) {
+            const int g = g0 + u, s = g & x_mask;
+            const uint32_t a = tmem_base + buf_col0 + (uint32_t)(u & 3) * buf_stride, off = (uint32_t)s * x_stage;
+            const uint64_t db = db0 + (uint64_t)(off >> 4);
+            wait(full + 8 * s, (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 45);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (!wide) {
+              // The activations' scale factors, in order in front of the MMAs that read them; what they
+              // overwrite was read by this thread's MMAs of four units ago, which have completed (the
+              // decoders waited for them).
+#pragma unroll
+              for (int k = 0; k < 4; ++k) copy_sf(a + 48u + 4u * k, x_ring + off + 512u * k);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              umma_fp4_ts(acc, a + 8u * k, db + (uint64_t)(2 * k), idesc, a + 32u + 4u * k, a + sf_col + 4u * k, u > u_first || k > 0);
+            umma_commit(done + 8 * s);
+          }
+          umma_commit(acc_full);
+        }
+      }
+    }
+  } else {
+    // ------------------------- decoders -------------------------------------
+    const int d = threadIdx.x - 32 * kCtlWarps;              // 0 .. 511
+    const int quarter = warp & 3, wg = (warp - kCtlWarps) >> 2;
+    const int row = quarter * 32 + lane;                     // weight row of the tile = tensor-memory lane
+    const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    const uint32_t buf = lane_base + buf_col0 + (uint32_t)wg * buf_stride;
+    const uint32_t lane4 = win | (F == kLit ? (uint32_t)lane * 4u : (uint32_t)(lane & ((int)(T::kStride / 4) - 1)) * 4u);
+    int have_role = -1;
+    if constexpr (F != kLit) {
+      for (int i = d; i < 4096; i += 32 * kDecWarps) {
+        const uint32_t b = gb_f32_to_e4m3(fminf(__ldg(p.compose + i), 448.0f));
+        asm volatile("st.shared.u8 [%0], %1;" ::"r"(scale_tab + (uint32_t)i), "r"(b) : "memory");
+      }
+    }
+    bool waited = false;
+    int rs = 0, item = 0, g0 = 0;
+    uint32_t rph = 0, flip = 0;
+    for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
+      const Tile R = tile_at(t);
+      if (R.n_pass == 0) continue;
+      if (R.role != have_role) {                             // the CTA's rows change codebook
+        if (have_role >= 0) asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
+        build_lut<F>(reinterpret_cast<const uint16_t*>(p.codebook) + p.role[R.role].cb, d, kLut | win);
+        have_role = R.role;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
+      }
+      if (!waited) { gb_pdl_wait(); waited = true; }         // y may still be read by the launch ahead
+      for (int pass = 0; pass < R.n_pass; ++pass, ++item, g0 += units) {
+        const int rows = min(p.pass_rows, R.cnt - pass * p.pass_rows);
+        const float* xsc = p.x_scale + (int64_t)(R.x_tile + pass) * p.pass_rows;
+        const float xs0 = lane < rows ? xsc[lane] : 0.0f, xs1 = lane + 32 < rows ? xsc[lane + 32] : 0.0f;
+        for (int u0 = 0; u0 < units; u0 += T::kSbPerStage) {
+          wait(raw_full + 8 * rs, rph, abort_flag, p.status, 47);
+          const int i = (wg - u0) & 3;                       // this warpgroup's superblock of the stage, if any
+          if (i < T::kSbPerStage && u0 + i < units) {
+            const uint32_t stage = p.raw_off[rs] | win;
+            const uint32_t rp = stage + (uint32_t)row * G::kPitch + (uint32_t)(i * T::kSb);
+            uint32_t v[32], sfa[16];
+            if constexpr (F == kLit) {
+              const uint4 c0 = lds128(rp), c1 = lds128(rp + 16);
+              const uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+              const uint32_t sg = stage + (uint32_t)lane * G::kPitch + (uint32_t)(i * T::kSb) + 32u;
+              uint32_t any = 0;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {                  // scale bytes of rows lane, lane + 32, lane + 64, lane + 96
+                const uint4 s = lds128(sg + (uint32_t)(j * 32) * G::kPitch);
+                sfa[j] = s.x; sfa[4 + j] = s.y; sfa[8 + j] = s.z; sfa[12 + j] = s.w;
+                any |= s.x | s.y | s.z | s.w;
+              }
+#pragma unroll
+              for (int c = 0; c < 32; ++c) v[c] = codeword<F>(cw, c, lane4);
+              if (__builtin_expect(any & 0x80808080u, 0)) {  // scale factors carry no sign: it moves into the nibbles
+                const uint4 own = lds128(rp + 32);
+                const uint32_t os[4] = {own.x, own.y, own.z, own.w};
+#pragma unroll
+                for (int g = 0; g < 16; ++g) {
+                  const uint32_t neg = (os[g >> 2] >> (8 * (g & 3))) & 0x80u ? 0x88888888u : 0u;
+                  v[2 * g] ^= neg;
+                  v[2 * g + 1] ^= neg;
+                  sfa[g] &= 0x7F7F7F7Fu;
+                }
+              }
+            } else {
+              uint32_t w[T::kSb / 4];
+#pragma unroll
+              for (int q = 0; q < T::kSb / 16; ++q) {
+                const uint4 x = lds128(rp + 16u * q);
+                w[4 * q] = x.x; w[4 * q + 1] = x.y; w[4 * q + 2] = x.z; w[4 * q + 3] = x.w;
+              }
+              // the super byte sits right behind the 4k index bytes, then sixteen nibbles
+              const uint4 tb = lds128(scale_tab + (w[F] & 0xFFu) * 16u);
+              const uint32_t n0 = __funnelshift_r(w[F], w[F + 1], 8), n1 = __funnelshift_r(w[F + 1], w[F + 2], 8);
+              // two buffers: a warp that writes the next unit's bytes has passed this unit's barrier,
+              // which no warp reaches before it has read the unit before
+              const uint32_t st = sfa_stage + (uint32_t)(wg * 4096) + flip * 2048u;
+              flip ^= 1u;
+              sts128(st + (uint32_t)(row * 16),
+                     make_uint4(four_scales(tb, n0), four_scales(tb, n0 >> 16), four_scales(tb, n1), four_scales(tb, n1 >> 16)));
+#pragma unroll
+              for (int c = 0; c < 32; ++c) v[c] = codeword<F>(w, c, lane4);
+              asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory");   // the four warps of this warpgroup
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint4 s = lds128(st + (uint32_t)((lane + 32 * j) * 16));
+                sfa[j] = s.x; sfa[4 + j] = s.y; sfa[8 + j] = s.z; sfa[12 + j] = s.w;
+              }
+            }
+            // The buffer's last unit has been multiplied (at the start of an item all have).  The slot's
+            // next completion is a later unit of this warpgroup, so it cannot run ahead of this wait.
+            const int u = u0 + i, g = g0 + u;
+            if (u >= 4) wait(done + 8 * ((g - 4) & x_mask), (uint32_t)((g - 4) >> x_log) & 1u, abort_flag, p.status, 48);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            tmem_st16(buf, *reinterpret_cast<const uint32_t(*)[16]>(&v[0]));
+            tmem_st16(buf + 16u, *reinterpret_cast<const uint32_t(*)[16]>(&v[16]));
+            tmem_st16(buf + 32u, sfa);
+            if (wide) {
+              // the activations' two sets of scale factors (the two issuers have no time for the copies)
+              wait(x_full + 8 * (g & x_mask), (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 46);
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  const uint4 s = lds128(x_ring + (uint32_t)(g & x_mask) * x_stage + (uint32_t)(q * 2048 + k * 512 + lane * 16));
+                  sfa[4 * k] = s.x; sfa[4 * k + 1] = s.y; sfa[4 * k + 2] = s.z; sfa[4 * k + 3] = s.w;
+                }
+                tmem_st16(buf + 48u + 16u * q, sfa);
+              }
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full + 8 * (g & x_mask));
+          }
+          if (lane == 0) mbar_arrive(raw_empty + 8 * rs);
+          if (++rs == p.raw_stages) { rs = 0; rph ^= 1; }
+        }
+
+        // ------------------------- read-out ------------------------------------
+        wait(acc_full, item & 1, abort_flag, p.status, 49);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const bool ok = *abort_flag == 0;
+        const int64_t col = (int64_t)R.n0 + row;
+        const uint32_t Rt = (uint32_t)term_rows(wide, rows);
+        auto emit = [&](int m, float sum) {
+          const float scale = __shfl_sync(0xffffffffu, m < 32 ? xs0 : xs1, m & 31);
+          if (m >= rows) return;
+          const float val = sum * scale;
+          if (!kGrouped && p.slices > 1) {
+            // into the shared memory of the row's owner: slot [row / slices][slice][128 weight rows]
+            uint32_t dst;
+            const uint32_t local = (p.red_off | win) + (uint32_t)(((m / p.slices) * p.slices + slice) * kBM + row) * 4u;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(local), "r"(m % p.slices));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(val) : "memory");
+          } else if (ok && col < R.n_end) {
+            int64_t orow = m;
+            if (kGrouped) {
+              const int j = R.lo + pass * p.pass_rows + m;         // sorted position of the row
+              orow = p.row_map ? p.row_map[j] : j;
+            }
+            p.y[orow * p.N + col] = (uint16_t)gb_f32_to_bf16_bits(val * p.global_scale);
+          }
+        };
+        if (wide) {
+          for (int c = wg; c * 8 < rows; c += 4) {
+            uint32_t h[8], l[8], e[8];
+            const uint32_t at = lane_base + (uint32_t)(c * 8);
+            tmem_ld8(at, h);
+            tmem_ld8(at + 128u, l);
+            tmem_ld8(at + Rt, e);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              emit(c * 8 + i, fmaf(__uint_as_float(e[i]), 0x1p-7f, fmaf(__uint_as_float(l[i]), 0x1p-4f, __uint_as_float(h[i]))));
+          }
+        } else if (wg * 4 < rows) {
+          // four rows per warpgroup, all loads in flight; issuers without a unit leave their accumulator untouched
+          const int accs = min(4, units);
+          uint32_t h[4][4], l[4][4], e[4][4];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            const uint32_t at = lane_base + (uint32_t)min(a, accs - 1) * acc_stride + (uint32_t)(wg * 4);
+            tmem_ld4(at, h[a]);
+            tmem_ld4(at + Rt, l[a]);
+            tmem_ld4(at + 2 * Rt, e[a]);
+          }
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+              if (a < accs)
+                sum += fmaf(__uint_as_float(e[a][i]), 0x1p-7f, fmaf(__uint_as_float(l[a][i]), 0x1p-4f, __uint_as_float(h[a][i])));
+            emit(wg * 4 + i, sum);
+          }
+        }
+        if (!kGrouped && p.slices > 1) {
+          // every warp tells every CTA of the cluster that its sums are in place, then the owners add
+          __syncwarp();
+          if (lane < p.slices) {
+            uint32_t dst;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(red_full), "r"(lane));
+            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(dst) : "memory");
+          }
+          wait<true>(red_full, 0, abort_flag, p.status, 50);
+          for (int i = d; ; i += 32 * kDecWarps) {
+            const int own = i / kBM, r = i % kBM, m = own * p.slices + slice;
+            if (m >= rows) break;
+            float s = 0.0f;
+            for (int q = 0; q < p.slices; ++q) {
+              float f;
+              asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"((p.red_off | win) + (uint32_t)((own * p.slices + q) * kBM + r) * 4u));
+              s += f;
+            }
+            if (*abort_flag == 0 && R.n0 + r < R.n_end) p.y[(int64_t)m * p.N + R.n0 + r] = (uint16_t)gb_f32_to_bf16_bits(s * p.global_scale);
+          }
+        }
+        // hand the accumulators back for the next item (pass or tile)
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (p.slices > 1)                                        // no CTA leaves while a peer may still reach its shared memory
+    cluster_sync();
+  if (warp == 2)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+}
+
+// ---- the activations' operand ------------------------------------------------------------------
+struct Group { uint32_t q[2], e[2]; uint32_t hi, lo, dl; };   // codes of q, codes of the correction, three scale bytes
+
+// The three terms of one group of sixteen bf16 values; `shift` = 7 - exponent of the row's largest m1.
+GB_DEVINL Group split_group(const uint32_t (&w)[8], float amax, bool nan, int scale_rule, int shift) {
+  Group r;
+  amax = fmaxf(amax, 1e-8f);
+  const float scale = gb_fp4_group_scale(amax, scale_rule);
+  if (nan || !(scale < __int_as_float(0x7F800000))) {       // the whole group is NaN (and with it the row's results)
+    r.q[0] = r.q[1] = r.e[0] = r.e[1] = 0x22222222u;
+    r.hi = r.lo = r.dl = 0x7Fu;
+    return r;
+  }
+  const bool plain = gb_plain_division(scale);
+  const float rinv = __frcp_rn(scale);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t q = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t x = w[4 * h + i];
+      const float a = gb_bf16_bits_to_f32(x & 0xFFFFu), b = gb_bf16_bits_to_f32(x >> 16);
+      uint32_t c;
+      if (plain) c = gb_cvt_e2m1x2(gb_e2m1_rtn(__fdiv_rn(a, scale)), gb_e2m1_rtn(__fdiv_rn(b, scale)));
+      else c = gb_e2m1_div2(a, b, scale, rinv);
+      q |= c << (8 * i);
+    }
+    r.q[h] = q;
+  }
+  const float m1 = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(scale));
+  const float m3 = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(__fmul_rn(1.5f, scale)));
+  const int e1 = (int)((__float_as_uint(m1) >> 23) & 0xFFu) - 127;      // m1 is normal: scale >= 1e-8 / 6
+  // half-ulps of m1 by which bf16(1.5 s) misses 1.5 m1 (exact in fp32)
+  const int n = (int)((m3 - 1.5f * m1) * __uint_as_float((uint32_t)(127 + 8 - e1 > 254 ? 254 : 127 + 8 - e1) << 23));
+  // m1 normalised, its upper four significant bits (truncated to UE4M3), the rest times 16
+  const int e = e1 + shift;                                            // <= 7
+  const float V = e >= -40 ? __uint_as_float((__float_as_uint(m1) & 0x007FFFFFu) | ((uint32_t)(127 + e) << 23)) : 0.0f;
+  const uint32_t vb = __float_as_uint(V);
+  r.hi = V >= 0x1p-6f ? (vb >> 20) - (120u << 3) : (uint32_t)(V * 512.0f);
+  r.lo = gb_f32_to_e4m3((V - gb_e4m3_to_f32(r.hi)) * 16.0f);
+  const int de = e + 7;                                                // exponent field of 2^e
+  r.dl = e >= -6 ? (uint32_t)de << 3 : e >= -9 ? 1u << (e + 9) : 0u;
+  const uint32_t an = (uint32_t)(n < 0 ? -n : n), flip = n < 0 ? 0x88888888u : 0u;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t q = r.q[h];
+    const uint32_t b0 = q & 0x11111111u, b1 = (q >> 1) & 0x11111111u, b2 = (q >> 2) & 0x11111111u;
+    const uint32_t on = b0 & (b1 | b2), m = (on << 4) - on;            // nibbles with q = +-1.5, 3, 6: 0xF
+    const uint32_t one = (b1 & ~b2) | ((b2 & ~b1) << 1) | ((b1 & b2) << 2);      // n = 1: 0.5, 1, 2
+    const uint32_t mag = an == 3 ? q & 0x77777777u : an == 2 ? q & 0x66666666u : an == 1 ? one : 0u;
+    r.e[h] = (mag | ((q ^ flip) & 0x88888888u)) & m;
+  }
+  return r;
+}
+
+// Stores one group's terms for row m of a tile with `rows` rows; called by whole quads of lanes (four
+// neighbouring groups) so that the scale bytes leave as words.
+GB_DEVINL void store_group(const Group& G, uint8_t* tile, int64_t unit_stride, bool wide, int rows, int m, int g, unsigned mask) {
+  const int sb = g >> 4, gi = g & 15;
+  uint8_t* unit = tile + sb * unit_stride;
+  uint8_t* codes = unit + sf_bytes(wide);
+  const int R = term_rows(wide, rows);
+  auto put = [&](int n, uint2 c) {
+    *reinterpret_cast<uint2*>(codes + (n >> 3) * 1024 + (n & 7) * 128 + (((gi >> 1) ^ (n & 7)) << 4) + (gi & 1) * 8) = c;
+  };
+  const uint2 q = make_uint2(G.q[0], G.q[1]), e = make_uint2(G.e[0], G.e[1]);
+  put(m, q);
+  put(R + m, wide ? e : q);
+  if (!wide) put(2 * R + m, e);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {                             // hi, lo, dlt
+    const uint32_t b = t == 0 ? G.hi : t == 1 ? G.lo : G.dl;
+    const uint32_t b1 = __shfl_down_sync(mask, b, 1), b2 = __shfl_down_sync(mask, b, 2), b3 = __shfl_down_sync(mask, b, 3);
+    const int n = !wide ? t * R + m : t == 1 ? m : (t == 2 ? R : 0) + m;
+    if ((gi & 3) == 0)
+      *reinterpret_cast<uint32_t*>(unit + (wide && t == 1 ? 2048 : 0) + (gi >> 2) * 512 + (n & 31) * 16 + ((n >> 5) & 3) * 4) =
+          b | (b1 << 8) | (b2 << 16) | (b3 << 24);
+  }
+}
+
+struct RowsParams {
+  const uint4* x;            // bf16 rows [*, K]
+  uint8_t* xop;
+  float* x_scale;
+  int64_t x_unit;
+  int K, n_sb, scale_rule, pass_rows;
+  int rows;                  // dense: M
+  // grouped: sorted row j = blockIdx.x belongs to expert ids[order[j]]
+  const int32_t* ids;
+  const int32_t* order;
+  const int32_t* seg;
+  int E, topk;
+  int swiglu;                // x holds [gate | up] rows in sorted order
+  const int32_t* inv;        // token mode: sorted position of every pair
+};
+
+constexpr int kRowsMaxGroups = 4;
+
+// kMode 0: dense, one CTA per row.  1: one CTA per token, its row goes to each of its experts' tiles.
+// 2: one CTA per sorted row of [gate | up]: SwiGLU (with the bf16 roundings of F.silu(gate) * up), then the split.
+template <int kG, int kMode>
+__global__ void __launch_bounds__(1024)
+fp4_rows_kernel(const __grid_constant__ RowsParams p) {
+  gb_pdl_launch_dependents();
+  gb_pdl_wait();
+  const int groups = p.K / 16;
+  const int j = blockIdx.x;
+  if (kMode == 2 && j >= p.seg[p.E]) return;
+  const uint4* xr = p.x + (int64_t)j * (kMode == 2 ? 4 : 2) * groups;
+  __shared__ float red[32];
+  uint32_t w[kG][8];
+  float amax[kG];
+  bool nan[kG];
+  float top = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kG; ++i) {
+    const int g = threadIdx.x + i * blockDim.x;
+    amax[i] = 0.0f;
+    nan[i] = false;
+    if (g < groups) {
+      if (kMode == 2) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint4 a = xr[2 * g + h], b = xr[2 * groups + 2 * g + h];
+          const uint32_t gw[4] = {a.x, a.y, a.z, a.w}, uw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float s0 = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_silu(gb_bf16_bits_to_f32(gw[q] & 0xFFFFu))));
+            const float s1 = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_silu(gb_bf16_bits_to_f32(gw[q] >> 16))));
+            w[i][4 * h + q] = gb_pack_bf16x2(s0 * gb_bf16_bits_to_f32(uw[q] & 0xFFFFu), s1 * gb_bf16_bits_to_f32(uw[q] >> 16));
+          }
+        }
+      } else {
+        const uint4 a = xr[2 * g], b = xr[2 * g + 1];
+        w[i][0] = a.x; w[i][1] = a.y; w[i][2] = a.z; w[i][3] = a.w;
+        w[i][4] = b.x; w[i][5] = b.y; w[i][6] = b.z; w[i][7] = b.w;
+      }
+      amax[i] = gb_amax_bf16(w[i], &nan[i]);
+      if (amax[i] < __int_as_float(0x7F800000)) top = fmaxf(top, amax[i]);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = top;
+  __syncthreads();
+  top = (int)(threadIdx.x & 31) < (int)(blockDim.x >> 5) ? red[threadIdx.x & 31] : 0.0f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  const float m1 = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_fp4_group_scale(fmaxf(top, 1e-8f), p.scale_rule)));
+  const int shift = 7 - ((int)((__float_as_uint(m1) >> 23) & 0xFFu) - 127);
+  const float back = __uint_as_float((uint32_t)(127 - shift) << 23);
+
+  Group grp[kG];
+#pragma unroll
+  for (int i = 0; i < kG; ++i)
+    if ((int)(threadIdx.x + i * blockDim.x) < groups) grp[i] = split_group(w[i], amax[i], nan[i], p.scale_rule, shift);
+
+  const int copies = kMode == 1 ? p.topk : 1;
+  for (int s = 0; s < copies; ++s) {
+    int tile = 0, m = j, rows = p.rows;
+    if (kMode != 0) {
+      const int pair = kMode == 1 ? j * p.topk + s : p.order[j];
+      const int e = p.ids[pair];
+      if (e < 0 || e >= p.E) continue;                       // a dropped pair (uniform over the CTA)
+      const int lo = p.seg[e], cnt = p.seg[e + 1] - lo;
+      const int r = (kMode == 1 ? p.inv[pair] : j) - lo, pass = r / p.pass_rows;
+      m = r - pass * p.pass_rows;
+      rows = min(p.pass_rows, cnt - pass * p.pass_rows);
+      tile = lo / p.pass_rows + e + pass;
+    }
+    if (threadIdx.x == 0) p.x_scale[(int64_t)tile * p.pass_rows + m] = back;
+    uint8_t* dst = p.xop + (int64_t)tile * p.n_sb * p.x_unit;
+#pragma unroll
+    for (int i = 0; i < kG; ++i) {
+      const int g = threadIdx.x + i * blockDim.x;
+      const unsigned here = __ballot_sync(0xffffffffu, g < groups);
+      if (g < groups) store_group(grp[i], dst, p.x_unit, is_wide(p.pass_rows), rows, m, g, here);
+    }
+  }
+}
+
+// ---- host side -----------------------------------------------------------------------------------
+int fp4_format(const gb_weight* w, bool scales_e4m3) {
+  const gb_format& f = w->fmt;
+  if (f.grid != GB_GRID_FP4 || (w->row_stride % 16) != 0 || ((uintptr_t)w->qw & 15u) != 0 || ((uintptr_t)w->codebook & 15u) != 0)
+    return -1;
+  if (f.mode == GB_MODE_FULL && f.k_bits == 8 && f.scale_coding == GB_SCALE_V1 && f.type_size == 48) return kLit;
+  if (f.mode == GB_MODE_PRODUCT && f.n_sub == 2 && f.scale_coding == GB_SCALE_V2 && w->compose != nullptr && scales_e4m3) {
+    switch (f.k_bits) {
+      case 12: return f.type_size == Fmt<12>::kSb ? 12 : -1;
+      case 16: return f.type_size == Fmt<16>::kSb ? 16 : -1;
+      case 20: return f.type_size == Fmt<20>::kSb ? 20 : -1;
+      case 24: return f.type_size == Fmt<24>::kSb ? 24 : -1;
+      default: return -1;
+    }
+  }
+  return -1;
+}
+
+struct Info { int sb, per_stage, pitch; uint32_t box, lut, extra; };
+template <int F> Info info_of() {
+  return {Fmt<F>::kSb, Fmt<F>::kSbPerStage, Geo<F>::kPitch, (uint32_t)Geo<F>::kBoxBytes, Fmt<F>::kLutBytes,
+          Fmt<F>::kScaleTab + (F == kLit ? 0u : 16384u)};
+}
+Info info(int F) {
+  switch (F) {
+    case kLit: return info_of<kLit>();
+    case 12: return info_of<12>();
+    case 16: return info_of<16>();
+    case 20: return info_of<20>();
+    default: return info_of<24>();
+  }
+}
+
+// Shared memory: [kDynBase, kLut) and [behind the tables, end).  The activation ring holds eight units where
+// they fit beside two raw stages, else four (a unit's slot and its operand buffer are handed back by
+// one barrier, so only multiples of the four buffers work); what is left goes to the raw ring.
+bool layout(const Info& f, Fp4Params& p) {
+  for (p.x_stages = 8; p.x_stages >= 4; p.x_stages -= 4) {
+    struct Region { uint32_t at, end; } reg[2] = {{kDynBase, kLut}, {kLut + f.lut, kSmemEnd}};
+    auto take = [&](uint32_t bytes, uint32_t align, uint32_t* out) {
+      for (int r = 0; r < 2; ++r) {
+        const uint32_t a = (reg[r].at + align - 1) & ~(align - 1);
+        if (a + bytes <= reg[r].end) { *out = a; reg[r].at = a + bytes; return true; }
+      }
+      return false;
+    };
+    if (!take((uint32_t)(p.x_stages * p.x_unit), 1024, &p.x_off)) continue;
+    if (!take(512 + f.extra, 128, &p.misc_off)) continue;
+    if (p.slices > 1 && !take((uint32_t)((p.M + p.slices - 1) / p.slices * p.slices * kBM * 4), 128, &p.red_off)) continue;
+    for (p.raw_stages = 0; p.raw_stages < kMaxRaw && take(f.box, 128, &p.raw_off[p.raw_stages]);) ++p.raw_stages;
+    if (p.raw_stages >= 2) return true;
+  }
+  return false;
+}
+
+std::mutex g_mutex;
+int g_clusters[64][kMaxSlices + 1];                        // clusters of a size that run at once, per device (0: not asked yet)
+
+int max_clusters(int size) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  int& n = g_clusters[dev][size];
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, (unsigned)size);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemMax;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)size; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, fp4_decode_kernel<false, kLit>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); return 0; }
+  }
+  return n;
+}
+
+template <bool kGrouped>
+cudaError_t launch(int F, dim3 grid, cudaStream_t stream, const CUtensorMap& map_w, const Fp4Params& p) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmemMax;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (gb_pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (p.slices > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = 1; attr[n].val.clusterDim.y = (unsigned)p.slices; attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  gb_count_launch();
+  switch (F) {
+    case kLit: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, kLit>, map_w, p);
+    case 12: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, 12>, map_w, p);
+    case 16: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, 16>, map_w, p);
+    case 20: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, 20>, map_w, p);
+    default: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, 24>, map_w, p);
+  }
+}
+
+template <int kMode>
+int launch_rows(int64_t ctas, int64_t K, cudaStream_t stream, const RowsParams& p) {
+  const int64_t groups = K / 16;
+  const int per = groups <= 512 ? 1 : groups <= 1024 ? 2 : kRowsMaxGroups;
+  const int64_t threads = ((groups + per - 1) / per + 31) / 32 * 32;
+  if (threads > 1024) return GB_EUNSUPPORTED;
+#define GB_FP4_ROWS(G) GB_CUDA_OK(gb_launch(fp4_rows_kernel<G, kMode>, dim3((unsigned)ctas), dim3((unsigned)threads), 0, stream, p))
+  switch (per) {
+    case 1: GB_FP4_ROWS(1); break;
+    case 2: GB_FP4_ROWS(2); break;
+    default: GB_FP4_ROWS(kRowsMaxGroups); break;
+  }
+#undef GB_FP4_ROWS
+  return GB_OK;
+}
+
+int64_t align256(int64_t v) { return (v + 255) & ~255ll; }
+
+}  // namespace
+
+int gb_prepare_gemv_fp4() {
+#define GB_FP4_ATTR(F)                                                                                                     \
+  GB_CUDA_OK(cudaFuncSetAttribute((const void*)fp4_decode_kernel<false, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax)); \
+  GB_CUDA_OK(cudaFuncSetAttribute((const void*)fp4_decode_kernel<true, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax))
+  GB_FP4_ATTR(kLit);
+  GB_FP4_ATTR(12);
+  GB_FP4_ATTR(16);
+  GB_FP4_ATTR(20);
+  GB_FP4_ATTR(24);
+#undef GB_FP4_ATTR
+  return GB_OK;
+}
+
+// Whether the kernel takes the weight (any row count; 64 rows per launch).
+bool gb_gemv_fp4_applies(const gb_weight* w, bool scales_e4m3) {
+  return fp4_format(w, scales_e4m3) >= 0 && w->rows >= 64 && w->K / 16 <= 1024 * kRowsMaxGroups;
+}
+
+// The operand of up to 64 rows and the rows' scales.
+int64_t gb_gemv_fp4_workspace_bytes(int64_t M, int64_t K) {
+  const int rows = (int)(M > kMaxRows ? kMaxRows : M);
+  return align256((K / 256) * unit_bytes(is_wide(rows), rows)) + align256(rows * 4);
+}
+
+int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, int n_roles, const int64_t* role_rows,
+                int scale_rule, void* y, void* workspace, int64_t workspace_bytes, void* stream_) {
+  const int F = fp4_format(w, scales_e4m3);
+  if (F < 0 || ((uintptr_t)x & 15u) != 0 || n_roles > kMaxRoles || (n_roles <= 1 && w->cb_row_offset != nullptr)) return GB_EUNSUPPORTED;
+  const int sms = gb_sm_count();
+  if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
+  if (workspace == nullptr || workspace_bytes < gb_gemv_fp4_workspace_bytes(M, w->K))
+    return gb_fail(GB_EWORKSPACE, "workspace of %lld bytes is too small (need %lld)", (long long)workspace_bytes,
+                   (long long)gb_gemv_fp4_workspace_bytes(M, w->K));
+  const Info f = info(F);
+  cudaStream_t stream = (cudaStream_t)stream_;
+  CUtensorMap map_w;
+  int rc = gb_tensor_map_bytes_2d(&map_w, w->qw, (uint64_t)(w->K / 256) * f.sb, (uint64_t)w->rows, (uint64_t)w->row_stride, f.pitch, kBM);
+  if (rc != GB_OK) return rc;
+  for (int64_t m0 = 0; m0 < M; m0 += kMaxRows) {
+    Fp4Params p = {};
+    p.N = w->rows; p.K = w->K;
+    p.M = (int)(M - m0 < kMaxRows ? M - m0 : kMaxRows);
+    p.n_sb = (int)(w->K / 256);
+    p.pass_rows = p.M;
+    p.x_unit = unit_bytes(is_wide(p.M), p.M);
+    p.xop = (const uint8_t*)workspace;
+    p.x_scale = (const float*)((const uint8_t*)workspace + align256(p.n_sb * p.x_unit));
+    p.codebook = w->codebook;
+    p.compose = w->compose;
+    p.global_scale = w->global_scale == 0.0f ? 1.0f : w->global_scale;
+    p.y = (uint16_t*)y + m0 * w->rows;
+    p.status = gb_status_word();
+    p.n_roles = n_roles < 1 ? 1 : n_roles;
+    int64_t row = 0;
+    for (int r = 0; r < p.n_roles; ++r) {
+      const int64_t rows = n_roles < 1 ? w->rows : role_rows[r];
+      p.role[r] = {(int)row, (int)rows, p.n_tiles, r * gb_codebook_elems(w->fmt)};
+      p.n_tiles += (int)((rows + kBM - 1) / kBM);
+      row += rows;
+    }
+    GB_REQUIRE(row == w->rows, "the roles hold %lld rows, the matrix %lld", (long long)row, (long long)w->rows);
+    // K slices: enough CTAs for the SMs when there are few tiles; no more clusters than run at once,
+    // at least two superblocks per slice
+    int want = 1;
+    for (int s = 2; s <= kMaxSlices && p.n_tiles * s <= sms && s * 2 <= p.n_sb; ++s)
+      if (p.n_tiles <= max_clusters(s)) want = s;
+    p.units = (p.n_sb + want - 1) / want;
+    p.units = (p.units + f.per_stage - 1) / f.per_stage * f.per_stage;
+    p.slices = (p.n_sb + p.units - 1) / p.units;
+    if (!layout(f, p)) return gb_fail(GB_EUNSUPPORTED, "no shared-memory layout for %d rows", p.M);
+    RowsParams rp = {};
+    rp.x = (const uint4*)((const uint16_t*)x + m0 * w->K);
+    rp.xop = (uint8_t*)workspace;
+    rp.x_scale = (float*)((uint8_t*)workspace + align256(p.n_sb * p.x_unit));
+    rp.x_unit = p.x_unit;
+    rp.K = (int)w->K; rp.n_sb = p.n_sb; rp.scale_rule = scale_rule; rp.pass_rows = p.pass_rows; rp.rows = p.M;
+    rc = launch_rows<0>(p.M, w->K, stream, rp);
+    if (rc != GB_OK) return rc;
+    const int ctas = p.slices > 1 || p.n_tiles <= sms ? p.n_tiles : sms;
+    GB_CUDA_OK(launch<false>(F, dim3((unsigned)ctas, (unsigned)p.slices), stream, map_w, p));
+  }
+  return GB_OK;
+}
+
+// ---- routed experts ------------------------------------------------------------------------------
+namespace {
+
+// Every scale of the two-tier weight an exact positive E4M3 value?  Raises *flag otherwise.
+__global__ void __launch_bounds__(256)
+scales_exact_kernel(const uint8_t* qw, int64_t row_stride, int64_t rows, int n_sb, int type_size, int super_at,
+                    const float* compose, int* flag) {
+  __shared__ uint8_t bad[256];
+  {
+    bool ok = true;
+    for (int i = 0; i < 16; ++i) {
+      const float v = compose[threadIdx.x * 16 + i];
+      ok &= v >= 0.0f && v <= 448.0f && gb_e4m3_to_f32(gb_f32_to_e4m3(fminf(v, 448.0f))) == v;
+    }
+    bad[threadIdx.x] = ok ? 0 : 1;
+  }
+  __syncthreads();
+  bool any = false;
+  const int64_t units = rows * n_sb;
+  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = u / n_sb;
+    any |= bad[qw[r * row_stride + (u - r * n_sb) * type_size + super_at]] != 0;
+  }
+  if (any) *flag = 1;
+}
+
+// Rows per pass of a grouped launch: more rows per pass decode the weights less often, fewer leave
+// room for more accumulators and deeper rings.  From the average number of rows per expert.
+int pass_rows_for(int F, int64_t P, int64_t E) {
+  const int64_t avg = P / (E > 0 ? E : 1);
+  if (F == 20 || F == 24) return 16;                       // their tables leave no more room
+  return avg <= 8 ? 16 : avg <= 24 ? 32 : 64;
+}
+
+}  // namespace
+
+extern "C" {
+
+int gb_scales_e4m3(const gb_weight* w, int64_t rows, int32_t* flag, void* stream) {
+  int rc = gb_check_weight(w);
+  if (rc != GB_OK) return rc;
+  GB_REQUIRE(flag != nullptr && w->compose != nullptr && rows >= 1, "gb_scales_e4m3 wants a two-tier weight and a flag");
+  const int sms = gb_sm_count();
+  if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
+  GB_CUDA_OK(cudaMemsetAsync(flag, 0, sizeof(int32_t), (cudaStream_t)stream));
+  gb_count_launch();
+  scales_exact_kernel<<<sms * 4, 256, 0, (cudaStream_t)stream>>>(w->qw, w->row_stride, rows, (int)(w->K / 256), w->fmt.type_size,
+                                                                 4 * w->fmt.k_bits, w->compose, flag);
+  GB_LAUNCH_OK("scales_exact_kernel");
+  return GB_OK;
+}
+
+int gb_gemv_hinted(const void* x, int64_t M, const gb_weight* w, const gb_hints* hints, int scale_rule, void* y,
+                   void* workspace, int64_t workspace_bytes, void* stream) {
+  int rc = gb_check_weight(w);
+  if (rc != GB_OK) return rc;
+  GB_REQUIRE(x && y && hints, "null pointer argument");
+  GB_REQUIRE(M >= 1 && M <= 128, "decode-batch kernels take 1..128 rows, got M=%lld", (long long)M);
+  GB_REQUIRE(hints->n_roles >= 0 && hints->n_roles <= GB_MAX_ROLES, "%d roles", hints->n_roles);
+  const int act = w->fmt.grid == GB_GRID_FP4 ? GB_ACT_FP4_GROUP16 : GB_ACT_FP8_TOKEN;
+  if (act == GB_ACT_FP4_GROUP16 && gb_gemv_fp4_applies(w, hints->scales_e4m3 != 0)) {
+    rc = gb_gemv_fp4(x, M, w, hints->scales_e4m3 != 0, hints->n_roles, hints->role_rows, scale_rule, y, workspace,
+                     workspace_bytes, stream);
+    if (rc != GB_EUNSUPPORTED) return rc;
+  }
+  return gb_gemv(x, M, w, act, scale_rule, y, workspace, workspace_bytes, stream);
+}
+
+int gb_moe_fp4_pass_rows(const gb_weight* w, int scales_e4m3, int64_t P, int64_t E) {
+  if (gb_check_weight(w) != GB_OK) return 0;
+  const int F = fp4_format(w, scales_e4m3 != 0);
+  if (F < 0 || w->cb_row_offset != nullptr || w->rows % kBM != 0 || w->K / 16 > 1024 * kRowsMaxGroups) return 0;
+  return pass_rows_for(F, P, E);
+}
+
+int64_t gb_moe_fp4_operand_bytes(int64_t P, int64_t E, int64_t K, int pass_rows) {
+  if (pass_rows < 1) return 0;
+  const int64_t tiles = P / pass_rows + E + 1;
+  return align256(tiles * (K / 256) * unit_bytes(is_wide(pass_rows), pass_rows)) + align256(tiles * pass_rows * 4);
+}
+
+static int rows_params(RowsParams* p, const void* x, int64_t P, int64_t E, int64_t K, int pass_rows, const int32_t* ids,
+                       const int32_t* seg, int scale_rule, void* operand) {
+  GB_REQUIRE(x && ids && seg && operand, "null pointer argument");
+  GB_REQUIRE(P >= 1 && P < (1ll << 30) && E >= 1 && K > 0 && K % 256 == 0 && pass_rows >= 1 && pass_rows <= kMaxRows,
+             "bad shape P=%lld E=%lld K=%lld", (long long)P, (long long)E, (long long)K);
+  GB_REQUIRE(((uintptr_t)x & 15u) == 0 && ((uintptr_t)operand & 255u) == 0, "rows must be 16-byte aligned, the operand 256-byte");
+  const int64_t tiles = P / pass_rows + E + 1;
+  p->x = (const uint4*)x;
+  p->xop = (uint8_t*)operand;
+  p->x_unit = unit_bytes(is_wide(pass_rows), pass_rows);
+  p->x_scale = (float*)((uint8_t*)operand + align256(tiles * (K / 256) * p->x_unit));
+  p->K = (int)K; p->n_sb = (int)(K / 256); p->scale_rule = scale_rule; p->pass_rows = pass_rows;
+  p->ids = ids; p->seg = seg; p->E = (int)E;
+  return GB_OK;
+}
+
+int gb_moe_fp4_rows(const void* x, const int32_t* ids, const int32_t* inv, const int32_t* seg, int64_t T, int64_t topk,
+                    int64_t E, int64_t K, int pass_rows, int scale_rule, void* operand, void* stream) {
+  RowsParams p = {};
+  int rc = rows_params(&p, x, T * topk, E, K, pass_rows, ids, seg, scale_rule, operand);
+  if (rc != GB_OK) return rc;
+  GB_REQUIRE(inv != nullptr, "null pointer argument");
+  p.inv = inv; p.topk = (int)topk;
+  return launch_rows<1>(T, K, (cudaStream_t)stream, p);
+}
+
+int gb_moe_fp4_swiglu_rows(const void* h, const int32_t* ids, const int32_t* order, const int32_t* seg, int64_t P, int64_t E,
+                           int64_t inter, int pass_rows, int scale_rule, void* operand, void* stream) {
+  RowsParams p = {};
+  int rc = rows_params(&p, h, P, E, inter, pass_rows, ids, seg, scale_rule, operand);
+  if (rc != GB_OK) return rc;
+  GB_REQUIRE(order != nullptr, "null pointer argument");
+  p.order = order;
+  return launch_rows<2>(P, inter, (cudaStream_t)stream, p);
+}
+
+int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, int64_t expert_stride, int64_t E,
+                    const int32_t* seg, const int32_t* row_map, int64_t P, int pass_rows, void* y, void* stream_) {
+  GB_REQUIRE(operand && w && seg && y, "null pointer argument");
+  int rc = gb_check_weight(w);
+  if (rc != GB_OK) return rc;
+  const int64_t N = w->rows, K = w->K;
+  const int F = fp4_format(w, scales_e4m3 != 0);
+  if (F < 0 || gb_moe_fp4_pass_rows(w, scales_e4m3, P, E) < pass_rows || expert_stride != N * w->row_stride || E * N >= (1ll << 31))
+    return gb_fail(GB_EUNSUPPORTED, "not a stack the fp4 expert kernel takes");
+  const int sms = gb_sm_count();
+  if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
+  const Info f = info(F);
+  const int64_t tiles = P / pass_rows + E + 1;
+  Fp4Params p = {};
+  p.N = N; p.K = K; p.n_sb = (int)(K / 256); p.units = p.n_sb; p.slices = 1;
+  p.pass_rows = pass_rows;
+  p.x_unit = unit_bytes(is_wide(pass_rows), pass_rows);
+  p.xop = (const uint8_t*)operand;
+  p.x_scale = (const float*)((const uint8_t*)operand + align256(tiles * p.n_sb * p.x_unit));
+  p.codebook = w->codebook; p.compose = w->compose;
+  p.global_scale = w->global_scale == 0.0f ? 1.0f : w->global_scale;
+  p.y = (uint16_t*)y;
+  p.status = gb_status_word();
+  p.n_roles = 1;
+  p.seg = seg; p.row_map = row_map;
+  p.tiles_n = (int)(N / kBM);
+  p.n_tiles = (int)(E * p.tiles_n);
+  if (!layout(f, p)) return gb_fail(GB_EUNSUPPORTED, "no shared-memory layout for %d rows per pass", pass_rows);
+  CUtensorMap map_w;
+  rc = gb_tensor_map_bytes_2d(&map_w, w->qw, (uint64_t)p.n_sb * f.sb, (uint64_t)(E * N), (uint64_t)w->row_stride, f.pitch, kBM);
+  if (rc != GB_OK) return rc;
+  GB_CUDA_OK(launch<true>(F, dim3((unsigned)(p.n_tiles < sms ? p.n_tiles : sms)), (cudaStream_t)stream_, map_w, p));
+  return GB_OK;
+}
+
+}  // extern "C"

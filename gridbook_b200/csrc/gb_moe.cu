@@ -11,7 +11,7 @@ constexpr int kRouteThreads = 1024;
 __global__ void __launch_bounds__(kRouteThreads)
 moe_route_kernel(const int32_t* __restrict__ ids, int P, int E, int first_expert, int32_t* __restrict__ counts,
                  int32_t* __restrict__ offsets, int32_t* __restrict__ order,
-                 const float* __restrict__ weights, float* __restrict__ pair_w, int tiled) {
+                 int32_t* __restrict__ inv, const float* __restrict__ weights, float* __restrict__ pair_w, int tiled) {
   extern __shared__ int32_t sh[];   // [E] counts, [E+1] offsets; tiled: + [E][32] + [E]
   int32_t* cnt = sh;
   int32_t* off = sh + E;
@@ -57,7 +57,11 @@ moe_route_kernel(const int32_t* __restrict__ ids, int P, int E, int first_expert
         const int i = base + lane;
         const bool hit = i < P && ids[i] - first_expert == e;
         const unsigned mask = __ballot_sync(0xffffffffu, hit);
-        if (hit) order[pos + __popc(mask & ((1u << lane) - 1u))] = i;
+        if (hit) {
+          const int at = pos + __popc(mask & ((1u << lane) - 1u));
+          order[at] = i;
+          if (inv) inv[i] = at;
+        }
         pos += __popc(mask);
       }
     }
@@ -99,7 +103,11 @@ moe_route_kernel(const int32_t* __restrict__ ids, int P, int E, int first_expert
       if (lane == 31) cursor[e] = start + incl;
     }
     __syncthreads();
-    if (id >= 0) order[wcnt[id * nwarps + warp] + rank] = i;
+    if (id >= 0) {
+      const int at = wcnt[id * nwarps + warp] + rank;
+      order[at] = i;
+      if (inv) inv[i] = at;
+    }
     __syncthreads();
   }
 }
@@ -180,7 +188,7 @@ route_scan_kernel(int32_t* __restrict__ hist, int tiles, int P, int E, int32_t* 
 __global__ void __launch_bounds__(kRouteThreads)
 route_scatter_kernel(const int32_t* __restrict__ ids, int P, int E, int first_expert,
                      const int32_t* __restrict__ hist, const int32_t* __restrict__ offsets,
-                     int32_t* __restrict__ order) {
+                     int32_t* __restrict__ order, int32_t* __restrict__ inv) {
   extern __shared__ int32_t wcnt[];   // [E][32]: warp w's count of expert e, then its start
   constexpr int nwarps = kRouteThreads / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -209,7 +217,11 @@ route_scatter_kernel(const int32_t* __restrict__ ids, int P, int E, int first_ex
     wcnt[e * nwarps + lane] = offsets[e] + hist[(int64_t)blockIdx.x * E + e] + incl - v;
   }
   __syncthreads();
-  if (id >= 0) order[wcnt[id * nwarps + warp] + rank] = i;
+  if (id >= 0) {
+    const int at = wcnt[id * nwarps + warp] + rank;
+    order[at] = i;
+    if (inv) inv[i] = at;
+  }
 }
 
 // Optional cross-GPU part of the combine (expert parallelism): before any row of y is read,
@@ -325,9 +337,9 @@ int64_t gb_moe_route_workspace_bytes(int64_t T, int64_t topk, int64_t E) {
   return ((P + kRouteThreads - 1) / kRouteThreads) * E * (int64_t)sizeof(int32_t);
 }
 
-int gb_moe_route_ws(const int32_t* topk_ids, int64_t T, int64_t topk, int64_t E, int64_t expert_base,
-                    int32_t* counts, int32_t* offsets, int32_t* order, const float* topk_weights, float* pair_w,
-                    void* workspace, int64_t ws_bytes, void* stream) {
+int gb_moe_route_inv(const int32_t* topk_ids, int64_t T, int64_t topk, int64_t E, int64_t expert_base,
+                     int32_t* counts, int32_t* offsets, int32_t* order, int32_t* inv, const float* topk_weights,
+                     float* pair_w, void* workspace, int64_t ws_bytes, void* stream) {
   GB_REQUIRE(topk_ids && counts && offsets && order, "null pointer argument");
   GB_REQUIRE((topk_weights == nullptr) == (pair_w == nullptr), "topk_weights and pair_w go together");
   GB_REQUIRE(T >= 0 && topk >= 1 && E >= 1 && E <= 4096, "bad routing shape T=%lld topk=%lld E=%lld",
@@ -347,7 +359,7 @@ int gb_moe_route_ws(const int32_t* topk_ids, int64_t T, int64_t topk, int64_t E,
                          hist, tiles, P, (int)E, counts, offsets, order));
     GB_CUDA_OK(gb_launch(route_scatter_kernel, dim3(tiles), dim3(kRouteThreads),
                          (size_t)E * (kRouteThreads / 32) * sizeof(int32_t), st, topk_ids, P, (int)E,
-                         (int)expert_base, (const int32_t*)hist, (const int32_t*)offsets, order));
+                         (int)expert_base, (const int32_t*)hist, (const int32_t*)offsets, order, inv));
     return GB_OK;
   }
   // a warp per expert scanning all pairs costs E*P; from a few thousand pairs on, tiles of
@@ -355,9 +367,16 @@ int gb_moe_route_ws(const int32_t* topk_ids, int64_t T, int64_t topk, int64_t E,
   const int tiled = T * topk >= 4096 && E <= 256;
   const size_t smem = (size_t)(2 * E + 1 + (tiled ? E * (kRouteThreads / 32 + 1) : 0)) * sizeof(int32_t);
   GB_CUDA_OK(gb_launch(moe_route_kernel, dim3(1), dim3(kRouteThreads), smem, st, topk_ids,
-                       (int)(T * topk), (int)E, (int)expert_base, counts, offsets, order, topk_weights, pair_w,
+                       (int)(T * topk), (int)E, (int)expert_base, counts, offsets, order, inv, topk_weights, pair_w,
                        tiled));
   return GB_OK;
+}
+
+int gb_moe_route_ws(const int32_t* topk_ids, int64_t T, int64_t topk, int64_t E, int64_t expert_base,
+                    int32_t* counts, int32_t* offsets, int32_t* order, const float* topk_weights, float* pair_w,
+                    void* workspace, int64_t ws_bytes, void* stream) {
+  return gb_moe_route_inv(topk_ids, T, topk, E, expert_base, counts, offsets, order, nullptr, topk_weights, pair_w, workspace,
+                          ws_bytes, stream);
 }
 
 int gb_moe_route(const int32_t* topk_ids, int64_t T, int64_t topk, int64_t E, int64_t expert_base,

@@ -60,6 +60,14 @@ struct Lib {
   GB_FN(gb_moe_mlp_pairs);
   GB_FN(gb_moe_mlp_pairs_workspace_bytes);
   GB_FN(gb_moe_combine);
+  GB_FN(gb_gemv_hinted);
+  GB_FN(gb_scales_e4m3);
+  GB_FN(gb_moe_route_inv);
+  GB_FN(gb_moe_fp4_pass_rows);
+  GB_FN(gb_moe_fp4_operand_bytes);
+  GB_FN(gb_moe_fp4_rows);
+  GB_FN(gb_moe_fp4_swiglu_rows);
+  GB_FN(gb_moe_gemv_fp4);
 #undef GB_FN
 };
 Lib L;
@@ -97,6 +105,14 @@ void bind(const std::string& path) {
   GB_FN(gb_moe_mlp_pairs);
   GB_FN(gb_moe_mlp_pairs_workspace_bytes);
   GB_FN(gb_moe_combine);
+  GB_FN(gb_gemv_hinted);
+  GB_FN(gb_scales_e4m3);
+  GB_FN(gb_moe_route_inv);
+  GB_FN(gb_moe_fp4_pass_rows);
+  GB_FN(gb_moe_fp4_operand_bytes);
+  GB_FN(gb_moe_fp4_rows);
+  GB_FN(gb_moe_fp4_swiglu_rows);
+  GB_FN(gb_moe_gemv_fp4);
 #undef GB_FN
 }
 
@@ -111,6 +127,7 @@ using Opt = c10::optional<at::Tensor>;
 struct Weight {
   gb_weight w{};
   int64_t expert_stride = 0, experts = 1;
+  bool scales_e4m3 = false;      // two-tier: every composed scale is an exact E4M3 value
   std::vector<at::Tensor> keep;
   bool fp4() const { return w.fmt.grid == GB_GRID_FP4; }
   int act() const { return fp4() ? GB_ACT_FP4_GROUP16 : GB_ACT_FP8_TOKEN; }
@@ -138,6 +155,12 @@ Weight make_weight(const at::Tensor& qw, const at::Tensor& codebook, std::array<
   r.w.fmt = {fmt[0], fmt[1], fmt[2], fmt[3], fmt[4], fmt[5]};
   r.expert_stride = expert_stride;
   r.experts = experts;
+  if (r.w.fmt.scale_coding == GB_SCALE_V2) {               // looked at once, here: the kernels may then rely on it
+    const c10::cuda::CUDAGuard guard(qw.device());
+    at::Tensor flag = at::empty({1}, qw.options().dtype(at::kInt));
+    check(L.gb_scales_e4m3(&r.w, experts * rows, flag.data_ptr<int32_t>(), c10::cuda::getCurrentCUDAStream().stream()));
+    r.scales_e4m3 = flag.item<int32_t>() == 0;
+  }
   return r;
 }
 
@@ -179,11 +202,19 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
   Weight w;
   at::Tensor workspace, slots;
   int64_t row_batch_max = 16;
+  gb_hints hints{};
   std::atomic<int> prefill_route{kRouteNone};
   std::mutex mutex;
   std::map<std::vector<const LinearPlan*>, at::Tensor> shared_slots;
 
-  LinearPlan(Weight weight, at::Tensor ws, const Opt& armed) : w(std::move(weight)), workspace(std::move(ws)) {
+  // `role_rows`: row counts of the parts with a codebook of their own (empty: one codebook)
+  LinearPlan(Weight weight, at::Tensor ws, const Opt& armed, const std::vector<int64_t>& role_rows)
+      : w(std::move(weight)), workspace(std::move(ws)) {
+    hints.scales_e4m3 = w.scales_e4m3 ? 1 : 0;
+    if (role_rows.size() <= GB_MAX_ROLES) {                // more parts than that: the per-row offsets alone speak
+      hints.n_roles = (int32_t)role_rows.size();
+      for (size_t i = 0; i < role_rows.size(); ++i) hints.role_rows[i] = role_rows[i];
+    }
     if (armed.has_value() && armed->defined()) slots = *armed;
     row_batch_max = L.gb_gemv_row_batch_max(&w.w);
   }
@@ -212,7 +243,7 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
       at::Tensor ws = workspace;
       const int64_t need = L.gb_gemv_workspace_bytes(M, N, K);
       if (!ws.defined() || ws.numel() < need) ws = at::empty({need}, x.options().dtype(at::kByte));
-      check(L.gb_gemv(xc.data_ptr(), M, &w.w, w.act(), rule, out.data_ptr(), ws.data_ptr(), ws.numel(), stream));
+      check(L.gb_gemv_hinted(xc.data_ptr(), M, &w.w, &hints, rule, out.data_ptr(), ws.data_ptr(), ws.numel(), stream));
       return out;
     }
     prefill(xc, M, out, rule, nvfp4, stream);
@@ -301,14 +332,20 @@ struct MoEPlan {
   Weight w13, w2;
   Weight rows13, rows2;          // the stacks seen as one matrix of E * rows rows (for the expanders)
   int64_t E, hidden, inter;
-  bool sorted_ok, pair_ok;
+  bool sorted13, sorted2, pair_ok;   // per projection: a kernel that takes rows in expert order
   std::atomic<int> route{kRouteNone};
   std::mutex mutex;
   std::map<std::pair<int64_t, int64_t>, at::Tensor> x_rows;
 
-  MoEPlan(Weight a, Weight b, Weight ra, Weight rb, int64_t E_, int64_t hidden_, int64_t inter_, bool sorted_, bool pair_)
+  MoEPlan(Weight a, Weight b, Weight ra, Weight rb, int64_t E_, int64_t hidden_, int64_t inter_, bool sorted_13, bool sorted_2, bool pair_)
       : w13(std::move(a)), w2(std::move(b)), rows13(std::move(ra)), rows2(std::move(rb)), E(E_), hidden(hidden_),
-        inter(inter_), sorted_ok(sorted_), pair_ok(pair_) {}
+        inter(inter_), sorted13(L.gb_moe_fp4_pass_rows(&w13.w, w13.scales_e4m3, 1, E_) > 0 || sorted_13),
+        sorted2(L.gb_moe_fp4_pass_rows(&w2.w, w2.scales_e4m3, 1, E_) > 0 || sorted_2), pair_ok(pair_) {}
+
+  // both projections on the block-scaled FP4 tensor cores
+  bool fp4() const {
+    return L.gb_moe_fp4_pass_rows(&w13.w, w13.scales_e4m3, 1, E) > 0 && L.gb_moe_fp4_pass_rows(&w2.w, w2.scales_e4m3, 1, E) > 0;
+  }
 
   // token of every routed pair, one tensor per batch shape
   const int32_t* x_row(int64_t T, int64_t topk, const at::Tensor& like) {
@@ -339,6 +376,7 @@ struct MoEPlan {
     c.T = T; c.topk = topk; c.P = T * topk; c.rule = rule;
     c.stream = c10::cuda::getCurrentCUDAStream().stream();
     c.out = at::empty({T, hidden}, c.x.options());
+    const bool sorted_ok = sorted13 && sorted2;
     const int64_t prefill_min = sorted_ok ? lim.prefill_per_expert : std::min(lim.prefill_per_expert, lim.prefill_other);
     if (c.P >= prefill_min * E) prefill(c);
     else if (sorted_ok && c.P >= (pair_ok ? lim.sorted_per_expert * E : lim.sorted_other)) sorted(c);
@@ -356,21 +394,22 @@ struct MoEPlan {
     void* stream;
   };
 
-  struct Routing { int counts, offsets, order, pair_w, ws; int64_t ws_bytes; };
+  struct Routing { int counts, offsets, order, inv, pair_w, ws; int64_t ws_bytes; };
   Routing plan_routing(Arena& a, const Call& c) const {
     Routing r;
     r.counts = a.add(E * 4);
     r.offsets = a.add((E + 1) * 4);
     r.order = a.add(c.P * 4);
+    r.inv = a.add(c.P * 4);
     r.pair_w = a.add(c.P * 4);
     r.ws_bytes = L.gb_moe_route_workspace_bytes(c.T, c.topk, E);
     r.ws = a.add(r.ws_bytes);
     return r;
   }
   void run_routing(const Arena& a, const Routing& r, const Call& c) const {
-    check(L.gb_moe_route_ws(c.ids.data_ptr<int32_t>(), c.T, c.topk, E, 0, a.ptr<int32_t>(r.counts), a.ptr<int32_t>(r.offsets),
-                            a.ptr<int32_t>(r.order), c.tw.data_ptr<float>(), a.ptr<float>(r.pair_w),
-                            r.ws_bytes ? a.ptr(r.ws) : nullptr, r.ws_bytes, c.stream));
+    check(L.gb_moe_route_inv(c.ids.data_ptr<int32_t>(), c.T, c.topk, E, 0, a.ptr<int32_t>(r.counts), a.ptr<int32_t>(r.offsets),
+                             a.ptr<int32_t>(r.order), a.ptr<int32_t>(r.inv), c.tw.data_ptr<float>(), a.ptr<float>(r.pair_w),
+                             r.ws_bytes ? a.ptr(r.ws) : nullptr, r.ws_bytes, c.stream));
   }
   static void bucket(const Weight& w, const void* in, void* out, int64_t rows, const Call& c) {
     check(w.fp4() ? L.gb_fp4_act_qdq(in, out, rows, w.w.K, c.rule, c.stream)
@@ -442,23 +481,37 @@ struct MoEPlan {
     bucket(w2, a.ptr(hs), a.ptr(h), c.P, c);
   }
 
-  // Mid-size batches: the rows in expert order, then per projection one launch in which every
-  // (expert, 128-row tile) decodes its packed rows into tensor memory and multiplies them with the
-  // expert's rows on the tensor cores; the down projection stores its rows back in pair order.  The
-  // two stacks may be of different grids: each projection's rows go through its own grid's bucket.
+  // The rows in expert order, then per projection one launch in which every (expert, 128-row tile)
+  // decodes its packed rows into tensor memory and multiplies them with the expert's rows on the
+  // tensor cores; the down projection stores its rows back in pair order.  A stack of the fp4 grid runs
+  // on the block-scaled FP4 cores, its activations written as that kernel's operand in one launch (bucket
+  // and gather, or SwiGLU and bucket); the others bucket to bf16 rows.  The two stacks may be of
+  // different grids: each projection's rows go through its own grid's bucket.
   void sorted(Call& c) {
     Arena a;
     const Routing r = plan_routing(a, c);
-    const int xq = a.add(c.T * hidden * 2), xs = a.add(c.P * hidden * 2), h13 = a.add(c.P * 2 * inter * 2);
-    const int hs = a.add(w2.fp4() ? 0 : c.P * inter * 2), h = a.add(c.P * inter * 2), y = a.add(c.P * hidden * 2);
+    const int pr13 = L.gb_moe_fp4_pass_rows(&w13.w, w13.scales_e4m3, c.P, E), pr2 = L.gb_moe_fp4_pass_rows(&w2.w, w2.scales_e4m3, c.P, E);
+    const int64_t op13 = L.gb_moe_fp4_operand_bytes(c.P, E, hidden, pr13), op2 = L.gb_moe_fp4_operand_bytes(c.P, E, inter, pr2);
+    const int xq = a.add(pr13 ? 0 : c.T * hidden * 2), xs = a.add(pr13 ? op13 : c.P * hidden * 2), h13 = a.add(c.P * 2 * inter * 2);
+    const int hs = a.add(pr2 || w2.fp4() ? 0 : c.P * inter * 2), h = a.add(pr2 ? op2 : c.P * inter * 2), y = a.add(c.P * hidden * 2);
     a.alloc(c.x);
     run_routing(a, r, c);
-    const int32_t *off = a.ptr<int32_t>(r.offsets), *ord = a.ptr<int32_t>(r.order);
-    bucket(w13, c.x.data_ptr(), a.ptr(xq), c.T, c);
-    check(L.gb_moe_gather_rows(a.ptr(xq), x_row(c.T, c.topk, c.x), ord, off, E, c.P, hidden, a.ptr(xs), c.stream));
-    check(L.gb_moe_gemv_sorted(a.ptr(xs), &w13.w, w13.expert_stride, E, off, nullptr, c.P, a.ptr(h13), nullptr, c.stream));
-    swiglu(a, c, r, h13, hs, h);
-    check(L.gb_moe_gemv_sorted(a.ptr(h), &w2.w, w2.expert_stride, E, off, ord, c.P, a.ptr(y), nullptr, c.stream));
+    const int32_t *off = a.ptr<int32_t>(r.offsets), *ord = a.ptr<int32_t>(r.order), *ids = c.ids.data_ptr<int32_t>();
+    if (pr13) {
+      check(L.gb_moe_fp4_rows(c.x.data_ptr(), ids, a.ptr<int32_t>(r.inv), off, c.T, c.topk, E, hidden, pr13, c.rule, a.ptr(xs), c.stream));
+      check(L.gb_moe_gemv_fp4(a.ptr(xs), &w13.w, w13.scales_e4m3, w13.expert_stride, E, off, nullptr, c.P, pr13, a.ptr(h13), c.stream));
+    } else {
+      bucket(w13, c.x.data_ptr(), a.ptr(xq), c.T, c);
+      check(L.gb_moe_gather_rows(a.ptr(xq), x_row(c.T, c.topk, c.x), ord, off, E, c.P, hidden, a.ptr(xs), c.stream));
+      check(L.gb_moe_gemv_sorted(a.ptr(xs), &w13.w, w13.expert_stride, E, off, nullptr, c.P, a.ptr(h13), nullptr, c.stream));
+    }
+    if (pr2) {
+      check(L.gb_moe_fp4_swiglu_rows(a.ptr(h13), ids, ord, off, c.P, E, inter, pr2, c.rule, a.ptr(h), c.stream));
+      check(L.gb_moe_gemv_fp4(a.ptr(h), &w2.w, w2.scales_e4m3, w2.expert_stride, E, off, ord, c.P, pr2, a.ptr(y), c.stream));
+    } else {
+      swiglu(a, c, r, h13, hs, h);
+      check(L.gb_moe_gemv_sorted(a.ptr(h), &w2.w, w2.expert_stride, E, off, ord, c.P, a.ptr(y), nullptr, c.stream));
+    }
     combine(a.ptr(y), a.ptr<float>(r.pair_w), c, false);
     route = kMoeSorted;
   }
@@ -503,11 +556,12 @@ PYBIND11_MODULE(_gb_torch, m) {
   m.def("abi_version", [] { return GB_ABI_VERSION; });
   py::class_<Weight>(m, "Weight").def(py::init(&make_weight));
   py::class_<LinearPlan, std::shared_ptr<LinearPlan>>(m, "LinearPlan")
-      .def(py::init<Weight, at::Tensor, const Opt&>())
+      .def(py::init<Weight, at::Tensor, const Opt&, const std::vector<int64_t>&>())
       .def("__call__", &LinearPlan::forward, py::call_guard<py::gil_scoped_release>())
       .def_property_readonly("prefill_route", [](const LinearPlan& p) { return p.prefill_route.load(); });
   py::class_<MoEPlan, std::shared_ptr<MoEPlan>>(m, "MoEPlan")
-      .def(py::init<Weight, Weight, Weight, Weight, int64_t, int64_t, int64_t, bool, bool>())
+      .def(py::init<Weight, Weight, Weight, Weight, int64_t, int64_t, int64_t, bool, bool, bool>())
+      .def_property_readonly("fp4", &MoEPlan::fp4)
       .def("__call__", &MoEPlan::forward, py::call_guard<py::gil_scoped_release>())
       .def_property_readonly("route", [](const MoEPlan& p) { return p.route.load(); });
   m.def("shared_row", &shared_row);

@@ -146,12 +146,12 @@ class PrismaQuantCBLinearMethod(LinearMethodBase):
         cb_dev = (flat if self.is_fp4 else codec.flat_codebook_fp8(flat, self.prefix)).to(dev)
         compose = codec.build_compose_table(self._sub_table).to(dev) if self.is_v2 else None
         fmt = self.fmt
-        if (self.pad_two_tier_superblocks and fmt.is_fp4 and fmt.mode == "product" and fmt.k == 16 and fmt.n_sub == 2
-                and fmt.scale_coding == "v2" and cb_row_offset is None and N >= 128 and K >= 1024):
-            # 73-byte superblocks -> 80-byte slots, once: the rows become fetchable by TMA and every
-            # batch size runs on the tensor-core decode kernel (the bytes themselves stay packed)
-            fmt = fmt.padded(80)
-            qw = codec.pad_superblocks(qw, self.fmt.type_size, 80)
+        slot = codec.resident_slot(fmt) if self.pad_two_tier_superblocks else None
+        if slot is not None:
+            # 73-byte superblocks -> 80-byte slots (k = 16; the other widths alike), once: the rows become
+            # fetchable by TMA and every batch size runs on the tensor cores (the bytes stay packed)
+            fmt = fmt.padded(slot)
+            qw = codec.pad_superblocks(qw, self.fmt.type_size, slot)
         packed = codec.with_tail_slack(qw)
         layer.cb_qweight.data = packed          # same bytes, slack-backed storage
         ws = layer.weight_scale.data.float().contiguous() if not self.is_fp4 else None
@@ -167,7 +167,8 @@ class PrismaQuantCBLinearMethod(LinearMethodBase):
         layer._cb_slots = (kernels.new_tab_slots([layer._cb_weight])
                            if kernels.table_kernel_applies(layer._cb_weight) else None)
         layer._cb_plan = _native.host(f"{self.prefix}: CB Linear").LinearPlan(
-            kernels.host_weight(layer._cb_weight), layer._cb_workspace, layer._cb_slots)
+            kernels.host_weight(layer._cb_weight), layer._cb_workspace, layer._cb_slots,
+            widths if cb_row_offset is not None else [])
         layer._cb_route = _Route(layer._cb_plan, kernel="gemv_kernel", format=str(self.fmt), N=N, K=K)
 
     # ------------------------------------------------------------------ forward

@@ -32,6 +32,9 @@ PREFILL_MIN_PAIRS_PER_EXPERT = 384
 # on 32 experts of hidden 7168, intermediate 2048).
 SORTED_MIN_PAIRS_PER_EXPERT = 4
 SORTED_MIN_PAIRS_OTHER = 16
+# Stacks of the fp4 grid multiply the sorted rows on the block-scaled FP4 tensor cores, several times the
+# rate of the decoded bf16 stack's GEMM: they stay on that route.
+PREFILL_MIN_PAIRS_FP4 = 1 << 30
 # Stacks the sorted-rows kernel does not decode (per-role codebooks, other widths and modes) go from
 # the decode kernel's 16-row passes straight to the decoded stack + grouped GEMM, whose crossover
 # with the decode kernel was measured at ~800 tokens of 128 experts top-8.
@@ -201,11 +204,12 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
         p = getattr(layer, qw_name)
         dev = p.device
         qw = p.data
-        if (self.pad_two_tier_superblocks and fmt.is_fp4 and fmt.mode == "product" and fmt.k == 16 and fmt.n_sub == 2
-                and fmt.scale_coding == "v2" and len(blocks) == 1 and qw.shape[1] % 128 == 0 and k_in >= 256):
-            # 73-byte superblocks -> 80-byte slots, once (the sorted-rows kernel fetches rows by TMA)
-            qw = codec.pad_superblocks(qw, fmt.type_size, 80)
-            fmt = fmt.padded(80)
+        slot = codec.resident_slot(fmt) if self.pad_two_tier_superblocks and len(blocks) == 1 else None
+        if slot is not None and qw.shape[1] % 128 == 0:
+            # 73-byte superblocks -> 80-byte slots (k = 16; the other widths alike), once: the expert
+            # kernels fetch rows by TMA
+            qw = codec.pad_superblocks(qw, fmt.type_size, slot)
+            fmt = fmt.padded(slot)
         packed = codec.with_tail_slack(qw)
         p.data = packed
         cb_dev = (flat if fmt.is_fp4 else codec.flat_codebook_fp8(flat, self.prefix)).to(dev)
@@ -271,12 +275,14 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
                                           layer._cb_inter, "w2")
         layer._cb_E = layer.w13_cb_qweight.shape[0]
         w13, w2 = layer._cb_w13, layer._cb_w2
-        sorted_ok = (kernels.moe_gemv_sorted_applies(w13) and kernels.moe_gemv_sorted_applies(w2)
-                     and not (w2.fmt.is_fp4 and layer._cb_inter % 16))
+        sorted2 = kernels.moe_gemv_sorted_applies(w2) and not (w2.fmt.is_fp4 and layer._cb_inter % 16)
         pair_ok = kernels.pair_kernel_applies(w13) and kernels.pair_kernel_applies(w2)
         layer._cb_plan = _native.host(f"{self.prefix}: CB routed experts").MoEPlan(
             kernels.host_weight(w13), kernels.host_weight(w2), kernels.host_weight(kernels.stack_rows(w13)),
-            kernels.host_weight(kernels.stack_rows(w2)), layer._cb_E, layer._cb_hidden, layer._cb_inter, sorted_ok, pair_ok)
+            kernels.host_weight(kernels.stack_rows(w2)), layer._cb_E, layer._cb_hidden, layer._cb_inter,
+            kernels.moe_gemv_sorted_applies(w13), sorted2, pair_ok)
+        if layer._cb_plan.fp4 and self.prefill_min_pairs_per_expert == PREFILL_MIN_PAIRS_PER_EXPERT:
+            self.prefill_min_pairs_per_expert = PREFILL_MIN_PAIRS_FP4
         layer._cb_layer_id = ops.register_cb_layer(self, layer)
         print(f"[prismaquant-cb] {self.prefix}: decode=grouped-cuda (sm_100a) "
               f"w13={self.fmt13.grid}/k{self.fmt13.k} w2={self.fmt2.grid}/k{self.fmt2.k}",

@@ -144,6 +144,26 @@ GB_API int gb_gemv(const void* x_bf16, int64_t M, const gb_weight* w, int act, i
  * format and layout (up to 128).  No counterpart in the reference. */
 GB_API int gb_gemv_row_batch_max(const gb_weight* w);
 
+/* What a caller that prepared a layer once knows about it beyond gb_weight. */
+#define GB_MAX_ROLES 8
+typedef struct gb_hints {
+  int32_t scales_e4m3;            /* two-tier scales: every composed scale is an exact E4M3 value (gb_scales_e4m3) */
+  int32_t n_roles;                /* parts of a fused matrix that carry their own codebook (0 or 1: one codebook);
+                                     part i uses codebook block i, as cb_row_offset says per row */
+  int64_t role_rows[GB_MAX_ROLES];
+} gb_hints;
+/* Clears *flag (device) and raises it when a scale of rows [0, rows) of a two-tier weight is not an
+ * exact E4M3 value.  Run once after loading.  No counterpart in the reference. */
+GB_API int gb_scales_e4m3(const gb_weight* w, int64_t rows, int32_t* flag, void* stream);
+/* gb_gemv with the grid's own activation bucket fused and with hints: the fp4 formats the hints
+ * qualify - the literal one, the two-tier product formats k = 12, 16, 20, 24 in superblock slots
+ * of a multiple of sixteen bytes, one codebook per role or for all rows - run on the block-scaled
+ * FP4 tensor cores (tcgen05 kind::mxf4nvf4): packed rows decoded to E2M1 nibbles in tensor memory,
+ * activations split exactly into three E2M1 x UE4M3 terms, fp32 accumulate, same results as gb_gemv up to the
+ * order of the sum.  Everything else goes to gb_gemv.  Replaces the same reference entries as gb_gemv. */
+GB_API int gb_gemv_hinted(const void* x_bf16, int64_t M, const gb_weight* w, const gb_hints* hints, int scale_rule,
+                          void* y_bf16, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* Row counts at which gb_gemv changes kernel for the literal format: up to `dot_rows` rows run one
  * inner-product-table GEMV per row (default 4, at most 8), from `umma_min` rows on the tensor-core
  * decode kernel (default 5; 129 switches that kernel off for every format).  0 restores a default.  Process-wide; for tests and tuning.  No
@@ -275,6 +295,12 @@ GB_API int gb_moe_route_ws(const int32_t* topk_ids, int64_t T, int64_t topk, int
                            int32_t* counts, int32_t* offsets, int32_t* order, const float* topk_weights,
                            float* pair_w, void* workspace, int64_t ws_bytes, void* stream);
 
+/* gb_moe_route_ws that also writes the inverse permutation: inv[p] = sorted position of pair p (unset for
+ * a dropped pair). */
+GB_API int gb_moe_route_inv(const int32_t* topk_ids, int64_t T, int64_t topk, int64_t E, int64_t expert_base,
+                            int32_t* counts, int32_t* offsets, int32_t* order, int32_t* inv, const float* topk_weights,
+                            float* pair_w, void* workspace, int64_t ws_bytes, void* stream);
+
 /* Grouped GEMV over routed pairs; replaces cb_moe_gemv_fp8 / cb_moe_gemv_fp4_v2 /
  * cb_moe_gemv_v2 (gridbook/csrc/cb_gemv.cu:1210-1681,1873-2138; gridbook/csrc/cb_gemv_v2.cu:233-366).
  * `w` describes ONE expert's matrix; expert e starts at qw + e*expert_stride bytes and
@@ -311,6 +337,24 @@ GB_API int gb_moe_gemv(const void* x_bf16, const int32_t* x_row, const gb_weight
 GB_API int gb_moe_gemv_sorted(const void* x_sorted_bf16, const gb_weight* w, int64_t expert_stride, int64_t E,
                               const int32_t* seg_offsets, const int32_t* row_map, int64_t P, void* y_bf16,
                               const gb_peer_rows* y_rows, void* stream);
+
+/* The grouped linear of fp4 stacks on the block-scaled FP4 tensor cores (see gb_gemv_hinted), same
+ * results as gb_moe_gemv_sorted on bucketed rows up to the order of the sum.  gb_moe_fp4_pass_rows
+ * says how many routed rows a launch takes per pass over an expert (0: not a stack this kernel takes);
+ * gb_moe_fp4_operand_bytes sizes the operand of the activations.  gb_moe_fp4_rows writes it from
+ * the T token rows (bucket and gather in one launch; `inv` from gb_moe_route_inv), gb_moe_fp4_swiglu_rows
+ * from the sorted [gate | up] rows (SwiGLU, bucket); gb_moe_gemv_fp4 multiplies: y[P, N], row j of the sorted
+ * order at row_map[j] (or j).  Replace the same reference entries as gb_moe_gemv_sorted. */
+GB_API int gb_moe_fp4_pass_rows(const gb_weight* w, int scales_e4m3, int64_t P, int64_t E);
+GB_API int64_t gb_moe_fp4_operand_bytes(int64_t P, int64_t E, int64_t K, int pass_rows);
+GB_API int gb_moe_fp4_rows(const void* x_bf16, const int32_t* topk_ids, const int32_t* inv, const int32_t* seg_offsets, int64_t T,
+                           int64_t topk, int64_t E, int64_t K, int pass_rows, int scale_rule, void* operand, void* stream);
+GB_API int gb_moe_fp4_swiglu_rows(const void* h_bf16, const int32_t* topk_ids, const int32_t* order, const int32_t* seg_offsets,
+                                  int64_t P, int64_t E, int64_t inter, int pass_rows, int scale_rule, void* operand,
+                                  void* stream);
+GB_API int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, int64_t expert_stride, int64_t E,
+                           const int32_t* seg_offsets, const int32_t* row_map, int64_t P, int pass_rows, void* y_bf16,
+                           void* stream);
 
 /* The same routed projection for SMALL batches of the literal format (fp4 grid, full mode,
  * k = 8, E4M3-direct scales, one codebook per stack): every routed pair p is its own M = 1 linear

@@ -1,0 +1,157 @@
+"""The decode-batch kernel on the block-scaled FP4 tensor cores: the exact three-term split of the bucketed
+activations, edges of the row, tile, slice and pass counts, codebooks that change with the role, scales
+of either sign and scales that are no E4M3 value (which must take the other kernel), dense and per expert."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import cb_oracle as O
+from oracle import oracle_kwargs
+from tests.helpers import assert_close_bf16, f32_of, oracle_linear
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    from gridbook_b200 import _native
+    _native.prepare(0)
+    return torch.device("cuda:0")
+
+
+def _fmt(name):
+    from gridbook_b200 import formats as F
+    if name == "lit":
+        return F.NVFP4_LITERAL
+    return F.CBFormat("fp4", int(name[1:]), n_sub=2, scale_coding="v2")
+
+
+def _tables(fmt, flat):
+    out, pos = [], 0
+    for r, d in fmt.table_shapes():
+        out.append(torch.from_numpy(flat[pos:pos + r * d].reshape(r, d).copy()))
+        pos += r * d
+    return out
+
+
+def _linear(fmt, d, parts, dev, **kw):
+    from gridbook_b200.linear import CBLinear
+    n = fmt.codebook_elems()
+    books = [_tables(fmt, d["cb"][i * n:(i + 1) * n]) for i in range(d["cb"].size // n)]
+    lin = CBLinear(fmt, d["K"], parts, books, global_scale=d["global_scale"] or 1.0, **kw)
+    return lin.load(torch.from_numpy(d["qw"]), None, dev)
+
+
+def _wide_rows(M, K, seed):
+    """Groups from far below to far above the row's typical magnitude, a zero group and a zero row."""
+    rng = np.random.default_rng(seed)
+    x = rng.standard_normal((M, K // 16, 16)).astype(np.float32)
+    x *= np.exp2(rng.integers(-9, 3, (M, K // 16, 1))).astype(np.float32)
+    x[:, 3] = 0.0
+    x = x.reshape(M, K)
+    if M > 2:
+        x[M // 2] = 0.0
+    return O.bf16_round(x)
+
+
+@pytest.mark.parametrize("name", ["lit", "k12", "k16", "k20", "k24"])
+@pytest.mark.parametrize("M,N,K", [(2, 64, 256), (5, 129, 512), (8, 200, 2048), (9, 384, 1280), (16, 640, 5120), (3, 1024, 17408)])
+def test_decode_rows_match_the_oracle(dev, name, M, N, K):
+    from gridbook_b200 import _native, synth
+    fmt = _fmt(name)
+    d = synth.make_linear(fmt, N, K, seed=M + N, global_scale=1.0 / 448.0 if name == "lit" else None, super_span=None)
+    lin = _linear(fmt, d, [N], dev)
+    for x in (synth.make_activations(M, K, seed=K), _wide_rows(M, K, M)):
+        y = lin(synth.bf16_tensor(x, dev))
+        torch.cuda.synchronize()
+        assert _native.device_status(0) == 0
+        assert_close_bf16(f32_of(y), oracle_linear(x, d), f"{name} {M}x{N}x{K}", atol_rel=1e-6)
+
+
+@pytest.mark.parametrize("name", ["lit", "k16"])
+@pytest.mark.parametrize("M", [1, 15, 17, 31, 32, 33, 48, 64, 65, 100, 128])
+def test_row_counts_past_sixteen(dev, name, M):
+    from gridbook_b200 import _native, kernels, synth
+    fmt = _fmt(name)
+    N, K = 320, 1536
+    d = synth.make_linear(fmt, N, K, seed=M, global_scale=1.0 / 448.0 if name == "lit" else None)
+    lin = _linear(fmt, d, [N], dev)
+    if M > kernels.row_batch_max_rows(lin._cb_weight):
+        pytest.skip("past the decode batches of this format")
+    x = _wide_rows(M, K, M)
+    y = lin(synth.bf16_tensor(x, dev))
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    assert_close_bf16(f32_of(y), oracle_linear(x, d), f"{name} M={M}", atol_rel=1e-6)
+
+
+@pytest.mark.parametrize("name", ["lit", "k16", "k20"])
+@pytest.mark.parametrize("parts,K", [([96, 96], 1024), ([256, 64, 64], 2560), ([40, 200, 130, 14], 512), ([17408, 17408], 256)])
+def test_roles_with_their_own_codebooks(dev, name, parts, K):
+    from gridbook_b200 import _native, synth
+    fmt = _fmt(name)
+    N, M = sum(parts), 7
+    d = synth.make_linear(fmt, N, K, seed=N, n_books=len(parts))
+    d["cb_row_offset"] = np.repeat(np.arange(len(parts)), parts).astype(np.int32) * fmt.codebook_elems()
+    lin = _linear(fmt, d, parts, dev)
+    x = synth.make_activations(M, K, seed=5)
+    y = lin(synth.bf16_tensor(x, dev))
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    assert_close_bf16(f32_of(y), oracle_linear(x, d), f"{name} roles {parts}")
+
+
+def test_negative_scale_bytes_and_non_finite_rows(dev):
+    from gridbook_b200 import synth
+    fmt = _fmt("lit")
+    M, N, K = 6, 256, 1024
+    d = synth.make_linear(fmt, N, K, seed=4)
+    blk = d["qw"].reshape(N, K // 256, 48)
+    blk[:, :, 32:] |= (np.random.default_rng(1).integers(0, 2, (N, K // 256, 16)) * 128).astype(np.uint8)
+    lin = _linear(fmt, d, [N], dev)
+    x = synth.make_activations(M, K, seed=1)
+    assert_close_bf16(f32_of(lin(synth.bf16_tensor(x, dev))), oracle_linear(x, d), "negative scales")
+    x[2, 40] = np.nan
+    x[4, 500] = np.inf
+    y = f32_of(lin(synth.bf16_tensor(x, dev)))
+    assert np.isnan(y[2]).all() and np.isnan(y[4]).all() and np.isfinite(y[[0, 1, 3, 5]]).all()
+    keep = [0, 1, 3, 5]
+    assert_close_bf16(y[keep], oracle_linear(x[keep], d), "finite rows beside them")
+
+
+def test_scales_off_the_e4m3_grid_take_the_other_kernel(dev):
+    """Super exponents past the E4M3 range: the block-scaled operand cannot hold them."""
+    from gridbook_b200 import synth
+    fmt = _fmt("k16")
+    M, N, K = 4, 256, 1024
+    d = synth.make_linear(fmt, N, K, seed=8)
+    d["qw"].reshape(N, K // 256, 73)[:, :, 64] = np.random.default_rng(2).choice([100, 126, 140], (N, K // 256)).astype(np.uint8)
+    lin = _linear(fmt, d, [N], dev)
+    x = synth.make_activations(M, K, seed=3)
+    assert_close_bf16(f32_of(lin(synth.bf16_tensor(x, dev))), oracle_linear(x, d), "scales off the grid")
+
+
+@pytest.mark.parametrize("f13,f2", [("lit", "lit"), ("k16", "k16"), ("k20", "lit"), ("k12", "k24")])
+@pytest.mark.parametrize("T", [3, 40, 150, 700])
+def test_routed_layer_matches_the_loop_chain(dev, f13, f2, T):
+    """Experts without rows, with a few and with several passes; a dropped (-1) slot."""
+    from gridbook_b200 import _native, synth
+    from gridbook_b200.moe import CBMoE
+    fmt13, fmt2 = _fmt(f13), _fmt(f2)
+    E, hidden, inter, topk = 8, 512, 256, 2
+    w13d, w2d = synth.make_moe(fmt13, fmt2, E, hidden, inter, seed=T)
+    ids, tw = synth.make_routing(T, E - 1, topk, seed=T)
+    ids[2, 1] = -1
+    x = synth.make_activations(T, hidden, seed=T + 1)
+    ref = O.moe_loop_chain(x, np.where(ids < 0, 0, ids), np.where(ids < 0, 0.0, tw).astype(np.float32), w13d, w2d, E=E,
+                           hidden=hidden, inter=inter, fmt13=oracle_kwargs(fmt13), fmt2=oracle_kwargs(fmt2), scale_rule="recip")
+    moe = CBMoE(fmt13, fmt2, E, hidden, inter, _tables(fmt13, w13d["cb"]), _tables(fmt2, w2d["cb"]))
+    moe.load(torch.from_numpy(w13d["qw"]), torch.from_numpy(w2d["qw"]), None, None, dev)
+    moe.method.sorted_min_pairs_per_expert = 0
+    moe.method.sorted_min_pairs_other = 0
+    got = f32_of(moe(synth.bf16_tensor(x, dev), torch.from_numpy(tw).to(dev), torch.from_numpy(ids).to(dev)))
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    assert "sorted rows" in moe._cb_route
+    assert np.linalg.norm(got - ref) / np.linalg.norm(ref) <= 3e-3
+    assert np.abs(got - ref).max() <= 2e-2 * max(1.0, np.abs(ref).max())
