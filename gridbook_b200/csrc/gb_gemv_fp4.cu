@@ -26,7 +26,8 @@
 // the rows kernel below writes it swizzled, scale factors in front), sixteen warps decode.  A UNIT is
 // one superblock of K (256 weights): unit u is decoded by warpgroup u mod 4 into operand buffer u mod 4
 // of TENSOR MEMORY (32 columns of nibbles, 16 of scale factors) and multiplied by four MMAs of K = 64
-// (or eight); the issuing thread copies the activations' scale factors to tensor memory itself.
+// (or eight).  The decoders also move the activations' scale factors to tensor memory: tcgen05.cp takes its
+// issuing thread a hundred clocks each, four or eight per unit.
 // Bound by the decoders' instructions and the latency of the hand-overs between the roles
 // (a tcgen05.mma takes 72 clocks of its issuer whatever its N up to 128, a commit reaches its waiter
 // after about 250), then by shared-memory lookups (4 bytes per codeword from 32 copies: no conflicts).
@@ -43,7 +44,7 @@ namespace {
 
 constexpr int kBM = 128;
 constexpr int kDecWarps = 16;
-constexpr int kCtlWarps = 6;                              // packed rows, activations, up to four MMA issuers
+constexpr int kCtlWarps = 8;                              // packed rows, activations, up to four MMA issuers, two idle
 constexpr int kThreads = 32 * (kCtlWarps + kDecWarps);
 constexpr int kMaxRows = 64;                              // activation rows per pass (three columns each)
 constexpr int kMaxRaw = 4, kMaxX = 8;
@@ -89,8 +90,8 @@ struct Fp4Params {
   int n_sb, units;           // superblocks per row / per K slice (the last slice may have fewer)
   int slices;                // = cluster size along y
   int pass_rows;             // most rows per pass (dense: M)
-  int x_stages, raw_stages;  // ring depths: 4 or 8, 2 to 4
-  uint32_t x_off, raw_off[kMaxRaw], misc_off, red_off;
+  int x_stages, raw_stages;  // ring depths: 4 or 8, 2 or 4
+  uint32_t x_off, raw_off, misc_off, red_off;
   const uint8_t* xop;        // activation operand: [tile][superblock][scale factors | codes]
   int64_t x_unit;            // bytes of one superblock of it
   const float* x_scale;      // [tile][pass_rows] power of two of every row
@@ -106,12 +107,14 @@ struct Fp4Params {
   int tiles_n;
 };
 
-// Columns.  Narrow (up to 16 rows per pass): column t * R + m of term t of row m, one MMA of N = 3 R
-// rounded up to 16.  Wide: R code rows of q and R of the correction, scale factors [hi | dlt] and [lo].
-// R = rows rounded up to 8 (narrow) or 16.
+// Columns.  Narrow (up to 16 rows per pass): term t of row m in column 12 (m / 4) + 4 t + m % 4, so that the
+// twelve columns of four rows are read out together; one MMA of N = 3 R rounded up to 16.  Wide: R code
+// rows of q, then R of the correction, scale factors [hi | dlt] and [lo].  R = rows rounded up to 8
+// (narrow) or 16.
 constexpr int kNarrowRows = 16;
 __host__ __device__ constexpr bool is_wide(int pass_rows) { return pass_rows > kNarrowRows; }
 __host__ __device__ constexpr int term_rows(bool wide, int rows) { return wide ? (rows + 15) / 16 * 16 : (rows + 7) / 8 * 8; }
+__host__ __device__ constexpr int narrow_col(int t, int m) { return 12 * (m >> 2) + 4 * t + (m & 3); }
 __host__ __device__ constexpr int mma_cols(bool wide, int rows) {
   return wide ? 2 * term_rows(true, rows) : (3 * term_rows(false, rows) + 15) / 16 * 16;
 }
@@ -184,14 +187,6 @@ GB_DEVINL void umma_fp4_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, u
       "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], [%1], %2, %3, [%5], [%6], p;\n}\n"
       ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)acc), "r"(sfa), "r"(sfb) : "memory");
 }
-// 512 bytes of scale factors (128 columns x 4 groups) from shared to tensor memory, into all four lane
-// quarters; in order with the MMAs the same thread issues.
-GB_DEVINL void copy_sf(uint32_t taddr, uint32_t smem_addr) {
-  uint64_t d = (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)(128u >> 4) << 32;                        // eight-row groups of 16-byte rows, no swizzle
-  d |= (uint64_t)1 << 46;
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(d) : "memory");
-}
 GB_DEVINL void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -201,13 +196,23 @@ GB_DEVINL void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
       ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
         "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
+GB_DEVINL void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
+        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
+        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
+}
 GB_DEVINL void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
 }
-GB_DEVINL void tmem_ld4(uint32_t taddr, uint32_t (&v)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr));
+GB_DEVINL void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+                 "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(taddr));
 }
 GB_DEVINL void cluster_sync() {
   __syncwarp();
@@ -245,6 +250,12 @@ GB_DEVINL uint32_t nib4(uint2 w) {
   }
   return r;
 }
+
+// Who waits for a raw stage.  A warp must see every phase of a barrier it waits for (a parity wait cannot
+// tell a phase from the one two before).  With two superblocks per stage, or four stages, the stages of
+// a slot always hold units of the same warpgroups, so only those wait and hand the stage back; the wide
+// formats (one superblock per stage, room for two stages) let every warpgroup see every stage.
+template <int F> constexpr bool kAllSee = Fmt<F>::kSbPerStage == 1;
 
 // Lookup tables of one codebook, built by the 512 decoder threads.
 template <int F>
@@ -314,7 +325,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const uint32_t win = gb_smem_u32(smem_raw) & 0xFF000000u;
   const uint32_t misc = p.misc_off | win;
   const uint32_t raw_full = misc, raw_empty = misc + 8 * kMaxRaw;
-  // per unit slot: activations landed / operand complete (decoded, and narrow: landed) / multiplied
+  // per unit slot: activations landed / operand complete / multiplied
   const uint32_t x_full = misc + 64, full = x_full + 8 * kMaxX, done = full + 8 * kMaxX;
   const uint32_t acc_full = done + 8 * kMaxX, acc_empty = acc_full + 8, red_full = acc_full + 16;
   const uint32_t slot_addr = acc_full + 24;
@@ -336,6 +347,8 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const uint32_t acc_stride = wide ? 128u : 64u;
   const uint32_t buf_col0 = wide ? 192u : 256u, buf_stride = wide ? 80u : 64u;
   const int sfx = sf_bytes(wide);
+  const int raw_mask = p.raw_stages - 1, raw_log = p.raw_stages == 4 ? 2 : 1;
+  const uint32_t raw_ring = p.raw_off | win;
   const int x_mask = p.x_stages - 1, x_log = p.x_stages == 8 ? 3 : 2;
   const uint32_t x_ring = p.x_off | win, x_stage = (uint32_t)p.x_unit;
 
@@ -347,11 +360,11 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxRaw; ++s) {
       mbar_init(raw_full + 8 * s, 1);
-      mbar_init(raw_empty + 8 * s, kDecWarps);
+      mbar_init(raw_empty + 8 * s, kAllSee<F> ? kDecWarps : 4 * T::kSbPerStage);
     }
     for (int s = 0; s < kMaxX; ++s) {
       mbar_init(x_full + 8 * s, 1);
-      mbar_init(full + 8 * s, wide ? 4 : 5);
+      mbar_init(full + 8 * s, 4);                            // the four warps that decode the unit
       mbar_init(done + 8 * s, wide ? 2 : 1);
     }
     mbar_init(acc_full, (uint32_t)n_iss);
@@ -360,7 +373,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     *abort_flag = 0;
     gb_fence_barrier_init();
   }
-  if (warp == 2) {
+  if (warp == 4) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_addr), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -407,16 +420,16 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   if (warp == 0) {
     // ------------------------- packed weight rows -------------------------
     if (lane == 0) {
-      int rs = 0;
-      uint32_t ph = 1;
+      int n = 0;                                           // stages since the start
       for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
         const Tile R = tile_at(t);
         for (int pass = 0; pass < R.n_pass; ++pass)
-          for (int u = 0; u < units; u += T::kSbPerStage) {
-            wait(raw_empty + 8 * rs, ph, abort_flag, p.status, 42);
-            mbar_expect(raw_full + 8 * rs, G::kBoxBytes);
-            tma_load_2d(p.raw_off[rs] | win, &map_w, (sb_begin + u) * T::kSb, R.w_row0, raw_full + 8 * rs);
-            if (++rs == p.raw_stages) { rs = 0; ph ^= 1; }
+          for (int u = 0; u < units; u += T::kSbPerStage, ++n) {
+            const int s = n & raw_mask;
+            wait(raw_empty + 8 * s, ((uint32_t)(n >> raw_log) & 1u) ^ 1u, abort_flag, p.status, 42);
+            if (*abort_flag) continue;                     // no copy may be in flight when the CTA leaves
+            mbar_expect(raw_full + 8 * s, G::kBoxBytes);
+            tma_load_2d(raw_ring + (uint32_t)s * G::kBoxBytes, &map_w, (sb_begin + u) * T::kSb, R.w_row0, raw_full + 8 * s);
           }
       }
     }
@@ -424,7 +437,6 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     // ------------------------- activation operand --------------------------
     if (lane == 0) {
       gb_pdl_wait();
-      const uint32_t land = wide ? x_full : full;
       int g = 0;                                           // units since the start, over all tiles and passes
       for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
         const Tile R = tile_at(t);
@@ -435,8 +447,9 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
           for (int u = 0; u < units; ++u, ++g, src += p.x_unit) {
             const int s = g & x_mask;
             wait(done + 8 * s, ((uint32_t)(g >> x_log) & 1u) ^ 1u, abort_flag, p.status, 43);
-            mbar_expect(land + 8 * s, bytes);
-            bulk_load(x_ring + (uint32_t)s * x_stage, src, bytes, land + 8 * s);
+            if (*abort_flag) continue;
+            mbar_expect(x_full + 8 * s, bytes);
+            bulk_load(x_ring + (uint32_t)s * x_stage, src, bytes, x_full + 8 * s);
           }
         }
       }
@@ -468,14 +481,8 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             const uint32_t a = tmem_base + buf_col0 + (uint32_t)(u & 3) * buf_stride, off = (uint32_t)s * x_stage;
             const uint64_t db = db0 + (uint64_t)(off >> 4);
             wait(full + 8 * s, (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 45);
+            if (*abort_flag) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (!wide) {
-              // The activations' scale factors, in order in front of the MMAs that read them; what they
-              // overwrite was read by this thread's MMAs of four units ago, which have completed (the
-              // decoders waited for them).
-#pragma unroll
-              for (int k = 0; k < 4; ++k) copy_sf(a + 48u + 4u * k, x_ring + off + 512u * k);
-            }
 #pragma unroll
             for (int k = 0; k < 4; ++k)
               umma_fp4_ts(acc, a + 8u * k, db + (uint64_t)(2 * k), idesc, a + 32u + 4u * k, a + sf_col + 4u * k, u > u_first || k > 0);
@@ -501,8 +508,9 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       }
     }
     bool waited = false;
-    int rs = 0, item = 0, g0 = 0;
-    uint32_t rph = 0, flip = 0;
+    int item = 0, g0 = 0, n0 = 0;                            // items, units and raw stages so far
+    uint32_t flip = 0;
+    const int stages = (units + T::kSbPerStage - 1) / T::kSbPerStage;
     for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
       const Tile R = tile_at(t);
       if (R.n_pass == 0) continue;
@@ -513,41 +521,40 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
       }
       if (!waited) { gb_pdl_wait(); waited = true; }         // y may still be read by the launch ahead
-      for (int pass = 0; pass < R.n_pass; ++pass, ++item, g0 += units) {
+      for (int pass = 0; pass < R.n_pass; ++pass, ++item, g0 += units, n0 += stages) {
         const int rows = min(p.pass_rows, R.cnt - pass * p.pass_rows);
         const float* xsc = p.x_scale + (int64_t)(R.x_tile + pass) * p.pass_rows;
         const float xs0 = lane < rows ? xsc[lane] : 0.0f, xs1 = lane + 32 < rows ? xsc[lane + 32] : 0.0f;
-        for (int u0 = 0; u0 < units; u0 += T::kSbPerStage) {
-          wait(raw_full + 8 * rs, rph, abort_flag, p.status, 47);
-          const int i = (wg - u0) & 3;                       // this warpgroup's superblock of the stage, if any
-          if (i < T::kSbPerStage && u0 + i < units) {
-            const uint32_t stage = p.raw_off[rs] | win;
-            const uint32_t rp = stage + (uint32_t)row * G::kPitch + (uint32_t)(i * T::kSb);
-            uint32_t v[32], sfa[16];
+#pragma unroll 1
+        for (int u = kAllSee<F> ? 0 : wg; u < stages * T::kSbPerStage; u += kAllSee<F> ? 1 : 4) {
+          const int n = n0 + u / T::kSbPerStage, rs = n & raw_mask;
+          if (kAllSee<F> && (u & 3) != wg) {
+            wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
+            if (lane == 0) mbar_arrive(raw_empty + 8 * rs);
+            continue;
+          }
+          if (u < units) {
+            wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
+            const uint32_t stage = raw_ring + (uint32_t)rs * G::kBoxBytes + (uint32_t)(u % T::kSbPerStage) * T::kSb;
+            const uint32_t rp = stage + (uint32_t)row * G::kPitch;
+            uint32_t v[32], sfa[16], sg, sg_step;            // sfa: scale words of rows lane, lane + 32, lane + 64, lane + 96
             if constexpr (F == kLit) {
-              const uint4 c0 = lds128(rp), c1 = lds128(rp + 16);
+              const uint4 c0 = lds128(rp), c1 = lds128(rp + 16), own = lds128(rp + 32);
               const uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-              const uint32_t sg = stage + (uint32_t)lane * G::kPitch + (uint32_t)(i * T::kSb) + 32u;
-              uint32_t any = 0;
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {                  // scale bytes of rows lane, lane + 32, lane + 64, lane + 96
-                const uint4 s = lds128(sg + (uint32_t)(j * 32) * G::kPitch);
-                sfa[j] = s.x; sfa[4 + j] = s.y; sfa[8 + j] = s.z; sfa[12 + j] = s.w;
-                any |= s.x | s.y | s.z | s.w;
-              }
 #pragma unroll
               for (int c = 0; c < 32; ++c) v[c] = codeword<F>(cw, c, lane4);
-              if (__builtin_expect(any & 0x80808080u, 0)) {  // scale factors carry no sign: it moves into the nibbles
-                const uint4 own = lds128(rp + 32);
+              if (__builtin_expect((own.x | own.y | own.z | own.w) & 0x80808080u, 0)) {
+                // scale factors carry no sign: it moves into the nibbles
                 const uint32_t os[4] = {own.x, own.y, own.z, own.w};
 #pragma unroll
                 for (int g = 0; g < 16; ++g) {
                   const uint32_t neg = (os[g >> 2] >> (8 * (g & 3))) & 0x80u ? 0x88888888u : 0u;
                   v[2 * g] ^= neg;
                   v[2 * g + 1] ^= neg;
-                  sfa[g] &= 0x7F7F7F7Fu;
                 }
               }
+              sg = stage + (uint32_t)lane * G::kPitch + 32u;
+              sg_step = 32u * G::kPitch;
             } else {
               uint32_t w[T::kSb / 4];
 #pragma unroll
@@ -555,52 +562,65 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 const uint4 x = lds128(rp + 16u * q);
                 w[4 * q] = x.x; w[4 * q + 1] = x.y; w[4 * q + 2] = x.z; w[4 * q + 3] = x.w;
               }
+              __syncwarp();
+              if (lane == 0) mbar_arrive(raw_empty + 8 * rs);  // the whole superblock is in registers
               // the super byte sits right behind the 4k index bytes, then sixteen nibbles
               const uint4 tb = lds128(scale_tab + (w[F] & 0xFFu) * 16u);
-              const uint32_t n0 = __funnelshift_r(w[F], w[F + 1], 8), n1 = __funnelshift_r(w[F + 1], w[F + 2], 8);
+              const uint32_t n0s = __funnelshift_r(w[F], w[F + 1], 8), n1s = __funnelshift_r(w[F + 1], w[F + 2], 8);
               // two buffers: a warp that writes the next unit's bytes has passed this unit's barrier,
               // which no warp reaches before it has read the unit before
               const uint32_t st = sfa_stage + (uint32_t)(wg * 4096) + flip * 2048u;
               flip ^= 1u;
               sts128(st + (uint32_t)(row * 16),
-                     make_uint4(four_scales(tb, n0), four_scales(tb, n0 >> 16), four_scales(tb, n1), four_scales(tb, n1 >> 16)));
+                     make_uint4(four_scales(tb, n0s), four_scales(tb, n0s >> 16), four_scales(tb, n1s), four_scales(tb, n1s >> 16)));
 #pragma unroll
               for (int c = 0; c < 32; ++c) v[c] = codeword<F>(w, c, lane4);
               asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory");   // the four warps of this warpgroup
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint4 s = lds128(st + (uint32_t)((lane + 32 * j) * 16));
-                sfa[j] = s.x; sfa[4 + j] = s.y; sfa[8 + j] = s.z; sfa[12 + j] = s.w;
-              }
+              sg = st + (uint32_t)lane * 16u;
+              sg_step = 512u;
             }
             // The buffer's last unit has been multiplied (at the start of an item all have).  The slot's
             // next completion is a later unit of this warpgroup, so it cannot run ahead of this wait.
-            const int u = u0 + i, g = g0 + u;
+            const int g = g0 + u;
             if (u >= 4) wait(done + 8 * ((g - 4) & x_mask), (uint32_t)((g - 4) >> x_log) & 1u, abort_flag, p.status, 48);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tmem_st16(buf, *reinterpret_cast<const uint32_t(*)[16]>(&v[0]));
-            tmem_st16(buf + 16u, *reinterpret_cast<const uint32_t(*)[16]>(&v[16]));
+            tmem_st32(buf, v);
+            uint32_t any = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 s = lds128(sg + (uint32_t)j * sg_step);
+              sfa[j] = s.x; sfa[4 + j] = s.y; sfa[8 + j] = s.z; sfa[12 + j] = s.w;
+              any |= s.x | s.y | s.z | s.w;
+            }
+            if (F == kLit && __builtin_expect(any & 0x80808080u, 0)) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) sfa[j] &= 0x7F7F7F7Fu;
+            }
             tmem_st16(buf + 32u, sfa);
+            // the activations' scale factors: atom k is what MMA k reads, its line l the four columns of
+            // lane l of every quarter
+            wait(x_full + 8 * (g & x_mask), (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 46);
+            const uint32_t sx = x_ring + (uint32_t)(g & x_mask) * x_stage + (uint32_t)lane * 16u;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const uint4 s = lds128(sx + 512u * k);
+              sfa[4 * k] = s.x; sfa[4 * k + 1] = s.y; sfa[4 * k + 2] = s.z; sfa[4 * k + 3] = s.w;
+            }
+            tmem_st16(buf + 48u, sfa);
             if (wide) {
-              // the activations' two sets of scale factors (the two issuers have no time for the copies)
-              wait(x_full + 8 * (g & x_mask), (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 46);
 #pragma unroll
-              for (int q = 0; q < 2; ++q) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  const uint4 s = lds128(x_ring + (uint32_t)(g & x_mask) * x_stage + (uint32_t)(q * 2048 + k * 512 + lane * 16));
-                  sfa[4 * k] = s.x; sfa[4 * k + 1] = s.y; sfa[4 * k + 2] = s.z; sfa[4 * k + 3] = s.w;
-                }
-                tmem_st16(buf + 48u + 16u * q, sfa);
+              for (int k = 0; k < 4; ++k) {
+                const uint4 s = lds128(sx + 2048u + 512u * k);
+                sfa[4 * k] = s.x; sfa[4 * k + 1] = s.y; sfa[4 * k + 2] = s.z; sfa[4 * k + 3] = s.w;
               }
+              tmem_st16(buf + 64u, sfa);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * (g & x_mask));
           }
-          if (lane == 0) mbar_arrive(raw_empty + 8 * rs);
-          if (++rs == p.raw_stages) { rs = 0; rph ^= 1; }
+          if ((F == kLit || u >= units) && lane == 0) mbar_arrive(raw_empty + 8 * rs);   // also for a stage's missing second superblock
         }
 
         // ------------------------- read-out ------------------------------------
@@ -641,26 +661,26 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
               emit(c * 8 + i, fmaf(__uint_as_float(e[i]), 0x1p-7f, fmaf(__uint_as_float(l[i]), 0x1p-4f, __uint_as_float(h[i]))));
           }
         } else if (wg * 4 < rows) {
-          // four rows per warpgroup, all loads in flight; issuers without a unit leave their accumulator untouched
+          // four rows per warpgroup; issuers without a unit leave their accumulator untouched
           const int accs = min(4, units);
-          uint32_t h[4][4], l[4][4], e[4][4];
+          float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            const uint32_t at = lane_base + (uint32_t)min(a, accs - 1) * acc_stride + (uint32_t)(wg * 4);
-            tmem_ld4(at, h[a]);
-            tmem_ld4(at + Rt, l[a]);
-            tmem_ld4(at + 2 * Rt, e[a]);
+          for (int a0 = 0; a0 < 4; a0 += 2) {
+            if (a0 >= accs) break;
+            uint32_t v[2][16];
+            const uint32_t at = lane_base + (uint32_t)(wg * 12);
+            tmem_ld16(at + (uint32_t)a0 * acc_stride, v[0]);
+            tmem_ld16(at + (uint32_t)min(a0 + 1, accs - 1) * acc_stride, v[1]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (a0 + a < accs)
+                  sum[i] += fmaf(__uint_as_float(v[a][8 + i]), 0x1p-7f, fmaf(__uint_as_float(v[a][4 + i]), 0x1p-4f, __uint_as_float(v[a][i])));
           }
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            float sum = 0.0f;
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-              if (a < accs)
-                sum += fmaf(__uint_as_float(e[a][i]), 0x1p-7f, fmaf(__uint_as_float(l[a][i]), 0x1p-4f, __uint_as_float(h[a][i])));
-            emit(wg * 4 + i, sum);
-          }
+          for (int i = 0; i < 4; ++i) emit(wg * 4 + i, sum[i]);
         }
         if (!kGrouped && p.slices > 1) {
           // every warp tells every CTA of the cluster that its sums are in place, then the owners add
@@ -694,7 +714,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   __syncthreads();
   if (p.slices > 1)                                        // no CTA leaves while a peer may still reach its shared memory
     cluster_sync();
-  if (warp == 2)
+  if (warp == 4)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
 }
 
@@ -764,14 +784,19 @@ GB_DEVINL void store_group(const Group& G, uint8_t* tile, int64_t unit_stride, b
     *reinterpret_cast<uint2*>(codes + (n >> 3) * 1024 + (n & 7) * 128 + (((gi >> 1) ^ (n & 7)) << 4) + (gi & 1) * 8) = c;
   };
   const uint2 q = make_uint2(G.q[0], G.q[1]), e = make_uint2(G.e[0], G.e[1]);
-  put(m, q);
-  put(R + m, wide ? e : q);
-  if (!wide) put(2 * R + m, e);
+  if (wide) {
+    put(m, q);
+    put(R + m, e);
+  } else {
+    put(narrow_col(0, m), q);
+    put(narrow_col(1, m), q);
+    put(narrow_col(2, m), e);
+  }
 #pragma unroll
   for (int t = 0; t < 3; ++t) {                             // hi, lo, dlt
     const uint32_t b = t == 0 ? G.hi : t == 1 ? G.lo : G.dl;
     const uint32_t b1 = __shfl_down_sync(mask, b, 1), b2 = __shfl_down_sync(mask, b, 2), b3 = __shfl_down_sync(mask, b, 3);
-    const int n = !wide ? t * R + m : t == 1 ? m : (t == 2 ? R : 0) + m;
+    const int n = !wide ? narrow_col(t, m) : t == 2 ? R + m : m;
     if ((gi & 3) == 0)
       *reinterpret_cast<uint32_t*>(unit + (wide && t == 1 ? 2048 : 0) + (gi >> 2) * 512 + (n & 31) * 16 + ((n >> 5) & 3) * 4) =
           b | (b1 << 8) | (b2 << 16) | (b3 << 24);
@@ -914,7 +939,8 @@ Info info(int F) {
 
 // Shared memory: [kDynBase, kLut) and [behind the tables, end).  The activation ring holds eight units where
 // they fit beside two raw stages, else four (a unit's slot and its operand buffer are handed back by
-// one barrier, so only multiples of the four buffers work); what is left goes to the raw ring.
+// one barrier, so only multiples of the four buffers work); what is left goes to the raw ring (four stages or
+// two).
 bool layout(const Info& f, Fp4Params& p) {
   for (p.x_stages = 8; p.x_stages >= 4; p.x_stages -= 4) {
     struct Region { uint32_t at, end; } reg[2] = {{kDynBase, kLut}, {kLut + f.lut, kSmemEnd}};
@@ -928,8 +954,8 @@ bool layout(const Info& f, Fp4Params& p) {
     if (!take((uint32_t)(p.x_stages * p.x_unit), 1024, &p.x_off)) continue;
     if (!take(512 + f.extra, 128, &p.misc_off)) continue;
     if (p.slices > 1 && !take((uint32_t)((p.M + p.slices - 1) / p.slices * p.slices * kBM * 4), 128, &p.red_off)) continue;
-    for (p.raw_stages = 0; p.raw_stages < kMaxRaw && take(f.box, 128, &p.raw_off[p.raw_stages]);) ++p.raw_stages;
-    if (p.raw_stages >= 2) return true;
+    for (p.raw_stages = kMaxRaw; p.raw_stages >= 2; p.raw_stages >>= 1)
+      if (take(f.box * (uint32_t)p.raw_stages, 128, &p.raw_off)) return true;
   }
   return false;
 }
