@@ -78,8 +78,8 @@ int gb_tensor_map_operand(void* map_out, const void* base, int64_t rows, int64_t
 // 1..128 activation rows of the literal format, the two-tier k = 16 format with 80-byte superblocks
 // or the fp8 k = 32 format: decode into tensor memory, tcgen05 MMA with the weights on the M side
 // (gb_gemv_umma.cu); GB_EUNSUPPORTED when the format, layout or row count is not its own.
-int gb_gemv_umma(const void* x, int64_t M, const gb_weight* w, int act, int scale_rule, void* y, void* workspace,
-                 int64_t workspace_bytes, void* stream);
+int gb_gemv_umma(const void* x, int64_t M, const gb_weight* w, int n_roles, const int64_t* role_rows, int act, int scale_rule,
+                 void* y, void* workspace, int64_t workspace_bytes, void* stream);
 int64_t gb_gemv_umma_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int gb_gemv_umma_max_rows(const gb_weight* w);
 bool gb_gemv_umma_is_literal(const gb_weight* w);

@@ -938,7 +938,7 @@ int gb_gemv(const void* x, int64_t M, const gb_weight* w, int act, int scale_rul
     // decoded once whatever the row count.  The literal format has faster table kernels for a few
     // rows; the product formats it serves (padded two-tier k = 16, fp8 k = 32 and k = 16) take it from
     // one row on.  A threshold past 128 switches the kernel off for every format.
-    rc = gb_gemv_umma(x, M, w, act, scale_rule, y, workspace, workspace_bytes, stream_);
+    rc = gb_gemv_umma(x, M, w, 0, nullptr, act, scale_rule, y, workspace, workspace_bytes, stream_);
     if (rc != GB_EUNSUPPORTED) return rc;
   }
   if (M > 16)

@@ -1182,6 +1182,10 @@ int gb_gemv_hinted(const void* x, int64_t M, const gb_weight* w, const gb_hints*
                      workspace_bytes, stream);
     if (rc != GB_EUNSUPPORTED) return rc;
   }
+  if (hints->n_roles > 1) {                                // parts with their own codebook: the per-row offsets alone hide them
+    rc = gb_gemv_umma(x, M, w, hints->n_roles, hints->role_rows, act, scale_rule, y, workspace, workspace_bytes, stream);
+    if (rc != GB_EUNSUPPORTED) return rc;
+  }
   return gb_gemv(x, M, w, act, scale_rule, y, workspace, workspace_bytes, stream);
 }
 

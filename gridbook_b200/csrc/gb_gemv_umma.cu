@@ -41,7 +41,7 @@ constexpr int kMaxXStages = 8;
 constexpr int kMaxRawStages = 3;
 constexpr int kSmemCap = 227 * 1024;
 
-enum { kFmtLit = 0, kFmtK16 = 1, kFmtFp8 = 2, kFmtF8L = 3 };
+enum { kFmtLit = 0, kFmtK16 = 1, kFmtFp8 = 2, kFmtF8L = 3, kFmtFp8W = 4 };   // Fp8W: Fp8 with twice the copies, for up to 16 rows
 
 // Per format: bytes of a superblock, how a raw stage is cut into TMA boxes, ring depth, and the
 // bytes of the replicated codebook copies (+ scale table).
@@ -54,14 +54,20 @@ template <> struct Fm<kFmtK16> {
   static constexpr int kSb = 80, kSbPerBox = 2, kBoxes = 1, kStages = 2;
   static constexpr int kLut = 2 * 256 * 16 * 8 + 256 * 16 * 2;   // two sub-tables of 8-byte entries, 16 copies; bf16 scales
 };
-template <> struct Fm<kFmtFp8> {
+// fp8 k = 32: four sub-tables of two values, kept as bf16 pairs in 32 copies (no bank conflicts) where the
+// activation stages are small, in 16 (two lanes share a bank) otherwise.
+template <int kCopies> struct FmFp8 {
   static constexpr int kSb = 128, kSbPerBox = 1, kBoxes = 2, kStages = 2;
-  static constexpr int kLut = 4 * 256 * 32 * 2;           // four sub-tables of 2-byte entries, 32 copies
+  static constexpr int kStride = 4 * kCopies;             // bytes between entries
+  static constexpr int kLut = 4 * 256 * kStride;
 };
+template <> struct Fm<kFmtFp8> : FmFp8<16> {};
+template <> struct Fm<kFmtFp8W> : FmFp8<32> {};
 template <> struct Fm<kFmtF8L> {
   static constexpr int kSb = 64, kSbPerBox = 3, kBoxes = 1, kStages = 2;
-  static constexpr int kLut = 2 * 256 * 32 * 4;           // two sub-tables of 4-byte entries, 32 copies
+  static constexpr int kLut = 2 * 256 * 16 * 8;           // two sub-tables of four values as bf16, 16 copies
 };
+template <int F> constexpr bool kIsFp8 = F == kFmtFp8 || F == kFmtF8L || F == kFmtFp8W;
 template <int F> struct Geo {
   static constexpr int kPitch = Fm<F>::kSbPerBox * Fm<F>::kSb + 16;   // an odd number of 16-byte units
   static constexpr int kBoxBytes = kBM * kPitch;
@@ -70,6 +76,8 @@ template <int F> struct Geo {
   static constexpr int kFixed = 1024 + Fm<F>::kStages * kStageBytes + Fm<F>::kLut + 512;
   static_assert((kPitch / 16) % 2 == 1 && kPitch <= 256, "row pitch");
 };
+
+struct Role { int row0, rows, tile0; int64_t cb; };       // rows that share a codebook; first tile; element offset
 
 struct UmmaParams {
   int64_t N, K;
@@ -93,6 +101,8 @@ struct UmmaParams {
   const int32_t* row_map;    // [P] output row of a sorted row, or null = identity
   int tiles_n;               // 128-row tiles per expert
   int n_tiles;               // tiles of the launch (dense: row tiles; grouped: experts x tiles_n)
+  int n_roles;               // dense: parts with a codebook of their own
+  Role role[GB_MAX_ROLES];
   uint16_t* y_peer[GB_PEER_MAX];   // optional: output row r lives in y_peer[r / rows_per_rank]
   int64_t rows_per_rank;     // 0 = all rows in y
 };
@@ -219,46 +229,144 @@ GB_DEVINL void k16_decode4(uint32_t lut0, uint32_t lut1, uint32_t wa, uint32_t w
   }
 }
 
-// fp8 product format, k = 32: four codewords of four sub-indices; every sub-table entry is two E4M3
-// values; weight = bf16(value * row scale), the product taken in fp32.  `lut` is the lane's copy of
-// entry 0 of the first sub-table (entries 64 bytes apart, sub-tables 16 KiB apart).
-GB_DEVINL void fp8_decode4(uint32_t lut, uint4 cw, float rs, uint32_t (&v)[16]) {
+// fp8 grid: weight = bf16(value * row scale), one rounding of the fp32 product.  A value has four
+// significant bits, so per row only eight products (times powers of two) can occur, and a pair (hi, lo) of
+// bf16 numbers whose two-step product fma(v, hi, v * lo) rounds to the same bf16 for all eight gives every
+// weight in two packed bf16 instructions.  hi = bf16(scale), lo = bf16(scale - hi), moved by a few ulps
+// until it does; a row for which nothing in reach does (or whose scale is far from 1) keeps the fp32
+// product.  `lo` comes back with hi in the low half and lo in the high half; false: no such pair.
+GB_DEVINL bool fp8_row_factors(float rs, uint32_t* hi2, uint32_t* lo2) {
+  const uint32_t hb = gb_f32_to_bf16_bits(rs);
+  const float hi = gb_bf16_bits_to_f32(hb);
+  *hi2 = hb * 0x10001u;
+  *lo2 = 0u;
+  if (rs == 0.0f) return true;
+  if (!(fabsf(rs) > 0x1p-60f && fabsf(rs) < 0x1p60f)) return false;
+  const uint32_t lb = gb_f32_to_bf16_bits(rs - hi);
+  uint32_t want[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+    want[m] = gb_pack_bf16x2(__fmul_rn(1.0f + 0.25f * m, rs), __fmul_rn(1.125f + 0.25f * m, rs));
+  for (int k = 0; k < 9; ++k) {                            // lo, then one to four ulps either way
+    const uint32_t cand = (lb + (uint32_t)((k + 1) / 2 * ((k & 1) ? 1 : -1))) & 0xFFFFu, l2 = cand * 0x10001u;
+    bool same = true;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const uint32_t v = gb_pack_bf16x2(1.0f + 0.25f * m, 1.125f + 0.25f * m);
+      uint32_t t, w;
+      asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(t) : "r"(v), "r"(l2));
+      asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(w) : "r"(v), "r"(*hi2), "r"(t));
+      same &= w == want[m];
+    }
+    if (same) { *lo2 = l2; return true; }
+  }
+  return false;
+}
+
+template <bool kExact>
+GB_DEVINL uint32_t fp8_weight2(uint32_t pair, uint32_t hi2, uint32_t lo2, float rs) {
+  if (!kExact) return mul_pair_f32(pair, rs);
+  uint32_t t, w;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(t) : "r"(pair), "r"(lo2));
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(w) : "r"(pair), "r"(hi2), "r"(t));
+  return w;
+}
+
+template <int kImm>
+GB_DEVINL uint32_t lds_at(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(kImm));
+  return v;
+}
+
+// fp8 product format, k = 32: four codewords of four sub-indices; every sub-table entry is two values as
+// bf16.  `lut` is the lane's copy of entry 0 of the first sub-table.
+template <int F, bool kExact>
+GB_DEVINL void fp8_decode4(uint32_t lut, uint4 cw, uint32_t hi2, uint32_t lo2, float rs, uint32_t (&v)[16]) {
+  constexpr int kShift = Fm<F>::kStride == 128 ? 7 : 6;
+  constexpr uint32_t kMask = 0xFFu << kShift;
   const uint32_t w4[4] = {cw.x, cw.y, cw.z, cw.w};
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t off = (j == 0 ? w4[c] << 6 : w4[c] >> (8 * j - 6)) & 0x3FC0u;
-      uint16_t e;
-      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(e) : "r"(lut + (uint32_t)(j * 16384) + off));
-      uint32_t h2;
-      asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"(e));
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h2));
-      v[c * 4 + j] = gb_pack_bf16x2(f.x * rs, f.y * rs);
-    }
+    const uint32_t w = w4[c];
+    v[c * 4 + 0] = fp8_weight2<kExact>(lds_at<0 * 256 * Fm<F>::kStride>(lut + ((w << kShift) & kMask)), hi2, lo2, rs);
+    v[c * 4 + 1] = fp8_weight2<kExact>(lds_at<1 * 256 * Fm<F>::kStride>(lut + ((w >> (8 - kShift)) & kMask)), hi2, lo2, rs);
+    v[c * 4 + 2] = fp8_weight2<kExact>(lds_at<2 * 256 * Fm<F>::kStride>(lut + ((w >> (16 - kShift)) & kMask)), hi2, lo2, rs);
+    v[c * 4 + 3] = fp8_weight2<kExact>(lds_at<3 * 256 * Fm<F>::kStride>(lut + ((w >> (24 - kShift)) & kMask)), hi2, lo2, rs);
   }
 }
 
 // fp8 product format, k = 16: two index words (four codewords: low byte = first sub-table, high byte
-// = second); every sub-table entry is four E4M3 values (entries 128 bytes apart, the second
-// sub-table 32 KiB after the first).
-GB_DEVINL void f8l_decode4(uint32_t lut, uint32_t wa, uint32_t wb, float rs, uint32_t (&v)[16]) {
+// = second); every sub-table entry is four values as bf16 (entries 128 bytes apart, the second sub-table
+// 32 KiB after the first).
+template <bool kExact>
+GB_DEVINL void f8l_decode4(uint32_t lut, uint32_t wa, uint32_t wb, uint32_t hi2, uint32_t lo2, float rs, uint32_t (&v)[16]) {
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const uint32_t w = c < 2 ? wa : wb;
     const uint32_t off0 = ((c & 1) ? w >> 9 : w << 7) & 0x7F80u, off1 = ((c & 1) ? w >> 17 : w >> 1) & 0x7F80u;
-    uint32_t e[2];
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e[0]) : "r"(lut + off0));
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e[1]) : "r"(lut + 32768u + off1));
+    uint2 e0, e1;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(e0.x), "=r"(e0.y) : "r"(lut + off0));
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2+32768];" : "=r"(e1.x), "=r"(e1.y) : "r"(lut + off1));
+    v[c * 4 + 0] = fp8_weight2<kExact>(e0.x, hi2, lo2, rs);
+    v[c * 4 + 1] = fp8_weight2<kExact>(e0.y, hi2, lo2, rs);
+    v[c * 4 + 2] = fp8_weight2<kExact>(e1.x, hi2, lo2, rs);
+    v[c * 4 + 3] = fp8_weight2<kExact>(e1.y, hi2, lo2, rs);
+  }
+}
+
+// Two E4M3 bytes as bf16 (exact).
+GB_DEVINL uint32_t e4m3_pair_to_bf16(uint32_t b) {
+  return gb_pack_bf16x2(gb_e4m3_to_f32(b & 0xFFu), gb_e4m3_to_f32((b >> 8) & 0xFFu));
+}
+
+// The replicated lookup tables of one codebook, by the 512 decoder threads (d: 0 .. 511).
+template <int F>
+GB_DEVINL void build_tables(uint8_t* cb_s, const void* codebook, int64_t cb, const float* compose, int* inexact, int d) {
+  const int de = d & 255, dh = d >> 8;                      // entry, which half of the copies / which table
+  if constexpr (F == kFmtLit) {
+    // the codebook, eight copies side by side (copy j of an entry sits in the j-th 16-byte bank
+    // group), pre-multiplied by 2^120 (exact for the fp4 grid's values)
+    const uint4 e = __ldg(reinterpret_cast<const uint4*>(codebook) + de);
+    const uint32_t two120 = 0x7B807B80u;
+    const uint4 w = make_uint4(mul_bf16x2(e.x, two120), mul_bf16x2(e.y, two120), mul_bf16x2(e.z, two120),
+                               mul_bf16x2(e.w, two120));
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      uint32_t lo, hi;
-      asm("{\n.reg .b16 a, b;\nmov.b32 {a, b}, %2;\ncvt.rn.f16x2.e4m3x2 %0, a;\ncvt.rn.f16x2.e4m3x2 %1, b;\n}\n"
-          : "=r"(lo), "=r"(hi) : "r"(e[t]));
-      const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&lo));
-      const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-      v[c * 4 + 2 * t] = gb_pack_bf16x2(f0.x * rs, f0.y * rs);
-      v[c * 4 + 2 * t + 1] = gb_pack_bf16x2(f1.x * rs, f1.y * rs);
+    for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(cb_s)[de * 8 + dh * 4 + j] = w;
+  } else if constexpr (F == kFmtK16) {
+    // two sub-tables of 256 entries x four bf16, 16 copies each (8-byte loads go 16 lanes at a time);
+    // the scale table as bf16, with a note when a value does not survive the conversion
+    const uint2 e = __ldg(reinterpret_cast<const uint2*>(codebook) + dh * 256 + de);
+    uint2* l = reinterpret_cast<uint2*>(cb_s) + dh * 256 * 16;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) l[de * 16 + j] = e;
+    uint16_t* comp_s = reinterpret_cast<uint16_t*>(cb_s + 2 * 256 * 16 * 8);
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float f = __ldg(compose + d * 8 + j);
+      const uint32_t b = gb_f32_to_bf16_bits(f);
+      bad |= gb_bf16_bits_to_f32(b) != f;
+      comp_s[d * 8 + j] = (uint16_t)b;
+    }
+    if (bad) atomicOr(inexact, 1);
+  } else if constexpr (F == kFmtF8L) {
+    // two sub-tables of 256 entries x four values, 16 copies each (8-byte loads go 16 lanes at a time)
+    const uint32_t e = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(codebook) + cb) + dh * 256 + de);
+    const uint32_t lo = e4m3_pair_to_bf16(e), hi = e4m3_pair_to_bf16(e >> 16);
+    uint4* l = reinterpret_cast<uint4*>(cb_s) + (dh * 256 + de) * 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) l[j] = make_uint4(lo, hi, lo, hi);
+  } else {
+    // four sub-tables of 256 entries x two values
+    const uint16_t* t = reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(codebook) + cb);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int ent = (dh * 2 + q) * 256 + de;
+      const uint32_t e = e4m3_pair_to_bf16(__ldg(t + ent));
+      uint4* l = reinterpret_cast<uint4*>(cb_s + ent * Fm<F>::kStride);
+#pragma unroll
+      for (int j = 0; j < Fm<F>::kStride / 16; ++j) l[j] = make_uint4(e, e, e, e);
     }
   }
 }
@@ -303,11 +411,15 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // without rows.
   if (kGrouped) gb_pdl_wait();                             // the segment offsets come from the routing launch
   const int pass_rows = kGrouped ? kGroupRows : p.Mpad;
-  struct Tile { int n0, w_row0, seg_lo, cnt, n_pass; };
+  struct Tile { int n0, n_end, w_row0, seg_lo, cnt, n_pass, role; };
   auto tile_at = [&](int t) {
     Tile T;
-    T.n0 = t * kBM; T.w_row0 = T.n0; T.seg_lo = 0; T.cnt = p.M;
-    if (kGrouped) {
+    T.seg_lo = 0; T.cnt = p.M; T.role = 0; T.n_end = (int)p.N;
+    if (!kGrouped) {
+      while (T.role + 1 < p.n_roles && t >= p.role[T.role + 1].tile0) ++T.role;
+      T.n0 = T.w_row0 = p.role[T.role].row0 + (t - p.role[T.role].tile0) * kBM;
+      T.n_end = p.role[T.role].row0 + p.role[T.role].rows;
+    } else {
       const int e = t / p.tiles_n;
       T.n0 = (t - e * p.tiles_n) * kBM;
       T.w_row0 = e * (int)p.N + T.n0;
@@ -442,53 +554,8 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   } else {
     // ------------------------- decoders -------------------------------------
     const int d = threadIdx.x - 32 * kCtlWarps;              // 0 .. 511
-    const int de = d & 255, dh = d >> 8;                     // entry, which half of the copies / which table
-    if constexpr (F == kFmtLit) {
-      // the codebook, eight copies side by side (copy j of an entry sits in the j-th 16-byte bank
-      // group), pre-multiplied by 2^120 (exact for the fp4 grid's values)
-      const uint4 e = __ldg(reinterpret_cast<const uint4*>(p.codebook) + de);
-      const uint32_t two120 = 0x7B807B80u;
-      const uint4 w = make_uint4(mul_bf16x2(e.x, two120), mul_bf16x2(e.y, two120), mul_bf16x2(e.z, two120),
-                                 mul_bf16x2(e.w, two120));
-#pragma unroll
-      for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(cb_s)[de * 8 + dh * 4 + j] = w;
-    } else if constexpr (F == kFmtK16) {
-      // two sub-tables of 256 entries x four bf16, 16 copies each (8-byte loads go 16 lanes at a time);
-      // the scale table as bf16, with a note when a value does not survive the conversion
-      const uint2 e = __ldg(reinterpret_cast<const uint2*>(p.codebook) + dh * 256 + de);
-      uint2* l = reinterpret_cast<uint2*>(cb_s) + dh * 256 * 16;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) l[de * 16 + j] = e;
-      uint16_t* comp_s = reinterpret_cast<uint16_t*>(cb_s + 2 * 256 * 16 * 8);
-      bool bad = false;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float f = __ldg(p.compose + d * 8 + j);
-        const uint32_t b = gb_f32_to_bf16_bits(f);
-        bad |= gb_bf16_bits_to_f32(b) != f;
-        comp_s[d * 8 + j] = (uint16_t)b;
-      }
-      if (bad) atomicOr(inexact, 1);
-    } else if constexpr (F == kFmtF8L) {
-      // two sub-tables of 256 entries x four E4M3 bytes, 32 copies each (one per lane)
-      const uint32_t e = __ldg(reinterpret_cast<const uint32_t*>(p.codebook) + dh * 256 + de);
-      uint4* l = reinterpret_cast<uint4*>(cb_s) + (dh * 256 + de) * 8;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) l[j] = make_uint4(e, e, e, e);
-    } else {
-      // four sub-tables of 256 entries x two E4M3 bytes, 32 copies each (one per lane)
-      const uint16_t* cb = reinterpret_cast<const uint16_t*>(p.codebook);
-      uint32_t* l = reinterpret_cast<uint32_t*>(cb_s);
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int ent = (dh * 2 + t) * 256 + de;
-        const uint32_t e2 = (uint32_t)__ldg(cb + ent) * 0x10001u;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) l[ent * 16 + j] = e2;
-      }
-    }
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
-    gb_pdl_wait();                                           // y may still be read by the launch ahead
+    int have_role = -1;
+    bool waited = false;
     const int quarter = warp & 3;                            // the tensor-memory lanes this warp may touch
     const int wg = (warp - kCtlWarps) >> 2;                  // warpgroup = operand buffer: units wg, wg + 4, ...
     const int h = wg & 1;                                    // its half of a superblock ...
@@ -496,13 +563,24 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int row = quarter * 32 + lane;                     // weight row of the tile = tensor-memory lane
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t col = lane_base + kACol0 + (uint32_t)(wg * kABufCols);
-    const bool exact = *inexact == 0;
+    bool exact = true;
     int it = 0, g_sb = 0, item = 0;                          // raw stages, superblocks, (tile, pass) items so far
     for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
     const Tile T = tile_at(t);
-    float rs = 0.0f;                                         // fp8 grid: this row's scale
-    if constexpr (F == kFmtFp8 || F == kFmtF8L) {
-      if (T.n_pass > 0 && (int64_t)T.w_row0 + row < p.rows_total) rs = __ldg(p.row_scale + T.w_row0 + row);
+    if (T.n_pass == 0) continue;
+    if (T.role != have_role) {                               // the CTA's rows change codebook
+      if (have_role >= 0) asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
+      build_tables<F>(cb_s, p.codebook, kGrouped ? 0 : p.role[T.role].cb, p.compose, inexact, d);
+      have_role = T.role;
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
+      if (F == kFmtK16) exact = *inexact == 0;
+    }
+    if (!waited) { gb_pdl_wait(); waited = true; }           // y may still be read by the launch ahead
+    float rs = 0.0f;                                         // fp8 grid: this row's scale and its two factors
+    uint32_t hi2 = 0, lo2 = 0;
+    if constexpr (kIsFp8<F>) {
+      if ((int64_t)T.w_row0 + row < p.rows_total) rs = __ldg(p.row_scale + T.w_row0 + row);
+      exact = __all_sync(0xffffffffu, fp8_row_factors(rs, &hi2, &lo2));
     }
     for (int pass = 0; pass < T.n_pass; ++pass, ++item) {
     for (int r = r_begin; r < r_end; ++r, ++it) {
@@ -557,28 +635,36 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           tmem_st16(col + 32u, v0);
           tmem_st16(col + 48u, v1);
         } else if constexpr (F == kFmtF8L) {
-          const uint32_t lut = gb_smem_u32(cb_s) + (uint32_t)lane * 4u;
+          const uint32_t lut = gb_smem_u32(cb_s) + (uint32_t)(lane & 15) * 8u;
           const uint4 ia = rp[2 * h], ib = rp[2 * h + 1];    // eight index words: sixteen codewords
-          f8l_decode4(lut, ia.x, ia.y, rs, v0);
-          f8l_decode4(lut, ia.z, ia.w, rs, v1);
+          auto four = [&](uint32_t wa, uint32_t wb, uint32_t (&v)[16]) {
+            if (exact) f8l_decode4<true>(lut, wa, wb, hi2, lo2, rs, v);
+            else f8l_decode4<false>(lut, wa, wb, hi2, lo2, rs, v);
+          };
+          four(ia.x, ia.y, v0);
+          four(ia.z, ia.w, v1);
           if (sb_in_pass >= 2) wait_fast(&done[(g - 4) & xs_mask], (uint32_t)((g - 4) >> xs_log) & 1u, abort_flag, p.status, 25);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           tmem_st16(col, v0);
           tmem_st16(col + 16u, v1);
-          f8l_decode4(lut, ib.x, ib.y, rs, v0);
-          f8l_decode4(lut, ib.z, ib.w, rs, v1);
+          four(ib.x, ib.y, v0);
+          four(ib.z, ib.w, v1);
           tmem_st16(col + 32u, v0);
           tmem_st16(col + 48u, v1);
         } else {
-          const uint32_t lut = gb_smem_u32(cb_s) + (uint32_t)lane * 2u;
-          fp8_decode4(lut, rp[4 * h], rs, v0);
-          fp8_decode4(lut, rp[4 * h + 1], rs, v1);
+          const uint32_t lut = gb_smem_u32(cb_s) + (uint32_t)(lane & (Fm<F>::kStride / 4 - 1)) * 4u;
+          auto four = [&](uint4 cw, uint32_t (&v)[16]) {
+            if (exact) fp8_decode4<F, true>(lut, cw, hi2, lo2, rs, v);
+            else fp8_decode4<F, false>(lut, cw, hi2, lo2, rs, v);
+          };
+          four(rp[4 * h], v0);
+          four(rp[4 * h + 1], v1);
           if (sb_in_pass >= 2) wait_fast(&done[(g - 4) & xs_mask], (uint32_t)((g - 4) >> xs_log) & 1u, abort_flag, p.status, 25);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           tmem_st16(col, v0);
           tmem_st16(col + 16u, v1);
-          fp8_decode4(lut, rp[4 * h + 2], rs, v0);
-          fp8_decode4(lut, rp[4 * h + 3], rs, v1);
+          four(rp[4 * h + 2], v0);
+          four(rp[4 * h + 3], v1);
           tmem_st16(col + 32u, v0);
           tmem_st16(col + 48u, v1);
         }
@@ -617,7 +703,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(t[i]));
       }
-      if (ok && out_col < p.N) {
+      if (ok && out_col < T.n_end) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int m = c * 8 + i;
@@ -680,6 +766,7 @@ FmtInfo fmt_info(int F) {
   switch (F) {
     case kFmtLit: return {Fm<kFmtLit>::kSb, Geo<kFmtLit>::kSbPerStage, Geo<kFmtLit>::kPitch, Geo<kFmtLit>::kFixed};
     case kFmtK16: return {Fm<kFmtK16>::kSb, Geo<kFmtK16>::kSbPerStage, Geo<kFmtK16>::kPitch, Geo<kFmtK16>::kFixed};
+    case kFmtFp8W: return {Fm<kFmtFp8W>::kSb, Geo<kFmtFp8W>::kSbPerStage, Geo<kFmtFp8W>::kPitch, Geo<kFmtFp8W>::kFixed};
     case kFmtF8L: return {Fm<kFmtF8L>::kSb, Geo<kFmtF8L>::kSbPerStage, Geo<kFmtF8L>::kPitch, Geo<kFmtF8L>::kFixed};
     default: return {Fm<kFmtFp8>::kSb, Geo<kFmtFp8>::kSbPerStage, Geo<kFmtFp8>::kPitch, Geo<kFmtFp8>::kFixed};
   }
@@ -698,9 +785,8 @@ int umma_x_stages(int F, int Mpad) {
 int umma_smem_bytes(int F, int Mpad) { return fmt_info(F).fixed_smem + umma_x_stages(F, Mpad) * (2 * Mpad * 128); }
 
 // K slices: enough CTAs for the SMs when the layer has few 128-row tiles.
-void umma_plan(int F, int64_t N, int n_sb, int sms, int* slices, int* stages_per_slice) {
+void umma_plan(int F, int tiles, int n_sb, int sms, int* slices, int* stages_per_slice) {
   const int per_stage = fmt_info(F).sb_per_stage;
-  const int tiles = (int)((N + kBM - 1) / kBM);
   const int n_raw = (n_sb + per_stage - 1) / per_stage;
   int want = sms / tiles;
   if (want < 1) want = 1;
@@ -711,9 +797,9 @@ void umma_plan(int F, int64_t N, int n_sb, int sms, int* slices, int* stages_per
 
 // Which decoder serves the weight, or -1.  The two-tier format is taken with its superblocks padded
 // to 80 bytes only (type_size 80): 73-byte superblocks cannot be fetched by tiled TMA.
-int umma_format(const gb_weight* w) {
+int umma_format(const gb_weight* w, bool roles_known = false) {
   const gb_format& f = w->fmt;
-  if (w->cb_row_offset != nullptr || (w->row_stride % 16) != 0 || ((uintptr_t)w->qw & 15u) != 0 ||
+  if ((w->cb_row_offset != nullptr && !roles_known) || (w->row_stride % 16) != 0 || ((uintptr_t)w->qw & 15u) != 0 ||
       ((uintptr_t)w->codebook & 15u) != 0)
     return -1;
   if (f.grid == GB_GRID_FP4 && f.mode == GB_MODE_FULL && f.k_bits == 8 && f.scale_coding == GB_SCALE_V1 &&
@@ -731,8 +817,8 @@ int umma_format(const gb_weight* w) {
   return -1;
 }
 
-bool umma_applies(const gb_weight* w, int64_t M) {
-  const int F = umma_format(w);
+bool umma_applies(const gb_weight* w, int64_t M, bool roles_known) {
+  const int F = umma_format(w, roles_known);
   return F >= 0 && M >= 1 && M <= kMaxRows && w->K >= 1024 && w->rows >= kBM && umma_x_stages(F, (int)((M + 15) / 16 * 16)) >= 4;
 }
 
@@ -742,6 +828,9 @@ cudaError_t launch_umma(int F, dim3 grid, size_t smem, cudaStream_t stream, cons
   switch (F) {
     case kFmtLit: return gb_launch(umma_decode_kernel<kGrouped, kFmtLit>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
     case kFmtK16: return gb_launch(umma_decode_kernel<kGrouped, kFmtK16>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
+    case kFmtFp8W:
+      if constexpr (!kGrouped) return gb_launch(umma_decode_kernel<false, kFmtFp8W>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
+      else return cudaErrorInvalidValue;
     case kFmtF8L: return gb_launch(umma_decode_kernel<kGrouped, kFmtF8L>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
     default: return gb_launch(umma_decode_kernel<kGrouped, kFmtFp8>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
   }
@@ -765,6 +854,7 @@ int gb_prepare_umma() {
   GB_UMMA_ATTR(false, kFmtK16, kMaxRows);
   GB_UMMA_ATTR(false, kFmtFp8, kMaxRows);
   GB_UMMA_ATTR(false, kFmtF8L, kMaxRows);
+  GB_UMMA_ATTR(false, kFmtFp8W, kMaxRows);
   GB_UMMA_ATTR(true, kFmtLit, kGroupRows);
   GB_UMMA_ATTR(true, kFmtK16, kGroupRows);
   GB_UMMA_ATTR(true, kFmtFp8, kGroupRows);
@@ -783,16 +873,22 @@ int64_t gb_gemv_umma_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   int most = 1;
   for (int F = 0; F < 4; ++F) {
     int slices, per;
-    umma_plan(F, N, (int)(K / 256), sms, &slices, &per);
+    umma_plan(F, (int)((N + kBM - 1) / kBM), (int)(K / 256), sms, &slices, &per);
     if (slices > most) most = slices;
   }
   return xq + (most > 1 ? (int64_t)most * M * N * 4 : 0);
 }
 
-int gb_gemv_umma(const void* x, int64_t M, const gb_weight* w, int act, int scale_rule, void* y, void* workspace,
-                 int64_t workspace_bytes, void* stream_) {
-  if (!umma_applies(w, M) || ((uintptr_t)x & 15u) != 0) return GB_EUNSUPPORTED;
-  const int F = umma_format(w);
+int gb_gemv_umma(const void* x, int64_t M, const gb_weight* w, int n_roles, const int64_t* role_rows, int act, int scale_rule,
+                 void* y, void* workspace, int64_t workspace_bytes, void* stream_) {
+  if (n_roles > GB_MAX_ROLES || !umma_applies(w, M, n_roles > 1) || ((uintptr_t)x & 15u) != 0) return GB_EUNSUPPORTED;
+  int F = umma_format(w, n_roles > 1);
+  if (n_roles > 1) {                                       // as for a matrix of its own: at least one whole tile per part
+    if (w->fmt.grid != GB_GRID_FP8) return GB_EUNSUPPORTED;
+    for (int r = 0; r < n_roles; ++r)
+      if (role_rows[r] < kBM) return GB_EUNSUPPORTED;
+  }
+  if (F == kFmtFp8 && M <= 16) F = kFmtFp8W;
   const int sms = gb_sm_count();
   if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
   const int64_t N = w->rows, K = w->K;
@@ -800,7 +896,16 @@ int gb_gemv_umma(const void* x, int64_t M, const gb_weight* w, int act, int scal
   UmmaParams p = {};
   p.N = N; p.K = K; p.M = (int)M; p.Mpad = (int)((M + 15) / 16 * 16);
   p.n_sb = (int)(K / 256);
-  umma_plan(F, N, p.n_sb, sms, &p.slices, &p.stages_per_slice);
+  p.n_roles = n_roles < 1 ? 1 : n_roles;
+  int64_t row = 0;
+  for (int r = 0; r < p.n_roles; ++r) {
+    const int64_t rows = n_roles < 1 ? N : role_rows[r];
+    p.role[r] = {(int)row, (int)rows, p.n_tiles, r * gb_codebook_elems(w->fmt)};
+    p.n_tiles += (int)((rows + kBM - 1) / kBM);
+    row += rows;
+  }
+  GB_REQUIRE(row == N, "the roles hold %lld rows, the matrix %lld", (long long)row, (long long)N);
+  umma_plan(F, p.n_tiles, p.n_sb, sms, &p.slices, &p.stages_per_slice);
   const int64_t xq_bytes = act == GB_ACT_NONE ? 0 : ((M * K * 2 + 255) & ~255ll);
   const int64_t part_bytes = p.slices > 1 ? (int64_t)p.slices * M * N * 4 : 0;
   if (xq_bytes + part_bytes > 0 && (workspace == nullptr || workspace_bytes < xq_bytes + part_bytes))
@@ -828,7 +933,6 @@ int gb_gemv_umma(const void* x, int64_t M, const gb_weight* w, int act, int scal
   p.n_iss = p.Mpad <= 64 ? 4 : 2;
   p.status = gb_status_word();
   // one CTA per SM at most: a CTA walks several row tiles when the layer has more of them
-  p.n_tiles = (int)((N + kBM - 1) / kBM);
   const int ctas_x = p.n_tiles * p.slices <= sms ? p.n_tiles : (sms / p.slices > 0 ? sms / p.slices : 1);
   dim3 grid((unsigned)ctas_x, (unsigned)p.slices);
   GB_CUDA_OK(launch_umma<false>(F, grid, (size_t)umma_smem_bytes(F, p.Mpad), (cudaStream_t)stream_, map_w, map_x, p));
