@@ -68,6 +68,7 @@ int gb_prepare_dot();
 int gb_prepare_umma();
 int gb_prepare_tab();
 int gb_prepare_gemm_fp4();
+int gb_prepare_gemm_pair();
 int gb_prepare_gemv_fp4();
 // Longest a device-side wait may spin before it gives up and raises the status word
 // (two seconds unless gb_set_wait_limit_ms changed it).
@@ -75,6 +76,14 @@ unsigned long long gb_wait_limit_ns();
 // Swizzled (128-byte) operand map over a row-major [rows, K] matrix of 2- or 1-byte elements:
 // box = 128 bytes of K x box_rows rows, rows past the end read zero.
 int gb_tensor_map_operand(void* map_out, const void* base, int64_t rows, int64_t K, int elem_bytes, int box_rows);
+// Row-major bf16 output [M, N] in boxes of 32 x 32 with the 64-byte swizzle (N a multiple of 8).
+int gb_tensor_map_out(void* map_out, void* base, int64_t M, int64_t N);
+// The prefill GEMMs on CTA pairs (gb_gemm_pair.cu), for the shapes that gb_gemm_pair_applies names.
+bool gb_gemm_pair_applies(int64_t M);
+int gb_gemm_pair(const void* A, const void* B, void* D, int64_t M, int64_t N, int64_t K, int kind, const float* a_scale,
+                 const float* b_scale, float global_scale, cudaStream_t stream);
+int gb_gemm_fp4_pair(const void* A, const void* sfa, const void* B, const void* sfb, void* D, int64_t M, int64_t N, int64_t K,
+                     const float* a_scale, float global_scale, cudaStream_t stream);
 // 1..128 activation rows of the literal format, the two-tier k = 16 format with 80-byte superblocks
 // or the fp8 k = 32 format: decode into tensor memory, tcgen05 MMA with the weights on the M side
 // (gb_gemv_umma.cu); GB_EUNSUPPORTED when the format, layout or row count is not its own.

@@ -419,6 +419,22 @@ int gb_tensor_map_operand(void* map_out, const void* base, int64_t rows, int64_t
   return make_map((CUtensorMap*)map_out, base, rows, K, elem_bytes, box_rows);
 }
 
+// Row-major bf16 output [M, N] in boxes of 32 x 32, 64-byte swizzle.
+int gb_tensor_map_out(void* map_out, void* base, int64_t M, int64_t N) {
+  EncodeTiledFn enc;
+  int rc = get_encoder(&enc);
+  if (rc != GB_OK) return rc;
+  const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
+  const cuuint64_t strides[1] = {(cuuint64_t)N * 2};
+  const cuuint32_t box[2] = {32, 32};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = enc((CUtensorMap*)map_out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return gb_fail(GB_ECUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
+  return GB_OK;
+}
+
 int gb_prepare_gemm() {
   GB_CUDA_OK(cudaFuncSetAttribute((const void*)gemm_tn_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kGemmSmem));
@@ -440,6 +456,11 @@ int gb_gemm_tn(const void* A, const void* B, void* D, int64_t M, int64_t N, int6
              "operands must be 16-byte aligned");
   GB_REQUIRE(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), "dimension too large");
   if (gb_sm_count() <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
+  if (gb_gemm_pair_applies(M)) {
+    const int rc = gb_gemm_pair(A, B, D, M, N, K, kind, a_scale, b_scale, global_scale == 0.0f ? 1.0f : global_scale,
+                                (cudaStream_t)stream);
+    if (rc != GB_EUNSUPPORTED) return rc;
+  }
   CUtensorMap map_a, map_b;
   int rc = make_map(&map_a, A, M, K, eb, kBM);
   if (rc != GB_OK) return rc;

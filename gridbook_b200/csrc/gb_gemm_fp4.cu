@@ -450,6 +450,11 @@ int gb_gemm_fp4(const void* A, const void* sfa, const void* B, const void* sfb, 
   if (M == 0) return GB_OK;
   const int sms = gb_sm_count();
   if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
+  if (gb_gemm_pair_applies(M)) {
+    const int rc = gb_gemm_fp4_pair(A, sfa, B, sfb, D, M, N, K, a_scale, global_scale == 0.0f ? 1.0f : global_scale,
+                                    (cudaStream_t)stream);
+    if (rc != GB_EUNSUPPORTED) return rc;
+  }
   CUtensorMap map_a, map_b;
   int rc = gb_tensor_map_operand(&map_a, A, M, K / 2, 1, kBM);
   if (rc != GB_OK) return rc;

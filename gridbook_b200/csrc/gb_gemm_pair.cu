@@ -1,0 +1,534 @@
+// Prefill GEMMs on CTA pairs: D[M,N] = A[M,K] . B[N,K]^T, both operands K-major, bf16 (kind::f16),
+// E4M3 (kind::f8f6f4) or block-scaled E2M1 (kind::mxf4nvf4, UE4M3 scale factors per sixteen), fp32
+// accumulators in tensor memory, scaled bf16 epilogue.
+//
+// A single CTA's 128 x 256 tile takes 48 KiB of operands per 128-byte K slab into shared memory and
+// reads them out again for the tensor core: 192 bytes a clock at the full fp8 or fp4 rate, more than
+// the 128 that shared memory moves, and 28 TB/s out of L2 over the GPU.  A pair (tcgen05
+// cta_group::2) works on a 256 x 256 tile together: each CTA loads its own 128 rows of A and its own
+// half of the B rows, the tensor cores exchange the B halves, and a slab is 32 KiB per CTA for the
+// same work.  Every CTA fetches its own operands (the pair's loads report to the leader's barriers).
+//
+// The pair walks output tiles persistently.  Warps 0-7 drain the CTA's own 128 rows, warp 8 of each CTA
+// loads, warp 9 of the leader issues the MMAs of both tensor cores; two accumulators, so that draining
+// overlaps the next tile.
+//
+// The fp4 form has one accumulator: the columns beside it hold five or six sets of scale factors, which
+// warps 10-13 of the leader copy from both CTAs' shared memory (tcgen05.cp, one warp per MMA of a stage)
+// that many stages ahead of the MMAs.  A copy takes its issuing thread 45 clocks or more and a stage
+// needs twelve: from one warp they took longer than the stage's MMAs (8192 x 34816 x 5120: 759 us with
+// one warp, 647 with two, 635 with four, 559 with none at all).  The accumulator is drained into
+// registers in one go, so that the next tile's MMAs start early.
+//
+// Measured, us, one CTA per tile -> pairs (N x K of the four linears of a 5120-wide layer):
+//   fp8, 8192 rows: 34816 x 5120 1434 -> 1096, 5120 x 17408 729 -> 552, 6144 x 5120 263 -> 199, 2048 x 5120 101 -> 72
+//   fp8, 2048 rows: 370 -> 276, 218 -> 156, 80 -> 54, 36 -> 24
+//   fp4, 8192 rows: 960 -> 635, 437 -> 302, 184 -> 116, 66 -> 43
+//   fp4, 2048 rows: 253 -> 165, 145 -> 92, 54 -> 33, 21 -> 18
+// The fp8 form runs at 2.65 PFLOP/s, tensor pipe 71% busy at the 1.55 GHz that the power cap leaves.
+#include "gb_common.cuh"
+
+#include <cuda.h>
+#include <mutex>
+
+namespace {
+
+enum Kind { kBf16 = 0, kFp8 = 1, kFp4 = 2 };
+
+constexpr int kPairM = 256, kBM = 128;               // rows of a tile, rows of a CTA
+constexpr int kSlabBytes = 128;                      // K bytes per row and stage (one swizzle span)
+constexpr int kTmemCols = 512;
+constexpr int kEpiWarps = 8;                         // two per lane quarter, half of the columns each
+constexpr int kOutChunk = 2048;                      // 32 rows x 32 bf16 columns on their way out
+constexpr int kOutBytes = kEpiWarps * 2 * kOutChunk;
+constexpr int kGroupM = 16;                          // row tiles walked together before the next columns
+
+template <Kind kKind, int kBN>
+struct Shape {
+  static constexpr int kABytes = kBM * kSlabBytes;
+  static constexpr int kBBytes = kBN / 2 * kSlabBytes;
+  static constexpr int kAtoms = 2048;                                    // scale bytes of 128 rows x 16 groups
+  static constexpr int kSfBytes = kKind == kFp4 ? 3 * kAtoms : 0;        // A's rows, two 128-row groups of B
+  static constexpr int kStageBytes = kABytes + kBBytes + kSfBytes;
+  static constexpr int kStages = (227 * 1024 - 2048 - kOutBytes) / kStageBytes;
+  static constexpr int kSmem = kStages * kStageBytes + kOutBytes + 2048;
+  static constexpr int kThreads = kKind == kFp4 ? 448 : 320;
+  static constexpr int kAccs = kKind == kFp4 ? 1 : 2;
+  static constexpr uint32_t kSfCols = 48;                                // columns of a set: 16 of A, 32 of B
+  static constexpr int kSets = kKind == kFp4 ? (kTmemCols - kBN) / (int)kSfCols : 1;
+};
+
+struct PairParams {
+  int64_t M, N, K;
+  int k_tiles, m_tiles, n_tiles;
+  uint32_t idesc;
+  const float* a_scale;        // [M] or null
+  const float* b_scale;        // [N] or null
+  float global_scale;
+  int out_tma;                 // rows of D are a multiple of 16 bytes
+  uint16_t* D;
+  int* status;
+};
+
+GB_DEVINL uint32_t leader_addr(uint32_t addr) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+GB_DEVINL void arrive_cluster(uint32_t addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+GB_DEVINL bool try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+// A bounded wait that remembers a timeout for the rest of the CTA: later waits return at once.
+__device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  uint64_t t0 = 0;
+  for (uint32_t spin = 0; !*abort_flag; ++spin) {
+    if (try_wait(bar, parity)) return;
+    if ((spin & 255u) == 255u) {
+      const uint64_t now = gb_globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > 2000000000ull) { *abort_flag = 1; atomicExch(status, code); }
+    }
+  }
+}
+GB_DEVINL void wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (!try_wait(bar, parity)) wait_slow(bar, parity, abort_flag, status, code);
+}
+// Tile load into this CTA's shared memory that reports to a barrier of the pair.
+GB_DEVINL void tma_load_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar) : "memory");
+}
+GB_DEVINL void expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+GB_DEVINL void bar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+// K-major operand tile stored as rows of 128 bytes with the 128-byte swizzle.
+GB_DEVINL uint64_t desc_sw128(uint32_t smem_addr) {
+  return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)(1024u >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
+}
+// One scale-factor atom: 32 rows of 16 bytes, unswizzled, the 8-row groups 128 bytes apart; the copy
+// repeats it in the four lane quarters of both CTAs' tensor memory, each from its own shared memory.
+GB_DEVINL void sf_to_tmem(uint32_t tmem_col, uint32_t smem_addr) {
+  const uint64_t d = (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)(16u >> 4) << 16 | (uint64_t)(128u >> 4) << 32 | (uint64_t)1 << 46;
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_col), "l"(d) : "memory");
+}
+template <Kind kKind>
+GB_DEVINL void mma_pair(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t sfa, uint32_t sfb, bool accumulate) {
+  if (kKind == kFp4)
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n}\n"
+        ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)accumulate), "r"(sfa), "r"(sfb) : "memory");
+  else if (kKind == kFp8)
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n"
+        ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
+  else
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+        ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
+}
+// Completion of the MMAs issued so far, told to the barrier at this offset in both CTAs.
+GB_DEVINL void commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+GB_DEVINL void commit_leader(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+GB_DEVINL void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+GB_DEVINL void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(taddr));
+}
+
+// 32 accumulator columns of one output row, scaled and rounded to bf16 pairs.
+template <bool kColScale>
+GB_DEVINL void pack_chunk(const PairParams& p, const uint32_t (&v)[32], uint32_t* w, float rs, int col0) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    float lo = __uint_as_float(v[2 * j]) * rs, hi = __uint_as_float(v[2 * j + 1]) * rs;
+    if (kColScale && p.b_scale) {
+      const int c = col0 + 2 * j;
+      lo *= c < (int)p.N ? p.b_scale[c] : 0.0f;
+      hi *= c + 1 < (int)p.N ? p.b_scale[c + 1] : 0.0f;
+    }
+    w[j] = gb_pack_bf16x2(lo, hi);
+  }
+}
+
+// Output tile of a step: groups of kGroupM row tiles, inside a group the rows fastest.  The pairs that
+// run together (74) then share sixteen row tiles of A and about five column tiles of B, which stay in L2
+// while the group sweeps N (rows fastest over all of M re-read a 142 MB activation matrix from HBM for
+// every two or three columns of tiles).  8192 x 34816 x 5120 fp8 / fp4: groups of 4 1111 / 687 us, 8
+// 1065 / 652, 16 1041 / 632.
+GB_DEVINL void tile_at(const PairParams& p, int tile, int& mt, int& nt) {
+  const int per = kGroupM * p.n_tiles, g = tile / per, in = tile - g * per;
+  const int rows = min(kGroupM, p.m_tiles - g * kGroupM);
+  mt = g * kGroupM + in % rows;
+  nt = in / rows;
+}
+
+GB_DEVINL int first_col(const PairParams& p, int tile, int bn) {
+  int mt, nt;
+  tile_at(p, tile, mt, nt);
+  return nt * bn;
+}
+
+template <Kind kKind, int kBN>
+__global__ void __launch_bounds__(Shape<kKind, kBN>::kThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
+                 const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb, const PairParams p) {
+  using S = Shape<kKind, kBN>;
+  constexpr int kStages = S::kStages;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t ring = (gb_smem_u32(smem_raw) + 1023u) & ~1023u;        // the same offset in both CTAs
+  uint8_t* ring_ptr = smem_raw + (ring - gb_smem_u32(smem_raw));
+  const uint32_t out_ring = ring + kStages * S::kStageBytes;             // two chunks per epilogue warp
+  const uint32_t full_bar = out_ring + kOutBytes;             // leader: both CTAs' operand tiles have landed
+  const uint32_t empty_bar = full_bar + 8 * kStages;                     // the MMAs that read the stage are done
+  const uint32_t acc_full = empty_bar + 8 * kStages;                     // [2] accumulator complete
+  const uint32_t acc_empty = acc_full + 16;                              // [2] leader: drained by both CTAs
+  const uint32_t sf_full = acc_empty + 16;                               // [kSets] leader: column set written in both CTAs
+  const uint32_t sf_empty = sf_full + 8 * S::kSets;                      // [kSets] leader: the MMAs that read the set are done
+  const uint32_t slot = sf_empty + 8 * S::kSets;
+  volatile uint32_t* slot_ptr = reinterpret_cast<volatile uint32_t*>(ring_ptr + (slot - ring));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(slot_ptr + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  gb_pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      bar_init(full_bar + 8 * s, 1);
+      bar_init(empty_bar + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      bar_init(acc_full + 8 * b, 1);
+      bar_init(acc_empty + 8 * b, 2 * kEpiWarps);
+    }
+    for (int t = 0; t < S::kSets; ++t) {
+      bar_init(sf_full + 8 * t, 4);
+      bar_init(sf_empty + 8 * t, 1);
+    }
+    *abort_flag = 0;
+    gb_fence_barrier_init();
+  }
+  if (warp == kEpiWarps + 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"((uint32_t)kTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_sync();                                                        // both CTAs' barriers exist
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = *slot_ptr;
+  gb_pdl_wait();
+  const int total_tiles = p.m_tiles * p.n_tiles, stride = (int)(gridDim.x >> 1), first = (int)(blockIdx.x >> 1);
+  const int my_tiles = total_tiles > first ? (total_tiles - first + stride - 1) / stride : 0;
+
+  if (warp == kEpiWarps) {
+    // ------------------------------- producer (each CTA) -------------------------------
+    if (lane == 0) {
+      constexpr int slab_elems = kKind == kBf16 ? kSlabBytes / 2 : kSlabBytes;   // E2M1 pairs and E4M3 go by bytes
+      const uint32_t full_pair = leader_addr(full_bar);
+      int s = 0;
+      uint32_t ph = 1;
+      for (int tile = first; tile < total_tiles; tile += stride) {
+        int mt, nt;
+        tile_at(p, tile, mt, nt);
+        const int m0 = mt * kPairM + (int)rank * kBM, n0 = nt * kBN;
+        for (int kt = 0; kt < p.k_tiles; ++kt) {
+          wait(empty_bar + 8 * s, ph, abort_flag, p.status, 71);
+          if (*abort_flag) break;
+          const uint32_t st = ring + (uint32_t)s * S::kStageBytes;
+          if (rank == 0) expect_tx(full_bar + 8 * s, 2 * S::kStageBytes);
+          tma_load_pair(st, &map_a, kt * slab_elems, m0, full_pair + 8 * s);
+          tma_load_pair(st + S::kABytes, &map_b, kt * slab_elems, n0 + (int)rank * (kBN / 2), full_pair + 8 * s);
+          if (kKind == kFp4) {                               // row groups past the end read zero
+            const uint32_t sf = st + S::kABytes + S::kBBytes;
+            tma_load_pair(sf, &map_sfa, 0, (m0 / 128 * p.k_tiles + kt) * 8, full_pair + 8 * s);
+            tma_load_pair(sf + S::kAtoms, &map_sfb, 0, (n0 / 128 * p.k_tiles + kt) * 8, full_pair + 8 * s);
+            tma_load_pair(sf + 2 * S::kAtoms, &map_sfb, 0, ((n0 / 128 + 1) * p.k_tiles + kt) * 8, full_pair + 8 * s);
+          }
+          if (++s == kStages) { s = 0; ph ^= 1; }
+        }
+        if (*abort_flag) break;
+      }
+    }
+  } else if (warp == kEpiWarps + 1) {
+    // --------------------------- MMA issuer (the leader's) ------------------------------
+    if (lane == 0 && rank == 0) {
+      int s = 0, set = 0;
+      uint32_t ph = 0, sf_ph = 0;
+      for (int it = 0; it < my_tiles; ++it) {
+        const int buf = S::kAccs == 2 ? it & 1 : 0;
+        const uint32_t use = (uint32_t)(S::kAccs == 2 ? it >> 1 : it);
+        const bool shifted = first_col(p, first + it * stride, kBN) % 128 != 0;
+        wait(acc_empty + 8 * buf, (use & 1) ^ 1, abort_flag, p.status, 72);       // its last tile is drained
+        const uint32_t acc = tmem_base + (buf ? 256u : 0u);
+        for (int kt = 0; kt < p.k_tiles; ++kt) {
+          if (kKind == kFp4) wait(sf_full + 8 * set, sf_ph, abort_flag, p.status, 73);
+          else wait(full_bar + 8 * s, ph, abort_flag, p.status, 74);
+          if (*abort_flag) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t st = ring + (uint32_t)s * S::kStageBytes;
+          const uint64_t da = desc_sw128(st), db = desc_sw128(st + S::kABytes);
+          // 192 columns start in the middle of a 128-row group every other time: two columns on
+          const uint32_t sfa_t = tmem_base + kBN + S::kSfCols * set, sfb_t = sfa_t + 16u + (shifted ? 2u : 0u);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)                        // 32 bytes of K per instruction
+            mma_pair<kKind>(acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), p.idesc, sfa_t + 4u * k, sfb_t + 8u * k,
+                            kt > 0 || k > 0);
+          commit_pair(empty_bar + 8 * s);
+          if (kKind == kFp4) {
+            commit_leader(sf_empty + 8 * set);
+            if (++set == S::kSets) { set = 0; sf_ph ^= 1; }
+          }
+          if (++s == kStages) { s = 0; ph ^= 1; }
+        }
+        if (*abort_flag) break;
+        commit_pair(acc_full + 8 * buf);
+      }
+    }
+  } else if (warp >= kEpiWarps + 2) {
+    // ------------ scale factors -> tensor memory (the leader's, fp4): warp k the k-th MMA's ------------
+    const uint32_t k = (uint32_t)(warp - kEpiWarps - 2);
+    if (lane == 0 && rank == 0) {
+      int s = 0, set = 0;
+      uint32_t ph = 0, sf_ph = 1;
+      const int total = my_tiles * p.k_tiles;
+      for (int g = 0; g < total; ++g) {
+        wait(full_bar + 8 * s, ph, abort_flag, p.status, 75);
+        wait(sf_empty + 8 * set, sf_ph, abort_flag, p.status, 76);
+        if (*abort_flag) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t sf = ring + (uint32_t)s * S::kStageBytes + S::kABytes + S::kBBytes;
+        const uint32_t col = tmem_base + kBN + S::kSfCols * set;
+        sf_to_tmem(col + 4u * k, sf + 512u * k);
+        sf_to_tmem(col + 16u + 8u * k, sf + S::kAtoms + 512u * k);
+        sf_to_tmem(col + 20u + 8u * k, sf + 2 * S::kAtoms + 512u * k);
+        commit_leader(sf_full + 8 * set);
+        if (++set == S::kSets) { set = 0; sf_ph ^= 1; }
+        if (++s == kStages) { s = 0; ph ^= 1; }
+      }
+    }
+  } else if (warp < kEpiWarps) {
+    // ------------------------------- epilogue (each CTA) --------------------------------
+    // The warp's columns go into registers, scaled and rounded, before anything is stored: the MMAs of the
+    // next tile (fp4) wait for them.  Then out through shared memory, 32 x 32 values a TMA store; rows of
+    // 16-byte pieces straight from the registers reach L2 as half-written sectors.
+    const uint32_t acc_empty_pair = leader_addr(acc_empty);
+    constexpr int kCols = kBN / 2, kChunks = kCols / 32;
+    const int quarter = warp & 3, c_lo = (warp >> 2) * kCols;
+    const uint32_t out = out_ring + (uint32_t)warp * 2 * kOutChunk;
+    int it = 0;
+    for (int tile = first; tile < total_tiles; tile += stride, ++it) {
+      int mt, nt;
+      tile_at(p, tile, mt, nt);
+      const int buf = S::kAccs == 2 ? it & 1 : 0, n0 = nt * kBN + c_lo;
+      const int row0 = mt * kPairM + (int)rank * kBM + quarter * 32, row = row0 + lane;
+      const bool row_ok = row < p.M;
+      const float rs = (p.a_scale && row_ok ? p.a_scale[row] : 1.0f) * p.global_scale;
+      wait(acc_full + 8 * buf, (uint32_t)(S::kAccs == 2 ? it >> 1 : it) & 1, abort_flag, p.status, 77);
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf ? 256u : 0u) + (uint32_t)c_lo;
+      uint32_t w[kCols / 2], va[32];
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) {
+        tmem_ld32(tbase + 32u * c, va);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (c == kChunks - 1) {
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) arrive_cluster(acc_empty_pair + 8 * buf);
+        }
+        pack_chunk<kKind != kFp4>(p, va, &w[16 * c], rs, n0 + 32 * c);
+      }
+      if (p.out_tma) {
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+          const uint32_t dst = out + (uint32_t)(c & 1) * kOutChunk;
+          asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");       // the chunk before last has left its buffer
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < 4; ++q)                        // 64-byte swizzle: eight rows touch eight bank groups
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                         ::"r"(dst + (uint32_t)lane * 64u + (uint32_t)((q ^ ((lane >> 1) & 3)) * 16)), "r"(w[16 * c + 4 * q]),
+                           "r"(w[16 * c + 4 * q + 1]), "r"(w[16 * c + 4 * q + 2]), "r"(w[16 * c + 4 * q + 3]) : "memory");
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0 && row0 < p.M && n0 + 32 * c < p.N)  // what sticks out is not written
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                         ::"l"(reinterpret_cast<uint64_t>(&map_d)), "r"(n0 + 32 * c), "r"(row0), "r"(dst) : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      } else if (row_ok) {
+        uint16_t* d = p.D + (int64_t)row * p.N + n0;
+        const int cols = (int)p.N - n0;
+#pragma unroll
+        for (int c = 0; c < kCols; ++c)
+          if (c < cols) d[c] = (uint16_t)(w[c / 2] >> (16 * (c & 1)));
+      }
+    }
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+  __syncwarp();
+  if (*abort_flag && threadIdx.x == 0) __nanosleep(1000000);   // loads still in flight land before the memory goes
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_sync();                                            // the peer may still signal barriers here
+  if (warp == kEpiWarps + 1)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTmemCols) : "memory");
+}
+
+std::mutex g_mutex;
+int g_pairs[64][8];                                          // pairs that run at once, per device and kernel (0: not asked)
+
+template <Kind kKind, int kBN>
+int resident_pairs() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  int& n = g_pairs[dev][(int)kKind * 2 + (kBN == 256)];
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * 256);
+    cfg.blockDim = dim3(Shape<kKind, kBN>::kThreads);
+    cfg.dynamicSmemBytes = Shape<kKind, kBN>::kSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<kKind, kBN>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
+  }
+  return n;
+}
+
+template <Kind kKind, int kBN>
+int run(const void* A, const void* B, const void* sfa, const void* sfb, PairParams p, int row_bytes_elem, cudaStream_t stream) {
+  using S = Shape<kKind, kBN>;
+  const int pairs = resident_pairs<kKind, kBN>();
+  if (pairs <= 0) return GB_EUNSUPPORTED;
+  p.m_tiles = (int)((p.M + kPairM - 1) / kPairM);
+  p.n_tiles = (int)((p.N + kBN - 1) / kBN);
+  p.idesc |= ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kPairM >> 4) << 24);
+  CUtensorMap map_a, map_b, map_d = {}, map_sfa = {}, map_sfb = {};
+  const int64_t row = kKind == kFp4 ? p.K / 2 : p.K;
+  int rc = gb_tensor_map_operand(&map_a, A, p.M, row, row_bytes_elem, kBM);
+  if (rc != GB_OK) return rc;
+  rc = gb_tensor_map_operand(&map_b, B, p.N, row, row_bytes_elem, kBN / 2);
+  if (rc != GB_OK) return rc;
+  p.out_tma = p.N % 8 == 0;
+  if (p.out_tma) {
+    rc = gb_tensor_map_out(&map_d, p.D, p.M, p.N);
+    if (rc != GB_OK) return rc;
+  }
+  if (kKind == kFp4) {                                       // the planes as rows of 256 bytes: eight are four atoms
+    const int64_t a_rows = (p.M + 127) / 128 * p.k_tiles * 8, b_rows = (p.N + 127) / 128 * p.k_tiles * 8;
+    rc = gb_tensor_map_bytes_2d(&map_sfa, sfa, 256, (uint64_t)a_rows, 256, 256, 8);
+    if (rc != GB_OK) return rc;
+    rc = gb_tensor_map_bytes_2d(&map_sfb, sfb, 256, (uint64_t)b_rows, 256, 256, 8);
+    if (rc != GB_OK) return rc;
+  }
+  const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
+  GB_REQUIRE(tiles < (1ll << 31), "too many output tiles");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
+  cfg.blockDim = dim3(S::kThreads);
+  cfg.dynamicSmemBytes = S::kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = gb_pdl_enabled() ? 2 : 1;
+  gb_count_launch();
+  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<kKind, kBN>, map_a, map_b, map_d, map_sfa, map_sfb, p));
+  return GB_OK;
+}
+
+}  // namespace
+
+int gb_prepare_gemm_pair() {
+#define GB_ATTR(K, N) \
+  GB_CUDA_OK(cudaFuncSetAttribute((const void*)gemm_pair_kernel<K, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<K, N>::kSmem))
+  GB_ATTR(kBf16, 256);
+  GB_ATTR(kBf16, 192);
+  GB_ATTR(kFp8, 256);
+  GB_ATTR(kFp8, 192);
+  GB_ATTR(kFp4, 256);
+  GB_ATTR(kFp4, 192);
+#undef GB_ATTR
+  return GB_OK;
+}
+
+// From 129 rows on: with fewer, half of the pair's rows would be padding and the other kernel's
+// 128-row tiles do the same work on twice as many independent CTAs.
+bool gb_gemm_pair_applies(int64_t M) { return M > kBM; }
+
+namespace {
+// Width of a tile: 256 columns, or 192 where that saves more of the last wave than the sixth of extra
+// operand traffic costs (columns per pair and wave, 5% in favour of 256: 333 x 5120 x 17408 fp4 34 -> 32 us
+// with 192, 2048 x 34816 x 5120 165 -> 201).
+bool narrow_tiles(int64_t M, int64_t N) {
+  const int64_t pairs = gb_sm_count() / 2, mt = (M + kPairM - 1) / kPairM;
+  const int64_t w256 = (mt * ((N + 255) / 256) + pairs - 1) / pairs * 256, w192 = (mt * ((N + 191) / 192) + pairs - 1) / pairs * 192;
+  return w192 * 21 < w256 * 20;
+}
+}  // namespace
+
+int gb_gemm_pair(const void* A, const void* B, void* D, int64_t M, int64_t N, int64_t K, int kind, const float* a_scale,
+                 const float* b_scale, float global_scale, cudaStream_t stream) {
+  PairParams p = {};
+  p.M = M; p.N = N; p.K = K;
+  p.k_tiles = (int)(K * (kind == GB_GEMM_BF16 ? 2 : 1) / kSlabBytes);
+  p.idesc = (1u << 4) | (kind == GB_GEMM_BF16 ? (1u << 7) | (1u << 10) : 0u);
+  p.a_scale = a_scale; p.b_scale = b_scale;
+  p.global_scale = global_scale;
+  p.D = (uint16_t*)D;
+  p.status = gb_status_word();
+  const bool narrow = narrow_tiles(M, N);
+  if (kind == GB_GEMM_BF16)
+    return narrow ? run<kBf16, 192>(A, B, nullptr, nullptr, p, 2, stream) : run<kBf16, 256>(A, B, nullptr, nullptr, p, 2, stream);
+  return narrow ? run<kFp8, 192>(A, B, nullptr, nullptr, p, 1, stream) : run<kFp8, 256>(A, B, nullptr, nullptr, p, 1, stream);
+}
+
+int gb_gemm_fp4_pair(const void* A, const void* sfa, const void* B, const void* sfb, void* D, int64_t M, int64_t N, int64_t K,
+                     const float* a_scale, float global_scale, cudaStream_t stream) {
+  PairParams p = {};
+  p.M = M; p.N = N; p.K = K;
+  p.k_tiles = (int)(K / 256);
+  p.idesc = (1u << 7) | (1u << 10);
+  p.a_scale = a_scale;
+  p.global_scale = global_scale;
+  p.D = (uint16_t*)D;
+  p.status = gb_status_word();
+  const bool narrow = narrow_tiles(M, N);
+  return narrow ? run<kFp4, 192>(A, B, sfa, sfb, p, 1, stream) : run<kFp4, 256>(A, B, sfa, sfb, p, 1, stream);
+}
