@@ -425,83 +425,6 @@ int launch_expand(const gb_weight* w, int64_t row0, int64_t nrows, void* out0, v
   return GB_OK;
 }
 
-// ---- the literal format's native NVFP4 view, fast -------------------------------------------
-// Full mode, k = 8, E4M3-direct scales, one codebook: a codeword is one byte and its eight E2M1
-// values are one 32-bit word of a 256-entry table kept in shared memory.  Eight lanes take one
-// (row, superblock): each loads four codes as one word, looks them up and stores sixteen bytes
-// (128 contiguous bytes per unit); the first four of them also write the unit's sixteen group
-// scales, one word per 128 x 4 atom.  Memory-bound: 48 bytes read and 144 written per 256 weights.
-constexpr int kLitUnroll = 4;                              // steps in flight per warp, four units each
-
-__global__ void __launch_bounds__(kThreads)
-expand_literal_nvfp4_kernel(const uint8_t* __restrict__ qw, int64_t row_stride, const uint16_t* __restrict__ codebook,
-                            int64_t nrows, int64_t n_sb, uint4* __restrict__ out_packed,
-                            uint8_t* __restrict__ out_sf, int fold_sign) {
-  __shared__ uint32_t lut[256];
-  {
-    const uint4 e = __ldg(reinterpret_cast<const uint4*>(codebook) + threadIdx.x);     // kThreads == 256 entries
-    const uint32_t w[4] = {e.x, e.y, e.z, e.w};
-    uint32_t nib = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float v = gb_bf16_bits_to_f32((w[j >> 1] >> (16 * (j & 1))) & 0xffffu);
-      const float m = fabsf(v);
-      const uint32_t c = m < 2.0f ? (uint32_t)(m * 2.0f) : (m < 4.0f ? (uint32_t)m + 2u : (m < 6.0f ? 6u : 7u));
-      nib |= (c | (v < 0.0f ? 8u : 0u)) << (4 * j);
-    }
-    lut[threadIdx.x] = nib;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, sub = lane & 7, which = lane >> 3;
-  const int64_t units = nrows * n_sb;
-  const int64_t k_atoms = n_sb * 4;                        // atoms along K of one 128-row tile
-  const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
-  for (int64_t u0 = ((int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * (4 * kLitUnroll); u0 < units;
-       u0 += warps * (4 * kLitUnroll)) {
-    uint32_t codes[kLitUnroll], sc2[kLitUnroll], sc4[kLitUnroll];
-#pragma unroll
-    for (int i = 0; i < kLitUnroll; ++i) {
-      const int64_t u = u0 + 4 * i + which < units ? u0 + 4 * i + which : u0;
-      const int64_t r = u / n_sb, sb = u - r * n_sb;
-      const uint8_t* p = qw + r * row_stride + sb * 48;    // 16-byte aligned: rows are, and 48 is a multiple of 16
-      codes[i] = __ldg(reinterpret_cast<const uint32_t*>(p) + sub);
-      sc2[i] = __ldg(reinterpret_cast<const uint16_t*>(p + 32) + sub);                      // groups 2 sub, 2 sub + 1
-      sc4[i] = sub < 4 ? __ldg(reinterpret_cast<const uint32_t*>(p + 32) + sub) : 0u;       // the scales of atom `sub`
-    }
-#pragma unroll
-    for (int i = 0; i < kLitUnroll; ++i) {
-      const int64_t u = u0 + 4 * i + which;
-      if (u >= units) continue;
-      const int64_t r = u / n_sb, sb = u - r * n_sb;
-      uint32_t w0 = lut[codes[i] & 0xffu], w1 = lut[(codes[i] >> 8) & 0xffu];
-      uint32_t w2 = lut[(codes[i] >> 16) & 0xffu], w3 = lut[codes[i] >> 24];
-      if (fold_sign) {
-        if (sc2[i] & 0x80u) { w0 ^= 0x88888888u; w1 ^= 0x88888888u; }
-        if (sc2[i] & 0x8000u) { w2 ^= 0x88888888u; w3 ^= 0x88888888u; }
-      }
-      out_packed[u * 8 + sub] = make_uint4(w0, w1, w2, w3);
-      if (sub < 4) {
-        const int64_t off = (r / 128) * (512 * k_atoms) + (sb * 4 + sub) * 512 + (r % 32) * 16 + ((r / 32) % 4) * 4;
-        *reinterpret_cast<uint32_t*>(out_sf + off) = fold_sign ? (sc4[i] & 0x7F7F7F7Fu) : sc4[i];
-      }
-    }
-  }
-}
-
-int launch_expand_literal(const gb_weight* w, int64_t row0, int64_t nrows, void* out_packed, void* out_sf,
-                          int fold_sign, void* stream) {
-  const int64_t n_sb = w->K / 256, units = nrows * n_sb;
-  const int64_t per_cta = (kThreads / 32) * 4 * kLitUnroll;
-  int64_t blocks = (units + per_cta - 1) / per_cta;
-  const int64_t cap = (int64_t)gb_sm_count() * 16;
-  if (cap > 0 && blocks > cap) blocks = cap;
-  gb_count_launch();
-  expand_literal_nvfp4_kernel<<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(
-      w->qw + row0 * w->row_stride, w->row_stride, (const uint16_t*)w->codebook, nrows, n_sb, (uint4*)out_packed,
-      (uint8_t*)out_sf, fold_sign);
-  GB_LAUNCH_OK("expand_literal_nvfp4_kernel");
-  return GB_OK;
-}
 // The fp8 product formats k = 32 (four sub-tables of two values) and k = 16 (two sub-tables of four
 // values) -> the E4M3 value plane, one byte per weight: the sub-table entries are copied through as
 // they are.  Eight lanes per (row, superblock); a lane takes two codewords of each half of the
@@ -824,6 +747,225 @@ int launch_expand_product(const gb_weight* w, int64_t row0, int64_t nrows, void*
   GB_LAUNCH_OK("expand_product_kernel");
   return GB_OK;
 }
+// ---- native NVFP4 view, fast ------------------------------------------------------------------
+// The literal format (full mode, k = 8, E4M3 scales) and the two-tier product formats k = 12, 16, 20, 24
+// whose superblocks start on 4-byte boundaries (the resident slots do).  Eight lanes take one (row,
+// superblock): a lane fetches the one to three words that hold its four codewords, cuts them with
+// constant shifts, looks every (sub-)index up as its finished E2M1 nibbles and stores sixteen bytes; two
+// lanes join their group scales into the word of one 128 x 4 atom.  A CTA takes a run of rows and
+// rebuilds its tables where the codebook changes.
+//
+// Two thirds of the issue slots went to index arithmetic (64-bit divisions, bit windows of any width,
+// scale bytes fetched and looked up twice): 175 instructions per 32 lanes and step for the literal
+// format, 297 for K20.  34816 x 5120: literal 41 -> 33 us, K20 73 -> 54 us (5120 x 17408: 24 -> 19, 44 -> 31);
+// the bytes moved (133 and 178 MB) take 20 and 27 us.
+constexpr int kNvThreads = 512;
+constexpr int kNvUnroll = 2;                               // superblocks in flight per lane
+
+template <int F>
+struct NvFmt {
+  static constexpr bool kLit = F == 8;
+  static constexpr int kWords = kLit ? 1 : F <= 16 ? 2 : 3;              // words that hold 4 F bits from any 2-byte boundary
+  static constexpr int kEntries = kLit ? 256 : 2 << (F / 2);
+  static constexpr int kWide = kLit || F == 12 ? 2 : 1;                  // 16-bit halves of an entry
+  static constexpr int kCopies = F <= 16 ? 32 : F == 20 ? 8 : 4;
+  static constexpr int kShift = F == 20 ? 4 : F == 24 ? 3 : F == 16 ? 6 : 7;   // log2 of an entry's bytes, copies included
+  static constexpr int kLutBytes = kEntries << kShift;
+  static constexpr int kSmem = kLutBytes + (kLit ? 0 : 4096);            // and the two-tier scale bytes
+  static_assert(kCopies * kWide * 2 == 1 << kShift, "entry size");
+};
+
+struct NvArgs {
+  const uint8_t* qw;           // first row
+  int64_t row_stride, row0, nrows;
+  int slot, n_sb;              // bytes from superblock to superblock
+  int rows_per_cta;
+  const uint16_t* codebook;
+  const int32_t* cb_row_offset;
+  const float* compose;
+  uint4* out;
+  uint8_t* sf;
+  int fold_sign;
+};
+
+template <int F>
+__global__ void __launch_bounds__(kNvThreads, 3)
+expand_nvfp4_kernel(const __grid_constant__ NvArgs a) {
+  using T = NvFmt<F>;
+  extern __shared__ uint8_t smem[];
+  __shared__ int run_end_s;
+  const int tid = threadIdx.x, lane = tid & 31, sub = lane & 7;
+  uint8_t* comp_s = smem + T::kLutBytes;
+  gb_pdl_launch_dependents();
+  if (!T::kLit)
+#pragma unroll 4
+    for (int i = tid; i < 4096; i += kNvThreads) comp_s[i] = (uint8_t)gb_f32_to_e4m3(fminf(__ldg(a.compose + i), 448.0f));
+
+  const int64_t r_begin = (int64_t)blockIdx.x * a.rows_per_cta;
+  const int64_t r_end = r_begin + a.rows_per_cta < a.nrows ? r_begin + a.rows_per_cta : a.nrows;
+  const uint8_t* lut = smem + (lane & (T::kCopies - 1)) * T::kWide * 2;
+  const uint32_t n_sb = (uint32_t)a.n_sb;
+  const uint32_t dr = (kNvThreads / 8) / n_sb, ds = (kNvThreads / 8) % n_sb;   // a step of the CTA's lane groups
+  const int code_at = T::kLit ? 4 * sub : (sub * F / 2) & ~3;
+  const int cut = (sub * F / 2 & 2) * 8;                   // odd lanes of F = 12 and 20 start in mid-word
+
+  for (int64_t run = r_begin; run < r_end;) {
+    int64_t cb_base = 0, run_end = r_end;
+    if (a.cb_row_offset) {                                 // rows [run, run_end) use one codebook block
+      cb_base = a.cb_row_offset[a.row0 + run];
+      __syncthreads();
+      if (tid == 0) run_end_s = (int)(r_end - run);
+      __syncthreads();
+      for (int64_t r = run + tid; r < r_end; r += kNvThreads)
+        if (a.cb_row_offset[a.row0 + r] != (int32_t)cb_base) { atomicMin(&run_end_s, (int)(r - run)); break; }
+      __syncthreads();
+      run_end = run + run_end_s;
+    }
+    // an entry is converted once; its copies go out as 8 or 16 bytes a store, rotated by lane over the banks
+#pragma unroll 4
+    for (int e = tid; e < T::kEntries; e += kNvThreads) {
+      const uint16_t* c = a.codebook + cb_base + (int64_t)e * (T::kLit ? 8 : 4);
+      uint32_t nib = 0;
+#pragma unroll
+      for (int j = 0; j < (T::kLit ? 8 : 4); ++j) nib |= e2m1_nibble(__ldg(c + j)) << (4 * j);
+      if (T::kWide == 1) nib |= nib << 16;
+      constexpr int kVec = 1 << T::kShift >= 16 ? (1 << T::kShift) / 16 : 1;
+      if (T::kShift == 3) reinterpret_cast<uint2*>(smem)[e] = make_uint2(nib, nib);
+#pragma unroll
+      for (int q = 0; q < (T::kShift == 3 ? 0 : kVec); ++q)
+        reinterpret_cast<uint4*>(smem)[e * kVec + ((q + lane) & (kVec - 1))] = make_uint4(nib, nib, nib, nib);
+    }
+    __syncthreads();
+    if (run == r_begin) gb_pdl_wait();                     // the output may still be read by an earlier launch
+
+    const uint32_t units = (uint32_t)(run_end - run) * n_sb;
+    uint32_t u = (uint32_t)(tid >> 3);
+    uint32_t rr = u / n_sb, s = u - rr * n_sb;
+    auto step = [&](uint32_t& r2, uint32_t& s2) {
+      r2 += dr;
+      s2 += ds;
+      if (s2 >= n_sb) { s2 -= n_sb; ++r2; }
+    };
+    for (; u - (uint32_t)(lane >> 3) < units; u += kNvUnroll * (kNvThreads / 8)) {     // whole warps: the shuffle below
+      uint32_t w[kNvUnroll][T::kWords], sc[kNvUnroll], sup[kNvUnroll], row[kNvUnroll], col[kNvUnroll];
+      bool live[kNvUnroll];
+#pragma unroll
+      for (int i = 0; i < kNvUnroll; ++i) {
+        live[i] = u + i * (kNvThreads / 8) < units;
+        row[i] = live[i] ? rr : 0u;
+        col[i] = live[i] ? s : 0u;
+        const uint8_t* sb = a.qw + (run + row[i]) * a.row_stride + (int64_t)col[i] * a.slot;
+#pragma unroll
+        for (int q = 0; q < T::kWords; ++q) w[i][q] = __ldg(reinterpret_cast<const uint32_t*>(sb + code_at) + q);
+        if (T::kLit) sc[i] = __ldg(reinterpret_cast<const uint16_t*>(sb + 32) + sub);     // groups 2 sub, 2 sub + 1
+        else { sup[i] = __ldg(sb + 4 * F); sc[i] = __ldg(sb + 4 * F + 1 + sub); }
+        step(rr, s);
+      }
+#pragma unroll
+      for (int i = 0; i < kNvUnroll; ++i) {
+        uint32_t v[4];
+        if (T::kLit) {
+          v[0] = *reinterpret_cast<const uint32_t*>(lut + ((w[i][0] & 0xFFu) << 7));
+          v[1] = *reinterpret_cast<const uint32_t*>(lut + ((w[i][0] >> 1) & 0x7F80u));
+          v[2] = *reinterpret_cast<const uint32_t*>(lut + ((w[i][0] >> 9) & 0x7F80u));
+          v[3] = *reinterpret_cast<const uint32_t*>(lut + ((w[i][0] >> 17) & 0x7F80u));
+        } else {
+          uint32_t b[3] = {w[i][0], w[i][1], T::kWords == 3 ? w[i][T::kWords - 1] : 0u};
+          if (F == 12 || F == 20) {
+            b[0] = __funnelshift_r(b[0], b[1], cut);
+            b[1] = __funnelshift_r(b[1], b[2], cut);
+            b[2] >>= cut;
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t half[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              constexpr uint32_t kMask = ((1u << (F / 2)) - 1u) << T::kShift;
+              const int bit = c * F + h * (F / 2), wd = bit >> 5, at = bit & 31;
+              uint32_t x;                                  // the sub-index shifted to its entry's byte offset
+              if (at + F / 2 > 32) x = __funnelshift_r(b[wd], b[wd + 1 < 3 ? wd + 1 : 2], at) << T::kShift;
+              else x = at >= T::kShift ? b[wd] >> (at - T::kShift) : b[wd] << (T::kShift - at);
+              const uint8_t* at_p = lut + (h * T::kLutBytes / 2) + (x & kMask);
+              half[h] = T::kWide == 2 ? *reinterpret_cast<const uint32_t*>(at_p) : *reinterpret_cast<const uint16_t*>(at_p);
+            }
+            v[c] = half[0] | (half[1] << 16);
+          }
+        }
+        uint32_t sc2 = sc[i];
+        if (!T::kLit) {
+          const uint8_t* t = comp_s + sup[i] * 16u;
+          sc2 = t[sc[i] & 15u] | ((uint32_t)t[sc[i] >> 4] << 8);
+        }
+        if (a.fold_sign) {                                 // UE4M3 scale factors carry no sign
+          if (sc2 & 0x80u) { v[0] ^= 0x88888888u; v[1] ^= 0x88888888u; }
+          if (sc2 & 0x8000u) { v[2] ^= 0x88888888u; v[3] ^= 0x88888888u; }
+          sc2 &= 0x7F7Fu;
+        }
+        const uint32_t sc4 = sc2 | (__shfl_down_sync(0xffffffffu, sc2, 1) << 16);
+        if (live[i]) {
+          const int64_t r = run + row[i];
+          a.out[(r * n_sb + col[i]) * 8 + sub] = make_uint4(v[0], v[1], v[2], v[3]);
+          if ((sub & 1) == 0)
+            *reinterpret_cast<uint32_t*>(a.sf + (r >> 7) * (int64_t)(2048u * n_sb) + (int64_t)(col[i] * 2048u) +
+                                         (uint32_t)(sub * 256) + ((uint32_t)r & 31u) * 16u + (((uint32_t)r >> 5) & 3u) * 4u) = sc4;
+        }
+      }
+    }
+    run = run_end;
+    if (run < r_end) __syncthreads();                      // the next run rebuilds the tables
+  }
+}
+
+// GB_EUNSUPPORTED: the weight is not the kernel's.
+int launch_expand_nvfp4(const gb_weight* w, int64_t row0, int64_t nrows, void* out, void* sf, int fold_sign, void* stream) {
+  const gb_format& f = w->fmt;
+  const bool lit = f.mode == GB_MODE_FULL && f.k_bits == 8 && f.scale_coding == GB_SCALE_V1;
+  const bool prod = f.mode == GB_MODE_PRODUCT && f.n_sub == 2 && f.scale_coding == GB_SCALE_V2 &&
+                    (f.k_bits == 12 || f.k_bits == 16 || f.k_bits == 20 || f.k_bits == 24);
+  if (!(lit || prod) || f.type_size % 4 != 0 || w->row_stride % 4 != 0 || ((uintptr_t)w->qw & 3u) != 0 ||
+      ((uintptr_t)out & 15u) != 0 || ((uintptr_t)sf & 3u) != 0 || ((uintptr_t)w->codebook & 1u) != 0)
+    return GB_EUNSUPPORTED;
+  ExpandArgs e;
+  if (lit && nrows == 0 && row0 >= 0 && row0 <= w->rows) return GB_OK;
+  int rc = make_expand_args(w, row0, nrows, &e);
+  if (rc != GB_OK) return rc;
+  GB_REQUIRE(out != nullptr, "null output");
+  if (prod && (e.split.width[0] != f.k_bits / 2 || e.split.width[1] != f.k_bits / 2 || e.split.shift[0] != 0 ||
+               e.split.shift[1] != f.k_bits / 2 || e.split.base[0] != 0 || e.split.base[1] != 4 << (f.k_bits / 2)))
+    return GB_EUNSUPPORTED;
+  NvArgs a = {};
+  a.qw = w->qw + row0 * w->row_stride;
+  a.row_stride = w->row_stride; a.row0 = row0; a.nrows = nrows;
+  a.slot = f.type_size;
+  a.n_sb = (int)(w->K / 256);
+  a.codebook = (const uint16_t*)w->codebook;
+  a.cb_row_offset = w->cb_row_offset;
+  a.compose = w->compose;
+  a.out = (uint4*)out; a.sf = (uint8_t*)sf; a.fold_sign = fold_sign;
+  // one wave of three CTAs per SM over the rows, at least 128 superblocks each so that the tables pay
+  const int64_t ctas = (int64_t)gb_sm_count() * 3;
+  if (ctas <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
+  int64_t rows_per = (nrows + ctas - 1) / ctas;
+  const int64_t least = (128 + a.n_sb - 1) / a.n_sb;
+  if (rows_per < least) rows_per = least;
+  GB_REQUIRE(rows_per * a.n_sb < (1ll << 30), "too many superblocks per CTA");
+  a.rows_per_cta = (int)rows_per;
+  const unsigned blocks = (unsigned)((nrows + rows_per - 1) / rows_per);
+#define GB_EXPAND_NVFP4(F)                                                                                              \
+  GB_CUDA_OK(cudaFuncSetAttribute((const void*)expand_nvfp4_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, NvFmt<F>::kSmem)); \
+  GB_CUDA_OK(gb_launch(expand_nvfp4_kernel<F>, dim3(blocks), dim3(kNvThreads), NvFmt<F>::kSmem, (cudaStream_t)stream, a))
+  switch (f.k_bits) {
+    case 8: GB_EXPAND_NVFP4(8); break;
+    case 12: GB_EXPAND_NVFP4(12); break;
+    case 16: GB_EXPAND_NVFP4(16); break;
+    case 20: GB_EXPAND_NVFP4(20); break;
+    default: GB_EXPAND_NVFP4(24); break;
+  }
+#undef GB_EXPAND_NVFP4
+  return GB_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -863,17 +1005,9 @@ int gb_expand_fp4_nvfp4(const gb_weight* w, int64_t row0, int64_t nrows, void* o
                         void* out_sf, int sf_swizzled, void* stream) {
   GB_REQUIRE(w && w->fmt.grid == GB_GRID_FP4, "gb_expand_fp4_nvfp4 wants an fp4-grid weight");
   GB_REQUIRE(out_sf != nullptr, "null scale-factor output");
-  const gb_format& f = w->fmt;
-  if (sf_swizzled != 0 && f.mode == GB_MODE_FULL && f.k_bits == 8 && f.scale_coding == GB_SCALE_V1 &&
-      w->cb_row_offset == nullptr && ((uintptr_t)w->codebook & 15u) == 0 && ((uintptr_t)out_packed & 15u) == 0 &&
-      ((uintptr_t)out_sf & 3u) == 0 && ((uintptr_t)w->qw & 15u) == 0 && w->row_stride % 16 == 0 && kThreads == 256) {
-    int rc = gb_check_weight(w);
-    if (rc != GB_OK) return rc;
-    GB_REQUIRE(out_packed != nullptr, "null output pointer");
-    GB_REQUIRE(row0 >= 0 && nrows >= 0 && row0 + nrows <= w->rows, "rows [%lld, %lld) outside [0, %lld)",
-               (long long)row0, (long long)(row0 + nrows), (long long)w->rows);
-    if (nrows == 0) return GB_OK;
-    return launch_expand_literal(w, row0, nrows, out_packed, out_sf, sf_swizzled == 2, stream);
+  if (sf_swizzled != 0) {
+    const int rc = launch_expand_nvfp4(w, row0, nrows, out_packed, out_sf, sf_swizzled == 2, stream);
+    if (rc != GB_EUNSUPPORTED) return rc;
   }
   if (sf_swizzled != 0 && ((uintptr_t)out_sf & 3u) == 0 && product_serves(w, out_packed, kOutNvfp4))
     return launch_expand_product<kOutNvfp4>(w, row0, nrows, out_packed, out_sf, sf_swizzled == 2, stream);

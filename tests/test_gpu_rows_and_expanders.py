@@ -105,3 +105,23 @@ def test_combine_both_widths(dev, T, topk, H):
     yw = torch.where(live[:, None], y.float() * w.to(torch.bfloat16).float()[:, None], torch.zeros((), device=dev))
     want = yw.reshape(T, topk, H).double().sum(1)
     assert torch.all((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-6)
+
+
+@pytest.mark.parametrize("rows,K,books", [(1, 256, 1), (129, 512, 3), (1000, 1024, 7), (700, 5120, 1)])
+@pytest.mark.parametrize("k", [8, 12, 16, 20, 24])
+def test_nvfp4_view_of_resident_slots_is_exact(dev, k, rows, K, books):
+    """The expander of aligned superblocks: one superblock a row, fewer superblocks than a step of the
+    CTA, rows that end inside a step, a codebook per part."""
+    from gridbook_b200 import codec, kernels, synth
+    from gridbook_b200.formats import NVFP4_LITERAL, CBFormat
+    fmt = NVFP4_LITERAL if k == 8 else CBFormat("fp4", k, n_sub=2, scale_coding="v2")
+    d = synth.make_linear(fmt, rows, K, seed=rows + k, n_books=books, super_span=None)
+    up, slot = d, codec.resident_slot(fmt)
+    if slot is not None:
+        up = dict(d, fmt=fmt.padded(slot), qw=codec.pad_superblocks(torch.from_numpy(d["qw"]), fmt.type_size, slot).numpy())
+    off = d["cb_row_offset"] if d["cb_row_offset"] is not None else np.zeros(rows, np.int32)
+    rp, rs = O.decode_nvfp4_tile(d["qw"], d["cb"], off, N=rows, K=K, compose=d["compose"],
+                                 **{a: v for a, v in oracle_kwargs(fmt).items() if a != "grid"})
+    packed, sf = kernels.expand_fp4_nvfp4(synth.to_device_weight(up, dev), swizzled=True)
+    assert np.array_equal(packed.cpu().numpy(), rp)
+    assert np.array_equal(sf.cpu().numpy(), O.swizzle_sf_plane(rs))
