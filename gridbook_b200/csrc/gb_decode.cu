@@ -760,7 +760,6 @@ int launch_expand_product(const gb_weight* w, int64_t row0, int64_t nrows, void*
 // format, 297 for K20.  34816 x 5120: literal 41 -> 33 us, K20 73 -> 54 us (5120 x 17408: 24 -> 19, 44 -> 31);
 // the bytes moved (133 and 178 MB) take 20 and 27 us.
 constexpr int kNvThreads = 512;
-constexpr int kNvUnroll = 2;                               // superblocks in flight per lane
 
 template <int F>
 struct NvFmt {
@@ -770,6 +769,7 @@ struct NvFmt {
   static constexpr int kWide = kLit || F == 12 ? 2 : 1;                  // 16-bit halves of an entry
   static constexpr int kCopies = F <= 16 ? 32 : F == 20 ? 8 : 4;
   static constexpr int kShift = F == 20 ? 4 : F == 24 ? 3 : F == 16 ? 6 : 7;   // log2 of an entry's bytes, copies included
+  static constexpr int kUnroll = kLit ? 4 : 2;                           // superblocks in flight per lane
   static constexpr int kLutBytes = kEntries << kShift;
   static constexpr int kSmem = kLutBytes + (kLit ? 0 : 4096);            // and the two-tier scale bytes
   static_assert(kCopies * kWide * 2 == 1 << kShift, "entry size");
@@ -805,7 +805,7 @@ expand_nvfp4_kernel(const __grid_constant__ NvArgs a) {
   const int64_t r_end = r_begin + a.rows_per_cta < a.nrows ? r_begin + a.rows_per_cta : a.nrows;
   const uint8_t* lut = smem + (lane & (T::kCopies - 1)) * T::kWide * 2;
   const uint32_t n_sb = (uint32_t)a.n_sb;
-  const uint32_t dr = (kNvThreads / 8) / n_sb, ds = (kNvThreads / 8) % n_sb;   // a step of the CTA's lane groups
+  const uint32_t dr = (kNvThreads / 32) / n_sb, ds = (kNvThreads / 32) % n_sb;   // a step of the CTA's warps
   const int code_at = T::kLit ? 4 * sub : (sub * F / 2) & ~3;
   const int cut = (sub * F / 2 & 2) * 8;                   // odd lanes of F = 12 and 20 start in mid-word
 
@@ -838,31 +838,27 @@ expand_nvfp4_kernel(const __grid_constant__ NvArgs a) {
     __syncthreads();
     if (run == r_begin) gb_pdl_wait();                     // the output may still be read by an earlier launch
 
-    const uint32_t units = (uint32_t)(run_end - run) * n_sb;
-    uint32_t u = (uint32_t)(tid >> 3);
+    // a warp's unit: one superblock of four neighbouring rows, whose scale words lie 16 bytes apart
+    const uint32_t rows = (uint32_t)(run_end - run), units = (rows + 3) / 4 * n_sb;
+    uint32_t u = (uint32_t)(tid >> 5);
     uint32_t rr = u / n_sb, s = u - rr * n_sb;
-    auto step = [&](uint32_t& r2, uint32_t& s2) {
-      r2 += dr;
-      s2 += ds;
-      if (s2 >= n_sb) { s2 -= n_sb; ++r2; }
-    };
-    for (; u - (uint32_t)(lane >> 3) < units; u += kNvUnroll * (kNvThreads / 8)) {     // whole warps: the shuffle below
-      uint32_t w[kNvUnroll][T::kWords], sc[kNvUnroll], sup[kNvUnroll], row[kNvUnroll], col[kNvUnroll];
-      bool live[kNvUnroll];
+    for (; u < units; u += T::kUnroll * (kNvThreads / 32)) {
+      uint32_t w[T::kUnroll][T::kWords], sc[T::kUnroll], sup[T::kUnroll], row[T::kUnroll], col[T::kUnroll];
 #pragma unroll
-      for (int i = 0; i < kNvUnroll; ++i) {
-        live[i] = u + i * (kNvThreads / 8) < units;
-        row[i] = live[i] ? rr : 0u;
-        col[i] = live[i] ? s : 0u;
-        const uint8_t* sb = a.qw + (run + row[i]) * a.row_stride + (int64_t)col[i] * a.slot;
+      for (int i = 0; i < T::kUnroll; ++i) {
+        row[i] = rr * 4 + (uint32_t)(lane >> 3);
+        col[i] = s;
+        const uint8_t* sb = a.qw + (run + min(row[i], rows - 1)) * a.row_stride + (int64_t)col[i] * a.slot;
 #pragma unroll
         for (int q = 0; q < T::kWords; ++q) w[i][q] = __ldg(reinterpret_cast<const uint32_t*>(sb + code_at) + q);
         if (T::kLit) sc[i] = __ldg(reinterpret_cast<const uint16_t*>(sb + 32) + sub);     // groups 2 sub, 2 sub + 1
         else { sup[i] = __ldg(sb + 4 * F); sc[i] = __ldg(sb + 4 * F + 1 + sub); }
-        step(rr, s);
+        rr += dr;
+        s += ds;
+        if (s >= n_sb) { s -= n_sb; ++rr; }
       }
 #pragma unroll
-      for (int i = 0; i < kNvUnroll; ++i) {
+      for (int i = 0; i < T::kUnroll; ++i) {
         uint32_t v[4];
         if (T::kLit) {
           v[0] = *reinterpret_cast<const uint32_t*>(lut + ((w[i][0] & 0xFFu) << 7));
@@ -903,7 +899,7 @@ expand_nvfp4_kernel(const __grid_constant__ NvArgs a) {
           sc2 &= 0x7F7Fu;
         }
         const uint32_t sc4 = sc2 | (__shfl_down_sync(0xffffffffu, sc2, 1) << 16);
-        if (live[i]) {
+        if (row[i] < rows) {
           const int64_t r = run + row[i];
           a.out[(r * n_sb + col[i]) * 8 + sub] = make_uint4(v[0], v[1], v[2], v[3]);
           if ((sub & 1) == 0)
@@ -949,6 +945,7 @@ int launch_expand_nvfp4(const gb_weight* w, int64_t row0, int64_t nrows, void* o
   int64_t rows_per = (nrows + ctas - 1) / ctas;
   const int64_t least = (128 + a.n_sb - 1) / a.n_sb;
   if (rows_per < least) rows_per = least;
+  rows_per = (rows_per + 3) / 4 * 4;
   GB_REQUIRE(rows_per * a.n_sb < (1ll << 30), "too many superblocks per CTA");
   a.rows_per_cta = (int)rows_per;
   const unsigned blocks = (unsigned)((nrows + rows_per - 1) / rows_per);
