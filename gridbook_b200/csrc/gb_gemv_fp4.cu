@@ -105,6 +105,8 @@ struct Fp4Params {
   const int32_t* seg;        // grouped: [E + 1]
   const int32_t* row_map;
   int tiles_n;
+  int E;
+  uint32_t seg_off;          // their copy in shared memory, 0: no room
 };
 
 // Columns.  Narrow (up to 16 rows per pass): term t of row m in column 12 (m / 4) + 4 t + m % 4, so that the
@@ -257,7 +259,8 @@ GB_DEVINL uint32_t nib4(uint2 w) {
 // formats (one superblock per stage, room for two stages) let every warpgroup see every stage.
 template <int F> constexpr bool kAllSee = Fmt<F>::kSbPerStage == 1;
 
-// Lookup tables of one codebook, built by the 512 decoder threads.
+// Lookup tables of one codebook, built by the 512 decoder threads; the order of a thread's stores rotates
+// with it, since the entries of neighbouring threads start in the same bank.
 template <int F>
 GB_DEVINL void build_lut(const uint16_t* cb, int d, uint32_t lut) {
   if constexpr (F == kLit) {
@@ -265,7 +268,7 @@ GB_DEVINL void build_lut(const uint16_t* cb, int d, uint32_t lut) {
     const uint4 q = *reinterpret_cast<const uint4*>(cb + e * 8);
     const uint32_t w = nib4(make_uint2(q.x, q.y)) | (nib4(make_uint2(q.z, q.w)) << 16);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sts128(lut + (uint32_t)e * 256u + (uint32_t)(half * 4 + j) * 16u, make_uint4(w, w, w, w));
+    for (int j = 0; j < 4; ++j) sts128(lut + (uint32_t)e * 256u + (uint32_t)((half * 4 + j + d) & 7) * 16u, make_uint4(w, w, w, w));
   } else {
     using T = Fmt<F>;
     const uint2* t0 = reinterpret_cast<const uint2*>(cb);
@@ -274,7 +277,8 @@ GB_DEVINL void build_lut(const uint16_t* cb, int d, uint32_t lut) {
       uint32_t w = nib4(t0[e]);
       if (e < (1 << T::kW1)) w |= nib4(t1[e]) << 16;
 #pragma unroll
-      for (int j = 0; j < T::kCopies / 4; ++j) sts128(lut + (uint32_t)e * T::kStride + (uint32_t)j * 16u, make_uint4(w, w, w, w));
+      for (int j = 0; j < T::kCopies / 4; ++j)
+        sts128(lut + (uint32_t)e * T::kStride + (uint32_t)((j + e / (128 / T::kStride)) & (T::kCopies / 4 - 1)) * 16u, make_uint4(w, w, w, w));
     }
   }
 }
@@ -313,6 +317,19 @@ GB_DEVINL uint32_t four_scales(uint4 t, uint32_t c) {
   uint32_t m;                                              // 0xFF where the code is 8..15 (sign replication), else 0x80
   asm("prmt.b32 %0, %1, %1, %2;" : "=r"(m) : "r"(0x80808080u), "r"(c & 0x8888u));
   return lo ^ ((lo ^ hi) & m & 0x7F7F7F7Fu);
+}
+
+// The E4M3 byte of every (super, sub) pair of the two-tier formats.
+template <int F>
+GB_DEVINL void build_scale_tab(const Fp4Params& p, int d, uint32_t scale_tab) {
+  if constexpr (F != kLit) {
+    for (int i = d * 4; i < 4096; i += 4 * 32 * kDecWarps) {
+      uint32_t w = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w |= gb_f32_to_e4m3(fminf(__ldg(p.compose + i + j), 448.0f)) << (8 * j);
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(scale_tab + (uint32_t)i), "r"(w) : "memory");
+    }
+  }
 }
 
 template <bool kGrouped, int F>
@@ -392,7 +409,27 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   }
   const uint32_t tmem_base = *tmem_slot;
 
-  if (kGrouped) gb_pdl_wait();                             // the segment offsets come from an earlier launch
+  int have_role = -1;
+  if (kGrouped) {
+    // the tables need nothing of an earlier launch, the segment offsets do: every role looks through the
+    // experts for its tiles, so they are copied next to it (ten tiles a CTA, 500 clocks each from L2)
+    if (warp >= kCtlWarps) {
+      build_scale_tab<F>(p, threadIdx.x - 32 * kCtlWarps, scale_tab);
+      build_lut<F>(reinterpret_cast<const uint16_t*>(p.codebook), threadIdx.x - 32 * kCtlWarps, kLut | win);
+      have_role = 0;
+    }
+    gb_pdl_wait();
+    if (p.seg_off != 0)
+      for (int i = threadIdx.x; i <= p.E; i += kThreads)
+        asm volatile("st.shared.s32 [%0], %1;" ::"r"((p.seg_off | win) + 4u * (uint32_t)i), "r"(p.seg[i]) : "memory");
+    __syncthreads();
+  }
+  auto seg_at = [&](int e) {
+    if (p.seg_off == 0) return p.seg[e];
+    int v;
+    asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"((p.seg_off | win) + 4u * (uint32_t)e));
+    return v;
+  };
   struct Tile { int n0, n_end, w_row0, lo, cnt, n_pass, x_tile, role; };
   auto tile_at = [&](int t) {
     Tile R;
@@ -401,8 +438,8 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       R.n0 = (t - e * p.tiles_n) * kBM;
       R.n_end = (int)p.N;
       R.w_row0 = e * (int)p.N + R.n0;
-      R.lo = p.seg[e];
-      R.cnt = p.seg[e + 1] - R.lo;
+      R.lo = seg_at(e);
+      R.cnt = seg_at(e + 1) - R.lo;
       R.n_pass = R.cnt > 0 ? (R.cnt + p.pass_rows - 1) / p.pass_rows : 0;
       R.x_tile = R.lo / p.pass_rows + e;                   // tiles of different (expert, pass) never coincide
       R.role = 0;
@@ -462,7 +499,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     if (lane == 0 && i < n_iss) {
       const uint32_t acc = tmem_base + (uint32_t)i * acc_stride;
       const uint32_t sf_col = 48u + (wide ? (uint32_t)i * 16u : 0u);
-      const int u_first = wide ? 0 : i, u_step = wide ? 1 : 4;
+      const int u_step = wide ? 1 : 4;
       const uint64_t db0 = desc_sw128(x_ring + (uint32_t)sfx);
       int g0 = 0, item = 0;                                // units / (tile, pass) items since the start
       for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
@@ -476,9 +513,10 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             wait(acc_empty, (item - 1) & 1, abort_flag, p.status, 44);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           }
+          const int u_first = wide ? 0 : (i - g0) & 3;
           for (int u = u_first; u < units; u += u_step) {
             const int g = g0 + u, s = g & x_mask;
-            const uint32_t a = tmem_base + buf_col0 + (uint32_t)(u & 3) * buf_stride, off = (uint32_t)s * x_stage;
+            const uint32_t a = tmem_base + buf_col0 + (uint32_t)(g & 3) * buf_stride, off = (uint32_t)s * x_stage;
             const uint64_t db = db0 + (uint64_t)(off >> 4);
             wait(full + 8 * s, (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 45);
             if (*abort_flag) break;
@@ -500,40 +538,53 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t buf = lane_base + buf_col0 + (uint32_t)wg * buf_stride;
     const uint32_t lane4 = win | (F == kLit ? (uint32_t)lane * 4u : (uint32_t)(lane & ((int)(T::kStride / 4) - 1)) * 4u);
-    int have_role = -1;
-    if constexpr (F != kLit) {
-      for (int i = d; i < 4096; i += 32 * kDecWarps) {
-        const uint32_t b = gb_f32_to_e4m3(fminf(__ldg(p.compose + i), 448.0f));
-        asm volatile("st.shared.u8 [%0], %1;" ::"r"(scale_tab + (uint32_t)i), "r"(b) : "memory");
-      }
-    }
+    if (!kGrouped) build_scale_tab<F>(p, d, scale_tab);
     bool waited = false;
+    float xs0 = 0.0f, xs1 = 0.0f;                            // powers of two of rows lane, lane + 32
     int item = 0, g0 = 0, n0 = 0;                            // items, units and raw stages so far
     uint32_t flip = 0;
     const int stages = (units + T::kSbPerStage - 1) / T::kSbPerStage;
-    for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
-      const Tile R = tile_at(t);
-      if (R.n_pass == 0) continue;
-      if (R.role != have_role) {                             // the CTA's rows change codebook
+    // An item's accumulators are read out after the warpgroup has decoded its first unit of the NEXT item:
+    // the last multiplications, their completion and the read-out then overlap decoding, and the next
+    // item's multiplications find their operands ready.  (Nothing that first unit waits for needs this
+    // read-out: its buffer, its activations' slot and its raw stage were last used by earlier items.)
+    int t = blockIdx.x, pass = 0, out_t = -1, out_pass = 0;  // current item; the item to be read out
+    Tile R = {};
+    auto settle = [&]() {                                    // t: the next tile with rows, from t on
+      for (; t < p.n_tiles; t += gridDim.x) {
+        R = tile_at(t);
+        if (R.n_pass > 0) break;
+      }
+    };
+    settle();
+    while (t < p.n_tiles || out_t >= 0) {
+      const bool live = t < p.n_tiles;
+      if (live && R.role != have_role) {                     // the CTA's rows change codebook
         if (have_role >= 0) asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
         build_lut<F>(reinterpret_cast<const uint16_t*>(p.codebook) + p.role[R.role].cb, d, kLut | win);
         have_role = R.role;
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
       }
-      if (!waited) { gb_pdl_wait(); waited = true; }         // y may still be read by the launch ahead
-      for (int pass = 0; pass < R.n_pass; ++pass, ++item, g0 += units, n0 += stages) {
-        const int rows = min(p.pass_rows, R.cnt - pass * p.pass_rows);
-        const float* xsc = p.x_scale + (int64_t)(R.x_tile + pass) * p.pass_rows;
-        const float xs0 = lane < rows ? xsc[lane] : 0.0f, xs1 = lane + 32 < rows ? xsc[lane + 32] : 0.0f;
+      if (!waited) {                                         // y may still be read by the launch ahead
+        gb_pdl_wait();
+        waited = true;
+        if (!kGrouped) {
+          xs0 = lane < p.M ? p.x_scale[lane] : 0.0f;
+          xs1 = lane + 32 < p.M ? p.x_scale[lane + 32] : 0.0f;
+        }
+      }
+      {
+        const int u_end = live ? stages * T::kSbPerStage : 0, u_step = kAllSee<F> ? 1 : 4;
+        int u = kAllSee<F> ? 0 : (wg - g0) & 3;
 #pragma unroll 1
-        for (int u = kAllSee<F> ? 0 : wg; u < stages * T::kSbPerStage; u += kAllSee<F> ? 1 : 4) {
+        do {
           const int n = n0 + u / T::kSbPerStage, rs = n & raw_mask;
-          if (kAllSee<F> && (u & 3) != wg) {
+          const bool mine = !kAllSee<F> || ((g0 + u) & 3) == wg;
+          if (u < u_end && !mine) {
             wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
             if (lane == 0) mbar_arrive(raw_empty + 8 * rs);
-            continue;
           }
-          if (u < units) {
+          if (mine && u < units && live) {
             wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
             const uint32_t stage = raw_ring + (uint32_t)rs * G::kBoxBytes + (uint32_t)(u % T::kSbPerStage) * T::kSb;
             const uint32_t rp = stage + (uint32_t)row * G::kPitch;
@@ -579,10 +630,9 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
               sg = st + (uint32_t)lane * 16u;
               sg_step = 512u;
             }
-            // The buffer's last unit has been multiplied (at the start of an item all have).  The slot's
-            // next completion is a later unit of this warpgroup, so it cannot run ahead of this wait.
+            // The buffer's last unit has been multiplied.  The slot's next completion is a later unit of this warpgroup, so it cannot run ahead of this wait.
             const int g = g0 + u;
-            if (u >= 4) wait(done + 8 * ((g - 4) & x_mask), (uint32_t)((g - 4) >> x_log) & 1u, abort_flag, p.status, 48);
+            if (g >= 4) wait(done + 8 * ((g - 4) & x_mask), (uint32_t)((g - 4) >> x_log) & 1u, abort_flag, p.status, 48);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             tmem_st32(buf, v);
             uint32_t any = 0;
@@ -620,93 +670,133 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * (g & x_mask));
           }
-          if ((F == kLit || u >= units) && lane == 0) mbar_arrive(raw_empty + 8 * rs);   // also for a stage's missing second superblock
-        }
-
-        // ------------------------- read-out ------------------------------------
-        wait(acc_full, item & 1, abort_flag, p.status, 49);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const bool ok = *abort_flag == 0;
-        const int64_t col = (int64_t)R.n0 + row;
-        const uint32_t Rt = (uint32_t)term_rows(wide, rows);
-        auto emit = [&](int m, float sum) {
-          const float scale = __shfl_sync(0xffffffffu, m < 32 ? xs0 : xs1, m & 31);
-          if (m >= rows) return;
-          const float val = sum * scale;
-          if (!kGrouped && p.slices > 1) {
-            // into the shared memory of the row's owner: slot [row / slices][slice][128 weight rows]
-            uint32_t dst;
-            const uint32_t local = (p.red_off | win) + (uint32_t)(((m / p.slices) * p.slices + slice) * kBM + row) * 4u;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(local), "r"(m % p.slices));
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(val) : "memory");
-          } else if (ok && col < R.n_end) {
-            int64_t orow = m;
+          if (mine && u < u_end && (F == kLit || u >= units) && lane == 0) mbar_arrive(raw_empty + 8 * rs);   // also for a stage's missing second superblock
+          if (out_t >= 0 && (mine || u + u_step >= u_end)) {
+            // ------------------------- read-out ------------------------------------
+            // Sums into registers, the accumulators handed back, then the stores.
+            const Tile Q = tile_at(out_t);
+            const int rows = min(p.pass_rows, Q.cnt - out_pass * p.pass_rows);
+            int to0 = lane, to1 = lane + 32;                 // output rows
             if (kGrouped) {
-              const int j = R.lo + pass * p.pass_rows + m;         // sorted position of the row
-              orow = p.row_map ? p.row_map[j] : j;
+              const float* xsc = p.x_scale + (int64_t)(Q.x_tile + out_pass) * p.pass_rows;
+              xs0 = lane < rows ? xsc[lane] : 0.0f;
+              xs1 = lane + 32 < rows ? xsc[lane + 32] : 0.0f;
+              to0 += Q.lo + out_pass * p.pass_rows;          // sorted positions
+              to1 = to0 + 32;
+              if (p.row_map) {
+                to0 = lane < rows ? p.row_map[to0] : 0;
+                to1 = lane + 32 < rows ? p.row_map[to1] : 0;
+              }
             }
-            p.y[orow * p.N + col] = (uint16_t)gb_f32_to_bf16_bits(val * p.global_scale);
-          }
-        };
-        if (wide) {
-          for (int c = wg; c * 8 < rows; c += 4) {
-            uint32_t h[8], l[8], e[8];
-            const uint32_t at = lane_base + (uint32_t)(c * 8);
-            tmem_ld8(at, h);
-            tmem_ld8(at + 128u, l);
-            tmem_ld8(at + Rt, e);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            out_t = -1;
+            wait(acc_full, (item - 1) & 1, abort_flag, p.status, 49);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const bool ok = *abort_flag == 0;
+            const int64_t col = (int64_t)Q.n0 + row;
+            const uint32_t Rt = (uint32_t)term_rows(wide, rows);
+            float sum[16];
+            if (wide) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-              emit(c * 8 + i, fmaf(__uint_as_float(e[i]), 0x1p-7f, fmaf(__uint_as_float(l[i]), 0x1p-4f, __uint_as_float(h[i]))));
-          }
-        } else if (wg * 4 < rows) {
-          // four rows per warpgroup; issuers without a unit leave their accumulator untouched
-          const int accs = min(4, units);
-          float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+              for (int j = 0; j < 2; ++j) {
+                const int c = wg + 4 * j;
+                if (c * 8 >= rows) break;
+                uint32_t h[8], l[8], e[8];
+                const uint32_t at = lane_base + (uint32_t)(c * 8);
+                tmem_ld8(at, h);
+                tmem_ld8(at + 128u, l);
+                tmem_ld8(at + Rt, e);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int a0 = 0; a0 < 4; a0 += 2) {
-            if (a0 >= accs) break;
-            uint32_t v[2][16];
-            const uint32_t at = lane_base + (uint32_t)(wg * 12);
-            tmem_ld16(at + (uint32_t)a0 * acc_stride, v[0]);
-            tmem_ld16(at + (uint32_t)min(a0 + 1, accs - 1) * acc_stride, v[1]);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                for (int i = 0; i < 8; ++i)
+                  sum[8 * j + i] = fmaf(__uint_as_float(e[i]), 0x1p-7f, fmaf(__uint_as_float(l[i]), 0x1p-4f, __uint_as_float(h[i])));
+              }
+            } else if (wg * 4 < rows) {
+              // four rows per warpgroup; issuers without a unit leave their accumulator untouched.  Units 0, 4, ..
+              // of the item first, then 1, 5, ..: the order does not depend on where the item's first unit fell
+              const int accs = min(4, units), a_first = g0 - units;
 #pragma unroll
-            for (int a = 0; a < 2; ++a)
+              for (int i = 0; i < 4; ++i) sum[i] = 0.0f;
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
-                if (a0 + a < accs)
-                  sum[i] += fmaf(__uint_as_float(v[a][8 + i]), 0x1p-7f, fmaf(__uint_as_float(v[a][4 + i]), 0x1p-4f, __uint_as_float(v[a][i])));
-          }
+              for (int a0 = 0; a0 < 4; a0 += 2) {
+                if (a0 >= accs) break;
+                uint32_t v[2][16];
+                const uint32_t at = lane_base + (uint32_t)(wg * 12);
+                tmem_ld16(at + (uint32_t)((a_first + a0) & 3) * acc_stride, v[0]);
+                tmem_ld16(at + (uint32_t)((a_first + min(a0 + 1, accs - 1)) & 3) * acc_stride, v[1]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int i = 0; i < 4; ++i) emit(wg * 4 + i, sum[i]);
-        }
-        if (!kGrouped && p.slices > 1) {
-          // every warp tells every CTA of the cluster that its sums are in place, then the owners add
-          __syncwarp();
-          if (lane < p.slices) {
-            uint32_t dst;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(red_full), "r"(lane));
-            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(dst) : "memory");
-          }
-          wait<true>(red_full, 0, abort_flag, p.status, 50);
-          for (int i = d; ; i += 32 * kDecWarps) {
-            const int own = i / kBM, r = i % kBM, m = own * p.slices + slice;
-            if (m >= rows) break;
-            float s = 0.0f;
-            for (int q = 0; q < p.slices; ++q) {
-              float f;
-              asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"((p.red_off | win) + (uint32_t)((own * p.slices + q) * kBM + r) * 4u));
-              s += f;
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                  for (int i = 0; i < 4; ++i)
+                    if (a0 + a < accs)
+                      sum[i] += fmaf(__uint_as_float(v[a][8 + i]), 0x1p-7f, fmaf(__uint_as_float(v[a][4 + i]), 0x1p-4f, __uint_as_float(v[a][i])));
+              }
             }
-            if (*abort_flag == 0 && R.n0 + r < R.n_end) p.y[(int64_t)m * p.N + R.n0 + r] = (uint16_t)gb_f32_to_bf16_bits(s * p.global_scale);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty);
+            auto emit = [&](int m, float total) {
+              const float scale = __shfl_sync(0xffffffffu, m < 32 ? xs0 : xs1, m & 31);
+              const int orow = __shfl_sync(0xffffffffu, m < 32 ? to0 : to1, m & 31);
+              if (m >= rows) return;
+              const float val = total * scale;
+              if (!kGrouped && p.slices > 1) {
+                // into the shared memory of the row's owner: slot [row / slices][slice][128 weight rows]
+                uint32_t dst;
+                const uint32_t local = (p.red_off | win) + (uint32_t)(((m / p.slices) * p.slices + slice) * kBM + row) * 4u;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(local), "r"(m % p.slices));
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(val) : "memory");
+              } else if (ok && col < Q.n_end) {
+                p.y[(int64_t)orow * p.N + col] = (uint16_t)gb_f32_to_bf16_bits(val * p.global_scale);
+              }
+            };
+            if (wide) {
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                const int c = wg + 4 * j;
+                if (c * 8 >= rows) break;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) emit(c * 8 + i, sum[8 * j + i]);
+              }
+            } else if (wg * 4 < rows) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) emit(wg * 4 + i, sum[i]);
+            }
+            if (!kGrouped && p.slices > 1) {
+              // every warp tells every CTA of the cluster that its sums are in place, then the owners add
+              __syncwarp();
+              if (lane < p.slices) {
+                uint32_t dst;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(red_full), "r"(lane));
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(dst) : "memory");
+              }
+              wait<true>(red_full, 0, abort_flag, p.status, 50);
+              for (int i = d; ; i += 32 * kDecWarps) {
+                const int own = i / kBM, r = i % kBM, m = own * p.slices + slice;
+                if (m >= rows) break;
+                float s = 0.0f;
+                for (int q = 0; q < p.slices; ++q) {
+                  float f;
+                  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"((p.red_off | win) + (uint32_t)((own * p.slices + q) * kBM + r) * 4u));
+                  s += f;
+                }
+                if (*abort_flag == 0 && Q.n0 + r < Q.n_end) p.y[(int64_t)m * p.N + Q.n0 + r] = (uint16_t)gb_f32_to_bf16_bits(s * p.global_scale);
+              }
+            }
           }
-        }
-        // hand the accumulators back for the next item (pass or tile)
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty);
+          u += u_step;
+        } while (u < u_end);
+      }
+      if (!live) break;
+      out_t = t;
+      out_pass = pass;
+      ++item;
+      g0 += units;
+      n0 += stages;
+      if (++pass >= R.n_pass) {
+        pass = 0;
+        t += gridDim.x;
+        settle();
       }
     }
   }
@@ -955,7 +1045,10 @@ bool layout(const Info& f, Fp4Params& p) {
     if (!take(512 + f.extra, 128, &p.misc_off)) continue;
     if (p.slices > 1 && !take((uint32_t)((p.M + p.slices - 1) / p.slices * p.slices * kBM * 4), 128, &p.red_off)) continue;
     for (p.raw_stages = kMaxRaw; p.raw_stages >= 2; p.raw_stages >>= 1)
-      if (take(f.box * (uint32_t)p.raw_stages, 128, &p.raw_off)) return true;
+      if (take(f.box * (uint32_t)p.raw_stages, 128, &p.raw_off)) {
+        if (p.E > 0 && !take(4u * (uint32_t)(p.E + 1), 128, &p.seg_off)) p.seg_off = 0;
+        return true;
+      }
   }
   return false;
 }
@@ -1265,6 +1358,7 @@ int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, in
   p.seg = seg; p.row_map = row_map;
   p.tiles_n = (int)(N / kBM);
   p.n_tiles = (int)(E * p.tiles_n);
+  p.E = (int)E;
   if (!layout(f, p)) return gb_fail(GB_EUNSUPPORTED, "no shared-memory layout for %d rows per pass", pass_rows);
   CUtensorMap map_w;
   rc = gb_tensor_map_bytes_2d(&map_w, w->qw, (uint64_t)p.n_sb * f.sb, (uint64_t)(E * N), (uint64_t)w->row_stride, f.pitch, kBM);

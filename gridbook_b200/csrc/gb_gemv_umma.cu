@@ -320,7 +320,10 @@ GB_DEVINL uint32_t e4m3_pair_to_bf16(uint32_t b) {
   return gb_pack_bf16x2(gb_e4m3_to_f32(b & 0xFFu), gb_e4m3_to_f32((b >> 8) & 0xFFu));
 }
 
-// The replicated lookup tables of one codebook, by the 512 decoder threads (d: 0 .. 511).
+// The replicated lookup tables of one codebook, by the 512 decoder threads (d: 0 .. 511).  An entry and its
+// copies fill 64 or 128 bytes, so neighbouring threads would write the same banks: the order of the stores
+// rotates with the thread (fp8 k = 32: 8192 clocks of shared-memory writes in front of every launch
+// without it, 1024 with it).
 template <int F>
 GB_DEVINL void build_tables(uint8_t* cb_s, const void* codebook, int64_t cb, const float* compose, int* inexact, int d) {
   const int de = d & 255, dh = d >> 8;                      // entry, which half of the copies / which table
@@ -332,14 +335,14 @@ GB_DEVINL void build_tables(uint8_t* cb_s, const void* codebook, int64_t cb, con
     const uint4 w = make_uint4(mul_bf16x2(e.x, two120), mul_bf16x2(e.y, two120), mul_bf16x2(e.z, two120),
                                mul_bf16x2(e.w, two120));
 #pragma unroll
-    for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(cb_s)[de * 8 + dh * 4 + j] = w;
+    for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(cb_s)[de * 8 + ((dh * 4 + j + d) & 7)] = w;
   } else if constexpr (F == kFmtK16) {
     // two sub-tables of 256 entries x four bf16, 16 copies each (8-byte loads go 16 lanes at a time);
     // the scale table as bf16, with a note when a value does not survive the conversion
     const uint2 e = __ldg(reinterpret_cast<const uint2*>(codebook) + dh * 256 + de);
     uint2* l = reinterpret_cast<uint2*>(cb_s) + dh * 256 * 16;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) l[de * 16 + j] = e;
+    for (int j = 0; j < 8; ++j) reinterpret_cast<uint4*>(l)[de * 8 + ((j + d) & 7)] = make_uint4(e.x, e.y, e.x, e.y);
     uint16_t* comp_s = reinterpret_cast<uint16_t*>(cb_s + 2 * 256 * 16 * 8);
     bool bad = false;
 #pragma unroll
@@ -356,9 +359,11 @@ GB_DEVINL void build_tables(uint8_t* cb_s, const void* codebook, int64_t cb, con
     const uint32_t lo = e4m3_pair_to_bf16(e), hi = e4m3_pair_to_bf16(e >> 16);
     uint4* l = reinterpret_cast<uint4*>(cb_s) + (dh * 256 + de) * 8;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) l[j] = make_uint4(lo, hi, lo, hi);
+    for (int j = 0; j < 8; ++j) l[(j + d) & 7] = make_uint4(lo, hi, lo, hi);
   } else {
     // four sub-tables of 256 entries x two values
+    constexpr int kVecs = Fm<F>::kStride / 16;
+    static_assert(kVecs == 4 || kVecs == 8, "copies of an entry");
     const uint16_t* t = reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(codebook) + cb);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -366,7 +371,7 @@ GB_DEVINL void build_tables(uint8_t* cb_s, const void* codebook, int64_t cb, con
       const uint32_t e = e4m3_pair_to_bf16(__ldg(t + ent));
       uint4* l = reinterpret_cast<uint4*>(cb_s + ent * Fm<F>::kStride);
 #pragma unroll
-      for (int j = 0; j < Fm<F>::kStride / 16; ++j) l[j] = make_uint4(e, e, e, e);
+      for (int j = 0; j < kVecs; ++j) l[(j + d / (8 / kVecs)) & (kVecs - 1)] = make_uint4(e, e, e, e);
     }
   }
 }
