@@ -27,7 +27,7 @@ REQUIRED_SYMBOLS = (
     "gb_moe_gemv_pairs_workspace_bytes", "gb_moe_gemv_pairs",
     "gb_moe_mlp_pairs_workspace_bytes", "gb_moe_mlp_pairs",
     "gb_expand_fp8_bf16", "gb_fp8_quantize_rows", "gb_gemm_tn", "gb_gemm_tn_grouped", "gb_moe_gather_rows", "gb_moe_swiglu_rows", "gb_moe_gemv_sorted",
-    "gb_moe_route_inv", "gb_moe_fp4_pass_rows", "gb_moe_fp4_operand_bytes", "gb_moe_fp4_rows", "gb_moe_fp4_swiglu_rows", "gb_moe_gemv_fp4",
+    "gb_moe_route_inv", "gb_moe_fp4_pass_rows", "gb_moe_fp4_operand_bytes", "gb_moe_fp4_rows", "gb_moe_fp4_swiglu_rows", "gb_moe_gemv_fp4", "gb_moe_gemm_fp4",
     "gb_peer_alloc", "gb_peer_free", "gb_peer_export", "gb_peer_open", "gb_peer_close",
     "gb_peer_allgather", "gb_peer_allgather_ll", "gb_peer_barrier", "gb_launch_count", "gb_gemv_allgather", "gb_moe_combine_peer",
 )

@@ -78,6 +78,20 @@ unsigned long long gb_wait_limit_ns();
 int gb_tensor_map_operand(void* map_out, const void* base, int64_t rows, int64_t K, int elem_bytes, int box_rows);
 // Row-major bf16 output [M, N] in boxes of 32 x 32 with the 64-byte swizzle (N a multiple of 8).
 int gb_tensor_map_out(void* map_out, void* base, int64_t M, int64_t N);
+// Activation operand of the grouped GEMM (gb_moe_gemm_fp4): tiles of 64 rows, [tile][64 code rows of q, 64 of the
+// correction][K / 2 bytes], then the scale-factor atoms of 192 columns a tile, then the rows' powers of two.
+// Column 96 (m / 32) + 32 t + m % 32 of a tile is term t of row m.
+struct GbFp4Tiles { int64_t tiles, sf_groups, sf_at, scale_at, bytes; };
+inline GbFp4Tiles gb_fp4_tiles(int64_t P, int64_t E, int64_t K) {
+  GbFp4Tiles t;
+  auto up = [](int64_t v) { return (v + 255) & ~(int64_t)255; };
+  t.tiles = P / 64 + E + 1;
+  t.sf_groups = (t.tiles * 192 + 127) / 128;
+  t.sf_at = up(t.tiles * 128 * (K / 2));
+  t.scale_at = t.sf_at + up(t.sf_groups * (K / 64) * 512);
+  t.bytes = t.scale_at + up(t.tiles * 64 * 4);
+  return t;
+}
 // The prefill GEMMs on CTA pairs (gb_gemm_pair.cu), for the shapes that gb_gemm_pair_applies names.
 bool gb_gemm_pair_applies(int64_t M);
 int gb_gemm_pair(const void* A, const void* B, void* D, int64_t M, int64_t N, int64_t K, int kind, const float* a_scale,

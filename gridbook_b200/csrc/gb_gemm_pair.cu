@@ -40,22 +40,27 @@ constexpr int kSlabBytes = 128;                      // K bytes per row and stag
 constexpr int kTmemCols = 512;
 constexpr int kEpiWarps = 8;                         // two per lane quarter, half of the columns each
 constexpr int kOutChunk = 2048;                      // 32 rows x 32 bf16 columns on their way out
-constexpr int kOutBytes = kEpiWarps * 2 * kOutChunk;
+constexpr int kMaxGroups = 1024;                     // experts of one grouped launch
+constexpr int kTileRows = 64;                        // grouped: activation rows of a tile, three columns each
 constexpr int kGroupM = 16;                          // row tiles walked together before the next columns
 
-template <Kind kKind, int kBN>
+template <Kind kKind, int kBN, bool kGrouped = false>
 struct Shape {
   static constexpr int kABytes = kBM * kSlabBytes;
   static constexpr int kBBytes = kBN / 2 * kSlabBytes;
   static constexpr int kAtoms = 2048;                                    // scale bytes of 128 rows x 16 groups
   static constexpr int kSfBytes = kKind == kFp4 ? 3 * kAtoms : 0;        // A's rows, two 128-row groups of B
   static constexpr int kStageBytes = kABytes + kBBytes + kSfBytes;
+  // output chunks on their way out; grouped: segment offsets and the prefix of the row tiles
+  static constexpr int kOutBytes = kGrouped ? 2 * (kMaxGroups + 1) * 4 + 8 : kEpiWarps * 2 * kOutChunk;
   static constexpr int kStages = (227 * 1024 - 2048 - kOutBytes) / kStageBytes;
   static constexpr int kSmem = kStages * kStageBytes + kOutBytes + 2048;
   static constexpr int kThreads = kKind == kFp4 ? 448 : 320;
-  static constexpr int kAccs = kKind == kFp4 ? 1 : 2;
+  static constexpr int kAccs = kKind == kFp4 && !kGrouped ? 1 : 2;
+  static constexpr uint32_t kAcc1 = kKind == kFp4 ? kBN : 256;           // column of the second accumulator
+  static constexpr uint32_t kSf0 = kKind == kFp4 ? kAccs * kBN : 0;      // first column of the scale factors
   static constexpr uint32_t kSfCols = 48;                                // columns of a set: 16 of A, 32 of B
-  static constexpr int kSets = kKind == kFp4 ? (kTmemCols - kBN) / (int)kSfCols : 1;
+  static constexpr int kSets = kKind == kFp4 ? (kTmemCols - kAccs * kBN) / (int)kSfCols : 1;
 };
 
 struct PairParams {
@@ -68,6 +73,11 @@ struct PairParams {
   int out_tma;                 // rows of D are a multiple of 16 bytes
   uint16_t* D;
   int* status;
+  // grouped: a tile is 256 weight rows of an expert times up to 64 of its activation rows
+  const int32_t* seg;          // [E + 1]
+  const int32_t* row_map;      // output row of a sorted row, or null
+  const float* x_scale;        // [row tile][64]
+  int E;
 };
 
 GB_DEVINL uint32_t leader_addr(uint32_t addr) {
@@ -75,12 +85,14 @@ GB_DEVINL uint32_t leader_addr(uint32_t addr) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
   return r;
 }
+// Relaxed: what it guards is tensor memory, which the loads have left; a release at cluster scope would wait for
+// the output stores in flight, once a tile.
 GB_DEVINL void arrive_cluster(uint32_t addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
 GB_DEVINL bool try_wait(uint32_t bar, uint32_t parity) {
   uint32_t done;
-  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
@@ -189,23 +201,46 @@ GB_DEVINL void tile_at(const PairParams& p, int tile, int& mt, int& nt) {
   nt = in / rows;
 }
 
-GB_DEVINL int first_col(const PairParams& p, int tile, int bn) {
-  int mt, nt;
-  tile_at(p, tile, mt, nt);
-  return nt * bn;
+// One tile: first row of A, first row of B; grouped: expert's weight row, its activation rows.
+struct Tile { int m0, n0; int w0, lo, rows, x_tile; };
+
+template <int kBN, bool kGrouped>
+GB_DEVINL Tile tile_info(const PairParams& p, int tile, const int* seg_s, const int* base_s) {
+  Tile t = {};
+  if (!kGrouped) {
+    int mt, nt;
+    tile_at(p, tile, mt, nt);
+    t.m0 = mt * kPairM;
+    t.n0 = nt * kBN;
+  } else {
+    const int gp = tile / p.m_tiles;                         // row tile; the expert's weight tiles run fastest
+    int e = 0, hi = p.E;                                     // largest e with base_s[e] <= gp
+    while (hi - e > 1) {
+      const int mid = (e + hi) >> 1;
+      if (base_s[mid] <= gp) e = mid; else hi = mid;
+    }
+    const int pass = gp - base_s[e], lo = seg_s[e];
+    t.w0 = (tile - gp * p.m_tiles) * kPairM;
+    t.m0 = e * (int)p.N + t.w0;
+    t.lo = lo + pass * kTileRows;
+    t.rows = min(kTileRows, seg_s[e + 1] - t.lo);
+    t.x_tile = lo / kTileRows + e + pass;                    // tiles of different (expert, pass) never coincide
+    t.n0 = t.x_tile * kBN;
+  }
+  return t;
 }
 
-template <Kind kKind, int kBN>
-__global__ void __launch_bounds__(Shape<kKind, kBN>::kThreads, 1)
+template <Kind kKind, int kBN, bool kGrouped>
+__global__ void __launch_bounds__(Shape<kKind, kBN, kGrouped>::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_d,
                  const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb, const PairParams p) {
-  using S = Shape<kKind, kBN>;
+  using S = Shape<kKind, kBN, kGrouped>;
   constexpr int kStages = S::kStages;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t ring = (gb_smem_u32(smem_raw) + 1023u) & ~1023u;        // the same offset in both CTAs
   uint8_t* ring_ptr = smem_raw + (ring - gb_smem_u32(smem_raw));
   const uint32_t out_ring = ring + kStages * S::kStageBytes;             // two chunks per epilogue warp
-  const uint32_t full_bar = out_ring + kOutBytes;             // leader: both CTAs' operand tiles have landed
+  const uint32_t full_bar = out_ring + (S::kOutBytes + 7) / 8 * 8;             // leader: both CTAs' operand tiles have landed
   const uint32_t empty_bar = full_bar + 8 * kStages;                     // the MMAs that read the stage are done
   const uint32_t acc_full = empty_bar + 8 * kStages;                     // [2] accumulator complete
   const uint32_t acc_empty = acc_full + 16;                              // [2] leader: drained by both CTAs
@@ -245,7 +280,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *slot_ptr;
   gb_pdl_wait();
-  const int total_tiles = p.m_tiles * p.n_tiles, stride = (int)(gridDim.x >> 1), first = (int)(blockIdx.x >> 1);
+  int* seg_s = reinterpret_cast<int*>(ring_ptr + (out_ring - ring));
+  int* base_s = seg_s + kMaxGroups + 1;                                  // row tiles in front of an expert
+  if (kGrouped) {
+    if (warp == 0) {
+      int carry = 0;
+      for (int e0 = 0; e0 < p.E; e0 += 32) {
+        const int e = e0 + lane;
+        const int lo = e < p.E ? p.seg[e] : 0, hi = e < p.E ? p.seg[e + 1] : 0;
+        const int tiles = (hi - lo + kTileRows - 1) / kTileRows;
+        int incl = tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += v;
+        }
+        if (e < p.E) {
+          seg_s[e] = lo;
+          base_s[e] = carry + incl - tiles;
+          if (e == p.E - 1) { seg_s[p.E] = hi; base_s[p.E] = carry + incl; }
+        }
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+      }
+    }
+    __syncthreads();
+  }
+  const int total_tiles = kGrouped ? base_s[p.E] * p.m_tiles : p.m_tiles * p.n_tiles;
+  const int stride = (int)(gridDim.x >> 1), first = (int)(blockIdx.x >> 1);
   const int my_tiles = total_tiles > first ? (total_tiles - first + stride - 1) / stride : 0;
 
   if (warp == kEpiWarps) {
@@ -256,16 +317,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       int s = 0;
       uint32_t ph = 1;
       for (int tile = first; tile < total_tiles; tile += stride) {
-        int mt, nt;
-        tile_at(p, tile, mt, nt);
-        const int m0 = mt * kPairM + (int)rank * kBM, n0 = nt * kBN;
+        const Tile T = tile_info<kBN, kGrouped>(p, tile, seg_s, base_s);
+        const int m0 = T.m0 + (int)rank * kBM, n0 = T.n0;
         for (int kt = 0; kt < p.k_tiles; ++kt) {
           wait(empty_bar + 8 * s, ph, abort_flag, p.status, 71);
           if (*abort_flag) break;
           const uint32_t st = ring + (uint32_t)s * S::kStageBytes;
           if (rank == 0) expect_tx(full_bar + 8 * s, 2 * S::kStageBytes);
           tma_load_pair(st, &map_a, kt * slab_elems, m0, full_pair + 8 * s);
-          tma_load_pair(st + S::kABytes, &map_b, kt * slab_elems, n0 + (int)rank * (kBN / 2), full_pair + 8 * s);
+          if (kGrouped) {                                    // 32 rows: codes of q for hi and for lo, of the correction
+            const uint32_t b = st + S::kABytes;
+            const int r0 = T.x_tile * 2 * kTileRows + (int)rank * 32;
+            tma_load_pair(b, &map_b, kt * slab_elems, r0, full_pair + 8 * s);
+            tma_load_pair(b + 4096, &map_b, kt * slab_elems, r0, full_pair + 8 * s);
+            tma_load_pair(b + 8192, &map_b, kt * slab_elems, r0 + kTileRows, full_pair + 8 * s);
+          } else {
+            tma_load_pair(st + S::kABytes, &map_b, kt * slab_elems, n0 + (int)rank * (kBN / 2), full_pair + 8 * s);
+          }
           if (kKind == kFp4) {                               // row groups past the end read zero
             const uint32_t sf = st + S::kABytes + S::kBBytes;
             tma_load_pair(sf, &map_sfa, 0, (m0 / 128 * p.k_tiles + kt) * 8, full_pair + 8 * s);
@@ -285,9 +353,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       for (int it = 0; it < my_tiles; ++it) {
         const int buf = S::kAccs == 2 ? it & 1 : 0;
         const uint32_t use = (uint32_t)(S::kAccs == 2 ? it >> 1 : it);
-        const bool shifted = first_col(p, first + it * stride, kBN) % 128 != 0;
+        const bool shifted = kKind == kFp4 && kBN % 128 != 0 && tile_info<kBN, kGrouped>(p, first + it * stride, seg_s, base_s).n0 % 128 != 0;
         wait(acc_empty + 8 * buf, (use & 1) ^ 1, abort_flag, p.status, 72);       // its last tile is drained
-        const uint32_t acc = tmem_base + (buf ? 256u : 0u);
+        const uint32_t acc = tmem_base + (buf ? S::kAcc1 : 0u);
         for (int kt = 0; kt < p.k_tiles; ++kt) {
           if (kKind == kFp4) wait(sf_full + 8 * set, sf_ph, abort_flag, p.status, 73);
           else wait(full_bar + 8 * s, ph, abort_flag, p.status, 74);
@@ -296,7 +364,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           const uint32_t st = ring + (uint32_t)s * S::kStageBytes;
           const uint64_t da = desc_sw128(st), db = desc_sw128(st + S::kABytes);
           // 192 columns start in the middle of a 128-row group every other time: two columns on
-          const uint32_t sfa_t = tmem_base + kBN + S::kSfCols * set, sfb_t = sfa_t + 16u + (shifted ? 2u : 0u);
+          const uint32_t sfa_t = tmem_base + S::kSf0 + S::kSfCols * set, sfb_t = sfa_t + 16u + (shifted ? 2u : 0u);
 #pragma unroll
           for (int k = 0; k < 4; ++k)                        // 32 bytes of K per instruction
             mma_pair<kKind>(acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), p.idesc, sfa_t + 4u * k, sfb_t + 8u * k,
@@ -325,7 +393,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (*abort_flag) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t sf = ring + (uint32_t)s * S::kStageBytes + S::kABytes + S::kBBytes;
-        const uint32_t col = tmem_base + kBN + S::kSfCols * set;
+        const uint32_t col = tmem_base + S::kSf0 + S::kSfCols * set;
         sf_to_tmem(col + 4u * k, sf + 512u * k);
         sf_to_tmem(col + 16u + 8u * k, sf + S::kAtoms + 512u * k);
         sf_to_tmem(col + 20u + 8u * k, sf + 2 * S::kAtoms + 512u * k);
@@ -344,6 +412,37 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int quarter = warp & 3, c_lo = (warp >> 2) * kCols;
     const uint32_t out = out_ring + (uint32_t)warp * 2 * kOutChunk;
     int it = 0;
+    if constexpr (kGrouped) {
+      // Lane = weight row, i.e. output feature; column 96 h + 32 t + i = term t of activation row 32 h + i.  A
+      // warp takes its half's three terms, adds them and stores 64 contiguous bytes per activation row.
+      const int half = warp >> 2;
+      for (int tile = first; tile < total_tiles; tile += stride, ++it) {
+        const Tile T = tile_info<kBN, kGrouped>(p, tile, seg_s, base_s);
+        const int buf = it & 1, w = T.w0 + (int)rank * kBM + quarter * 32 + lane, m = half * 32 + lane;
+        const float xs = m < T.rows ? p.x_scale[(int64_t)T.x_tile * kTileRows + m] : 0.0f;
+        const int to = m < T.rows ? (p.row_map ? p.row_map[T.lo + m] : T.lo + m) : 0;
+        wait(acc_full + 8 * buf, (uint32_t)(it >> 1) & 1, abort_flag, p.status, 77);
+        if (__any_sync(0xffffffffu, *abort_flag)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf ? S::kAcc1 : 0u) + (uint32_t)(half * 96);
+        uint32_t hi[32], lo[32], dl[32];
+        tmem_ld32(at, hi);
+        tmem_ld32(at + 32u, lo);
+        tmem_ld32(at + 64u, dl);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive_cluster(acc_empty_pair + 8 * buf);
+        const int n = T.rows - half * 32;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float v = fmaf(__uint_as_float(dl[i]), 0x1p-7f, fmaf(__uint_as_float(lo[i]), 0x1p-4f, __uint_as_float(hi[i])));
+          const float r = v * __shfl_sync(0xffffffffu, xs, i) * p.global_scale;
+          const int64_t row = __shfl_sync(0xffffffffu, to, i);
+          if (i < n && w < p.N) p.D[row * p.N + w] = (uint16_t)gb_f32_to_bf16_bits(r);
+        }
+      }
+    } else {
     for (int tile = first; tile < total_tiles; tile += stride, ++it) {
       int mt, nt;
       tile_at(p, tile, mt, nt);
@@ -354,7 +453,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       wait(acc_full + 8 * buf, (uint32_t)(S::kAccs == 2 ? it >> 1 : it) & 1, abort_flag, p.status, 77);
       if (__any_sync(0xffffffffu, *abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf ? 256u : 0u) + (uint32_t)c_lo;
+      const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf ? S::kAcc1 : 0u) + (uint32_t)c_lo;
       uint32_t w[kCols / 2], va[32];
 #pragma unroll
       for (int c = 0; c < kChunks; ++c) {
@@ -394,6 +493,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       }
     }
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
   }
   __syncwarp();
   if (*abort_flag && threadIdx.x == 0) __nanosleep(1000000);   // loads still in flight land before the memory goes
@@ -407,23 +507,23 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 std::mutex g_mutex;
 int g_pairs[64][8];                                          // pairs that run at once, per device and kernel (0: not asked)
 
-template <Kind kKind, int kBN>
+template <Kind kKind, int kBN, bool kGrouped = false>
 int resident_pairs() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   std::lock_guard<std::mutex> lock(g_mutex);
-  int& n = g_pairs[dev][(int)kKind * 2 + (kBN == 256)];
+  int& n = g_pairs[dev][kGrouped ? 6 : (int)kKind * 2 + (kBN == 256)];
   if (n == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * 256);
-    cfg.blockDim = dim3(Shape<kKind, kBN>::kThreads);
-    cfg.dynamicSmemBytes = Shape<kKind, kBN>::kSmem;
+    cfg.blockDim = dim3(Shape<kKind, kBN, kGrouped>::kThreads);
+    cfg.dynamicSmemBytes = Shape<kKind, kBN, kGrouped>::kSmem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<kKind, kBN>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<kKind, kBN, kGrouped>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
   }
   return n;
 }
@@ -469,7 +569,7 @@ int run(const void* A, const void* B, const void* sfa, const void* sfb, PairPara
   cfg.attrs = attr;
   cfg.numAttrs = gb_pdl_enabled() ? 2 : 1;
   gb_count_launch();
-  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<kKind, kBN>, map_a, map_b, map_d, map_sfa, map_sfb, p));
+  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<kKind, kBN, false>, map_a, map_b, map_d, map_sfa, map_sfb, p));
   return GB_OK;
 }
 
@@ -477,7 +577,7 @@ int run(const void* A, const void* B, const void* sfa, const void* sfb, PairPara
 
 int gb_prepare_gemm_pair() {
 #define GB_ATTR(K, N) \
-  GB_CUDA_OK(cudaFuncSetAttribute((const void*)gemm_pair_kernel<K, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<K, N>::kSmem))
+  GB_CUDA_OK(cudaFuncSetAttribute((const void*)gemm_pair_kernel<K, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<K, N>::kSmem))
   GB_ATTR(kBf16, 256);
   GB_ATTR(kBf16, 192);
   GB_ATTR(kFp8, 256);
@@ -485,6 +585,8 @@ int gb_prepare_gemm_pair() {
   GB_ATTR(kFp4, 256);
   GB_ATTR(kFp4, 192);
 #undef GB_ATTR
+  GB_CUDA_OK(cudaFuncSetAttribute((const void*)gemm_pair_kernel<kFp4, 192, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  Shape<kFp4, 192, true>::kSmem));
   return GB_OK;
 }
 
@@ -532,3 +634,57 @@ int gb_gemm_fp4_pair(const void* A, const void* sfa, const void* B, const void* 
   const bool narrow = narrow_tiles(M, N);
   return narrow ? run<kFp4, 192>(A, B, sfa, sfb, p, 1, stream) : run<kFp4, 256>(A, B, sfa, sfb, p, 1, stream);
 }
+
+extern "C" {
+
+int gb_moe_gemm_fp4(const void* operand, const void* packed, const void* sf, int64_t N, int64_t K, int64_t E, const int32_t* seg,
+                    const int32_t* row_map, int64_t P, float global_scale, void* y, void* stream) {
+  using S = Shape<kFp4, 192, true>;
+  GB_REQUIRE(operand && packed && sf && seg && y, "null pointer argument");
+  GB_REQUIRE(N > 0 && N % kBM == 0 && K > 0 && K % 256 == 0, "N=%lld must be a multiple of %d, K=%lld of 256", (long long)N, kBM, (long long)K);
+  GB_REQUIRE(P >= 1 && P < (1ll << 30) && E >= 1 && E <= kMaxGroups && E * N < (1ll << 31) && K < (1ll << 31),
+             "bad shape P=%lld E=%lld N=%lld", (long long)P, (long long)E, (long long)N);
+  GB_REQUIRE(((uintptr_t)operand & 255u) == 0 && ((uintptr_t)packed & 15u) == 0 && ((uintptr_t)sf & 15u) == 0,
+             "operands must be aligned: 256 and 16 bytes");
+  const int pairs = resident_pairs<kFp4, 192, true>();
+  if (pairs <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
+  const GbFp4Tiles op = gb_fp4_tiles(P, E, K);
+  PairParams p = {};
+  p.M = E * N; p.N = N; p.K = K;
+  p.k_tiles = (int)(K / 256);
+  p.m_tiles = (int)((N + kPairM - 1) / kPairM);
+  p.idesc = (1u << 7) | (1u << 10) | ((uint32_t)(192 >> 3) << 17) | ((uint32_t)(kPairM >> 4) << 24);
+  p.global_scale = global_scale == 0.0f ? 1.0f : global_scale;
+  p.D = (uint16_t*)y;
+  p.status = gb_status_word();
+  p.seg = seg; p.row_map = row_map; p.E = (int)E;
+  p.x_scale = (const float*)((const uint8_t*)operand + op.scale_at);
+  CUtensorMap map_a, map_b, map_d = {}, map_sfa, map_sfb;
+  int rc = gb_tensor_map_operand(&map_a, packed, E * N, K / 2, 1, kBM);
+  if (rc != GB_OK) return rc;
+  rc = gb_tensor_map_operand(&map_b, operand, op.tiles * 2 * kTileRows, K / 2, 1, 32);
+  if (rc != GB_OK) return rc;
+  rc = gb_tensor_map_bytes_2d(&map_sfa, sf, 256, (uint64_t)(E * N / 128 * p.k_tiles * 8), 256, 256, 8);
+  if (rc != GB_OK) return rc;
+  rc = gb_tensor_map_bytes_2d(&map_sfb, (const uint8_t*)operand + op.sf_at, 256, (uint64_t)(op.sf_groups * p.k_tiles * 8), 256, 256, 8);
+  if (rc != GB_OK) return rc;
+  const int64_t tiles = op.tiles * p.m_tiles;                // at least as many as the routing can make
+  GB_REQUIRE(tiles < (1ll << 31), "too many output tiles");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
+  cfg.blockDim = dim3(S::kThreads);
+  cfg.dynamicSmemBytes = S::kSmem;
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = gb_pdl_enabled() ? 2 : 1;
+  gb_count_launch();
+  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<kFp4, 192, true>, map_a, map_b, map_d, map_sfa, map_sfb, p));
+  return GB_OK;
+}
+
+}  // extern "C"

@@ -356,6 +356,10 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const int slice = blockIdx.y;
   const int sb_begin = slice * p.units;
   const int units = min(p.units, p.n_sb - sb_begin);
+  // Units are numbered over all items, an item's count rounded up to whole raw stages: a unit without weights
+  // passes every barrier and multiplies nothing.  So the warpgroup, the raw slot and the activation slot of a
+  // unit follow from its number alone, and a warpgroup sees every phase of every barrier that it waits for.
+  const int span = (units + T::kSbPerStage - 1) / T::kSbPerStage * T::kSbPerStage;
   // Layout of tensor memory.  Narrow: four accumulators of 64 columns, one per warpgroup and issuer; wide:
   // [hi | dlt] in columns [0, 128), [lo] in [128, 192), one issuer each.  Then the four operand
   // buffers: nibbles (32), weight scale factors (16), activation scale factors (16 per set).
@@ -481,10 +485,11 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
           const int rows = min(p.pass_rows, R.cnt - pass * p.pass_rows);
           const uint32_t bytes = (uint32_t)unit_bytes(wide, rows);
           const uint8_t* src = p.xop + ((int64_t)(R.x_tile + pass) * p.n_sb + sb_begin) * p.x_unit;
-          for (int u = 0; u < units; ++u, ++g, src += p.x_unit) {
+          for (int u = 0; u < span; ++u, ++g, src += p.x_unit) {
             const int s = g & x_mask;
             wait(done + 8 * s, ((uint32_t)(g >> x_log) & 1u) ^ 1u, abort_flag, p.status, 43);
             if (*abort_flag) continue;
+            if (u >= units) { mbar_arrive(x_full + 8 * s); continue; }
             mbar_expect(x_full + 8 * s, bytes);
             bulk_load(x_ring + (uint32_t)s * x_stage, src, bytes, x_full + 8 * s);
           }
@@ -504,7 +509,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       int g0 = 0, item = 0;                                // units / (tile, pass) items since the start
       for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
         const Tile R = tile_at(t);
-        for (int pass = 0; pass < R.n_pass; ++pass, ++item, g0 += units) {
+        for (int pass = 0; pass < R.n_pass; ++pass, ++item, g0 += span) {
           const int rows = min(p.pass_rows, R.cnt - pass * p.pass_rows);
           const int n = wide && i == 1 ? term_rows(true, rows) : mma_cols(wide, rows);
           // E2M1 x E2M1, UE4M3 scale factors, both K-major, fp32 accumulate; N >> 3, M >> 4
@@ -514,7 +519,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           }
           const int u_first = wide ? 0 : (i - g0) & 3;
-          for (int u = u_first; u < units; u += u_step) {
+          for (int u = u_first; u < span; u += u_step) {
             const int g = g0 + u, s = g & x_mask;
             const uint32_t a = tmem_base + buf_col0 + (uint32_t)(g & 3) * buf_stride, off = (uint32_t)s * x_stage;
             const uint64_t db = db0 + (uint64_t)(off >> 4);
@@ -522,7 +527,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             if (*abort_flag) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+            for (int k = 0; k < (u < units ? 4 : 0); ++k)
               umma_fp4_ts(acc, a + 8u * k, db + (uint64_t)(2 * k), idesc, a + 32u + 4u * k, a + sf_col + 4u * k, u > u_first || k > 0);
             umma_commit(done + 8 * s);
           }
@@ -543,7 +548,6 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     float xs0 = 0.0f, xs1 = 0.0f;                            // powers of two of rows lane, lane + 32
     int item = 0, g0 = 0, n0 = 0;                            // items, units and raw stages so far
     uint32_t flip = 0;
-    const int stages = (units + T::kSbPerStage - 1) / T::kSbPerStage;
     // An item's accumulators are read out after the warpgroup has decoded its first unit of the NEXT item:
     // the last multiplications, their completion and the read-out then overlap decoding, and the next
     // item's multiplications find their operands ready.  (Nothing that first unit waits for needs this
@@ -574,7 +578,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
       }
       {
-        const int u_end = live ? stages * T::kSbPerStage : 0, u_step = kAllSee<F> ? 1 : 4;
+        const int u_end = live ? span : 0, u_step = kAllSee<F> ? 1 : 4;
         int u = kAllSee<F> ? 0 : (wg - g0) & 3;
 #pragma unroll 1
         do {
@@ -583,6 +587,13 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
           if (u < u_end && !mine) {
             wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
             if (lane == 0) mbar_arrive(raw_empty + 8 * rs);
+          }
+          if (mine && u >= units && u < u_end) {             // a stage's missing second superblock
+            wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
+            const int g = g0 + u;
+            if (g >= 4) wait(done + 8 * ((g - 4) & x_mask), (uint32_t)((g - 4) >> x_log) & 1u, abort_flag, p.status, 48);
+            wait(x_full + 8 * (g & x_mask), (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 46);
+            if (lane == 0) { mbar_arrive(raw_empty + 8 * rs); mbar_arrive(full + 8 * (g & x_mask)); }
           }
           if (mine && u < units && live) {
             wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
@@ -670,7 +681,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * (g & x_mask));
           }
-          if (mine && u < u_end && (F == kLit || u >= units) && lane == 0) mbar_arrive(raw_empty + 8 * rs);   // also for a stage's missing second superblock
+          if (F == kLit && mine && u < units && live && lane == 0) mbar_arrive(raw_empty + 8 * rs);
           if (out_t >= 0 && (mine || u + u_step >= u_end)) {
             // ------------------------- read-out ------------------------------------
             // Sums into registers, the accumulators handed back, then the stores.
@@ -713,7 +724,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             } else if (wg * 4 < rows) {
               // four rows per warpgroup; issuers without a unit leave their accumulator untouched.  Units 0, 4, ..
               // of the item first, then 1, 5, ..: the order does not depend on where the item's first unit fell
-              const int accs = min(4, units), a_first = g0 - units;
+              const int accs = min(4, units), a_first = g0 - span;
 #pragma unroll
               for (int i = 0; i < 4; ++i) sum[i] = 0.0f;
 #pragma unroll
@@ -791,8 +802,8 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       out_t = t;
       out_pass = pass;
       ++item;
-      g0 += units;
-      n0 += stages;
+      g0 += span;
+      n0 += span / T::kSbPerStage;
       if (++pass >= R.n_pass) {
         pass = 0;
         t += gridDim.x;
@@ -893,10 +904,27 @@ GB_DEVINL void store_group(const Group& G, uint8_t* tile, int64_t unit_stride, b
   }
 }
 
+// The same as the grouped GEMM's operand (gb_fp4_tiles): row m of tile `tile`.
+GB_DEVINL void store_group_matrix(const Group& G, uint8_t* xop, uint8_t* sf, int K, int64_t tile, int m, int g, unsigned mask) {
+  uint8_t* codes = xop + ((tile * 128 + m) * (int64_t)K) / 2 + g * 8;
+  *reinterpret_cast<uint2*>(codes) = make_uint2(G.q[0], G.q[1]);
+  *reinterpret_cast<uint2*>(codes + (int64_t)K * 32) = make_uint2(G.e[0], G.e[1]);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {                             // hi, lo, dlt
+    const uint32_t b = t == 0 ? G.hi : t == 1 ? G.lo : G.dl;
+    const uint32_t b1 = __shfl_down_sync(mask, b, 1), b2 = __shfl_down_sync(mask, b, 2), b3 = __shfl_down_sync(mask, b, 3);
+    const int64_t c = tile * 192 + (m >> 5) * 96 + t * 32 + (m & 31);
+    if ((g & 3) == 0)
+      *reinterpret_cast<uint32_t*>(sf + (c >> 7) * ((int64_t)K * 8) + (g >> 2) * 512 + (c & 31) * 16 + ((c >> 5) & 3) * 4) =
+          b | (b1 << 8) | (b2 << 16) | (b3 << 24);
+  }
+}
+
 struct RowsParams {
   const uint4* x;            // bf16 rows [*, K]
   uint8_t* xop;
   float* x_scale;
+  uint8_t* sf;               // matrix form (x_unit = 0): the scale-factor plane
   int64_t x_unit;
   int K, n_sb, scale_rule, pass_rows;
   int rows;                  // dense: M
@@ -989,7 +1017,9 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
     for (int i = 0; i < kG; ++i) {
       const int g = threadIdx.x + i * blockDim.x;
       const unsigned here = __ballot_sync(0xffffffffu, g < groups);
-      if (g < groups) store_group(grp[i], dst, p.x_unit, is_wide(p.pass_rows), rows, m, g, here);
+      if (g >= groups) continue;
+      if (kMode != 0 && p.x_unit == 0) store_group_matrix(grp[i], p.xop, p.sf, p.K, tile, m, g, here);
+      else store_group(grp[i], dst, p.x_unit, is_wide(p.pass_rows), rows, m, g, here);
     }
   }
 }
@@ -1290,6 +1320,7 @@ int gb_moe_fp4_pass_rows(const gb_weight* w, int scales_e4m3, int64_t P, int64_t
 }
 
 int64_t gb_moe_fp4_operand_bytes(int64_t P, int64_t E, int64_t K, int pass_rows) {
+  if (pass_rows == 0) return gb_fp4_tiles(P, E, K).bytes;
   if (pass_rows < 1) return 0;
   const int64_t tiles = P / pass_rows + E + 1;
   return align256(tiles * (K / 256) * unit_bytes(is_wide(pass_rows), pass_rows)) + align256(tiles * pass_rows * 4);
@@ -1298,14 +1329,21 @@ int64_t gb_moe_fp4_operand_bytes(int64_t P, int64_t E, int64_t K, int pass_rows)
 static int rows_params(RowsParams* p, const void* x, int64_t P, int64_t E, int64_t K, int pass_rows, const int32_t* ids,
                        const int32_t* seg, int scale_rule, void* operand) {
   GB_REQUIRE(x && ids && seg && operand, "null pointer argument");
-  GB_REQUIRE(P >= 1 && P < (1ll << 30) && E >= 1 && K > 0 && K % 256 == 0 && pass_rows >= 1 && pass_rows <= kMaxRows,
+  GB_REQUIRE(P >= 1 && P < (1ll << 30) && E >= 1 && K > 0 && K % 256 == 0 && pass_rows >= 0 && pass_rows <= kMaxRows,
              "bad shape P=%lld E=%lld K=%lld", (long long)P, (long long)E, (long long)K);
   GB_REQUIRE(((uintptr_t)x & 15u) == 0 && ((uintptr_t)operand & 255u) == 0, "rows must be 16-byte aligned, the operand 256-byte");
-  const int64_t tiles = P / pass_rows + E + 1;
   p->x = (const uint4*)x;
   p->xop = (uint8_t*)operand;
-  p->x_unit = unit_bytes(is_wide(pass_rows), pass_rows);
-  p->x_scale = (float*)((uint8_t*)operand + align256(tiles * (K / 256) * p->x_unit));
+  if (pass_rows == 0) {
+    const GbFp4Tiles op = gb_fp4_tiles(P, E, K);
+    p->sf = (uint8_t*)operand + op.sf_at;
+    p->x_scale = (float*)((uint8_t*)operand + op.scale_at);
+    pass_rows = 64;
+  } else {
+    const int64_t tiles = P / pass_rows + E + 1;
+    p->x_unit = unit_bytes(is_wide(pass_rows), pass_rows);
+    p->x_scale = (float*)((uint8_t*)operand + align256(tiles * (K / 256) * p->x_unit));
+  }
   p->K = (int)K; p->n_sb = (int)(K / 256); p->scale_rule = scale_rule; p->pass_rows = pass_rows;
   p->ids = ids; p->seg = seg; p->E = (int)E;
   return GB_OK;

@@ -68,6 +68,7 @@ struct Lib {
   GB_FN(gb_moe_fp4_rows);
   GB_FN(gb_moe_fp4_swiglu_rows);
   GB_FN(gb_moe_gemv_fp4);
+  GB_FN(gb_moe_gemm_fp4);
 #undef GB_FN
 };
 Lib L;
@@ -113,6 +114,7 @@ void bind(const std::string& path) {
   GB_FN(gb_moe_fp4_rows);
   GB_FN(gb_moe_fp4_swiglu_rows);
   GB_FN(gb_moe_gemv_fp4);
+  GB_FN(gb_moe_gemm_fp4);
 #undef GB_FN
 }
 
@@ -192,6 +194,7 @@ void need_bf16(const at::Tensor& t, const char* what) {
 }
 
 constexpr int64_t kDecodeMaxRows = 16;
+constexpr int64_t kFp4GemmMinRows = 160;
 constexpr float kNvfp4ActRange = 448.0f;      // a row's largest group scale factor: the top of the UE4M3 range
 
 // Routes a plan has taken, reported to the host code by number.
@@ -490,24 +493,39 @@ struct MoEPlan {
   void sorted(Call& c) {
     Arena a;
     const Routing r = plan_routing(a, c);
-    const int pr13 = L.gb_moe_fp4_pass_rows(&w13.w, w13.scales_e4m3, c.P, E), pr2 = L.gb_moe_fp4_pass_rows(&w2.w, w2.scales_e4m3, c.P, E);
+    const int fp13 = L.gb_moe_fp4_pass_rows(&w13.w, w13.scales_e4m3, c.P, E), fp2 = L.gb_moe_fp4_pass_rows(&w2.w, w2.scales_e4m3, c.P, E);
+    // decoded once and multiplied by the grouped GEMM (pass rows 0) where several passes would decode every weight again
+    const bool once = c.P >= kFp4GemmMinRows * E && E <= 1024;
+    const bool once13 = fp13 && once, once2 = fp2 && once;
+    const int pr13 = once13 ? 0 : fp13, pr2 = once2 ? 0 : fp2;
+    const int64_t flat13 = once13 ? E * w13.w.rows : 0, flat2 = once2 ? E * w2.w.rows : 0;
+    const int wq = a.add(std::max(flat13 * w13.w.K, flat2 * w2.w.K) / 2);
+    const int wsf = a.add(std::max(L.gb_nvfp4_sf_bytes(flat13, w13.w.K), L.gb_nvfp4_sf_bytes(flat2, w2.w.K)));
     const int64_t op13 = L.gb_moe_fp4_operand_bytes(c.P, E, hidden, pr13), op2 = L.gb_moe_fp4_operand_bytes(c.P, E, inter, pr2);
-    const int xq = a.add(pr13 ? 0 : c.T * hidden * 2), xs = a.add(pr13 ? op13 : c.P * hidden * 2), h13 = a.add(c.P * 2 * inter * 2);
-    const int hs = a.add(pr2 || w2.fp4() ? 0 : c.P * inter * 2), h = a.add(pr2 ? op2 : c.P * inter * 2), y = a.add(c.P * hidden * 2);
+    const int xq = a.add(fp13 ? 0 : c.T * hidden * 2), xs = a.add(fp13 ? op13 : c.P * hidden * 2), h13 = a.add(c.P * 2 * inter * 2);
+    const int hs = a.add(fp2 || w2.fp4() ? 0 : c.P * inter * 2), h = a.add(fp2 ? op2 : c.P * inter * 2), y = a.add(c.P * hidden * 2);
     a.alloc(c.x);
     run_routing(a, r, c);
     const int32_t *off = a.ptr<int32_t>(r.offsets), *ord = a.ptr<int32_t>(r.order), *ids = c.ids.data_ptr<int32_t>();
-    if (pr13) {
+    auto multiply = [&](const Weight& w, const Weight& flat, bool once_w, int pr, int operand, const int32_t* map, void* to) {
+      if (!once_w) {
+        check(L.gb_moe_gemv_fp4(a.ptr(operand), &w.w, w.scales_e4m3, w.expert_stride, E, off, map, c.P, pr, to, c.stream));
+        return;
+      }
+      check(L.gb_expand_fp4_nvfp4(&flat.w, 0, flat.w.rows, a.ptr(wq), a.ptr(wsf), 2, c.stream));
+      check(L.gb_moe_gemm_fp4(a.ptr(operand), a.ptr(wq), a.ptr(wsf), w.w.rows, w.w.K, E, off, map, c.P, w.w.global_scale, to, c.stream));
+    };
+    if (fp13) {
       check(L.gb_moe_fp4_rows(c.x.data_ptr(), ids, a.ptr<int32_t>(r.inv), off, c.T, c.topk, E, hidden, pr13, c.rule, a.ptr(xs), c.stream));
-      check(L.gb_moe_gemv_fp4(a.ptr(xs), &w13.w, w13.scales_e4m3, w13.expert_stride, E, off, nullptr, c.P, pr13, a.ptr(h13), c.stream));
+      multiply(w13, rows13, once13, pr13, xs, nullptr, a.ptr(h13));
     } else {
       bucket(w13, c.x.data_ptr(), a.ptr(xq), c.T, c);
       check(L.gb_moe_gather_rows(a.ptr(xq), x_row(c.T, c.topk, c.x), ord, off, E, c.P, hidden, a.ptr(xs), c.stream));
       check(L.gb_moe_gemv_sorted(a.ptr(xs), &w13.w, w13.expert_stride, E, off, nullptr, c.P, a.ptr(h13), nullptr, c.stream));
     }
-    if (pr2) {
+    if (fp2) {
       check(L.gb_moe_fp4_swiglu_rows(a.ptr(h13), ids, ord, off, c.P, E, inter, pr2, c.rule, a.ptr(h), c.stream));
-      check(L.gb_moe_gemv_fp4(a.ptr(h), &w2.w, w2.scales_e4m3, w2.expert_stride, E, off, ord, c.P, pr2, a.ptr(y), c.stream));
+      multiply(w2, rows2, once2, pr2, h, ord, a.ptr(y));
     } else {
       swiglu(a, c, r, h13, hs, h);
       check(L.gb_moe_gemv_sorted(a.ptr(h), &w2.w, w2.expert_stride, E, off, ord, c.P, a.ptr(y), nullptr, c.stream));

@@ -355,6 +355,12 @@ GB_API int gb_moe_fp4_swiglu_rows(const void* h_bf16, const int32_t* topk_ids, c
 GB_API int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, int64_t expert_stride, int64_t E,
                            const int32_t* seg_offsets, const int32_t* row_map, int64_t P, int pass_rows, void* y_bf16,
                            void* stream);
+/* The same for many rows per expert, from the stack decoded once: `packed` and `sf` are the NVFP4 view of its
+ * E * N rows (gb_expand_fp4_nvfp4, scale factors swizzled, signs folded), the operand is written by
+ * gb_moe_fp4_rows / gb_moe_fp4_swiglu_rows with pass_rows = 0.  N a multiple of 128, K of 256, E <= 1024. */
+GB_API int gb_moe_gemm_fp4(const void* operand, const void* packed, const void* sf, int64_t N, int64_t K, int64_t E,
+                           const int32_t* seg_offsets, const int32_t* row_map, int64_t P, float global_scale, void* y_bf16,
+                           void* stream);
 
 /* The same routed projection for SMALL batches of the literal format (fp4 grid, full mode,
  * k = 8, E4M3-direct scales, one codebook per stack): every routed pair p is its own M = 1 linear
