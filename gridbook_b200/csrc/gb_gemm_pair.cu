@@ -411,7 +411,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     constexpr int kCols = kBN / 2, kChunks = kCols / 32;
     const int quarter = warp & 3, c_lo = (warp >> 2) * kCols;
     const uint32_t out = out_ring + (uint32_t)warp * 2 * kOutChunk;
-    int it = 0;
+    int it = 0, flip = 0;
     if constexpr (kGrouped) {
       // Lane = weight row, i.e. output feature; column 96 h + 32 t + i = term t of activation row 32 h + i.  A
       // warp takes its half's three terms, adds them and stores 64 contiguous bytes per activation row.
@@ -469,7 +469,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if (p.out_tma) {
 #pragma unroll
         for (int c = 0; c < kChunks; ++c) {
-          const uint32_t dst = out + (uint32_t)(c & 1) * kOutChunk;
+          const uint32_t dst = out + (uint32_t)flip * kOutChunk;       // in turn across tiles: their chunks may be odd in number
+          flip ^= 1;
           asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");       // the chunk before last has left its buffer
           __syncwarp();
 #pragma unroll
