@@ -927,6 +927,7 @@ struct RowsParams {
   uint8_t* sf;               // matrix form (x_unit = 0): the scale-factor plane
   int64_t x_unit;
   int K, n_sb, scale_rule, pass_rows;
+  int split;                 // dense: CTAs per row
   int rows;                  // dense: M
   // grouped: sorted row j = blockIdx.x belongs to expert ids[order[j]]
   const int32_t* ids;
@@ -938,8 +939,11 @@ struct RowsParams {
 };
 
 constexpr int kRowsMaxGroups = 4;
+constexpr int kMaxRowSplit = 8;
+constexpr int kRowSplitGroups = 320;                       // groups of a row per CTA of its cluster
 
-// kMode 0: dense, one CTA per row.  1: one CTA per token, its row goes to each of its experts' tiles.
+// kMode 0: dense, a cluster of `split` CTAs per row (a single CTA holding 1088 groups of a 17408-wide row took
+// 16 us for 64 rows: 64 SMs, four groups a thread in turn).  1: one CTA per token, its row goes to each of its experts' tiles.
 // 2: one CTA per sorted row of [gate | up]: SwiGLU (with the bf16 roundings of F.silu(gate) * up), then the split.
 template <int kG, int kMode>
 __global__ void __launch_bounds__(1024)
@@ -947,7 +951,8 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
   gb_pdl_launch_dependents();
   gb_pdl_wait();
   const int groups = p.K / 16;
-  const int j = blockIdx.x;
+  const int j = kMode == 0 ? (int)blockIdx.x / p.split : (int)blockIdx.x;
+  const int g_first = (kMode == 0 ? (int)blockIdx.x % p.split * (int)blockDim.x : 0) + (int)threadIdx.x;
   if (kMode == 2 && j >= p.seg[p.E]) return;
   const uint4* xr = p.x + (int64_t)j * (kMode == 2 ? 4 : 2) * groups;
   __shared__ float red[32];
@@ -957,7 +962,7 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
   float top = 0.0f;
 #pragma unroll
   for (int i = 0; i < kG; ++i) {
-    const int g = threadIdx.x + i * blockDim.x;
+    const int g = g_first + i * (int)blockDim.x;
     amax[i] = 0.0f;
     nan[i] = false;
     if (g < groups) {
@@ -989,6 +994,17 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
   top = (int)(threadIdx.x & 31) < (int)(blockDim.x >> 5) ? red[threadIdx.x & 31] : 0.0f;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if (kMode == 0 && p.split > 1) {                         // the largest of the row's CTAs
+    __shared__ float peers[kMaxRowSplit];
+    if ((int)threadIdx.x < p.split) {
+      uint32_t dst;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                   : "=r"(dst) : "r"(gb_smem_u32(&peers[(int)blockIdx.x % p.split])), "r"(threadIdx.x));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(top) : "memory");
+    }
+    cluster_sync();                                        // the last access to another CTA's memory lies in front of it
+    for (int q = 0; q < p.split; ++q) top = fmaxf(top, peers[q]);
+  }
   const float m1 = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_fp4_group_scale(fmaxf(top, 1e-8f), p.scale_rule)));
   const int shift = 7 - ((int)((__float_as_uint(m1) >> 23) & 0xFFu) - 127);
   const float back = __uint_as_float((uint32_t)(127 - shift) << 23);
@@ -996,7 +1012,7 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
   Group grp[kG];
 #pragma unroll
   for (int i = 0; i < kG; ++i)
-    if ((int)(threadIdx.x + i * blockDim.x) < groups) grp[i] = split_group(w[i], amax[i], nan[i], p.scale_rule, shift);
+    if (g_first + i * (int)blockDim.x < groups) grp[i] = split_group(w[i], amax[i], nan[i], p.scale_rule, shift);
 
   const int copies = kMode == 1 ? p.topk : 1;
   for (int s = 0; s < copies; ++s) {
@@ -1011,11 +1027,11 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
       rows = min(p.pass_rows, cnt - pass * p.pass_rows);
       tile = lo / p.pass_rows + e + pass;
     }
-    if (threadIdx.x == 0) p.x_scale[(int64_t)tile * p.pass_rows + m] = back;
+    if (threadIdx.x == 0 && (kMode != 0 || blockIdx.x % p.split == 0)) p.x_scale[(int64_t)tile * p.pass_rows + m] = back;
     uint8_t* dst = p.xop + (int64_t)tile * p.n_sb * p.x_unit;
 #pragma unroll
     for (int i = 0; i < kG; ++i) {
-      const int g = threadIdx.x + i * blockDim.x;
+      const int g = g_first + i * (int)blockDim.x;
       const unsigned here = __ballot_sync(0xffffffffu, g < groups);
       if (g >= groups) continue;
       if (kMode != 0 && p.x_unit == 0) store_group_matrix(grp[i], p.xop, p.sf, p.K, tile, m, g, here);
@@ -1073,12 +1089,18 @@ bool layout(const Info& f, Fp4Params& p) {
     };
     if (!take((uint32_t)(p.x_stages * p.x_unit), 1024, &p.x_off)) continue;
     if (!take(512 + f.extra, 128, &p.misc_off)) continue;
-    if (p.slices > 1 && !take((uint32_t)((p.M + p.slices - 1) / p.slices * p.slices * kBM * 4), 128, &p.red_off)) continue;
-    for (p.raw_stages = kMaxRaw; p.raw_stages >= 2; p.raw_stages >>= 1)
-      if (take(f.box * (uint32_t)p.raw_stages, 128, &p.raw_off)) {
+    const uint32_t red = p.slices > 1 ? (uint32_t)((p.M + p.slices - 1) / p.slices * p.slices * kBM * 4) : 0u;
+    // the raw ring first: in front of it the sums could leave room for two stages only (5120 x 17408, sixteen
+    // rows: 21 us instead of 15.7)
+    for (p.raw_stages = kMaxRaw; p.raw_stages >= 2; p.raw_stages >>= 1) {
+      const Region keep[2] = {reg[0], reg[1]};
+      if (take(f.box * (uint32_t)p.raw_stages, 128, &p.raw_off) && (red == 0 || take(red, 128, &p.red_off))) {
         if (p.E > 0 && !take(4u * (uint32_t)(p.E + 1), 128, &p.seg_off)) p.seg_off = 0;
         return true;
       }
+      reg[0] = keep[0];
+      reg[1] = keep[1];
+    }
   }
   return false;
 }
@@ -1137,18 +1159,44 @@ cudaError_t launch(int F, dim3 grid, cudaStream_t stream, const CUtensorMap& map
 }
 
 template <int kMode>
-int launch_rows(int64_t ctas, int64_t K, cudaStream_t stream, const RowsParams& p) {
+int launch_rows(int64_t rows, int64_t K, cudaStream_t stream, RowsParams p) {
   const int64_t groups = K / 16;
-  const int per = groups <= 512 ? 1 : groups <= 1024 ? 2 : kRowsMaxGroups;
-  const int64_t threads = ((groups + per - 1) / per + 31) / 32 * 32;
-  if (threads > 1024) return GB_EUNSUPPORTED;
-#define GB_FP4_ROWS(G) GB_CUDA_OK(gb_launch(fp4_rows_kernel<G, kMode>, dim3((unsigned)ctas), dim3((unsigned)threads), 0, stream, p))
-  switch (per) {
-    case 1: GB_FP4_ROWS(1); break;
-    case 2: GB_FP4_ROWS(2); break;
-    default: GB_FP4_ROWS(kRowsMaxGroups); break;
+  p.split = 1;
+  if (kMode == 0) {
+    p.split = groups > 512 ? (int)((groups + kRowSplitGroups - 1) / kRowSplitGroups) : 1;   // 384 groups: 1 us slower in two
+    if (p.split > kMaxRowSplit) p.split = kMaxRowSplit;
   }
-#undef GB_FP4_ROWS
+  const int64_t share = (groups + p.split - 1) / p.split;
+  const int per = kMode == 0 || share <= 512 ? 1 : share <= 1024 ? 2 : kRowsMaxGroups;
+  const int64_t threads = ((share + per - 1) / per + 31) / 32 * 32;
+  if (threads > 1024) return GB_EUNSUPPORTED;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(rows * p.split));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (gb_pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (p.split > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = (unsigned)p.split; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  gb_count_launch();
+  if constexpr (kMode == 0) {
+    GB_CUDA_OK(cudaLaunchKernelEx(&cfg, fp4_rows_kernel<1, kMode>, p));
+  } else {
+    switch (per) {
+      case 1: GB_CUDA_OK(cudaLaunchKernelEx(&cfg, fp4_rows_kernel<1, kMode>, p)); break;
+      case 2: GB_CUDA_OK(cudaLaunchKernelEx(&cfg, fp4_rows_kernel<2, kMode>, p)); break;
+      default: GB_CUDA_OK(cudaLaunchKernelEx(&cfg, fp4_rows_kernel<kRowsMaxGroups, kMode>, p)); break;
+    }
+  }
   return GB_OK;
 }
 
