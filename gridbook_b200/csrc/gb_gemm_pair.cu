@@ -201,34 +201,48 @@ GB_DEVINL void tile_at(const PairParams& p, int tile, int& mt, int& nt) {
   nt = in / rows;
 }
 
-// One tile: first row of A, first row of B; grouped: expert's weight row, its activation rows.
-struct Tile { int m0, n0; int w0, lo, rows, x_tile; };
-
+// The tiles of a pair, first, first + stride, ..: first row of A, first row of B; grouped: the expert's weight row and
+// its activation rows.  The expert is found by stepping on from the last tile's (a few experts per step of 74 tiles).
 template <int kBN, bool kGrouped>
-GB_DEVINL Tile tile_info(const PairParams& p, int tile, const int* seg_s, const int* base_s) {
-  Tile t = {};
-  if (!kGrouped) {
-    int mt, nt;
-    tile_at(p, tile, mt, nt);
-    t.m0 = mt * kPairM;
-    t.n0 = nt * kBN;
-  } else {
-    const int gp = tile / p.m_tiles;                         // row tile; the expert's weight tiles run fastest
-    int e = 0, hi = p.E;                                     // largest e with base_s[e] <= gp
-    while (hi - e > 1) {
-      const int mid = (e + hi) >> 1;
-      if (base_s[mid] <= gp) e = mid; else hi = mid;
+struct Tiles {
+  int m0 = 0, n0 = 0, w0 = 0, lo = 0, rows = 0, x_tile = 0;
+  int tile, gp = 0, mt = 0, e = 0;
+  int step, step_gp = 0, step_mt = 0;
+  GB_DEVINL Tiles(const PairParams& p, int first, int stride) : tile(first - stride), step(stride) {
+    if (kGrouped) {                                          // the expert's weight tiles run fastest
+      step_gp = stride / p.m_tiles;
+      step_mt = stride - step_gp * p.m_tiles;
+      gp = first / p.m_tiles;
+      mt = first - gp * p.m_tiles;
+      gp -= step_gp;
+      mt -= step_mt;
+      if (mt < 0) { mt += p.m_tiles; --gp; }
     }
-    const int pass = gp - base_s[e], lo = seg_s[e];
-    t.w0 = (tile - gp * p.m_tiles) * kPairM;
-    t.m0 = e * (int)p.N + t.w0;
-    t.lo = lo + pass * kTileRows;
-    t.rows = min(kTileRows, seg_s[e + 1] - t.lo);
-    t.x_tile = lo / kTileRows + e + pass;                    // tiles of different (expert, pass) never coincide
-    t.n0 = t.x_tile * kBN;
   }
-  return t;
-}
+  GB_DEVINL bool next(const PairParams& p, int total, const int* seg_s, const int* base_s) {
+    tile += step;
+    if (tile >= total) return false;
+    if (!kGrouped) {
+      int tm, tn;
+      tile_at(p, tile, tm, tn);
+      m0 = tm * kPairM;
+      n0 = tn * kBN;
+      return true;
+    }
+    gp += step_gp;
+    mt += step_mt;
+    if (mt >= p.m_tiles) { mt -= p.m_tiles; ++gp; }
+    while (base_s[e + 1] <= gp) ++e;                         // experts without rows are stepped over
+    const int pass = gp - base_s[e], first_row = seg_s[e];
+    w0 = mt * kPairM;
+    m0 = e * (int)p.N + w0;
+    lo = first_row + pass * kTileRows;
+    rows = min(kTileRows, seg_s[e + 1] - lo);
+    x_tile = first_row / kTileRows + e + pass;               // tiles of different (expert, pass) never coincide
+    n0 = x_tile * kBN;
+    return true;
+  }
+};
 
 template <Kind kKind, int kBN, bool kGrouped>
 __global__ void __launch_bounds__(Shape<kKind, kBN, kGrouped>::kThreads, 1)
@@ -316,8 +330,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const uint32_t full_pair = leader_addr(full_bar);
       int s = 0;
       uint32_t ph = 1;
-      for (int tile = first; tile < total_tiles; tile += stride) {
-        const Tile T = tile_info<kBN, kGrouped>(p, tile, seg_s, base_s);
+      for (Tiles<kBN, kGrouped> T(p, first, stride); T.next(p, total_tiles, seg_s, base_s);) {
         const int m0 = T.m0 + (int)rank * kBM, n0 = T.n0;
         for (int kt = 0; kt < p.k_tiles; ++kt) {
           wait(empty_bar + 8 * s, ph, abort_flag, p.status, 71);
@@ -350,10 +363,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (lane == 0 && rank == 0) {
       int s = 0, set = 0;
       uint32_t ph = 0, sf_ph = 0;
+      Tiles<kBN, kGrouped> T(p, first, stride);
       for (int it = 0; it < my_tiles; ++it) {
         const int buf = S::kAccs == 2 ? it & 1 : 0;
         const uint32_t use = (uint32_t)(S::kAccs == 2 ? it >> 1 : it);
-        const bool shifted = kKind == kFp4 && kBN % 128 != 0 && tile_info<kBN, kGrouped>(p, first + it * stride, seg_s, base_s).n0 % 128 != 0;
+        bool shifted = false;
+        if (kKind == kFp4 && kBN % 128 != 0) {
+          T.next(p, total_tiles, seg_s, base_s);
+          shifted = T.n0 % 128 != 0;
+        }
         wait(acc_empty + 8 * buf, (use & 1) ^ 1, abort_flag, p.status, 72);       // its last tile is drained
         const uint32_t acc = tmem_base + (buf ? S::kAcc1 : 0u);
         for (int kt = 0; kt < p.k_tiles; ++kt) {
@@ -416,12 +434,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       // Lane = weight row, i.e. output feature; column 96 h + 32 t + i = term t of activation row 32 h + i.  A
       // warp takes its half's three terms, adds them and stores 64 contiguous bytes per activation row.
       const int half = warp >> 2;
-      for (int tile = first; tile < total_tiles; tile += stride, ++it) {
-        const Tile T = tile_info<kBN, kGrouped>(p, tile, seg_s, base_s);
-        const int buf = it & 1, w = T.w0 + (int)rank * kBM + quarter * 32 + lane, m = half * 32 + lane;
+      for (Tiles<kBN, kGrouped> T(p, first, stride); T.next(p, total_tiles, seg_s, base_s); ++it) {
+        const int buf = S::kAccs == 2 ? it & 1 : 0, w = T.w0 + (int)rank * kBM + quarter * 32 + lane, m = half * 32 + lane;
         const float xs = m < T.rows ? p.x_scale[(int64_t)T.x_tile * kTileRows + m] : 0.0f;
         const int to = m < T.rows ? (p.row_map ? p.row_map[T.lo + m] : T.lo + m) : 0;
-        wait(acc_full + 8 * buf, (uint32_t)(it >> 1) & 1, abort_flag, p.status, 77);
+        wait(acc_full + 8 * buf, (uint32_t)(S::kAccs == 2 ? it >> 1 : it) & 1, abort_flag, p.status, 77);
         if (__any_sync(0xffffffffu, *abort_flag)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf ? S::kAcc1 : 0u) + (uint32_t)(half * 96);

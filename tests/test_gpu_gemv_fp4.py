@@ -155,3 +155,28 @@ def test_routed_layer_matches_the_loop_chain(dev, f13, f2, T):
     assert "sorted rows" in moe._cb_route
     assert np.linalg.norm(got - ref) / np.linalg.norm(ref) <= 3e-3
     assert np.abs(got - ref).max() <= 2e-2 * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("name", ["lit", "k16", "k20"])
+@pytest.mark.parametrize("T", [40, 60, 300, 1700])
+def test_several_tiles_per_cta_with_an_odd_number_of_superblocks(dev, name, T):
+    """More expert tiles than SMs, three superblocks of K in the down projection: units change from tile
+    to tile; up to sixteen rows a pass, more, and the stack decoded once (1700 tokens: 170 rows an
+    expert) against the decoded bf16 stack's grouped GEMM, run to run the same bits."""
+    from gridbook_b200 import synth
+    from gridbook_b200.moe import CBMoE
+    fmt = _fmt(name)
+    E, hidden, inter, topk = 40, 1024, 768, 4
+    w13d, w2d = synth.make_moe(fmt, fmt, E, hidden, inter, seed=T)
+    ids, tw = synth.make_routing(T, E, topk, seed=T)
+    x = synth.bf16_tensor(synth.make_activations(T, hidden, seed=T + 1), dev)
+    moe = CBMoE(fmt, fmt, E, hidden, inter, _tables(fmt, w13d["cb"]), _tables(fmt, w2d["cb"]))
+    moe.load(torch.from_numpy(w13d["qw"]), torch.from_numpy(w2d["qw"]), None, None, dev)
+    args = x, torch.from_numpy(tw).to(dev), torch.from_numpy(ids).to(dev)
+    got = [moe(*args).float() for _ in range(3)]
+    assert "sorted rows" in moe._cb_route
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    moe.method.prefill_min_pairs_per_expert = 1
+    ref = moe(*args).float()
+    assert "grouped prefill" in moe._cb_route
+    assert float((got[0] - ref).norm() / ref.norm()) <= 3e-3
