@@ -194,7 +194,11 @@ void need_bf16(const at::Tensor& t, const char* what) {
 }
 
 constexpr int64_t kDecodeMaxRows = 16;
-constexpr int64_t kFp4GemmMinRows = 160;
+// Routed rows per expert from which a stack is decoded once into its NVFP4 view and multiplied by the grouped GEMM,
+// instead of decoded in every pass of up to 64 rows.  128 experts, hidden 2048, intermediate 768: literal 299 against
+// 338 us at 96 rows and equal at 128, K16 350 / 364 at 96 and 454 / 417 at 128.  K20 and K24 hold one superblock per
+// raw stage and decode at half the rate: 286 / 299 at 16 rows, 388 / 284 at 32.
+constexpr int64_t kFp4GemmMinRows = 120, kFp4GemmMinRowsWide = 20;
 constexpr float kNvfp4ActRange = 448.0f;      // a row's largest group scale factor: the top of the UE4M3 range
 
 // Routes a plan has taken, reported to the host code by number.
@@ -495,8 +499,10 @@ struct MoEPlan {
     const Routing r = plan_routing(a, c);
     const int fp13 = L.gb_moe_fp4_pass_rows(&w13.w, w13.scales_e4m3, c.P, E), fp2 = L.gb_moe_fp4_pass_rows(&w2.w, w2.scales_e4m3, c.P, E);
     // decoded once and multiplied by the grouped GEMM (pass rows 0) where several passes would decode every weight again
-    const bool once = c.P >= kFp4GemmMinRows * E && E <= 1024;
-    const bool once13 = fp13 && once, once2 = fp2 && once;
+    auto once = [&](const Weight& w, int fp) {
+      return fp > 0 && E <= 1024 && c.P >= E * (w.w.fmt.k_bits >= 20 ? kFp4GemmMinRowsWide : kFp4GemmMinRows);
+    };
+    const bool once13 = once(w13, fp13), once2 = once(w2, fp2);
     const int pr13 = once13 ? 0 : fp13, pr2 = once2 ? 0 : fp2;
     const int64_t flat13 = once13 ? E * w13.w.rows : 0, flat2 = once2 ? E * w2.w.rows : 0;
     const int wq = a.add(std::max(flat13 * w13.w.K, flat2 * w2.w.K) / 2);
