@@ -228,13 +228,14 @@ GB_DEVINL uint32_t gb_e2m1_div2(float v0, float v1, float scale, float rinv) {
   return gb_cvt_e2m1x2(x0, x1);
 }
 
-// E4M3 bytes of clamp(v / scale, +-448), one rounding each; NaN clamps to -448 as fmaxf leaves it.
+// E4M3 bytes of clamp(v / scale, +-448), one rounding each (the conversion saturates); NaN gives -448 as fmaxf
+// leaves it.
 // `plain`: a divisor gb_div does not take.
 GB_DEVINL uint32_t gb_e4m3_div2(float v0, float v1, float scale, float rinv, bool plain) {
   float x0, x1;
   if (plain) { x0 = __fdiv_rn(v0, scale); x1 = __fdiv_rn(v1, scale); }
   else { x0 = gb_div(v0, scale, rinv); x1 = gb_div(v1, scale, rinv); }
-  return gb_cvt_e4m3x2(fminf(fmaxf(x0, -448.0f), 448.0f), fminf(fmaxf(x1, -448.0f), 448.0f));
+  return gb_cvt_e4m3x2(fmaxf(x0, -448.0f), fmaxf(x1, -448.0f));
 }
 
 // Two E2M1 codes (one byte) -> fp32.
@@ -269,19 +270,25 @@ GB_DEVINL uint32_t gb_fp4_bucket2(float v0, float v1, float scale, float rinv, b
   return gb_pack_bf16x2(fmaf(q.x, scale, 0.0f), fmaf(q.y, scale, 0.0f));
 }
 
+// Larger of two pairs of bf16, a NaN loses; larger of a pair of magnitudes as fp32.
+GB_DEVINL uint32_t gb_max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+GB_DEVINL float gb_max_of_bf16x2(uint32_t m) { return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u)); }
+
 // Largest magnitude of the words' bf16 values, NaNs ignored, and whether one of them is a NaN.
 template <int kWords>
 GB_DEVINL float gb_amax_bf16(const uint32_t (&w)[kWords], bool* has_nan) {
-  float amax = 0.0f;
-  bool nan = false;
+  uint32_t m = 0u, n = 0u;                                 // packed maxima, the second keeps NaNs
 #pragma unroll
   for (int i = 0; i < kWords; ++i) {
-    const float a = gb_bf16_bits_to_f32(w[i] & 0xFFFFu), b = gb_bf16_bits_to_f32(w[i] >> 16);
-    amax = fmaxf(amax, fmaxf(fabsf(a), fabsf(b)));
-    nan |= isnan(a) || isnan(b);
+    m = gb_max_bf16x2(m, w[i] & 0x7FFF7FFFu);
+    asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(n) : "r"(w[i] & 0x7FFF7FFFu));
   }
-  *has_nan = nan;
-  return amax;
+  *has_nan = (n & 0x7FFFu) > 0x7F80u || (n >> 16 & 0x7FFFu) > 0x7F80u;
+  return gb_max_of_bf16x2(m);
 }
 
 template <int kWords>

@@ -334,19 +334,20 @@ nvfp4_quantize_rows_kernel(const uint4* __restrict__ x, uint2* __restrict__ pack
   }
   const uint4* xr = x + row * 2 * groups;
   __shared__ float red[32];
-  uint32_t w[kG][8];
+  uint32_t w[kG][8], gtop[kG];                             // packed magnitude maxima of the groups
   float amax = 0.0f;
   for (int g0 = threadIdx.x; g0 < groups; g0 += kG * blockDim.x) {    // once, unless the row is longer than the registers
 #pragma unroll
     for (int j = 0; j < kG; ++j) {
       const int g = g0 + j * blockDim.x;
       const bool in = g < groups;
+      gtop[j] = 0u;
       const uint4 a = in ? xr[2 * g] : make_uint4(0u, 0u, 0u, 0u), b = in ? xr[2 * g + 1] : make_uint4(0u, 0u, 0u, 0u);
       w[j][0] = a.x; w[j][1] = a.y; w[j][2] = a.z; w[j][3] = a.w;
       w[j][4] = b.x; w[j][5] = b.y; w[j][6] = b.z; w[j][7] = b.w;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        amax = fmaxf(amax, fmaxf(fabsf(gb_bf16_bits_to_f32(w[j][i] & 0xffffu)), fabsf(gb_bf16_bits_to_f32(w[j][i] >> 16))));
+      for (int i = 0; i < 8; ++i) gtop[j] = gb_max_bf16x2(gtop[j], w[j][i] & 0x7FFF7FFFu);
+      amax = fmaxf(amax, gb_max_of_bf16x2(gtop[j]));
     }
   }
 #pragma unroll
@@ -370,14 +371,16 @@ nvfp4_quantize_rows_kernel(const uint4* __restrict__ x, uint2* __restrict__ pack
         const uint4 a = xr[2 * g], b = xr[2 * g + 1];
         w[j][0] = a.x; w[j][1] = a.y; w[j][2] = a.z; w[j][3] = a.w;
         w[j][4] = b.x; w[j][5] = b.y; w[j][6] = b.z; w[j][7] = b.w;
+        gtop[j] = 0u;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) gtop[j] = gb_max_bf16x2(gtop[j], w[j][i] & 0x7FFF7FFFu);
       }
       float xs[16];
-      float gmax = 0.0f;
+      const float gmax = __fmul_rn(gb_max_of_bf16x2(gtop[j]), gs);      // rounding keeps the order: the largest |xs|
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         xs[2 * i] = __fmul_rn(gb_bf16_bits_to_f32(w[j][i] & 0xffffu), gs);
         xs[2 * i + 1] = __fmul_rn(gb_bf16_bits_to_f32(w[j][i] >> 16), gs);
-        gmax = fmaxf(gmax, fmaxf(fabsf(xs[2 * i]), fabsf(xs[2 * i + 1])));
       }
       const float sf = live ? fminf(__fdiv_rn(gmax, 6.0f), 448.0f) : 0.0f;
       const uint32_t sf_byte = gb_f32_to_e4m3(sf);
@@ -425,7 +428,8 @@ int gb_nvfp4_quantize_rows(const void* x, int64_t M, int64_t K, float range, voi
   if (M == 0) return GB_OK;
   GB_REQUIRE(K / 16 < (1ll << 31), "dimension too large");
   const int64_t padded = (M + 127) / 128 * 128, groups = K / 16;
-  const int per = groups <= 512 ? 1 : groups <= 1024 ? 2 : kQuantMaxGroups;
+  int per = groups <= 512 ? 1 : groups <= 1024 ? 2 : kQuantMaxGroups;
+  if (per == 1 && M >= 8 * gb_sm_count()) per = 2;         // several waves of rows: smaller CTAs, more rows in flight
   int64_t threads = ((groups + per - 1) / per + 31) / 32 * 32;
   if (threads > 1024) threads = 1024;
 #define GB_NVFP4_ROWS(G)                                                                                          \
