@@ -20,7 +20,7 @@ REQUIRED_SYMBOLS = (
     "gb_abi_version", "gb_last_error", "gb_prepare", "gb_device_status", "gb_gemv_row_batch_max",
     "gb_fp8_act_qdq", "gb_fp4_act_qdq",
     "gb_expand_fp8", "gb_expand_fp4_bf16", "gb_expand_fp4_nvfp4",
-    "gb_gemv_workspace_bytes", "gb_gemv", "gb_gemv_static", "gb_gemv_hinted", "gb_scales_e4m3",
+    "gb_gemv_workspace_bytes", "gb_gemv", "gb_gemv_static", "gb_gemv_hinted", "gb_gemv_hinted_workspace_bytes", "gb_scales_e4m3",
     "gb_gemv_tab_slots_bytes", "gb_gemv_tab_arm", "gb_gemv_tab", "gb_device_status_reset", "gb_set_wait_limit_ms",
     "gb_set_row_routes", "gb_nvfp4_sf_bytes", "gb_nvfp4_quantize_rows", "gb_gemm_fp4",
     "gb_moe_route", "gb_moe_route_ws", "gb_moe_route_workspace_bytes", "gb_moe_gemv_workspace_bytes", "gb_moe_gemv", "gb_moe_combine",
@@ -116,6 +116,8 @@ def _declare(lib) -> None:
     lib.gb_expand_fp4_nvfp4.argtypes = [wp, i64, i64, vp, vp, i32, vp]
     lib.gb_gemv_workspace_bytes.argtypes = [i64, i64, i64]
     lib.gb_gemv_workspace_bytes.restype = i64
+    lib.gb_gemv_hinted_workspace_bytes.argtypes = [i64, i64, i64]
+    lib.gb_gemv_hinted_workspace_bytes.restype = i64
     lib.gb_gemv.argtypes = [vp, i64, wp, i32, i32, vp, vp, i64, vp]
     lib.gb_gemv_static.argtypes = [vp, i64, wp, i32, i32, vp, vp]
     wpp = ctypes.POINTER(wp)

@@ -912,9 +912,12 @@ int64_t gb_gemv_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   const int64_t umma_path = gb_gemv_umma_workspace_bytes(M, N, K);   // rows 2..128, literal format
   int64_t need = mma_path > dot_path ? mma_path : dot_path;
   if (umma_path > need) need = umma_path;
-  const int64_t fp4_path = gb_gemv_fp4_workspace_bytes(M, K);
-  if (fp4_path > need) need = fp4_path;
   return need > rows_path ? need : rows_path;
+}
+
+int64_t gb_gemv_hinted_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  const int64_t need = gb_gemv_workspace_bytes(M, N, K), fp4_path = gb_gemv_fp4_workspace_bytes(M, K);
+  return fp4_path > need ? fp4_path : need;
 }
 
 int gb_gemv_row_batch_max(const gb_weight* w) {

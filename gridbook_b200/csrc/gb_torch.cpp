@@ -34,7 +34,7 @@ namespace {
 struct Lib {
 #define GB_FN(name) decltype(&::name) name = nullptr
   GB_FN(gb_last_error);
-  GB_FN(gb_gemv_workspace_bytes);
+  GB_FN(gb_gemv_hinted_workspace_bytes);
   GB_FN(gb_gemv);
   GB_FN(gb_gemv_row_batch_max);
   GB_FN(gb_gemv_tab);
@@ -80,7 +80,7 @@ void bind(const std::string& path) {
   L.name = reinterpret_cast<decltype(L.name)>(dlsym(h, #name));                       \
   if (!L.name) throw std::runtime_error(path + " lacks the required symbol " #name)
   GB_FN(gb_last_error);
-  GB_FN(gb_gemv_workspace_bytes);
+  GB_FN(gb_gemv_hinted_workspace_bytes);
   GB_FN(gb_gemv);
   GB_FN(gb_gemv_row_batch_max);
   GB_FN(gb_gemv_tab);
@@ -248,7 +248,7 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
     }
     if (M <= kDecodeMaxRows || M <= std::min(midm_max, row_batch_max)) {
       at::Tensor ws = workspace;
-      const int64_t need = L.gb_gemv_workspace_bytes(M, N, K);
+      const int64_t need = L.gb_gemv_hinted_workspace_bytes(M, N, K);
       if (!ws.defined() || ws.numel() < need) ws = at::empty({need}, x.options().dtype(at::kByte));
       check(L.gb_gemv_hinted(xc.data_ptr(), M, &w.w, &hints, rule, out.data_ptr(), ws.data_ptr(), ws.numel(), stream));
       return out;

@@ -160,7 +160,7 @@ class PrismaQuantCBLinearMethod(LinearMethodBase):
                                                global_scale=self.global_scale)
         layer._cb_N, layer._cb_K = N, K
         layer._cb_workspace = torch.empty(
-            _native.load().gb_gemv_workspace_bytes(DECODE_MAX_M, N, K), dtype=torch.uint8, device=dev)
+            _native.load().gb_gemv_hinted_workspace_bytes(DECODE_MAX_M, N, K), dtype=torch.uint8, device=dev)
         layer._cb_layer_id = ops.register_cb_layer(self, layer)
         ops.warn_if_capture_sizes_exceed_the_decode_gates()
         # one activation row of the literal format: the one-launch table kernel and its armed slots

@@ -160,9 +160,11 @@ GB_API int gb_scales_e4m3(const gb_weight* w, int64_t rows, int32_t* flag, void*
  * of a multiple of sixteen bytes, one codebook per role or for all rows - run on the block-scaled
  * FP4 tensor cores (tcgen05 kind::mxf4nvf4): packed rows decoded to E2M1 nibbles in tensor memory,
  * activations split exactly into three E2M1 x UE4M3 terms, fp32 accumulate, same results as gb_gemv up to the
- * order of the sum.  Everything else goes to gb_gemv.  Replaces the same reference entries as gb_gemv. */
+ * order of the sum.  Everything else goes to gb_gemv.  workspace: gb_gemv_hinted_workspace_bytes()
+ * bytes.  Replaces the same reference entries as gb_gemv. */
 GB_API int gb_gemv_hinted(const void* x_bf16, int64_t M, const gb_weight* w, const gb_hints* hints, int scale_rule,
                           void* y_bf16, void* workspace, int64_t workspace_bytes, void* stream);
+GB_API int64_t gb_gemv_hinted_workspace_bytes(int64_t M, int64_t N, int64_t K);
 
 /* Row counts at which gb_gemv changes kernel for the literal format: up to `dot_rows` rows run one
  * inner-product-table GEMV per row (default 4, at most 8), from `umma_min` rows on the tensor-core
