@@ -151,13 +151,13 @@ GB_DEVINL void mma_pair(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, ui
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
         ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)accumulate) : "memory");
 }
-// Completion of the MMAs issued so far, told to the barrier at this offset in both CTAs.
-GB_DEVINL void commit_pair(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"((uint16_t)3) : "memory");
-}
-GB_DEVINL void commit_leader(uint32_t bar) {
+// Completion of the MMAs (or copies) issued so far, told to a barrier of either CTA.
+GB_DEVINL void commit_to(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+GB_DEVINL void commit_pair(uint32_t bar, uint32_t to_peer) {
+  commit_to(bar);
+  commit_to(bar + to_peer);
 }
 GB_DEVINL void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
@@ -361,6 +361,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   } else if (warp == kEpiWarps + 1) {
     // --------------------------- MMA issuer (the leader's) ------------------------------
     if (lane == 0 && rank == 0) {
+      uint32_t to_peer;                                      // distance of the peer's barriers
+      asm volatile("mapa.shared::cluster.u32 %0, %1, 1;" : "=r"(to_peer) : "r"(full_bar));
+      to_peer -= full_bar;
       int s = 0, set = 0;
       uint32_t ph = 0, sf_ph = 0;
       Tiles<kBN, kGrouped> T(p, first, stride);
@@ -387,15 +390,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           for (int k = 0; k < 4; ++k)                        // 32 bytes of K per instruction
             mma_pair<kKind>(acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), p.idesc, sfa_t + 4u * k, sfb_t + 8u * k,
                             kt > 0 || k > 0);
-          commit_pair(empty_bar + 8 * s);
+          commit_pair(empty_bar + 8 * s, to_peer);
           if (kKind == kFp4) {
-            commit_leader(sf_empty + 8 * set);
+            commit_to(sf_empty + 8 * set);
             if (++set == S::kSets) { set = 0; sf_ph ^= 1; }
           }
           if (++s == kStages) { s = 0; ph ^= 1; }
         }
         if (*abort_flag) break;
-        commit_pair(acc_full + 8 * buf);
+        commit_pair(acc_full + 8 * buf, to_peer);
       }
     }
   } else if (warp >= kEpiWarps + 2) {
@@ -415,7 +418,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         sf_to_tmem(col + 4u * k, sf + 512u * k);
         sf_to_tmem(col + 16u + 8u * k, sf + S::kAtoms + 512u * k);
         sf_to_tmem(col + 20u + 8u * k, sf + 2 * S::kAtoms + 512u * k);
-        commit_leader(sf_full + 8 * set);
+        commit_to(sf_full + 8 * set);
         if (++set == S::kSets) { set = 0; sf_ph ^= 1; }
         if (++s == kStages) { s = 0; ph ^= 1; }
       }
