@@ -31,6 +31,10 @@ PREFILL_MIN_PAIRS_PER_EXPERT = 384
 # rows from SORTED_MIN_PAIRS_OTHER routed pairs in all (two tokens at top-8: 223 us against 272 us
 # on 32 experts of hidden 7168, intermediate 2048).
 SORTED_MIN_PAIRS_PER_EXPERT = 4
+# On the block-scaled FP4 cores the sorted rows of many experts cross over earlier: 128 experts as above, 48
+# tokens (3 pairs per expert) 125 us per pair against 115 sorted, 63 tokens 154 against 119; with 64 experts
+# three pairs per expert are even (58 and 59 us), with 32 the fixed launches of the sorted route weigh more.
+SORTED_MIN_PAIRS_FP4, SORTED_FP4_EXPERTS = 3, 128
 SORTED_MIN_PAIRS_OTHER = 16
 # Stacks of the fp4 grid multiply the sorted rows on the block-scaled FP4 tensor cores, several times the
 # rate of the decoded bf16 stack's GEMM: they stay on that route.
@@ -283,6 +287,7 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
             kernels.moe_gemv_sorted_applies(w13), sorted2, pair_ok)
         if layer._cb_plan.fp4 and self.prefill_min_pairs_per_expert == PREFILL_MIN_PAIRS_PER_EXPERT:
             self.prefill_min_pairs_per_expert = PREFILL_MIN_PAIRS_FP4
+        layer._cb_sorted_early = layer._cb_plan.fp4 and layer._cb_E >= SORTED_FP4_EXPERTS
         layer._cb_layer_id = ops.register_cb_layer(self, layer)
         print(f"[prismaquant-cb] {self.prefix}: decode=grouped-cuda (sm_100a) "
               f"w13={self.fmt13.grid}/k{self.fmt13.k} w2={self.fmt2.grid}/k{self.fmt2.k}",
@@ -324,8 +329,11 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
         number of routed pairs and this method's thresholds (MoEPlan in csrc/gb_torch.cpp).  No host
         read, so every size can be captured."""
         plan = layer._cb_plan
+        sorted_min = self.sorted_min_pairs_per_expert
+        if sorted_min == SORTED_MIN_PAIRS_PER_EXPERT and layer._cb_sorted_early:
+            sorted_min = SORTED_MIN_PAIRS_FP4
         out = plan(x, topk_weights, topk_ids, kernels.rule_code(ops.ACT_SCALE_RULE),
-                   (self.pair_kernel_max_pairs, self.sorted_min_pairs_per_expert, self.sorted_min_pairs_other,
+                   (self.pair_kernel_max_pairs, sorted_min, self.sorted_min_pairs_other,
                     self.prefill_min_pairs_per_expert, self.prefill_min_pairs_other, FUSED_BUCKET_MAX_PAIRS))
         layer.__dict__["_cb_route"] = _ROUTES[plan.route]
         return out
