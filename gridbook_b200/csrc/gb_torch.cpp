@@ -227,11 +227,15 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
   }
 
   at::Tensor forward(const at::Tensor& x, int rule, bool nvfp4, int64_t midm_max) {
-    need_cuda(x);
     const int64_t N = w.w.rows, K = w.w.K;
-    if (x.dim() < 1 || x.numel() % K != 0) throw std::runtime_error("activations do not divide into rows of " + std::to_string(K));
-    const int64_t M = x.numel() / K;
+    if (x.dim() < 1) throw std::runtime_error("activations are rows of " + std::to_string(K) + " values, got a scalar");
     std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+    int64_t M = 1;
+    for (size_t i = 0; i + 1 < shape.size(); ++i) M *= shape[i];
+    // the output has M rows: an input of another width, whatever its element count, would make the kernels write others
+    if (M > 0 && shape.back() != K)
+      throw std::runtime_error("activations are rows of " + std::to_string(K) + " values, got rows of " + std::to_string(shape.back()));
+    need_cuda(x);
     shape.back() = N;
     if (M == 0) return at::empty(shape, x.options());
     need_bf16(x, "the codebook linear");
@@ -301,7 +305,7 @@ py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, con
   const size_t n = plans.size();
   if (n < 2 || n > 4 || !x.is_cuda() || x.dim() < 1) return py::none();
   const int64_t K = plans[0]->w.w.K;
-  if (x.numel() != K) return py::none();
+  if (x.numel() != K || x.size(-1) != K) return py::none();   // another width: refused where the layers are called one by one
   for (const auto& p : plans)
     if (!p->slots.defined() || p->w.w.K != K) return py::none();
   need_bf16(x, "the table GEMV");

@@ -120,3 +120,20 @@ def test_other_formats_are_declined(dev):
     slots = kernels.new_tab_slots([lit])
     x = synth.bf16_tensor(synth.make_activations(1, 1024, seed=1), dev)
     assert kernels.gemv_tab(x, [w], slots) is None
+
+
+def test_shared_row_takes_one_row_of_the_layers_width_only(dev):
+    """Rows of another width with the same element count are refused by the layers, one by one."""
+    from gridbook_b200 import synth
+    from gridbook_b200.formats import NVFP4_LITERAL
+    from gridbook_b200.linear import CBLinear, apply_shared_row
+    K = 1024
+    lins = []
+    for i, N in enumerate((256, 128)):
+        lin = CBLinear(NVFP4_LITERAL, K, [N], [synth.codebook_tables(NVFP4_LITERAL, i)], global_scale=1.0 / 448.0)
+        gen = torch.Generator(device=dev).manual_seed(i)
+        lins.append(lin.load(synth.make_packed_device(NVFP4_LITERAL, N, K, gen, dev), None, dev))
+    for shape in [(2, K // 2), (4, 2 * K), (K // 4, 4)]:
+        with pytest.raises(RuntimeError, match=f"rows of {K} values"):
+            apply_shared_row(lins, torch.zeros(shape, dtype=torch.bfloat16, device=dev))
+    assert [tuple(y.shape) for y in apply_shared_row(lins, torch.zeros(1, K, dtype=torch.bfloat16, device=dev))] == [(1, 256), (1, 128)]

@@ -820,3 +820,18 @@ def test_expert_stacks_that_were_never_filled_are_refused_after_loading():
     with pytest.raises(NativeKernelUnavailableError, match="CUDA device"):
         alone.load(torch.zeros(2, 512, 48, dtype=torch.uint8), torch.zeros(2, 256, 48, dtype=torch.uint8), device="cpu")
     assert M.unfilled_cb_params(alone) == []
+
+
+def test_linear_plan_refuses_rows_of_another_width_before_anything_else():
+    """The output of a linear has one row per leading index of its input: an input whose element count
+    is a multiple of K but whose rows are not K wide would make the kernels write other rows."""
+    from gridbook_b200 import _native, formats as F, kernels
+    K = 1024
+    w = _cpu_weight(F.NVFP4_LITERAL, K=K)
+    plan = _native.host().LinearPlan(kernels.host_weight(w), torch.empty(16, dtype=torch.uint8), None, [])
+    for shape in [(4, 2 * K), (2, K // 2), (2 * K,), (3, 2, K // 2), (1, 4, 8 * K), (3, 0), ()]:
+        with pytest.raises(RuntimeError, match=f"rows of {K} values"):
+            plan(torch.empty(shape, dtype=torch.bfloat16), 0, True, 128)
+    for shape in [(4, K), (K,), (0, K), (2, 0, 3)]:          # a shape that fits (or an empty batch) is refused only for the device
+        with pytest.raises(RuntimeError, match="CUDA tensors only"):
+            plan(torch.empty(shape, dtype=torch.bfloat16), 0, True, 128)
