@@ -85,22 +85,34 @@ GB_DEVINL uint32_t leader_addr(uint32_t addr) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
   return r;
 }
-// Relaxed: what it guards is tensor memory, which the loads have left; a release at cluster scope would wait for
-// the output stores in flight, once a tile.
+// An accumulator goes back from the epilogue warps of both CTAs to the leader's MMA issuer.  What the pair of arrive
+// and wait hands over is tensor memory alone, so the tensor-memory fences order it and the barrier may be
+// relaxed (the PTX pattern for tcgen05 instructions of different threads: tcgen05.ld, wait::ld,
+// fence::before_thread_sync, arrive.relaxed.cluster | try_wait.relaxed.cluster, fence::after_thread_sync,
+// tcgen05.mma) - at cluster scope on both sides, since the threads may be of different CTAs.  An arrive that
+// released would wait for the output stores in flight, once a tile: 4096 tokens of a routed layer 637 -> 664 us,
+// 333 rows of a dense one 248 -> 254; one thread of the peer that collects its warps' arrives and releases them
+// together: 640, 252.
 GB_DEVINL void arrive_cluster(uint32_t addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
+template <bool kTmemOfPair>
 GB_DEVINL bool try_wait(uint32_t bar, uint32_t parity) {
   uint32_t done;
-  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  if (kTmemOfPair)
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  else
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
 // A bounded wait that remembers a timeout for the rest of the CTA: later waits return at once.
+template <bool kTmemOfPair>
 __device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   uint64_t t0 = 0;
   for (uint32_t spin = 0; !*abort_flag; ++spin) {
-    if (try_wait(bar, parity)) return;
+    if (try_wait<kTmemOfPair>(bar, parity)) return;
     if ((spin & 255u) == 255u) {
       const uint64_t now = gb_globaltimer_ns();
       if (t0 == 0) t0 = now;
@@ -108,8 +120,9 @@ __device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, volatile i
     }
   }
 }
+template <bool kTmemOfPair = false>
 GB_DEVINL void wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  if (!try_wait(bar, parity)) wait_slow(bar, parity, abort_flag, status, code);
+  if (!try_wait<kTmemOfPair>(bar, parity)) wait_slow<kTmemOfPair>(bar, parity, abort_flag, status, code);
 }
 // Tile load into this CTA's shared memory that reports to a barrier of the pair.
 GB_DEVINL void tma_load_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
@@ -375,7 +388,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           T.next(p, total_tiles, seg_s, base_s);
           shifted = T.n0 % 128 != 0;
         }
-        wait(acc_empty + 8 * buf, (use & 1) ^ 1, abort_flag, p.status, 72);       // its last tile is drained
+        wait<true>(acc_empty + 8 * buf, (use & 1) ^ 1, abort_flag, p.status, 72); // its last tile is drained
         const uint32_t acc = tmem_base + (buf ? S::kAcc1 : 0u);
         for (int kt = 0; kt < p.k_tiles; ++kt) {
           if (kKind == kFp4) wait(sf_full + 8 * set, sf_ph, abort_flag, p.status, 73);

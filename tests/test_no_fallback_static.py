@@ -87,3 +87,14 @@ def test_no_except_clause_swallows_a_missing_kernel():
             caught = ast.unparse(node.type) if node.type is not None else "BaseException"
             assert "NativeKernelUnavailableError" not in caught, f"{name}:{node.lineno} catches the fail-closed error"
             assert "StaleExtensionError" not in caught, f"{name}:{node.lineno} catches the stale-library error"
+
+
+def test_arrivals_from_another_cta_are_waited_for_at_cluster_scope():
+    """A source that arrives on a barrier of another CTA of its cluster also has a wait whose scope is the
+    cluster: a wait at the scope of the CTA does not pair up with it."""
+    csrc = os.path.join(PKG, "csrc")
+    for f in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, f)) as fh:
+            text = fh.read()
+        if re.search(r"mbarrier\.arrive\.\w+\.cluster\.shared::cluster", text):
+            assert re.search(r"mbarrier\.try_wait\.parity\.\w+\.cluster", text), f
