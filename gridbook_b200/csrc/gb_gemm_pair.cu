@@ -86,21 +86,21 @@ GB_DEVINL uint32_t leader_addr(uint32_t addr) {
   return r;
 }
 // An accumulator goes back from the epilogue warps of both CTAs to the leader's MMA issuer.  What the pair of arrive
-// and wait hands over is tensor memory alone, so the tensor-memory fences order it and the barrier may be
+// and wait hands over is tensor memory alone, so the tensor-memory fences order it and the arrive may be
 // relaxed (the PTX pattern for tcgen05 instructions of different threads: tcgen05.ld, wait::ld,
-// fence::before_thread_sync, arrive.relaxed.cluster | try_wait.relaxed.cluster, fence::after_thread_sync,
-// tcgen05.mma) - at cluster scope on both sides, since the threads may be of different CTAs.  An arrive that
-// released would wait for the output stores in flight, once a tile: 4096 tokens of a routed layer 637 -> 664 us,
+// fence::before_thread_sync, arrive.relaxed.cluster | try_wait.relaxed.cluster or stronger,
+// fence::after_thread_sync, tcgen05.mma) - at cluster scope on both sides, since the threads may be of different
+// CTAs; so are the other waits that the peer's arrivals end.  An arrive that released would wait for the output stores in flight, once a tile: 4096 tokens of a routed layer 637 -> 664 us,
 // 333 rows of a dense one 248 -> 254; one thread of the peer that collects its warps' arrives and releases them
 // together: 640, 252.
 GB_DEVINL void arrive_cluster(uint32_t addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
-template <bool kTmemOfPair>
+template <bool kOfPair>
 GB_DEVINL bool try_wait(uint32_t bar, uint32_t parity) {
   uint32_t done;
-  if (kTmemOfPair)
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+  if (kOfPair)
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   else
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
@@ -108,11 +108,11 @@ GB_DEVINL bool try_wait(uint32_t bar, uint32_t parity) {
   return done != 0;
 }
 // A bounded wait that remembers a timeout for the rest of the CTA: later waits return at once.
-template <bool kTmemOfPair>
+template <bool kOfPair>
 __device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   uint64_t t0 = 0;
   for (uint32_t spin = 0; !*abort_flag; ++spin) {
-    if (try_wait<kTmemOfPair>(bar, parity)) return;
+    if (try_wait<kOfPair>(bar, parity)) return;
     if ((spin & 255u) == 255u) {
       const uint64_t now = gb_globaltimer_ns();
       if (t0 == 0) t0 = now;
@@ -120,9 +120,9 @@ __device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, volatile i
     }
   }
 }
-template <bool kTmemOfPair = false>
+template <bool kOfPair = false>
 GB_DEVINL void wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  if (!try_wait<kTmemOfPair>(bar, parity)) wait_slow<kTmemOfPair>(bar, parity, abort_flag, status, code);
+  if (!try_wait<kOfPair>(bar, parity)) wait_slow<kOfPair>(bar, parity, abort_flag, status, code);
 }
 // Tile load into this CTA's shared memory that reports to a barrier of the pair.
 GB_DEVINL void tma_load_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
@@ -346,7 +346,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       for (Tiles<kBN, kGrouped> T(p, first, stride); T.next(p, total_tiles, seg_s, base_s);) {
         const int m0 = T.m0 + (int)rank * kBM, n0 = T.n0;
         for (int kt = 0; kt < p.k_tiles; ++kt) {
-          wait(empty_bar + 8 * s, ph, abort_flag, p.status, 71);
+          wait<true>(empty_bar + 8 * s, ph, abort_flag, p.status, 71);
           if (*abort_flag) break;
           const uint32_t st = ring + (uint32_t)s * S::kStageBytes;
           if (rank == 0) expect_tx(full_bar + 8 * s, 2 * S::kStageBytes);
@@ -454,7 +454,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int buf = S::kAccs == 2 ? it & 1 : 0, w = T.w0 + (int)rank * kBM + quarter * 32 + lane, m = half * 32 + lane;
         const float xs = m < T.rows ? p.x_scale[(int64_t)T.x_tile * kTileRows + m] : 0.0f;
         const int to = m < T.rows ? (p.row_map ? p.row_map[T.lo + m] : T.lo + m) : 0;
-        wait(acc_full + 8 * buf, (uint32_t)(S::kAccs == 2 ? it >> 1 : it) & 1, abort_flag, p.status, 77);
+        wait<true>(acc_full + 8 * buf, (uint32_t)(S::kAccs == 2 ? it >> 1 : it) & 1, abort_flag, p.status, 77);
         if (__any_sync(0xffffffffu, *abort_flag)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf ? S::kAcc1 : 0u) + (uint32_t)(half * 96);
@@ -483,7 +483,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const int row0 = mt * kPairM + (int)rank * kBM + quarter * 32, row = row0 + lane;
       const bool row_ok = row < p.M;
       const float rs = (p.a_scale && row_ok ? p.a_scale[row] : 1.0f) * p.global_scale;
-      wait(acc_full + 8 * buf, (uint32_t)(S::kAccs == 2 ? it >> 1 : it) & 1, abort_flag, p.status, 77);
+      wait<true>(acc_full + 8 * buf, (uint32_t)(S::kAccs == 2 ? it >> 1 : it) & 1, abort_flag, p.status, 77);
       if (__any_sync(0xffffffffu, *abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tbase = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf ? S::kAcc1 : 0u) + (uint32_t)c_lo;
