@@ -79,9 +79,10 @@ int gb_tensor_map_operand(void* map_out, const void* base, int64_t rows, int64_t
 // Row-major bf16 output [M, N] in boxes of 32 x 32 with the 64-byte swizzle (N a multiple of 8).
 int gb_tensor_map_out(void* map_out, void* base, int64_t M, int64_t N);
 // Activation operand of the grouped GEMM (gb_moe_gemm_fp4): tiles of 64 rows, [tile][64 code rows of q, 64 of the
-// correction][K / 2 bytes], then the scale-factor atoms of 192 columns a tile, then the rows' powers of two.
+// correction][K / 2 bytes], then the scale-factor atoms of 192 columns a tile, then the rows' powers of two, then
+// the scales of the groups left out as [tile][64][K / 16] (gb_left_out).
 // Column 96 (m / 32) + 32 t + m % 32 of a tile is term t of row m.
-struct GbFp4Tiles { int64_t tiles, sf_groups, sf_at, scale_at, bytes; };
+struct GbFp4Tiles { int64_t tiles, sf_groups, sf_at, scale_at, tail_at, bytes; };
 inline GbFp4Tiles gb_fp4_tiles(int64_t P, int64_t E, int64_t K) {
   GbFp4Tiles t;
   auto up = [](int64_t v) { return (v + 255) & ~(int64_t)255; };
@@ -89,7 +90,8 @@ inline GbFp4Tiles gb_fp4_tiles(int64_t P, int64_t E, int64_t K) {
   t.sf_groups = (t.tiles * 192 + 127) / 128;
   t.sf_at = up(t.tiles * 128 * (K / 2));
   t.scale_at = t.sf_at + up(t.sf_groups * (K / 64) * 512);
-  t.bytes = t.scale_at + up(t.tiles * 64 * 4);
+  t.tail_at = t.scale_at + up(t.tiles * 64 * 4);
+  t.bytes = t.tail_at + up(t.tiles * 64 * (K / 16) * 4);
   return t;
 }
 // The prefill GEMMs on CTA pairs (gb_gemm_pair.cu), for the shapes that gb_gemm_pair_applies names.
@@ -338,6 +340,56 @@ GB_DEVINL uint4 gb_fp4_group16_qdq_pair(uint4 in, int scale_rule) {
   nan |= __shfl_xor_sync(0xffffffffu, nan, 1);
   gb_fp4_bucket_words(w, amax, nan != 0, scale_rule);
   return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// The three-term operand of the block-scaled FP4 kernels (gb_gemv_fp4.cu) holds the groups of a row that lie within
+// 2^13 of each other.  Other groups are left out: `tail` has their fp32 scales ([row][K / 16], zero for every other
+// group), and the low bits of the row's power of two say which sixteenths of the row hold any.  They are
+// multiplied on the plain fp32 units: the lane's weight row times groups [g_begin, g_end) of four activation
+// rows (those in `rows`), added to acc.  codes(r, g): the E2M1 codes of a group; load(g): what the lane's weight
+// row needs of it (32 rows: some three hundred shared-memory-path cycles, hence four rows for each); dot(raw, x): its
+// sixteen weights times x, which lane i (and i + 16) holds element i of.
+constexpr uint32_t kGbLeftOutBits = 0xFFFFu, kGbRowScaleMask = 0x7F800000u;
+GB_DEVINL int gb_left_out_span(int n_sb) { return (n_sb + 15) / 16; }   // superblocks per bit
+template <typename Codes, typename Load, typename Dot>
+GB_DEVINL void gb_left_out(float (&acc)[4], const float* tail, int64_t pitch, uint32_t rows, int g_begin, int g_end, Codes codes,
+                           Load load, Dot dot) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int g0 = g_begin; g0 < g_end; g0 += 32) {
+    float s[4];
+    bool any = false;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      s[r] = (rows >> r & 1u) && g0 + lane < g_end ? tail[r * pitch + g0 + lane] : 0.0f;
+      any |= s[r] != 0.0f;
+    }
+#pragma unroll 1
+    for (uint32_t have = __ballot_sync(0xffffffffu, any); have != 0; have &= have - 1) {
+      const int b = __ffs(have) - 1, g = g0 + b;
+      const auto raw = load(g);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float scale = __shfl_sync(0xffffffffu, s[r], b);
+        if (scale == 0.0f) continue;                       // the same in every lane
+        const uint2 q = codes(r, g);
+        const uint32_t c = ((lane & 8) ? q.y : q.x) >> (4 * (lane & 7));   // bucketed value: bf16(q * scale)
+        acc[r] += dot(raw, gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(__fmul_rn(gb_e2m1x2_to_f32(c & 0xFu).x, scale))));
+      }
+    }
+  }
+}
+// What the groups left out of a row add to a sum that still carries the row's normalisation.
+GB_DEVINL float gb_normalised(float v, uint32_t x_word) { return v * __uint_as_float((254u << 23) - (x_word & kGbRowScaleMask)); }
+// Adds v to four tensor-memory columns of the warp's lanes.
+GB_DEVINL void gb_tmem_add(uint32_t taddr, const float (&v)[4]) {
+  uint32_t u[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i) u[i] = __float_as_uint(__uint_as_float(u[i]) + v[i]);
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]) : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // gate / (1 + exp(-gate)) with the quotient taken as a product with the reciprocal and one correction

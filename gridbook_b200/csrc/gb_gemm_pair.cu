@@ -77,6 +77,8 @@ struct PairParams {
   const int32_t* seg;          // [E + 1]
   const int32_t* row_map;      // output row of a sorted row, or null
   const float* x_scale;        // [row tile][64]
+  const float* tail;           // [row tile][64][K / 16], and the operands as they lie in memory: for groups left out
+  const uint8_t *codes, *packed, *sf;
   int E;
 };
 
@@ -458,6 +460,49 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (__any_sync(0xffffffffu, *abort_flag)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + (buf ? S::kAcc1 : 0u) + (uint32_t)(half * 96);
+        if (__builtin_expect(__any_sync(0xffffffffu, __float_as_uint(xs) & kGbLeftOutBits), 0)) {
+          // groups left out: added to the sums in tensor memory
+          const int64_t w_row = T.m0 - T.w0 + min(w, (int)p.N - 1);
+          const uint8_t* wp = p.packed + w_row * (p.K / 2);
+          const uint8_t* sf = p.sf + (w_row >> 7) * (p.K * 8) + (w_row & 31) * 16 + (w_row >> 5 & 3) * 4;
+          const int n_sb = (int)(p.K / 256), per = gb_left_out_span(n_sb);
+          struct Raw { uint2 c; float scale; };
+#pragma unroll 1
+          for (int i0 = 0; i0 < 32; i0 += 4) {
+            uint32_t word[4], bits = 0u, marked = 0u;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              word[r] = __float_as_uint(__shfl_sync(0xffffffffu, xs, i0 + r));
+              bits |= word[r] & kGbLeftOutBits;
+              marked |= (word[r] & kGbLeftOutBits) != 0 ? 1u << r : 0u;
+            }
+            if (bits == 0) continue;
+            const int64_t m0 = (int64_t)T.x_tile * kTileRows + half * 32 + i0;
+            const uint8_t* codes = p.codes + (m0 + (int64_t)T.x_tile * kTileRows) * (p.K / 2);
+            float add[4] = {};
+#pragma unroll 1
+            for (; bits != 0; bits &= bits - 1) {
+              const int b = __ffs(bits) - 1;
+              gb_left_out(
+                  add, p.tail + m0 * (p.K / 16), p.K / 16, marked, b * per * 16, min((b + 1) * per, n_sb) * 16,
+                  [&](int r, int g) { return *reinterpret_cast<const uint2*>(codes + r * (p.K / 2) + g * 8); },
+                  [&](int g) { return Raw{*reinterpret_cast<const uint2*>(wp + g * 8), gb_e4m3_to_f32(sf[(g >> 2) * 512 + (g & 3)])}; },
+                  [](const Raw& q, float x) {
+                    float s = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                      const float2 v = gb_e2m1x2_to_f32((j < 4 ? q.c.x : q.c.y) >> (8 * (j & 3)) & 0xFFu);
+                      s = fmaf(__shfl_sync(0xffffffffu, x, 2 * j), v.x, s);
+                      s = fmaf(__shfl_sync(0xffffffffu, x, 2 * j + 1), v.y, s);
+                    }
+                    return s * q.scale;
+                  });
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) add[r] = gb_normalised(add[r], word[r]);
+            gb_tmem_add(at + (uint32_t)i0, add);
+          }
+        }
         uint32_t hi[32], lo[32], dl[32];
         tmem_ld32(at, hi);
         tmem_ld32(at + 32u, lo);
@@ -470,7 +515,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const float v = fmaf(__uint_as_float(dl[i]), 0x1p-7f, fmaf(__uint_as_float(lo[i]), 0x1p-4f, __uint_as_float(hi[i])));
-          const float r = v * __shfl_sync(0xffffffffu, xs, i) * p.global_scale;
+          const float r = v * __uint_as_float(__float_as_uint(__shfl_sync(0xffffffffu, xs, i)) & kGbRowScaleMask) * p.global_scale;
           const int64_t row = __shfl_sync(0xffffffffu, to, i);
           if (i < n && w < p.N) p.D[row * p.N + w] = (uint16_t)gb_f32_to_bf16_bits(r);
         }
@@ -693,6 +738,10 @@ int gb_moe_gemm_fp4(const void* operand, const void* packed, const void* sf, int
   p.status = gb_status_word();
   p.seg = seg; p.row_map = row_map; p.E = (int)E;
   p.x_scale = (const float*)((const uint8_t*)operand + op.scale_at);
+  p.tail = (const float*)((const uint8_t*)operand + op.tail_at);
+  p.codes = (const uint8_t*)operand;
+  p.packed = (const uint8_t*)packed;
+  p.sf = (const uint8_t*)sf;
   CUtensorMap map_a, map_b, map_d = {}, map_sfa, map_sfb;
   int rc = gb_tensor_map_operand(&map_a, packed, E * N, K / 2, 1, kBM);
   if (rc != GB_OK) return rc;

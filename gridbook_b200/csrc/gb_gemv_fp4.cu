@@ -14,8 +14,11 @@
 //   * dlt : bf16(1.5 s) - 1.5 m1 is n half-ulps of m1 with |n| <= 3, so for q = 1.5, 3, 6 the missing
 //           part is (n q / 3) half-ulps: again an E2M1 value times a power of two.
 // Every term is normalised per row by a power of two that puts the row's largest m1 into [128, 256).
-// UE4M3 reaches down to 2^-9, so the split is exact for groups within 2^13 of the row's largest; a
-// smaller group loses less than 2^-21 of the row's largest scale, below the fp32 sum's own rounding.
+// UE4M3 is normal down to 2^-6, so the split is exact for groups within 2^13 of the row's largest.  A row that
+// spans more is normalised around its mean exponent instead; what is still out of range - an outlier channel,
+// or groups far below the rest - is left out of the operand and added while the sums are read out
+// (gb_left_out).  No group may be dropped: a weight row may be zero wherever the activations are large, and
+// its result is then the small groups' alone.
 //
 // Up to sixteen rows the three terms are columns of one MMA (N <= 48).  Past them two MMAs share the
 // codes of q: N = 2 R with the scale factors [hi | dlt] over the code rows [q | e], N = R with lo over
@@ -94,7 +97,10 @@ struct Fp4Params {
   uint32_t x_off, raw_off, misc_off, red_off;
   const uint8_t* xop;        // activation operand: [tile][superblock][scale factors | codes]
   int64_t x_unit;            // bytes of one superblock of it
-  const float* x_scale;      // [tile][pass_rows] power of two of every row
+  const float* x_scale;      // [tile][pass_rows] power of two of every row; low bits: where groups are left out
+  const float* tail;         // [tile][pass_rows][K / 16] scales of the groups left out, of the rows that have any
+  const uint8_t* qw;         // the packed rows again, for those
+  int64_t row_stride;
   const void* codebook;      // bf16 flat
   const float* compose;
   float global_scale;
@@ -123,6 +129,8 @@ __host__ __device__ constexpr int mma_cols(bool wide, int rows) {
 // Bytes in front of the codes of a unit: scale-factor atoms of 128 columns (wide: two sets).
 __host__ __device__ constexpr int sf_bytes(bool wide) { return wide ? 4096 : 2048; }
 __host__ __device__ constexpr int unit_bytes(bool wide, int rows) { return sf_bytes(wide) + mma_cols(wide, rows) * 128; }
+// Offset of group gi of code row n behind them (128-byte swizzle).
+__host__ __device__ constexpr int code_at(int n, int gi) { return (n >> 3) * 1024 + (n & 7) * 128 + (((gi >> 1) ^ (n & 7)) << 4) + (gi & 1) * 8; }
 
 // ---- PTX ---------------------------------------------------------------------------------------
 GB_DEVINL void mbar_init(uint32_t bar, uint32_t count) {
@@ -330,6 +338,46 @@ GB_DEVINL void build_scale_tab(const Fp4Params& p, int d, uint32_t scale_tab) {
       asm volatile("st.shared.u32 [%0], %1;" ::"r"(scale_tab + (uint32_t)i), "r"(w) : "memory");
     }
   }
+}
+
+// Group g of a packed row (sixteen bf16 codebook values and their scale), from global memory: the tables in shared
+// memory may already be another role's.
+struct RowGroup { uint2 v[4]; float scale; };
+template <int F>
+GB_DEVINL RowGroup row_group(const uint8_t* row, const uint16_t* cb, const float* compose, int g) {
+  const uint8_t* sb = row + (g >> 4) * Fmt<F>::kSb;
+  const int gi = g & 15;
+  RowGroup r;
+  if constexpr (F == kLit) {
+    r.scale = gb_e4m3_to_f32(sb[32 + gi]);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const uint4 e = *reinterpret_cast<const uint4*>(cb + 8 * sb[2 * gi + c]);
+      r.v[2 * c] = make_uint2(e.x, e.y);
+      r.v[2 * c + 1] = make_uint2(e.z, e.w);
+    }
+  } else {
+    using T = Fmt<F>;
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(sb);
+    r.scale = fminf(compose[sb[4 * F] * 16 + (sb[4 * F + 1 + (gi >> 1)] >> (4 * (gi & 1)) & 0xF)], 448.0f);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int bit = (2 * gi + c) * F;
+      const uint32_t x = __funnelshift_r(words[bit >> 5], words[(bit >> 5) + 1], bit & 31);
+      r.v[2 * c] = reinterpret_cast<const uint2*>(cb)[x & ((1u << T::kW0) - 1u)];
+      r.v[2 * c + 1] = reinterpret_cast<const uint2*>(cb)[T::kEntries + (x >> T::kW0 & ((1u << T::kW1) - 1u))];
+    }
+  }
+  return r;
+}
+GB_DEVINL float dot16(const RowGroup& r, float x) {
+  float s = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const uint32_t w = i & 2 ? r.v[i >> 2].y : r.v[i >> 2].x;
+    s = fmaf(__shfl_sync(0xffffffffu, x, i), i & 1 ? __uint_as_float(w & 0xFFFF0000u) : __uint_as_float(w << 16), s);
+  }
+  return s * r.scale;
 }
 
 template <bool kGrouped, int F>
@@ -545,7 +593,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t lane4 = win | (F == kLit ? (uint32_t)lane * 4u : (uint32_t)(lane & ((int)(T::kStride / 4) - 1)) * 4u);
     if (!kGrouped) build_scale_tab<F>(p, d, scale_tab);
     bool waited = false;
-    float xs0 = 0.0f, xs1 = 0.0f;                            // powers of two of rows lane, lane + 32
+    float xs0 = 0.0f, xs1 = 0.0f;                            // scale words of rows lane, lane + 32
     int item = 0, g0 = 0, n0 = 0;                            // items, units and raw stages so far
     uint32_t flip = 0;
     // An item's accumulators are read out after the warpgroup has decoded its first unit of the NEXT item:
@@ -699,10 +747,53 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 to1 = lane + 32 < rows ? p.row_map[to1] : 0;
               }
             }
+            const int q_pass = out_pass;
             out_t = -1;
             wait(acc_full, (item - 1) & 1, abort_flag, p.status, 49);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool ok = *abort_flag == 0;
+            if (__builtin_expect(__any_sync(0xffffffffu, (__float_as_uint(xs0) | __float_as_uint(xs1)) & kGbLeftOutBits), 0)) {
+              // Groups left out: added to the sums in tensor memory, spread over the warpgroups, which have a
+              // column of the row each (the accumulators of the first units; hi, lo, dlt).
+              const int64_t tile = Q.x_tile + (kGrouped ? q_pass : 0);
+              const uint8_t* w_row = p.qw + (Q.w_row0 + (kGrouped ? row : min(row, (int)p.N - 1 - Q.n0))) * p.row_stride;
+              const uint16_t* cb = reinterpret_cast<const uint16_t*>(p.codebook) + p.role[Q.role].cb;
+              const int parts = wide ? 3 : min(4, units), per = gb_left_out_span(p.n_sb);
+              const uint32_t slot = lane_base + (wide ? (wg == 0 ? 0u : wg == 1 ? 128u : (uint32_t)term_rows(wide, rows))
+                                                      : (uint32_t)((g0 - span + wg) & 3) * acc_stride);
+              const float unit = wide ? (wg == 0 ? 1.0f : wg == 1 ? 0x1p4f : 0x1p7f) : 1.0f;
+#pragma unroll 1
+              for (int m0 = 0; m0 < (wg < parts ? rows : 0); m0 += 4) {
+                uint32_t word[4], bits = 0u, marked = 0u;
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                  word[r] = __float_as_uint(__shfl_sync(0xffffffffu, m0 < 32 ? xs0 : xs1, (m0 + r) & 31));
+                  bits |= word[r] & kGbLeftOutBits;
+                  marked |= (word[r] & kGbLeftOutBits) != 0 ? 1u << r : 0u;
+                }
+                if (bits == 0) continue;
+                float add[4] = {};
+                const int n0 = wide ? m0 : narrow_col(0, m0);
+#pragma unroll 1
+                for (; bits != 0; bits &= bits - 1) {
+                  const int b = __ffs(bits) - 1;
+                  if ((b + (m0 >> 2)) % parts != wg) continue;
+                  gb_left_out(
+                      add, p.tail + (tile * p.pass_rows + m0) * (p.K / 16), p.K / 16, marked, max(b * per, sb_begin) * 16,
+                      min((b + 1) * per, sb_begin + units) * 16,
+                      [&](int r, int g) {
+                        return *reinterpret_cast<const uint2*>(p.xop + (tile * p.n_sb + (g >> 4)) * p.x_unit + sfx + code_at(n0 + r, g & 15));
+                      },
+                      [&](int g) { return row_group<F>(w_row, cb, p.compose, g); }, [](const RowGroup& r, float x) { return dot16(r, x); });
+                }
+#pragma unroll
+                for (int r = 0; r < 4; ++r) add[r] = gb_normalised(add[r], word[r]) * unit;
+                gb_tmem_add(slot + (uint32_t)n0, add);
+              }
+              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+              asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
             const int64_t col = (int64_t)Q.n0 + row;
             const uint32_t Rt = (uint32_t)term_rows(wide, rows);
             float sum[16];
@@ -747,7 +838,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty);
             auto emit = [&](int m, float total) {
-              const float scale = __shfl_sync(0xffffffffu, m < 32 ? xs0 : xs1, m & 31);
+              const float scale = __uint_as_float(__float_as_uint(__shfl_sync(0xffffffffu, m < 32 ? xs0 : xs1, m & 31)) & kGbRowScaleMask);
               const int orow = __shfl_sync(0xffffffffu, m < 32 ? to0 : to1, m & 31);
               if (m >= rows) return;
               const float val = total * scale;
@@ -820,11 +911,13 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 }
 
 // ---- the activations' operand ------------------------------------------------------------------
-struct Group { uint32_t q[2], e[2]; uint32_t hi, lo, dl; };   // codes of q, codes of the correction, three scale bytes
+struct Group { uint32_t q[2], e[2]; uint32_t hi, lo, dl; float tail; };   // codes of q, of the correction, three scale bytes; the scale, if left out
 
-// The three terms of one group of sixteen bf16 values; `shift` = 7 - exponent of the row's largest m1.
+// The three terms of one group of sixteen bf16 values; `shift` normalises the row.
+constexpr int kMinExp = -6, kMaxExp = 7;                   // normalised exponents of m1 whose terms are all exact
 GB_DEVINL Group split_group(const uint32_t (&w)[8], float amax, bool nan, int scale_rule, int shift) {
   Group r;
+  r.tail = 0.0f;
   amax = fmaxf(amax, 1e-8f);
   const float scale = gb_fp4_group_scale(amax, scale_rule);
   if (nan || !(scale < __int_as_float(0x7F800000))) {       // the whole group is NaN (and with it the row's results)
@@ -854,13 +947,16 @@ GB_DEVINL Group split_group(const uint32_t (&w)[8], float amax, bool nan, int sc
   // half-ulps of m1 by which bf16(1.5 s) misses 1.5 m1 (exact in fp32)
   const int n = (int)((m3 - 1.5f * m1) * __uint_as_float((uint32_t)(127 + 8 - e1 > 254 ? 254 : 127 + 8 - e1) << 23));
   // m1 normalised, its upper four significant bits (truncated to UE4M3), the rest times 16
-  const int e = e1 + shift;                                            // <= 7
-  const float V = e >= -40 ? __uint_as_float((__float_as_uint(m1) & 0x007FFFFFu) | ((uint32_t)(127 + e) << 23)) : 0.0f;
-  const uint32_t vb = __float_as_uint(V);
-  r.hi = V >= 0x1p-6f ? (vb >> 20) - (120u << 3) : (uint32_t)(V * 512.0f);
-  r.lo = gb_f32_to_e4m3((V - gb_e4m3_to_f32(r.hi)) * 16.0f);
-  const int de = e + 7;                                                // exponent field of 2^e
-  r.dl = e >= -6 ? (uint32_t)de << 3 : e >= -9 ? 1u << (e + 9) : 0u;
+  const int e = e1 + shift;
+  if (e >= kMinExp && e <= kMaxExp) {
+    const uint32_t vb = (__float_as_uint(m1) & 0x007FFFFFu) | ((uint32_t)(127 + e) << 23);
+    r.hi = (vb >> 20) - (120u << 3);
+    r.lo = gb_f32_to_e4m3((__uint_as_float(vb) - gb_e4m3_to_f32(r.hi)) * 16.0f);
+    r.dl = (uint32_t)(e + 7) << 3;
+  } else {                                                             // left out of the operand
+    r.hi = r.lo = r.dl = 0u;
+    if (((r.q[0] | r.q[1]) & 0x77777777u) != 0) r.tail = scale;
+  }
   const uint32_t an = (uint32_t)(n < 0 ? -n : n), flip = n < 0 ? 0x88888888u : 0u;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -882,7 +978,7 @@ GB_DEVINL void store_group(const Group& G, uint8_t* tile, int64_t unit_stride, b
   uint8_t* codes = unit + sf_bytes(wide);
   const int R = term_rows(wide, rows);
   auto put = [&](int n, uint2 c) {
-    *reinterpret_cast<uint2*>(codes + (n >> 3) * 1024 + (n & 7) * 128 + (((gi >> 1) ^ (n & 7)) << 4) + (gi & 1) * 8) = c;
+    *reinterpret_cast<uint2*>(codes + code_at(n, gi)) = c;
   };
   const uint2 q = make_uint2(G.q[0], G.q[1]), e = make_uint2(G.e[0], G.e[1]);
   if (wide) {
@@ -924,6 +1020,7 @@ struct RowsParams {
   const uint4* x;            // bf16 rows [*, K]
   uint8_t* xop;
   float* x_scale;
+  float* tail;
   uint8_t* sf;               // matrix form (x_unit = 0): the scale-factor plane
   int64_t x_unit;
   int K, n_sb, scale_rule, pass_rows;
@@ -942,6 +1039,22 @@ constexpr int kRowsMaxGroups = 4;
 constexpr int kMaxRowSplit = 8;
 constexpr int kMaxCopies = 32;                             // destinations looked up ahead
 constexpr int kRowSplitGroups = 320;                       // groups of a row per CTA of its cluster
+
+// Exponent of the bf16 group scale of a group whose largest magnitude is amax: -30 .. 125.
+GB_DEVINL int scale_exponent(float amax, int scale_rule) {
+  const float m1 = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_fp4_group_scale(fmaxf(amax, 1e-8f), scale_rule)));
+  return (int)((__float_as_uint(m1) >> 23) & 0xFFu) - 127;
+}
+constexpr uint32_t kZeroCodes = (127u - 32u) << 23;        // 2^-32: below this every code is zero (the scale's floor is 1e-8 / 6)
+
+// A value of this CTA into its slot of every CTA of the cluster.
+GB_DEVINL void to_peers(uint32_t* slots, uint32_t v, int split) {
+  if ((int)threadIdx.x < split) {
+    uint32_t dst;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(gb_smem_u32(&slots[(int)blockIdx.x % split])), "r"(threadIdx.x));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst), "r"(v) : "memory");
+  }
+}
 
 // kMode 0: dense, a cluster of `split` CTAs per row (a single CTA holding 1088 groups of a 17408-wide row took
 // 16 us for 64 rows: 64 SMs, four groups a thread in turn).  1: one CTA per token, its row goes to each of its experts' tiles.
@@ -980,11 +1093,11 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
     }
   }
   const uint4* xr = p.x + (int64_t)j * (kMode == 2 ? 4 : 2) * groups;
-  __shared__ float red[32];
+  __shared__ uint2 red[32];                                // magnitudes order as their bits do
   uint32_t w[kG][8];
   float amax[kG];
   bool nan[kG];
-  float top = 0.0f;
+  uint32_t top = 0u, low = 0x7F800000u;                    // largest and smallest group of the row
 #pragma unroll
   for (int i = 0; i < kG; ++i) {
     const int g = g_first + i * (int)blockDim.x;
@@ -1009,35 +1122,96 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
         w[i][4] = b.x; w[i][5] = b.y; w[i][6] = b.z; w[i][7] = b.w;
       }
       amax[i] = gb_amax_bf16(w[i], &nan[i]);
-      if (amax[i] < __int_as_float(0x7F800000)) top = fmaxf(top, amax[i]);
+      const uint32_t bits = __float_as_uint(amax[i]);
+      if (bits < 0x7F800000u) {
+        top = max(top, bits);
+        if (bits >= kZeroCodes) low = min(low, bits);
+      }
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = top;
+  auto reduce = [&]() {
+    top = __reduce_max_sync(0xffffffffu, top);
+    low = __reduce_min_sync(0xffffffffu, low);
+  };
+  reduce();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_uint2(top, low);
   __syncthreads();
-  top = (int)(threadIdx.x & 31) < (int)(blockDim.x >> 5) ? red[threadIdx.x & 31] : 0.0f;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  if (kMode == 0 && p.split > 1) {                         // the largest of the row's CTAs
-    __shared__ float peers[kMaxRowSplit];
-    if ((int)threadIdx.x < p.split) {
-      uint32_t dst;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                   : "=r"(dst) : "r"(gb_smem_u32(&peers[(int)blockIdx.x % p.split])), "r"(threadIdx.x));
-      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(top) : "memory");
-    }
-    cluster_sync();                                        // the last access to another CTA's memory lies in front of it
-    for (int q = 0; q < p.split; ++q) top = fmaxf(top, peers[q]);
+  if ((int)(threadIdx.x & 31) < (int)(blockDim.x >> 5)) {
+    top = red[threadIdx.x & 31].x;
+    low = red[threadIdx.x & 31].y;
   }
-  const float m1 = gb_bf16_bits_to_f32(gb_f32_to_bf16_bits(gb_fp4_group_scale(fmaxf(top, 1e-8f), p.scale_rule)));
-  const int shift = 7 - ((int)((__float_as_uint(m1) >> 23) & 0xFFu) - 127);
-  const float back = __uint_as_float((uint32_t)(127 - shift) << 23);
-
+  reduce();
+  if (kMode == 0 && p.split > 1) {                         // over the row's CTAs
+    __shared__ uint32_t peer_top[kMaxRowSplit], peer_low[kMaxRowSplit];
+    to_peers(peer_top, top, p.split);
+    to_peers(peer_low, low, p.split);
+    cluster_sync();                                        // the last access to another CTA's memory lies in front of it
+    for (int q = 0; q < p.split; ++q) {
+      top = max(top, peer_top[q]);
+      low = min(low, peer_low[q]);
+    }
+  }
+  int anchor = scale_exponent(__uint_as_float(top), p.scale_rule);   // exponent of m1 that becomes kMaxExp
+  const bool marked = low < 0x7F800000u && anchor - scale_exponent(__uint_as_float(low), p.scale_rule) > kMaxExp - kMinExp;
+  if (__builtin_expect(marked, 0)) {                       // half the range above the mean exponent of the groups with codes
+    __shared__ int sums[2];
+    if (threadIdx.x < 2) sums[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kG; ++i)
+      if (__float_as_uint(amax[i]) >= kZeroCodes && __float_as_uint(amax[i]) < 0x7F800000u) {
+        atomicAdd(&sums[0], scale_exponent(amax[i], p.scale_rule));
+        atomicAdd(&sums[1], 1);
+      }
+    __syncthreads();
+    int sum = sums[0], count = sums[1];
+    if (kMode == 0 && p.split > 1) {
+      __shared__ uint32_t peer_sum[kMaxRowSplit], peer_count[kMaxRowSplit];
+      to_peers(peer_sum, (uint32_t)sum, p.split);
+      to_peers(peer_count, (uint32_t)count, p.split);
+      cluster_sync();
+      sum = count = 0;
+      for (int q = 0; q < p.split; ++q) {
+        sum += (int)peer_sum[q];
+        count += (int)peer_count[q];
+      }
+    }
+    // at most 2^60 below the largest: what is left out is added in the row's normalised units
+    anchor = max(min(anchor, sum / count + (kMaxExp - kMinExp) / 2), anchor - 60);
+  }
   Group grp[kG];
 #pragma unroll
   for (int i = 0; i < kG; ++i)
-    if (g_first + i * (int)blockDim.x < groups) grp[i] = split_group(w[i], amax[i], nan[i], p.scale_rule, shift);
+    if (g_first + i * (int)blockDim.x < groups) grp[i] = split_group(w[i], amax[i], nan[i], p.scale_rule, kMaxExp - anchor);
+  uint32_t left_out = 0u;                                  // one bit for each sixteenth of the row
+  if (__builtin_expect(marked, 0)) {
+    __shared__ uint32_t all;
+    if (threadIdx.x == 0) all = 0u;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kG; ++i) {
+      const int g = g_first + i * (int)blockDim.x;
+      if (g < groups && grp[i].tail != 0.0f) atomicOr(&all, 1u << ((g >> 4) / gb_left_out_span(p.n_sb)));
+    }
+    __syncthreads();
+    left_out = all;
+    if (kMode == 0 && p.split > 1) {
+      __shared__ uint32_t peer_all[kMaxRowSplit];
+      to_peers(peer_all, left_out, p.split);
+      cluster_sync();
+      for (int q = 0; q < p.split; ++q) left_out |= peer_all[q];
+    }
+    for (int s = 0; s < copies; ++s) {
+      int tile = 0, m = j, rows = 0;
+      if (kMode != 0) place(s, tile, m, rows);
+#pragma unroll
+      for (int i = 0; i < kG; ++i) {
+        const int g = g_first + i * (int)blockDim.x;
+        if (tile >= 0 && g < groups) p.tail[((int64_t)tile * p.pass_rows + m) * groups + g] = grp[i].tail;
+      }
+    }
+  }
+  const float back = __uint_as_float(((uint32_t)(127 - kMaxExp + anchor) << 23) | left_out);
 
   for (int s = 0; s < copies; ++s) {
     int tile = 0, m = j, rows = p.rows;
@@ -1241,10 +1415,10 @@ bool gb_gemv_fp4_applies(const gb_weight* w, bool scales_e4m3) {
   return fp4_format(w, scales_e4m3) >= 0 && w->rows >= 64 && w->K / 16 <= 1024 * kRowsMaxGroups;
 }
 
-// The operand of up to 64 rows and the rows' scales.
+// The operand of up to 64 rows, the rows' scales, the scales of groups left out.
 int64_t gb_gemv_fp4_workspace_bytes(int64_t M, int64_t K) {
   const int rows = (int)(M > kMaxRows ? kMaxRows : M);
-  return align256((K / 256) * unit_bytes(is_wide(rows), rows)) + align256(rows * 4);
+  return align256((K / 256) * unit_bytes(is_wide(rows), rows)) + align256(rows * 4) + align256(rows * (K / 16) * 4);
 }
 
 int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, int n_roles, const int64_t* role_rows,
@@ -1270,6 +1444,9 @@ int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, 
     p.x_unit = unit_bytes(is_wide(p.M), p.M);
     p.xop = (const uint8_t*)workspace;
     p.x_scale = (const float*)((const uint8_t*)workspace + align256(p.n_sb * p.x_unit));
+    p.tail = (const float*)((const uint8_t*)p.x_scale + align256(p.M * 4));
+    p.qw = w->qw;
+    p.row_stride = w->row_stride;
     p.codebook = w->codebook;
     p.compose = w->compose;
     p.global_scale = w->global_scale == 0.0f ? 1.0f : w->global_scale;
@@ -1296,7 +1473,8 @@ int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, 
     RowsParams rp = {};
     rp.x = (const uint4*)((const uint16_t*)x + m0 * w->K);
     rp.xop = (uint8_t*)workspace;
-    rp.x_scale = (float*)((uint8_t*)workspace + align256(p.n_sb * p.x_unit));
+    rp.x_scale = const_cast<float*>(p.x_scale);
+    rp.tail = const_cast<float*>(p.tail);
     rp.x_unit = p.x_unit;
     rp.K = (int)w->K; rp.n_sb = p.n_sb; rp.scale_rule = scale_rule; rp.pass_rows = p.pass_rows; rp.rows = p.M;
     rc = launch_rows<0>(p.M, w->K, stream, rp);
@@ -1390,7 +1568,8 @@ int64_t gb_moe_fp4_operand_bytes(int64_t P, int64_t E, int64_t K, int pass_rows)
   if (pass_rows == 0) return gb_fp4_tiles(P, E, K).bytes;
   if (pass_rows < 1) return 0;
   const int64_t tiles = P / pass_rows + E + 1;
-  return align256(tiles * (K / 256) * unit_bytes(is_wide(pass_rows), pass_rows)) + align256(tiles * pass_rows * 4);
+  return align256(tiles * (K / 256) * unit_bytes(is_wide(pass_rows), pass_rows)) + align256(tiles * pass_rows * 4) +
+         align256(tiles * pass_rows * (K / 16) * 4);
 }
 
 static int rows_params(RowsParams* p, const void* x, int64_t P, int64_t E, int64_t K, int pass_rows, const int32_t* ids,
@@ -1405,11 +1584,13 @@ static int rows_params(RowsParams* p, const void* x, int64_t P, int64_t E, int64
     const GbFp4Tiles op = gb_fp4_tiles(P, E, K);
     p->sf = (uint8_t*)operand + op.sf_at;
     p->x_scale = (float*)((uint8_t*)operand + op.scale_at);
+    p->tail = (float*)((uint8_t*)operand + op.tail_at);
     pass_rows = 64;
   } else {
     const int64_t tiles = P / pass_rows + E + 1;
     p->x_unit = unit_bytes(is_wide(pass_rows), pass_rows);
     p->x_scale = (float*)((uint8_t*)operand + align256(tiles * (K / 256) * p->x_unit));
+    p->tail = (float*)((uint8_t*)p->x_scale + align256(tiles * pass_rows * 4));
   }
   p->K = (int)K; p->n_sb = (int)(K / 256); p->scale_rule = scale_rule; p->pass_rows = pass_rows;
   p->ids = ids; p->seg = seg; p->E = (int)E;
@@ -1455,6 +1636,9 @@ int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, in
   p.x_unit = unit_bytes(is_wide(pass_rows), pass_rows);
   p.xop = (const uint8_t*)operand;
   p.x_scale = (const float*)((const uint8_t*)operand + align256(tiles * p.n_sb * p.x_unit));
+  p.tail = (const float*)((const uint8_t*)p.x_scale + align256(tiles * pass_rows * 4));
+  p.qw = w->qw;
+  p.row_stride = w->row_stride;
   p.codebook = w->codebook; p.compose = w->compose;
   p.global_scale = w->global_scale == 0.0f ? 1.0f : w->global_scale;
   p.y = (uint16_t*)y;

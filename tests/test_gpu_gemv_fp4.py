@@ -180,3 +180,104 @@ def test_several_tiles_per_cta_with_an_odd_number_of_superblocks(dev, name, T):
     ref = moe(*args).float()
     assert "grouped prefill" in moe._cb_route
     assert float((got[0] - ref).norm() / ref.norm()) <= 3e-3
+
+
+def _zero_first_group(fmt, qw, cb):
+    """Entry 0 of every (sub-)table becomes the zero codeword; returns a function that points the first
+    group of the given packed rows at it."""
+    pos = 0
+    for _ in range(cb.size // fmt.codebook_elems()):
+        for r, dim in fmt.table_shapes():
+            cb[pos:pos + dim] = 0.0
+            pos += r * dim
+
+    def clear(rows):
+        rows[..., :2 if fmt.mode == "full" else fmt.k // 4] = 0
+    return clear
+
+
+def _outlier_rows(M, K, seed):
+    """Every third row: a first group 2^14 and more above all the others, which span 2^20 themselves;
+    the next: groups anywhere within 2^30; the third kind is ordinary."""
+    rng = np.random.default_rng(seed)
+    x = rng.standard_normal((M, K // 16, 16)).astype(np.float32)
+    x[0::3] *= np.exp2(rng.integers(-28, -8, x[0::3].shape[:2] + (1,))).astype(np.float32)
+    x[0::3, 0] = rng.standard_normal(x[0::3, 0].shape) * 128.0
+    x[1::3] *= np.exp2(rng.integers(-25, 6, x[1::3].shape[:2] + (1,))).astype(np.float32)
+    return O.bf16_round(x.reshape(M, K))
+
+
+@pytest.mark.parametrize("name", ["lit", "k12", "k16", "k20", "k24"])
+@pytest.mark.parametrize("M,N,K", [(2, 64, 256), (7, 384, 1280), (16, 200, 5120), (3, 136, 17408), (20, 129, 768), (64, 320, 1536),
+                                   (70, 128, 1024)])
+def test_groups_far_below_the_rows_largest_keep_their_precision(dev, name, M, N, K):
+    """Half of the weight rows are zero under the outlier, so that their result is the small groups' alone;
+    every row is held to the oracle by its own magnitude."""
+    from gridbook_b200 import _native, kernels, synth
+    fmt = _fmt(name)
+    d = synth.make_linear(fmt, N, K, seed=M + K, global_scale=1.0 / 448.0 if name == "lit" else None)
+    _zero_first_group(fmt, d["qw"], d["cb"])(d["qw"][::2])
+    lin = _linear(fmt, d, [N], dev)
+    if M > kernels.row_batch_max_rows(lin._cb_weight):
+        pytest.skip("past the decode batches of this format")
+    x = _outlier_rows(M, K, M)
+    y = f32_of(lin(synth.bf16_tensor(x, dev)))
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    ref = oracle_linear(x, d)
+    for part in (slice(0, None, 2), slice(1, None, 2)):      # weight rows without and with the outlier
+        for m in range(M):
+            top = np.abs(ref[m, part]).max()
+            assert_close_bf16(y[m, part] / top, ref[m, part] / top, f"{name} {M}x{N}x{K} row {m}", atol_rel=1e-6)
+
+
+def test_left_out_groups_under_codebooks_per_role(dev):
+    """The rows of a tile are multiplied by their own role's codebook, also where the CTA has moved on to the next."""
+    from gridbook_b200 import _native, synth
+    fmt, M, K, parts = _fmt("k16"), 6, 512, [12800, 12800]
+    N = sum(parts)
+    d = synth.make_linear(fmt, N, K, seed=3, n_books=2)
+    d["cb_row_offset"] = np.repeat(np.arange(2), parts).astype(np.int32) * fmt.codebook_elems()
+    _zero_first_group(fmt, d["qw"], d["cb"])(d["qw"])
+    x = _outlier_rows(M, K, 1)
+    y = f32_of(_linear(fmt, d, parts, dev)(synth.bf16_tensor(x, dev)))
+    assert _native.device_status(0) == 0
+    ref = oracle_linear(x, d)
+    for m in range(M):
+        top = np.abs(ref[m]).max()
+        assert_close_bf16(y[m] / top, ref[m] / top, f"row {m}", atol_rel=1e-6)
+
+
+@pytest.mark.parametrize("f13,f2", [("lit", "lit"), ("k16", "k16"), ("k20", "lit"), ("lit", "k24")])
+@pytest.mark.parametrize("T", [6, 50, 150, 700])
+def test_left_out_groups_of_a_routed_layer(dev, f13, f2, T):
+    """Outliers in front of both projections whose weights are zero under them (but for the sixteen features
+    that carry the outlier into the second): few rows a pass, more, and the stack decoded once."""
+    from gridbook_b200 import _native, synth
+    from gridbook_b200.moe import CBMoE
+    fmt13, fmt2 = _fmt(f13), _fmt(f2)
+    E, hidden, inter, topk = 8, 512, 768, 2
+    w13d, w2d = synth.make_moe(fmt13, fmt2, E, hidden, inter, seed=T)
+    clear13, clear2 = _zero_first_group(fmt13, w13d["qw"], w13d["cb"]), _zero_first_group(fmt2, w2d["qw"], w2d["cb"])
+    w13 = w13d["qw"].reshape(E, 2 * inter, -1)
+    clear13(w13[:, 16:inter])
+    clear13(w13[:, inter + 16:])
+    clear2(w2d["qw"].reshape(E, hidden, -1))
+    ids, tw = synth.make_routing(T, E, topk, seed=T)
+    rng = np.random.default_rng(T)
+    x = rng.standard_normal((T, hidden)).astype(np.float32)
+    x[:, 16:] *= np.float32(2.0 ** -5)
+    x[:, :16] *= np.float32(2.0 ** 11)
+    x = O.bf16_round(x)
+    ref = O.moe_loop_chain(x, ids, tw, w13d, w2d, E=E, hidden=hidden, inter=inter, fmt13=oracle_kwargs(fmt13),
+                           fmt2=oracle_kwargs(fmt2), scale_rule="recip")
+    moe = CBMoE(fmt13, fmt2, E, hidden, inter, _tables(fmt13, w13d["cb"]), _tables(fmt2, w2d["cb"]))
+    moe.load(torch.from_numpy(w13d["qw"]), torch.from_numpy(w2d["qw"]), None, None, dev)
+    moe.method.sorted_min_pairs_per_expert = 0
+    moe.method.sorted_min_pairs_other = 0
+    got = f32_of(moe(synth.bf16_tensor(x, dev), torch.from_numpy(tw).to(dev), torch.from_numpy(ids).to(dev)))
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    assert "sorted rows" in moe._cb_route
+    err = np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert err.max() <= 1e-2                                 # one step of the second bucket in a few values, as in the test above
