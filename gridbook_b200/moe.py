@@ -15,8 +15,8 @@ from .formats import CBFormat
 
 # Route thresholds, in routed pairs (per expert where it says so).  They are crossovers measured on
 # one B200 with 128 experts, hidden 2048, intermediate 768 (literal fp4 format); every method
-# instance carries its own copy (attributes of the same lower-case names) that a caller may set
-# for another shape.
+# instance has attributes of the same lower-case names that a caller may set for another shape.  What
+# a caller has set is taken as it is, also where it equals a default; None restores the default.
 PAIR_KERNEL_MAX_PAIRS = 768       # routed pairs up to which every pair runs as its own table GEMV
 FUSED_BUCKET_MAX_PAIRS = 32       # routed pairs up to which the grouped kernel buckets its own rows
 # From this many routed pairs per expert (on average) the routed layer decodes each stack once
@@ -83,10 +83,30 @@ def unfilled_cb_params(layer) -> list[str]:
     return missing
 
 
+def _threshold(name: str, default: int) -> property:
+    """A route threshold of a method: the caller's value once there is one, else the default."""
+
+    def read(method):
+        return method._limit(name, default)
+
+    def write(method, value):
+        method.__dict__["_set_" + name] = value
+
+    return property(read, write)
+
+
 class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
     """CB decode for routed experts.  ``scheme`` is the gate_up format; ``scheme_down``
     (optional, not expressible in the reference: gridbook/config.py:1631-1640) gives the
     down projection its own format."""
+
+    sorted_min_pairs_per_expert = _threshold("sorted_min_pairs_per_expert", SORTED_MIN_PAIRS_PER_EXPERT)
+    prefill_min_pairs_per_expert = _threshold("prefill_min_pairs_per_expert", PREFILL_MIN_PAIRS_PER_EXPERT)
+
+    def _limit(self, name: str, default: int) -> int:
+        """The threshold a caller has set, else ``default`` (some stacks have one of their own)."""
+        value = self.__dict__.get("_set_" + name)
+        return default if value is None else value
 
     def __init__(self, quant_config, moe, scheme: dict, prefix: str, scheme_down: dict | None = None) -> None:
         super().__init__(moe)
@@ -105,11 +125,11 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
             "w2": codec.static_activation_contract(self.scheme_down, f"{prefix}.w2")}
         self.k, self.n_sub, self.type_size = self.fmt13.k, self.fmt13.n_sub, self.fmt13.type_size
         self.pair_kernel_max_pairs = PAIR_KERNEL_MAX_PAIRS
-        self.sorted_min_pairs_per_expert = SORTED_MIN_PAIRS_PER_EXPERT
+        self.sorted_min_pairs_per_expert = None
         self.sorted_min_pairs_other = SORTED_MIN_PAIRS_OTHER
         self.prefill_min_pairs_other = PREFILL_MIN_PAIRS_OTHER
         self.pad_two_tier_superblocks = True   # fp4 k = 16 two-tier stacks: 73-byte superblocks in 80-byte slots
-        self.prefill_min_pairs_per_expert = PREFILL_MIN_PAIRS_PER_EXPERT
+        self.prefill_min_pairs_per_expert = None
 
     # ------------------------------------------------------------------ parameters
     def create_weights(self, layer, num_experts: int, hidden_size: int,
@@ -285,9 +305,10 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
             kernels.host_weight(w13), kernels.host_weight(w2), kernels.host_weight(kernels.stack_rows(w13)),
             kernels.host_weight(kernels.stack_rows(w2)), layer._cb_E, layer._cb_hidden, layer._cb_inter,
             kernels.moe_gemv_sorted_applies(w13), sorted2, pair_ok)
-        if layer._cb_plan.fp4 and self.prefill_min_pairs_per_expert == PREFILL_MIN_PAIRS_PER_EXPERT:
-            self.prefill_min_pairs_per_expert = PREFILL_MIN_PAIRS_FP4
-        layer._cb_sorted_early = layer._cb_plan.fp4 and layer._cb_E >= SORTED_FP4_EXPERTS
+        # defaults of this stack for the thresholds that no caller has set
+        fp4 = layer._cb_plan.fp4
+        layer._cb_sorted_min = SORTED_MIN_PAIRS_FP4 if fp4 and layer._cb_E >= SORTED_FP4_EXPERTS else SORTED_MIN_PAIRS_PER_EXPERT
+        layer._cb_prefill_min = PREFILL_MIN_PAIRS_FP4 if fp4 else PREFILL_MIN_PAIRS_PER_EXPERT
         layer._cb_layer_id = ops.register_cb_layer(self, layer)
         print(f"[prismaquant-cb] {self.prefix}: decode=grouped-cuda (sm_100a) "
               f"w13={self.fmt13.grid}/k{self.fmt13.k} w2={self.fmt2.grid}/k{self.fmt2.k}",
@@ -329,12 +350,10 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
         number of routed pairs and this method's thresholds (MoEPlan in csrc/gb_torch.cpp).  No host
         read, so every size can be captured."""
         plan = layer._cb_plan
-        sorted_min = self.sorted_min_pairs_per_expert
-        if sorted_min == SORTED_MIN_PAIRS_PER_EXPERT and layer._cb_sorted_early:
-            sorted_min = SORTED_MIN_PAIRS_FP4
         out = plan(x, topk_weights, topk_ids, kernels.rule_code(ops.ACT_SCALE_RULE),
-                   (self.pair_kernel_max_pairs, sorted_min, self.sorted_min_pairs_other,
-                    self.prefill_min_pairs_per_expert, self.prefill_min_pairs_other, FUSED_BUCKET_MAX_PAIRS))
+                   (self.pair_kernel_max_pairs, self._limit("sorted_min_pairs_per_expert", layer._cb_sorted_min),
+                    self.sorted_min_pairs_other, self._limit("prefill_min_pairs_per_expert", layer._cb_prefill_min),
+                    self.prefill_min_pairs_other, FUSED_BUCKET_MAX_PAIRS))
         layer.__dict__["_cb_route"] = _ROUTES[plan.route]
         return out
 

@@ -835,3 +835,36 @@ def test_linear_plan_refuses_rows_of_another_width_before_anything_else():
     for shape in [(4, K), (K,), (0, K), (2, 0, 3)]:          # a shape that fits (or an empty batch) is refused only for the device
         with pytest.raises(RuntimeError, match="CUDA tensors only"):
             plan(torch.empty(shape, dtype=torch.bfloat16), 0, True, 128)
+
+
+@pytest.mark.parametrize("name,position,other", [("sorted_min_pairs_per_expert", 1, 3), ("prefill_min_pairs_per_expert", 3, 1 << 30)])
+def test_a_threshold_set_to_a_default_by_the_caller_is_taken_as_set(name, position, other):
+    """Some stacks have a default of their own; it gives way to any value that the caller has set, the
+    general default among them."""
+    from types import SimpleNamespace
+    from gridbook_b200 import formats as F, moe
+    from gridbook_b200.linear import _scheme_of
+    method = moe.PrismaQuantCBMoEMethod(None, None, _scheme_of(F.NVFP4_LITERAL), "m")
+    seen = []
+
+    class Plan:
+        route = 2
+
+        def __call__(self, x, weights, ids, rule, limits):
+            seen.append(limits)
+            return x
+
+    layer = SimpleNamespace(_cb_plan=Plan(), _cb_sorted_min=3, _cb_prefill_min=1 << 30)
+
+    def limit():
+        method._apply_inline(layer, 0, 0, 0)
+        return seen[-1][position]
+
+    default = getattr(method, name)
+    assert default == getattr(moe, name.upper()) and limit() == other
+    setattr(method, name, default)
+    assert getattr(method, name) == default and limit() == default
+    setattr(method, name, 7)
+    assert getattr(method, name) == 7 and limit() == 7
+    setattr(method, name, None)
+    assert getattr(method, name) == default and limit() == other
