@@ -211,8 +211,10 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
   int64_t row_batch_max = 16;
   gb_hints hints{};
   std::atomic<int> prefill_route{kRouteNone};
+  const int64_t serial = next_serial++;            // never given twice, as an address is
   std::mutex mutex;
-  std::map<std::vector<const LinearPlan*>, at::Tensor> shared_slots;
+  std::map<std::vector<int64_t>, at::Tensor> shared_slots;   // by the serials of the plans that share a row
+  static std::atomic<int64_t> next_serial;
 
   // `role_rows`: row counts of the parts with a codebook of their own (empty: one codebook)
   LinearPlan(Weight weight, at::Tensor ws, const Opt& armed, const std::vector<int64_t>& role_rows)
@@ -300,6 +302,8 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
   }
 };
 
+std::atomic<int64_t> LinearPlan::next_serial{0};
+
 // Several linears that read the same activation row, one launch; None when they have no such kernel.
 py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, const at::Tensor& x, int rule) {
   const size_t n = plans.size();
@@ -312,10 +316,10 @@ py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, con
   const c10::cuda::CUDAGuard guard(x.device());
   const gb_weight* ws[4];
   void* ys[4];
-  std::vector<const LinearPlan*> key;
+  std::vector<int64_t> key;
   for (size_t i = 0; i < n; ++i) {
     ws[i] = &plans[i]->w.w;
-    key.push_back(plans[i].get());
+    key.push_back(plans[i]->serial);
   }
   at::Tensor slots;
   {
@@ -586,6 +590,7 @@ PYBIND11_MODULE(_gb_torch, m) {
   py::class_<LinearPlan, std::shared_ptr<LinearPlan>>(m, "LinearPlan")
       .def(py::init<Weight, at::Tensor, const Opt&, const std::vector<int64_t>&>())
       .def("__call__", &LinearPlan::forward, py::call_guard<py::gil_scoped_release>())
+      .def_property_readonly("serial", [](const LinearPlan& p) { return p.serial; })
       .def_property_readonly("prefill_route", [](const LinearPlan& p) { return p.prefill_route.load(); });
   py::class_<MoEPlan, std::shared_ptr<MoEPlan>>(m, "MoEPlan")
       .def(py::init<Weight, Weight, Weight, Weight, int64_t, int64_t, int64_t, bool, bool, bool>())

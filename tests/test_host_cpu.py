@@ -868,3 +868,15 @@ def test_a_threshold_set_to_a_default_by_the_caller_is_taken_as_set(name, positi
     assert getattr(method, name) == 7 and limit() == 7
     setattr(method, name, None)
     assert getattr(method, name) == default and limit() == other
+
+
+def test_plans_are_told_apart_by_a_number_that_is_never_given_twice():
+    """What one plan keeps for a set of plans is found by their numbers: an address may come back."""
+    from gridbook_b200 import _native, formats as F, kernels
+    w = kernels.host_weight(_cpu_weight(F.NVFP4_LITERAL))
+    seen = []
+    for _ in range(8):
+        plan = _native.host().LinearPlan(w, torch.empty(16, dtype=torch.uint8), None, [])
+        seen.append(plan.serial)
+        del plan
+    assert len(set(seen)) == 8
