@@ -11,6 +11,8 @@
 // The library is reached through dlsym on the path the ctypes loader uses, so that both bind the
 // same file and a missing symbol fails closed.
 #include <ATen/ATen.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/utils/pybind.h>
@@ -193,6 +195,23 @@ void need_bf16(const at::Tensor& t, const char* what) {
   if (t.scalar_type() != at::kBFloat16) throw py::type_error(std::string(what) + " takes bf16 activations");
 }
 
+bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
+
+// A tensor that later calls read too, and the kernels that filled it.  Not made under capture: they would be
+// recorded instead of run, and a call outside the graph would find the tensor unfilled.
+struct Kept {
+  at::Tensor t;
+  c10::cuda::CUDAStream stream;
+  at::cuda::CUDAEvent filled;
+  explicit Kept(at::Tensor tensor) : t(std::move(tensor)), stream(c10::cuda::getCurrentCUDAStream()) { filled.record(stream); }
+  // for the current stream; what a capture starts from has run
+  const at::Tensor& ready() {
+    const auto now = c10::cuda::getCurrentCUDAStream();
+    if (now != stream && !capturing()) filled.block(now);
+    return t;
+  }
+};
+
 constexpr int64_t kDecodeMaxRows = 16;
 // Routed rows per expert from which a stack is decoded once into its NVFP4 view and multiplied by the grouped GEMM,
 // instead of decoded in every pass of up to 64 rows.  128 experts, hidden 2048, intermediate 768: literal 299 against
@@ -213,7 +232,7 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
   std::atomic<int> prefill_route{kRouteNone};
   const int64_t serial = next_serial++;            // never given twice, as an address is
   std::mutex mutex;
-  std::map<std::vector<int64_t>, at::Tensor> shared_slots;   // by the serials of the plans that share a row
+  std::map<std::vector<int64_t>, Kept> shared_slots;   // by the serials of the plans that share a row
   static std::atomic<int64_t> next_serial;
 
   // `role_rows`: row counts of the parts with a codebook of their own (empty: one codebook)
@@ -324,9 +343,14 @@ py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, con
   at::Tensor slots;
   {
     std::lock_guard<std::mutex> lock(plans[0]->mutex);
-    at::Tensor& s = plans[0]->shared_slots[key];
-    if (!s.defined()) s = at::full({L.gb_gemv_tab_slots_bytes(ws, (int)n)}, 0xFF, x.options().dtype(at::kByte));
-    slots = s;
+    auto& kept = plans[0]->shared_slots;
+    auto it = kept.find(key);
+    if (it == kept.end()) {
+      slots = at::full({L.gb_gemv_tab_slots_bytes(ws, (int)n)}, 0xFF, x.options().dtype(at::kByte));
+      if (!capturing()) kept.emplace(key, Kept(slots));    // else the graph arms its own
+    } else {
+      slots = it->second.ready();
+    }
   }
   const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
   std::vector<at::Tensor> outs;
@@ -350,7 +374,7 @@ struct MoEPlan {
   bool sorted13, sorted2, pair_ok;   // per projection: a kernel that takes rows in expert order
   std::atomic<int> route{kRouteNone};
   std::mutex mutex;
-  std::map<std::pair<int64_t, int64_t>, at::Tensor> x_rows;
+  std::map<int64_t, std::vector<Kept>> x_rows;   // per top-k, each at least twice the last: a batch reads the front of one
 
   MoEPlan(Weight a, Weight b, Weight ra, Weight rb, int64_t E_, int64_t hidden_, int64_t inter_, bool sorted_13, bool sorted_2, bool pair_)
       : w13(std::move(a)), w2(std::move(b)), rows13(std::move(ra)), rows2(std::move(rb)), E(E_), hidden(hidden_),
@@ -362,13 +386,16 @@ struct MoEPlan {
     return L.gb_moe_fp4_pass_rows(&w13.w, w13.scales_e4m3, 1, E) > 0 && L.gb_moe_fp4_pass_rows(&w2.w, w2.scales_e4m3, 1, E) > 0;
   }
 
-  // token of every routed pair, one tensor per batch shape
-  const int32_t* x_row(int64_t T, int64_t topk, const at::Tensor& like) {
+  // Token of every routed pair.  Earlier, shorter tensors stay: a captured graph may read them.
+  at::Tensor x_row(int64_t T, int64_t topk, const at::Tensor& like) {
+    auto make = [&](int64_t pairs) { return at::arange(pairs, like.options().dtype(at::kInt)).floor_divide(topk).to(at::kInt).contiguous(); };
     std::lock_guard<std::mutex> lock(mutex);
-    at::Tensor& t = x_rows[{T, topk}];
-    if (!t.defined())
-      t = at::arange(T * topk, like.options().dtype(at::kInt)).floor_divide(topk).to(at::kInt).contiguous();
-    return t.data_ptr<int32_t>();
+    std::vector<Kept>& kept = x_rows[topk];
+    for (Kept& k : kept)
+      if (k.t.numel() >= T * topk) return k.ready();
+    if (capturing()) return make(T * topk);
+    kept.emplace_back(make(std::max(T * topk, kept.empty() ? 64 * topk : 2 * kept.back().t.numel())));
+    return kept.back().t;
   }
 
   struct Limits { int64_t pair_max, sorted_per_expert, sorted_other, prefill_per_expert, prefill_other, fused_bucket_max; };
@@ -391,6 +418,7 @@ struct MoEPlan {
     c.T = T; c.topk = topk; c.P = T * topk; c.rule = rule;
     c.stream = c10::cuda::getCurrentCUDAStream().stream();
     c.out = at::empty({T, hidden}, c.x.options());
+    c.plan = this;
     const bool sorted_ok = sorted13 && sorted2;
     const int64_t prefill_min = sorted_ok ? lim.prefill_per_expert : std::min(lim.prefill_per_expert, lim.prefill_other);
     if (c.P >= prefill_min * E) prefill(c);
@@ -403,7 +431,12 @@ struct MoEPlan {
 
  private:
   struct Call {
-    at::Tensor x, ids, tw, out;
+    at::Tensor x, ids, tw, out, tokens;
+    MoEPlan* plan;
+    const int32_t* x_row() {
+      if (!tokens.defined()) tokens = plan->x_row(T, topk, x);
+      return tokens.data_ptr<int32_t>();
+    }
     int64_t T, topk, P;
     int rule;
     void* stream;
@@ -444,7 +477,7 @@ struct MoEPlan {
     const int64_t need = L.gb_moe_mlp_pairs_workspace_bytes(c.P, w13.w.K, w2.w.K);
     const int y = a.add(c.P * hidden * 2), ws = a.add(need);
     a.alloc(c.x);
-    const int rc = L.gb_moe_mlp_pairs(c.x.data_ptr(), x_row(c.T, c.topk, c.x), &w13.w, w13.expert_stride, &w2.w,
+    const int rc = L.gb_moe_mlp_pairs(c.x.data_ptr(), c.x_row(), &w13.w, w13.expert_stride, &w2.w,
                                       w2.expert_stride, E, 0, c.ids.data_ptr<int32_t>(), c.P, 0, GB_ACT_FP4_GROUP16, c.rule,
                                       a.ptr(y), nullptr, a.ptr(ws), std::max<int64_t>(need, 16), c.stream);
     if (rc == GB_EUNSUPPORTED) return false;
@@ -472,7 +505,7 @@ struct MoEPlan {
       bucket(w13, in, a.ptr(xq), c.T, c);
       in = a.ptr(xq);
     }
-    check(L.gb_moe_gemv(in, x_row(c.T, c.topk, c.x), &w13.w, w13.expert_stride, E, off, ord, c.P, 1,
+    check(L.gb_moe_gemv(in, c.x_row(), &w13.w, w13.expert_stride, E, off, ord, c.P, 1,
                         fuse13 ? GB_ACT_FP4_GROUP16 : GB_ACT_NONE, c.rule, a.ptr(h), nullptr, nullptr, 0, c.stream));
     in = a.ptr(h);
     if (!fuse2) {
@@ -534,7 +567,7 @@ struct MoEPlan {
       multiply(w13, rows13, once13, pr13, xs, nullptr, a.ptr(h13));
     } else {
       bucket(w13, c.x.data_ptr(), a.ptr(xq), c.T, c);
-      check(L.gb_moe_gather_rows(a.ptr(xq), x_row(c.T, c.topk, c.x), ord, off, E, c.P, hidden, a.ptr(xs), c.stream));
+      check(L.gb_moe_gather_rows(a.ptr(xq), c.x_row(), ord, off, E, c.P, hidden, a.ptr(xs), c.stream));
       check(L.gb_moe_gemv_sorted(a.ptr(xs), &w13.w, w13.expert_stride, E, off, nullptr, c.P, a.ptr(h13), nullptr, c.stream));
     }
     if (fp2) {
@@ -572,7 +605,7 @@ struct MoEPlan {
                                  one.w.global_scale, c.stream));
     };
     bucket(w13, c.x.data_ptr(), a.ptr(xq), c.T, c);
-    check(L.gb_moe_gather_rows(a.ptr(xq), x_row(c.T, c.topk, c.x), ord, off, E, c.P, hidden, a.ptr(xs), c.stream));
+    check(L.gb_moe_gather_rows(a.ptr(xq), c.x_row(), ord, off, E, c.P, hidden, a.ptr(xs), c.stream));
     stage(rows13, w13, a.ptr(xs), a.ptr(h13), nullptr);
     swiglu(a, c, r, h13, hs, h);
     stage(rows2, w2, a.ptr(h), a.ptr(y), ord);             // rows back in pair order

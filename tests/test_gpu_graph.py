@@ -66,3 +66,50 @@ def test_block_capture_equals_eager(block, T):
         torch.cuda.synchronize()
         assert torch.equal(out, want) and torch.equal(kv, want_kv), (T, seed)
     assert _native.device_status(0) == 0
+
+
+def test_first_call_of_a_shape_under_capture(block):
+    """Nothing that a capture made is taken by a later call outside the graph: it was recorded, not run."""
+    from gridbook_b200 import _native, synth
+    dev, lins, moe, hidden, inter, E, _ = block
+    from gridbook_b200.linear import apply_shared_row
+    T, topk = 6, 3                                       # a top-k that no other test uses
+    ids, tw = synth.make_routing(T, E, topk, seed=T)
+    x = synth.bf16_tensor(synth.make_activations(T, hidden, seed=T), dev)
+    tw_d, ids_d = torch.from_numpy(tw).to(dev), torch.from_numpy(ids).to(dev)
+    pair = [lins["kv"], lins["q"]]                       # an order that no other test uses
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = moe(x, tw_d, ids_d)
+        rows = apply_shared_row(pair, x[:1])
+    want, want_rows = moe(x, tw_d, ids_d), apply_shared_row(pair, x[:1])     # before any replay
+    one_by_one = torch.cat([moe(x[t:t + 1], tw_d[t:t + 1], ids_d[t:t + 1]) for t in range(T)])
+    torch.cuda.synchronize()
+    assert torch.equal(want, one_by_one)
+    assert all(torch.equal(a, lin(x[:1])) for a, lin in zip(want_rows, pair))
+    for _ in range(2):
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and all(torch.equal(a, b) for a, b in zip(rows, want_rows))
+    assert _native.device_status(0) == 0
+
+
+def test_batch_sizes_share_what_a_plan_keeps(block):
+    """Every batch size reads the front of one list of tokens, on whichever stream it runs."""
+    from gridbook_b200 import synth
+    dev, _, moe, hidden, inter, E, _ = block
+    topk, x = 2, synth.bf16_tensor(synth.make_activations(200, hidden, seed=9), dev)
+    ids, tw = synth.make_routing(200, E, topk, seed=9)
+    tw_d, ids_d = torch.from_numpy(tw).to(dev), torch.from_numpy(ids).to(dev)
+    moe(x[:8], tw_d[:8], ids_d[:8])
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for T in range(1, 200):
+        moe(x[:T], tw_d[:T], ids_d[:T])
+        with torch.cuda.stream(side):
+            moe(x[:T], tw_d[:T], ids_d[:T])
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() - before <= 16 << 10   # lists of 256 and 512 pairs; one each would be 200 KB
