@@ -402,14 +402,18 @@ struct MoEPlan {
 
   at::Tensor forward(const at::Tensor& x, const at::Tensor& topk_weights, const at::Tensor& topk_ids, int rule,
                      std::array<int64_t, 6> limits) {
+    const Limits lim{limits[0], limits[1], limits[2], limits[3], limits[4], limits[5]};
+    // the kernels take their extents from the ids: everything else has to fit them
+    if (topk_ids.dim() != 2) throw std::runtime_error("routed layer: expert ids of shape [tokens, top-k] expected");
+    const int64_t T = topk_ids.size(0), topk = topk_ids.size(1);
+    if (T > 0 && x.numel() != T * hidden) throw std::runtime_error("routed layer: " + std::to_string(T) + " tokens of " +
+                                                                   std::to_string(hidden) + " values expected");
+    if (topk_weights.numel() != T * topk) throw std::runtime_error("routed layer: " + std::to_string(T) + " x " + std::to_string(topk) +
+                                                                   " router weights expected");
     need_cuda(x);
     need_cuda(topk_ids);
     need_cuda(topk_weights);
-    const Limits lim{limits[0], limits[1], limits[2], limits[3], limits[4], limits[5]};
-    const int64_t T = topk_ids.size(0), topk = topk_ids.size(1);
     if (T == 0) return at::empty_like(x);
-    if (x.numel() != T * hidden) throw std::runtime_error("routed layer: " + std::to_string(T) + " tokens of " +
-                                                          std::to_string(hidden) + " values expected");
     const c10::cuda::CUDAGuard guard(x.device());
     Call c;
     c.x = x.to(at::kBFloat16).contiguous();

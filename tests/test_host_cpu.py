@@ -880,3 +880,21 @@ def test_plans_are_told_apart_by_a_number_that_is_never_given_twice():
         seen.append(plan.serial)
         del plan
     assert len(set(seen)) == 8
+
+
+def test_routed_plan_refuses_shapes_that_do_not_fit_the_expert_ids():
+    """Every extent of a routed batch comes from the [tokens, top-k] ids: fewer router weights or token
+    values than they call for would be read past their end."""
+    from gridbook_b200 import _native, formats as F, kernels
+    hidden, inter, E = 512, 256, 4
+    w13 = kernels.host_weight(_cpu_weight(F.NVFP4_LITERAL, rows=2 * inter, K=hidden, experts=E))
+    w2 = kernels.host_weight(_cpu_weight(F.NVFP4_LITERAL, rows=hidden, K=inter, experts=E))
+    plan = _native.host().MoEPlan(w13, w2, w13, w2, E, hidden, inter, False, False, False)
+    x = torch.empty(3, hidden, dtype=torch.bfloat16)
+    limits = (1, 1, 1, 1, 1, 1)
+    for ids, weights, message in [((3, 2), (3, 1), "router weights"), ((3, 2), (2, 2), "router weights"), ((4, 2), (4, 2), "tokens of"),
+                                  ((6,), (6,), "shape"), ((3, 2, 2), (3, 2, 2), "shape")]:
+        with pytest.raises(RuntimeError, match=message):
+            plan(x, torch.empty(weights), torch.empty(ids, dtype=torch.int32), 0, limits)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        plan(x, torch.empty(3, 2), torch.empty(3, 2, dtype=torch.int32), 0, limits)
