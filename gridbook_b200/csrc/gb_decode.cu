@@ -11,7 +11,9 @@ constexpr int kThreads = 256;
 // ---------------------------------------------------------------------------
 // Activation buckets (gridbook/codec.py:248-260, 428-437)
 // ---------------------------------------------------------------------------
-// One thread per group of 16: two 16-byte loads, amax, scale, 16 roundings.
+// One thread per group of 16: two 16-byte loads, amax, scale, 16 roundings.  kAligned = false: rows that start
+// anywhere, value by value.
+template <bool kAligned>
 __global__ void __launch_bounds__(kThreads)
 fp4_group16_qdq_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ out,
                        int64_t n_groups, int scale_rule) {
@@ -19,13 +21,28 @@ fp4_group16_qdq_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ ou
   gb_pdl_wait();
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= n_groups) return;
-  const uint4* src = reinterpret_cast<const uint4*>(x + g * 16);
-  const uint4 r0 = src[0], r1 = src[1];
-  uint32_t packed[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+  uint32_t packed[8];
+  if (kAligned) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + g * 16);
+    const uint4 r0 = src[0], r1 = src[1];
+    packed[0] = r0.x; packed[1] = r0.y; packed[2] = r0.z; packed[3] = r0.w;
+    packed[4] = r1.x; packed[5] = r1.y; packed[6] = r1.z; packed[7] = r1.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) packed[i] = x[g * 16 + 2 * i] | (uint32_t)x[g * 16 + 2 * i + 1] << 16;
+  }
   gb_fp4_group16_qdq(packed, scale_rule);
-  uint4* dst = reinterpret_cast<uint4*>(out + g * 16);
-  dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-  dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+  if (kAligned) {
+    uint4* dst = reinterpret_cast<uint4*>(out + g * 16);
+    dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      out[g * 16 + 2 * i] = (uint16_t)packed[i];
+      out[g * 16 + 2 * i + 1] = (uint16_t)(packed[i] >> 16);
+    }
+  }
 }
 
 // Per-token E4M3 bucket: one CTA per row, the row held in registers (kVec vectors of eight values
@@ -385,8 +402,9 @@ int gb_fp4_act_qdq(const void* x, void* out, int64_t M, int64_t K, int scale_rul
   if (M == 0) return GB_OK;
   const int64_t groups = M * (K / 16);
   const unsigned blocks = (unsigned)((groups + kThreads - 1) / kThreads);
-  GB_CUDA_OK(gb_launch(fp4_group16_qdq_kernel, dim3(blocks), dim3(kThreads), 0, (cudaStream_t)stream,
-                       (const uint16_t*)x, (uint16_t*)out, groups, scale_rule));
+  const bool aligned = (((uintptr_t)x | (uintptr_t)out) & 15u) == 0;
+  GB_CUDA_OK(gb_launch(aligned ? fp4_group16_qdq_kernel<true> : fp4_group16_qdq_kernel<false>, dim3(blocks), dim3(kThreads), 0,
+                       (cudaStream_t)stream, (const uint16_t*)x, (uint16_t*)out, groups, scale_rule));
   return GB_OK;
 }
 

@@ -934,6 +934,8 @@ int gb_gemv(const void* x, int64_t M, const gb_weight* w, int act, int scale_rul
   GB_REQUIRE(x && y, "null activation or output pointer");
   GB_REQUIRE(M >= 1 && M <= 128, "decode-batch kernels take 1..128 rows, got M=%lld", (long long)M);
   GB_REQUIRE(act == GB_ACT_NONE || act == GB_ACT_FP4_GROUP16 || act == GB_ACT_FP8_TOKEN, "unknown act %d", act);
+  // a bucket of its own rewrites the rows; without one they are read as they lie
+  GB_REQUIRE(act != GB_ACT_NONE || ((uintptr_t)x & 15u) == 0, "rows must be 16-byte aligned");
   const int sms = gb_sm_count();
   if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
   if (M >= umma_min_rows() || (umma_min_rows() <= 128 && !gb_gemv_umma_is_literal(w))) {
@@ -1027,6 +1029,7 @@ int gb_moe_gemv(const void* x, const int32_t* x_row, const gb_weight* w, int64_t
   GB_REQUIRE(!swiglu || w->rows % 2 == 0, "swiglu needs an even row count");
   GB_REQUIRE(act == GB_ACT_NONE || act == GB_ACT_FP4_GROUP16,
              "the routed kernel fuses the fp4 group-16 bucket only (act %d)", act);
+  GB_REQUIRE(((uintptr_t)x & 15u) == 0, "rows must be 16-byte aligned");
   if (P == 0) return GB_OK;
   const int sms = gb_sm_count();
   if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());

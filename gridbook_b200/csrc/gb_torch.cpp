@@ -417,6 +417,7 @@ struct MoEPlan {
     const c10::cuda::CUDAGuard guard(x.device());
     Call c;
     c.x = x.to(at::kBFloat16).contiguous();
+    if (((uintptr_t)c.x.data_ptr() & 15u) != 0) c.x = c.x.clone();   // a view into the middle of another tensor
     c.ids = topk_ids.to(at::kInt).contiguous();
     c.tw = topk_weights.to(at::kFloat).contiguous();
     c.T = T; c.topk = topk; c.P = T * topk; c.rule = rule;

@@ -125,3 +125,34 @@ def test_nvfp4_view_of_resident_slots_is_exact(dev, k, rows, K, books):
     packed, sf = kernels.expand_fp4_nvfp4(synth.to_device_weight(up, dev), swizzled=True)
     assert np.array_equal(packed.cpu().numpy(), rp)
     assert np.array_equal(sf.cpu().numpy(), O.swizzle_sf_plane(rs))
+
+
+@pytest.mark.parametrize("name", ["lit", "k16", "k12", "fp8k32", "fp8k30"])
+def test_rows_that_start_in_the_middle_of_another_tensor(dev, name):
+    """Contiguous activations whose first element is not at a multiple of sixteen bytes: decode batches and
+    routed layers give what they give for a copy of them."""
+    from gridbook_b200 import _native, formats as F, kernels, synth
+    from gridbook_b200.linear import CBLinear
+    from gridbook_b200.moe import CBMoE
+    fmt = {"lit": F.NVFP4_LITERAL, "k16": F.NVFP4_CB_K16, "k12": F.CBFormat("fp4", 12, n_sub=2, scale_coding="v2"),
+           "fp8k32": F.FP8_CB_K32, "fp8k30": F.CBFormat("fp8", 30, n_sub=4)}[name]
+    N, K, E, inter = 256, 1024, 8, 256
+    gen = torch.Generator(device=dev).manual_seed(5)
+    scale = (lambda *s: None) if fmt.is_fp4 else (lambda *s: torch.rand(s, generator=gen, device=dev) + 0.5)
+    lin = CBLinear(fmt, K, [N], [synth.codebook_tables(fmt, 1)]).load(synth.make_packed_device(fmt, N, K, gen, dev), scale(N), dev)
+    moe = CBMoE(fmt, fmt, E, K, inter, synth.codebook_tables(fmt, 1), synth.codebook_tables(fmt, 2))
+    moe.load(synth.make_packed_device(fmt, E * 2 * inter, K, gen, dev).view(E, 2 * inter, -1),
+             synth.make_packed_device(fmt, E * K, inter, gen, dev).view(E, K, -1), scale(E, 2 * inter), scale(E, K), dev)
+    for rows, first in ((1, 1), (1, 2), (3, 1), (16, 5)):
+        flat = torch.randn(rows * K + 16, generator=gen, device=dev).to(torch.bfloat16)
+        x = flat[first:first + rows * K].view(rows, K)
+        assert x.is_contiguous() and x.data_ptr() % 16
+        assert torch.equal(kernels.fp4_act_qdq(x), kernels.fp4_act_qdq(x.clone()))
+        assert torch.equal(kernels.fp8_act_qdq(x), kernels.fp8_act_qdq(x.clone()))
+        a, b = lin(x).float(), lin(x.clone()).float()        # another kernel may serve the odd start: sums in another order
+        assert float((a - b).norm() / b.norm()) <= 1e-3
+        ids = torch.randint(0, E, (rows, 2), generator=gen, device=dev, dtype=torch.int32)
+        tw = torch.full((rows, 2), 0.5, device=dev)
+        assert torch.equal(moe(x, tw, ids), moe(x.clone(), tw, ids))
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0

@@ -898,3 +898,18 @@ def test_routed_plan_refuses_shapes_that_do_not_fit_the_expert_ids():
             plan(x, torch.empty(weights), torch.empty(ids, dtype=torch.int32), 0, limits)
     with pytest.raises(RuntimeError, match="CUDA tensors only"):
         plan(x, torch.empty(3, 2), torch.empty(3, 2, dtype=torch.int32), 0, limits)
+
+
+def test_rows_off_the_vector_alignment_are_refused_where_they_are_read_as_they_lie():
+    """Checked in front of any CUDA call: the kernels fetch sixteen bytes at a time."""
+    from gridbook_b200 import _native as nat
+    lib = nat.load()
+    fmt = nat.GbFormat(grid=0, mode=0, k_bits=16, n_sub=2, type_size=73, scale_coding=2)
+    w = nat.GbWeight(qw=16, row_stride=73, codebook=16, cb_row_offset=None, compose=16, weight_scale=None,
+                     global_scale=1.0, rows=8, K=256, fmt=fmt)
+    at = ctypes.c_void_p
+    assert lib.gb_gemv(at(18), 1, ctypes.byref(w), nat.ACT_NONE, 0, at(16), at(16), 1 << 20, None) == 1
+    assert b"16-byte aligned" in lib.gb_last_error()
+    for act in (nat.ACT_NONE, nat.ACT_FP4_GROUP16):
+        assert lib.gb_moe_gemv(at(18), None, ctypes.byref(w), 8 * 73, 2, at(16), at(16), 4, 0, act, 0, at(16), None, None, 0, None) == 1
+        assert b"16-byte aligned" in lib.gb_last_error()
