@@ -753,17 +753,17 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool ok = *abort_flag == 0;
             if (__builtin_expect(__any_sync(0xffffffffu, (__float_as_uint(xs0) | __float_as_uint(xs1)) & kGbLeftOutBits), 0)) {
-              // Groups left out: added to the sums in tensor memory, spread over the warpgroups, which have a
-              // column of the row each (the accumulators of the first units; hi, lo, dlt).
+              // Groups left out: added to the sums in tensor memory, by the warps that read those out.  (Spread over the
+              // warpgroups they would have to wait for each other here, while the formats whose raw stages
+              // every warpgroup sees need all of them to go on.)
               const int64_t tile = Q.x_tile + (kGrouped ? q_pass : 0);
               const uint8_t* w_row = p.qw + (Q.w_row0 + (kGrouped ? row : min(row, (int)p.N - 1 - Q.n0))) * p.row_stride;
               const uint16_t* cb = reinterpret_cast<const uint16_t*>(p.codebook) + p.role[Q.role].cb;
-              const int parts = wide ? 3 : min(4, units), per = gb_left_out_span(p.n_sb);
-              const uint32_t slot = lane_base + (wide ? (wg == 0 ? 0u : wg == 1 ? 128u : (uint32_t)term_rows(wide, rows))
-                                                      : (uint32_t)((g0 - span + wg) & 3) * acc_stride);
-              const float unit = wide ? (wg == 0 ? 1.0f : wg == 1 ? 0x1p4f : 0x1p7f) : 1.0f;
+              const int per = gb_left_out_span(p.n_sb);
 #pragma unroll 1
-              for (int m0 = 0; m0 < (wg < parts ? rows : 0); m0 += 4) {
+              for (int j = 0; j < (wide ? 4 : 1); ++j) {
+                const int m0 = wide ? (wg + 4 * (j >> 1)) * 8 + 4 * (j & 1) : wg * 4;
+                if (m0 >= rows) break;
                 uint32_t word[4], bits = 0u, marked = 0u;
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
@@ -777,7 +777,6 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll 1
                 for (; bits != 0; bits &= bits - 1) {
                   const int b = __ffs(bits) - 1;
-                  if ((b + (m0 >> 2)) % parts != wg) continue;
                   gb_left_out(
                       add, p.tail + (tile * p.pass_rows + m0) * (p.K / 16), p.K / 16, marked, max(b * per, sb_begin) * 16,
                       min((b + 1) * per, sb_begin + units) * 16,
@@ -787,12 +786,9 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                       [&](int g) { return row_group<F>(w_row, cb, p.compose, g); }, [](const RowGroup& r, float x) { return dot16(r, x); });
                 }
 #pragma unroll
-                for (int r = 0; r < 4; ++r) add[r] = gb_normalised(add[r], word[r]) * unit;
-                gb_tmem_add(slot + (uint32_t)n0, add);
+                for (int r = 0; r < 4; ++r) add[r] = gb_normalised(add[r], word[r]);
+                gb_tmem_add(lane_base + (wide ? 0u : (uint32_t)((g0 - span) & 3) * acc_stride) + (uint32_t)n0, add);
               }
-              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-              asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
             const int64_t col = (int64_t)Q.n0 + row;
             const uint32_t Rt = (uint32_t)term_rows(wide, rows);

@@ -281,3 +281,35 @@ def test_left_out_groups_of_a_routed_layer(dev, f13, f2, T):
     assert "sorted rows" in moe._cb_route
     err = np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)
     assert err.max() <= 1e-2                                 # one step of the second bucket in a few values, as in the test above
+
+
+@pytest.mark.parametrize("name", ["lit", "k16", "k20", "k24"])
+@pytest.mark.parametrize("T", [40, 150, 450])
+def test_left_out_groups_between_tiles_of_one_cta(dev, name, T):
+    """Sums that groups are added to are read out while the CTA's next tile is decoded: more expert tiles than SMs,
+    several passes of a tile, against the decoded bf16 stack's grouped GEMM."""
+    from gridbook_b200 import _native, synth
+    from gridbook_b200.moe import CBMoE
+    fmt = _fmt(name)
+    E, hidden, inter, topk = 40, 2048, 768, 4
+    w13d, w2d = synth.make_moe(fmt, fmt, E, hidden, inter, seed=T)
+    _zero_first_group(fmt, w13d["qw"], w13d["cb"])(w13d["qw"].reshape(E, 2 * inter, -1))
+    ids, tw = synth.make_routing(T, E, topk, seed=T)
+    moe = CBMoE(fmt, fmt, E, hidden, inter, _tables(fmt, w13d["cb"]), _tables(fmt, w2d["cb"]))
+    moe.load(torch.from_numpy(w13d["qw"]), torch.from_numpy(w2d["qw"]), None, None, dev)
+    x = _outlier_rows(T, hidden, T)
+    args = synth.bf16_tensor(x, dev), torch.from_numpy(tw).to(dev), torch.from_numpy(ids).to(dev)
+    moe.method.sorted_min_pairs_per_expert = 0
+    moe.method.prefill_min_pairs_per_expert = 1 << 30
+    got = moe(*args).float()
+    assert "sorted rows" in moe._cb_route
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    moe.method.prefill_min_pairs_per_expert = 1
+    ref = moe(*args).float()
+    assert "grouped prefill" in moe._cb_route
+    # A first projection that rounds to the other bf16 neighbour can move a value of the second bucket by a step,
+    # at most a third of the larger neighbour (4 and 6 on the E2M1 grid), so a row that one value dominates moves
+    # by up to a third; a row whose small groups were dropped is off by its whole length.
+    err = (got - ref).norm(dim=1) / ref.norm(dim=1)
+    assert float(err.max()) <= 1 / 3 and float(err.mean()) <= 3e-3
