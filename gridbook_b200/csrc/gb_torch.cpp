@@ -214,10 +214,17 @@ struct Kept {
 
 constexpr int64_t kDecodeMaxRows = 16;
 // Routed rows per expert from which a stack is decoded once into its NVFP4 view and multiplied by the grouped GEMM,
-// instead of decoded in every pass of up to 64 rows.  128 experts, hidden 2048, intermediate 768: literal 299 against
-// 338 us at 96 rows and equal at 128, K16 350 / 364 at 96 and 454 / 417 at 128.  K20 and K24 hold one superblock per
-// raw stage and decode at half the rate: 286 / 299 at 16 rows, 388 / 284 at 32.
-constexpr int64_t kFp4GemmMinRows = 120, kFp4GemmMinRowsWide = 20;
+// instead of decoded in every pass of up to 64 rows.  The larger an expert, the later: its decoded copy is written
+// and read once whatever the rows, while the passes lose less to their hand-overs.  Whole layer, us, passes / once,
+// literal and K16: hidden 1024, intermediate 512, 64 experts, 112 rows 109 / 108, 117 / 115; 2048 x 768, 128 experts,
+// 128 rows 400 / 400, 431 / 431; 2048 x 1536, 32 experts, 144 rows 209 / 201, 231 / 217; 4096 x 1536, 64 experts,
+// 208 rows 800 / 831, 883 / 876; 7168 x 2048, 32 experts, 128 rows 510 / 705, 572 / 768 and 320 rows 1108 / 1197,
+// 1279 / 1296; 4096 x 4096, 16 experts, 352 rows 700 / 735, 849 / 779.
+// K20 and K24 hold one superblock per raw stage, take 16 rows a pass and cross over earlier and alike: 16 rows 306 / 312
+// (2048 x 768), 467 / 580 (7168 x 2048), 95 / 95 (1024 x 512), 24 rows 365 / 320, 571 / 580, 108 / 99.
+int64_t fp4_gemm_min_rows(const gb_weight& w, int64_t expert_weights) {
+  return w.fmt.k_bits >= 20 ? 20 : 100 + expert_weights / 65536;
+}
 constexpr float kNvfp4ActRange = 448.0f;      // a row's largest group scale factor: the top of the UE4M3 range
 
 // Routes a plan has taken, reported to the host code by number.
@@ -546,7 +553,7 @@ struct MoEPlan {
     const int fp13 = L.gb_moe_fp4_pass_rows(&w13.w, w13.scales_e4m3, c.P, E), fp2 = L.gb_moe_fp4_pass_rows(&w2.w, w2.scales_e4m3, c.P, E);
     // decoded once and multiplied by the grouped GEMM (pass rows 0) where several passes would decode every weight again
     auto once = [&](const Weight& w, int fp) {
-      return fp > 0 && E <= 1024 && c.P >= E * (w.w.fmt.k_bits >= 20 ? kFp4GemmMinRowsWide : kFp4GemmMinRows);
+      return fp > 0 && E <= 1024 && c.P >= E * fp4_gemm_min_rows(w.w, hidden * inter);
     };
     const bool once13 = once(w13, fp13), once2 = once(w2, fp2);
     const int pr13 = once13 ? 0 : fp13, pr2 = once2 ? 0 : fp2;

@@ -31,10 +31,11 @@ PREFILL_MIN_PAIRS_PER_EXPERT = 384
 # rows from SORTED_MIN_PAIRS_OTHER routed pairs in all (two tokens at top-8: 223 us against 272 us
 # on 32 experts of hidden 7168, intermediate 2048).
 SORTED_MIN_PAIRS_PER_EXPERT = 4
-# On the block-scaled FP4 cores the sorted rows of many experts cross over earlier: 128 experts as above, 48
-# tokens (3 pairs per expert) 125 us per pair against 115 sorted, 63 tokens 154 against 119; with 64 experts
-# three pairs per expert are even (58 and 59 us), with 32 the fixed launches of the sorted route weigh more.
-SORTED_MIN_PAIRS_FP4, SORTED_FP4_EXPERTS = 3, 128
+# On the block-scaled FP4 cores the sorted rows of many experts cross over earlier, unless the experts are small: at
+# three pairs per expert, per pair / sorted in us, 2048 x 768 with 64 experts 70 / 75, 96 85 / 98, 112 111 / 110, 128
+# 124 / 119, 192 168 / 164, 256 233 / 210; 4096 x 1536 with 128 402 / 270; but 1024 x 512 with 128 55 / 70, 256 106 / 118
+# (four pairs: 72 / 72 and 128 / 128).
+SORTED_MIN_PAIRS_FP4, SORTED_FP4_EXPERTS, SORTED_FP4_EXPERT_WEIGHTS = 3, 128, 2048 * 768
 SORTED_MIN_PAIRS_OTHER = 16
 # Stacks of the fp4 grid multiply the sorted rows on the block-scaled FP4 tensor cores, several times the
 # rate of the decoded bf16 stack's GEMM: they stay on that route.
@@ -81,6 +82,12 @@ def unfilled_cb_params(layer) -> list[str]:
         if not getattr(p, CB_FILLED_ATTR, False):
             missing.append(name)
     return missing
+
+
+def _sorted_min_pairs(fp4: bool, experts: int, expert_weights: int) -> int:
+    """Default of ``sorted_min_pairs_per_expert`` of a loaded stack; ``expert_weights``: hidden x intermediate."""
+    early = fp4 and experts >= SORTED_FP4_EXPERTS and expert_weights >= SORTED_FP4_EXPERT_WEIGHTS
+    return SORTED_MIN_PAIRS_FP4 if early else SORTED_MIN_PAIRS_PER_EXPERT
 
 
 def _threshold(name: str, default: int) -> property:
@@ -307,7 +314,7 @@ class PrismaQuantCBMoEMethod(FusedMoEMethodBase):
             kernels.moe_gemv_sorted_applies(w13), sorted2, pair_ok)
         # defaults of this stack for the thresholds that no caller has set
         fp4 = layer._cb_plan.fp4
-        layer._cb_sorted_min = SORTED_MIN_PAIRS_FP4 if fp4 and layer._cb_E >= SORTED_FP4_EXPERTS else SORTED_MIN_PAIRS_PER_EXPERT
+        layer._cb_sorted_min = _sorted_min_pairs(fp4, layer._cb_E, layer._cb_hidden * layer._cb_inter)
         layer._cb_prefill_min = PREFILL_MIN_PAIRS_FP4 if fp4 else PREFILL_MIN_PAIRS_PER_EXPERT
         layer._cb_layer_id = ops.register_cb_layer(self, layer)
         print(f"[prismaquant-cb] {self.prefix}: decode=grouped-cuda (sm_100a) "

@@ -913,3 +913,10 @@ def test_rows_off_the_vector_alignment_are_refused_where_they_are_read_as_they_l
     for act in (nat.ACT_NONE, nat.ACT_FP4_GROUP16):
         assert lib.gb_moe_gemv(at(18), None, ctypes.byref(w), 8 * 73, 2, at(16), at(16), 4, 0, act, 0, at(16), None, None, 0, None) == 1
         assert b"16-byte aligned" in lib.gb_last_error()
+
+
+def test_sorted_rows_start_early_only_where_that_was_measured():
+    from gridbook_b200.moe import _sorted_min_pairs
+    assert _sorted_min_pairs(True, 128, 2048 * 768) == 3 and _sorted_min_pairs(True, 256, 7168 * 2048) == 3
+    for fp4, experts, weights in [(True, 127, 2048 * 768), (True, 128, 1024 * 512), (True, 256, 2048 * 512), (False, 256, 7168 * 2048)]:
+        assert _sorted_min_pairs(fp4, experts, weights) == 4
