@@ -43,6 +43,8 @@ NOMINAL_TFLOPS = {"bf16": 2250.0, "fp8": 4500.0, "fp4": 9000.0}       # dense, p
 TRAFFIC = {"gemv_tab_kernel": (1.002, "profiles/gemv_tab_kernel_literal_m1_gate_up.md"),
            "gemv_dot_kernel": (1.002, "profiles/gemv_dot_kernel_literal_m1_gate_up.md"),
            "gemv_kernel": (1.01, "profiles/gemv_kernel_k16v2_m1_gate_up.md"),
+           "fp4_decode_kernel": (1.015, "profiles/fp4_decode_kernel_m16_m64_gate_up.md"),
+           "fp4_decode_kernel/k16v2": (1.10, "profiles/fp4_decode_kernel_m16_m64_gate_up.md"),
            "umma_decode_kernel": (1.006, "profiles/umma_decode_kernel_literal_k16v2_m16_gate_up.md"),
            # two-tier layers are fetched in 80-byte superblock slots: 80 / 73 of the algorithmic bytes
            "umma_decode_kernel/k16v2": (1.10, "profiles/umma_decode_kernel_literal_k16v2_m16_gate_up.md")}
@@ -457,8 +459,10 @@ def run_gpu(args):
     launch_ms = ms_kernel / args.steps / n_linear
     achieved = launch_bytes / (launch_ms * 1e-3) / 1e9
     w0 = locals_[0][3]._cb_weight if len(locals_[0]) > 3 else locals_[0][0]._cb_weight
+    # sharded layers go through gb_gemv and the peer kernels, whole ones through their plan
+    on_fp4 = world == 1 and fmt.is_fp4
     on_umma = 16 < kernels.row_batch_max_rows(w0) >= M and (args.format != "literal" or M >= 5)
-    dominant_kernel = ("gemv_tab_kernel" if tab else "umma_decode_kernel" if on_umma
+    dominant_kernel = ("gemv_tab_kernel" if tab else "fp4_decode_kernel" if on_fp4 else "umma_decode_kernel" if on_umma
                        else "gemv_dot_kernel" if (M <= 4 and args.format == "literal") else "gemv_kernel")
     traffic_ratio, traffic_source = TRAFFIC.get(f"{dominant_kernel}/{args.format}", TRAFFIC[dominant_kernel])
     line = {
@@ -838,7 +842,8 @@ def bench_prefill(args, device):
                     kernels.gemm_fp4(a, sfa, b, sfb, a_scale=asc)
                     ms_gemm = timed_ms(lambda: kernels.gemm_fp4(a, sfa, b, sfb, a_scale=asc), 3, sync)
                     tf = flops / ms_gemm / 1e9
-                    entry.update({"kernel": "gemm_fp4_kernel", "gemm_tflops": round(tf, 1), "gemm_ms": round(ms_gemm, 4),
+                    pair = "gemm_pair_kernel (kind::mxf4nvf4)" if M > 128 else "gemm_fp4_kernel"
+                    entry.update({"kernel": pair, "gemm_tflops": round(tf, 1), "gemm_ms": round(ms_gemm, 4),
                                   "pct_fp4_nominal": round(100 * tf / NOMINAL_TFLOPS["fp4"], 2),
                                   "pct_of_4x_measured_bf16": round(100 * tf / (4 * bf16_meas), 2)})
                     del a, sfa, b, sfb
@@ -853,14 +858,14 @@ def bench_prefill(args, device):
                                     "unit": "TFLOP/s", "frac": round(tf / NOMINAL_TFLOPS["fp4"], 4),
                                     "peak_kind": "fp4 dense, nominal (no measured fp4 figure on this pool)",
                                     "frac_of_4x_measured_bf16": round(tf / (4 * bf16_meas), 4),
-                                    "kernel": "gemm_fp4_kernel", "workload": f"{name} {N}x{K}, M={M}, literal"}
+                                    "kernel": pair, "workload": f"{name} {N}x{K}, M={M}, literal"}
                 else:
                     a, sa = kernels.fp8_quantize_rows(x)
                     b = kernels.expand_fp8(w)
                     kernels.gemm_tn(a, b, a_scale=sa, b_scale=w.weight_scale)
                     ms_gemm = timed_ms(lambda: kernels.gemm_tn(a, b, a_scale=sa, b_scale=w.weight_scale), 3, sync)
                     tf = flops / ms_gemm / 1e9
-                    entry.update({"kernel": "gemm_tn_kernel (kind::f8f6f4)", "gemm_tflops": round(tf, 1),
+                    entry.update({"kernel": f"gemm_{'pair' if M > 128 else 'tn'}_kernel (kind::f8f6f4)", "gemm_tflops": round(tf, 1),
                                   "gemm_ms": round(ms_gemm, 4),
                                   "pct_fp8_nominal": round(100 * tf / NOMINAL_TFLOPS["fp8"], 2),
                                   "pct_of_2x_measured_bf16": round(100 * tf / (2 * bf16_meas), 2)})
