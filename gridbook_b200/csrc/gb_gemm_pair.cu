@@ -20,12 +20,13 @@
 // one warp, 647 with two, 635 with four, 559 with none at all).  The accumulator is drained into
 // registers in one go, so that the next tile's MMAs start early.
 //
-// Measured, us, one CTA per tile -> pairs (N x K of the four linears of a 5120-wide layer):
-//   fp8, 8192 rows: 34816 x 5120 1434 -> 1096, 5120 x 17408 729 -> 552, 6144 x 5120 263 -> 199, 2048 x 5120 101 -> 72
-//   fp8, 2048 rows: 370 -> 276, 218 -> 156, 80 -> 54, 36 -> 24
-//   fp4, 8192 rows: 960 -> 635, 437 -> 302, 184 -> 116, 66 -> 43
-//   fp4, 2048 rows: 253 -> 165, 145 -> 92, 54 -> 33, 21 -> 18
-// The fp8 form runs at 2.65 PFLOP/s, tensor pipe 71% busy at the 1.55 GHz that the power cap leaves.
+// Measured, us, one CTA per tile -> pairs, launches back to back (N x K of the four linears of a 5120-wide layer;
+// lowest and highest of three runs on different boxes, which differ in what the power cap leaves):
+//   fp8, 8192 rows: 34816 x 5120 1434 -> 1081..1247, 5120 x 17408 729 -> 544..558, 6144 x 5120 263 -> 200..205, 2048 x 5120 101 -> 83..94
+//   fp8, 2048 rows: 370 -> 278..281, 218 -> 167..187, 80 -> 56..68, 36 -> 26..32
+//   fp4, 8192 rows: 960 -> 604..624, 437 -> 295..390, 184 -> 114..138, 66 -> 49..55
+//   fp4, 2048 rows: 253 -> 159..191, 145 -> 102..133, 54 -> 34..43, 21 -> 15..21
+// The fp8 gate_up at 8192 rows under a profiler: 2.7 PFLOP/s, tensor pipe 79% busy at the 1.45 GHz that the power cap leaves.
 #include "gb_common.cuh"
 
 #include <cuda.h>

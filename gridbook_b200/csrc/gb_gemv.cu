@@ -942,7 +942,9 @@ int gb_gemv(const void* x, int64_t M, const gb_weight* w, int act, int scale_rul
     // decode into tensor memory, tensor-core MMA with the weights on the M side; every weight is
     // decoded once whatever the row count.  The literal format has faster table kernels for a few
     // rows; the product formats it serves (padded two-tier k = 16, fp8 k = 32 and k = 16) take it from
-    // one row on.  A threshold past 128 switches the kernel off for every format.
+    // one row on.  A threshold past 128 switches the kernel off for every format.  The fp4 formats get here
+    // from callers of this entry and of the sharded layers; a layer's own plan calls gb_gemv_hinted, which
+    // keeps them on the block-scaled cores up to K = 65536.
     rc = gb_gemv_umma(x, M, w, 0, nullptr, act, scale_rule, y, workspace, workspace_bytes, stream_);
     if (rc != GB_EUNSUPPORTED) return rc;
   }

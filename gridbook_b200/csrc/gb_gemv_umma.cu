@@ -23,6 +23,10 @@
 // Four packed formats: the literal one (fp4 grid, full k = 8, E4M3 scale bytes: 48-byte
 // superblocks), the two-tier product format fp4 k = 16 with its superblocks padded from 73 to 80
 // bytes (so that rows can be fetched by TMA), and the fp8 product format k = 32 (128 bytes).
+//
+// Who calls it: the fp8 grid, dense and per expert; two-tier layers with a scale that is no E4M3 value; the sharded
+// layers and experts of the peer-memory path.  The literal format and the other two-tier layers of an unsharded model
+// run on the block-scaled FP4 cores (gb_gemv_fp4.cu) wherever that kernel takes them.
 #include "gb_common.cuh"
 
 #include <cuda.h>

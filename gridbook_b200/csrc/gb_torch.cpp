@@ -33,44 +33,20 @@ namespace py = pybind11;
 
 namespace {
 
+// The library's entries used here.
+#define GB_ENTRIES(F) \
+  F(gb_last_error) F(gb_gemv_hinted_workspace_bytes) F(gb_gemv) F(gb_gemv_row_batch_max) F(gb_gemv_tab) \
+  F(gb_gemv_tab_slots_bytes) F(gb_fp4_act_qdq) F(gb_fp8_act_qdq) F(gb_fp8_quantize_rows) F(gb_nvfp4_sf_bytes) \
+  F(gb_nvfp4_quantize_rows) F(gb_expand_fp4_nvfp4) F(gb_expand_fp4_bf16) F(gb_expand_fp8) F(gb_expand_fp8_bf16) \
+  F(gb_gemm_fp4) F(gb_gemm_tn) F(gb_gemm_tn_grouped) F(gb_moe_route_ws) F(gb_moe_route_workspace_bytes) \
+  F(gb_moe_gather_rows) F(gb_moe_swiglu_rows) F(gb_moe_gemv) F(gb_moe_gemv_sorted) F(gb_moe_mlp_pairs) \
+  F(gb_moe_mlp_pairs_workspace_bytes) F(gb_moe_combine) F(gb_gemv_hinted) F(gb_scales_e4m3) F(gb_moe_route_inv) \
+  F(gb_moe_fp4_pass_rows) F(gb_moe_fp4_operand_bytes) F(gb_moe_fp4_rows) F(gb_moe_fp4_swiglu_rows) \
+  F(gb_moe_gemv_fp4) F(gb_moe_gemm_fp4)
+
 struct Lib {
-#define GB_FN(name) decltype(&::name) name = nullptr
-  GB_FN(gb_last_error);
-  GB_FN(gb_gemv_hinted_workspace_bytes);
-  GB_FN(gb_gemv);
-  GB_FN(gb_gemv_row_batch_max);
-  GB_FN(gb_gemv_tab);
-  GB_FN(gb_gemv_tab_slots_bytes);
-  GB_FN(gb_fp4_act_qdq);
-  GB_FN(gb_fp8_act_qdq);
-  GB_FN(gb_fp8_quantize_rows);
-  GB_FN(gb_nvfp4_sf_bytes);
-  GB_FN(gb_nvfp4_quantize_rows);
-  GB_FN(gb_expand_fp4_nvfp4);
-  GB_FN(gb_expand_fp4_bf16);
-  GB_FN(gb_expand_fp8);
-  GB_FN(gb_expand_fp8_bf16);
-  GB_FN(gb_gemm_fp4);
-  GB_FN(gb_gemm_tn);
-  GB_FN(gb_gemm_tn_grouped);
-  GB_FN(gb_moe_route_ws);
-  GB_FN(gb_moe_route_workspace_bytes);
-  GB_FN(gb_moe_gather_rows);
-  GB_FN(gb_moe_swiglu_rows);
-  GB_FN(gb_moe_gemv);
-  GB_FN(gb_moe_gemv_sorted);
-  GB_FN(gb_moe_mlp_pairs);
-  GB_FN(gb_moe_mlp_pairs_workspace_bytes);
-  GB_FN(gb_moe_combine);
-  GB_FN(gb_gemv_hinted);
-  GB_FN(gb_scales_e4m3);
-  GB_FN(gb_moe_route_inv);
-  GB_FN(gb_moe_fp4_pass_rows);
-  GB_FN(gb_moe_fp4_operand_bytes);
-  GB_FN(gb_moe_fp4_rows);
-  GB_FN(gb_moe_fp4_swiglu_rows);
-  GB_FN(gb_moe_gemv_fp4);
-  GB_FN(gb_moe_gemm_fp4);
+#define GB_FN(name) decltype(&::name) name = nullptr;
+  GB_ENTRIES(GB_FN)
 #undef GB_FN
 };
 Lib L;
@@ -78,45 +54,10 @@ Lib L;
 void bind(const std::string& path) {
   void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
   if (!h) throw std::runtime_error("cannot load " + path + ": " + dlerror());
-#define GB_FN(name)                                                                   \
-  L.name = reinterpret_cast<decltype(L.name)>(dlsym(h, #name));                       \
-  if (!L.name) throw std::runtime_error(path + " lacks the required symbol " #name)
-  GB_FN(gb_last_error);
-  GB_FN(gb_gemv_hinted_workspace_bytes);
-  GB_FN(gb_gemv);
-  GB_FN(gb_gemv_row_batch_max);
-  GB_FN(gb_gemv_tab);
-  GB_FN(gb_gemv_tab_slots_bytes);
-  GB_FN(gb_fp4_act_qdq);
-  GB_FN(gb_fp8_act_qdq);
-  GB_FN(gb_fp8_quantize_rows);
-  GB_FN(gb_nvfp4_sf_bytes);
-  GB_FN(gb_nvfp4_quantize_rows);
-  GB_FN(gb_expand_fp4_nvfp4);
-  GB_FN(gb_expand_fp4_bf16);
-  GB_FN(gb_expand_fp8);
-  GB_FN(gb_expand_fp8_bf16);
-  GB_FN(gb_gemm_fp4);
-  GB_FN(gb_gemm_tn);
-  GB_FN(gb_gemm_tn_grouped);
-  GB_FN(gb_moe_route_ws);
-  GB_FN(gb_moe_route_workspace_bytes);
-  GB_FN(gb_moe_gather_rows);
-  GB_FN(gb_moe_swiglu_rows);
-  GB_FN(gb_moe_gemv);
-  GB_FN(gb_moe_gemv_sorted);
-  GB_FN(gb_moe_mlp_pairs);
-  GB_FN(gb_moe_mlp_pairs_workspace_bytes);
-  GB_FN(gb_moe_combine);
-  GB_FN(gb_gemv_hinted);
-  GB_FN(gb_scales_e4m3);
-  GB_FN(gb_moe_route_inv);
-  GB_FN(gb_moe_fp4_pass_rows);
-  GB_FN(gb_moe_fp4_operand_bytes);
-  GB_FN(gb_moe_fp4_rows);
-  GB_FN(gb_moe_fp4_swiglu_rows);
-  GB_FN(gb_moe_gemv_fp4);
-  GB_FN(gb_moe_gemm_fp4);
+#define GB_FN(name)                                              \
+  L.name = reinterpret_cast<decltype(L.name)>(dlsym(h, #name));  \
+  if (!L.name) throw std::runtime_error(path + " lacks the required symbol " #name);
+  GB_ENTRIES(GB_FN)
 #undef GB_FN
 }
 
@@ -593,6 +534,7 @@ struct MoEPlan {
     route = kMoeSorted;
   }
 
+  // (Stacks that the FP4 cores take come here only when a caller has set the limit: their default is never.)
   // Many tokens per expert: each stack decoded once into a transient bf16 tile of the exact served
   // weights, one grouped tensor-core GEMM over the expert segments per projection - the reference's
   // grouped bf16 route (gridbook/moe.py:2388-2504 with gridbook/ops.py:137-306).  Both grids keep the

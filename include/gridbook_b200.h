@@ -159,8 +159,8 @@ GB_API int gb_scales_e4m3(const gb_weight* w, int64_t rows, int32_t* flag, void*
  * qualify - the literal one, the two-tier product formats k = 12, 16, 20, 24 in superblock slots
  * of a multiple of sixteen bytes, one codebook per role or for all rows - run on the block-scaled
  * FP4 tensor cores (tcgen05 kind::mxf4nvf4): packed rows decoded to E2M1 nibbles in tensor memory,
- * activations split exactly into three E2M1 x UE4M3 terms, fp32 accumulate, same results as gb_gemv up to the
- * order of the sum.  Everything else goes to gb_gemv.  workspace: gb_gemv_hinted_workspace_bytes()
+ * activations split exactly into three E2M1 x UE4M3 terms (groups that no common range holds are added in
+ * fp32), fp32 accumulate, same results as gb_gemv up to the order of the sum.  Everything else goes to gb_gemv.  workspace: gb_gemv_hinted_workspace_bytes()
  * bytes.  Replaces the same reference entries as gb_gemv. */
 GB_API int gb_gemv_hinted(const void* x_bf16, int64_t M, const gb_weight* w, const gb_hints* hints, int scale_rule,
                           void* y_bf16, void* workspace, int64_t workspace_bytes, void* stream);
