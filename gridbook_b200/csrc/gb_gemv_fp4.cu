@@ -1616,6 +1616,8 @@ int gb_moe_fp4_swiglu_rows(const void* h, const int32_t* ids, const int32_t* ord
 int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, int64_t expert_stride, int64_t E,
                     const int32_t* seg, const int32_t* row_map, int64_t P, int pass_rows, void* y, void* stream_) {
   GB_REQUIRE(operand && w && seg && y, "null pointer argument");
+  GB_REQUIRE(P >= 1 && P < (1ll << 30) && E >= 1 && pass_rows >= 1 && pass_rows <= kMaxRows, "bad shape P=%lld E=%lld, %d rows per pass",
+             (long long)P, (long long)E, pass_rows);
   int rc = gb_check_weight(w);
   if (rc != GB_OK) return rc;
   const int64_t N = w->rows, K = w->K;

@@ -920,3 +920,16 @@ def test_sorted_rows_start_early_only_where_that_was_measured():
     assert _sorted_min_pairs(True, 128, 2048 * 768) == 3 and _sorted_min_pairs(True, 256, 7168 * 2048) == 3
     for fp4, experts, weights in [(True, 127, 2048 * 768), (True, 128, 1024 * 512), (True, 256, 2048 * 512), (False, 256, 7168 * 2048)]:
         assert _sorted_min_pairs(fp4, experts, weights) == 4
+
+
+def test_grouped_fp4_entry_refuses_row_counts_that_no_operand_has():
+    """pass_rows = 0 names the grouped GEMM's operand; as a divisor it ended the process."""
+    from gridbook_b200 import _native as nat
+    lib = nat.load()
+    fmt = nat.GbFormat(grid=0, mode=1, k_bits=8, n_sub=1, type_size=48, scale_coding=1)
+    w = nat.GbWeight(qw=256, row_stride=48, codebook=256, cb_row_offset=None, compose=None, weight_scale=None,
+                     global_scale=1.0, rows=128, K=256, fmt=fmt)
+    at, n = ctypes.c_void_p, ctypes.c_int64
+    for P, E, pass_rows in [(4, 2, 0), (4, 2, -1), (4, 2, 65), (0, 2, 16), (4, 0, 16)]:
+        assert lib.gb_moe_gemv_fp4(at(256), ctypes.byref(w), 1, n(128 * 48), n(E), at(256), None, n(P), pass_rows, at(256), None) == 1
+        assert b"rows per pass" in lib.gb_last_error()
