@@ -347,8 +347,9 @@ GB_DEVINL uint4 gb_fp4_group16_qdq_pair(uint4 in, int scale_rule) {
 // group), and the low bits of the row's power of two say which sixteenths of the row hold any.  They are
 // multiplied on the plain fp32 units: the lane's weight row times groups [g_begin, g_end) of four activation
 // rows (those in `rows`), added to acc.  codes(r, g): the E2M1 codes of a group; load(g): what the lane's weight
-// row needs of it (32 rows: some three hundred shared-memory-path cycles, hence four rows for each); dot(raw, x): its
-// sixteen weights times x, which lane i (and i + 16) holds element i of.
+// row needs of it (some three hundred L1 wavefronts for the 32 rows of a warp, which bound the work where many
+// groups are left out; hence four activation rows for each load); dot(raw, x): its sixteen weights times x, which
+// lane i (and i + 16) holds element i of.
 constexpr uint32_t kGbLeftOutBits = 0xFFFFu, kGbRowScaleMask = 0x7F800000u;
 GB_DEVINL int gb_left_out_span(int n_sb) { return (n_sb + 15) / 16; }   // superblocks per bit
 template <typename Codes, typename Load, typename Dot>
