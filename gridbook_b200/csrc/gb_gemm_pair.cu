@@ -15,9 +15,9 @@
 //
 // The fp4 form has one accumulator: the columns beside it hold five or six sets of scale factors, which
 // warps 10-13 of the leader copy from both CTAs' shared memory (tcgen05.cp, one warp per MMA of a stage)
-// that many stages ahead of the MMAs.  A copy takes its issuing thread 45 clocks or more and a stage
-// needs twelve: from one warp they took longer than the stage's MMAs (8192 x 34816 x 5120: 759 us with
-// one warp, 647 with two, 635 with four, 559 with none at all).  The accumulator is drained into
+// that many stages ahead of the MMAs: a stage needs twelve copies, and from one warp they took longer than the
+// stage's MMAs (8192 x 34816 x 5120, issued as one lane's code: 759 us with one warp, 647 with two, 635 with four,
+// 559 with none at all).  The accumulator is drained into
 // registers in one go, so that the next tile's MMAs start early.
 //
 // Measured, us, one CTA per tile -> pairs, launches back to back (N x K of the four linears of a 5120-wide layer;
@@ -127,6 +127,23 @@ template <bool kOfPair = false>
 GB_DEVINL void wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   if (!try_wait<kOfPair>(bar, parity)) wait_slow<kOfPair>(bar, parity, abort_flag, status, code);
 }
+// The same for a whole warp that goes on together; false: given up.
+template <bool kOfPair = false>
+GB_DEVINL bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (__all_sync(0xffffffffu, try_wait<kOfPair>(bar, parity))) return true;
+  wait_slow<kOfPair>(bar, parity, abort_flag, status, code);
+  return !__any_sync(0xffffffffu, *abort_flag != 0);
+}
+// The loading, issuing and copying warps walk their loops as a whole, with values that are the same in every lane, and one
+// elected lane issues: the operands stay in uniform registers.  (In code that only lane 0 enters, each is
+// moved there first: 53 clocks to issue an MMA whatever its size, 45 or more a copy.  One dense layer, us: 333 rows K20
+// 249 -> 233, 2048 rows literal 522 -> 491, 8192 rows fp8 2853 -> 2677; routed, 4096 tokens, 656 -> 613.)
+GB_DEVINL bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
+GB_DEVINL int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 // Tile load into this CTA's shared memory that reports to a barrier of the pair.
 GB_DEVINL void tma_load_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
@@ -341,27 +358,30 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
   if (warp == kEpiWarps) {
     // ------------------------------- producer (each CTA) -------------------------------
-    if (lane == 0) {
-      constexpr int slab_elems = kKind == kBf16 ? kSlabBytes / 2 : kSlabBytes;   // E2M1 pairs and E4M3 go by bytes
-      const uint32_t full_pair = leader_addr(full_bar);
-      int s = 0;
-      uint32_t ph = 1;
-      for (Tiles<kBN, kGrouped> T(p, first, stride); T.next(p, total_tiles, seg_s, base_s);) {
-        const int m0 = T.m0 + (int)rank * kBM, n0 = T.n0;
-        for (int kt = 0; kt < p.k_tiles; ++kt) {
-          wait<true>(empty_bar + 8 * s, ph, abort_flag, p.status, 71);
-          if (*abort_flag) break;
+    constexpr int slab_elems = kKind == kBf16 ? kSlabBytes / 2 : kSlabBytes;   // E2M1 pairs and E4M3 go by bytes
+    const uint32_t full_pair = (uint32_t)uniform((int)leader_addr(full_bar));
+    const int me = uniform((int)rank);
+    const bool one = elect_one();
+    int s = 0;
+    uint32_t ph = 1;
+    bool ok = true;
+    for (Tiles<kBN, kGrouped> T(p, first, stride); ok && T.next(p, total_tiles, seg_s, base_s);) {
+      const int m0 = uniform(T.m0) + me * kBM, n0 = uniform(T.n0), x_tile = uniform(T.x_tile);
+      for (int kt = 0; kt < p.k_tiles; ++kt) {
+        ok = warp_wait<true>(empty_bar + 8 * s, ph, abort_flag, p.status, 71);
+        if (!ok) break;
+        if (one) {
           const uint32_t st = ring + (uint32_t)s * S::kStageBytes;
-          if (rank == 0) expect_tx(full_bar + 8 * s, 2 * S::kStageBytes);
+          if (me == 0) expect_tx(full_bar + 8 * s, 2 * S::kStageBytes);
           tma_load_pair(st, &map_a, kt * slab_elems, m0, full_pair + 8 * s);
           if (kGrouped) {                                    // 32 rows: codes of q for hi and for lo, of the correction
             const uint32_t b = st + S::kABytes;
-            const int r0 = T.x_tile * 2 * kTileRows + (int)rank * 32;
+            const int r0 = x_tile * 2 * kTileRows + me * 32;
             tma_load_pair(b, &map_b, kt * slab_elems, r0, full_pair + 8 * s);
             tma_load_pair(b + 4096, &map_b, kt * slab_elems, r0, full_pair + 8 * s);
             tma_load_pair(b + 8192, &map_b, kt * slab_elems, r0 + kTileRows, full_pair + 8 * s);
           } else {
-            tma_load_pair(st + S::kABytes, &map_b, kt * slab_elems, n0 + (int)rank * (kBN / 2), full_pair + 8 * s);
+            tma_load_pair(st + S::kABytes, &map_b, kt * slab_elems, n0 + me * (kBN / 2), full_pair + 8 * s);
           }
           if (kKind == kFp4) {                               // row groups past the end read zero
             const uint32_t sf = st + S::kABytes + S::kBBytes;
@@ -369,72 +389,81 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             tma_load_pair(sf + S::kAtoms, &map_sfb, 0, (n0 / 128 * p.k_tiles + kt) * 8, full_pair + 8 * s);
             tma_load_pair(sf + 2 * S::kAtoms, &map_sfb, 0, ((n0 / 128 + 1) * p.k_tiles + kt) * 8, full_pair + 8 * s);
           }
-          if (++s == kStages) { s = 0; ph ^= 1; }
         }
-        if (*abort_flag) break;
+        __syncwarp();
+        if (++s == kStages) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp == kEpiWarps + 1) {
     // --------------------------- MMA issuer (the leader's) ------------------------------
-    if (lane == 0 && rank == 0) {
+    if (uniform((int)rank) == 0) {
       uint32_t to_peer;                                      // distance of the peer's barriers
       asm volatile("mapa.shared::cluster.u32 %0, %1, 1;" : "=r"(to_peer) : "r"(full_bar));
-      to_peer -= full_bar;
+      to_peer = (uint32_t)uniform((int)(to_peer - full_bar));
+      const uint32_t tmem = (uint32_t)uniform((int)tmem_base);
+      const int tiles = uniform(my_tiles);
+      const bool one = elect_one();
       int s = 0, set = 0;
       uint32_t ph = 0, sf_ph = 0;
+      bool ok = true;
       Tiles<kBN, kGrouped> T(p, first, stride);
-      for (int it = 0; it < my_tiles; ++it) {
+      for (int it = 0; ok && it < tiles; ++it) {
         const int buf = S::kAccs == 2 ? it & 1 : 0;
         const uint32_t use = (uint32_t)(S::kAccs == 2 ? it >> 1 : it);
         bool shifted = false;
         if (kKind == kFp4 && kBN % 128 != 0) {
           T.next(p, total_tiles, seg_s, base_s);
-          shifted = T.n0 % 128 != 0;
+          shifted = uniform(T.n0) % 128 != 0;
         }
-        wait<true>(acc_empty + 8 * buf, (use & 1) ^ 1, abort_flag, p.status, 72); // its last tile is drained
-        const uint32_t acc = tmem_base + (buf ? S::kAcc1 : 0u);
+        ok = warp_wait<true>(acc_empty + 8 * buf, (use & 1) ^ 1, abort_flag, p.status, 72);   // its last tile is drained
+        if (!ok) break;
+        const uint32_t acc = tmem + (buf ? S::kAcc1 : 0u);
         for (int kt = 0; kt < p.k_tiles; ++kt) {
-          if (kKind == kFp4) wait(sf_full + 8 * set, sf_ph, abort_flag, p.status, 73);
-          else wait(full_bar + 8 * s, ph, abort_flag, p.status, 74);
-          if (*abort_flag) break;
+          ok = kKind == kFp4 ? warp_wait(sf_full + 8 * set, sf_ph, abort_flag, p.status, 73)
+                             : warp_wait(full_bar + 8 * s, ph, abort_flag, p.status, 74);
+          if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t st = ring + (uint32_t)s * S::kStageBytes;
           const uint64_t da = desc_sw128(st), db = desc_sw128(st + S::kABytes);
           // 192 columns start in the middle of a 128-row group every other time: two columns on
-          const uint32_t sfa_t = tmem_base + S::kSf0 + S::kSfCols * set, sfb_t = sfa_t + 16u + (shifted ? 2u : 0u);
+          const uint32_t sfa_t = tmem + S::kSf0 + S::kSfCols * set, sfb_t = sfa_t + 16u + (shifted ? 2u : 0u);
+          if (one) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)                        // 32 bytes of K per instruction
-            mma_pair<kKind>(acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), p.idesc, sfa_t + 4u * k, sfb_t + 8u * k,
-                            kt > 0 || k > 0);
-          commit_pair(empty_bar + 8 * s, to_peer);
-          if (kKind == kFp4) {
-            commit_to(sf_empty + 8 * set);
-            if (++set == S::kSets) { set = 0; sf_ph ^= 1; }
+            for (int k = 0; k < 4; ++k)                      // 32 bytes of K per instruction
+              mma_pair<kKind>(acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), p.idesc, sfa_t + 4u * k, sfb_t + 8u * k,
+                              kt > 0 || k > 0);
+            commit_pair(empty_bar + 8 * s, to_peer);
+            if (kKind == kFp4) commit_to(sf_empty + 8 * set);
           }
+          __syncwarp();
+          if (kKind == kFp4 && ++set == S::kSets) { set = 0; sf_ph ^= 1; }
           if (++s == kStages) { s = 0; ph ^= 1; }
         }
-        if (*abort_flag) break;
-        commit_pair(acc_full + 8 * buf, to_peer);
+        if (ok && one) commit_pair(acc_full + 8 * buf, to_peer);
+        __syncwarp();
       }
     }
   } else if (warp >= kEpiWarps + 2) {
     // ------------ scale factors -> tensor memory (the leader's, fp4): warp k the k-th MMA's ------------
-    const uint32_t k = (uint32_t)(warp - kEpiWarps - 2);
-    if (lane == 0 && rank == 0) {
+    const uint32_t k = (uint32_t)(uniform(warp) - kEpiWarps - 2);
+    if (uniform((int)rank) == 0) {
+      const uint32_t tmem = (uint32_t)uniform((int)tmem_base);
+      const bool one = elect_one();
       int s = 0, set = 0;
       uint32_t ph = 0, sf_ph = 1;
-      const int total = my_tiles * p.k_tiles;
+      const int total = uniform(my_tiles) * p.k_tiles;
       for (int g = 0; g < total; ++g) {
-        wait(full_bar + 8 * s, ph, abort_flag, p.status, 75);
-        wait(sf_empty + 8 * set, sf_ph, abort_flag, p.status, 76);
-        if (*abort_flag) break;
+        if (!warp_wait(full_bar + 8 * s, ph, abort_flag, p.status, 75) || !warp_wait(sf_empty + 8 * set, sf_ph, abort_flag, p.status, 76)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t sf = ring + (uint32_t)s * S::kStageBytes + S::kABytes + S::kBBytes;
-        const uint32_t col = tmem_base + S::kSf0 + S::kSfCols * set;
-        sf_to_tmem(col + 4u * k, sf + 512u * k);
-        sf_to_tmem(col + 16u + 8u * k, sf + S::kAtoms + 512u * k);
-        sf_to_tmem(col + 20u + 8u * k, sf + 2 * S::kAtoms + 512u * k);
-        commit_to(sf_full + 8 * set);
+        const uint32_t col = tmem + S::kSf0 + S::kSfCols * set;
+        if (one) {
+          sf_to_tmem(col + 4u * k, sf + 512u * k);
+          sf_to_tmem(col + 16u + 8u * k, sf + S::kAtoms + 512u * k);
+          sf_to_tmem(col + 20u + 8u * k, sf + 2 * S::kAtoms + 512u * k);
+          commit_to(sf_full + 8 * set);
+        }
+        __syncwarp();
         if (++set == S::kSets) { set = 0; sf_ph ^= 1; }
         if (++s == kStages) { s = 0; ph ^= 1; }
       }
