@@ -26,14 +26,17 @@
 //
 // Work split as in gb_gemv_umma.cu: a CTA owns 128 weight rows (the M side) and a K slice; one warp
 // streams the packed rows (tiled TMA), one the operand of the activations (one bulk copy per superblock:
-// the rows kernel below writes it swizzled, scale factors in front), sixteen warps decode.  A UNIT is
-// one superblock of K (256 weights): unit u is decoded by warpgroup u mod 4 into operand buffer u mod 4
-// of TENSOR MEMORY (32 columns of nibbles, 16 of scale factors) and multiplied by four MMAs of K = 64
-// (or eight).  The decoders also move the activations' scale factors to tensor memory: tcgen05.cp takes its
-// issuing thread a hundred clocks each, four or eight per unit.
-// Bound by the decoders' instructions and the latency of the hand-overs between the roles
-// (a tcgen05.mma takes 72 clocks of its issuer whatever its N up to 128, a commit reaches its waiter
-// after about 250), then by shared-memory lookups (4 bytes per codeword from 32 copies: no conflicts).
+// the rows kernel below writes it swizzled, scale factors in front), two issue MMAs, four move the activations'
+// scale factors to tensor memory, sixteen decode.  A UNIT is one superblock of K (256 weights): unit u is
+// decoded by warpgroup u mod 4 into operand buffer u mod 4 of TENSOR MEMORY (32 columns of nibbles, 16 of scale
+// factors) and multiplied by four MMAs of K = 64 (or eight).
+// Bound by the instructions of the decoders, who wait little: a unit of the literal format takes 570 clocks (HBM
+// 260), of K16 660 (430); without loads, lookups and MMAs it would still take 430.  What was tried for the scale factors of
+// the activations: by the decoders (320 of the 2300 clocks a unit then took its warpgroup); tcgen05.cp from two to four
+// warps (shares the tensor pipe with the MMAs: eight copies and eight MMAs of a wide unit 900 clocks).
+// us, before those warps, the uniform issue below, rings of four or eight units for every format and the present
+// stores / now, launches back to back, rows kernel included: 34816 x 5120, 16 rows literal 21.5 / 18.6, K12 26.4 / 22.7, K16 26.6 / 21.9,
+// K20 40.9 / 26.2; 64 rows literal 29.7 / 24.5, 48 rows K16 32.9 / 26.6; 5120 x 17408, 16 rows K16 20.6 / 17.3.
 //
 // A layer with few 128-row tiles is sliced along K over a thread-block cluster: every CTA of the
 // cluster pushes its fp32 sums into the shared memory of the CTA that owns the activation row, which
@@ -42,6 +45,7 @@
 
 #include <cuda.h>
 #include <mutex>
+#include <type_traits>
 
 namespace {
 
@@ -50,13 +54,13 @@ constexpr int kDecWarps = 16;
 constexpr int kCtlWarps = 8;                              // packed rows, activations, up to four MMA issuers, two idle
 constexpr int kThreads = 32 * (kCtlWarps + kDecWarps);
 constexpr int kMaxRows = 64;                              // activation rows per pass (three columns each)
-constexpr int kMaxRaw = 4, kMaxX = 8;
+constexpr int kMaxRaw = 8, kMaxX = 8;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kDynBase = 0x400u;                     // dynamic shared memory starts here (checked); in a
                                                           // cluster the CTA's rank sits in the address's top byte
 constexpr uint32_t kSmemMax = 227 * 1024;
 constexpr uint32_t kSmemEnd = kDynBase + kSmemMax;
-constexpr uint32_t kLut = 0x10000u;                       // shared-window address of the lookup tables
+constexpr uint32_t kLut = 0x800u;                         // shared-window address of the lookup tables, behind the barriers
 constexpr int kMaxRoles = GB_MAX_ROLES;
 constexpr int kMaxSlices = 8;
 
@@ -66,9 +70,9 @@ enum { kLit = 8 };                                        // other formats: the 
 template <int F> struct Fmt {                             // two-tier product format, k = F
   static constexpr int kW0 = (F + 1) / 2, kW1 = F / 2;    // sub-index widths
   static constexpr int kSb = (4 * F + 9 + 15) / 16 * 16;  // slot of a superblock
-  static constexpr int kSbPerStage = F > 16 ? 1 : 2;       // the tables of the wide formats leave less room
+  static constexpr int kSbPerStage = 1;
   static constexpr int kEntries = 1 << kW0;
-  static constexpr int kCopies = kEntries <= 1024 ? 32 : 32 * 1024 / kEntries;
+  static constexpr int kCopies = kEntries <= 512 ? 32 : 16 * 1024 / kEntries;
   static constexpr uint32_t kStride = kCopies * 4;        // bytes between entries: both sub-tables in one word
   static constexpr uint32_t kLutBytes = kEntries * kStride;
   static constexpr uint32_t kScaleTab = 4096;             // E4M3 byte of every (super, sub) pair
@@ -94,7 +98,7 @@ struct Fp4Params {
   int slices;                // = cluster size along y
   int pass_rows;             // most rows per pass (dense: M)
   int x_stages, raw_stages;  // ring depths: 4 or 8, 2 or 4
-  uint32_t x_off, raw_off, misc_off, red_off;
+  uint32_t x_off, raw_off, sf_off, red_off;
   const uint8_t* xop;        // activation operand: [tile][superblock][scale factors | codes]
   int64_t x_unit;            // bytes of one superblock of it
   const float* x_scale;      // [tile][pass_rows] power of two of every row; low bits: where groups are left out
@@ -173,6 +177,12 @@ template <bool kCluster = false>
 GB_DEVINL void wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   if (!(kCluster ? mbar_try_cluster(bar, parity) : mbar_try(bar, parity))) wait_slow<kCluster>(bar, parity, abort_flag, status, code);
 }
+// The same for a whole warp that goes on together; false: given up.
+GB_DEVINL bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  wait_slow<false>(bar, parity, abort_flag, status, code);
+  return !__any_sync(0xffffffffu, *abort_flag != 0);
+}
 GB_DEVINL void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -181,6 +191,17 @@ GB_DEVINL void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1,
 GB_DEVINL void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+GB_DEVINL bool mbar_test(uint32_t bar, uint32_t parity) {   // never suspends: for a look ahead of the wait
+  uint32_t done;
+  asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+GB_DEVINL bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
 }
 GB_DEVINL uint64_t desc_sw128(uint32_t addr) {
   uint64_t d = 0;
@@ -261,15 +282,14 @@ GB_DEVINL uint32_t nib4(uint2 w) {
   return r;
 }
 
-// Who waits for a raw stage.  A warp must see every phase of a barrier it waits for (a parity wait cannot
-// tell a phase from the one two before).  With two superblocks per stage, or four stages, the stages of
-// a slot always hold units of the same warpgroups, so only those wait and hand the stage back; the wide
-// formats (one superblock per stage, room for two stages) let every warpgroup see every stage.
-template <int F> constexpr bool kAllSee = Fmt<F>::kSbPerStage == 1;
+// Sub-indices that are whole bytes (k = 16): a byte permutation drops one into byte 1 of a lookup's address, one
+// instruction instead of two, and the second sub-table's entries are kept in place (bits 16 to 31).  Their
+// tables take 256 bytes an entry, which the wide passes have no room for.  34816 x 5120, 16 rows: 22.9 -> 22.5 us.
+template <int F, bool kWide> constexpr bool kByteCodes = F == 16 && !kWide;
 
 // Lookup tables of one codebook, built by the 512 decoder threads; the order of a thread's stores rotates
 // with it, since the entries of neighbouring threads start in the same bank.
-template <int F>
+template <int F, bool kWide>
 GB_DEVINL void build_lut(const uint16_t* cb, int d, uint32_t lut) {
   if constexpr (F == kLit) {
     const int e = d & 255, half = d >> 8;
@@ -277,6 +297,11 @@ GB_DEVINL void build_lut(const uint16_t* cb, int d, uint32_t lut) {
     const uint32_t w = nib4(make_uint2(q.x, q.y)) | (nib4(make_uint2(q.z, q.w)) << 16);
 #pragma unroll
     for (int j = 0; j < 4; ++j) sts128(lut + (uint32_t)e * 256u + (uint32_t)((half * 4 + j + d) & 7) * 16u, make_uint4(w, w, w, w));
+  } else if constexpr (kByteCodes<F, kWide>) {
+    const int e = d & 255, second = d >> 8;
+    const uint32_t w = nib4(reinterpret_cast<const uint2*>(cb)[d]) << (16 * second);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sts128(lut + (uint32_t)e * 256u + (uint32_t)second * 128u + (uint32_t)((j + d) & 7) * 16u, make_uint4(w, w, w, w));
   } else {
     using T = Fmt<F>;
     const uint2* t0 = reinterpret_cast<const uint2*>(cb);
@@ -294,7 +319,8 @@ GB_DEVINL void build_lut(const uint16_t* cb, int d, uint32_t lut) {
 // Byte offset of the sub-index at bits [bit, bit + width) of the code words, times the entry stride.
 template <int F, int kWidth>
 GB_DEVINL uint32_t entry_offset(const uint32_t* w, int bit, uint32_t lane4) {
-  constexpr int kShift = F == kLit ? 8 : (Fmt<F>::kStride == 128 ? 7 : Fmt<F>::kStride == 64 ? 6 : 5);
+  constexpr int kShift = F == kLit ? 8 : (Fmt<F>::kStride == 128 ? 7 : Fmt<F>::kStride == 64 ? 6 : 4);
+  static_assert(F == kLit || Fmt<F>::kStride == 1 << kShift, "entry stride");
   constexpr uint32_t kMask = ((1u << kWidth) - 1u) << kShift;
   const int i = bit >> 5, s = bit & 31;
   uint32_t x;
@@ -304,13 +330,17 @@ GB_DEVINL uint32_t entry_offset(const uint32_t* w, int bit, uint32_t lane4) {
 }
 
 // Eight weights of codeword c as nibbles.
-template <int F>
+template <int F, bool kWide>
 GB_DEVINL uint32_t codeword(const uint32_t* w, int c, uint32_t lane4) {
   if constexpr (F == kLit) {
     // [lane4's byte 0, code, lane4's bytes 2 and 3]: lane offset, entry, the window's rank byte
     const uint32_t a = c % 4 == 0 ? __byte_perm(w[c / 4], lane4, 0x7604) : c % 4 == 1 ? __byte_perm(w[c / 4], lane4, 0x7614)
                      : c % 4 == 2 ? __byte_perm(w[c / 4], lane4, 0x7624) : __byte_perm(w[c / 4], lane4, 0x7634);
     return lds_imm<kLut>(a);
+  } else if constexpr (kByteCodes<F, kWide>) {
+    const uint32_t a0 = c % 2 == 0 ? __byte_perm(w[c / 2], lane4, 0x7604) : __byte_perm(w[c / 2], lane4, 0x7624);
+    const uint32_t a1 = c % 2 == 0 ? __byte_perm(w[c / 2], lane4, 0x7614) : __byte_perm(w[c / 2], lane4, 0x7634);
+    return lds_imm<kLut>(a0) | lds_imm<kLut + 128>(a1);
   } else {
     using T = Fmt<F>;
     const uint32_t a0 = entry_offset<F, T::kW0>(w, c * F, lane4), a1 = entry_offset<F, T::kW1>(w, c * F + T::kW0, lane4);
@@ -380,7 +410,7 @@ GB_DEVINL float dot16(const RowGroup& r, float x) {
   return s * r.scale;
 }
 
-template <bool kGrouped, int F>
+template <bool kGrouped, bool kWide, int F>
 __global__ void __launch_bounds__(kThreads, 1)
 fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Fp4Params p) {
   using T = Fmt<F>;
@@ -388,17 +418,16 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   extern __shared__ uint8_t smem_raw[];
   // barriers and small state
   const uint32_t win = gb_smem_u32(smem_raw) & 0xFF000000u;
-  const uint32_t misc = p.misc_off | win;
+  const uint32_t misc = kDynBase | win;
   const uint32_t raw_full = misc, raw_empty = misc + 8 * kMaxRaw;
   // per unit slot: activations landed / operand complete / multiplied
-  const uint32_t x_full = misc + 64, full = x_full + 8 * kMaxX, done = full + 8 * kMaxX;
+  const uint32_t x_full = raw_empty + 8 * kMaxRaw, full = x_full + 8 * kMaxX, done = full + 8 * kMaxX;
   const uint32_t acc_full = done + 8 * kMaxX, acc_empty = acc_full + 8, red_full = acc_full + 16;
   const uint32_t slot_addr = acc_full + 24;
-  uint8_t* misc_ptr = smem_raw + (p.misc_off - kDynBase);
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(misc_ptr + (slot_addr - misc));
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(misc_ptr + (slot_addr - misc) + 4);
-  const uint32_t sfa_stage = misc + 512;                   // two-tier: scale bytes of a unit, two buffers of 2 KiB per warpgroup
-  const uint32_t scale_tab = sfa_stage + (F == kLit ? 0u : 16384u);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_raw + (slot_addr - misc));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_raw + (slot_addr - misc) + 4);
+  const uint32_t scale_tab = p.sf_off | win;               // two-tier: the scale table, then
+  const uint32_t sfa_stage = scale_tab + 4096u;            // scale bytes of a unit, two buffers of 2 KiB per warpgroup
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slice = blockIdx.y;
@@ -406,19 +435,22 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const int units = min(p.units, p.n_sb - sb_begin);
   // Units are numbered over all items, an item's count rounded up to whole raw stages: a unit without weights
   // passes every barrier and multiplies nothing.  So the warpgroup, the raw slot and the activation slot of a
-  // unit follow from its number alone, and a warpgroup sees every phase of every barrier that it waits for.
+  // unit follow from its number alone.  A warp must see every phase of a barrier it waits for (a parity wait cannot
+  // tell a phase from the one two before); with four or eight units in a ring, a slot's units are always the same
+  // warpgroup's, so only that one waits for it.
   const int span = (units + T::kSbPerStage - 1) / T::kSbPerStage * T::kSbPerStage;
   // Layout of tensor memory.  Narrow: four accumulators of 64 columns, one per warpgroup and issuer; wide:
   // [hi | dlt] in columns [0, 128), [lo] in [128, 192), one issuer each.  Then the four operand
   // buffers: nibbles (32), weight scale factors (16), activation scale factors (16 per set).
-  const bool wide = is_wide(p.pass_rows);
-  const int n_iss = wide ? 2 : 4;
-  const uint32_t acc_stride = wide ? 128u : 64u;
-  const uint32_t buf_col0 = wide ? 192u : 256u, buf_stride = wide ? 80u : 64u;
-  const int sfx = sf_bytes(wide);
-  const int raw_mask = p.raw_stages - 1, raw_log = p.raw_stages == 4 ? 2 : 1;
+  constexpr bool wide = kWide;
+  constexpr int n_iss = 2;
+  constexpr uint32_t acc_stride = wide ? 128u : 64u;
+  constexpr uint32_t buf_col0 = wide ? 192u : 256u, buf_stride = wide ? 80u : 64u;
+  constexpr int sfx = sf_bytes(wide);
+  // each ring holds four units or eight
+  const int raw_stages = p.raw_stages, raw_two = raw_stages * T::kSbPerStage == 8 ? 1 : 0, raw_log = raw_stages == 8 ? 3 : raw_stages == 4 ? 2 : 1;
   const uint32_t raw_ring = p.raw_off | win;
-  const int x_mask = p.x_stages - 1, x_log = p.x_stages == 8 ? 3 : 2;
+  const int x_two = p.x_stages == 8 ? 1 : 0, x_mask = p.x_stages - 1, x_log = 2 + x_two;
   const uint32_t x_ring = p.x_off | win, x_stage = (uint32_t)p.x_unit;
 
   gb_pdl_launch_dependents();
@@ -429,11 +461,11 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxRaw; ++s) {
       mbar_init(raw_full + 8 * s, 1);
-      mbar_init(raw_empty + 8 * s, kAllSee<F> ? kDecWarps : 4 * T::kSbPerStage);
+      mbar_init(raw_empty + 8 * s, 4 * T::kSbPerStage);
     }
     for (int s = 0; s < kMaxX; ++s) {
       mbar_init(x_full + 8 * s, 1);
-      mbar_init(full + 8 * s, 4);                            // the four warps that decode the unit
+      mbar_init(full + 8 * s, 8);                            // four warps that decode the unit, four that store the scale factors
       mbar_init(done + 8 * s, wide ? 2 : 1);
     }
     mbar_init(acc_full, (uint32_t)n_iss);
@@ -467,7 +499,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     // experts for its tiles, so they are copied next to it (ten tiles a CTA, 500 clocks each from L2)
     if (warp >= kCtlWarps) {
       build_scale_tab<F>(p, threadIdx.x - 32 * kCtlWarps, scale_tab);
-      build_lut<F>(reinterpret_cast<const uint16_t*>(p.codebook), threadIdx.x - 32 * kCtlWarps, kLut | win);
+      build_lut<F, kWide>(reinterpret_cast<const uint16_t*>(p.codebook), threadIdx.x - 32 * kCtlWarps, kLut | win);
       have_role = 0;
     }
     gb_pdl_wait();
@@ -506,82 +538,143 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     return R;
   };
 
+  // The loading and issuing warps walk their loops whole, with values that are the same in every lane, and one elected
+  // lane issues: the operands then stay in uniform registers.  In code that only lane 0 enters an MMA takes 53 clocks to
+  // issue whatever its N; this way 11 (N = 16), 22 (48), 60 (128), and four of N = 48 have completed after 180 clocks instead of 413.
   if (warp == 0) {
     // ------------------------- packed weight rows -------------------------
-    if (lane == 0) {
-      int n = 0;                                           // stages since the start
-      for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
-        const Tile R = tile_at(t);
-        for (int pass = 0; pass < R.n_pass; ++pass)
-          for (int u = 0; u < units; u += T::kSbPerStage, ++n) {
-            const int s = n & raw_mask;
-            wait(raw_empty + 8 * s, ((uint32_t)(n >> raw_log) & 1u) ^ 1u, abort_flag, p.status, 42);
-            if (*abort_flag) continue;                     // no copy may be in flight when the CTA leaves
+    const bool leader = elect_one();
+    int n = 0;                                             // stages since the start
+    bool ok = true;
+    for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
+      const Tile R = tile_at(t);
+      const int n_pass = kGrouped ? __shfl_sync(0xffffffffu, R.n_pass, 0) : 1;
+      for (int pass = 0; pass < n_pass && ok; ++pass)
+        for (int u = 0; u < units; u += T::kSbPerStage, ++n) {
+          const int s = n & (raw_stages - 1);
+          ok = warp_wait(raw_empty + 8 * s, ((uint32_t)(n >> raw_log) & 1u) ^ 1u, abort_flag, p.status, 42);
+          if (!ok) break;                                  // no copy may be in flight when the CTA leaves
+          if (leader) {
             mbar_expect(raw_full + 8 * s, G::kBoxBytes);
             tma_load_2d(raw_ring + (uint32_t)s * G::kBoxBytes, &map_w, (sb_begin + u) * T::kSb, R.w_row0, raw_full + 8 * s);
           }
-      }
+          __syncwarp();
+        }
     }
   } else if (warp == 1) {
     // ------------------------- activation operand --------------------------
-    if (lane == 0) {
-      gb_pdl_wait();
-      int g = 0;                                           // units since the start, over all tiles and passes
-      for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
-        const Tile R = tile_at(t);
-        for (int pass = 0; pass < R.n_pass; ++pass) {
-          const int rows = min(p.pass_rows, R.cnt - pass * p.pass_rows);
-          const uint32_t bytes = (uint32_t)unit_bytes(wide, rows);
-          const uint8_t* src = p.xop + ((int64_t)(R.x_tile + pass) * p.n_sb + sb_begin) * p.x_unit;
-          for (int u = 0; u < span; ++u, ++g, src += p.x_unit) {
-            const int s = g & x_mask;
-            wait(done + 8 * s, ((uint32_t)(g >> x_log) & 1u) ^ 1u, abort_flag, p.status, 43);
-            if (*abort_flag) continue;
-            if (u >= units) { mbar_arrive(x_full + 8 * s); continue; }
-            mbar_expect(x_full + 8 * s, bytes);
-            bulk_load(x_ring + (uint32_t)s * x_stage, src, bytes, x_full + 8 * s);
+    gb_pdl_wait();
+    const bool leader = elect_one();
+    int g = 0;                                             // units since the start, over all tiles and passes
+    bool ok = true;
+    for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
+      const Tile R = tile_at(t);
+      const int n_pass = kGrouped ? __shfl_sync(0xffffffffu, R.n_pass, 0) : 1, cnt = kGrouped ? __shfl_sync(0xffffffffu, R.cnt, 0) : p.M;
+      const int x_tile = kGrouped ? __shfl_sync(0xffffffffu, R.x_tile, 0) : 0;
+      for (int pass = 0; pass < n_pass && ok; ++pass) {
+        const int rows = min(p.pass_rows, cnt - pass * p.pass_rows);
+        const uint32_t bytes = (uint32_t)unit_bytes(wide, rows);
+        const uint8_t* src = p.xop + ((int64_t)(x_tile + pass) * p.n_sb + sb_begin) * p.x_unit;
+        for (int u = 0; u < span; ++u, ++g, src += p.x_unit) {
+          const int s = g & x_mask;
+          ok = warp_wait(done + 8 * s, ((uint32_t)(g >> x_log) & 1u) ^ 1u, abort_flag, p.status, 43);
+          if (!ok) break;
+          if (leader) {
+            if (T::kSbPerStage > 1 && u >= units) {
+              mbar_arrive(x_full + 8 * s);
+            } else {
+              mbar_expect(x_full + 8 * s, bytes);
+              bulk_load(x_ring + (uint32_t)s * x_stage, src, bytes, x_full + 8 * s);
+            }
           }
+          __syncwarp();
         }
       }
     }
-  } else if (warp < kCtlWarps) {
+  } else if (warp < 4) {
     // ------------------------- MMA issuers ---------------------------------
-    // Narrow: issuer i takes the units of warpgroup i into accumulator i.  Wide: issuer 0 multiplies every
-    // unit with [hi | dlt], issuer 1 with [lo].
-    const int i = warp - 2;
-    if (lane == 0 && i < n_iss) {
-      const uint32_t acc = tmem_base + (uint32_t)i * acc_stride;
-      const uint32_t sf_col = 48u + (wide ? (uint32_t)i * 16u : 0u);
-      const int u_step = wide ? 1 : 4;
-      const uint64_t db0 = desc_sw128(x_ring + (uint32_t)sfx);
-      int g0 = 0, item = 0;                                // units / (tile, pass) items since the start
-      for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
-        const Tile R = tile_at(t);
-        for (int pass = 0; pass < R.n_pass; ++pass, ++item, g0 += span) {
-          const int rows = min(p.pass_rows, R.cnt - pass * p.pass_rows);
-          const int n = wide && i == 1 ? term_rows(true, rows) : mma_cols(wide, rows);
-          // E2M1 x E2M1, UE4M3 scale factors, both K-major, fp32 accumulate; N >> 3, M >> 4
-          const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-          if (item > 0) {
-            wait(acc_empty, (item - 1) & 1, abort_flag, p.status, 44);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          }
-          const int u_first = wide ? 0 : (i - g0) & 3;
-          for (int u = u_first; u < span; u += u_step) {
-            const int g = g0 + u, s = g & x_mask;
-            const uint32_t a = tmem_base + buf_col0 + (uint32_t)(g & 3) * buf_stride, off = (uint32_t)s * x_stage;
-            const uint64_t db = db0 + (uint64_t)(off >> 4);
-            wait(full + 8 * s, (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 45);
-            if (*abort_flag) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // Narrow: issuer i takes every other unit, into the accumulator of its warpgroup.  Wide: issuer 0 multiplies
+    // every unit with [hi | dlt], issuer 1 with [lo].
+    const int i = __shfl_sync(0xffffffffu, warp, 0) - 2;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const bool leader = elect_one();
+    constexpr int u_step = wide ? 1 : 2;
+    const uint32_t sf_col = 48u + (wide ? (uint32_t)i * 16u : 0u);
+    const uint64_t db0 = desc_sw128(x_ring + (uint32_t)sfx);
+    int g0 = 0, item = 0;                                  // units / (tile, pass) items since the start
+    bool gone = false;
+    for (int t = blockIdx.x; t < p.n_tiles && !gone; t += gridDim.x) {
+      const Tile R = tile_at(t);
+      const int n_pass = kGrouped ? __shfl_sync(0xffffffffu, R.n_pass, 0) : 1, cnt = kGrouped ? __shfl_sync(0xffffffffu, R.cnt, 0) : p.M;
+      for (int pass = 0; pass < n_pass && !gone; ++pass, ++item, g0 += span) {
+        const int rows = min(p.pass_rows, cnt - pass * p.pass_rows);
+        const int n = wide && i == 1 ? term_rows(true, rows) : mma_cols(wide, rows);
+        // E2M1 x E2M1, UE4M3 scale factors, both K-major, fp32 accumulate; N >> 3, M >> 4
+        const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+        if (item > 0) {
+          wait(acc_empty, (item - 1) & 1, abort_flag, p.status, 44);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        for (int u = wide ? 0 : (i - g0) & 1; u < span; u += u_step) {
+          const int g = g0 + u, s = g & x_mask;
+          const uint32_t acc = tmem + (uint32_t)(wide ? i : g & 3) * acc_stride;
+          const uint32_t a = tmem + buf_col0 + (uint32_t)(g & 3) * buf_stride, off = (uint32_t)s * x_stage;
+          const uint64_t db = db0 + (uint64_t)(off >> 4);
+          if (!warp_wait(full + 8 * s, (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 45)) { gone = true; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (leader) {
+            if (T::kSbPerStage == 1 || u < units) {
 #pragma unroll
-            for (int k = 0; k < (u < units ? 4 : 0); ++k)
-              umma_fp4_ts(acc, a + 8u * k, db + (uint64_t)(2 * k), idesc, a + 32u + 4u * k, a + sf_col + 4u * k, u > u_first || k > 0);
+              for (int k = 0; k < 4; ++k)
+                umma_fp4_ts(acc, a + 8u * k, db + (uint64_t)(2 * k), idesc, a + 32u + 4u * k, a + sf_col + 4u * k, u >= (wide ? 1 : 4) || k > 0);
+            }
             umma_commit(done + 8 * s);
           }
-          umma_commit(acc_full);
+          __syncwarp();
         }
+        if (leader) umma_commit(acc_full);
+        __syncwarp();
       }
+    }
+  } else if (warp < kCtlWarps) {
+    // ------------------------- activation scale factors ---------------------
+    // From shared to tensor memory, one warp per lane quarter: atom k is what MMA k reads, its line l the four columns
+    // of lane l of every quarter.
+    // The next unit's are read while the stores of this one complete: every unit passes these four warps.
+    const uint32_t sf_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + buf_col0 + 48u;
+    int64_t total = 0;                                     // units of the CTA
+    for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) total += (kGrouped ? tile_at(t).n_pass : 1) * span;
+    const int n_units = (int)total;
+    uint32_t v[wide ? 2 : 1][16];
+    auto arrived = [&](int g) { return mbar_test(x_full + 8 * (g & x_mask), (uint32_t)(g >> x_log) & 1u); };
+    auto fetch = [&](int g) {                              // (a unit without weights reads what an earlier one left)
+      const uint32_t sx = x_ring + (uint32_t)(g & x_mask) * x_stage + (uint32_t)lane * 16u;
+#pragma unroll
+      for (int k = 0; k < (wide ? 8 : 4); ++k) {
+        const uint4 q = lds128(sx + 512u * k);
+        uint32_t* o = &v[k >> 2][4 * (k & 3)];
+        o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
+      }
+    };
+    bool have = false;
+    for (int g = 0; g < n_units; ++g) {
+      const int s = g & x_mask;
+      const bool free = g < 4 || mbar_test(done + 8 * ((g - 4) & x_mask), (uint32_t)((g - 4) >> x_log) & 1u);
+      if (!have) {
+        wait(x_full + 8 * s, (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 46);
+        fetch(g);
+      }
+      if (!free) wait(done + 8 * ((g - 4) & x_mask), (uint32_t)((g - 4) >> x_log) & 1u, abort_flag, p.status, 52);
+      const uint32_t col = sf_base + (uint32_t)(g & 3) * buf_stride;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tmem_st16(col, v[0]);
+      if constexpr (wide) tmem_st16(col + 16u, v[1]);
+      have = __all_sync(0xffffffffu, arrived(g + 1)) && g + 1 < n_units;
+      if (have) fetch(g + 1);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + 8 * s);
     }
   } else {
     // ------------------------- decoders -------------------------------------
@@ -590,12 +683,20 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const int row = quarter * 32 + lane;                     // weight row of the tile = tensor-memory lane
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t buf = lane_base + buf_col0 + (uint32_t)wg * buf_stride;
-    const uint32_t lane4 = win | (F == kLit ? (uint32_t)lane * 4u : (uint32_t)(lane & ((int)(T::kStride / 4) - 1)) * 4u);
+    const uint32_t lane4 = win | (F == kLit || kByteCodes<F, kWide> ? (uint32_t)lane * 4u : (uint32_t)(lane & ((int)(T::kStride / 4) - 1)) * 4u);
     if (!kGrouped) build_scale_tab<F>(p, d, scale_tab);
     bool waited = false;
     float xs0 = 0.0f, xs1 = 0.0f;                            // scale words of rows lane, lane + 32
-    int item = 0, g0 = 0, n0 = 0;                            // items, units and raw stages so far
-    uint32_t flip = 0;
+    int item = 0, g0 = 0;                                    // items and units so far
+    // This warpgroup's units are wg, wg + 4, ..; the j-th of them:
+    int g = wg, j = 0;
+    const uint32_t raw_slot = (uint32_t)(wg / T::kSbPerStage), raw_step = 4u / T::kSbPerStage;   // raw slots: first, to the second
+    const uint32_t raw_row = raw_ring + raw_slot * G::kBoxBytes + (uint32_t)(wg % T::kSbPerStage) * T::kSb;
+    auto raw_bar = [&](uint32_t base, int n) { return base + 8u * (raw_slot + raw_step * (uint32_t)(n & raw_two)); };
+    auto raw_phase = [&](int n) { return (uint32_t)(n >> raw_two) & 1u; };
+    auto x_bar = [&](uint32_t base, int n) { return base + 8u * ((uint32_t)wg + 4u * (uint32_t)(n & x_two)); };
+    auto x_phase = [&](int n) { return (uint32_t)(n >> x_two) & 1u; };
+    bool raw_ok = false;                                     // the next unit's rows have been seen to be there
     // An item's accumulators are read out after the warpgroup has decoded its first unit of the NEXT item:
     // the last multiplications, their completion and the read-out then overlap decoding, and the next
     // item's multiplications find their operands ready.  (Nothing that first unit waits for needs this
@@ -613,126 +714,105 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       const bool live = t < p.n_tiles;
       if (live && R.role != have_role) {                     // the CTA's rows change codebook
         if (have_role >= 0) asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
-        build_lut<F>(reinterpret_cast<const uint16_t*>(p.codebook) + p.role[R.role].cb, d, kLut | win);
+        build_lut<F, kWide>(reinterpret_cast<const uint16_t*>(p.codebook) + p.role[R.role].cb, d, kLut | win);
         have_role = R.role;
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
       }
-      if (!waited) {                                         // y may still be read by the launch ahead
-        gb_pdl_wait();
-        waited = true;
-        if (!kGrouped) {
-          xs0 = lane < p.M ? p.x_scale[lane] : 0.0f;
-          xs1 = lane + 32 < p.M ? p.x_scale[lane + 32] : 0.0f;
-        }
-      }
       {
-        const int u_end = live ? span : 0, u_step = kAllSee<F> ? 1 : 4;
-        int u = kAllSee<F> ? 0 : (wg - g0) & 3;
+        const int g_end = live ? g0 + span : g0;
 #pragma unroll 1
         do {
-          const int n = n0 + u / T::kSbPerStage, rs = n & raw_mask;
-          const bool mine = !kAllSee<F> || ((g0 + u) & 3) == wg;
-          if (u < u_end && !mine) {
-            wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
-            if (lane == 0) mbar_arrive(raw_empty + 8 * rs);
-          }
-          if (mine && u >= units && u < u_end) {             // a stage's missing second superblock
-            wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
-            const int g = g0 + u;
-            if (g >= 4) wait(done + 8 * ((g - 4) & x_mask), (uint32_t)((g - 4) >> x_log) & 1u, abort_flag, p.status, 48);
-            wait(x_full + 8 * (g & x_mask), (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 46);
-            if (lane == 0) { mbar_arrive(raw_empty + 8 * rs); mbar_arrive(full + 8 * (g & x_mask)); }
-          }
-          if (mine && u < units && live) {
-            wait(raw_full + 8 * rs, (uint32_t)(n >> raw_log) & 1u, abort_flag, p.status, 47);
-            const uint32_t stage = raw_ring + (uint32_t)rs * G::kBoxBytes + (uint32_t)(u % T::kSbPerStage) * T::kSb;
-            const uint32_t rp = stage + (uint32_t)row * G::kPitch;
-            uint32_t v[32], sfa[16], sg, sg_step;            // sfa: scale words of rows lane, lane + 32, lane + 64, lane + 96
-            if constexpr (F == kLit) {
-              const uint4 c0 = lds128(rp), c1 = lds128(rp + 16), own = lds128(rp + 32);
-              const uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+          if (g < g_end) {
+            if (!raw_ok) wait(raw_bar(raw_full, j), raw_phase(j), abort_flag, p.status, 47);
+            // The buffer's last unit has been multiplied: looked at early, waited for where it matters.  The slot's next
+            // completion is a later unit of this warpgroup, so it cannot run ahead of this wait.
+            bool free = j == 0;
+            if (T::kSbPerStage == 1 || g - g0 < units) {
+              const uint32_t stage = raw_row + (uint32_t)(j & raw_two) * (raw_step * G::kBoxBytes);
+              const uint32_t rp = stage + (uint32_t)row * G::kPitch;
+              uint32_t v[32], sfa[16], sg;                   // sfa: scale words of rows lane, lane + 32, lane + 64, lane + 96
+              constexpr uint32_t sg_step = F == kLit ? 32u * G::kPitch : 512u;
+              if constexpr (F == kLit) {
+                const uint4 c0 = lds128(rp), c1 = lds128(rp + 16), own = lds128(rp + 32);
+                if (j > 0) free = mbar_test(x_bar(done, j - 1), x_phase(j - 1));
+                const uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
-              for (int c = 0; c < 32; ++c) v[c] = codeword<F>(cw, c, lane4);
-              if (__builtin_expect((own.x | own.y | own.z | own.w) & 0x80808080u, 0)) {
-                // scale factors carry no sign: it moves into the nibbles
-                const uint32_t os[4] = {own.x, own.y, own.z, own.w};
+                for (int c = 0; c < 32; ++c) v[c] = codeword<F, kWide>(cw, c, lane4);
+                if (__builtin_expect((own.x | own.y | own.z | own.w) & 0x80808080u, 0)) {
+                  // scale factors carry no sign: it moves into the nibbles
+                  const uint32_t os[4] = {own.x, own.y, own.z, own.w};
 #pragma unroll
-                for (int g = 0; g < 16; ++g) {
-                  const uint32_t neg = (os[g >> 2] >> (8 * (g & 3))) & 0x80u ? 0x88888888u : 0u;
-                  v[2 * g] ^= neg;
-                  v[2 * g + 1] ^= neg;
+                  for (int q = 0; q < 16; ++q) {
+                    const uint32_t neg = (os[q >> 2] >> (8 * (q & 3))) & 0x80u ? 0x88888888u : 0u;
+                    v[2 * q] ^= neg;
+                    v[2 * q + 1] ^= neg;
+                  }
                 }
+                sg = stage + (uint32_t)lane * G::kPitch + 32u;
+              } else {
+                uint32_t w[T::kSb / 4];
+#pragma unroll
+                for (int q = 0; q < T::kSb / 16; ++q) {
+                  const uint4 x = lds128(rp + 16u * q);
+                  w[4 * q] = x.x; w[4 * q + 1] = x.y; w[4 * q + 2] = x.z; w[4 * q + 3] = x.w;
+                }
+                if (j > 0) free = mbar_test(x_bar(done, j - 1), x_phase(j - 1));
+                // the super byte sits right behind the 4k index bytes, then sixteen nibbles
+                const uint4 tb = lds128(scale_tab + (w[F] & 0xFFu) * 16u);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(raw_bar(raw_empty, j));  // the whole superblock is in registers
+                const uint32_t n0s = __funnelshift_r(w[F], w[F + 1], 8), n1s = __funnelshift_r(w[F + 1], w[F + 2], 8);
+                // two buffers: a warp that writes the next unit's bytes has passed this unit's barrier,
+                // which no warp reaches before it has read the unit before
+                const uint32_t st = sfa_stage + (uint32_t)(wg * 4096) + (uint32_t)(j & 1) * 2048u;
+                sts128(st + (uint32_t)(row * 16),
+                       make_uint4(four_scales(tb, n0s), four_scales(tb, n0s >> 16), four_scales(tb, n1s), four_scales(tb, n1s >> 16)));
+#pragma unroll
+                for (int c = 0; c < 32; ++c) v[c] = codeword<F, kWide>(w, c, lane4);
+                asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory");   // the four warps of this warpgroup
+                sg = st + (uint32_t)lane * 16u;
               }
-              sg = stage + (uint32_t)lane * G::kPitch + 32u;
-              sg_step = 32u * G::kPitch;
-            } else {
-              uint32_t w[T::kSb / 4];
+              if (!free) wait(x_bar(done, j - 1), x_phase(j - 1), abort_flag, p.status, 48);
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              tmem_st32(buf, v);
+              uint32_t any = 0;
 #pragma unroll
-              for (int q = 0; q < T::kSb / 16; ++q) {
-                const uint4 x = lds128(rp + 16u * q);
-                w[4 * q] = x.x; w[4 * q + 1] = x.y; w[4 * q + 2] = x.z; w[4 * q + 3] = x.w;
+              for (int q = 0; q < 4; ++q) {
+                const uint4 s = lds128(sg + (uint32_t)q * sg_step);
+                sfa[q] = s.x; sfa[4 + q] = s.y; sfa[8 + q] = s.z; sfa[12 + q] = s.w;
+                any |= s.x | s.y | s.z | s.w;
               }
-              __syncwarp();
-              if (lane == 0) mbar_arrive(raw_empty + 8 * rs);  // the whole superblock is in registers
-              // the super byte sits right behind the 4k index bytes, then sixteen nibbles
-              const uint4 tb = lds128(scale_tab + (w[F] & 0xFFu) * 16u);
-              const uint32_t n0s = __funnelshift_r(w[F], w[F + 1], 8), n1s = __funnelshift_r(w[F + 1], w[F + 2], 8);
-              // two buffers: a warp that writes the next unit's bytes has passed this unit's barrier,
-              // which no warp reaches before it has read the unit before
-              const uint32_t st = sfa_stage + (uint32_t)(wg * 4096) + flip * 2048u;
-              flip ^= 1u;
-              sts128(st + (uint32_t)(row * 16),
-                     make_uint4(four_scales(tb, n0s), four_scales(tb, n0s >> 16), four_scales(tb, n1s), four_scales(tb, n1s >> 16)));
+              if (F == kLit && __builtin_expect(any & 0x80808080u, 0)) {
 #pragma unroll
-              for (int c = 0; c < 32; ++c) v[c] = codeword<F>(w, c, lane4);
-              asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory");   // the four warps of this warpgroup
-              sg = st + (uint32_t)lane * 16u;
-              sg_step = 512u;
-            }
-            // The buffer's last unit has been multiplied.  The slot's next completion is a later unit of this warpgroup, so it cannot run ahead of this wait.
-            const int g = g0 + u;
-            if (g >= 4) wait(done + 8 * ((g - 4) & x_mask), (uint32_t)((g - 4) >> x_log) & 1u, abort_flag, p.status, 48);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            tmem_st32(buf, v);
-            uint32_t any = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint4 s = lds128(sg + (uint32_t)j * sg_step);
-              sfa[j] = s.x; sfa[4 + j] = s.y; sfa[8 + j] = s.z; sfa[12 + j] = s.w;
-              any |= s.x | s.y | s.z | s.w;
-            }
-            if (F == kLit && __builtin_expect(any & 0x80808080u, 0)) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) sfa[j] &= 0x7F7F7F7Fu;
-            }
-            tmem_st16(buf + 32u, sfa);
-            // the activations' scale factors: atom k is what MMA k reads, its line l the four columns of
-            // lane l of every quarter
-            wait(x_full + 8 * (g & x_mask), (uint32_t)(g >> x_log) & 1u, abort_flag, p.status, 46);
-            const uint32_t sx = x_ring + (uint32_t)(g & x_mask) * x_stage + (uint32_t)lane * 16u;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint4 s = lds128(sx + 512u * k);
-              sfa[4 * k] = s.x; sfa[4 * k + 1] = s.y; sfa[4 * k + 2] = s.z; sfa[4 * k + 3] = s.w;
-            }
-            tmem_st16(buf + 48u, sfa);
-            if (wide) {
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const uint4 s = lds128(sx + 2048u + 512u * k);
-                sfa[4 * k] = s.x; sfa[4 * k + 1] = s.y; sfa[4 * k + 2] = s.z; sfa[4 * k + 3] = s.w;
+                for (int q = 0; q < 16; ++q) sfa[q] &= 0x7F7F7F7Fu;
               }
-              tmem_st16(buf + 64u, sfa);
+              tmem_st16(buf + 32u, sfa);
+              raw_ok = mbar_test(raw_bar(raw_full, j + 1), raw_phase(j + 1));
+              asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            } else {                                         // a stage's missing second superblock
+              if (!free) wait(x_bar(done, j - 1), x_phase(j - 1), abort_flag, p.status, 48);
+              raw_ok = false;
             }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(full + 8 * (g & x_mask));
+            if (lane == 0) {
+              mbar_arrive(x_bar(full, j));
+              if (F == kLit) mbar_arrive(raw_bar(raw_empty, j));
+            }
+            g += 4;
+            ++j;
           }
-          if (F == kLit && mine && u < units && live && lane == 0) mbar_arrive(raw_empty + 8 * rs);
-          if (out_t >= 0 && (mine || u + u_step >= u_end)) {
+          if (out_t >= 0) {
             // ------------------------- read-out ------------------------------------
             // Sums into registers, the accumulators handed back, then the stores.
+            if (!waited) {                                   // the rows' scales come from the launch ahead, which may still read y
+              gb_pdl_wait();
+              waited = true;
+              if (!kGrouped) {
+                xs0 = lane < p.M ? p.x_scale[lane] : 0.0f;
+                xs1 = lane + 32 < p.M ? p.x_scale[lane + 32] : 0.0f;
+              }
+            }
             const Tile Q = tile_at(out_t);
             const int rows = min(p.pass_rows, Q.cnt - out_pass * p.pass_rows);
             int to0 = lane, to1 = lane + 32;                 // output rows
@@ -754,8 +834,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             const bool ok = *abort_flag == 0;
             if (__builtin_expect(__any_sync(0xffffffffu, (__float_as_uint(xs0) | __float_as_uint(xs1)) & kGbLeftOutBits), 0)) {
               // Groups left out: added to the sums in tensor memory, by the warps that read those out.  (Spread over the
-              // warpgroups they would have to wait for each other here, while the formats whose raw stages
-              // every warpgroup sees need all of them to go on.)  17408 x 5120, K16, 16 rows, 15.6 us: one tiny group in
+              // warpgroups they would have to wait for each other here.)  17408 x 5120, K16, 16 rows, 15.6 us: one tiny group in
               // one row 17.1, an outlier channel in all rows 19.0, one row over 2^30 165, all of them 556.  Inline and
               // with nothing held over it: as a function, or with the sums in registers, it cost the ordinary read-out
               // its registers (two layers at 16 rows 164 -> 188..208 us, this way 167..169).
@@ -836,32 +915,56 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty);
-            auto emit = [&](int m, float total) {
-              const float scale = __uint_as_float(__float_as_uint(__shfl_sync(0xffffffffu, m < 32 ? xs0 : xs1, m & 31)) & kGbRowScaleMask);
-              const int orow = __shfl_sync(0xffffffffu, m < 32 ? to0 : to1, m & 31);
-              if (m >= rows) return;
-              const float val = total * scale;
+            // kRows rows from m0 on.  Their scales in one or two loads: a shuffle, a mask and a selection per row, and a division by the
+            // slice count, made 190 clocks a row of these stores (64 rows, 34816 x 5120: 3 us of each tile).
+            auto emit = [&](auto n_rows, int m0, const float* total) {
+              constexpr int kRows = decltype(n_rows)::value;
+              if (m0 >= rows) return;
+              const uint4* words = reinterpret_cast<const uint4*>(p.x_scale + (kGrouped ? (int64_t)(Q.x_tile + q_pass) * p.pass_rows : 0) + m0);
+              float val[kRows];
+#pragma unroll
+              for (int q = 0; q < kRows / 4; ++q) {
+                const uint4 w = words[q];
+                val[4 * q] = total[4 * q] * __uint_as_float(w.x & kGbRowScaleMask);
+                val[4 * q + 1] = total[4 * q + 1] * __uint_as_float(w.y & kGbRowScaleMask);
+                val[4 * q + 2] = total[4 * q + 2] * __uint_as_float(w.z & kGbRowScaleMask);
+                val[4 * q + 3] = total[4 * q + 3] * __uint_as_float(w.w & kGbRowScaleMask);
+              }
               if (!kGrouped && p.slices > 1) {
                 // into the shared memory of the row's owner: slot [row / slices][slice][128 weight rows]
-                uint32_t dst;
-                const uint32_t local = (p.red_off | win) + (uint32_t)(((m / p.slices) * p.slices + slice) * kBM + row) * 4u;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(local), "r"(m % p.slices));
-                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(val) : "memory");
-              } else if (ok && col < Q.n_end) {
-                p.y[(int64_t)orow * p.N + col] = (uint16_t)gb_f32_to_bf16_bits(val * p.global_scale);
+                int own = m0 / p.slices, to = m0 - own * p.slices;
+#pragma unroll
+                for (int i = 0; i < kRows; ++i) {
+                  if (m0 + i < rows) {
+                    uint32_t dst;
+                    const uint32_t local = (p.red_off | win) + (uint32_t)((own * p.slices + slice) * kBM + row) * 4u;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(local), "r"(to));
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(val[i]) : "memory");
+                  }
+                  if (++to == p.slices) { to = 0; ++own; }
+                }
+              } else {
+                const bool mine = ok && col < Q.n_end;
+                uint16_t* y = p.y + (kGrouped ? 0 : (int64_t)m0 * p.N) + col;
+#pragma unroll
+                for (int i = 0; i < kRows; ++i) {
+                  const int m = m0 + i;
+                  const uint16_t b = (uint16_t)gb_f32_to_bf16_bits(val[i] * p.global_scale);
+                  if (kGrouped) {
+                    const int orow = __shfl_sync(0xffffffffu, m < 32 ? to0 : to1, m & 31);
+                    if (m < rows && mine) y[(int64_t)orow * p.N] = b;
+                  } else {
+                    if (m < rows && mine) *y = b;
+                    y += p.N;
+                  }
+                }
               }
             };
             if (wide) {
-#pragma unroll
-              for (int j = 0; j < 2; ++j) {
-                const int c = wg + 4 * j;
-                if (c * 8 >= rows) break;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) emit(c * 8 + i, sum[8 * j + i]);
-              }
-            } else if (wg * 4 < rows) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) emit(wg * 4 + i, sum[i]);
+              emit(std::integral_constant<int, 8>(), wg * 8, sum);
+              emit(std::integral_constant<int, 8>(), wg * 8 + 32, sum + 8);
+            } else {
+              emit(std::integral_constant<int, 4>(), wg * 4, sum);
             }
             if (!kGrouped && p.slices > 1) {
               // every warp tells every CTA of the cluster that its sums are in place, then the owners add
@@ -885,15 +988,13 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
               }
             }
           }
-          u += u_step;
-        } while (u < u_end);
+        } while (g < g_end);
       }
       if (!live) break;
       out_t = t;
       out_pass = pass;
       ++item;
       g0 += span;
-      n0 += span / T::kSbPerStage;
       if (++pass >= R.n_pass) {
         pass = 0;
         t += gridDim.x;
@@ -1251,49 +1352,43 @@ int fp4_format(const gb_weight* w, bool scales_e4m3) {
 }
 
 struct Info { int sb, per_stage, pitch; uint32_t box, lut, extra; };
-template <int F> Info info_of() {
-  return {Fmt<F>::kSb, Fmt<F>::kSbPerStage, Geo<F>::kPitch, (uint32_t)Geo<F>::kBoxBytes, Fmt<F>::kLutBytes,
+template <int F> Info info_of(bool wide) {
+  const uint32_t lut = (wide ? kByteCodes<F, true> : kByteCodes<F, false>) ? 256 * 256 : Fmt<F>::kLutBytes;
+  return {Fmt<F>::kSb, Fmt<F>::kSbPerStage, Geo<F>::kPitch, (uint32_t)Geo<F>::kBoxBytes, lut,
           Fmt<F>::kScaleTab + (F == kLit ? 0u : 16384u)};
 }
-Info info(int F) {
+Info info(int F, bool wide) {
   switch (F) {
-    case kLit: return info_of<kLit>();
-    case 12: return info_of<12>();
-    case 16: return info_of<16>();
-    case 20: return info_of<20>();
-    default: return info_of<24>();
+    case kLit: return info_of<kLit>(wide);
+    case 12: return info_of<12>(wide);
+    case 16: return info_of<16>(wide);
+    case 20: return info_of<20>(wide);
+    default: return info_of<24>(wide);
   }
 }
 
-// Shared memory: [kDynBase, kLut) and [behind the tables, end).  The activation ring holds eight units where
-// they fit beside two raw stages, else four (a unit's slot and its operand buffer are handed back by
-// one barrier, so only multiples of the four buffers work); what is left goes to the raw ring (four stages or
-// two).
+// Shared memory: barriers, tables, then the rings and what else the launch needs.  Both rings hold eight units
+// where they fit, else four (kernel: only these keep a slot's units with one warpgroup); the activations'
+// first, whose way round (multiplied, asked for, loaded) is the longer one.
 bool layout(const Info& f, Fp4Params& p) {
-  for (p.x_stages = 8; p.x_stages >= 4; p.x_stages -= 4) {
-    struct Region { uint32_t at, end; } reg[2] = {{kDynBase, kLut}, {kLut + f.lut, kSmemEnd}};
-    auto take = [&](uint32_t bytes, uint32_t align, uint32_t* out) {
-      for (int r = 0; r < 2; ++r) {
-        const uint32_t a = (reg[r].at + align - 1) & ~(align - 1);
-        if (a + bytes <= reg[r].end) { *out = a; reg[r].at = a + bytes; return true; }
-      }
-      return false;
-    };
-    if (!take((uint32_t)(p.x_stages * p.x_unit), 1024, &p.x_off)) continue;
-    if (!take(512 + f.extra, 128, &p.misc_off)) continue;
-    const uint32_t red = p.slices > 1 ? (uint32_t)((p.M + p.slices - 1) / p.slices * p.slices * kBM * 4) : 0u;
-    // the raw ring first: in front of it the sums could leave room for two stages only (5120 x 17408, sixteen
-    // rows: 21 us instead of 15.7)
-    for (p.raw_stages = kMaxRaw; p.raw_stages >= 2; p.raw_stages >>= 1) {
-      const Region keep[2] = {reg[0], reg[1]};
-      if (take(f.box * (uint32_t)p.raw_stages, 128, &p.raw_off) && (red == 0 || take(red, 128, &p.red_off))) {
-        if (p.E > 0 && !take(4u * (uint32_t)(p.E + 1), 128, &p.seg_off)) p.seg_off = 0;
-        return true;
-      }
-      reg[0] = keep[0];
-      reg[1] = keep[1];
+  const uint32_t red = p.slices > 1 ? (uint32_t)((p.M + p.slices - 1) / p.slices * p.slices * kBM * 4) : 0u;
+  for (p.x_stages = 8; p.x_stages >= 4; p.x_stages -= 4)
+    for (p.raw_stages = 8 / f.per_stage; p.raw_stages * f.per_stage >= 4; p.raw_stages >>= 1) {
+      uint32_t at = kLut + f.lut;
+      auto take = [&](uint32_t bytes, uint32_t align) {
+        const uint32_t a = (at + align - 1) & ~(align - 1);
+        at = a + bytes;
+        return a;
+      };
+      p.x_off = take((uint32_t)(p.x_stages * p.x_unit), 1024);
+      p.raw_off = take(f.box * (uint32_t)p.raw_stages, 128);
+      p.sf_off = take(f.extra, 128);
+      p.red_off = take(red, 128);
+      if (at > kSmemEnd) continue;
+      p.seg_off = p.E > 0 ? take(4u * (uint32_t)(p.E + 1), 128) : 0;
+      if (at > kSmemEnd) p.seg_off = 0;
+      return true;
     }
-  }
   return false;
 }
 
@@ -1315,7 +1410,7 @@ int max_clusters(int size) {
     attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)size; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, fp4_decode_kernel<false, kLit>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); return 0; }
+    if (cudaOccupancyMaxActiveClusters(&n, fp4_decode_kernel<false, false, kLit>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); return 0; }
   }
   return n;
 }
@@ -1341,12 +1436,17 @@ cudaError_t launch(int F, dim3 grid, cudaStream_t stream, const CUtensorMap& map
   cfg.attrs = attr;
   cfg.numAttrs = n;
   gb_count_launch();
+  const bool wide = is_wide(p.pass_rows);
   switch (F) {
-    case kLit: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, kLit>, map_w, p);
-    case 12: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, 12>, map_w, p);
-    case 16: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, 16>, map_w, p);
-    case 20: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, 20>, map_w, p);
-    default: return cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, 24>, map_w, p);
+#define GB_FP4_LAUNCH(f)                                                                       \
+  return wide ? cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, true, f>, map_w, p)       \
+              : cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, false, f>, map_w, p)
+    case kLit: GB_FP4_LAUNCH(kLit);
+    case 12: GB_FP4_LAUNCH(12);
+    case 16: GB_FP4_LAUNCH(16);
+    case 20: GB_FP4_LAUNCH(20);
+    default: GB_FP4_LAUNCH(24);
+#undef GB_FP4_LAUNCH
   }
 }
 
@@ -1397,15 +1497,15 @@ int64_t align256(int64_t v) { return (v + 255) & ~255ll; }
 }  // namespace
 
 int gb_prepare_gemv_fp4() {
-#define GB_FP4_ATTR(F)                                                                                                     \
-  GB_CUDA_OK(cudaFuncSetAttribute((const void*)fp4_decode_kernel<false, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax)); \
-  GB_CUDA_OK(cudaFuncSetAttribute((const void*)fp4_decode_kernel<true, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax))
+#define GB_FP4_ATTR1(G, W, F) GB_CUDA_OK(cudaFuncSetAttribute((const void*)fp4_decode_kernel<G, W, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax))
+#define GB_FP4_ATTR(F) GB_FP4_ATTR1(false, false, F); GB_FP4_ATTR1(false, true, F); GB_FP4_ATTR1(true, false, F); GB_FP4_ATTR1(true, true, F)
   GB_FP4_ATTR(kLit);
   GB_FP4_ATTR(12);
   GB_FP4_ATTR(16);
   GB_FP4_ATTR(20);
   GB_FP4_ATTR(24);
 #undef GB_FP4_ATTR
+#undef GB_FP4_ATTR1
   return GB_OK;
 }
 
@@ -1429,7 +1529,7 @@ int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, 
   if (workspace == nullptr || workspace_bytes < gb_gemv_fp4_workspace_bytes(M, w->K))
     return gb_fail(GB_EWORKSPACE, "workspace of %lld bytes is too small (need %lld)", (long long)workspace_bytes,
                    (long long)gb_gemv_fp4_workspace_bytes(M, w->K));
-  const Info f = info(F);
+  const Info f = info(F, is_wide((int)(M < kMaxRows ? M : kMaxRows)));
   cudaStream_t stream = (cudaStream_t)stream_;
   CUtensorMap map_w;
   int rc = gb_tensor_map_bytes_2d(&map_w, w->qw, (uint64_t)(w->K / 256) * f.sb, (uint64_t)w->rows, (uint64_t)w->row_stride, f.pitch, kBM);
@@ -1468,7 +1568,7 @@ int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, 
     p.units = (p.n_sb + want - 1) / want;
     p.units = (p.units + f.per_stage - 1) / f.per_stage * f.per_stage;
     p.slices = (p.n_sb + p.units - 1) / p.units;
-    if (!layout(f, p)) return gb_fail(GB_EUNSUPPORTED, "no shared-memory layout for %d rows", p.M);
+    if (!layout(info(F, is_wide(p.M)), p)) return gb_fail(GB_EUNSUPPORTED, "no shared-memory layout for %d rows", p.M);
     RowsParams rp = {};
     rp.x = (const uint4*)((const uint16_t*)x + m0 * w->K);
     rp.xop = (uint8_t*)workspace;
@@ -1629,7 +1729,7 @@ int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, in
     return gb_fail(GB_EUNSUPPORTED, "not a stack the fp4 expert kernel takes");
   const int sms = gb_sm_count();
   if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
-  const Info f = info(F);
+  const Info f = info(F, is_wide(pass_rows));
   const int64_t tiles = P / pass_rows + E + 1;
   Fp4Params p = {};
   p.N = N; p.K = K; p.n_sb = (int)(K / 256); p.units = p.n_sb; p.slices = 1;

@@ -313,3 +313,19 @@ def test_left_out_groups_between_tiles_of_one_cta(dev, name, T):
     # by up to a third; a row whose small groups were dropped is off by its whole length.
     err = (got - ref).norm(dim=1) / ref.norm(dim=1)
     assert float(err.max()) <= 1 / 3 and float(err.mean()) <= 3e-3
+
+
+@pytest.mark.parametrize("name,M", [("lit", 16), ("lit", 33), ("lit", 64), ("k12", 16), ("k16", 16), ("k16", 17), ("k16", 64), ("k20", 16)])
+def test_rings_wrap_from_tile_to_tile(dev, name, M):
+    """More tiles than SMs, an odd number of units per tile: every ring depth (four or eight units, by format and row
+    count) goes round, and crosses from one tile to the next, with a half-filled raw stage where one holds two."""
+    from gridbook_b200 import _native, synth
+    fmt = _fmt(name)
+    N, K = 128 * 2 * 148 + 40, 256 * 9
+    d = synth.make_linear(fmt, N, K, seed=M, global_scale=1.0 / 448.0 if name == "lit" else None)
+    lin = _linear(fmt, d, [N], dev)
+    x = _wide_rows(M, K, M)
+    y = lin(synth.bf16_tensor(x, dev))
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    assert_close_bf16(f32_of(y), oracle_linear(x, d), f"{name} M={M} {N}x{K}", atol_rel=1e-6)
