@@ -171,6 +171,21 @@ GB_DEVINL uint32_t mul_pair_f32(uint32_t pair, float s) {
   return gb_pack_bf16x2(__uint_as_float(pair << 16) * s, __uint_as_float(pair & 0xFFFF0000u) * s);
 }
 
+// The same for a whole warp that goes on together; false: given up.
+GB_DEVINL bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  uint32_t done;
+  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(done) : "r"(gb_smem_u32(bar)), "r"(parity) : "memory");
+  if (__all_sync(0xffffffffu, done)) return true;
+  wait_or_abort(bar, parity, abort_flag, status, code);
+  return !__any_sync(0xffffffffu, *abort_flag != 0);
+}
+GB_DEVINL bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
+
 // The same for the waits on the critical path of every unit: the abort flag is looked at only when
 // the barrier is not ready at once.
 GB_DEVINL void wait_fast(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
@@ -472,92 +487,107 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // u + 8, which the same warpgroup decodes after it has waited for u: no barrier can run ahead of
   // a waiter.
 
+  // The loading and issuing warps walk their loops whole, with values that are the same in every lane, and one elected
+  // lane issues: the operands then stay in uniform registers (in code that only lane 0 enters they are moved
+  // there first, 53 clocks to issue an MMA whatever its size).
   if (warp == 0) {
     // ------------------------- packed weight rows -------------------------
-    if (lane == 0) {
-      int it = 0;
-      for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
+    const bool leader = elect_one();
+    int it = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
       const Tile T = tile_at(t);
-      for (int pass = 0; pass < T.n_pass; ++pass)
-      for (int r = r_begin; r < r_end; ++r, ++it) {
-        const int rs = it % kRawStages;
-        wait_or_abort(&raw_empty[rs], ((it / kRawStages) & 1) ^ 1, abort_flag, p.status, 21);
-        gb_mbar_expect_tx(&raw_full[rs], G::kStageBytes);
+      const int n_pass = __shfl_sync(0xffffffffu, T.n_pass, 0);
+      for (int pass = 0; pass < n_pass && ok; ++pass)
+        for (int r = r_begin; r < r_end; ++r, ++it) {
+          const int rs = it % kRawStages;
+          ok = warp_wait(&raw_empty[rs], ((it / kRawStages) & 1) ^ 1, abort_flag, p.status, 21);
+          if (!ok) break;                                    // no copy may be in flight when the CTA leaves
+          if (leader) {
+            gb_mbar_expect_tx(&raw_full[rs], G::kStageBytes);
 #pragma unroll
-        for (int bx = 0; bx < Fm<F>::kBoxes; ++bx)
-          tma_load_2d(raw + (size_t)rs * G::kStageBytes + bx * G::kBoxBytes, &map_w,
-                      (r * kSbPerStage + bx * Fm<F>::kSbPerBox) * kSb, T.w_row0, &raw_full[rs]);
-      }
-      }
+            for (int bx = 0; bx < Fm<F>::kBoxes; ++bx)
+              tma_load_2d(raw + (size_t)rs * G::kStageBytes + bx * G::kBoxBytes, &map_w,
+                          (r * kSbPerStage + bx * Fm<F>::kSbPerBox) * kSb, T.w_row0, &raw_full[rs]);
+          }
+          __syncwarp();
+        }
     }
   } else if (warp == 1) {
     // ------------------------- activation slabs ---------------------------
-    if (lane == 0) {
-      gb_pdl_wait();                                         // x may come from the launch ahead
-      const int k_base = r_begin * kSbPerStage * 256;
-      int g = 0;                                             // units since the start, over all tiles and passes
-      for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
+    gb_pdl_wait();                                           // x may come from the launch ahead
+    const bool leader = elect_one();
+    const int k_base = r_begin * kSbPerStage * 256;
+    int g = 0;                                               // units since the start, over all tiles and passes
+    bool ok = true;
+    for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
       const Tile T = tile_at(t);
-      for (int pass = 0; pass < T.n_pass; ++pass)
-      for (int u = 0; u < units; ++u, ++g) {
-        const int s = g & xs_mask;
-        wait_or_abort(&done[s], ((uint32_t)(g >> xs_log) & 1u) ^ 1u, abort_flag, p.status, 22);
-        gb_mbar_expect_tx(&full[s], (uint32_t)x_stage_bytes);
-        uint8_t* dst = xs + (size_t)s * x_stage_bytes;
-        const int k0 = k_base + u * 128;
-        tma_load_2d(dst, &map_x, k0, T.seg_lo + pass * pass_rows, &full[s]);
-        tma_load_2d(dst + slab_bytes, &map_x, k0 + 64, T.seg_lo + pass * pass_rows, &full[s]);
-      }
-      }
+      const int n_pass = __shfl_sync(0xffffffffu, T.n_pass, 0), lo = __shfl_sync(0xffffffffu, T.seg_lo, 0);
+      for (int pass = 0; pass < n_pass && ok; ++pass)
+        for (int u = 0; u < units; ++u, ++g) {
+          const int s = g & xs_mask;
+          ok = warp_wait(&done[s], ((uint32_t)(g >> xs_log) & 1u) ^ 1u, abort_flag, p.status, 22);
+          if (!ok) break;
+          if (leader) {
+            gb_mbar_expect_tx(&full[s], (uint32_t)x_stage_bytes);
+            uint8_t* dst = xs + (size_t)s * x_stage_bytes;
+            const int k0 = k_base + u * 128;
+            tma_load_2d(dst, &map_x, k0, lo + pass * pass_rows, &full[s]);
+            tma_load_2d(dst + slab_bytes, &map_x, k0 + 64, lo + pass * pass_rows, &full[s]);
+          }
+          __syncwarp();
+        }
     }
   } else if (warp < kCtlWarps) {
     // ------------------------- MMA issuers ---------------------------------
     // Issuer i takes the units of operand buffer i (four issuers) or of buffers 2i and 2i + 1 (two
     // issuers, when the activation rows leave room for two accumulators only) into its own
     // accumulator; the read-out adds the accumulators in their fixed order.
-    const int i = warp - 2;
-    if (lane == 0 && i < p.n_iss) {
-      const uint32_t acc = tmem_base + (uint32_t)i * (kACol0 / (uint32_t)p.n_iss);
+    const int i = __shfl_sync(0xffffffffu, warp, 0) - 2;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const bool leader = elect_one();
+    if (i < p.n_iss) {
+      const uint32_t acc = tmem + (uint32_t)i * (kACol0 / (uint32_t)p.n_iss);
       const uint32_t slab16 = (uint32_t)slab_bytes >> 4;
       const uint64_t desc0 = smem_desc_sw128(gb_smem_u32(xs));
       int g0 = 0, item = 0;                                  // units / (tile, pass) items since the start
-      for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
-      const Tile T = tile_at(t);
-      for (int pass = 0; pass < T.n_pass; ++pass, g0 += units, ++item) {
-        // grouped mode: N = this pass's rows rounded up to 16.  The item before must have been read out.
-        uint32_t idesc = p.idesc;
-        if (kGrouped) {
-          const int rows = min(pass_rows, T.cnt - pass * pass_rows);
-          idesc = (p.idesc & ~(0x3Fu << 17)) | ((uint32_t)(((rows + 15) / 16 * 16) >> 3) << 17);
-        }
-        if (item > 0) {
-          wait_or_abort(acc_empty, (item - 1) & 1, abort_flag, p.status, 28);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        }
-        bool first = true;
-        for (int u = 0; u < units; ++u) {
-          if ((p.n_iss == 4 ? (u & 3) : ((u >> 1) & 1)) != i) continue;
-          const int g = g0 + u, s = g & xs_mask, ab = u & 3;
-          wait_fast(&full[s], (uint32_t)(g >> xs_log) & 1u, abort_flag, p.status, 23);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_tmem = tmem_base + kACol0 + (uint32_t)(ab * kABufCols);
-          const uint64_t db = desc0 + (uint64_t)((uint32_t)(s * x_stage_bytes) >> 4);
-          {
-            if (first) {
+      bool ok = true;
+      for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
+        const Tile T = tile_at(t);
+        const int n_pass = __shfl_sync(0xffffffffu, T.n_pass, 0), cnt = __shfl_sync(0xffffffffu, T.cnt, 0);
+        for (int pass = 0; pass < n_pass && ok; ++pass, g0 += units, ++item) {
+          // grouped mode: N = this pass's rows rounded up to 16.  The item before must have been read out.
+          uint32_t idesc = p.idesc;
+          if (kGrouped) {
+            const int rows = min(pass_rows, cnt - pass * pass_rows);
+            idesc = (p.idesc & ~(0x3Fu << 17)) | ((uint32_t)(((rows + 15) / 16 * 16) >> 3) << 17);
+          }
+          if (item > 0) {
+            ok = warp_wait(acc_empty, (item - 1) & 1, abort_flag, p.status, 28);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
+          bool first = true;
+          for (int u = 0; u < units; ++u) {
+            if ((p.n_iss == 4 ? (u & 3) : ((u >> 1) & 1)) != i) continue;
+            const int g = g0 + u, s = g & xs_mask, ab = u & 3;
+            ok = warp_wait(&full[s], (uint32_t)(g >> xs_log) & 1u, abort_flag, p.status, 23);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a_tmem = tmem + kACol0 + (uint32_t)(ab * kABufCols);
+            const uint64_t db = desc0 + (uint64_t)((uint32_t)(s * x_stage_bytes) >> 4);
+            if (leader) {
 #pragma unroll
               for (int k = 0; k < 8; ++k)                    // 16 weights of K per instruction
-                umma_bf16_ts(acc, a_tmem + (uint32_t)(k * 8), db + (uint64_t)((k >> 2) * slab16 + 2 * (k & 3)), idesc, k > 0);
-              first = false;
-            } else {
-#pragma unroll
-              for (int k = 0; k < 8; ++k)
-                umma_bf16_ts(acc, a_tmem + (uint32_t)(k * 8), db + (uint64_t)((k >> 2) * slab16 + 2 * (k & 3)), idesc, true);
+                umma_bf16_ts(acc, a_tmem + (uint32_t)(k * 8), db + (uint64_t)((k >> 2) * slab16 + 2 * (k & 3)), idesc, !first || k > 0);
+              umma_commit(&done[s]);
             }
+            __syncwarp();
+            first = false;
           }
-          umma_commit(&done[s]);
+          if (ok && leader) umma_commit(acc_full);
+          __syncwarp();
         }
-        umma_commit(acc_full);
-      }
       }
     }
   } else {
@@ -584,7 +614,6 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
       if (F == kFmtK16) exact = *inexact == 0;
     }
-    if (!waited) { gb_pdl_wait(); waited = true; }           // y may still be read by the launch ahead
     float rs = 0.0f;                                         // fp8 grid: this row's scale and its two factors
     uint32_t hi2 = 0, lo2 = 0;
     if constexpr (kIsFp8<F>) {
@@ -687,6 +716,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
 
     // ------------------------- read-out ------------------------------------
+    if (!waited) { gb_pdl_wait(); waited = true; }           // y may still be read by the launch ahead
     wait_or_abort(acc_full, item & 1, abort_flag, p.status, 26);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int col_part = (warp - kCtlWarps) >> 2;            // column chunks: every fourth
