@@ -451,85 +451,114 @@ int launch_expand(const gb_weight* w, int64_t row0, int64_t nrows, void* out0, v
 // superblock, so that every store instruction of the eight lanes writes 128 contiguous bytes.  The
 // sub-tables sit in shared memory as 32-bit words, eight copies each (copy = lane mod 8: lanes of
 // different copies never share a bank).  Memory-bound: 128 or 64 bytes read and 256 written per
-// 256 weights.
+// 256 weights.  A CTA takes a contiguous run of rows and rebuilds its tables where they change codebook (k = 16 with
+// a codebook per role took the generic kernel before: 8192 x 5120 99.7 -> 10.9 us).
 constexpr int kF8Unroll = 4;
+
+// Rows [run, end) from `run` on that share a codebook block; *base: its element offset.  Called by the whole CTA.
+GB_DEVINL int64_t codebook_run(const int32_t* offsets, int64_t run, int64_t end, int64_t* base, int* scratch) {
+  if (offsets == nullptr) { *base = 0; return end; }
+  const int32_t mine = offsets[run];
+  *base = mine;
+  __syncthreads();
+  if (threadIdx.x == 0) *scratch = (int)(end - run);
+  __syncthreads();
+  for (int64_t r = run + threadIdx.x; r < end; r += blockDim.x)
+    if (offsets[r] != mine) { atomicMin(scratch, (int)(r - run)); break; }
+  __syncthreads();
+  return run + *scratch;
+}
 
 template <bool kK32>
 __global__ void __launch_bounds__(kThreads)
-expand_fp8_fast_kernel(const uint8_t* __restrict__ qw, int64_t row_stride, const uint8_t* __restrict__ codebook,
-                       int64_t nrows, int64_t n_sb, uint4* __restrict__ out) {
+expand_fp8_fast_kernel(const uint8_t* __restrict__ qw, int64_t row_stride, const uint8_t* __restrict__ codebook, const int32_t* __restrict__ offsets,
+                       int64_t nrows, int n_sb, int rows_per_cta, uint4* __restrict__ out) {
   constexpr int kEntries = kK32 ? 1024 : 512;              // 4 x 256 two-byte or 2 x 256 four-byte entries
   constexpr int kSb = kK32 ? 128 : 64;
   __shared__ uint32_t lut[kEntries * 8];
-  for (int e = threadIdx.x; e < kEntries; e += kThreads) {
-    const uint32_t v = kK32 ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(codebook) + e)
-                            : __ldg(reinterpret_cast<const uint32_t*>(codebook) + e);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) lut[e * 8 + j] = v;
-  }
-  __syncthreads();
+  __shared__ int run_s;
   const int lane = threadIdx.x & 31, sub = lane & 7, which = lane >> 3;
   const uint32_t* my = lut + sub;
-  const int64_t units = nrows * n_sb;
-  const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
-  for (int64_t u0 = ((int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * (4 * kF8Unroll); u0 < units;
-       u0 += warps * (4 * kF8Unroll)) {
-    uint32_t in[kF8Unroll][kK32 ? 4 : 2];                  // two codewords of the first half, two of the second
-#pragma unroll
-    for (int i = 0; i < kF8Unroll; ++i) {
-      const int64_t u = u0 + 4 * i + which < units ? u0 + 4 * i + which : u0;
-      const int64_t r = u / n_sb, sb = u - r * n_sb;
-      const uint8_t* p = qw + r * row_stride + sb * kSb;
-      if (kK32) {
-        const uint2 a = __ldg(reinterpret_cast<const uint2*>(p) + sub), b = __ldg(reinterpret_cast<const uint2*>(p + 64) + sub);
-        in[i][0] = a.x; in[i][1] = a.y; in[i][2] = b.x; in[i][3] = b.y;
+  const int64_t r_begin = (int64_t)blockIdx.x * rows_per_cta, r_end = min(r_begin + rows_per_cta, nrows);
+  bool waited = false;
+  gb_pdl_launch_dependents();
+  for (int64_t run = r_begin; run < r_end;) {
+    int64_t base;
+    const int64_t run_end = codebook_run(offsets, run, r_end, &base, &run_s);
+    const uint8_t* book = codebook + base;
+    for (int e = threadIdx.x; e < kEntries; e += kThreads) {
+      uint32_t v;
+      if (((uintptr_t)book & 3u) != 0) {                   // a row's offset may be any
+        const uint8_t* c = book + e * (kK32 ? 2 : 4);
+        v = c[0] | (uint32_t)c[1] << 8 | (kK32 ? 0u : (uint32_t)c[2] << 16 | (uint32_t)c[3] << 24);
       } else {
-        in[i][0] = __ldg(reinterpret_cast<const uint32_t*>(p) + sub);
-        in[i][1] = __ldg(reinterpret_cast<const uint32_t*>(p + 32) + sub);
+        v = kK32 ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(book) + e) : __ldg(reinterpret_cast<const uint32_t*>(book) + e);
       }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) lut[e * 8 + j] = v;
     }
+    __syncthreads();
+    if (!waited) { gb_pdl_wait(); waited = true; }         // the output may still be read by the launch ahead
+    const uint8_t* rows = qw + run * row_stride;
+    uint4* to = out + run * n_sb * 16;
+    const uint32_t units = (uint32_t)(run_end - run) * (uint32_t)n_sb;   // fits: rows_per_cta * n_sb is checked
+    for (uint32_t u0 = (threadIdx.x >> 5) * (4 * kF8Unroll); u0 < units; u0 += (kThreads / 32) * (4 * kF8Unroll)) {
+      uint32_t in[kF8Unroll][kK32 ? 4 : 2];                // two codewords of the first half, two of the second
 #pragma unroll
-    for (int i = 0; i < kF8Unroll; ++i) {
-      const int64_t u = u0 + 4 * i + which;
-      if (u >= units) continue;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint4 o;
+      for (int i = 0; i < kF8Unroll; ++i) {
+        const uint32_t u = u0 + 4 * i + which < units ? u0 + 4 * i + which : u0;
+        const uint32_t r = u / (uint32_t)n_sb, sb = u - r * (uint32_t)n_sb;
+        const uint8_t* p = rows + r * row_stride + sb * kSb;
         if (kK32) {
-          const uint32_t c0 = in[i][2 * half], c1 = in[i][2 * half + 1];
-          o.x = my[(c0 & 0xffu) * 8] | (my[(256 + ((c0 >> 8) & 0xffu)) * 8] << 16);
-          o.y = my[(512 + ((c0 >> 16) & 0xffu)) * 8] | (my[(768 + (c0 >> 24)) * 8] << 16);
-          o.z = my[(c1 & 0xffu) * 8] | (my[(256 + ((c1 >> 8) & 0xffu)) * 8] << 16);
-          o.w = my[(512 + ((c1 >> 16) & 0xffu)) * 8] | (my[(768 + (c1 >> 24)) * 8] << 16);
+          const uint2 a = __ldg(reinterpret_cast<const uint2*>(p) + sub), b = __ldg(reinterpret_cast<const uint2*>(p + 64) + sub);
+          in[i][0] = a.x; in[i][1] = a.y; in[i][2] = b.x; in[i][3] = b.y;
         } else {
-          const uint32_t c = in[i][half];                  // two 16-bit codewords
-          o.x = my[(c & 0xffu) * 8];
-          o.y = my[(256 + ((c >> 8) & 0xffu)) * 8];
-          o.z = my[((c >> 16) & 0xffu) * 8];
-          o.w = my[(256 + (c >> 24)) * 8];
+          in[i][0] = __ldg(reinterpret_cast<const uint32_t*>(p) + sub);
+          in[i][1] = __ldg(reinterpret_cast<const uint32_t*>(p + 32) + sub);
         }
-        out[u * 16 + half * 8 + sub] = o;
+      }
+#pragma unroll
+      for (int i = 0; i < kF8Unroll; ++i) {
+        const uint32_t u = u0 + 4 * i + which;
+        if (u >= units) continue;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint4 o;
+          if (kK32) {
+            const uint32_t c0 = in[i][2 * half], c1 = in[i][2 * half + 1];
+            o.x = my[(c0 & 0xffu) * 8] | (my[(256 + ((c0 >> 8) & 0xffu)) * 8] << 16);
+            o.y = my[(512 + ((c0 >> 16) & 0xffu)) * 8] | (my[(768 + (c0 >> 24)) * 8] << 16);
+            o.z = my[(c1 & 0xffu) * 8] | (my[(256 + ((c1 >> 8) & 0xffu)) * 8] << 16);
+            o.w = my[(512 + ((c1 >> 16) & 0xffu)) * 8] | (my[(768 + (c1 >> 24)) * 8] << 16);
+          } else {
+            const uint32_t c = in[i][half];                // two 16-bit codewords
+            o.x = my[(c & 0xffu) * 8];
+            o.y = my[(256 + ((c >> 8) & 0xffu)) * 8];
+            o.z = my[((c >> 16) & 0xffu) * 8];
+            o.w = my[(256 + (c >> 24)) * 8];
+          }
+          to[(int64_t)u * 16 + half * 8 + sub] = o;
+        }
       }
     }
+    run = run_end;
+    if (run < r_end) __syncthreads();                      // the next run rebuilds the tables
   }
 }
 
 int launch_expand_fp8_fast(const gb_weight* w, int64_t row0, int64_t nrows, void* out, void* stream) {
-  const bool k32 = w->fmt.k_bits == 32;
-  const int64_t n_sb = w->K / 256, units = nrows * n_sb;
-  const int64_t per_cta = (kThreads / 32) * 4 * kF8Unroll;
-  int64_t blocks = (units + per_cta - 1) / per_cta;
-  const int64_t cap = (int64_t)gb_sm_count() * 8;
-  if (cap > 0 && blocks > cap) blocks = cap;
-  gb_count_launch();
-  const uint8_t* base = w->qw + row0 * w->row_stride;
-  if (k32)
-    expand_fp8_fast_kernel<true><<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(
-        base, w->row_stride, (const uint8_t*)w->codebook, nrows, n_sb, (uint4*)out);
-  else
-    expand_fp8_fast_kernel<false><<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(
-        base, w->row_stride, (const uint8_t*)w->codebook, nrows, n_sb, (uint4*)out);
-  GB_LAUNCH_OK("expand_fp8_fast_kernel");
+  const int sms = gb_sm_count();
+  if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
+  const int64_t n_sb = w->K / 256;
+  // eight CTAs per SM where there are rows for them, at least two steps of every warp each so that the tables pay
+  const int64_t least = (2 * (kThreads / 32) * 4 * kF8Unroll + n_sb - 1) / n_sb;
+  int64_t rows_per = (nrows + (int64_t)sms * 8 - 1) / ((int64_t)sms * 8);
+  if (rows_per < least) rows_per = least;
+  GB_REQUIRE(rows_per * n_sb < (1ll << 31), "too many superblocks per CTA");
+  const unsigned blocks = (unsigned)((nrows + rows_per - 1) / rows_per);
+  GB_CUDA_OK(gb_launch(w->fmt.k_bits == 32 ? expand_fp8_fast_kernel<true> : expand_fp8_fast_kernel<false>, dim3(blocks), dim3(kThreads), 0,
+                       (cudaStream_t)stream, w->qw + row0 * w->row_stride, w->row_stride, (const uint8_t*)w->codebook,
+                       w->cb_row_offset ? w->cb_row_offset + row0 : nullptr, nrows, (int)n_sb, (int)rows_per, (uint4*)out));
   return GB_OK;
 }
 
@@ -589,23 +618,16 @@ expand_product_kernel(const __grid_constant__ ProdArgs p, void* __restrict__ out
   const int k = a.fmt.k_bits;
   const bool v2 = a.fmt.scale_coding == GB_SCALE_V2;
   const uint32_t my = (uint32_t)(sub & (p.copies - 1));
+  bool waited = false;
+  gb_pdl_launch_dependents();
   if (kOut == kOutNvfp4 && v2)
     for (int i = tid; i < 4096; i += kProdThreads) comp_s[i] = (uint8_t)gb_f32_to_e4m3(fminf(__ldg(a.compose + i), 448.0f));
 
   const int64_t r_begin = (int64_t)blockIdx.x * p.rows_per_cta;
   const int64_t r_end = r_begin + p.rows_per_cta < a.nrows ? r_begin + p.rows_per_cta : a.nrows;
   for (int64_t run = r_begin; run < r_end;) {
-    int64_t cb_base = 0, run_end = r_end;
-    if (a.cb_row_offset) {                                 // rows [run, run_end) use one codebook block
-      cb_base = a.cb_row_offset[a.row0 + run];
-      __syncthreads();
-      if (tid == 0) run_end_s = (int)(r_end - run);
-      __syncthreads();
-      for (int64_t r = run + tid; r < r_end; r += kProdThreads)
-        if (a.cb_row_offset[a.row0 + r] != (int32_t)cb_base) { atomicMin(&run_end_s, (int)(r - run)); break; }
-      __syncthreads();
-      run_end = run + run_end_s;
-    }
+    int64_t cb_base;
+    const int64_t run_end = codebook_run(a.cb_row_offset ? a.cb_row_offset + a.row0 : nullptr, run, r_end, &cb_base, &run_end_s);
     for (int e = tid; e < p.entries; e += kProdThreads) {
       if constexpr (kFp8) {
         const uint8_t* c = reinterpret_cast<const uint8_t*>(a.codebook) + cb_base + (int64_t)e * 2;
@@ -624,6 +646,7 @@ expand_product_kernel(const __grid_constant__ ProdArgs p, void* __restrict__ out
       }
     }
     __syncthreads();
+    if (!waited) { gb_pdl_wait(); waited = true; }         // the output may still be read by the launch ahead
 
     // entry offset of sub-index i inside the table
     uint32_t base[kSubs], mask[kSubs];
@@ -762,9 +785,8 @@ int launch_expand_product(const gb_weight* w, int64_t row0, int64_t nrows, void*
   const unsigned blocks = (unsigned)((nrows + rows_per - 1) / rows_per);
   if (smem > 47 * 1024)                                   // the default limit counts the static words too
     GB_CUDA_OK(cudaFuncSetAttribute((const void*)expand_product_kernel<kOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  gb_count_launch();
-  expand_product_kernel<kOut><<<blocks, kProdThreads, smem, (cudaStream_t)stream>>>(p, out0, (uint8_t*)out_sf, fold_sign);
-  GB_LAUNCH_OK("expand_product_kernel");
+  GB_CUDA_OK(gb_launch(expand_product_kernel<kOut>, dim3(blocks), dim3(kProdThreads), (size_t)smem, (cudaStream_t)stream, p, out0,
+                       (uint8_t*)out_sf, fold_sign));
   return GB_OK;
 }
 // ---- native NVFP4 view, fast ------------------------------------------------------------------
@@ -992,8 +1014,7 @@ int gb_expand_fp8(const gb_weight* w, int64_t row0, int64_t nrows, void* out, vo
   const gb_format& f = w->fmt;
   if (f.mode == GB_MODE_PRODUCT && ((f.k_bits == 32 && f.n_sub == 4 && f.type_size == 128) ||
                                     (f.k_bits == 16 && f.n_sub == 2 && f.type_size == 64)) &&
-      w->cb_row_offset == nullptr && ((uintptr_t)w->codebook & 3u) == 0 && ((uintptr_t)out & 15u) == 0 &&
-      ((uintptr_t)w->qw & 15u) == 0 && w->row_stride % 16 == 0) {
+      ((uintptr_t)w->codebook & 3u) == 0 && ((uintptr_t)out & 15u) == 0 && ((uintptr_t)w->qw & 15u) == 0 && w->row_stride % 16 == 0) {
     int rc = gb_check_weight(w);
     if (rc != GB_OK) return rc;
     GB_REQUIRE(out != nullptr, "null output pointer");

@@ -156,3 +156,21 @@ def test_rows_that_start_in_the_middle_of_another_tensor(dev, name):
         assert torch.equal(moe(x, tw, ids), moe(x.clone(), tw, ids))
     torch.cuda.synchronize()
     assert _native.device_status(0) == 0
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("rows,K,books", [(1, 256, 1), (37, 768, 2), (4099, 512, 3), (1000, 2304, 7)])
+@pytest.mark.parametrize("k,n_sub", [(16, 2), (32, 4)])
+def test_fp8_expander_rebuilds_its_tables_where_rows_change_codebook(dev, k, n_sub, rows, K, books, shift):
+    """Runs of rows that end inside a CTA's share, a window of rows, codebook blocks at any byte."""
+    from gridbook_b200 import kernels, synth
+    from gridbook_b200.formats import CBFormat
+    fmt = CBFormat("fp8", k, n_sub=n_sub)
+    d = synth.make_linear(fmt, rows, K, seed=rows + k, n_books=books)
+    off = d["cb_row_offset"] if d["cb_row_offset"] is not None else np.zeros(rows, np.int32)
+    up = dict(d, cb=np.concatenate([np.zeros(shift, np.float32), d["cb"]]), cb_row_offset=off + np.int32(shift)) if shift or books > 1 else d
+    w = synth.to_device_weight(up, dev)
+    want = O.f32_to_e4m3(O.decode_values(d["qw"], d["cb"], off, N=rows, K=K, k_bits=k, n_sub=n_sub, type_size=fmt.type_size))
+    assert np.array_equal(kernels.expand_fp8(w).view(torch.uint8).cpu().numpy(), want)
+    lo, n = rows // 3, max(1, rows // 2)
+    assert np.array_equal(kernels.expand_fp8(w, lo, n).view(torch.uint8).cpu().numpy(), want[lo:lo + n])
