@@ -321,8 +321,8 @@ template <int kG>
 __global__ void __launch_bounds__(1024)
 nvfp4_quantize_rows_kernel(const uint4* __restrict__ x, uint2* __restrict__ packed, uint8_t* __restrict__ sfa,
                            float* __restrict__ a_scale, int64_t M, int groups, float range) {
-  gb_pdl_launch_dependents();
   gb_pdl_wait();
+  gb_pdl_launch_dependents();                            // behind the wait: the weights' expander runs beside this launch
   const int64_t row = blockIdx.x;
   const int64_t k_atoms = (groups + 3) / 4;
   auto sf_offset = [&](int g) {

@@ -1177,8 +1177,12 @@ GB_DEVINL void to_peers(uint32_t* slots, uint32_t v, int split) {
 template <int kG, int kMode>
 __global__ void __launch_bounds__(1024)
 fp4_rows_kernel(const __grid_constant__ RowsParams p) {
-  gb_pdl_launch_dependents();
+  // the grouped GEMM's operand (no unit size): the stack's expander runs beside this launch and needs what is ahead to
+  // have completed; the decode kernel waits for it all the same, and starts early
+  const bool late = kMode != 0 && p.x_unit == 0;
+  if (!late) gb_pdl_launch_dependents();
   gb_pdl_wait();
+  if (late) gb_pdl_launch_dependents();
   const int groups = p.K / 16;
   const int j = kMode == 0 ? (int)blockIdx.x / p.split : (int)blockIdx.x;
   const int g_first = (kMode == 0 ? (int)blockIdx.x % p.split * (int)blockDim.x : 0) + (int)threadIdx.x;

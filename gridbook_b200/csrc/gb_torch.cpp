@@ -38,7 +38,7 @@ namespace {
   F(gb_last_error) F(gb_gemv_hinted_workspace_bytes) F(gb_gemv) F(gb_gemv_row_batch_max) F(gb_gemv_tab) \
   F(gb_gemv_tab_slots_bytes) F(gb_fp4_act_qdq) F(gb_fp8_act_qdq) F(gb_fp8_quantize_rows) F(gb_nvfp4_sf_bytes) \
   F(gb_nvfp4_quantize_rows) F(gb_expand_fp4_nvfp4) F(gb_expand_fp4_bf16) F(gb_expand_fp8) F(gb_expand_fp8_bf16) \
-  F(gb_gemm_fp4) F(gb_gemm_tn) F(gb_gemm_tn_grouped) F(gb_moe_route_ws) F(gb_moe_route_workspace_bytes) \
+  F(gb_expand_fp4_nvfp4_beside) F(gb_expand_fp8_beside) F(gb_gemm_fp4) F(gb_gemm_tn) F(gb_gemm_tn_grouped) F(gb_moe_route_ws) F(gb_moe_route_workspace_bytes) \
   F(gb_moe_gather_rows) F(gb_moe_swiglu_rows) F(gb_moe_gemv) F(gb_moe_gemv_sorted) F(gb_moe_mlp_pairs) \
   F(gb_moe_mlp_pairs_workspace_bytes) F(gb_moe_combine) F(gb_gemv_hinted) F(gb_scales_e4m3) F(gb_moe_route_inv) \
   F(gb_moe_fp4_pass_rows) F(gb_moe_fp4_operand_bytes) F(gb_moe_fp4_rows) F(gb_moe_fp4_swiglu_rows) \
@@ -246,7 +246,7 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
       a.alloc(x);
       check(L.gb_nvfp4_quantize_rows(x.data_ptr(), M, K, kNvfp4ActRange, a.ptr(qa), a.ptr(sa), a.ptr<float>(as), stream));
       // scale factors of the rows past N stay unset: they only reach columns that are not stored
-      check(L.gb_expand_fp4_nvfp4(&w.w, 0, N, a.ptr(qb), a.ptr(sb), 2, stream));
+      check(L.gb_expand_fp4_nvfp4_beside(&w.w, 0, N, a.ptr(qb), a.ptr(sb), 2, stream));
       check(L.gb_gemm_fp4(a.ptr(qa), a.ptr(sa), a.ptr(qb), a.ptr(sb), out.data_ptr(), M, N, K, a.ptr<float>(as),
                           w.w.global_scale, stream));
       prefill_route = kRouteNvfp4;
@@ -261,7 +261,7 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
       const int q = a.add(M * K), as = a.add(M * 4), wt = a.add(N * K);
       a.alloc(x);
       check(L.gb_fp8_quantize_rows(x.data_ptr(), a.ptr(q), a.ptr<float>(as), M, K, rule, stream));
-      check(L.gb_expand_fp8(&w.w, 0, N, a.ptr(wt), stream));
+      check(L.gb_expand_fp8_beside(&w.w, 0, N, a.ptr(wt), stream));
       check(L.gb_gemm_tn(a.ptr(q), a.ptr(wt), out.data_ptr(), M, N, K, GB_GEMM_E4M3, a.ptr<float>(as), w.w.weight_scale,
                          w.w.global_scale, stream));
       prefill_route = kRouteFp8;
@@ -512,7 +512,7 @@ struct MoEPlan {
         check(L.gb_moe_gemv_fp4(a.ptr(operand), &w.w, w.scales_e4m3, w.expert_stride, E, off, map, c.P, pr, to, c.stream));
         return;
       }
-      check(L.gb_expand_fp4_nvfp4(&flat.w, 0, flat.w.rows, a.ptr(wq), a.ptr(wsf), 2, c.stream));
+      check(L.gb_expand_fp4_nvfp4_beside(&flat.w, 0, flat.w.rows, a.ptr(wq), a.ptr(wsf), 2, c.stream));   // behind the rows' launch
       check(L.gb_moe_gemm_fp4(a.ptr(operand), a.ptr(wq), a.ptr(wsf), w.w.rows, w.w.K, E, off, map, c.P, w.w.global_scale, to, c.stream));
     };
     if (fp13) {

@@ -103,6 +103,10 @@ GB_API int gb_fp4_act_qdq(const void* x_bf16, void* out_bf16, int64_t M, int64_t
  * rows [row0, row0+nrows) -> [nrows, K] E4M3 bytes */
 GB_API int gb_expand_fp8(const gb_weight* w, int64_t row0, int64_t nrows, void* out_e4m3,
                   void* stream);
+/* The same right behind the launch that quantises the rows of the same product: the launch ahead on the stream must be
+ * gb_fp8_quantize_rows, and nothing it reads or writes may overlap the output.  The two run side by side (programmatic
+ * dependent launch); what follows on the stream sees both complete. */
+GB_API int gb_expand_fp8_beside(const gb_weight* w, int64_t row0, int64_t nrows, void* out_e4m3, void* stream);
 /* The served fp8-grid weight of rows [row0, row0+nrows): -> [nrows, K] bf16 =
  * bf16(value * weight_scale[row]), the per-weight rounding of the decode contract
  * (gridbook/csrc/cb_gemv.cu:20-27,219-228), for bf16 tensor-core routes that must keep it. */
@@ -121,6 +125,10 @@ GB_API int gb_expand_fp4_bf16(const gb_weight* w, int64_t row0, int64_t nrows, v
  * carry no sign - a negative group scale moves its sign into the group's sixteen values. */
 GB_API int gb_expand_fp4_nvfp4(const gb_weight* w, int64_t row0, int64_t nrows, void* out_packed,
                         void* out_sf, int sf_swizzled, void* stream);
+/* The same right behind gb_nvfp4_quantize_rows, or behind gb_moe_fp4_rows / gb_moe_fp4_swiglu_rows with pass_rows 0, as
+ * gb_expand_fp8_beside. */
+GB_API int gb_expand_fp4_nvfp4_beside(const gb_weight* w, int64_t row0, int64_t nrows, void* out_packed, void* out_sf, int sf_swizzled,
+                                      void* stream);
 
 /* ---- decode-batch linear (M <= 16; up to gb_gemv_row_batch_max rows where that is larger) ---- */
 /* replaces cb_gemv_fp8 / cb_gemv_fp4_v2 (gridbook/csrc/cb_gemv.cu:658-712,1138-1198;

@@ -174,3 +174,35 @@ def test_fp8_expander_rebuilds_its_tables_where_rows_change_codebook(dev, k, n_s
     assert np.array_equal(kernels.expand_fp8(w).view(torch.uint8).cpu().numpy(), want)
     lo, n = rows // 3, max(1, rows // 2)
     assert np.array_equal(kernels.expand_fp8(w, lo, n).view(torch.uint8).cpu().numpy(), want[lo:lo + n])
+
+
+@pytest.mark.parametrize("M", [20, 140, 333, 1500])
+def test_prefill_linears_launched_back_to_back(dev, M):
+    """The expander of a linear runs beside the quantiser of its rows and overwrites what the linear before has read: a
+    chain without a pause gives the outputs of the same calls one at a time, in every format's expander."""
+    from gridbook_b200 import formats, synth
+    from gridbook_b200.linear import CBLinear
+    fmts = [formats.NVFP4_LITERAL, formats.FP8_LITERAL, formats.CBFormat("fp4", 20, n_sub=2, scale_coding="v2"), formats.FP8_CB_K32,
+            formats.CBFormat("fp8", 30, n_sub=4), formats.CBFormat("fp4", 12, n_sub=2, scale_coding="v2"), formats.CBFormat("fp4", 13, n_sub=2, scale_coding="v2")]
+    gen = torch.Generator(device=dev).manual_seed(M)
+    lins, K = [], 1024
+    for i, fmt in enumerate(fmts * 2):
+        parts = [640, 384] if i % 2 else [1024]
+        lin = CBLinear(fmt, K, parts, [synth.codebook_tables(fmt, i + j) for j in range(len(parts))], prefix=f"chain.{i}")
+        lin.method.midm_max_rows = 16
+        scale = None if fmt.is_fp4 else (torch.rand(sum(parts), generator=gen, device=dev) + 0.5) * 0.02
+        lins.append(lin.load(synth.make_packed_device(fmt, sum(parts), K, gen, dev), scale, dev))
+    x = torch.randn(M, K, generator=gen, device=dev).to(torch.bfloat16)
+
+    def chain(pause):
+        out = []
+        for lin in lins:
+            out.append(lin(x))
+            if pause:
+                torch.cuda.synchronize()
+        return out
+
+    one_at_a_time = chain(True)
+    for _ in range(5):
+        for a, b in zip(chain(False), one_at_a_time):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))
