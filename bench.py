@@ -842,7 +842,7 @@ def bench_prefill(args, device):
                     kernels.gemm_fp4(a, sfa, b, sfb, a_scale=asc)
                     ms_gemm = timed_ms(lambda: kernels.gemm_fp4(a, sfa, b, sfb, a_scale=asc), 3, sync)
                     tf = flops / ms_gemm / 1e9
-                    pair = "gemm_pair_kernel (kind::mxf4nvf4)" if M > 128 else "gemm_fp4_kernel"
+                    pair = "gemm_pair_kernel (kind::mxf4nvf4)" if M > 128 else "gemm_rows_kernel (kind::mxf4nvf4)"
                     entry.update({"kernel": pair, "gemm_tflops": round(tf, 1), "gemm_ms": round(ms_gemm, 4),
                                   "pct_fp4_nominal": round(100 * tf / NOMINAL_TFLOPS["fp4"], 2),
                                   "pct_of_4x_measured_bf16": round(100 * tf / (4 * bf16_meas), 2)})

@@ -14,7 +14,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libgridbook_b200.so")
 HOST_LIB = os.path.join(PKG, "_gb_torch.so")
 HOST_SOURCE = "gb_torch.cpp"
-SOURCES = ("gb_api.cu", "gb_decode.cu", "gb_gemv.cu", "gb_moe.cu", "gb_gemm.cu", "gb_gemv_dot.cu", "gb_peer.cu", "gb_gemv_umma.cu", "gb_gemv_tab.cu", "gb_gemm_fp4.cu", "gb_gemm_pair.cu", "gb_gemv_fp4.cu")
+SOURCES = ("gb_api.cu", "gb_decode.cu", "gb_gemv.cu", "gb_moe.cu", "gb_gemm.cu", "gb_gemv_dot.cu", "gb_peer.cu", "gb_gemv_umma.cu", "gb_gemv_tab.cu", "gb_gemm_fp4.cu", "gb_gemm_pair.cu", "gb_gemm_rows.cu", "gb_gemv_fp4.cu")
 HEADERS = ("gb_common.cuh", os.path.join("..", "..", "include", "gridbook_b200.h"))
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

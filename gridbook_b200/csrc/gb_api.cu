@@ -151,8 +151,8 @@ int gb_prepare(int device) {
   if (rc == GB_OK) rc = gb_prepare_dot();
   if (rc == GB_OK) rc = gb_prepare_umma();
   if (rc == GB_OK) rc = gb_prepare_tab();
-  if (rc == GB_OK) rc = gb_prepare_gemm_fp4();
   if (rc == GB_OK) rc = gb_prepare_gemm_pair();
+  if (rc == GB_OK) rc = gb_prepare_gemm_rows();
   if (rc == GB_OK) rc = gb_prepare_gemv_fp4();
   cudaSetDevice(prev);
   return rc;

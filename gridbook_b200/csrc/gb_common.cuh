@@ -67,8 +67,8 @@ int gb_prepare_gemm();
 int gb_prepare_dot();
 int gb_prepare_umma();
 int gb_prepare_tab();
-int gb_prepare_gemm_fp4();
 int gb_prepare_gemm_pair();
+int gb_prepare_gemm_rows();
 int gb_prepare_gemv_fp4();
 // Longest a device-side wait may spin before it gives up and raises the status word
 // (two seconds unless gb_set_wait_limit_ms changed it).
@@ -94,8 +94,13 @@ inline GbFp4Tiles gb_fp4_tiles(int64_t P, int64_t E, int64_t K) {
   t.bytes = t.tail_at + up(t.tiles * 64 * (K / 16) * 4);
   return t;
 }
-// The prefill GEMMs on CTA pairs (gb_gemm_pair.cu), for the shapes that gb_gemm_pair_applies names.
-bool gb_gemm_pair_applies(int64_t M);
+// The prefill GEMMs on CTA pairs (gb_gemm_pair.cu).
+// The same for few rows or narrow layers (gb_gemm_rows.cu), where gb_gemm_rows_applies says so.
+bool gb_gemm_rows_applies(bool fp4, int64_t M, int64_t N, int64_t k_tiles);
+int gb_gemm_rows(const void* X, const void* W, void* D, int64_t M, int64_t N, int64_t K, int kind, const float* a_scale,
+                 const float* b_scale, float global_scale, cudaStream_t stream);
+int gb_gemm_fp4_rows(const void* X, const void* sfx, const void* W, const void* sfw, void* D, int64_t M, int64_t N, int64_t K,
+                     const float* a_scale, float global_scale, cudaStream_t stream);
 int gb_gemm_pair(const void* A, const void* B, void* D, int64_t M, int64_t N, int64_t K, int kind, const float* a_scale,
                  const float* b_scale, float global_scale, cudaStream_t stream);
 int gb_gemm_fp4_pair(const void* A, const void* sfa, const void* B, const void* sfb, void* D, int64_t M, int64_t N, int64_t K,

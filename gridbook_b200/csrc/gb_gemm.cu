@@ -1,18 +1,18 @@
-// Prefill GEMM on the 5th-generation tensor cores: D[M,N] = A[M,K] . B[N,K]^T with both
+// Grouped GEMM of the routed prefill on the 5th-generation tensor cores, and the dense entry gb_gemm_tn (its kernels:
+// gb_gemm_pair.cu, gb_gemm_rows.cu).  D[j, N] = A[j, K] . B[e, N, K]^T for the rows j of expert e, both
 // operands K-major, bf16 x bf16 (kind::f16) or E4M3 x E4M3 (kind::f8f6f4), fp32 accumulators
 // in tensor memory, scaled bf16 epilogue.
 //
-// Persistent CTAs (one per SM) walk the 128 x 256 output tiles, M fastest.  Warp 4 (one
+// Persistent CTAs (one per SM) walk the 128 x 256 output tiles.  Warp 4 (one
 // thread) streams 128-byte-wide K slabs of A and B into a shared-memory ring with tiled TMA
 // loads (128-byte swizzle); warp 5 (one thread) issues tcgen05.mma on shared-memory matrix
 // descriptors and releases ring stages with tcgen05.commit; warps 0..3 read the accumulator
 // out of tensor memory (tcgen05.ld, one 32-lane quarter each), apply the row / column /
 // global scales and store bf16.  Tensor memory holds TWO accumulators (512 columns): while
 // the epilogue warps drain one, the MMAs of the next tile already fill the other, and the
-// TMA ring never drains between tiles.  B is the decoded weight tile the expanders write (gb_expand_fp8 /
-// gb_expand_fp4_bf16); A is the bucketed activation matrix.
+// TMA ring never drains between tiles.
 //
-// Grouped mode (routed prefill): A holds the routed rows sorted by expert, B the decoded stack
+// A holds the routed rows sorted by expert, B the decoded stack
 // [E*N, K]; expert e owns rows [seg[e], seg[e+1]) of A.  Every CTA builds the per-expert tile
 // prefix from the device-side segment offsets (no host read), walks tiles N fastest so the CTAs
 // running together share an expert's decoded weights through L2, and the epilogue masks the
@@ -38,7 +38,7 @@ constexpr int kGroupSmem = 2 * (kMaxGroups + 1) * 4 + 8;   // segment offsets + 
 struct GemmParams {
   int64_t M, N, K;
   int k_tiles;
-  int m_tiles, n_tiles;      // output tiles along M and N
+  int n_tiles;               // output tiles along N
   int elem_bytes;            // 2 (bf16) or 1 (e4m3)
   uint32_t idesc;
   const float* a_scale;      // [M] or null
@@ -52,34 +52,25 @@ struct GemmParams {
   int E;
 };
 
-// One output tile of either mode: first A row, end of the valid rows, first B row, first
+// One output tile: first A row, end of the valid rows, first B row, first
 // output column, and the B-scale offset of the expert.
 struct Tile {
   int m0, m_end, b_row0, n0, scale0;
 };
 
-template <bool kGrouped>
 GB_DEVINL Tile tile_of(const GemmParams& p, int tile, const int* seg_s, const int* base_s) {
   Tile t;
-  if (!kGrouped) {
-    t.m0 = (tile % p.m_tiles) * kBM;
-    t.n0 = (tile / p.m_tiles) * kBN;
-    t.m_end = (int)p.M;
-    t.b_row0 = t.n0;
-    t.scale0 = 0;
-  } else {
-    const int gm = tile / p.n_tiles;
-    t.n0 = (tile % p.n_tiles) * kBN;
-    int lo = 0, hi = p.E;                 // largest e with base_s[e] <= gm
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (base_s[mid] <= gm) lo = mid; else hi = mid;
-    }
-    t.m0 = seg_s[lo] + (gm - base_s[lo]) * kBM;
-    t.m_end = seg_s[lo + 1];
-    t.scale0 = lo * (int)p.N;
-    t.b_row0 = t.scale0 + t.n0;
+  const int gm = tile / p.n_tiles;
+  t.n0 = (tile % p.n_tiles) * kBN;
+  int lo = 0, hi = p.E;                   // largest e with base_s[e] <= gm
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (base_s[mid] <= gm) lo = mid; else hi = mid;
   }
+  t.m0 = seg_s[lo] + (gm - base_s[lo]) * kBM;
+  t.m_end = seg_s[lo + 1];
+  t.scale0 = lo * (int)p.N;
+  t.b_row0 = t.scale0 + t.n0;
   return t;
 }
 
@@ -129,7 +120,6 @@ GB_DEVINL void wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort
   }
 }
 
-template <bool kGrouped>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const GemmParams p) {
@@ -147,7 +137,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool fp8 = p.elem_bytes == 1;
-  if (kGrouped && warp == 0) {
+  if (warp == 0) {
     // row tiles of expert e: ceil(rows / 128); exclusive prefix by one warp, 32 experts a pass
     int carry = 0;
     for (int e0 = 0; e0 < p.E; e0 += 32) {
@@ -192,7 +182,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  const int total_tiles = kGrouped ? base_s[p.E] * p.n_tiles : p.m_tiles * p.n_tiles;
+  const int total_tiles = base_s[p.E] * p.n_tiles;
 
   // Every role walks the same tile sequence: tile = blockIdx.x, + gridDim.x, ...; M tiles vary
   // fastest, so the CTAs working at the same time share a few B (weight) tiles and sweep A,
@@ -203,7 +193,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const int slab_elems = kSlabBytes / p.elem_bytes;
       int kk = 0;                                        // K slabs issued so far, over all tiles
       for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-        const Tile t = tile_of<kGrouped>(p, tile, seg_s, base_s);
+        const Tile t = tile_of(p, tile, seg_s, base_s);
         for (int kt = 0; kt < p.k_tiles; ++kt, ++kk) {
           const int s = kk % kStages;
           wait_or_abort(&empty_bar[s], ((kk / kStages) & 1) ^ 1, abort_flag, p.status, 11);
@@ -243,7 +233,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     int it = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
       const int buf = it & 1;
-      const Tile t = tile_of<kGrouped>(p, tile, seg_s, base_s);
+      const Tile t = tile_of(p, tile, seg_s, base_s);
       const int n0 = t.n0;
       wait_or_abort(&acc_full[buf], (it >> 1) & 1, abort_flag, p.status, 13);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -251,7 +241,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const bool row_ok = row < t.m_end;
       const float rs = (p.a_scale && row_ok ? p.a_scale[row] : 1.0f) * p.global_scale;
       const float* b_scale = p.b_scale ? p.b_scale + t.scale0 : nullptr;
-      const int64_t out_row = kGrouped && p.row_map && row_ok ? p.row_map[row] : row;
+      const int64_t out_row = p.row_map && row_ok ? p.row_map[row] : row;
 #pragma unroll 1
       for (int c0 = 0; c0 < kBN; c0 += 32) {
         uint32_t v[32];
@@ -436,9 +426,7 @@ int gb_tensor_map_out(void* map_out, void* base, int64_t M, int64_t N) {
 }
 
 int gb_prepare_gemm() {
-  GB_CUDA_OK(cudaFuncSetAttribute((const void*)gemm_tn_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kGemmSmem));
-  GB_CUDA_OK(cudaFuncSetAttribute((const void*)gemm_tn_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  GB_CUDA_OK(cudaFuncSetAttribute((const void*)gemm_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kGemmSmem + kGroupSmem));
   return GB_OK;
 }
@@ -456,37 +444,12 @@ int gb_gemm_tn(const void* A, const void* B, void* D, int64_t M, int64_t N, int6
              "operands must be 16-byte aligned");
   GB_REQUIRE(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), "dimension too large");
   if (gb_sm_count() <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
-  if (gb_gemm_pair_applies(M)) {
-    const int rc = gb_gemm_pair(A, B, D, M, N, K, kind, a_scale, b_scale, global_scale == 0.0f ? 1.0f : global_scale,
-                                (cudaStream_t)stream);
+  const float gs = global_scale == 0.0f ? 1.0f : global_scale;
+  if (!gb_gemm_rows_applies(false, M, N, K * eb / kSlabBytes)) {
+    const int rc = gb_gemm_pair(A, B, D, M, N, K, kind, a_scale, b_scale, gs, (cudaStream_t)stream);
     if (rc != GB_EUNSUPPORTED) return rc;
   }
-  CUtensorMap map_a, map_b;
-  int rc = make_map(&map_a, A, M, K, eb, kBM);
-  if (rc != GB_OK) return rc;
-  rc = make_map(&map_b, B, N, K, eb, kBN);
-  if (rc != GB_OK) return rc;
-  GemmParams p = {};
-  p.M = M; p.N = N; p.K = K;
-  p.k_tiles = (int)(K * eb / kSlabBytes);
-  p.m_tiles = (int)((M + kBM - 1) / kBM);
-  p.n_tiles = (int)((N + kBN - 1) / kBN);
-  p.elem_bytes = eb;
-  // instruction descriptor: fp32 accumulate, A/B format, both K-major, N >> 3, M >> 4
-  p.idesc = (1u << 4) | ((kind == GB_GEMM_BF16 ? 1u : 0u) << 7) | ((kind == GB_GEMM_BF16 ? 1u : 0u) << 10) |
-            ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-  p.a_scale = a_scale; p.b_scale = b_scale;
-  p.global_scale = global_scale == 0.0f ? 1.0f : global_scale;
-  p.D = (uint16_t*)D;
-  p.status = gb_status_word();
-  const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
-  GB_REQUIRE(tiles < (1ll << 31), "too many output tiles");
-  const int sms = gb_sm_count();
-  dim3 grid((unsigned)(tiles < sms ? tiles : sms));          // persistent: one CTA per SM
-  gb_count_launch();
-  gemm_tn_kernel<false><<<grid, kGemmThreads, kGemmSmem, (cudaStream_t)stream>>>(map_a, map_b, p);
-  GB_LAUNCH_OK("gemm_tn_kernel");
-  return GB_OK;
+  return gb_gemm_rows(A, B, D, M, N, K, kind, a_scale, b_scale, gs, (cudaStream_t)stream);
 }
 
 int gb_gemm_tn_grouped(const void* A, const void* B, void* D, int64_t P, int64_t N, int64_t K, int kind, int64_t E,
@@ -511,7 +474,6 @@ int gb_gemm_tn_grouped(const void* A, const void* B, void* D, int64_t P, int64_t
   GemmParams p = {};
   p.M = P; p.N = N; p.K = K;
   p.k_tiles = (int)(K * eb / kSlabBytes);
-  p.m_tiles = 0;                                   // counted on the device from seg_offsets
   p.n_tiles = (int)((N + kBN - 1) / kBN);
   p.elem_bytes = eb;
   p.idesc = (1u << 4) | ((kind == GB_GEMM_BF16 ? 1u : 0u) << 7) | ((kind == GB_GEMM_BF16 ? 1u : 0u) << 10) |
@@ -527,8 +489,8 @@ int gb_gemm_tn_grouped(const void* A, const void* B, void* D, int64_t P, int64_t
   const int sms = gb_sm_count();
   dim3 grid((unsigned)(tiles < sms ? tiles : sms));
   gb_count_launch();
-  gemm_tn_kernel<true><<<grid, kGemmThreads, kGemmSmem + kGroupSmem, (cudaStream_t)stream>>>(map_a, map_b, p);
-  GB_LAUNCH_OK("gemm_tn_kernel<grouped>");
+  gemm_tn_kernel<<<grid, kGemmThreads, kGemmSmem + kGroupSmem, (cudaStream_t)stream>>>(map_a, map_b, p);
+  GB_LAUNCH_OK("gemm_tn_kernel");
   return GB_OK;
 }
 

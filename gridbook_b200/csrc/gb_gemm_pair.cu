@@ -699,10 +699,6 @@ int gb_prepare_gemm_pair() {
   return GB_OK;
 }
 
-// From 129 rows on: with fewer, half of the pair's rows would be padding and the other kernel's
-// 128-row tiles do the same work on twice as many independent CTAs.
-bool gb_gemm_pair_applies(int64_t M) { return M > kBM; }
-
 namespace {
 // Width of a tile: 256 columns, or 192 where that saves more of the last wave than the sixth of extra
 // operand traffic costs (columns per pair and wave, 5% in favour of 256: 333 x 5120 x 17408 fp4 34 -> 32 us
