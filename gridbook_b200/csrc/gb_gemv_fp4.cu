@@ -61,7 +61,7 @@ constexpr uint32_t kDynBase = 0x400u;                     // dynamic shared memo
 constexpr uint32_t kSmemMax = 227 * 1024;
 constexpr uint32_t kSmemEnd = kDynBase + kSmemMax;
 constexpr uint32_t kLut = 0x800u;                         // shared-window address of the lookup tables, behind the barriers
-constexpr int kMaxRoles = GB_MAX_ROLES;
+constexpr int kMaxRoles = GB_MAX_ROLES;                     // and no fewer than matrices, which count as roles
 constexpr int kMaxSlices = 8;
 
 enum { kLit = 8 };                                        // other formats: the product format's k
@@ -89,10 +89,22 @@ template <int F> struct Geo {
   static_assert(kPitch <= 256 && (kPitch / 16) % 2 == 1, "row pitch");
 };
 
-struct Role { int row0, rows, tile0; int64_t cb; };        // rows that share a codebook; first tile; element offset
+constexpr int kMaxMatrices = 4;
+// A matrix of the launch: several that read the same activation rows go out together.
+struct Matrix {
+  const uint8_t* qw;         // packed rows, once more for groups left out
+  int64_t row_stride, N;
+  const void* codebook;      // bf16 flat
+  const float* compose;
+  float global_scale;
+  uint16_t* y;
+};
+struct Maps { CUtensorMap m[kMaxMatrices]; };
+struct Role { int mat, row0, rows, tile0; int64_t cb; };   // rows of a matrix that share a codebook; first tile; element offset
 
 struct Fp4Params {
-  int64_t N, K;
+  Matrix mat[kMaxMatrices];  // grouped: the first is the stack, N the rows of an expert
+  int64_t K;
   int M;                     // dense: activation rows
   int n_sb, units;           // superblocks per row / per K slice (the last slice may have fewer)
   int slices;                // = cluster size along y
@@ -103,12 +115,6 @@ struct Fp4Params {
   int64_t x_unit;            // bytes of one superblock of it
   const float* x_scale;      // [tile][pass_rows] power of two of every row; low bits: where groups are left out
   const float* tail;         // [tile][pass_rows][K / 16] scales of the groups left out, of the rows that have any
-  const uint8_t* qw;         // the packed rows again, for those
-  int64_t row_stride;
-  const void* codebook;      // bf16 flat
-  const float* compose;
-  float global_scale;
-  uint16_t* y;
   int* status;
   int n_roles, n_tiles;
   Role role[kMaxRoles];
@@ -359,12 +365,12 @@ GB_DEVINL uint32_t four_scales(uint4 t, uint32_t c) {
 
 // The E4M3 byte of every (super, sub) pair of the two-tier formats.
 template <int F>
-GB_DEVINL void build_scale_tab(const Fp4Params& p, int d, uint32_t scale_tab) {
+GB_DEVINL void build_scale_tab(const float* compose, int d, uint32_t scale_tab) {
   if constexpr (F != kLit) {
     for (int i = d * 4; i < 4096; i += 4 * 32 * kDecWarps) {
       uint32_t w = 0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) w |= gb_f32_to_e4m3(fminf(__ldg(p.compose + i + j), 448.0f)) << (8 * j);
+      for (int j = 0; j < 4; ++j) w |= gb_f32_to_e4m3(fminf(__ldg(compose + i + j), 448.0f)) << (8 * j);
       asm volatile("st.shared.u32 [%0], %1;" ::"r"(scale_tab + (uint32_t)i), "r"(w) : "memory");
     }
   }
@@ -412,7 +418,7 @@ GB_DEVINL float dot16(const RowGroup& r, float x) {
 
 template <bool kGrouped, bool kWide, int F>
 __global__ void __launch_bounds__(kThreads, 1)
-fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Fp4Params p) {
+fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4Params p) {
   using T = Fmt<F>;
   using G = Geo<F>;
   extern __shared__ uint8_t smem_raw[];
@@ -498,8 +504,8 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     // the tables need nothing of an earlier launch, the segment offsets do: every role looks through the
     // experts for its tiles, so they are copied next to it (ten tiles a CTA, 500 clocks each from L2)
     if (warp >= kCtlWarps) {
-      build_scale_tab<F>(p, threadIdx.x - 32 * kCtlWarps, scale_tab);
-      build_lut<F, kWide>(reinterpret_cast<const uint16_t*>(p.codebook), threadIdx.x - 32 * kCtlWarps, kLut | win);
+      build_scale_tab<F>(p.mat[0].compose, threadIdx.x - 32 * kCtlWarps, scale_tab);
+      build_lut<F, kWide>(reinterpret_cast<const uint16_t*>(p.mat[0].codebook), threadIdx.x - 32 * kCtlWarps, kLut | win);
       have_role = 0;
     }
     gb_pdl_wait();
@@ -514,14 +520,14 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"((p.seg_off | win) + 4u * (uint32_t)e));
     return v;
   };
-  struct Tile { int n0, n_end, w_row0, lo, cnt, n_pass, x_tile, role; };
+  struct Tile { int n0, n_end, w_row0, lo, cnt, n_pass, x_tile, role; };   // role 0: grouped
   auto tile_at = [&](int t) {
     Tile R;
     if (kGrouped) {
       const int e = t / p.tiles_n;
       R.n0 = (t - e * p.tiles_n) * kBM;
-      R.n_end = (int)p.N;
-      R.w_row0 = e * (int)p.N + R.n0;
+      R.n_end = (int)p.mat[0].N;
+      R.w_row0 = e * (int)p.mat[0].N + R.n0;
       R.lo = seg_at(e);
       R.cnt = seg_at(e + 1) - R.lo;
       R.n_pass = R.cnt > 0 ? (R.cnt + p.pass_rows - 1) / p.pass_rows : 0;
@@ -556,7 +562,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
           if (!ok) break;                                  // no copy may be in flight when the CTA leaves
           if (leader) {
             mbar_expect(raw_full + 8 * s, G::kBoxBytes);
-            tma_load_2d(raw_ring + (uint32_t)s * G::kBoxBytes, &map_w, (sb_begin + u) * T::kSb, R.w_row0, raw_full + 8 * s);
+            tma_load_2d(raw_ring + (uint32_t)s * G::kBoxBytes, &maps.m[kGrouped ? 0 : p.role[R.role].mat], (sb_begin + u) * T::kSb, R.w_row0, raw_full + 8 * s);
           }
           __syncwarp();
         }
@@ -684,7 +690,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t buf = lane_base + buf_col0 + (uint32_t)wg * buf_stride;
     const uint32_t lane4 = win | (F == kLit || kByteCodes<F, kWide> ? (uint32_t)lane * 4u : (uint32_t)(lane & ((int)(T::kStride / 4) - 1)) * 4u);
-    if (!kGrouped) build_scale_tab<F>(p, d, scale_tab);
+    int have_mat = kGrouped ? 0 : -1;                        // whose scale table it is
     bool waited = false;
     float xs0 = 0.0f, xs1 = 0.0f;                            // scale words of rows lane, lane + 32
     int item = 0, g0 = 0;                                    // items and units so far
@@ -714,7 +720,10 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       const bool live = t < p.n_tiles;
       if (live && R.role != have_role) {                     // the CTA's rows change codebook
         if (have_role >= 0) asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
-        build_lut<F, kWide>(reinterpret_cast<const uint16_t*>(p.codebook) + p.role[R.role].cb, d, kLut | win);
+        const Matrix& W = p.mat[p.role[R.role].mat];
+        if (F != kLit && p.role[R.role].mat != have_mat) build_scale_tab<F>(W.compose, d, scale_tab);
+        have_mat = p.role[R.role].mat;
+        build_lut<F, kWide>(reinterpret_cast<const uint16_t*>(W.codebook) + p.role[R.role].cb, d, kLut | win);
         have_role = R.role;
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecWarps) : "memory");
       }
@@ -814,6 +823,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
               }
             }
             const Tile Q = tile_at(out_t);
+            const Matrix& W = p.mat[kGrouped ? 0 : p.role[Q.role].mat];
             const int rows = min(p.pass_rows, Q.cnt - out_pass * p.pass_rows);
             int to0 = lane, to1 = lane + 32;                 // output rows
             if (kGrouped) {
@@ -839,8 +849,8 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
               // with nothing held over it: as a function, or with the sums in registers, it cost the ordinary read-out
               // its registers (two layers at 16 rows 164 -> 188..208 us, this way 167..169).
               const int64_t tile = Q.x_tile + (kGrouped ? q_pass : 0);
-              const uint8_t* w_row = p.qw + (Q.w_row0 + (kGrouped ? row : min(row, (int)p.N - 1 - Q.n0))) * p.row_stride;
-              const uint16_t* cb = reinterpret_cast<const uint16_t*>(p.codebook) + p.role[Q.role].cb;
+              const uint8_t* w_row = W.qw + (Q.w_row0 + (kGrouped ? row : min(row, (int)W.N - 1 - Q.n0))) * W.row_stride;
+              const uint16_t* cb = reinterpret_cast<const uint16_t*>(W.codebook) + p.role[Q.role].cb;
               const int per = gb_left_out_span(p.n_sb);
 #pragma unroll 1
               for (int j = 0; j < (wide ? 4 : 1); ++j) {
@@ -865,7 +875,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                       [&](int r, int g) {
                         return *reinterpret_cast<const uint2*>(p.xop + (tile * p.n_sb + (g >> 4)) * p.x_unit + sfx + code_at(n0 + r, g & 15));
                       },
-                      [&](int g) { return row_group<F>(w_row, cb, p.compose, g); }, [](const RowGroup& r, float x) { return dot16(r, x); });
+                      [&](int g) { return row_group<F>(w_row, cb, W.compose, g); }, [](const RowGroup& r, float x) { return dot16(r, x); });
                 }
 #pragma unroll
                 for (int r = 0; r < 4; ++r) add[r] = gb_normalised(add[r], word[r]);
@@ -945,17 +955,17 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 }
               } else {
                 const bool mine = ok && col < Q.n_end;
-                uint16_t* y = p.y + (kGrouped ? 0 : (int64_t)m0 * p.N) + col;
+                uint16_t* y = W.y + (kGrouped ? 0 : (int64_t)m0 * W.N) + col;
 #pragma unroll
                 for (int i = 0; i < kRows; ++i) {
                   const int m = m0 + i;
-                  const uint16_t b = (uint16_t)gb_f32_to_bf16_bits(val[i] * p.global_scale);
+                  const uint16_t b = (uint16_t)gb_f32_to_bf16_bits(val[i] * W.global_scale);
                   if (kGrouped) {
                     const int orow = __shfl_sync(0xffffffffu, m < 32 ? to0 : to1, m & 31);
-                    if (m < rows && mine) y[(int64_t)orow * p.N] = b;
+                    if (m < rows && mine) y[(int64_t)orow * W.N] = b;
                   } else {
                     if (m < rows && mine) *y = b;
-                    y += p.N;
+                    y += W.N;
                   }
                 }
               }
@@ -984,7 +994,7 @@ fp4_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"((p.red_off | win) + (uint32_t)((own * p.slices + q) * kBM + r) * 4u));
                   s += f;
                 }
-                if (*abort_flag == 0 && Q.n0 + r < Q.n_end) p.y[(int64_t)m * p.N + Q.n0 + r] = (uint16_t)gb_f32_to_bf16_bits(s * p.global_scale);
+                if (*abort_flag == 0 && Q.n0 + r < Q.n_end) W.y[(int64_t)m * W.N + Q.n0 + r] = (uint16_t)gb_f32_to_bf16_bits(s * W.global_scale);
               }
             }
           }
@@ -1435,7 +1445,7 @@ int max_clusters(int size) {
 }
 
 template <bool kGrouped>
-cudaError_t launch(int F, dim3 grid, cudaStream_t stream, const CUtensorMap& map_w, const Fp4Params& p) {
+cudaError_t launch(int F, dim3 grid, cudaStream_t stream, const Maps& maps, const Fp4Params& p) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads);
@@ -1458,8 +1468,8 @@ cudaError_t launch(int F, dim3 grid, cudaStream_t stream, const CUtensorMap& map
   const bool wide = is_wide(p.pass_rows);
   switch (F) {
 #define GB_FP4_LAUNCH(f)                                                                       \
-  return wide ? cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, true, f>, map_w, p)       \
-              : cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, false, f>, map_w, p)
+  return wide ? cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, true, f>, maps, p)       \
+              : cudaLaunchKernelEx(&cfg, fp4_decode_kernel<kGrouped, false, f>, maps, p)
     case kLit: GB_FP4_LAUNCH(kLit);
     case 12: GB_FP4_LAUNCH(12);
     case 16: GB_FP4_LAUNCH(16);
@@ -1539,46 +1549,49 @@ int64_t gb_gemv_fp4_workspace_bytes(int64_t M, int64_t K) {
   return align256((K / 256) * unit_bytes(is_wide(rows), rows)) + align256(rows * 4) + align256(rows * (K / 16) * 4);
 }
 
-int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, int n_roles, const int64_t* role_rows,
-                int scale_rule, void* y, void* workspace, int64_t workspace_bytes, void* stream_) {
-  const int F = fp4_format(w, scales_e4m3);
-  if (F < 0 || ((uintptr_t)x & 15u) != 0 || n_roles > kMaxRoles || (n_roles <= 1 && w->cb_row_offset != nullptr)) return GB_EUNSUPPORTED;
+namespace {
+// y_i[M, N_i] for matrices of one format and width: the rows' operand once, then one launch.  Roles: of a single matrix.
+int gemv_fp4(const void* x, int64_t M, const gb_weight* const* w, int n_mat, bool scales_e4m3, int n_roles, const int64_t* role_rows,
+             int scale_rule, void* const* y, void* workspace, int64_t workspace_bytes, void* stream_) {
+  const int F = fp4_format(w[0], scales_e4m3);
   const int sms = gb_sm_count();
   if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
-  if (workspace == nullptr || workspace_bytes < gb_gemv_fp4_workspace_bytes(M, w->K))
+  if (workspace == nullptr || workspace_bytes < gb_gemv_fp4_workspace_bytes(M, w[0]->K))
     return gb_fail(GB_EWORKSPACE, "workspace of %lld bytes is too small (need %lld)", (long long)workspace_bytes,
-                   (long long)gb_gemv_fp4_workspace_bytes(M, w->K));
-  const Info f = info(F, is_wide((int)(M < kMaxRows ? M : kMaxRows)));
+                   (long long)gb_gemv_fp4_workspace_bytes(M, w[0]->K));
   cudaStream_t stream = (cudaStream_t)stream_;
-  CUtensorMap map_w;
-  int rc = gb_tensor_map_bytes_2d(&map_w, w->qw, (uint64_t)(w->K / 256) * f.sb, (uint64_t)w->rows, (uint64_t)w->row_stride, f.pitch, kBM);
-  if (rc != GB_OK) return rc;
+  const int64_t K = w[0]->K;
+  Maps maps;
+  for (int i = 0; i < n_mat; ++i) {
+    const Info f = info(F, false);                         // the packed rows are read alike
+    const int rc = gb_tensor_map_bytes_2d(&maps.m[i], w[i]->qw, (uint64_t)(K / 256) * f.sb, (uint64_t)w[i]->rows, (uint64_t)w[i]->row_stride, f.pitch, kBM);
+    if (rc != GB_OK) return rc;
+  }
+  for (int i = n_mat; i < kMaxMatrices; ++i) maps.m[i] = maps.m[0];
   for (int64_t m0 = 0; m0 < M; m0 += kMaxRows) {
     Fp4Params p = {};
-    p.N = w->rows; p.K = w->K;
+    p.K = K;
     p.M = (int)(M - m0 < kMaxRows ? M - m0 : kMaxRows);
-    p.n_sb = (int)(w->K / 256);
+    p.n_sb = (int)(K / 256);
     p.pass_rows = p.M;
     p.x_unit = unit_bytes(is_wide(p.M), p.M);
     p.xop = (const uint8_t*)workspace;
     p.x_scale = (const float*)((const uint8_t*)workspace + align256(p.n_sb * p.x_unit));
     p.tail = (const float*)((const uint8_t*)p.x_scale + align256(p.M * 4));
-    p.qw = w->qw;
-    p.row_stride = w->row_stride;
-    p.codebook = w->codebook;
-    p.compose = w->compose;
-    p.global_scale = w->global_scale == 0.0f ? 1.0f : w->global_scale;
-    p.y = (uint16_t*)y + m0 * w->rows;
     p.status = gb_status_word();
-    p.n_roles = n_roles < 1 ? 1 : n_roles;
-    int64_t row = 0;
-    for (int r = 0; r < p.n_roles; ++r) {
-      const int64_t rows = n_roles < 1 ? w->rows : role_rows[r];
-      p.role[r] = {(int)row, (int)rows, p.n_tiles, r * gb_codebook_elems(w->fmt)};
-      p.n_tiles += (int)((rows + kBM - 1) / kBM);
-      row += rows;
+    for (int i = 0; i < n_mat; ++i) {
+      p.mat[i] = {w[i]->qw, w[i]->row_stride, w[i]->rows, w[i]->codebook, w[i]->compose, w[i]->global_scale == 0.0f ? 1.0f : w[i]->global_scale,
+                  (uint16_t*)y[i] + m0 * w[i]->rows};
+      int64_t row = 0;
+      for (int r = 0; r < (n_roles < 1 ? 1 : n_roles); ++r) {
+        const int64_t rows = n_roles < 1 ? w[i]->rows : role_rows[r];
+        p.role[p.n_roles++] = {i, (int)row, (int)rows, p.n_tiles, r * gb_codebook_elems(w[i]->fmt)};
+        p.n_tiles += (int)((rows + kBM - 1) / kBM);
+        row += rows;
+      }
+      GB_REQUIRE(row == w[i]->rows, "the roles hold %lld rows, the matrix %lld", (long long)row, (long long)w[i]->rows);
     }
-    GB_REQUIRE(row == w->rows, "the roles hold %lld rows, the matrix %lld", (long long)row, (long long)w->rows);
+    const Info f = info(F, is_wide(p.M));
     // K slices: enough CTAs for the SMs when there are few tiles; no more clusters than run at once,
     // at least two superblocks per slice
     int want = 1;
@@ -1587,20 +1600,28 @@ int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, 
     p.units = (p.n_sb + want - 1) / want;
     p.units = (p.units + f.per_stage - 1) / f.per_stage * f.per_stage;
     p.slices = (p.n_sb + p.units - 1) / p.units;
-    if (!layout(info(F, is_wide(p.M)), p)) return gb_fail(GB_EUNSUPPORTED, "no shared-memory layout for %d rows", p.M);
+    if (!layout(f, p)) return gb_fail(GB_EUNSUPPORTED, "no shared-memory layout for %d rows", p.M);
     RowsParams rp = {};
-    rp.x = (const uint4*)((const uint16_t*)x + m0 * w->K);
+    rp.x = (const uint4*)((const uint16_t*)x + m0 * K);
     rp.xop = (uint8_t*)workspace;
     rp.x_scale = const_cast<float*>(p.x_scale);
     rp.tail = const_cast<float*>(p.tail);
     rp.x_unit = p.x_unit;
-    rp.K = (int)w->K; rp.n_sb = p.n_sb; rp.scale_rule = scale_rule; rp.pass_rows = p.pass_rows; rp.rows = p.M;
-    rc = launch_rows<0>(p.M, w->K, stream, rp);
+    rp.K = (int)K; rp.n_sb = p.n_sb; rp.scale_rule = scale_rule; rp.pass_rows = p.pass_rows; rp.rows = p.M;
+    const int rc = launch_rows<0>(p.M, K, stream, rp);
     if (rc != GB_OK) return rc;
     const int ctas = p.slices > 1 || p.n_tiles <= sms ? p.n_tiles : sms;
-    GB_CUDA_OK(launch<false>(F, dim3((unsigned)ctas, (unsigned)p.slices), stream, map_w, p));
+    GB_CUDA_OK(launch<false>(F, dim3((unsigned)ctas, (unsigned)p.slices), stream, maps, p));
   }
   return GB_OK;
+}
+}  // namespace
+
+int gb_gemv_fp4(const void* x, int64_t M, const gb_weight* w, bool scales_e4m3, int n_roles, const int64_t* role_rows,
+                int scale_rule, void* y, void* workspace, int64_t workspace_bytes, void* stream) {
+  if (fp4_format(w, scales_e4m3) < 0 || ((uintptr_t)x & 15u) != 0 || n_roles > kMaxRoles || (n_roles <= 1 && w->cb_row_offset != nullptr))
+    return GB_EUNSUPPORTED;
+  return gemv_fp4(x, M, &w, 1, scales_e4m3, n_roles, role_rows, scale_rule, &y, workspace, workspace_bytes, stream);
 }
 
 // ---- routed experts ------------------------------------------------------------------------------
@@ -1673,6 +1694,24 @@ int gb_gemv_hinted(const void* x, int64_t M, const gb_weight* w, const gb_hints*
     if (rc != GB_EUNSUPPORTED) return rc;
   }
   return gb_gemv(x, M, w, act, scale_rule, y, workspace, workspace_bytes, stream);
+}
+
+int gb_gemv_shared(const void* x, int64_t M, const gb_weight* const* w, int n_weights, int scales_e4m3, int scale_rule, void* const* y,
+                   void* workspace, int64_t workspace_bytes, void* stream) {
+  GB_REQUIRE(x && w && y, "null pointer argument");
+  GB_REQUIRE(n_weights >= 1 && n_weights <= kMaxMatrices, "1..%d matrices per call, got %d", kMaxMatrices, n_weights);
+  GB_REQUIRE(M >= 1 && M <= 128, "decode-batch kernels take 1..128 rows, got M=%lld", (long long)M);
+  for (int i = 0; i < n_weights; ++i) {
+    const int rc = gb_check_weight(w[i]);
+    if (rc != GB_OK) return rc;
+    GB_REQUIRE(y[i] != nullptr, "null output %d", i);
+    GB_REQUIRE(w[i]->K == w[0]->K, "matrix %d has K=%lld, matrix 0 K=%lld: they must read the same rows", i, (long long)w[i]->K, (long long)w[0]->K);
+    if (!gb_gemv_fp4_applies(w[i], scales_e4m3 != 0) || fp4_format(w[i], scales_e4m3 != 0) != fp4_format(w[0], scales_e4m3 != 0) ||
+        w[i]->cb_row_offset != nullptr)
+      return GB_EUNSUPPORTED;
+  }
+  if (((uintptr_t)x & 15u) != 0) return GB_EUNSUPPORTED;
+  return gemv_fp4(x, M, w, n_weights, scales_e4m3 != 0, 0, nullptr, scale_rule, y, workspace, workspace_bytes, stream);
 }
 
 int gb_moe_fp4_pass_rows(const gb_weight* w, int scales_e4m3, int64_t P, int64_t E) {
@@ -1751,17 +1790,13 @@ int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, in
   const Info f = info(F, is_wide(pass_rows));
   const int64_t tiles = P / pass_rows + E + 1;
   Fp4Params p = {};
-  p.N = N; p.K = K; p.n_sb = (int)(K / 256); p.units = p.n_sb; p.slices = 1;
+  p.K = K; p.n_sb = (int)(K / 256); p.units = p.n_sb; p.slices = 1;
   p.pass_rows = pass_rows;
   p.x_unit = unit_bytes(is_wide(pass_rows), pass_rows);
   p.xop = (const uint8_t*)operand;
   p.x_scale = (const float*)((const uint8_t*)operand + align256(tiles * p.n_sb * p.x_unit));
   p.tail = (const float*)((const uint8_t*)p.x_scale + align256(tiles * pass_rows * 4));
-  p.qw = w->qw;
-  p.row_stride = w->row_stride;
-  p.codebook = w->codebook; p.compose = w->compose;
-  p.global_scale = w->global_scale == 0.0f ? 1.0f : w->global_scale;
-  p.y = (uint16_t*)y;
+  p.mat[0] = {w->qw, w->row_stride, N, w->codebook, w->compose, w->global_scale == 0.0f ? 1.0f : w->global_scale, (uint16_t*)y};
   p.status = gb_status_word();
   p.n_roles = 1;
   p.seg = seg; p.row_map = row_map;
@@ -1769,10 +1804,11 @@ int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, in
   p.n_tiles = (int)(E * p.tiles_n);
   p.E = (int)E;
   if (!layout(f, p)) return gb_fail(GB_EUNSUPPORTED, "no shared-memory layout for %d rows per pass", pass_rows);
-  CUtensorMap map_w;
-  rc = gb_tensor_map_bytes_2d(&map_w, w->qw, (uint64_t)p.n_sb * f.sb, (uint64_t)(E * N), (uint64_t)w->row_stride, f.pitch, kBM);
+  Maps maps;
+  rc = gb_tensor_map_bytes_2d(&maps.m[0], w->qw, (uint64_t)p.n_sb * f.sb, (uint64_t)(E * N), (uint64_t)w->row_stride, f.pitch, kBM);
   if (rc != GB_OK) return rc;
-  GB_CUDA_OK(launch<true>(F, dim3((unsigned)(p.n_tiles < sms ? p.n_tiles : sms)), (cudaStream_t)stream_, map_w, p));
+  for (int i = 1; i < kMaxMatrices; ++i) maps.m[i] = maps.m[0];
+  GB_CUDA_OK(launch<true>(F, dim3((unsigned)(p.n_tiles < sms ? p.n_tiles : sms)), (cudaStream_t)stream_, maps, p));
   return GB_OK;
 }
 

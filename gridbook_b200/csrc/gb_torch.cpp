@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <pybind11/stl.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <atomic>
@@ -38,7 +39,7 @@ namespace {
   F(gb_last_error) F(gb_gemv_hinted_workspace_bytes) F(gb_gemv) F(gb_gemv_row_batch_max) F(gb_gemv_tab) \
   F(gb_gemv_tab_slots_bytes) F(gb_fp4_act_qdq) F(gb_fp8_act_qdq) F(gb_fp8_quantize_rows) F(gb_nvfp4_sf_bytes) \
   F(gb_nvfp4_quantize_rows) F(gb_expand_fp4_nvfp4) F(gb_expand_fp4_bf16) F(gb_expand_fp8) F(gb_expand_fp8_bf16) \
-  F(gb_expand_fp4_nvfp4_beside) F(gb_expand_fp8_beside) F(gb_gemm_fp4) F(gb_gemm_tn) F(gb_gemm_tn_grouped) F(gb_moe_route_ws) F(gb_moe_route_workspace_bytes) \
+  F(gb_gemv_shared) F(gb_expand_fp4_nvfp4_beside) F(gb_expand_fp8_beside) F(gb_gemm_fp4) F(gb_gemm_tn) F(gb_gemm_tn_grouped) F(gb_moe_route_ws) F(gb_moe_route_workspace_bytes) \
   F(gb_moe_gather_rows) F(gb_moe_swiglu_rows) F(gb_moe_gemv) F(gb_moe_gemv_sorted) F(gb_moe_mlp_pairs) \
   F(gb_moe_mlp_pairs_workspace_bytes) F(gb_moe_combine) F(gb_gemv_hinted) F(gb_scales_e4m3) F(gb_moe_route_inv) \
   F(gb_moe_fp4_pass_rows) F(gb_moe_fp4_operand_bytes) F(gb_moe_fp4_rows) F(gb_moe_fp4_swiglu_rows) \
@@ -271,11 +272,89 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
 
 std::atomic<int64_t> LinearPlan::next_serial{0};
 
-// Several linears that read the same activation row, one launch; None when they have no such kernel.
-py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, const at::Tensor& x, int rule) {
+// Whether a layer's prefill of the fp4 grid quantises its rows to NVFP4, and its largest decode batch.
+using Route = std::pair<bool, int64_t>;
+
+// Several linears that read the same rows: the rows are bucketed or quantised once, and the decode batches of the fp4 formats
+// go out as one launch (two layers of K16 at 16 rows 137 -> 127 us, one literal layer at 64 rows 91 -> 81).  None: one by one.
+py::object shared_rows(const std::vector<std::shared_ptr<LinearPlan>>& plans, const at::Tensor& x, int rule, const std::vector<Route>& routes) {
+  const size_t n = plans.size();
+  const int64_t K = plans[0]->w.w.K, M = x.numel() / K;
+  if (x.size(-1) != K || M < 1 || routes.size() != n || x.scalar_type() != at::kBFloat16) return py::none();
+  bool decode = true, prefill = true;
+  for (size_t i = 0; i < n; ++i) {
+    const LinearPlan& p = *plans[i];
+    if (p.w.w.K != K || p.w.fp4() != plans[0]->w.fp4() || routes[i].first != routes[0].first) return py::none();
+    const bool few = M <= kDecodeMaxRows || M <= std::min(routes[i].second, p.row_batch_max);
+    decode = decode && few && p.hints.n_roles <= 1 && p.w.w.cb_row_offset == nullptr && p.w.scales_e4m3 == plans[0]->w.scales_e4m3;
+    prefill = prefill && !few;
+  }
+  const bool fp4 = plans[0]->w.fp4();
+  if (!decode && !(prefill && (routes[0].first || !fp4))) return py::none();
+  const c10::cuda::CUDAGuard guard(x.device());
+  void* stream = c10::cuda::getCurrentCUDAStream().stream();
+  const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+  const gb_weight* ws[4];
+  void* ys[4];
+  std::vector<at::Tensor> outs;
+  for (size_t i = 0; i < n; ++i) {
+    std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = plans[i]->w.w.rows;
+    outs.push_back(at::empty(shape, x.options()));
+    ws[i] = &plans[i]->w.w;
+    ys[i] = outs.back().data_ptr();
+  }
+  Arena a;
+  if (decode && fp4) {
+    const int scratch = a.add(L.gb_gemv_hinted_workspace_bytes(M, ws[0]->rows, K));
+    a.alloc(xc);
+    const int rc = L.gb_gemv_shared(xc.data_ptr(), M, ws, (int)n, plans[0]->w.scales_e4m3 ? 1 : 0, rule, ys, a.ptr(scratch),
+                                    L.gb_gemv_hinted_workspace_bytes(M, ws[0]->rows, K), stream);
+    if (rc == GB_EUNSUPPORTED) return py::none();
+    check(rc);
+  } else if (decode) {
+    int64_t need = 0;
+    for (size_t i = 0; i < n; ++i) need = std::max(need, L.gb_gemv_hinted_workspace_bytes(M, ws[i]->rows, K));
+    const int xq = a.add(M * K * 2), scratch = a.add(need);
+    a.alloc(xc);
+    check(L.gb_fp8_act_qdq(xc.data_ptr(), a.ptr(xq), M, K, rule, stream));
+    for (size_t i = 0; i < n; ++i) check(L.gb_gemv(a.ptr(xq), M, ws[i], GB_ACT_NONE, rule, ys[i], a.ptr(scratch), need, stream));
+  } else {
+    if (((uintptr_t)xc.data_ptr() & 15u) != 0) return py::none();
+    const int q = a.add(fp4 ? M * K / 2 : M * K), sf = a.add(fp4 ? L.gb_nvfp4_sf_bytes(M, K) : 0), as = a.add(M * 4);
+    int wq[4], wsf[4];
+    for (size_t i = 0; i < n; ++i) {
+      wq[i] = a.add(fp4 ? ws[i]->rows * K / 2 : ws[i]->rows * K);
+      wsf[i] = a.add(fp4 ? L.gb_nvfp4_sf_bytes(ws[i]->rows, K) : 0);
+    }
+    a.alloc(xc);
+    if (fp4) check(L.gb_nvfp4_quantize_rows(xc.data_ptr(), M, K, kNvfp4ActRange, a.ptr(q), a.ptr(sf), a.ptr<float>(as), stream));
+    else check(L.gb_fp8_quantize_rows(xc.data_ptr(), a.ptr(q), a.ptr<float>(as), M, K, rule, stream));
+    for (size_t i = 0; i < n; ++i) {                       // the first right behind the quantiser, beside it
+      if (fp4) check((i == 0 ? L.gb_expand_fp4_nvfp4_beside : L.gb_expand_fp4_nvfp4)(ws[i], 0, ws[i]->rows, a.ptr(wq[i]), a.ptr(wsf[i]), 2, stream));
+      else check((i == 0 ? L.gb_expand_fp8_beside : L.gb_expand_fp8)(ws[i], 0, ws[i]->rows, a.ptr(wq[i]), stream));
+    }
+    for (size_t i = 0; i < n; ++i) {
+      if (fp4)
+        check(L.gb_gemm_fp4(a.ptr(q), a.ptr(sf), a.ptr(wq[i]), a.ptr(wsf[i]), ys[i], M, ws[i]->rows, K, a.ptr<float>(as), ws[i]->global_scale, stream));
+      else
+        check(L.gb_gemm_tn(a.ptr(q), a.ptr(wq[i]), ys[i], M, ws[i]->rows, K, GB_GEMM_E4M3, a.ptr<float>(as), ws[i]->weight_scale,
+                           ws[i]->global_scale, stream));
+      plans[i]->prefill_route = fp4 ? kRouteNvfp4 : kRouteFp8;
+    }
+  }
+  return py::cast(outs);
+}
+
+// Several linears that read the same activation row, one launch; None when they have no such kernel.  `routes`: of the
+// layers whose calls may be replaced for more rows than one; empty: none.
+py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, const at::Tensor& x, int rule, const std::vector<Route>& routes) {
   const size_t n = plans.size();
   if (n < 2 || n > 4 || !x.is_cuda() || x.dim() < 1) return py::none();
   const int64_t K = plans[0]->w.w.K;
+  bool tables = x.numel() == K;
+  for (const auto& p : plans) tables = tables && p->slots.defined();
+  if (!tables) return shared_rows(plans, x, rule, routes);
   if (x.numel() != K || x.size(-1) != K) return py::none();   // another width: refused where the layers are called one by one
   for (const auto& p : plans)
     if (!p->slots.defined() || p->w.w.K != K) return py::none();
@@ -584,5 +663,5 @@ PYBIND11_MODULE(_gb_torch, m) {
       .def_property_readonly("fp4", &MoEPlan::fp4)
       .def("__call__", &MoEPlan::forward, py::call_guard<py::gil_scoped_release>())
       .def_property_readonly("route", [](const MoEPlan& p) { return p.route.load(); });
-  m.def("shared_row", &shared_row);
+  m.def("shared_row", &shared_row, py::arg("plans"), py::arg("x"), py::arg("rule"), py::arg("routes") = std::vector<Route>());
 }

@@ -191,15 +191,25 @@ class PrismaQuantCBLinearMethod(LinearMethodBase):
         return layer._cb_plan(x, kernels.rule_code(ops.ACT_SCALE_RULE), self.prefill_route == "nvfp4", self.midm_max_rows)
 
 
+def _is_bare(layer) -> bool:
+    """Whether a call of the layer is its plan's and nothing else: no subclass, no replaced method, no hook that wants to see it."""
+    module = torch.nn.modules.module
+    return (type(layer) is CBLinear and type(layer.method) is PrismaQuantCBLinearMethod and "forward" not in layer.__dict__
+            and "apply" not in layer.method.__dict__ and not layer._forward_hooks and not layer._forward_pre_hooks
+            and not module._global_forward_hooks and not module._global_forward_pre_hooks)
+
+
 def apply_shared_row(layers, x: torch.Tensor):
-    """Several CB Linears that read the SAME activation row (q and kv of an attention block, gate
-    and up kept as separate modules): one launch builds the inner-product tables once per CTA and
-    streams all of them.  Falls back to one call per layer when the batch is not a single row or a
-    layer's format has no table kernel.  -> list of outputs, in the order of ``layers``."""
+    """Several CB Linears that read the SAME activation rows (q and kv of an attention block, gate
+    and up kept as separate modules).  One row of the literal format: one launch builds the inner-product tables
+    once per CTA and streams all of them.  More rows: they are bucketed or quantised once, and the decode batches
+    of the fp4 formats go out as one launch.  Falls back to one call per layer where the layers
+    have no such kernel in common, or are more than bare CBLinears.  -> list of outputs, in the order of ``layers``."""
     layers = list(layers)
     plans = [l.__dict__.get("_cb_plan") for l in layers]
     if all(p is not None for p in plans) and kernels.takes_plan(x):
-        outs = _native.host().shared_row(plans, x, kernels.rule_code(ops.ACT_SCALE_RULE))
+        routes = [(l.method.prefill_route == "nvfp4", l.method.midm_max_rows) for l in layers] if all(map(_is_bare, layers)) else []
+        outs = _native.host().shared_row(plans, x, kernels.rule_code(ops.ACT_SCALE_RULE), routes)
         if outs is not None:
             return outs
     return [l(x) for l in layers]
