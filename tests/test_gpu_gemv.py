@@ -384,3 +384,27 @@ def test_two_tier_scale_table_that_is_not_exact_in_bf16_takes_the_fp32_path(dev)
     dp = dict(d, fmt=fmt.padded(80), qw=codec.pad_superblocks(torch.from_numpy(d["qw"]), 73, 80).numpy())
     y = kernels.gemv(synth.bf16_tensor(x, dev), synth.to_device_weight(dp, dev), act="fp4")
     assert_close_bf16(f32_of(y), ref, "inexact table")
+
+
+@pytest.mark.parametrize("E", [1, 7, 128, 256, 257])
+@pytest.mark.parametrize("T,topk", [(1, 1), (31, 1), (33, 1), (1023, 1), (256, 4), (205, 5), (1024, 2), (2049, 2), (1366, 3), (1024, 8), (1025, 8)])
+def test_routing_is_stable_at_every_step_of_the_one_cta_kernels(dev, T, topk, E):
+    """Pairs of one to four steps a warp and past them, experts of the next table and past it, experts without pairs,
+    dropped pairs (below and above the experts), an expert window that starts in the middle."""
+    from gridbook_b200 import kernels
+    rng = np.random.default_rng(T + E)
+    base = 3
+    ids = rng.integers(base - 2, base + E + 2, (T, topk)).astype(np.int32)
+    ids[rng.random((T, topk)) < 0.3] = base + E // 2          # one expert with many pairs
+    flat = ids.reshape(-1) - base
+    live = (flat >= 0) & (flat < E)
+    w = rng.random((T, topk)).astype(np.float32)
+    counts, offsets, order, pair_w = kernels.moe_route(torch.from_numpy(ids).to(dev), E, torch.from_numpy(w).to(dev), expert_base=base)
+    want = np.bincount(flat[live], minlength=E)
+    keyed = np.where(live, flat, E)
+    perm = np.argsort(keyed, kind="stable")[:live.sum()]
+    assert np.array_equal(counts.cpu().numpy(), want)
+    assert np.array_equal(offsets.cpu().numpy(), np.concatenate([[0], np.cumsum(want)]))
+    assert np.array_equal(order.cpu().numpy()[:live.sum()], perm) and not order.cpu().numpy()[live.sum():].any()
+    rounded = torch.from_numpy(w).to(torch.bfloat16).float().numpy().reshape(-1)
+    assert np.array_equal(pair_w.cpu().numpy().reshape(-1), np.where(live, rounded, 0.0).astype(np.float32))
