@@ -16,9 +16,10 @@
 // during the K loop.  Four warpgroups of decoders, one per operand buffer (half a superblock of K,
 // 64 columns), take the units in turn, so decoding, the MMAs of the units before and the loads
 // overlap.  The decoders read the accumulators out at the end (lane = weight row, column =
-// activation row), add them and store bf16, or fp32 partial sums per K slice that a small second
-// kernel adds (summing them in the last CTA of a tile to arrive instead was measured: slower from
-// 16 rows on - one CTA's serial L2 reads against a launch that uses the whole GPU).
+// activation row), add them and store bf16.  A layer with few 128-row tiles is sliced along K over a thread-block
+// cluster: the CTAs push their fp32 sums into the shared memory of the one that owns the activation row, which adds them in
+// slice order (through HBM and a small second launch before: 2048 x 2048 k = 16, 16 rows
+// 6.75 -> 6.23 us, 120 rows 26.1 -> 10.7, 5120 x 17408 K32, 4 rows 25.6 -> 24.8, 8192 x 5120 13.1 -> 13.6).
 //
 // Four packed formats: the literal one (fp4 grid, full k = 8, E4M3 scale bytes: 48-byte
 // superblocks), the two-tier product format fp4 k = 16 with its superblocks padded from 73 to 80
@@ -30,6 +31,7 @@
 #include "gb_common.cuh"
 
 #include <cuda.h>
+#include <mutex>
 
 namespace {
 
@@ -38,6 +40,7 @@ constexpr int kDecWarps = 16;                             // four warpgroups, on
 constexpr int kCtlWarps = 6;                              // raw producer, x producer, four MMA issuers
 constexpr int kUmmaThreads = 32 * (kCtlWarps + kDecWarps);
 constexpr int kMaxRows = 128;                             // activation rows
+constexpr int kMaxSlices = 8;                             // of K: CTAs of a cluster
 constexpr int kABufCols = 64;                             // half a superblock: 128 weights of K as bf16 pairs
 constexpr uint32_t kACol0 = 256;                          // columns [0, 256): one accumulator per MMA issuer
 constexpr uint32_t kTmemCols = 512;
@@ -97,7 +100,6 @@ struct UmmaParams {
   int64_t rows_total;       // rows of the matrix (or of the whole expert stack)
   float global_scale;
   uint16_t* y;              // [M, N] bf16 (one slice)
-  float* partial;           // [slices, M, N] fp32 (several slices)
   uint32_t idesc;            // with N = Mpad (dense); grouped mode sets N per pass
   int* status;
   // grouped mode (routed experts): x rows are sorted by expert, expert e owns rows [seg[e], seg[e+1])
@@ -184,6 +186,16 @@ GB_DEVINL bool elect_one() {
   uint32_t one;
   asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
   return one != 0;
+}
+
+GB_DEVINL void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+GB_DEVINL void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 // The same for the waits on the critical path of every unit: the abort flag is looked at only when
@@ -716,6 +728,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
 
     // ------------------------- read-out ------------------------------------
+    if (!kGrouped && p.slices > 1) break;                    // by the cluster, below
     if (!waited) { gb_pdl_wait(); waited = true; }           // y may still be read by the launch ahead
     wait_or_abort(acc_full, item & 1, abort_flag, p.status, 26);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -757,8 +770,6 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 orow -= home * p.rows_per_rank;
               }
               ybase[orow * p.N + out_col] = (uint16_t)gb_f32_to_bf16_bits(__uint_as_float(v[i]) * p.global_scale);
-            } else if (p.slices > 1) {
-              p.partial[((int64_t)blockIdx.y * p.M + m) * p.N + out_col] = __uint_as_float(v[i]);
             } else {
               p.y[(int64_t)m * p.N + out_col] = (uint16_t)gb_f32_to_bf16_bits(__uint_as_float(v[i]) * p.global_scale);
             }
@@ -773,25 +784,65 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     }
   }
+  if (!kGrouped && p.slices > 1) {
+    // One tile per CTA.  The sums go over the rings: every CTA of the cluster has finished its MMAs, and with them its
+    // loads.  [slice][own row][weight row], rows owned in eights.
+    const Tile T = tile_at(blockIdx.x);
+    const int own = ((p.M + 7) / 8 + p.slices - 1) / p.slices * 8, slice = (int)blockIdx.y;
+    const int w = warp - kCtlWarps, row = (warp & 3) * 32 + lane;
+    const uint32_t sums = gb_smem_u32(xs);
+    if (warp >= kCtlWarps) {
+      wait_or_abort(acc_full, 0, abort_flag, p.status, 26);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    cluster_sync();
+    if (warp >= kCtlWarps && *abort_flag == 0) {
+      const int n_accs = min(p.n_iss, p.n_iss == 4 ? units : sb_slice);
+      const uint32_t acc_stride = kACol0 / (uint32_t)p.n_iss;
+      for (int c = w >> 2; c < (p.M + 7) / 8; c += kDecWarps / 4) {
+        uint32_t v[8];
+        const uint32_t taddr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(c * 8);
+        tmem_ld8(taddr, v);
+        for (int a = 1; a < n_accs; ++a) {                   // the other issuers' accumulators, in their fixed order
+          uint32_t t[8];
+          tmem_ld8(taddr + (uint32_t)a * acc_stride, t);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(t[i]));
+        }
+        const int to = c * 8 / own, at = c * 8 - to * own;
+        uint32_t dst;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(sums + (uint32_t)((slice * own + at) * kBM + row) * 4u), "r"(to));
+#pragma unroll
+        for (int i = 0; i < 8; ++i)                          // rows past the last are sums of zeros
+          asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + (uint32_t)i * kBM * 4u), "r"(v[i]) : "memory");
+      }
+    }
+    cluster_sync();                                          // the last access to another CTA's memory lies in front of it
+    if (warp >= kCtlWarps) {
+      gb_pdl_wait();                                         // y may still be read by the launch ahead
+      const int f = lane * 4, left = T.n_end - T.n0 - f, last = min(own, p.M - slice * own);
+      for (int r = w; r < last && *abort_flag == 0; r += kDecWarps) {
+        float sum[4] = {};
+        for (int q = 0; q < p.slices; ++q) {
+          float v[4];
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(sums + (uint32_t)((q * own + r) * kBM + f) * 4u));
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sum[i] += v[i];
+        }
+        uint16_t* y = p.y + (int64_t)(slice * own + r) * p.N + T.n0 + f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (i < left) y[i] = (uint16_t)gb_f32_to_bf16_bits(sum[i] * p.global_scale);
+      }
+    }
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 2) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols)
                  : "memory");
   }
-}
-
-// y[m][n] = bf16(global_scale * sum over the K slices), in slice order.
-__global__ void __launch_bounds__(256)
-umma_finalize_kernel(const float* __restrict__ partial, int slices, int64_t MN, float global_scale,
-                     uint16_t* __restrict__ y) {
-  gb_pdl_launch_dependents();
-  gb_pdl_wait();
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= MN) return;
-  float acc = 0.0f;
-  for (int s = 0; s < slices; ++s) acc += partial[(int64_t)s * MN + i];
-  y[i] = (uint16_t)gb_f32_to_bf16_bits(acc * global_scale);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -823,13 +874,36 @@ int umma_x_stages(int F, int Mpad) {
 
 int umma_smem_bytes(int F, int Mpad) { return fmt_info(F).fixed_smem + umma_x_stages(F, Mpad) * (2 * Mpad * 128); }
 
-// K slices: enough CTAs for the SMs when the layer has few 128-row tiles.
+std::mutex g_mutex;
+int g_clusters[64][kMaxSlices + 1];                        // clusters of a size that run at once, per device (0: not asked yet)
+
+int max_clusters(int size) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  int& n = g_clusters[dev][size];
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, (unsigned)size);
+    cfg.blockDim = dim3(kUmmaThreads);
+    cfg.dynamicSmemBytes = kSmemCap;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)size; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, umma_decode_kernel<false, kFmtFp8>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
+  }
+  return n;
+}
+
+// K slices: enough CTAs for the SMs when the layer has few 128-row tiles; no more clusters than run at once.
 void umma_plan(int F, int tiles, int n_sb, int sms, int* slices, int* stages_per_slice) {
   const int per_stage = fmt_info(F).sb_per_stage;
   const int n_raw = (n_sb + per_stage - 1) / per_stage;
-  int want = sms / tiles;
-  if (want < 1) want = 1;
-  if (want > n_raw) want = n_raw;
+  int want = 1;
+  for (int s = 2; s <= kMaxSlices && tiles * s <= sms && s <= n_raw; ++s)
+    if (tiles <= max_clusters(s)) want = s;
   *stages_per_slice = (n_raw + want - 1) / want;
   *slices = (n_raw + *stages_per_slice - 1) / *stages_per_slice;
 }
@@ -864,14 +938,33 @@ bool umma_applies(const gb_weight* w, int64_t M, bool roles_known) {
 template <bool kGrouped>
 cudaError_t launch_umma(int F, dim3 grid, size_t smem, cudaStream_t stream, const CUtensorMap& map_w,
                         const CUtensorMap& map_x, const UmmaParams& p) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kUmmaThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (gb_pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (p.slices > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = 1; attr[n].val.clusterDim.y = (unsigned)p.slices; attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  gb_count_launch();
   switch (F) {
-    case kFmtLit: return gb_launch(umma_decode_kernel<kGrouped, kFmtLit>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
-    case kFmtK16: return gb_launch(umma_decode_kernel<kGrouped, kFmtK16>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
+    case kFmtLit: return cudaLaunchKernelEx(&cfg, umma_decode_kernel<kGrouped, kFmtLit>, map_w, map_x, p);
+    case kFmtK16: return cudaLaunchKernelEx(&cfg, umma_decode_kernel<kGrouped, kFmtK16>, map_w, map_x, p);
     case kFmtFp8W:
-      if constexpr (!kGrouped) return gb_launch(umma_decode_kernel<false, kFmtFp8W>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
+      if constexpr (!kGrouped) return cudaLaunchKernelEx(&cfg, umma_decode_kernel<false, kFmtFp8W>, map_w, map_x, p);
       else return cudaErrorInvalidValue;
-    case kFmtF8L: return gb_launch(umma_decode_kernel<kGrouped, kFmtF8L>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
-    default: return gb_launch(umma_decode_kernel<kGrouped, kFmtFp8>, grid, dim3(kUmmaThreads), smem, stream, map_w, map_x, p);
+    case kFmtF8L: return cudaLaunchKernelEx(&cfg, umma_decode_kernel<kGrouped, kFmtF8L>, map_w, map_x, p);
+    default: return cudaLaunchKernelEx(&cfg, umma_decode_kernel<kGrouped, kFmtFp8>, map_w, map_x, p);
   }
 }
 
@@ -902,20 +995,10 @@ int gb_prepare_umma() {
   return GB_OK;
 }
 
-// An upper bound over the formats: the bucketed activations plus one fp32 partial plane per K slice
-// (never more slices than SMs per row tile).
+// The bucketed activations.
 int64_t gb_gemv_umma_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M < 1 || M > kMaxRows || K < 1024 || N < kBM) return 0;
-  const int64_t xq = (M * K * 2 + 255) & ~255ll;
-  int sms = gb_sm_count();
-  if (sms <= 0) sms = 148;
-  int most = 1;
-  for (int F = 0; F < 4; ++F) {
-    int slices, per;
-    umma_plan(F, (int)((N + kBM - 1) / kBM), (int)(K / 256), sms, &slices, &per);
-    if (slices > most) most = slices;
-  }
-  return xq + (most > 1 ? (int64_t)most * M * N * 4 : 0);
+  return (M * K * 2 + 255) & ~255ll;
 }
 
 int gb_gemv_umma(const void* x, int64_t M, const gb_weight* w, int n_roles, const int64_t* role_rows, int act, int scale_rule,
@@ -946,10 +1029,8 @@ int gb_gemv_umma(const void* x, int64_t M, const gb_weight* w, int n_roles, cons
   GB_REQUIRE(row == N, "the roles hold %lld rows, the matrix %lld", (long long)row, (long long)N);
   umma_plan(F, p.n_tiles, p.n_sb, sms, &p.slices, &p.stages_per_slice);
   const int64_t xq_bytes = act == GB_ACT_NONE ? 0 : ((M * K * 2 + 255) & ~255ll);
-  const int64_t part_bytes = p.slices > 1 ? (int64_t)p.slices * M * N * 4 : 0;
-  if (xq_bytes + part_bytes > 0 && (workspace == nullptr || workspace_bytes < xq_bytes + part_bytes))
-    return gb_fail(GB_EWORKSPACE, "workspace of %lld bytes is too small (need %lld)", (long long)workspace_bytes,
-                   (long long)(xq_bytes + part_bytes));
+  if (xq_bytes > 0 && (workspace == nullptr || workspace_bytes < xq_bytes))
+    return gb_fail(GB_EWORKSPACE, "workspace of %lld bytes is too small (need %lld)", (long long)workspace_bytes, (long long)xq_bytes);
   const void* xin = x;
   if (act != GB_ACT_NONE) {
     int rc = act == GB_ACT_FP4_GROUP16 ? gb_fp4_act_qdq(x, workspace, M, K, scale_rule, stream_)
@@ -965,22 +1046,15 @@ int gb_gemv_umma(const void* x, int64_t M, const gb_weight* w, int n_roles, cons
   if (rc != GB_OK) return rc;
   fill_weight_params(p, w, N);
   p.y = (uint16_t*)y;
-  p.partial = p.slices > 1 ? (float*)((uint8_t*)workspace + xq_bytes) : nullptr;
   // fp32 accumulate, bf16 x bf16, both K-major, N = activation rows (padded), M = 128 weight rows
   p.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.Mpad >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
   p.x_stages = umma_x_stages(F, p.Mpad);
   p.n_iss = p.Mpad <= 64 ? 4 : 2;
   p.status = gb_status_word();
-  // one CTA per SM at most: a CTA walks several row tiles when the layer has more of them
-  const int ctas_x = p.n_tiles * p.slices <= sms ? p.n_tiles : (sms / p.slices > 0 ? sms / p.slices : 1);
+  // one CTA per SM at most: a CTA walks several row tiles when the layer has more of them (then there is one K slice)
+  const int ctas_x = p.n_tiles * p.slices <= sms ? p.n_tiles : sms;
   dim3 grid((unsigned)ctas_x, (unsigned)p.slices);
   GB_CUDA_OK(launch_umma<false>(F, grid, (size_t)umma_smem_bytes(F, p.Mpad), (cudaStream_t)stream_, map_w, map_x, p));
-  if (p.slices > 1) {
-    const int64_t MN = M * N;
-    GB_CUDA_OK(gb_launch(umma_finalize_kernel, dim3((unsigned)((MN + 255) / 256)), dim3(256), 0,
-                         (cudaStream_t)stream_, (const float*)p.partial, p.slices, MN, p.global_scale,
-                         (uint16_t*)y));
-  }
   return GB_OK;
 }
 
