@@ -47,6 +47,7 @@ constexpr uint32_t kTmemCols = 512;
 constexpr int kMaxXStages = 8;
 constexpr int kMaxRawStages = 3;
 constexpr int kSmemCap = 227 * 1024;
+constexpr uint32_t kLutAt = 0x400u;                       // where dynamic shared memory starts (checked): the codebook copies
 
 enum { kFmtLit = 0, kFmtK16 = 1, kFmtFp8 = 2, kFmtF8L = 3, kFmtFp8W = 4 };   // Fp8W: Fp8 with twice the copies, for up to 16 rows
 
@@ -303,42 +304,53 @@ GB_DEVINL uint32_t fp8_weight2(uint32_t pair, uint32_t hi2, uint32_t lo2, float 
   return w;
 }
 
-template <int kImm>
+template <uint32_t kImm>
 GB_DEVINL uint32_t lds_at(uint32_t a) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(kImm));
   return v;
 }
 
+template <uint32_t kImm>
+GB_DEVINL uint2 lds2_at(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2+%3];" : "=r"(v.x), "=r"(v.y) : "r"(a), "n"(kImm));
+  return v;
+}
+// Address of a lookup: byte kByte of the code word dropped into byte 1 of the lane's offset (entries are 256 bytes apart), one
+// instruction where a shift, a mask and an addition were three.  34816 x 5120, us, before -> now: K32, 4 rows, two roles 39.8 -> 35.3;
+// k = 16, 16 rows 33.8 -> 31.1, 64 rows 38.1 -> 36.2; 8192 x 5120, K32, 4 rows 13.7 -> 12.1.
+template <int kByte>
+GB_DEVINL uint32_t code_byte(uint32_t w, uint32_t lane) { return __byte_perm(w, lane, 0x7604 | (kByte << 4)); }
+
 // fp8 product format, k = 32: four codewords of four sub-indices; every sub-table entry is two values as
-// bf16.  `lut` is the lane's copy of entry 0 of the first sub-table.
+// bf16.  The copies of an entry of the four sub-tables lie side by side (or, where they are twice as many, of two: the other two
+// 64 KiB on).
+template <int F> constexpr uint32_t kSubAt(int i) {
+  return kLutAt + (Fm<F>::kStride == 128 ? (uint32_t)(i >> 1) * 65536u + (uint32_t)(i & 1) * 128u : (uint32_t)i * 64u);
+}
 template <int F, bool kExact>
-GB_DEVINL void fp8_decode4(uint32_t lut, uint4 cw, uint32_t hi2, uint32_t lo2, float rs, uint32_t (&v)[16]) {
-  constexpr int kShift = Fm<F>::kStride == 128 ? 7 : 6;
-  constexpr uint32_t kMask = 0xFFu << kShift;
+GB_DEVINL void fp8_decode4(uint32_t lane4, uint4 cw, uint32_t hi2, uint32_t lo2, float rs, uint32_t (&v)[16]) {
   const uint32_t w4[4] = {cw.x, cw.y, cw.z, cw.w};
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const uint32_t w = w4[c];
-    v[c * 4 + 0] = fp8_weight2<kExact>(lds_at<0 * 256 * Fm<F>::kStride>(lut + ((w << kShift) & kMask)), hi2, lo2, rs);
-    v[c * 4 + 1] = fp8_weight2<kExact>(lds_at<1 * 256 * Fm<F>::kStride>(lut + ((w >> (8 - kShift)) & kMask)), hi2, lo2, rs);
-    v[c * 4 + 2] = fp8_weight2<kExact>(lds_at<2 * 256 * Fm<F>::kStride>(lut + ((w >> (16 - kShift)) & kMask)), hi2, lo2, rs);
-    v[c * 4 + 3] = fp8_weight2<kExact>(lds_at<3 * 256 * Fm<F>::kStride>(lut + ((w >> (24 - kShift)) & kMask)), hi2, lo2, rs);
+    v[c * 4 + 0] = fp8_weight2<kExact>(lds_at<kSubAt<F>(0)>(code_byte<0>(w, lane4)), hi2, lo2, rs);
+    v[c * 4 + 1] = fp8_weight2<kExact>(lds_at<kSubAt<F>(1)>(code_byte<1>(w, lane4)), hi2, lo2, rs);
+    v[c * 4 + 2] = fp8_weight2<kExact>(lds_at<kSubAt<F>(2)>(code_byte<2>(w, lane4)), hi2, lo2, rs);
+    v[c * 4 + 3] = fp8_weight2<kExact>(lds_at<kSubAt<F>(3)>(code_byte<3>(w, lane4)), hi2, lo2, rs);
   }
 }
 
 // fp8 product format, k = 16: two index words (four codewords: low byte = first sub-table, high byte
-// = second); every sub-table entry is four values as bf16 (entries 128 bytes apart, the second sub-table
-// 32 KiB after the first).
+// = second); every sub-table entry is four values as bf16 in sixteen copies, the second sub-table's behind the first's.
 template <bool kExact>
-GB_DEVINL void f8l_decode4(uint32_t lut, uint32_t wa, uint32_t wb, uint32_t hi2, uint32_t lo2, float rs, uint32_t (&v)[16]) {
+GB_DEVINL void f8l_decode4(uint32_t lane8, uint32_t wa, uint32_t wb, uint32_t hi2, uint32_t lo2, float rs, uint32_t (&v)[16]) {
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const uint32_t w = c < 2 ? wa : wb;
-    const uint32_t off0 = ((c & 1) ? w >> 9 : w << 7) & 0x7F80u, off1 = ((c & 1) ? w >> 17 : w >> 1) & 0x7F80u;
-    uint2 e0, e1;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(e0.x), "=r"(e0.y) : "r"(lut + off0));
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2+32768];" : "=r"(e1.x), "=r"(e1.y) : "r"(lut + off1));
+    const uint2 e0 = lds2_at<kLutAt>((c & 1) ? code_byte<2>(w, lane8) : code_byte<0>(w, lane8));
+    const uint2 e1 = lds2_at<kLutAt + 128>((c & 1) ? code_byte<3>(w, lane8) : code_byte<1>(w, lane8));
     v[c * 4 + 0] = fp8_weight2<kExact>(e0.x, hi2, lo2, rs);
     v[c * 4 + 1] = fp8_weight2<kExact>(e0.y, hi2, lo2, rs);
     v[c * 4 + 2] = fp8_weight2<kExact>(e1.x, hi2, lo2, rs);
@@ -388,7 +400,7 @@ GB_DEVINL void build_tables(uint8_t* cb_s, const void* codebook, int64_t cb, con
     // two sub-tables of 256 entries x four values, 16 copies each (8-byte loads go 16 lanes at a time)
     const uint32_t e = __ldg(reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(codebook) + cb) + dh * 256 + de);
     const uint32_t lo = e4m3_pair_to_bf16(e), hi = e4m3_pair_to_bf16(e >> 16);
-    uint4* l = reinterpret_cast<uint4*>(cb_s) + (dh * 256 + de) * 8;
+    uint4* l = reinterpret_cast<uint4*>(cb_s + de * 256 + dh * 128);
 #pragma unroll
     for (int j = 0; j < 8; ++j) l[(j + d) & 7] = make_uint4(lo, hi, lo, hi);
   } else {
@@ -400,7 +412,7 @@ GB_DEVINL void build_tables(uint8_t* cb_s, const void* codebook, int64_t cb, con
     for (int q = 0; q < 2; ++q) {
       const int ent = (dh * 2 + q) * 256 + de;
       const uint32_t e = e4m3_pair_to_bf16(__ldg(t + ent));
-      uint4* l = reinterpret_cast<uint4*>(cb_s + ent * Fm<F>::kStride);
+      uint4* l = reinterpret_cast<uint4*>(cb_s + (kSubAt<F>(dh * 2 + q) - kLutAt) + de * 256);
 #pragma unroll
       for (int j = 0; j < kVecs; ++j) l[(j + d / (8 / kVecs)) & (kVecs - 1)] = make_uint4(e, e, e, e);
     }
@@ -414,13 +426,13 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   using G = Geo<F>;
   constexpr int kSb = Fm<F>::kSb, kRawStages = Fm<F>::kStages, kSbPerStage = G::kSbPerStage;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* cb_s = smem_raw;                                // codebook copies (+ scale table), at an address known beforehand
+  uint8_t* smem = smem_raw + Fm<F>::kLut;
   const int slab_bytes = p.Mpad * 128;                     // one 64-wide K slab of the activations
   const int x_stage_bytes = 2 * slab_bytes;                // half a superblock of K
   uint8_t* xs = smem;                                      // x_stages x (two slabs)
   uint8_t* raw = xs + (size_t)p.x_stages * x_stage_bytes;  // kRawStages x packed rows
-  uint8_t* cb_s = raw + kRawStages * G::kStageBytes;       // codebook copies (+ scale table)
-  uint64_t* raw_full = reinterpret_cast<uint64_t*>(cb_s + Fm<F>::kLut);
+  uint64_t* raw_full = reinterpret_cast<uint64_t*>(raw + kRawStages * G::kStageBytes);
   uint64_t* raw_empty = raw_full + kMaxRawStages;
   uint64_t* full = raw_empty + kMaxRawStages;              // per unit slot: activations landed + operand decoded
   uint64_t* done = full + kMaxXStages;                     // per unit slot: the unit's MMAs have completed
@@ -440,6 +452,11 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int xs_log = p.x_stages == 8 ? 3 : 2;
 
   gb_pdl_launch_dependents();
+  const uint32_t win = gb_smem_u32(smem_raw) & 0xFF000000u;   // in a cluster the CTA's rank
+  if ((gb_smem_u32(smem_raw) ^ win) != kLutAt) {           // the addresses of the lookups assume it
+    if (threadIdx.x == 0) atomicExch(p.status, 29);
+    return;
+  }
   // A CTA walks the 128-row tiles blockIdx.x, blockIdx.x + gridDim.x, ... (codebook copies, tensor
   // memory and barriers are set up once; the rings run on across tiles).  Dense: one pass over rows
   // [0, M) of x per tile.  Grouped: tile = (expert, 128 rows of it), the expert's rows of the sorted
@@ -685,7 +702,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           tmem_st16(col + 32u, v0);
           tmem_st16(col + 48u, v1);
         } else if constexpr (F == kFmtF8L) {
-          const uint32_t lut = gb_smem_u32(cb_s) + (uint32_t)(lane & 15) * 8u;
+          const uint32_t lut = win | (uint32_t)(lane & 15) * 8u;
           const uint4 ia = rp[2 * h], ib = rp[2 * h + 1];    // eight index words: sixteen codewords
           auto four = [&](uint32_t wa, uint32_t wb, uint32_t (&v)[16]) {
             if (exact) f8l_decode4<true>(lut, wa, wb, hi2, lo2, rs, v);
@@ -702,7 +719,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           tmem_st16(col + 32u, v0);
           tmem_st16(col + 48u, v1);
         } else {
-          const uint32_t lut = gb_smem_u32(cb_s) + (uint32_t)(lane & (Fm<F>::kStride / 4 - 1)) * 4u;
+          const uint32_t lut = win | (uint32_t)(lane & (Fm<F>::kStride / 4 - 1)) * 4u;
           auto four = [&](uint4 cw, uint32_t (&v)[16]) {
             if (exact) fp8_decode4<F, true>(lut, cw, hi2, lo2, rs, v);
             else fp8_decode4<F, false>(lut, cw, hi2, lo2, rs, v);
