@@ -5,7 +5,7 @@
 //
 // Persistent CTAs (one per SM) walk the 128 x 256 output tiles.  Warp 4 (one
 // thread) streams 128-byte-wide K slabs of A and B into a shared-memory ring with tiled TMA
-// loads (128-byte swizzle); warp 5 (one thread) issues tcgen05.mma on shared-memory matrix
+// loads (128-byte swizzle); warp 5 issues tcgen05.mma on shared-memory matrix
 // descriptors and releases ring stages with tcgen05.commit; warps 0..3 read the accumulator
 // out of tensor memory (tcgen05.ld, one 32-lane quarter each), apply the row / column /
 // global scales and store bf16.  Tensor memory holds TWO accumulators (512 columns): while
@@ -206,27 +206,38 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else if (warp == 5) {
     // ------------------------------- MMA issuer ---------------------------------
-    if (lane == 0) {
-      int kk = 0, it = 0;
-      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
-        const int buf = it & 1;
-        // the epilogue must have drained this accumulator (its use two tiles ago)
-        wait_or_abort(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 14);
+    // The warp as a whole, with values that are the same in every lane; one elected lane issues (see gb_gemm_pair.cu).
+    // From one lane's own branch 4096 tokens x 8 of 16 fp8 experts took 1.5 % longer.
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const int tiles = __shfl_sync(0xffffffffu, total_tiles, 0);
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    int s = 0, it = 0;
+    uint32_t ph = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
+      const int buf = it & 1;
+      // the epilogue must have drained this accumulator (its use two tiles ago)
+      wait_or_abort(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 14);
+      __syncwarp();
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t tmem_d = tmem + (uint32_t)(buf * kBN);
+      for (int kt = 0; kt < p.k_tiles; ++kt) {
+        wait_or_abort(&full_bar[s], ph, abort_flag, p.status, 12);
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t tmem_d = tmem_base + (uint32_t)(buf * kBN);
-        for (int kt = 0; kt < p.k_tiles; ++kt, ++kk) {
-          const int s = kk % kStages;
-          wait_or_abort(&full_bar[s], (kk / kStages) & 1, abort_flag, p.status, 12);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_addr = gb_smem_u32(ring + (size_t)s * kStageBytes);
-          const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + kBM * kSlabBytes);
+        const uint32_t a_addr = gb_smem_u32(ring) + (uint32_t)s * kStageBytes;
+        const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + kBM * kSlabBytes);
+        if (one) {
 #pragma unroll
           for (int k = 0; k < kSlabBytes / 32; ++k)       // 32 bytes of K per instruction
             umma(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), p.idesc, kt > 0 || k > 0, fp8);
           umma_commit(&empty_bar[s]);                      // stage free once these MMAs have read it
         }
-        umma_commit(&acc_full[buf]);                       // accumulator complete
+        __syncwarp();
+        if (++s == kStages) { s = 0; ph ^= 1u; }
       }
+      if (one) umma_commit(&acc_full[buf]);                // accumulator complete
+      __syncwarp();
     }
   } else {
     // ------------------------------- epilogue -----------------------------------
