@@ -462,7 +462,6 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // [0, M) of x per tile.  Grouped: tile = (expert, 128 rows of it), the expert's rows of the sorted
   // x in passes of 64 (the weights are decoded again per pass), nothing to do for an expert
   // without rows.
-  if (kGrouped) gb_pdl_wait();                             // the segment offsets come from the routing launch
   const int pass_rows = kGrouped ? kGroupRows : p.Mpad;
   struct Tile { int n0, n_end, w_row0, seg_lo, cnt, n_pass, role; };
   auto tile_at = [&](int t) {
@@ -506,6 +505,12 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  if (kGrouped) {
+    // the tables need nothing of an earlier launch, the segment offsets come from the routing launch
+    if (warp >= kCtlWarps) build_tables<F>(cb_s, p.codebook, 0, p.compose, inexact, threadIdx.x - 32 * kCtlWarps);
+    gb_pdl_wait();
+    __syncthreads();
+  }
   // From here the warps go their own ways: the packed weights do not depend on the launch ahead, so
   // their loads start at once; the decoders build the codebook copies meanwhile; everything that
   // reads x or writes y first waits for the launch ahead.
@@ -622,7 +627,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   } else {
     // ------------------------- decoders -------------------------------------
     const int d = threadIdx.x - 32 * kCtlWarps;              // 0 .. 511
-    int have_role = -1;
+    int have_role = kGrouped ? 0 : -1;
     bool waited = false;
     const int quarter = warp & 3;                            // the tensor-memory lanes this warp may touch
     const int wg = (warp - kCtlWarps) >> 2;                  // warpgroup = operand buffer: units wg, wg + 4, ...
@@ -631,7 +636,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int row = quarter * 32 + lane;                     // weight row of the tile = tensor-memory lane
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t col = lane_base + kACol0 + (uint32_t)(wg * kABufCols);
-    bool exact = true;
+    bool exact = !kGrouped || F != kFmtK16 || *inexact == 0;
     int it = 0, g_sb = 0, item = 0;                          // raw stages, superblocks, (tile, pass) items so far
     for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x) {
     const Tile T = tile_at(t);
