@@ -1172,7 +1172,7 @@ GB_DEVINL int scale_exponent(float amax, int scale_rule) {
 }
 constexpr uint32_t kZeroCodes = (127u - 32u) << 23;        // 2^-32: below this every code is zero (the scale's floor is 1e-8 / 6)
 
-// A value of this CTA into its slot of every CTA of the cluster.
+// A value of this CTA into its slot of every CTA of the cluster, all of which must have started.
 GB_DEVINL void to_peers(uint32_t* slots, uint32_t v, int split) {
   if ((int)threadIdx.x < split) {
     uint32_t dst;
@@ -1191,6 +1191,9 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
   // have completed; the decode kernel waits for it all the same, and starts early
   const bool late = kMode != 0 && p.x_unit == 0;
   if (!late) gb_pdl_launch_dependents();
+  // A peer's shared memory may be written only once its CTA has started.  Said here, waited for in front of the first such
+  // store: the row's load and the CTA's own maximum lie in between.
+  if (kMode == 0 && p.split > 1) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
   gb_pdl_wait();
   if (late) gb_pdl_launch_dependents();
   const int groups = p.K / 16;
@@ -1272,6 +1275,7 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
   reduce();
   if (kMode == 0 && p.split > 1) {                         // over the row's CTAs
     __shared__ uint32_t peer_top[kMaxRowSplit], peer_low[kMaxRowSplit];
+    asm volatile("barrier.cluster.wait;" ::: "memory");
     to_peers(peer_top, top, p.split);
     to_peers(peer_low, low, p.split);
     cluster_sync();                                        // the last access to another CTA's memory lies in front of it

@@ -68,6 +68,22 @@ def test_decode_rows_match_the_oracle(dev, name, M, N, K):
         assert_close_bf16(f32_of(y), oracle_linear(x, d), f"{name} {M}x{N}x{K}", atol_rel=1e-6)
 
 
+@pytest.mark.parametrize("M,K", [(64, 17408), (100, 8448), (1, 40960)])
+def test_rows_split_over_a_cluster(dev, M, K):
+    """Rows that two to eight CTAs hold: more clusters than run at once, uneven shares, one row alone; each row's largest
+    group in another CTA's share."""
+    from gridbook_b200 import _native, synth
+    fmt, N = _fmt("k16"), 64
+    d = synth.make_linear(fmt, N, K, seed=M)
+    lin = _linear(fmt, d, [N], dev)
+    x = _wide_rows(M, K, M).reshape(M, K // 16, 16)
+    x[np.arange(M), np.arange(M) * 37 % (K // 16)] *= np.float32(64)
+    y = lin(synth.bf16_tensor(x.reshape(M, K), dev))
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    assert_close_bf16(f32_of(y), oracle_linear(x.reshape(M, K), d), f"M={M} K={K}", atol_rel=1e-6)
+
+
 @pytest.mark.parametrize("name", ["lit", "k16"])
 @pytest.mark.parametrize("M", [1, 15, 17, 31, 32, 33, 48, 64, 65, 100, 128])
 def test_row_counts_past_sixteen(dev, name, M):

@@ -98,3 +98,20 @@ def test_arrivals_from_another_cta_are_waited_for_at_cluster_scope():
             text = fh.read()
         if re.search(r"mbarrier\.arrive\.\w+\.cluster\.shared::cluster", text):
             assert re.search(r"mbarrier\.try_wait\.parity\.\w+\.cluster", text), f
+
+
+def test_peers_are_written_to_only_after_the_whole_cluster_has_started():
+    """In every kernel that stores into the shared memory of another CTA of its cluster, a wait for the whole cluster
+    stands in front of the first such store: a CTA that has not started has no shared memory to write to."""
+    csrc = os.path.join(PKG, "csrc")
+    found = 0
+    for f in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, f)) as fh:
+            text = re.sub(r"//[^\n]*", "", fh.read())
+        for kernel in re.split(r"\b__global__\b", text)[1:]:
+            store = re.search(r"\bto_peers\(|st\.shared::cluster", kernel)
+            if store:
+                found += 1
+                name = re.search(r"(\w+)\(const", kernel).group(1)
+                assert re.search(r"cluster_sync\(\);|barrier\.cluster\.wait", kernel[:store.start()]), f"{f}: {name}"
+    assert found >= 4
