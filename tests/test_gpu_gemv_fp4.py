@@ -73,7 +73,7 @@ def test_rows_split_over_a_cluster(dev, M, K):
     """Rows that two to eight CTAs hold: more clusters than run at once, uneven shares, one row alone; each row's largest
     group in another CTA's share."""
     from gridbook_b200 import _native, synth
-    fmt, N = _fmt("k16"), 64
+    fmt, N = _fmt("k16"), 136
     d = synth.make_linear(fmt, N, K, seed=M)
     lin = _linear(fmt, d, [N], dev)
     x = _wide_rows(M, K, M).reshape(M, K // 16, 16)
