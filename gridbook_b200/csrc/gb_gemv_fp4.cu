@@ -113,7 +113,7 @@ struct Fp4Params {
   uint32_t x_off, raw_off, sf_off, red_off;
   const uint8_t* xop;        // activation operand: [tile][superblock][scale factors | codes]
   int64_t x_unit;            // bytes of one superblock of it
-  const float* x_scale;      // [tile][pass_rows] power of two of every row; low bits: where groups are left out
+  const float* x_scale;      // [tile][scale_pitch(pass_rows)] power of two of every row; low bits: where groups are left out
   const float* tail;         // [tile][pass_rows][K / 16] scales of the groups left out, of the rows that have any
   int* status;
   int n_roles, n_tiles;
@@ -131,6 +131,8 @@ struct Fp4Params {
 // (narrow) or 16.
 constexpr int kNarrowRows = 16;
 __host__ __device__ constexpr bool is_wide(int pass_rows) { return pass_rows > kNarrowRows; }
+// Distance between the row scales of two tiles: they are read four and eight at a time.
+__host__ __device__ constexpr int scale_pitch(int pass_rows) { return (pass_rows + 7) / 8 * 8; }
 __host__ __device__ constexpr int term_rows(bool wide, int rows) { return wide ? (rows + 15) / 16 * 16 : (rows + 7) / 8 * 8; }
 __host__ __device__ constexpr int narrow_col(int t, int m) { return 12 * (m >> 2) + 4 * t + (m & 3); }
 __host__ __device__ constexpr int mma_cols(bool wide, int rows) {
@@ -827,7 +829,7 @@ fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4
             const int rows = min(p.pass_rows, Q.cnt - out_pass * p.pass_rows);
             int to0 = lane, to1 = lane + 32;                 // output rows
             if (kGrouped) {
-              const float* xsc = p.x_scale + (int64_t)(Q.x_tile + out_pass) * p.pass_rows;
+              const float* xsc = p.x_scale + (int64_t)(Q.x_tile + out_pass) * scale_pitch(p.pass_rows);
               xs0 = lane < rows ? xsc[lane] : 0.0f;
               xs1 = lane + 32 < rows ? xsc[lane + 32] : 0.0f;
               to0 += Q.lo + out_pass * p.pass_rows;          // sorted positions
@@ -930,7 +932,7 @@ fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4
             auto emit = [&](auto n_rows, int m0, const float* total) {
               constexpr int kRows = decltype(n_rows)::value;
               if (m0 >= rows) return;
-              const uint4* words = reinterpret_cast<const uint4*>(p.x_scale + (kGrouped ? (int64_t)(Q.x_tile + q_pass) * p.pass_rows : 0) + m0);
+              const uint4* words = reinterpret_cast<const uint4*>(p.x_scale + (kGrouped ? (int64_t)(Q.x_tile + q_pass) * scale_pitch(p.pass_rows) : 0) + m0);
               float val[kRows];
 #pragma unroll
               for (int q = 0; q < kRows / 4; ++q) {
@@ -1353,7 +1355,7 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
       else place(s, tile, m, rows);
       if (tile < 0) continue;                                // uniform over the CTA
     }
-    if (threadIdx.x == 0 && (kMode != 0 || blockIdx.x % p.split == 0)) p.x_scale[(int64_t)tile * p.pass_rows + m] = back;
+    if (threadIdx.x == 0 && (kMode != 0 || blockIdx.x % p.split == 0)) p.x_scale[(int64_t)tile * scale_pitch(p.pass_rows) + m] = back;
     uint8_t* dst = p.xop + (int64_t)tile * p.n_sb * p.x_unit;
 #pragma unroll
     for (int i = 0; i < kG; ++i) {
@@ -1729,7 +1731,7 @@ int64_t gb_moe_fp4_operand_bytes(int64_t P, int64_t E, int64_t K, int pass_rows)
   if (pass_rows == 0) return gb_fp4_tiles(P, E, K).bytes;
   if (pass_rows < 1) return 0;
   const int64_t tiles = P / pass_rows + E + 1;
-  return align256(tiles * (K / 256) * unit_bytes(is_wide(pass_rows), pass_rows)) + align256(tiles * pass_rows * 4) +
+  return align256(tiles * (K / 256) * unit_bytes(is_wide(pass_rows), pass_rows)) + align256(tiles * scale_pitch(pass_rows) * 4) +
          align256(tiles * pass_rows * (K / 16) * 4);
 }
 
@@ -1751,7 +1753,7 @@ static int rows_params(RowsParams* p, const void* x, int64_t P, int64_t E, int64
     const int64_t tiles = P / pass_rows + E + 1;
     p->x_unit = unit_bytes(is_wide(pass_rows), pass_rows);
     p->x_scale = (float*)((uint8_t*)operand + align256(tiles * (K / 256) * p->x_unit));
-    p->tail = (float*)((uint8_t*)p->x_scale + align256(tiles * pass_rows * 4));
+    p->tail = (float*)((uint8_t*)p->x_scale + align256(tiles * scale_pitch(pass_rows) * 4));
   }
   p->K = (int)K; p->n_sb = (int)(K / 256); p->scale_rule = scale_rule; p->pass_rows = pass_rows;
   p->ids = ids; p->seg = seg; p->E = (int)E;
@@ -1799,7 +1801,7 @@ int gb_moe_gemv_fp4(const void* operand, const gb_weight* w, int scales_e4m3, in
   p.x_unit = unit_bytes(is_wide(pass_rows), pass_rows);
   p.xop = (const uint8_t*)operand;
   p.x_scale = (const float*)((const uint8_t*)operand + align256(tiles * p.n_sb * p.x_unit));
-  p.tail = (const float*)((const uint8_t*)p.x_scale + align256(tiles * pass_rows * 4));
+  p.tail = (const float*)((const uint8_t*)p.x_scale + align256(tiles * scale_pitch(pass_rows) * 4));
   p.mat[0] = {w->qw, w->row_stride, N, w->codebook, w->compose, w->global_scale == 0.0f ? 1.0f : w->global_scale, (uint16_t*)y};
   p.status = gb_status_word();
   p.n_roles = 1;

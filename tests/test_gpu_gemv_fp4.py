@@ -375,3 +375,39 @@ def test_rows_shared_by_several_matrices(dev, name, M):
     hook = lins[1].register_forward_hook(lambda mod, args, out: seen.append(1))
     assert len(apply_shared_row(lins, x)) == 3 and (M == 1 and name == "lit") != bool(seen)
     hook.remove()
+
+
+@pytest.mark.parametrize("name,pass_rows", [("lit", 1), ("lit", 5), ("k16", 7), ("lit", 13), ("k16", 18), ("lit", 33), ("lit", 61)])
+def test_any_number_of_rows_per_pass(dev, name, pass_rows):
+    """The C entries take every row count up to the one that is named for the stack: what 16 or 64 rows a pass give."""
+    import ctypes
+    from gridbook_b200 import _native as nat, kernels, synth
+    fmt = _fmt(name)
+    E, N, K, P = 3, 256, 512, 300
+    d = synth.make_linear(fmt, E * N, K, seed=pass_rows, global_scale=1.0 / 448.0 if name == "lit" else None)
+    if name == "k16":
+        from gridbook_b200 import codec
+        d = dict(d, fmt=fmt.padded(80), qw=codec.pad_superblocks(torch.from_numpy(d["qw"]), 73, 80).numpy())
+    w = synth.to_device_weight(d, dev)
+    nw = w.native()
+    nw.rows = N
+    gen = torch.Generator(device=dev).manual_seed(pass_rows)
+    x = torch.randn(P, K, generator=gen, device=dev).to(torch.bfloat16)
+    ids = torch.randint(0, E, (P,), generator=gen, device=dev, dtype=torch.int32)
+    inv = torch.argsort(torch.argsort(ids, stable=True)).to(torch.int32)
+    seg = torch.zeros(E + 1, dtype=torch.int32, device=dev)
+    seg[1:] = torch.bincount(ids, minlength=E).cumsum(0)
+    lib, ptr, i64, stream = nat.load(), lambda t: ctypes.c_void_p(t.data_ptr()), ctypes.c_int64, ctypes.c_void_p(nat.stream_ptr(dev))
+
+    def product(rows):
+        assert lib.gb_moe_fp4_pass_rows(ctypes.byref(nw), 1, i64(P), i64(E)) >= rows
+        op = torch.zeros(lib.gb_moe_fp4_operand_bytes(i64(P), i64(E), i64(K), rows), dtype=torch.uint8, device=dev)
+        y = torch.empty(P, N, dtype=torch.bfloat16, device=dev)
+        nat.check(lib.gb_moe_fp4_rows(ptr(x), ptr(ids), ptr(inv), ptr(seg), i64(P), i64(1), i64(E), i64(K), rows, 0, ptr(op), stream), lib)
+        nat.check(lib.gb_moe_gemv_fp4(ptr(op), ctypes.byref(nw), 1, i64(N * nw.row_stride), i64(E), ptr(seg), None, i64(P), rows, ptr(y), stream), lib)
+        return y
+
+    got, want = product(pass_rows), product(16 if pass_rows <= 16 else 64)
+    torch.cuda.synchronize()
+    assert nat.device_status(0) == 0
+    assert_close_bf16(f32_of(got), f32_of(want), f"{name} {pass_rows} rows a pass", atol_rel=1e-6)

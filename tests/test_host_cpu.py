@@ -933,3 +933,18 @@ def test_grouped_fp4_entry_refuses_row_counts_that_no_operand_has():
     for P, E, pass_rows in [(4, 2, 0), (4, 2, -1), (4, 2, 65), (0, 2, 16), (4, 0, 16)]:
         assert lib.gb_moe_gemv_fp4(at(256), ctypes.byref(w), 1, n(128 * 48), n(E), at(256), None, n(P), pass_rows, at(256), None) == 1
         assert b"rows per pass" in lib.gb_last_error()
+
+
+def test_row_scales_of_every_tile_start_where_four_are_read_at_once():
+    """The operand of a routed fp4 batch keeps the row scales of a tile eight apart or a multiple of it, whatever the rows per
+    pass: they are read sixteen bytes at a time, up to the eighth of the last row's chunk."""
+    from gridbook_b200 import _native as nat
+    lib, n = nat.load(), ctypes.c_int64
+    up = lambda v: (v + 255) // 256 * 256                    # noqa: E731
+    for P, E, K in [(700, 4, 256), (4000, 128, 512)]:
+        for rows in range(1, 65):
+            tiles = P // rows + E + 1
+            codes = (rows + 15) // 16 * 32 if rows > 16 else ((rows + 7) // 8 * 24 + 15) // 16 * 16
+            unit = (4096 if rows > 16 else 2048) + codes * 128
+            want = up(tiles * (K // 256) * unit) + up(tiles * ((rows + 7) // 8 * 8) * 4) + up(tiles * rows * (K // 16) * 4)
+            assert lib.gb_moe_fp4_operand_bytes(n(P), n(E), n(K), rows) == want, (P, E, K, rows)
