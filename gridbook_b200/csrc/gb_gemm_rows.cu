@@ -231,16 +231,19 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     __syncwarp();
   } else {
     for (int m = threadIdx.x; m < rows; m += 32 * kEpiWarps) rs_s[m] = (p.a_scale ? p.a_scale[m0 + m] : 1.0f) * p.global_scale;
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
     if (!warp_wait(acc_bar, 0, &abort_s, p.status, 83)) abort_s = 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // The row scales are there, and all eight warps see the same flag behind it: the wait may run out in one and end in
+    // another, and they meet at barriers below.  (The other two warps raise it only where the accumulator is never complete.)
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
   }
 
+  const bool live = warp < kEpiWarps && !abort_s;
   const int quarter = warp & 3, feature = quarter * 32 + lane;
   const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16);
   if (p.slices == 1) {
     // Out through shared memory, over the operand ring: rows of 16-byte pieces instead of 64 bytes per warp and row
-    if (warp < kEpiWarps && !abort_s) {
+    if (live) {
       const float bs = p.b_scale && n0 + feature < p.N ? p.b_scale[n0 + feature] : 1.0f;
       for (int c = (warp >> 2) * 16; c < cols; c += 32) {
         uint32_t v[16];
@@ -276,7 +279,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // every CTA of the cluster has finished its MMAs, and with them its loads.  Rows are owned in sixteens.
     const int own = (cols / 16 + p.slices - 1) / p.slices * 16;
     cluster_sync();
-    if (warp < kEpiWarps && !abort_s) {
+    if (live) {
       for (int c = (warp >> 2) * 16; c < cols; c += 32) {
         uint32_t v[16];
         tmem_ld16(acc + (uint32_t)c, v);
@@ -291,7 +294,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       }
     }
     cluster_sync();                                          // the last access to another CTA's memory lies in front of it
-    if (warp < kEpiWarps && !abort_s) {
+    if (live) {
       const int f = lane * 4, left = (int)min((int64_t)kBM, p.N - n0) - f;
       float bs[4];
 #pragma unroll
