@@ -154,6 +154,37 @@ struct Kept {
   }
 };
 
+// A number that the runtime gives no second stream, as it may a handle.
+unsigned long long number_of(cudaStream_t stream) {
+  unsigned long long id = 0;
+  C10_CUDA_CHECK(cudaStreamGetId(stream, &id));
+  return id;
+}
+
+// Armed slots of the table kernel (gb_gemv_tab): calls that may overlap on the GPU need a buffer each, so every stream has
+// its own.  Graphs have one more, armed outside any capture, for a replay may run beside eager calls; replays of graphs
+// that hold the same layers must not overlap.
+struct ArmedSlots {
+  static constexpr size_t kMostStreams = 8;        // past these, and for a set whose first call is captured: armed on each call
+  std::mutex mutex;
+  at::Tensor captured;
+  std::vector<std::pair<unsigned long long, at::Tensor>> of_stream;
+
+  static at::Tensor armed(int64_t bytes, const at::Tensor& like) { return at::full({bytes}, 0xFF, like.options().dtype(at::kByte)); }
+  at::Tensor get(int64_t bytes, const at::Tensor& like, cudaStream_t stream) {
+    const bool capture = capturing();
+    std::lock_guard<std::mutex> lock(mutex);
+    if (capture) return captured.defined() ? captured : armed(bytes, like);
+    if (!captured.defined()) captured = armed(bytes, like);
+    const unsigned long long id = number_of(stream);
+    for (const auto& s : of_stream)
+      if (s.first == id) return s.second;
+    at::Tensor t = armed(bytes, like);
+    if (of_stream.size() < kMostStreams) of_stream.emplace_back(id, t);
+    return t;
+  }
+};
+
 constexpr int64_t kDecodeMaxRows = 16;
 // Routed rows per expert from which a stack is decoded once into its NVFP4 view and multiplied by the grouped GEMM,
 // instead of decoded in every pass of up to 64 rows.  The larger an expert, the later: its decoded copy is written
@@ -175,13 +206,18 @@ enum { kMoePrefill = 1, kMoeSorted = 2, kMoePairs = 3, kMoeGrouped = 4 };
 
 struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
   Weight w;
-  at::Tensor workspace, slots;
+  // Scratch of decode calls on the stream that loaded the layer, one call at a time; elsewhere, and in a graph, where it may
+  // be another call's at the same time, a call brings its own.
+  at::Tensor workspace;
+  unsigned long long home = 0;
+  bool tables = false;                             // the table kernel takes the layer
+  ArmedSlots slots;
   int64_t row_batch_max = 16;
   gb_hints hints{};
   std::atomic<int> prefill_route{kRouteNone};
   const int64_t serial = next_serial++;            // never given twice, as an address is
-  std::mutex mutex;
-  std::map<std::vector<int64_t>, Kept> shared_slots;   // by the serials of the plans that share a row
+  std::mutex mutex, scratch_mutex;
+  std::map<std::vector<int64_t>, ArmedSlots> shared_slots;   // by the serials of the plans that share a row
   static std::atomic<int64_t> next_serial;
 
   // `role_rows`: row counts of the parts with a codebook of their own (empty: one codebook)
@@ -192,7 +228,13 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
       hints.n_roles = (int32_t)role_rows.size();
       for (size_t i = 0; i < role_rows.size(); ++i) hints.role_rows[i] = role_rows[i];
     }
-    if (armed.has_value() && armed->defined()) slots = *armed;
+    if (workspace.defined() && workspace.is_cuda()) home = number_of(c10::cuda::getCurrentCUDAStream(workspace.get_device()));
+    if (armed.has_value() && armed->defined()) {
+      const c10::cuda::CUDAGuard guard(armed->device());
+      slots.of_stream.emplace_back(number_of(c10::cuda::getCurrentCUDAStream()), *armed);
+      slots.captured = ArmedSlots::armed(armed->numel(), *armed);
+      tables = true;
+    }
     row_batch_max = L.gb_gemv_row_batch_max(&w.w);
   }
 
@@ -210,20 +252,27 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
     if (M == 0) return at::empty(shape, x.options());
     need_bf16(x, "the codebook linear");
     const c10::cuda::CUDAGuard guard(x.device());
-    void* stream = c10::cuda::getCurrentCUDAStream().stream();
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
     at::Tensor out = at::empty(shape, x.options());
-    if (M == 1 && slots.defined()) {
+    if (M == 1 && tables) {
       const gb_weight* ws[1] = {&w.w};
       void* ys[1] = {out.data_ptr()};
-      const int rc = L.gb_gemv_tab(xc.data_ptr(), ws, ys, 1, w.act(), rule, slots.data_ptr(), slots.numel(), stream);
+      const at::Tensor armed = slots.get(L.gb_gemv_tab_slots_bytes(ws, 1), x, stream);
+      const int rc = L.gb_gemv_tab(xc.data_ptr(), ws, ys, 1, w.act(), rule, armed.data_ptr(), armed.numel(), stream);
       if (rc == GB_OK) return out;
       if (rc != GB_EUNSUPPORTED) check(rc);
     }
     if (M <= kDecodeMaxRows || M <= std::min(midm_max, row_batch_max)) {
-      at::Tensor ws = workspace;
       const int64_t need = L.gb_gemv_hinted_workspace_bytes(M, N, K);
-      if (!ws.defined() || ws.numel() < need) ws = at::empty({need}, x.options().dtype(at::kByte));
+      at::Tensor ws;
+      std::unique_lock<std::mutex> lock(scratch_mutex, std::defer_lock);
+      if (workspace.defined() && workspace.numel() >= need && !capturing() && number_of(stream) == home) {
+        lock.lock();                                       // until both launches of the call are on the stream
+        ws = workspace;
+      } else {
+        ws = at::empty({need}, x.options().dtype(at::kByte));
+      }
       check(L.gb_gemv_hinted(xc.data_ptr(), M, &w.w, &hints, rule, out.data_ptr(), ws.data_ptr(), ws.numel(), stream));
       return out;
     }
@@ -353,11 +402,11 @@ py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, con
   if (n < 2 || n > 4 || !x.is_cuda() || x.dim() < 1) return py::none();
   const int64_t K = plans[0]->w.w.K;
   bool tables = x.numel() == K;
-  for (const auto& p : plans) tables = tables && p->slots.defined();
+  for (const auto& p : plans) tables = tables && p->tables;
   if (!tables) return shared_rows(plans, x, rule, routes);
   if (x.numel() != K || x.size(-1) != K) return py::none();   // another width: refused where the layers are called one by one
   for (const auto& p : plans)
-    if (!p->slots.defined() || p->w.w.K != K) return py::none();
+    if (!p->tables || p->w.w.K != K) return py::none();
   need_bf16(x, "the table GEMV");
   const c10::cuda::CUDAGuard guard(x.device());
   const gb_weight* ws[4];
@@ -367,18 +416,13 @@ py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, con
     ws[i] = &plans[i]->w.w;
     key.push_back(plans[i]->serial);
   }
-  at::Tensor slots;
+  ArmedSlots* kept;
   {
     std::lock_guard<std::mutex> lock(plans[0]->mutex);
-    auto& kept = plans[0]->shared_slots;
-    auto it = kept.find(key);
-    if (it == kept.end()) {
-      slots = at::full({L.gb_gemv_tab_slots_bytes(ws, (int)n)}, 0xFF, x.options().dtype(at::kByte));
-      if (!capturing()) kept.emplace(key, Kept(slots));    // else the graph arms its own
-    } else {
-      slots = it->second.ready();
-    }
+    kept = &plans[0]->shared_slots[key];                   // a node of the map: it stays where it is
   }
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+  const at::Tensor slots = kept->get(L.gb_gemv_tab_slots_bytes(ws, (int)n), x, stream);
   const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
   std::vector<at::Tensor> outs;
   for (size_t i = 0; i < n; ++i) {
@@ -387,8 +431,7 @@ py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, con
     outs.push_back(at::empty(shape, x.options()));
     ys[i] = outs.back().data_ptr();
   }
-  const int rc = L.gb_gemv_tab(xc.data_ptr(), ws, ys, (int)n, plans[0]->w.act(), rule, slots.data_ptr(), slots.numel(),
-                               c10::cuda::getCurrentCUDAStream().stream());
+  const int rc = L.gb_gemv_tab(xc.data_ptr(), ws, ys, (int)n, plans[0]->w.act(), rule, slots.data_ptr(), slots.numel(), stream);
   if (rc == GB_EUNSUPPORTED) return py::none();
   check(rc);
   return py::cast(outs);

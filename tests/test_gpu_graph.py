@@ -113,3 +113,85 @@ def test_batch_sizes_share_what_a_plan_keeps(block):
             moe(x[:T], tw_d[:T], ids_d[:T])
     torch.cuda.synchronize()
     assert torch.cuda.memory_allocated() - before <= 16 << 10   # lists of 256 and 512 pairs; one each would be 200 KB
+
+
+def _layer(name, N, K, dev):
+    from gridbook_b200 import formats, synth
+    from gridbook_b200.linear import CBLinear
+    fmt = {"literal": formats.NVFP4_LITERAL, "k16": formats.NVFP4_CB_K16, "fp8k32": formats.FP8_CB_K32}[name]
+    gen = torch.Generator(device=dev).manual_seed(N)
+    lin = CBLinear(fmt, K, [N], [synth.codebook_tables(fmt, N)], global_scale=1.0 / 448.0 if name == "literal" else 1.0, prefix=f"s{N}")
+    scale = None if fmt.is_fp4 else (torch.rand(N, generator=gen, device=dev) + 0.5) * 0.02
+    return lin.load(synth.make_packed_device(fmt, N, K, gen, dev), scale, dev)
+
+
+def _rows(n, M, K, dev):
+    gen = torch.Generator(device=dev).manual_seed(n)
+    return [torch.randn(M, K, generator=gen, device=dev).to(torch.bfloat16) for _ in range(n)]
+
+
+@pytest.mark.parametrize("name", ["literal", "k16", "fp8k32"])
+def test_one_layer_on_several_streams_and_threads(name):
+    """Decode calls of one layer that overlap on the GPU, from two streams and a graph, and calls of two threads that share a
+    stream: each has scratch of its own."""
+    import threading
+    from gridbook_b200 import _native
+    _native.prepare(0)
+    dev = torch.device("cuda:0")
+    lin = _layer(name, 1536, 4096, dev)
+    xs = _rows(3, 4, 4096, dev)
+    want = [lin(x) for x in xs]
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        captured = lin(xs[2])
+    torch.cuda.synchronize()
+    streams = [torch.cuda.current_stream(), torch.cuda.Stream(), torch.cuda.Stream()]
+    got = [[], [], []]
+    for _ in range(40):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                if i == 2:
+                    g.replay()
+                    got[2].append(captured.clone())
+                else:
+                    got[i].append(lin(xs[i]))
+    torch.cuda.synchronize()
+
+    def calls(i):
+        got[i] += [lin(xs[i]) for _ in range(100)]
+
+    threads = [threading.Thread(target=calls, args=(i,)) for i in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    for i in range(3):
+        assert all(torch.equal(y, want[i]) for y in got[i]), (name, i)
+
+
+def test_one_row_of_a_layer_on_several_streams():
+    """The table kernel's slots are one stream's each, and a graph's: streams past the number that is kept, one layer and two
+    that share a row, in turn."""
+    from gridbook_b200 import _native
+    from gridbook_b200.linear import apply_shared_row
+    _native.prepare(0)
+    dev = torch.device("cuda:0")
+    a, b = _layer("literal", 1024, 2048, dev), _layer("literal", 512, 2048, dev)
+    (x,) = _rows(1, 1, 2048, dev)
+    want = [a(x), *apply_shared_row([a, b], x)]
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        captured = [a(x), *apply_shared_row([a, b], x)]
+    torch.cuda.synchronize()
+    for _ in range(2):
+        for s in [torch.cuda.Stream() for _ in range(10)]:
+            s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(s):
+                g.replay()
+                got = [a(x), *apply_shared_row([a, b], x)]
+            torch.cuda.current_stream().wait_stream(s)
+            torch.cuda.synchronize()
+            assert all(torch.equal(u, v) and torch.equal(w, v) for u, w, v in zip(got, captured, want))
+    assert _native.device_status(0) == 0
