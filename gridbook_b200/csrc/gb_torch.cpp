@@ -371,24 +371,22 @@ py::object shared_rows(const std::vector<std::shared_ptr<LinearPlan>>& plans, co
   } else {
     if (((uintptr_t)xc.data_ptr() & 15u) != 0) return py::none();
     const int q = a.add(fp4 ? M * K / 2 : M * K), sf = a.add(fp4 ? L.gb_nvfp4_sf_bytes(M, K) : 0), as = a.add(M * 4);
-    int wq[4], wsf[4];
-    for (size_t i = 0; i < n; ++i) {
-      wq[i] = a.add(fp4 ? ws[i]->rows * K / 2 : ws[i]->rows * K);
-      wsf[i] = a.add(fp4 ? L.gb_nvfp4_sf_bytes(ws[i]->rows, K) : 0);
-    }
+    // one decoded copy at a time, in the place of the largest: multiplied while it lies in L2, and no more memory than one by one
+    int64_t rows = 0;
+    for (size_t i = 0; i < n; ++i) rows = std::max(rows, ws[i]->rows);
+    const int wq = a.add(fp4 ? rows * K / 2 : rows * K), wsf = a.add(fp4 ? L.gb_nvfp4_sf_bytes(rows, K) : 0);
     a.alloc(xc);
     if (fp4) check(L.gb_nvfp4_quantize_rows(xc.data_ptr(), M, K, kNvfp4ActRange, a.ptr(q), a.ptr(sf), a.ptr<float>(as), stream));
     else check(L.gb_fp8_quantize_rows(xc.data_ptr(), a.ptr(q), a.ptr<float>(as), M, K, rule, stream));
-    for (size_t i = 0; i < n; ++i) {                       // the first right behind the quantiser, beside it
-      if (fp4) check((i == 0 ? L.gb_expand_fp4_nvfp4_beside : L.gb_expand_fp4_nvfp4)(ws[i], 0, ws[i]->rows, a.ptr(wq[i]), a.ptr(wsf[i]), 2, stream));
-      else check((i == 0 ? L.gb_expand_fp8_beside : L.gb_expand_fp8)(ws[i], 0, ws[i]->rows, a.ptr(wq[i]), stream));
-    }
-    for (size_t i = 0; i < n; ++i) {
-      if (fp4)
-        check(L.gb_gemm_fp4(a.ptr(q), a.ptr(sf), a.ptr(wq[i]), a.ptr(wsf[i]), ys[i], M, ws[i]->rows, K, a.ptr<float>(as), ws[i]->global_scale, stream));
-      else
-        check(L.gb_gemm_tn(a.ptr(q), a.ptr(wq[i]), ys[i], M, ws[i]->rows, K, GB_GEMM_E4M3, a.ptr<float>(as), ws[i]->weight_scale,
+    for (size_t i = 0; i < n; ++i) {                       // the first expander right behind the quantiser, beside it
+      if (fp4) {
+        check((i == 0 ? L.gb_expand_fp4_nvfp4_beside : L.gb_expand_fp4_nvfp4)(ws[i], 0, ws[i]->rows, a.ptr(wq), a.ptr(wsf), 2, stream));
+        check(L.gb_gemm_fp4(a.ptr(q), a.ptr(sf), a.ptr(wq), a.ptr(wsf), ys[i], M, ws[i]->rows, K, a.ptr<float>(as), ws[i]->global_scale, stream));
+      } else {
+        check((i == 0 ? L.gb_expand_fp8_beside : L.gb_expand_fp8)(ws[i], 0, ws[i]->rows, a.ptr(wq), stream));
+        check(L.gb_gemm_tn(a.ptr(q), a.ptr(wq), ys[i], M, ws[i]->rows, K, GB_GEMM_E4M3, a.ptr<float>(as), ws[i]->weight_scale,
                            ws[i]->global_scale, stream));
+      }
       plans[i]->prefill_route = fp4 ? kRouteNvfp4 : kRouteFp8;
     }
   }

@@ -206,3 +206,31 @@ def test_prefill_linears_launched_back_to_back(dev, M):
     for _ in range(5):
         for a, b in zip(chain(False), one_at_a_time):
             assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("name", ["fp8k32", "lit"])
+def test_shared_prefill_holds_one_decoded_copy_at_a_time(dev, name):
+    """Three linears that read the same rows need no more memory at their peak together than one after the other."""
+    from gridbook_b200 import formats as F, synth
+    from gridbook_b200.linear import CBLinear, apply_shared_row
+    fmt, M, K = {"lit": F.NVFP4_LITERAL, "fp8k32": F.FP8_CB_K32}[name], 300, 2048
+    gen = torch.Generator(device=dev).manual_seed(1)
+    lins = []
+    for i, N in enumerate((2048, 4096, 3072)):
+        lin = CBLinear(fmt, K, [N], [synth.codebook_tables(fmt, i)], prefix=f"mem.{i}")
+        scale = None if fmt.is_fp4 else torch.rand(N, generator=gen, device=dev) + 0.5
+        lins.append(lin.load(synth.make_packed_device(fmt, N, K, gen, dev), scale, dev))
+    x = torch.randn(M, K, generator=gen, device=dev).to(torch.bfloat16)
+
+    def peak(call):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        out = call()
+        torch.cuda.synchronize()
+        return torch.cuda.max_memory_allocated() - before, out
+
+    (apart, want), (shared, got) = peak(lambda: [lin(x) for lin in lins]), peak(lambda: apply_shared_row(lins, x))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert shared <= apart + (64 << 10), (shared, apart)
