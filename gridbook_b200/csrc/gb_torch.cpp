@@ -154,11 +154,14 @@ struct Kept {
   }
 };
 
-// A number that the runtime gives no second stream, as it may a handle.
+// A number that the runtime gives no second stream, as it may a handle; 0 under capture.  The default stream, which is never
+// captured, is told without asking the runtime (two calls, 0.25 of the 7.2 us of a 4096 x 4096 row).
 unsigned long long number_of(cudaStream_t stream) {
+  if (stream == nullptr) return ~0ull;
+  if (capturing()) return 0;
   unsigned long long id = 0;
   C10_CUDA_CHECK(cudaStreamGetId(stream, &id));
-  return id;
+  return id + 1;
 }
 
 // Armed slots of the table kernel (gb_gemv_tab): calls that may overlap on the GPU need a buffer each, so every stream has
@@ -172,11 +175,10 @@ struct ArmedSlots {
 
   static at::Tensor armed(int64_t bytes, const at::Tensor& like) { return at::full({bytes}, 0xFF, like.options().dtype(at::kByte)); }
   at::Tensor get(int64_t bytes, const at::Tensor& like, cudaStream_t stream) {
-    const bool capture = capturing();
-    std::lock_guard<std::mutex> lock(mutex);
-    if (capture) return captured.defined() ? captured : armed(bytes, like);
-    if (!captured.defined()) captured = armed(bytes, like);
     const unsigned long long id = number_of(stream);
+    std::lock_guard<std::mutex> lock(mutex);
+    if (id == 0) return captured.defined() ? captured : armed(bytes, like);
+    if (!captured.defined()) captured = armed(bytes, like);
     for (const auto& s : of_stream)
       if (s.first == id) return s.second;
     at::Tensor t = armed(bytes, like);
@@ -267,7 +269,7 @@ struct LinearPlan : std::enable_shared_from_this<LinearPlan> {
       const int64_t need = L.gb_gemv_hinted_workspace_bytes(M, N, K);
       at::Tensor ws;
       std::unique_lock<std::mutex> lock(scratch_mutex, std::defer_lock);
-      if (workspace.defined() && workspace.numel() >= need && !capturing() && number_of(stream) == home) {
+      if (workspace.defined() && workspace.numel() >= need && home != 0 && number_of(stream) == home) {
         lock.lock();                                       // until both launches of the call are on the stream
         ws = workspace;
       } else {
