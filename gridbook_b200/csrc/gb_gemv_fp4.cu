@@ -1702,6 +1702,15 @@ int gb_gemv_hinted(const void* x, int64_t M, const gb_weight* w, const gb_hints*
   return gb_gemv(x, M, w, act, scale_rule, y, workspace, workspace_bytes, stream);
 }
 
+int gb_gemv_shared_applies(const gb_weight* const* w, int n_weights, int scales_e4m3) {
+  if (w == nullptr || n_weights < 1 || n_weights > kMaxMatrices) return 0;
+  for (int i = 0; i < n_weights; ++i)
+    if (gb_check_weight(w[i]) != GB_OK || w[i]->K != w[0]->K || !gb_gemv_fp4_applies(w[i], scales_e4m3 != 0) ||
+        fp4_format(w[i], scales_e4m3 != 0) != fp4_format(w[0], scales_e4m3 != 0) || w[i]->cb_row_offset != nullptr)
+      return 0;
+  return 1;
+}
+
 int gb_gemv_shared(const void* x, int64_t M, const gb_weight* const* w, int n_weights, int scales_e4m3, int scale_rule, void* const* y,
                    void* workspace, int64_t workspace_bytes, void* stream) {
   GB_REQUIRE(x && w && y, "null pointer argument");
@@ -1712,11 +1721,8 @@ int gb_gemv_shared(const void* x, int64_t M, const gb_weight* const* w, int n_we
     if (rc != GB_OK) return rc;
     GB_REQUIRE(y[i] != nullptr, "null output %d", i);
     GB_REQUIRE(w[i]->K == w[0]->K, "matrix %d has K=%lld, matrix 0 K=%lld: they must read the same rows", i, (long long)w[i]->K, (long long)w[0]->K);
-    if (!gb_gemv_fp4_applies(w[i], scales_e4m3 != 0) || fp4_format(w[i], scales_e4m3 != 0) != fp4_format(w[0], scales_e4m3 != 0) ||
-        w[i]->cb_row_offset != nullptr)
-      return GB_EUNSUPPORTED;
   }
-  if (((uintptr_t)x & 15u) != 0) return GB_EUNSUPPORTED;
+  if (!gb_gemv_shared_applies(w, n_weights, scales_e4m3) || ((uintptr_t)x & 15u) != 0) return GB_EUNSUPPORTED;
   return gemv_fp4(x, M, w, n_weights, scales_e4m3 != 0, 0, nullptr, scale_rule, y, workspace, workspace_bytes, stream);
 }
 

@@ -39,7 +39,7 @@ namespace {
   F(gb_last_error) F(gb_gemv_hinted_workspace_bytes) F(gb_gemv) F(gb_gemv_row_batch_max) F(gb_gemv_tab) \
   F(gb_gemv_tab_slots_bytes) F(gb_fp4_act_qdq) F(gb_fp8_act_qdq) F(gb_fp8_quantize_rows) F(gb_nvfp4_sf_bytes) \
   F(gb_nvfp4_quantize_rows) F(gb_expand_fp4_nvfp4) F(gb_expand_fp4_bf16) F(gb_expand_fp8) F(gb_expand_fp8_bf16) \
-  F(gb_gemv_shared) F(gb_expand_fp4_nvfp4_beside) F(gb_expand_fp8_beside) F(gb_gemm_fp4) F(gb_gemm_tn) F(gb_gemm_tn_grouped) F(gb_moe_route_ws) F(gb_moe_route_workspace_bytes) \
+  F(gb_gemv_shared) F(gb_gemv_shared_applies) F(gb_expand_fp4_nvfp4_beside) F(gb_expand_fp8_beside) F(gb_gemm_fp4) F(gb_gemm_tn) F(gb_gemm_tn_grouped) F(gb_moe_route_ws) F(gb_moe_route_workspace_bytes) \
   F(gb_moe_gather_rows) F(gb_moe_swiglu_rows) F(gb_moe_gemv) F(gb_moe_gemv_sorted) F(gb_moe_mlp_pairs) \
   F(gb_moe_mlp_pairs_workspace_bytes) F(gb_moe_combine) F(gb_gemv_hinted) F(gb_scales_e4m3) F(gb_moe_route_inv) \
   F(gb_moe_fp4_pass_rows) F(gb_moe_fp4_operand_bytes) F(gb_moe_fp4_rows) F(gb_moe_fp4_swiglu_rows) \
@@ -342,17 +342,21 @@ py::object shared_rows(const std::vector<std::shared_ptr<LinearPlan>>& plans, co
   }
   const bool fp4 = plans[0]->w.fp4();
   if (!decode && !(prefill && (routes[0].first || !fp4))) return py::none();
+  // decided before anything is allocated: layers that go one by one allocate again
+  const gb_weight* ws[4];
+  for (size_t i = 0; i < n; ++i) ws[i] = &plans[i]->w.w;
+  const bool odd = x.is_contiguous() && ((uintptr_t)x.data_ptr() & 15u) != 0;   // (a copy starts at a multiple of sixteen bytes)
+  if (decode && fp4 && (odd || L.gb_gemv_shared_applies(ws, (int)n, plans[0]->w.scales_e4m3 ? 1 : 0) == 0)) return py::none();
+  if (!decode && odd) return py::none();
   const c10::cuda::CUDAGuard guard(x.device());
   void* stream = c10::cuda::getCurrentCUDAStream().stream();
   const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
-  const gb_weight* ws[4];
   void* ys[4];
   std::vector<at::Tensor> outs;
   for (size_t i = 0; i < n; ++i) {
     std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
     shape.back() = plans[i]->w.w.rows;
     outs.push_back(at::empty(shape, x.options()));
-    ws[i] = &plans[i]->w.w;
     ys[i] = outs.back().data_ptr();
   }
   Arena a;
@@ -371,7 +375,6 @@ py::object shared_rows(const std::vector<std::shared_ptr<LinearPlan>>& plans, co
     check(L.gb_fp8_act_qdq(xc.data_ptr(), a.ptr(xq), M, K, rule, stream));
     for (size_t i = 0; i < n; ++i) check(L.gb_gemv(a.ptr(xq), M, ws[i], GB_ACT_NONE, rule, ys[i], a.ptr(scratch), need, stream));
   } else {
-    if (((uintptr_t)xc.data_ptr() & 15u) != 0) return py::none();
     const int q = a.add(fp4 ? M * K / 2 : M * K), sf = a.add(fp4 ? L.gb_nvfp4_sf_bytes(M, K) : 0), as = a.add(M * 4);
     // one decoded copy at a time, in the place of the largest: multiplied while it lies in L2, and no more memory than one by one
     int64_t rows = 0;

@@ -176,6 +176,7 @@ GB_API int64_t gb_gemv_hinted_workspace_bytes(int64_t M, int64_t N, int64_t K);
 /* Several matrices that read the same rows (q and kv of an attention block), 1 to 4 of them: y_i[M, N_i], as gb_gemv_hinted
  * gives each, with the rows bucketed once and one launch for all.  The fp4 formats named there, the same for every
  * matrix, one codebook each; anything else is GB_EUNSUPPORTED.  workspace: gb_gemv_hinted_workspace_bytes(M, any N, K). */
+GB_API int gb_gemv_shared_applies(const gb_weight* const* w, int n_weights, int scales_e4m3);   /* 1: it takes them (16-byte aligned rows) */
 GB_API int gb_gemv_shared(const void* x_bf16, int64_t M, const gb_weight* const* w, int n_weights, int scales_e4m3, int scale_rule,
                           void* const* y_bf16, void* workspace, int64_t workspace_bytes, void* stream);
 

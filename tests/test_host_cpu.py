@@ -948,3 +948,25 @@ def test_row_scales_of_every_tile_start_where_four_are_read_at_once():
             unit = (4096 if rows > 16 else 2048) + codes * 128
             want = up(tiles * (K // 256) * unit) + up(tiles * ((rows + 7) // 8 * 8) * 4) + up(tiles * rows * (K // 16) * 4)
             assert lib.gb_moe_fp4_operand_bytes(n(P), n(E), n(K), rows) == want, (P, E, K, rows)
+
+
+def test_which_matrices_share_a_decode_launch_is_known_before_the_call():
+    """Format, codebooks per row and width decide, without a device: layers that go one by one cost no allocation first."""
+    from gridbook_b200 import _native as nat
+    lib = nat.load()
+
+    def weight(k=16, type_size=80, rows=128, K=512, off=None, mode=0, n_sub=2, coding=2):
+        fmt = nat.GbFormat(grid=0, mode=mode, k_bits=k, n_sub=n_sub, type_size=type_size, scale_coding=coding)
+        return nat.GbWeight(qw=256, row_stride=K // 256 * type_size, codebook=256, cb_row_offset=off, compose=256 if coding == 2 else None,
+                            weight_scale=None, global_scale=1.0, rows=rows, K=K, fmt=fmt)
+
+    def applies(*ws, exact=1):
+        arr = (ctypes.POINTER(nat.GbWeight) * len(ws))(*[ctypes.pointer(w) for w in ws])
+        return lib.gb_gemv_shared_applies(arr, len(ws), exact)
+
+    lit = dict(k=8, type_size=48, mode=2, n_sub=1, coding=1)
+    assert applies(weight(), weight(rows=64)) == 1 and applies(weight(**lit), weight(**lit), weight(**lit), weight(**lit)) == 1
+    for others in [(weight(rows=63),), (weight(K=1024),), (weight(off=256),), (weight(k=20, type_size=96),), (weight(**lit),),
+                   (weight(type_size=73),), (weight(),) * 4]:
+        assert applies(weight(), *others) == 0
+    assert applies(weight(), weight(), exact=0) == 0 and applies() == 0
