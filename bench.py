@@ -842,8 +842,8 @@ def bench_prefill(args, device):
                     kernels.gemm_fp4(a, sfa, b, sfb, a_scale=asc)
                     ms_gemm = timed_ms(lambda: kernels.gemm_fp4(a, sfa, b, sfb, a_scale=asc), 3, sync)
                     tf = flops / ms_gemm / 1e9
-                    pair = "gemm_pair_kernel (kind::mxf4nvf4)" if M > 128 else "gemm_rows_kernel (kind::mxf4nvf4)"
-                    entry.update({"kernel": pair, "gemm_tflops": round(tf, 1), "gemm_ms": round(ms_gemm, 4),
+                    kernel = f"{kernels.gemm_kernel(M, N, K // 2, True)} (kind::mxf4nvf4)"
+                    entry.update({"kernel": kernel, "gemm_tflops": round(tf, 1), "gemm_ms": round(ms_gemm, 4),
                                   "pct_fp4_nominal": round(100 * tf / NOMINAL_TFLOPS["fp4"], 2),
                                   "pct_of_4x_measured_bf16": round(100 * tf / (4 * bf16_meas), 2)})
                     del a, sfa, b, sfb
@@ -858,14 +858,14 @@ def bench_prefill(args, device):
                                     "unit": "TFLOP/s", "frac": round(tf / NOMINAL_TFLOPS["fp4"], 4),
                                     "peak_kind": "fp4 dense, nominal (no measured fp4 figure on this pool)",
                                     "frac_of_4x_measured_bf16": round(tf / (4 * bf16_meas), 4),
-                                    "kernel": pair, "workload": f"{name} {N}x{K}, M={M}, literal"}
+                                    "kernel": kernel, "workload": f"{name} {N}x{K}, M={M}, literal"}
                 else:
                     a, sa = kernels.fp8_quantize_rows(x)
                     b = kernels.expand_fp8(w)
                     kernels.gemm_tn(a, b, a_scale=sa, b_scale=w.weight_scale)
                     ms_gemm = timed_ms(lambda: kernels.gemm_tn(a, b, a_scale=sa, b_scale=w.weight_scale), 3, sync)
                     tf = flops / ms_gemm / 1e9
-                    entry.update({"kernel": f"gemm_{'pair' if M > 128 else 'tn'}_kernel (kind::f8f6f4)", "gemm_tflops": round(tf, 1),
+                    entry.update({"kernel": f"{kernels.gemm_kernel(M, N, K, False)} (kind::f8f6f4)", "gemm_tflops": round(tf, 1),
                                   "gemm_ms": round(ms_gemm, 4),
                                   "pct_fp8_nominal": round(100 * tf / NOMINAL_TFLOPS["fp8"], 2),
                                   "pct_of_2x_measured_bf16": round(100 * tf / (2 * bf16_meas), 2)})

@@ -453,6 +453,10 @@ bool gb_gemm_rows_applies(bool fp4, int64_t M, int64_t N, int64_t k_tiles) {
   return M <= 192 || (M <= 1024 && s.tiles <= gb_sm_count() && s.per_slice <= 64);
 }
 
+extern "C" int gb_gemm_uses_rows(int fp4, int64_t M, int64_t N, int64_t k_bytes) {
+  return M >= 1 && N >= 1 && k_bytes >= kSlabBytes && gb_gemm_rows_applies(fp4 != 0, M, N, k_bytes / kSlabBytes) ? 1 : 0;
+}
+
 int gb_gemm_rows(const void* X, const void* W, void* D, int64_t M, int64_t N, int64_t K, int kind, const float* a_scale,
                  const float* b_scale, float global_scale, cudaStream_t stream) {
   GemmRowsParams p = {};

@@ -486,6 +486,11 @@ def gemm_fp4(a_packed: torch.Tensor, sfa: torch.Tensor, b_packed: torch.Tensor, 
     return out
 
 
+def gemm_kernel(M: int, N: int, k_bytes: int, fp4: bool) -> str:
+    """The kernel that :func:`gemm_fp4` or :func:`gemm_tn` launches for a product; ``k_bytes``: of a row of either operand."""
+    return "gemm_rows_kernel" if nat.load("prefill tensor-core GEMM").gb_gemm_uses_rows(int(fp4), M, N, k_bytes) else "gemm_pair_kernel"
+
+
 def gemm_tn(a: torch.Tensor, b: torch.Tensor, *, a_scale=None, b_scale=None, global_scale: float = 1.0):
     """bf16 D[M, N] = scales * A[M, K] . B[N, K]^T on the tcgen05 tensor cores; A and B both bf16
     or both float8_e4m3fn."""

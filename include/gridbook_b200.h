@@ -260,6 +260,10 @@ GB_API int gb_nvfp4_quantize_rows(const void* x_bf16, int64_t M, int64_t K, floa
 GB_API int gb_gemm_fp4(const void* A, const void* sfa, const void* B, const void* sfb, void* D_bf16, int64_t M,
                        int64_t N, int64_t K, const float* a_scale, float global_scale, void* stream);
 
+/* Whether gb_gemm_tn (fp4 = 0) or gb_gemm_fp4 (1) gives a product to the kernel for few rows or narrow layers, gemm_rows_kernel,
+ * instead of the CTA pairs of gemm_pair_kernel.  k_bytes: of a row of either operand. */
+GB_API int gb_gemm_uses_rows(int fp4, int64_t M, int64_t N, int64_t k_bytes);
+
 /* The same GEMM over expert segments (routed prefill): A [P,K] holds the routed rows sorted by
  * expert, expert e owning rows [seg_offsets[e], seg_offsets[e+1]) (gb_moe_route's offsets, read
  * on the device: no host read); B [E*N,K] is the decoded stack (gb_expand_* over all E*N rows);
