@@ -345,9 +345,9 @@ py::object shared_rows(const std::vector<std::shared_ptr<LinearPlan>>& plans, co
   // decided before anything is allocated: layers that go one by one allocate again
   const gb_weight* ws[4];
   for (size_t i = 0; i < n; ++i) ws[i] = &plans[i]->w.w;
-  const bool odd = x.is_contiguous() && ((uintptr_t)x.data_ptr() & 15u) != 0;   // (a copy starts at a multiple of sixteen bytes)
-  if (decode && fp4 && (odd || L.gb_gemv_shared_applies(ws, (int)n, plans[0]->w.scales_e4m3 ? 1 : 0) == 0)) return py::none();
-  if (!decode && odd) return py::none();
+  // rows off the vector alignment (as they lie: a copy starts on it) are the layers' to take or to refuse
+  if (x.is_contiguous() && ((uintptr_t)x.data_ptr() & 15u) != 0) return py::none();
+  if (decode && fp4 && L.gb_gemv_shared_applies(ws, (int)n, plans[0]->w.scales_e4m3 ? 1 : 0) == 0) return py::none();
   const c10::cuda::CUDAGuard guard(x.device());
   void* stream = c10::cuda::getCurrentCUDAStream().stream();
   const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
