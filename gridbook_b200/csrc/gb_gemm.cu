@@ -396,20 +396,34 @@ int get_encoder(EncodeTiledFn* out) {
   return GB_OK;
 }
 
-int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int elem_bytes, int box_rows) {
+// Rows of `pitch` bytes, `inner` elements each, in boxes of box_inner x box_rows.
+int encode_rows(void* map, CUtensorMapDataType type, void* base, uint64_t inner, uint64_t rows, uint64_t pitch, uint32_t box_inner,
+                uint32_t box_rows, CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promotion) {
   EncodeTiledFn enc;
   int rc = get_encoder(&enc);
   if (rc != GB_OK) return rc;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)K * elem_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)(kSlabBytes / elem_bytes), (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
-                         const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint64_t dims[2] = {inner, rows}, strides[1] = {pitch};
+  const cuuint32_t box[2] = {box_inner, box_rows}, estr[2] = {1, 1};
+  auto encode = [&]() {
+    return enc((CUtensorMap*)map, type, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+    // a thread that has launched nothing yet: the driver knows its device only from the runtime's first call that needs one
+    int device;
+    GB_CUDA_OK(cudaGetDevice(&device));
+    GB_CUDA_OK(cudaSetDevice(device));
+    r = encode();
+  }
   if (r != CUDA_SUCCESS) return gb_fail(GB_ECUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
   return GB_OK;
+}
+
+int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int elem_bytes, int box_rows) {
+  return encode_rows(map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, const_cast<void*>(base),
+                     (uint64_t)K, (uint64_t)rows, (uint64_t)K * elem_bytes, (uint32_t)(kSlabBytes / elem_bytes), (uint32_t)box_rows,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
 }
 
 }  // namespace
@@ -418,18 +432,8 @@ int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int el
 // row slices of a packed weight matrix.  `map_out` points at a CUtensorMap.
 int gb_tensor_map_bytes_2d(void* map_out, const void* base, uint64_t inner_bytes, uint64_t rows,
                            uint64_t pitch_bytes, uint32_t box_bytes, uint32_t box_rows) {
-  EncodeTiledFn enc;
-  int rc = get_encoder(&enc);
-  if (rc != GB_OK) return rc;
-  const cuuint64_t dims[2] = {(cuuint64_t)inner_bytes, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)pitch_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc((CUtensorMap*)map_out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims,
-                         strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return gb_fail(GB_ECUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
-  return GB_OK;
+  return encode_rows(map_out, CU_TENSOR_MAP_DATA_TYPE_UINT8, const_cast<void*>(base), inner_bytes, rows, pitch_bytes, box_bytes, box_rows,
+                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
 }
 
 int gb_tensor_map_operand(void* map_out, const void* base, int64_t rows, int64_t K, int elem_bytes, int box_rows) {
@@ -438,18 +442,8 @@ int gb_tensor_map_operand(void* map_out, const void* base, int64_t rows, int64_t
 
 // Row-major bf16 output [M, N] in boxes of 32 x 32, 64-byte swizzle.
 int gb_tensor_map_out(void* map_out, void* base, int64_t M, int64_t N) {
-  EncodeTiledFn enc;
-  int rc = get_encoder(&enc);
-  if (rc != GB_OK) return rc;
-  const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
-  const cuuint64_t strides[1] = {(cuuint64_t)N * 2};
-  const cuuint32_t box[2] = {32, 32};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc((CUtensorMap*)map_out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return gb_fail(GB_ECUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
-  return GB_OK;
+  return encode_rows(map_out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, (uint64_t)N, (uint64_t)M, (uint64_t)N * 2, 32, 32,
+                     CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
 }
 
 int gb_prepare_gemm() {

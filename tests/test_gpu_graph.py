@@ -167,8 +167,27 @@ def test_one_layer_on_several_streams_and_threads(name):
         t.join()
     torch.cuda.synchronize()
     assert _native.device_status(0) == 0
+    assert [len(g) for g in got] == [140, 140, 40]
     for i in range(3):
         assert all(torch.equal(y, want[i]) for y in got[i]), (name, i)
+
+
+@pytest.mark.parametrize("M", [1, 4, 300])
+@pytest.mark.parametrize("name", ["literal", "fp8k32"])
+def test_the_first_cuda_call_of_a_thread(name, M):
+    """A thread that has made no CUDA call yet has no context, in which the driver encodes a launch's tensor maps."""
+    from concurrent.futures import ThreadPoolExecutor
+    from gridbook_b200 import _native
+    _native.prepare(0)
+    dev = torch.device("cuda:0")
+    lin = _layer(name, 512, 2048, dev)
+    (x,) = _rows(1, M, 2048, dev)
+    want = lin(x)
+    torch.cuda.synchronize()
+    with ThreadPoolExecutor(1) as pool:
+        got = pool.submit(lin, x).result()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and _native.device_status(0) == 0
 
 
 def test_one_row_of_a_layer_on_several_streams():
