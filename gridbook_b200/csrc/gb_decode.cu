@@ -562,8 +562,10 @@ int launch_expand_fp8_fast(const gb_weight* w, int64_t row0, int64_t nrows, void
   const int sms = gb_sm_count();
   if (sms <= 0) return gb_fail(GB_ECUDA, "no usable CUDA device: %s", gb_last_error());
   const int64_t n_sb = w->K / 256;
-  // eight CTAs per SM where there are rows for them, at least two steps of every warp each so that the tables pay
-  const int64_t least = (2 * (kThreads / 32) * 4 * kF8Unroll + n_sb - 1) / n_sb;
+  // Eight CTAs per SM where there are rows for them, at least 64 superblocks each so that the tables pay.  Fewer and larger ones
+  // pile up on the SMs that the launch ahead leaves first: k = 32, 4096 x 4096 behind the quantiser of 700 rows, both launches / the
+  // whole linear, us: 256 superblocks 17.2 / 35.8, 128 11.8 / 29.2, 64 10.8 / 27.5, 32 the same.
+  const int64_t least = (64 + n_sb - 1) / n_sb;
   int64_t rows_per = (nrows + (int64_t)sms * 8 - 1) / ((int64_t)sms * 8);
   if (rows_per < least) rows_per = least;
   GB_REQUIRE(rows_per * n_sb < (1ll << 31), "too many superblocks per CTA");
