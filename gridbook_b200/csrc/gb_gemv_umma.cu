@@ -40,7 +40,7 @@ constexpr int kDecWarps = 16;                             // four warpgroups, on
 constexpr int kCtlWarps = 6;                              // raw producer, x producer, four MMA issuers
 constexpr int kUmmaThreads = 32 * (kCtlWarps + kDecWarps);
 constexpr int kMaxRows = 128;                             // activation rows
-constexpr int kMaxSlices = 8;                             // of K: CTAs of a cluster
+constexpr int kMaxSlices = 16;                            // of K: CTAs of a cluster (past eight only where the GPU has room, see max_clusters)
 constexpr int kABufCols = 64;                             // half a superblock: 128 weights of K as bf16 pairs
 constexpr uint32_t kACol0 = 256;                          // columns [0, 256): one accumulator per MMA issuer
 constexpr uint32_t kTmemCols = 512;
@@ -919,7 +919,9 @@ int max_clusters(int size) {
   return n;
 }
 
-// K slices: enough CTAs for the SMs when the layer has few 128-row tiles; no more clusters than run at once.
+// K slices: enough CTAs for the SMs when the layer has few 128-row tiles; no more clusters than run at once.  Eight at most lost
+// against a slice per raw stage and a second launch where two or four tiles have a long K (us, those / eight / sixteen: fp8 k = 32,
+// 256 x 17408, 4 rows 10.4 / 11.8 / 9.2, 64 rows 11.6 / 15.6 / 12.0, 512 x 16384, 4 rows 9.9 / 10.2 / 8.5); from 1024 weight rows on alike.
 void umma_plan(int F, int tiles, int n_sb, int sms, int* slices, int* stages_per_slice) {
   const int per_stage = fmt_info(F).sb_per_stage;
   const int n_raw = (n_sb + per_stage - 1) / per_stage;
@@ -1003,7 +1005,8 @@ void fill_weight_params(UmmaParams& p, const gb_weight* w, int64_t rows_total) {
 int gb_prepare_umma() {
 #define GB_UMMA_ATTR(G, F, rows)                                                                          \
   GB_CUDA_OK(cudaFuncSetAttribute((const void*)umma_decode_kernel<G, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                  kSmemCap))
+                                  kSmemCap));                                                             \
+  if (!G) GB_CUDA_OK(cudaFuncSetAttribute((const void*)umma_decode_kernel<G, F>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
   GB_UMMA_ATTR(false, kFmtLit, kMaxRows);
   GB_UMMA_ATTR(false, kFmtK16, kMaxRows);
   GB_UMMA_ATTR(false, kFmtFp8, kMaxRows);

@@ -43,3 +43,24 @@ def test_fp8_decode_rows(k, n_sub, M, parts, K, scales):
     # row by row magnitudes differ by powers of two: compare every output column on its own scale
     s = np.where(d["weight_scale"] == 0, 1.0, d["weight_scale"])
     assert_close_bf16(got / s, ref / s, f"k={k} M={M} {parts} {scales}", atol_rel=1e-6)
+
+
+@pytest.mark.parametrize("k,n_sub", [(32, 4), (16, 2)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 8192), (4, 256, 17408), (9, 512, 16384), (33, 130, 5632), (64, 256, 17408), (70, 128, 6400)])
+def test_narrow_layers_of_long_rows(k, n_sub, M, N, K):
+    """One to four row tiles: K over clusters of nine to sixteen CTAs where the GPU has room for them, more CTAs than groups of eight
+    rows to own, a last slice that is short."""
+    from gridbook_b200 import _native, kernels, synth
+    from gridbook_b200.formats import CBFormat
+    _native.prepare(0)
+    dev = torch.device("cuda:0")
+    fmt = CBFormat("fp8", k, n_sub=n_sub)
+    d = synth.make_linear(fmt, N, K, seed=N + M)
+    w = synth.to_device_weight(d, dev)
+    assert M <= kernels.row_batch_max_rows(w)
+    x = synth.make_activations(M, K, seed=3)
+    got, ref = f32_of(kernels.gemv(synth.bf16_tensor(x, dev), w, act="fp8")), oracle_linear(x, d)
+    torch.cuda.synchronize()
+    assert _native.device_status(0) == 0
+    s = np.where(d["weight_scale"] == 0, 1.0, d["weight_scale"])
+    assert_close_bf16(got / s, ref / s, f"k={k} M={M} {N}x{K}", atol_rel=1e-6)
