@@ -398,15 +398,15 @@ py::object shared_rows(const std::vector<std::shared_ptr<LinearPlan>>& plans, co
   return py::cast(outs);
 }
 
-// Several linears that read the same activation row, one launch; None when they have no such kernel.  `routes`: of the
-// layers whose calls may be replaced for more rows than one; empty: none.
-py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, const at::Tensor& x, int rule, const std::vector<Route>& routes) {
+// Several linears that read the same activation row, one launch; None when they have no such kernel.  `routes`: called for the
+// layers' routes where their calls may be replaced by more than the table kernel; none or empty: they may not.
+py::object shared_row(const std::vector<std::shared_ptr<LinearPlan>>& plans, const at::Tensor& x, int rule, const py::object& routes) {
   const size_t n = plans.size();
   if (n < 2 || n > 4 || !x.is_cuda() || x.dim() < 1) return py::none();
   const int64_t K = plans[0]->w.w.K;
   bool tables = x.numel() == K;
   for (const auto& p : plans) tables = tables && p->tables;
-  if (!tables) return shared_rows(plans, x, rule, routes);
+  if (!tables) return routes.is_none() ? py::none() : shared_rows(plans, x, rule, routes().cast<std::vector<Route>>());
   if (x.numel() != K || x.size(-1) != K) return py::none();   // another width: refused where the layers are called one by one
   for (const auto& p : plans)
     if (!p->tables || p->w.w.K != K) return py::none();
@@ -709,5 +709,5 @@ PYBIND11_MODULE(_gb_torch, m) {
       .def_property_readonly("fp4", &MoEPlan::fp4)
       .def("__call__", &MoEPlan::forward, py::call_guard<py::gil_scoped_release>())
       .def_property_readonly("route", [](const MoEPlan& p) { return p.route.load(); });
-  m.def("shared_row", &shared_row, py::arg("plans"), py::arg("x"), py::arg("rule"), py::arg("routes") = std::vector<Route>());
+  m.def("shared_row", &shared_row, py::arg("plans"), py::arg("x"), py::arg("rule"), py::arg("routes") = py::none());
 }
