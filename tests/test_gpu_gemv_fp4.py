@@ -352,8 +352,8 @@ def test_rings_wrap_from_tile_to_tile(dev, name, M):
 @pytest.mark.parametrize("name", ["lit", "k12", "k16", "k20", "fp8lit", "fp8k32", "fp8k30"])
 def test_rows_shared_by_several_matrices(dev, name, M):
     """Rows bucketed or quantised once for matrices of different heights, codebooks, scales and outputs (in one launch for the
-    decode batches of the fp4 grid): as each layer gives by itself, up to the order of the sum, with strided rows and rows off
-    the 16-byte alignment among them (refused alike where the layers refuse them), and nothing replaced where a layer is watched."""
+    decode batches of the fp4 grid): as each layer gives by itself, up to the order of the sum, with misaligned and
+    strided rows among them, and nothing replaced where a layer is watched."""
     from gridbook_b200 import _native, formats, synth
     from gridbook_b200.linear import CBLinear, apply_shared_row
     fmt = {"fp8lit": formats.FP8_LITERAL, "fp8k32": formats.FP8_CB_K32, "fp8k30": formats.CBFormat("fp8", 30, n_sub=4)}.get(name) or _fmt(name)
@@ -364,11 +364,41 @@ def test_rows_shared_by_several_matrices(dev, name, M):
         scale = None if fmt.is_fp4 else (torch.rand(N, generator=gen, device=dev) + 0.5) * 0.02
         lins.append(lin.load(synth.make_packed_device(fmt, N, K, gen, dev), scale, dev))
     wide = torch.randn(M, K + 64, generator=gen, device=dev).to(torch.bfloat16)
-    for x in (wide[:, :K].contiguous(), wide[:, 64:], *(wide.view(-1)[at:at + M * K].view(M, K) for at in (8, 1, 5))):
+    for x in (wide[:, :K].contiguous(), wide[:, 64:], wide.view(-1)[8:8 + M * K].view(M, K)):
+        want = [lin(x) for lin in lins]
+        got = apply_shared_row(lins, x)
+        torch.cuda.synchronize()
+        assert _native.device_status(0) == 0
+        for a, b in zip(got, want):
+            assert a.shape == b.shape and a.is_contiguous()
+            assert_close_bf16(f32_of(a), f32_of(b), f"{name} M={M}", atol_rel=1e-6)
+    seen = []
+    hook = lins[1].register_forward_hook(lambda mod, args, out: seen.append(1))
+    assert len(apply_shared_row(lins, x)) == 3 and (M == 1 and name == "lit") != bool(seen)
+    hook.remove()
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 100, 300])
+@pytest.mark.parametrize("name", ["lit", "k16", "fp8lit", "fp8k32", "fp8k30"])
+def test_rows_off_the_alignment_shared_by_several_matrices(dev, name, M):
+    """Rows that start two or ten bytes into another tensor: as each layer gives by itself, and refused in the same words where a
+    layer refuses them (past 16 rows most kernels read sixteen bytes at a time)."""
+    from gridbook_b200 import _native, formats, synth
+    from gridbook_b200.linear import CBLinear, apply_shared_row
+    fmt = {"fp8lit": formats.FP8_LITERAL, "fp8k32": formats.FP8_CB_K32, "fp8k30": formats.CBFormat("fp8", 30, n_sub=4)}.get(name) or _fmt(name)
+    K, lins = 2048, []
+    gen = torch.Generator(device=dev).manual_seed(M)
+    for i, N in enumerate((256, 520)):
+        lin = CBLinear(fmt, K, [N], [synth.codebook_tables(fmt, i)], prefix=f"off.{i}")
+        scale = None if fmt.is_fp4 else (torch.rand(N, generator=gen, device=dev) + 0.5) * 0.02
+        lins.append(lin.load(synth.make_packed_device(fmt, N, K, gen, dev), scale, dev))
+    wide = torch.randn(M * K + 64, generator=gen, device=dev).to(torch.bfloat16)
+    for at in (1, 5):
+        x = wide[at:at + M * K].view(M, K)
         try:
             want = [lin(x) for lin in lins]
-        except RuntimeError as e:                            # past 16 rows most kernels read sixteen bytes at a time
-            assert M > 16 and x.data_ptr() % 16
+        except RuntimeError as e:
+            assert M > 16
             with pytest.raises(RuntimeError) as again:
                 apply_shared_row(lins, x)
             assert str(again.value) == str(e)
@@ -377,12 +407,7 @@ def test_rows_shared_by_several_matrices(dev, name, M):
         torch.cuda.synchronize()
         assert _native.device_status(0) == 0
         for a, b in zip(got, want):
-            assert a.shape == b.shape and a.is_contiguous()
-            assert_close_bf16(f32_of(a), f32_of(b), f"{name} M={M}", atol_rel=1e-6)
-    x, seen = wide[:, :K].contiguous(), []
-    hook = lins[1].register_forward_hook(lambda mod, args, out: seen.append(1))
-    assert len(apply_shared_row(lins, x)) == 3 and (M == 1 and name == "lit") != bool(seen)
-    hook.remove()
+            assert_close_bf16(f32_of(a), f32_of(b), f"{name} M={M} at {at}", atol_rel=1e-6)
 
 
 @pytest.mark.parametrize("name,pass_rows", [("lit", 1), ("lit", 5), ("k16", 7), ("lit", 13), ("k16", 18), ("lit", 33), ("lit", 61)])
