@@ -84,6 +84,26 @@ int* gb_status_word() {
   return g_status[dev];
 }
 
+int GbClusters::ask(const void* kernel, int threads, size_t smem, int size) {
+  const int dev = current_device_slot();
+  if (dev < 0) return 0;
+  std::lock_guard<std::mutex> lock(mutex);
+  int& known = n[dev][size];
+  if (known == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, (unsigned)size);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)size; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&known, kernel, &cfg) != cudaSuccess) { known = 0; cudaGetLastError(); }
+  }
+  return known;
+}
+
 int gb_check_format(const gb_format& f, int64_t K) {
   GB_REQUIRE(K > 0 && K % 256 == 0, "K=%lld must be a positive multiple of 256", (long long)K);
   GB_REQUIRE(f.grid == GB_GRID_FP4 || f.grid == GB_GRID_FP8, "unknown grid %d", f.grid);

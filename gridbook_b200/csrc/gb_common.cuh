@@ -8,6 +8,8 @@
 #include <stdio.h>
 #include <stdarg.h>
 
+#include <mutex>
+
 #include "../../include/gridbook_b200.h"
 
 #define GB_DEVINL __device__ __forceinline__
@@ -22,6 +24,13 @@ int* gb_status_word();             // device int the kernels raise on a timed-ou
 
 bool gb_pdl_enabled();             // false when GRIDBOOK_B200_PDL=0 (plain stream order)
 void gb_count_launch();            // every kernel launch of this library bumps gb_launch_count()
+
+// Clusters of a kernel's CTAs (along y, up to sixteen) that run at once on the current device, by their size; asked once.
+struct GbClusters {
+  std::mutex mutex;
+  int n[64][17];                   // 0: not asked yet
+  int ask(const void* kernel, int threads, size_t smem, int size);
+};
 
 // Kernel launch with the programmatic-stream-serialization attribute (see gb_pdl_wait).
 template <typename... KArgs, typename... Args>
@@ -94,13 +103,13 @@ inline GbFp4Tiles gb_fp4_tiles(int64_t P, int64_t E, int64_t K) {
   t.bytes = t.tail_at + up(t.tiles * 64 * (K / 16) * 4);
   return t;
 }
-// The prefill GEMMs on CTA pairs (gb_gemm_pair.cu).
-// The same for few rows or narrow layers (gb_gemm_rows.cu), where gb_gemm_rows_applies says so.
+// The prefill GEMM for few rows or narrow layers (gb_gemm_rows.cu), where gb_gemm_rows_applies says so.
 bool gb_gemm_rows_applies(bool fp4, int64_t M, int64_t N, int64_t k_tiles);
 int gb_gemm_rows(const void* X, const void* W, void* D, int64_t M, int64_t N, int64_t K, int kind, const float* a_scale,
                  const float* b_scale, float global_scale, cudaStream_t stream);
 int gb_gemm_fp4_rows(const void* X, const void* sfx, const void* W, const void* sfw, void* D, int64_t M, int64_t N, int64_t K,
                      const float* a_scale, float global_scale, cudaStream_t stream);
+// The prefill GEMMs on CTA pairs (gb_gemm_pair.cu), for the others.
 int gb_gemm_pair(const void* A, const void* B, void* D, int64_t M, int64_t N, int64_t K, int kind, const float* a_scale,
                  const float* b_scale, float global_scale, cudaStream_t stream);
 int gb_gemm_fp4_pair(const void* A, const void* sfa, const void* B, const void* sfb, void* D, int64_t M, int64_t N, int64_t K,
@@ -486,6 +495,22 @@ GB_DEVINL uint32_t gb_smem_u32(const void* p) {
 
 GB_DEVINL void gb_mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gb_smem_u32(bar)), "r"(count));
+}
+
+// One lane of a warp that has converged.  Warps that load, issue MMAs or copy walk their loops as a whole, with values that
+// are the same in every lane, and the elected lane issues: the operands stay in uniform registers.  (In code that only
+// lane 0 enters, each is moved there first: 53 clocks to issue an MMA whatever its size, 45 or more a copy.  One dense layer,
+// us: 333 rows K20 249 -> 233, 2048 rows literal 522 -> 491, 8192 rows fp8 2853 -> 2677; routed, 4096 tokens, 656 -> 613.)
+GB_DEVINL bool gb_elect_one() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
+
+// All threads of a thread-block cluster; what was written before, to a peer's shared memory too, is visible behind it.
+GB_DEVINL void gb_cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 GB_DEVINL void gb_mbar_expect_tx(uint64_t* bar, uint32_t bytes) {

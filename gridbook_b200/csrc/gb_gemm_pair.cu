@@ -134,15 +134,7 @@ GB_DEVINL bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag
   wait_slow<kOfPair>(bar, parity, abort_flag, status, code);
   return !__any_sync(0xffffffffu, *abort_flag != 0);
 }
-// The loading, issuing and copying warps walk their loops as a whole, with values that are the same in every lane, and one
-// elected lane issues: the operands stay in uniform registers.  (In code that only lane 0 enters, each is
-// moved there first: 53 clocks to issue an MMA whatever its size, 45 or more a copy.  One dense layer, us: 333 rows K20
-// 249 -> 233, 2048 rows literal 522 -> 491, 8192 rows fp8 2853 -> 2677; routed, 4096 tokens, 656 -> 613.)
-GB_DEVINL bool elect_one() {
-  uint32_t one;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-  return one != 0;
-}
+// A value that is the same in every lane, for a warp that walks its loop whole (gb_elect_one).
 GB_DEVINL int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 // Tile load into this CTA's shared memory that reports to a barrier of the pair.
 GB_DEVINL void tma_load_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
@@ -191,9 +183,6 @@ GB_DEVINL void commit_to(uint32_t bar) {
 GB_DEVINL void commit_pair(uint32_t bar, uint32_t to_peer) {
   commit_to(bar);
   commit_to(bar + to_peer);
-}
-GB_DEVINL void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 GB_DEVINL void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
@@ -323,7 +312,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  cluster_sync();                                                        // both CTAs' barriers exist
+  gb_cluster_sync();                                                        // both CTAs' barriers exist
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *slot_ptr;
   gb_pdl_wait();
@@ -361,7 +350,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     constexpr int slab_elems = kKind == kBf16 ? kSlabBytes / 2 : kSlabBytes;   // E2M1 pairs and E4M3 go by bytes
     const uint32_t full_pair = (uint32_t)uniform((int)leader_addr(full_bar));
     const int me = uniform((int)rank);
-    const bool one = elect_one();
+    const bool one = gb_elect_one();
     int s = 0;
     uint32_t ph = 1;
     bool ok = true;
@@ -402,7 +391,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       to_peer = (uint32_t)uniform((int)(to_peer - full_bar));
       const uint32_t tmem = (uint32_t)uniform((int)tmem_base);
       const int tiles = uniform(my_tiles);
-      const bool one = elect_one();
+      const bool one = gb_elect_one();
       int s = 0, set = 0;
       uint32_t ph = 0, sf_ph = 0;
       bool ok = true;
@@ -448,7 +437,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t k = (uint32_t)(uniform(warp) - kEpiWarps - 2);
     if (uniform((int)rank) == 0) {
       const uint32_t tmem = (uint32_t)uniform((int)tmem_base);
-      const bool one = elect_one();
+      const bool one = gb_elect_one();
       int s = 0, set = 0;
       uint32_t ph = 0, sf_ph = 1;
       const int total = uniform(my_tiles) * p.k_tiles;
@@ -608,7 +597,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   if (*abort_flag && threadIdx.x == 0) __nanosleep(1000000);   // loads still in flight land before the memory goes
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  cluster_sync();                                            // the peer may still signal barriers here
+  gb_cluster_sync();                                            // the peer may still signal barriers here
   if (warp == kEpiWarps + 1)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTmemCols) : "memory");
 }

@@ -15,7 +15,6 @@
 #include "gb_common.cuh"
 
 #include <cuda.h>
-#include <mutex>
 
 namespace {
 
@@ -73,13 +72,6 @@ GB_DEVINL bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag
   wait_slow(bar, parity, abort_flag, status, code);
   return !__any_sync(0xffffffffu, *abort_flag != 0);
 }
-// The loading and issuing warps walk their loops whole with one elected lane issuing, so that the operands stay in uniform
-// registers (see gb_gemm_pair.cu).
-GB_DEVINL bool elect_one() {
-  uint32_t one;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-  return one != 0;
-}
 GB_DEVINL void expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -120,10 +112,6 @@ GB_DEVINL void mma(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_
 }
 GB_DEVINL void commit_to(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-GB_DEVINL void cluster_sync() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 GB_DEVINL void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -170,10 +158,11 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   const uint32_t tmem = __shfl_sync(0xffffffffu, slot_s, 0);
   gb_pdl_wait();
 
+  // The loading and issuing warps walk their loops whole with one elected lane issuing (gb_elect_one).
   if (warp == kEpiWarps) {
     // ------------------------------- producer -----------------------------------
     constexpr int slab_elems = kKind == kBf16 ? kSlabBytes / 2 : kSlabBytes;   // E2M1 pairs and E4M3 go by bytes
-    const bool one = elect_one();
+    const bool one = gb_elect_one();
     const int g0 = m0 / 128, groups = kKind == kFp4 ? (m0 + rows - 1) / 128 - g0 + 1 : 0;   // 128-row groups of the pass: one or two
     const uint32_t bytes = kBM * kSlabBytes + x_bytes + (kKind == kFp4 ? (uint32_t)(1 + groups) * kAtoms : 0u);
     int s = 0;
@@ -196,7 +185,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
   } else if (warp == kEpiWarps + 1) {
     // ------------------------------- MMA issuer ---------------------------------
-    const bool one = elect_one();
+    const bool one = gb_elect_one();
     const uint32_t idesc = p.idesc | (uint32_t)(cols >> 3) << 17 | (uint32_t)(kBM >> 4) << 24;
     const bool two = kKind == kFp4 && (m0 + rows - 1) / 128 > m0 / 128;
     const uint32_t shift = kKind == kFp4 && m0 % 128 != 0 ? 2u : 0u;         // a pass that starts in the middle of a 128-row group
@@ -278,7 +267,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // Sums into the shared memory of the CTA that owns the activation row, [slice][own row][feature], over the operand ring:
     // every CTA of the cluster has finished its MMAs, and with them its loads.  Rows are owned in sixteens.
     const int own = (cols / 16 + p.slices - 1) / p.slices * 16;
-    cluster_sync();
+    gb_cluster_sync();
     if (live) {
       for (int c = (warp >> 2) * 16; c < cols; c += 32) {
         uint32_t v[16];
@@ -293,7 +282,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + (uint32_t)i * kBM * 4u), "r"(v[i]) : "memory");
       }
     }
-    cluster_sync();                                          // the last access to another CTA's memory lies in front of it
+    gb_cluster_sync();                                          // the last access to another CTA's memory lies in front of it
     if (live) {
       const int f = lane * 4, left = (int)min((int64_t)kBM, p.N - n0) - f;
       float bs[4];
@@ -331,28 +320,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }
 
-std::mutex g_mutex;
-int g_clusters[64][kMaxSlices + 1];                          // clusters of a size that run at once, per device (0: not asked)
-
-int max_clusters(int size) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  std::lock_guard<std::mutex> lock(g_mutex);
-  int& n = g_clusters[dev][size];
-  if (n == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1, (unsigned)size);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemMax;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)size; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_rows_kernel<kFp8>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
-  }
-  return n;
-}
+GbClusters g_clusters;
+int max_clusters(int size) { return g_clusters.ask((const void*)gemm_rows_kernel<kFp8>, kThreads, kSmemMax, size); }
 
 // Rows of a pass: all of them, else 192 or 256 (starts stay multiples of 64, and a pass within two 128-row
 // groups of scale factors), whichever leaves fewer passes, then fewer empty rows.

@@ -44,7 +44,6 @@
 #include "gb_common.cuh"
 
 #include <cuda.h>
-#include <mutex>
 #include <type_traits>
 
 namespace {
@@ -206,11 +205,6 @@ GB_DEVINL bool mbar_test(uint32_t bar, uint32_t parity) {   // never suspends: f
                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
-GB_DEVINL bool elect_one() {
-  uint32_t one;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-  return one != 0;
-}
 GB_DEVINL uint64_t desc_sw128(uint32_t addr) {
   uint64_t d = 0;
   d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
@@ -252,10 +246,6 @@ GB_DEVINL void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
                  "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(taddr));
-}
-GB_DEVINL void cluster_sync() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 GB_DEVINL uint4 lds128(uint32_t a) {
   uint4 v;
@@ -497,7 +487,7 @@ fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4
       *abort_flag = 1;
       atomicExch(p.status, 51);
     }
-    cluster_sync();                                        // peers write into this CTA's shared memory later: all must have started
+    gb_cluster_sync();                                        // peers write into this CTA's shared memory later: all must have started
   }
   const uint32_t tmem_base = *tmem_slot;
 
@@ -551,7 +541,7 @@ fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4
   // issue whatever its N; this way 11 (N = 16), 22 (48), 60 (128), and four of N = 48 have completed after 180 clocks instead of 413.
   if (warp == 0) {
     // ------------------------- packed weight rows -------------------------
-    const bool leader = elect_one();
+    const bool leader = gb_elect_one();
     int n = 0;                                             // stages since the start
     bool ok = true;
     for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
@@ -572,7 +562,7 @@ fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4
   } else if (warp == 1) {
     // ------------------------- activation operand --------------------------
     gb_pdl_wait();
-    const bool leader = elect_one();
+    const bool leader = gb_elect_one();
     int g = 0;                                             // units since the start, over all tiles and passes
     bool ok = true;
     for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
@@ -605,7 +595,7 @@ fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4
     // every unit with [hi | dlt], issuer 1 with [lo].
     const int i = __shfl_sync(0xffffffffu, warp, 0) - 2;
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
-    const bool leader = elect_one();
+    const bool leader = gb_elect_one();
     constexpr int u_step = wide ? 1 : 2;
     const uint32_t sf_col = 48u + (wide ? (uint32_t)i * 16u : 0u);
     const uint64_t db0 = desc_sw128(x_ring + (uint32_t)sfx);
@@ -1017,7 +1007,7 @@ fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (p.slices > 1)                                        // no CTA leaves while a peer may still reach its shared memory
-    cluster_sync();
+    gb_cluster_sync();
   if (warp == 4)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
 }
@@ -1280,7 +1270,7 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
     asm volatile("barrier.cluster.wait;" ::: "memory");
     to_peers(peer_top, top, p.split);
     to_peers(peer_low, low, p.split);
-    cluster_sync();                                        // the last access to another CTA's memory lies in front of it
+    gb_cluster_sync();                                        // the last access to another CTA's memory lies in front of it
     for (int q = 0; q < p.split; ++q) {
       top = max(top, peer_top[q]);
       low = min(low, peer_low[q]);
@@ -1304,7 +1294,7 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
       __shared__ uint32_t peer_sum[kMaxRowSplit], peer_count[kMaxRowSplit];
       to_peers(peer_sum, (uint32_t)sum, p.split);
       to_peers(peer_count, (uint32_t)count, p.split);
-      cluster_sync();
+      gb_cluster_sync();
       sum = count = 0;
       for (int q = 0; q < p.split; ++q) {
         sum += (int)peer_sum[q];
@@ -1333,7 +1323,7 @@ fp4_rows_kernel(const __grid_constant__ RowsParams p) {
     if (kMode == 0 && p.split > 1) {
       __shared__ uint32_t peer_all[kMaxRowSplit];
       to_peers(peer_all, left_out, p.split);
-      cluster_sync();
+      gb_cluster_sync();
       for (int q = 0; q < p.split; ++q) left_out |= peer_all[q];
     }
     for (int s = 0; s < copies; ++s) {
@@ -1427,28 +1417,8 @@ bool layout(const Info& f, Fp4Params& p) {
   return false;
 }
 
-std::mutex g_mutex;
-int g_clusters[64][kMaxSlices + 1];                        // clusters of a size that run at once, per device (0: not asked yet)
-
-int max_clusters(int size) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  std::lock_guard<std::mutex> lock(g_mutex);
-  int& n = g_clusters[dev][size];
-  if (n == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1, (unsigned)size);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemMax;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)size; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, fp4_decode_kernel<false, false, kLit>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); return 0; }
-  }
-  return n;
-}
+GbClusters g_clusters;
+int max_clusters(int size) { return g_clusters.ask((const void*)fp4_decode_kernel<false, false, kLit>, kThreads, kSmemMax, size); }
 
 template <bool kGrouped>
 cudaError_t launch(int F, dim3 grid, cudaStream_t stream, const Maps& maps, const Fp4Params& p) {

@@ -31,7 +31,6 @@
 #include "gb_common.cuh"
 
 #include <cuda.h>
-#include <mutex>
 
 namespace {
 
@@ -40,7 +39,7 @@ constexpr int kDecWarps = 16;                             // four warpgroups, on
 constexpr int kCtlWarps = 6;                              // raw producer, x producer, four MMA issuers
 constexpr int kUmmaThreads = 32 * (kCtlWarps + kDecWarps);
 constexpr int kMaxRows = 128;                             // activation rows
-constexpr int kMaxSlices = 16;                            // of K: CTAs of a cluster (past eight only where the GPU has room, see max_clusters)
+constexpr int kMaxSlices = 16;                            // of K: CTAs of a cluster (past eight only where the GPU has room)
 constexpr int kABufCols = 64;                             // half a superblock: 128 weights of K as bf16 pairs
 constexpr uint32_t kACol0 = 256;                          // columns [0, 256): one accumulator per MMA issuer
 constexpr uint32_t kTmemCols = 512;
@@ -183,16 +182,7 @@ GB_DEVINL bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_fla
   wait_or_abort(bar, parity, abort_flag, status, code);
   return !__any_sync(0xffffffffu, *abort_flag != 0);
 }
-GB_DEVINL bool elect_one() {
-  uint32_t one;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-  return one != 0;
-}
 
-GB_DEVINL void cluster_sync() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
-}
 GB_DEVINL void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
@@ -526,7 +516,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // there first, 53 clocks to issue an MMA whatever its size).
   if (warp == 0) {
     // ------------------------- packed weight rows -------------------------
-    const bool leader = elect_one();
+    const bool leader = gb_elect_one();
     int it = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
@@ -550,7 +540,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   } else if (warp == 1) {
     // ------------------------- activation slabs ---------------------------
     gb_pdl_wait();                                           // x may come from the launch ahead
-    const bool leader = elect_one();
+    const bool leader = gb_elect_one();
     const int k_base = r_begin * kSbPerStage * 256;
     int g = 0;                                               // units since the start, over all tiles and passes
     bool ok = true;
@@ -579,7 +569,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     // accumulator; the read-out adds the accumulators in their fixed order.
     const int i = __shfl_sync(0xffffffffu, warp, 0) - 2;
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
-    const bool leader = elect_one();
+    const bool leader = gb_elect_one();
     if (i < p.n_iss) {
       const uint32_t acc = tmem + (uint32_t)i * (kACol0 / (uint32_t)p.n_iss);
       const uint32_t slab16 = (uint32_t)slab_bytes >> 4;
@@ -817,7 +807,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       wait_or_abort(acc_full, 0, abort_flag, p.status, 26);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
-    cluster_sync();
+    gb_cluster_sync();
     if (warp >= kCtlWarps && *abort_flag == 0) {
       const int n_accs = min(p.n_iss, p.n_iss == 4 ? units : sb_slice);
       const uint32_t acc_stride = kACol0 / (uint32_t)p.n_iss;
@@ -839,7 +829,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst + (uint32_t)i * kBM * 4u), "r"(v[i]) : "memory");
       }
     }
-    cluster_sync();                                          // the last access to another CTA's memory lies in front of it
+    gb_cluster_sync();                                          // the last access to another CTA's memory lies in front of it
     if (warp >= kCtlWarps) {
       gb_pdl_wait();                                         // y may still be read by the launch ahead
       const int f = lane * 4, left = T.n_end - T.n0 - f, last = min(own, p.M - slice * own);
@@ -896,28 +886,8 @@ int umma_x_stages(int F, int Mpad) {
 
 int umma_smem_bytes(int F, int Mpad) { return fmt_info(F).fixed_smem + umma_x_stages(F, Mpad) * (2 * Mpad * 128); }
 
-std::mutex g_mutex;
-int g_clusters[64][kMaxSlices + 1];                        // clusters of a size that run at once, per device (0: not asked yet)
-
-int max_clusters(int size) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  std::lock_guard<std::mutex> lock(g_mutex);
-  int& n = g_clusters[dev][size];
-  if (n == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1, (unsigned)size);
-    cfg.blockDim = dim3(kUmmaThreads);
-    cfg.dynamicSmemBytes = kSmemCap;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)size; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, umma_decode_kernel<false, kFmtFp8>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
-  }
-  return n;
-}
+GbClusters g_clusters;
+int max_clusters(int size) { return g_clusters.ask((const void*)umma_decode_kernel<false, kFmtFp8>, kUmmaThreads, kSmemCap, size); }
 
 // K slices: enough CTAs for the SMs when the layer has few 128-row tiles; no more clusters than run at once.  Eight at most lost
 // against a slice per raw stage and a second launch where two or four tiles have a long K (us, those / eight / sixteen: fp8 k = 32,
