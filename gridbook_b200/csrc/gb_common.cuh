@@ -527,6 +527,9 @@ GB_DEVINL void gb_mbar_arrive(uint64_t* bar) {
 // kernel before it on the stream is still running; gb_pdl_wait() returns once that kernel
 // (and everything before it) has completed and its writes are visible, so it must come before
 // the first read of anything an earlier kernel produced and before the first global write.
+// One exception: an expander behind the launch that quantises the rows (gb_expand_*_beside) writes first and waits before it
+// exits.  It may, because that launch lets it start only behind its OWN wait - all work further ahead, the last reader of the
+// expander's output too, has completed - and neither reads nor writes what the other writes.
 // What sits in front of it - barrier setup, the prefetch of weights, tables of constants -
 // overlaps the predecessor's tail.  gb_pdl_launch_dependents() lets the successor start.
 GB_DEVINL void gb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -184,9 +184,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
   const int total_tiles = base_s[p.E] * p.n_tiles;
 
-  // Every role walks the same tile sequence: tile = blockIdx.x, + gridDim.x, ...; M tiles vary
-  // fastest, so the CTAs working at the same time share a few B (weight) tiles and sweep A,
-  // which fits L2: the decoded weight tile is read from HBM once.
+  // Every role walks the same tile sequence: tile = blockIdx.x, + gridDim.x, ...; N tiles vary fastest, so the CTAs
+  // working at the same time share an expert's rows and sweep its decoded weights, which stay in L2.
   if (warp == 4) {
     // ------------------------------- TMA producer -------------------------------
     if (lane == 0) {

@@ -50,7 +50,7 @@ namespace {
 
 constexpr int kBM = 128;
 constexpr int kDecWarps = 16;
-constexpr int kCtlWarps = 8;                              // packed rows, activations, up to four MMA issuers, two idle
+constexpr int kCtlWarps = 8;                              // packed rows, activations, two MMA issuers, four for the scale factors
 constexpr int kThreads = 32 * (kCtlWarps + kDecWarps);
 constexpr int kMaxRows = 64;                              // activation rows per pass (three columns each)
 constexpr int kMaxRaw = 8, kMaxX = 8;
@@ -437,7 +437,7 @@ fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4
   // tell a phase from the one two before); with four or eight units in a ring, a slot's units are always the same
   // warpgroup's, so only that one waits for it.
   const int span = (units + T::kSbPerStage - 1) / T::kSbPerStage * T::kSbPerStage;
-  // Layout of tensor memory.  Narrow: four accumulators of 64 columns, one per warpgroup and issuer; wide:
+  // Layout of tensor memory.  Narrow: four accumulators of 64 columns, one per warpgroup, two issuers in turn; wide:
   // [hi | dlt] in columns [0, 128), [lo] in [128, 192), one issuer each.  Then the four operand
   // buffers: nibbles (32), weight scale factors (16), activation scale factors (16 per set).
   constexpr bool wide = kWide;
