@@ -11,7 +11,8 @@
 // front of them (in order on one thread; a stage has a column set of its own, free once the stage is).
 //
 // Bound by the operand loads: 16 KiB of weights and 128 bytes per activation row for every 128-byte K slab, of which an
-// SM takes in about 50 bytes a clock; by launch and prologue (2 us) where K is short.
+// SM takes in 42 bytes a clock behind the expander (128 rows of 8192 x 5120 fp8, 160 of 5120 x 17408 fp4; 31 and 38 where they come
+// from HBM, which, the tensor pipe and the issue slots are then at 30, 25 and 13 %); by launch and prologue (2 us) where K is short.
 #include "gb_common.cuh"
 
 #include <cuda.h>
