@@ -196,6 +196,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int kt = 0; kt < p.k_tiles; ++kt, ++kk) {
           const int s = kk % kStages;
           wait_or_abort(&empty_bar[s], ((kk / kStages) & 1) ^ 1, abort_flag, p.status, 11);
+          if (*abort_flag) break;                        // nothing more may be in flight when the CTA leaves
           gb_mbar_expect_tx(&full_bar[s], kStageBytes);
           uint8_t* a_dst = ring + (size_t)s * kStageBytes;
           tma_load_2d(a_dst, &map_a, kt * slab_elems, t.m0, &full_bar[s]);
@@ -221,7 +222,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t tmem_d = tmem + (uint32_t)(buf * kBN);
       for (int kt = 0; kt < p.k_tiles; ++kt) {
         wait_or_abort(&full_bar[s], ph, abort_flag, p.status, 12);
-        __syncwarp();
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a_addr = gb_smem_u32(ring) + (uint32_t)s * kStageBytes;
         const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + kBM * kSlabBytes);
@@ -300,6 +301,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (*abort_flag) __nanosleep(1000000);                   // loads and MMAs still in flight end before the memory goes
   if (warp == 5) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTmemCols)
                  : "memory");

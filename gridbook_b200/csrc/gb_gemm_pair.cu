@@ -594,9 +594,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   }
   __syncwarp();
-  if (*abort_flag && threadIdx.x == 0) __nanosleep(1000000);   // loads still in flight land before the memory goes
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (*abort_flag) __nanosleep(1000000);                   // loads and MMAs still in flight end before the memory goes
   gb_cluster_sync();                                            // the peer may still signal barriers here
   if (warp == kEpiWarps + 1)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTmemCols) : "memory");

@@ -314,9 +314,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
   }
   __syncwarp();
-  if (abort_s && threadIdx.x == 0) __nanosleep(1000000);     // loads still in flight land before the memory goes
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (abort_s) __nanosleep(1000000);                   // loads and MMAs still in flight end before the memory goes
   if (warp == kEpiWarps + 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }

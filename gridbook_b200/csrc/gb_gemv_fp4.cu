@@ -1006,6 +1006,7 @@ fp4_decode_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Fp4
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (*abort_flag) __nanosleep(1000000);                   // loads and MMAs still in flight end before the memory goes
   if (p.slices > 1)                                        // no CTA leaves while a peer may still reach its shared memory
     gb_cluster_sync();
   if (warp == 4)

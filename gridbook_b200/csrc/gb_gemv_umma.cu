@@ -851,6 +851,7 @@ umma_decode_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (*abort_flag) __nanosleep(1000000);                   // loads and MMAs still in flight end before the memory goes
   if (warp == 2) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols)
                  : "memory");

@@ -115,3 +115,24 @@ def test_peers_are_written_to_only_after_the_whole_cluster_has_started():
                 name = re.search(r"(\w+)\(const", kernel).group(1)
                 assert re.search(r"cluster_sync\(\);|barrier\.cluster\.wait", kernel[:store.start()]), f"{f}: {name}"
     assert found >= 4
+
+
+def test_a_kernel_that_gives_up_waits_for_what_it_has_in_flight():
+    """A bounded wait may run out while loads or MMAs of the CTA are on their way: their shared and tensor memory is given back only
+    after a while, and whoever issues them has stopped."""
+    csrc = os.path.join(PKG, "csrc")
+    found = 0
+    for f in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, f)) as fh:
+            text = re.sub(r"//[^\n]*", "", fh.read())
+        for kernel in re.split(r"\b__global__\b", text)[1:]:
+            free = kernel.find("tcgen05.dealloc")
+            if free < 0:
+                continue
+            found += 1
+            name = re.search(r"(\w+)\(const", kernel).group(1)
+            assert re.search(r"__syncthreads\(\);\s*if \(\*?abort_\w+\) __nanosleep\(", kernel[:free]), f"{f}: {name}"
+            loads = [m.start() for m in re.finditer(r"\btma_load\w*\(|\bbulk_load\(", kernel)]
+            waits = [m.end() for m in re.finditer(r"(?:if \(!|ok = )warp_wait[^\n]*\n|if \(\*abort_flag\) break;", kernel)]
+            assert loads and waits and min(waits) < min(loads), f"{f}: {name}"
+    assert found >= 5
